@@ -301,6 +301,10 @@ typedef struct {
 const char* umbs_version(void);
 unsigned long long umbs_launch_count(void);
 
+/* Blocks that gave up on a bounded wait inside a kernel since the library was loaded (0 unless something is broken; their
+ * results are not to be used).  Synchronises. */
+unsigned int umbs_kernel_timeouts(void);
+
 /* Bytes of scratch umbs_forward needs for a step of up to max_tokens tokens of which up to max_want want logits. */
 size_t umbs_workspace_bytes(const umbs_model_t* model, int max_tokens, int max_want);
 

@@ -1,0 +1,90 @@
+"""The tensor-core matrix product of steps with more than 16 rows (csrc/seq/seq_gemm_tc.cu) against float64, at the sizes where
+its tiles end: rows around 128, columns around 32 / 64 / 128 / 256, k around 64, odd row lengths of C, groups without rows.
+
+Tolerances: operands are bf16 and products exact, so an fp32 result differs from float64 by the rounding of a sum of K terms:
+K 2^-24 in the worst case, about sqrt(K) 2^-24 for random signs; 1e-5 covers K <= 1056 with a tensor core that truncates.
+bf16 results (8 significant bits) are off by at most 2^-8 relative each, so by no more in the norm."""
+import pytest
+import torch
+
+import seq_helpers as H
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+F32_TOL, BF16_TOL = 1e-5, 2.0 ** -8
+
+
+def _mat(seed, *shape, scale=1.0):
+    return (torch.randn(*shape, generator=torch.Generator().manual_seed(seed)) * scale).bfloat16().to(DEV)
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from umbrella_b200 import _lib_seq, ops_seq
+    yield ops_seq
+    assert _lib_seq.load().umbs_kernel_timeouts() == 0
+
+
+# one tile, its edges, several tiles per block; columns that leave 16-byte rows of C and columns that do not
+@pytest.mark.parametrize("M,N,K", [(17, 8, 32), (128, 64, 64), (127, 65, 96), (129, 257, 64), (300, 1544, 1056), (64, 6144, 128),
+                                   (2049, 513, 192), (1500, 3088, 256)])
+def test_plain(ops, M, N, K):
+    a, w = _mat(1, M, K), _mat(2, N, K)
+    ref = a.double() @ w.double().T
+    assert H.rel_err(ops.gemm(a, w, out_f32=True), ref.cpu()) < F32_TOL
+    assert H.rel_err(ops.gemm(a, w), ref.cpu()) < BF16_TOL
+
+
+def test_rows_are_bitwise_the_same_in_every_tile_width(ops):
+    a, w = _mat(3, 2100, 512), _mat(4, 2048, 512)               # 17 x 8 tiles of 256 columns; 64 rows alone: tiles of 64
+    full = ops.gemm(a, w, out_f32=True)
+    assert torch.equal(ops.gemm(a[1030:1094].contiguous(), w, out_f32=True), full[1030:1094])
+    assert torch.equal(ops.gemm(a[5:305].contiguous(), w, out_f32=True), full[5:305])
+
+
+@pytest.mark.parametrize("M,N,K", [(40, 33, 64), (200, 128, 96), (1000, 1000, 64)])
+def test_epilogues(ops, M, N, K):
+    from umbrella_b200 import _lib_seq as S
+    a, w, w2 = _mat(5, M, K), _mat(6, N, K, scale=K ** -0.5), _mat(7, 2 * N, K, scale=K ** -0.5)
+    bias, gate = torch.randn(2 * N, device=DEV), torch.randn(M, N, device=DEV)
+    z, z2 = a.double() @ w.double().T, a.double() @ w2.double().T
+    got = ops.gemm_ex(a, w, out_f32=True, bias=bias, out_gate=gate)
+    assert H.rel_err(got, ((z + bias[:N].double()) * torch.sigmoid(gate.double())).cpu()) < F32_TOL
+    got = ops.gemm_ex(a, w2, out_f32=True, act=S.UMBS_ACT_SILU, bias=bias)
+    g, u = (z2 + bias.double()).split(N, 1)
+    assert H.rel_err(got, (torch.nn.functional.silu(g) * u).cpu()) < F32_TOL
+    got = ops.gemm_unary(a, w, S.UMBS_UNARY_RELU2, out_f32=True, cols=N // 2)
+    assert H.rel_err(got, torch.cat([z[:, :N // 2].clamp(min=0) ** 2, z[:, N // 2:]], 1).cpu()) < F32_TOL
+
+
+@pytest.mark.parametrize("M,heads,n,k", [(33, 3, 48, 32), (260, 5, 128, 64), (130, 2, 320, 96)])
+def test_batched_over_heads(ops, M, heads, n, k):
+    a, w = _mat(8, M, heads * k), _mat(9, heads, n, k)
+    ref = torch.einsum("mhk,hnk->mhn", a.double().view(M, heads, k), w.double())
+    got = ops.gemm(a, w, out_f32=True, groups=heads, a_goff=k, c_goff=n + 2)     # (an odd place for every head's columns)
+    assert H.rel_err(got.view(M, heads, n + 2)[..., :n], ref.cpu()) < F32_TOL
+    gate = torch.randn(M, heads, device=DEV)
+    got = ops.gemm_head_gate(a, w, gate, heads, n, k)
+    assert H.rel_err(got, (ref * torch.sigmoid(gate.double())[..., None]).reshape(M, -1).cpu()) < BF16_TOL
+
+
+@pytest.mark.parametrize("sizes", [(17, 0, 3, 128, 129), (0, 0, 300, 1, 0), (700, 650, 640, 660, 655)])
+@pytest.mark.parametrize("K", [64, 160])
+def test_rows_sorted_by_expert(ops, sizes, K):
+    """Gathered rows with the gated activation, then the sorted rows themselves; groups without rows, of one row, of a tile and a row."""
+    E, n, total = len(sizes), 96, sum(sizes)
+    off = torch.tensor([0] + list(torch.tensor(sizes).cumsum(0)), dtype=torch.int32, device=DEV)
+    T = max(max(sizes), 20)
+    src = torch.randint(0, T, (total,), generator=torch.Generator().manual_seed(1)).to(torch.int32).to(DEV)
+    h, gu, down = _mat(10, T, K), _mat(11, E, 2 * n, K, scale=K ** -0.5), _mat(12, E, 72, n, scale=n ** -0.5)
+    y = ops.gemm(h, gu, groups=E, n=n, dual=True, limit=7.0, grp_off=off, row_src=src, rows=total, max_rows=T)
+    o = ops.gemm(y, down, out_f32=True, groups=E, grp_off=off, rows=total, max_rows=T)
+    at = 0
+    for e, m in enumerate(sizes):
+        if m == 0:
+            continue
+        z = h[src[at:at + m].long()].double() @ gu[e].double().T
+        g, u = z[:, :n].clamp(max=7.0), z[:, n:].clamp(-7.0, 7.0)
+        assert H.rel_err(y[at:at + m], (g * torch.sigmoid(1.702 * g) * (u + 1)).cpu()) < BF16_TOL
+        assert H.rel_err(o[at:at + m], (y[at:at + m].double() @ down[e].double().T).cpu()) < F32_TOL
+        at += m

@@ -128,6 +128,7 @@ _BP = C.POINTER(Batch)
 SIGNATURES = {
     "umbs_version": (C.c_char_p, []),
     "umbs_launch_count": (C.c_ulonglong, []),
+    "umbs_kernel_timeouts": (C.c_uint, []),
     "umbs_workspace_bytes": (c_size_t, [C.POINTER(Model), c_int, c_int]),
     "umbs_forward": (c_int, [C.POINTER(Model), _BP, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
     "umbs_gemm": (c_int, [c_int, c_void_p, c_int64, c_int, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int, c_int,

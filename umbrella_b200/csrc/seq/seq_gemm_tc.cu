@@ -1,0 +1,380 @@
+// Matrix products of steps with more than a few rows on the 5th-generation tensor cores: C = A W^T, bf16 operands, fp32 sums
+// in tensor memory.
+//
+// A persistent block per SM walks output tiles of 128 rows x BN columns.  Warp 0 copies weight tiles (and, for dense rows,
+// activation tiles) with TMA into a ring of 64-wide k steps, one thread of warp 1 issues tcgen05.mma, warps 2-5 empty the
+// accumulators -- two sets of them, so that a tile is stored while the next one is summed.  Rows that are gathered or sorted by
+// expert come from four more warps through 16-byte cp.async: which rows a tile has is known on the device alone, and a tile
+// of few rows fetches only those.
+//
+// An output element is one fp32 sum over k in the same order whatever its tile's size, so a row's result does not depend on
+// the rest of the batch; against float64 it is as far off as the mma.sync tiles that this replaced (2.1e-6 at K = 2048, in
+// both the tensor core's own accumulation).
+//
+// Bound: the tensor cores for dense prompts.  4096 x 2048 -> 6144 (fp32 out): 650 us on 128 x 64 mma.sync tiles (159 TFLOP/s,
+// fragments fetched from shared memory by every warp), 120 us here with the 100 MB memset of the output in both.  16 experts,
+// top 2, 4096 tokens of width 2048 with the routing around it: 808 -> 435 us; 64 tokens: 212 -> 152 us.
+#include <cuda.h>
+
+#include "../common.cuh"
+#include "seq_gemm.h"
+
+namespace umbs {
+using umb::smem_u32;
+
+constexpr int kTcRows = 128, kTcK = 64, kTcLag = 3;         // tile rows; k per ring stage; stages in flight per copying thread
+constexpr int kTcStageRow = 36;                             // fp32 row stride of an epilogue warp's 32 x 32 staging block
+
+struct TcArgs {
+    int groups, n_tiles, m_tiles, k_steps;
+    int vec_c;                                              // rows of C take 16-byte (fp32) / 8-byte (bf16) stores of 4 columns
+    int a_grouped, w_grouped;                               // the group coordinate of the tensor maps is used
+};
+
+__device__ unsigned int g_tc_timeouts;                      // launches that gave up on a wait (umbs_kernel_timeouts)
+
+// Every wait is bounded (about a second): a block that gives up raises the flag, and every role of it leaves its loop.
+__device__ __forceinline__ bool tc_give_up(volatile int* quit) {
+    if (!*quit) {
+        *quit = 1;
+        atomicAdd(&g_tc_timeouts, 1u);
+    }
+    return false;
+}
+__device__ __forceinline__ bool tc_spin(uint64_t* bar, uint32_t parity, volatile int* quit) {
+    for (int i = 0; i < (1 << 25); ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+        if (ok) return true;
+        if ((i & 1023) == 1023 && *quit) return false;
+    }
+    return tc_give_up(quit);
+}
+__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* quit) {
+    for (int i = 0; i < (1 << 20); ++i) {
+        if (umb::mbar_try_wait(bar, parity)) return true;   // (parks the thread for about a microsecond)
+        if (*quit) return false;
+    }
+    return tc_give_up(quit);
+}
+
+__device__ __forceinline__ void tma_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar)) : "memory");
+}
+
+__host__ __device__ constexpr uint32_t tc_idesc(uint32_t M, uint32_t N) {       // kind::f16, bf16 x bf16 -> fp32, both operands K-major
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
+}
+
+// The tiles of a block, in the order every role visits them: rows fastest, then columns, then groups.
+struct TileWalk {
+    const GemmArgs& a; const TcArgs& t;
+    int next, g, first, m_tiles, row_lo, rows, m0, n0;
+    __device__ TileWalk(const GemmArgs& a_, const TcArgs& t_) : a(a_), t(t_), next(blockIdx.x), g(-1), first(0), m_tiles(0), row_lo(0), rows(a_.M), m0(0), n0(0) {}
+    __device__ bool step() {
+        while (next >= first + m_tiles * t.n_tiles) {
+            if (++g >= t.groups) return false;
+            first += m_tiles * t.n_tiles;
+            if (a.grp_off != nullptr) {
+                row_lo = a.grp_off[g];
+                rows = a.grp_off[g + 1] - row_lo;
+                m_tiles = (rows + kTcRows - 1) / kTcRows;
+            } else {
+                m_tiles = t.m_tiles;
+            }
+        }
+        const int i = next - first;
+        m0 = i % m_tiles * kTcRows;
+        n0 = i / m_tiles;                                   // in tiles: the caller knows their width
+        next += gridDim.x;
+        return true;
+    }
+};
+
+template <int BN, bool DUAL>
+struct TcCfg {
+    static constexpr int kStages = BN == 256 ? 4 : (BN == 128 ? 6 : 8);
+    static constexpr int kABytes = kTcRows * 128, kWBytes = BN * 128, kStage = kABytes + kWBytes;
+    static constexpr int kOut = DUAL ? BN / 2 : BN;         // output columns of a tile
+    static constexpr int kSmem = 1024 + kStages * kStage + 4 * 32 * kTcStageRow * 4 + 256;
+};
+
+template <int BN, bool DUAL, bool A_TMA, typename TC>
+__global__ void __launch_bounds__(A_TMA ? 192 : 320, 1)
+gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const GemmArgs a, const TcArgs t) {
+    using Cfg = TcCfg<BN, DUAL>;
+    constexpr int kStages = Cfg::kStages, kOut = Cfg::kOut;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    float* s_out = reinterpret_cast<float*>(smem + kStages * Cfg::kStage);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(s_out + 4 * 32 * kTcStageRow);
+    uint64_t *full = bars, *empty = bars + kStages, *acc_full = bars + 2 * kStages, *acc_empty = acc_full + 2;
+    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    volatile int* quit = reinterpret_cast<volatile int*>(s_tmem + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        umb::tma_prefetch_desc(&map_w);
+        if (A_TMA) umb::tma_prefetch_desc(&map_a);
+        for (int i = 0; i < kStages; ++i) {
+            umb::mbar_init(full + i, A_TMA ? 1 : 5);        // the TMA thread, and the four copying warps
+            umb::mbar_init(empty + i, 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            umb::mbar_init(acc_full + i, 1);
+            umb::mbar_init(acc_empty + i, 4);
+        }
+        *quit = 0;
+        umb::fence_barrier_init();
+    }
+    if (warp == 1) {
+        umb::tmem_alloc(s_tmem, 2 * BN);
+        umb::tmem_relinquish();
+    }
+    umb::tc_fence_before();
+    __syncthreads();
+    umb::tc_fence_after();
+    const uint32_t tmem = *s_tmem;
+    TileWalk w(a, t);
+
+    if (warp == 0) {
+        if (lane == 0) {
+            uint32_t s = 0, ph = 1;
+            bool ok = true;
+            while (ok && w.step()) {
+                for (int k = 0; k < t.k_steps; ++k) {
+                    if (!(ok = tc_spin(empty + s, ph, quit))) break;
+                    unsigned char* st = smem + s * Cfg::kStage;
+                    umb::mbar_arrive_expect_tx(full + s, (A_TMA ? Cfg::kABytes : 0) + Cfg::kWBytes);
+                    if (A_TMA) tma_3d(st, &map_a, k * kTcK, w.m0, t.a_grouped ? w.g : 0, full + s);
+                    const int gw = t.w_grouped ? w.g : 0, n0 = w.n0 * kOut;
+                    tma_3d(st + Cfg::kABytes, &map_w, k * kTcK, n0, gw, full + s);
+                    if (DUAL) tma_3d(st + Cfg::kABytes + kOut * 128, &map_w, k * kTcK, a.N + n0, gw, full + s);
+                    if (++s == kStages) { s = 0; ph ^= 1; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = tc_idesc(kTcRows, BN);
+            uint32_t s = 0, ph = 0, it = 0;
+            bool ok = true;
+            for (; ok && w.step(); ++it) {
+                const uint32_t acc = it & 1, d = tmem + acc * BN;
+                if (!(ok = tc_spin(acc_empty + acc, ((it >> 1) & 1) ^ 1, quit))) break;
+                umb::tc_fence_after();
+                for (int k = 0; k < t.k_steps; ++k) {
+                    if (!(ok = tc_spin(full + s, ph, quit))) break;
+                    umb::tc_fence_after();
+                    const uint32_t st = smem_u32(smem + s * Cfg::kStage);
+                    const uint64_t ad = umb::umma_smem_desc_sw128(st), wd = umb::umma_smem_desc_sw128(st + Cfg::kABytes);
+#pragma unroll
+                    for (int kk = 0; kk < kTcK / 16; ++kk)
+                        umb::umma_ss_f16(d, ad + kk * 2, wd + kk * 2, idesc, (k | kk) ? 1u : 0u);
+                    umb::umma_commit(empty + s);
+                    if (++s == kStages) { s = 0; ph ^= 1; }
+                }
+                if (ok) umb::umma_commit(acc_full + acc);
+            }
+        }
+    } else if (warp < 6) {
+        const int q = warp & 3;                             // the quarter of tensor-memory lanes this warp may read
+        float* so = s_out + (warp - 2) * 32 * kTcStageRow;
+        const int rr = lane >> 3, cc = (lane & 7) * 4;
+        for (uint32_t it = 0; w.step(); ++it) {
+            const uint32_t acc = it & 1;
+            if (!tc_wait(acc_full + acc, (it >> 1) & 1, quit)) break;
+            umb::tc_fence_after();
+            const uint32_t src = tmem + acc * BN + ((uint32_t)(q * 32) << 16);
+            const int rows = w.rows - w.m0 - q * 32, n_hi = a.N - w.n0 * kOut;      // rows of this quarter, columns of the tile
+            TC* C = (TC*)a.C + (int64_t)w.g * a.c_goff + (int64_t)(w.row_lo + w.m0 + q * 32) * a.ldc + w.n0 * kOut;
+            const int64_t grow = w.row_lo + w.m0 + q * 32;
+#pragma unroll 1
+            for (int c0 = 0; c0 < kOut; c0 += 32) {
+                uint32_t v[32], u[DUAL ? 32 : 1];
+                UMB_TMEM_LD_X32(src + c0, v);
+                if (DUAL) UMB_TMEM_LD_X32(src + kOut + c0, u);
+                umb::tc_wait_ld();
+                if (c0 + 32 >= kOut) {                      // read to the end: the next tile but one may be summed here
+                    umb::tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) umb::mbar_arrive(acc_empty + acc);
+                }
+                if (c0 >= n_hi || rows <= 0) continue;
+                if (DUAL || a.bias != nullptr || a.unary) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        v[j] = __float_as_uint(finish_sum<DUAL>(a, __uint_as_float(v[j]), DUAL ? __uint_as_float(u[DUAL ? j : 0]) : 0.f,
+                                                                min(w.n0 * kOut + c0 + j, a.N - 1)));
+                }
+#pragma unroll
+                for (int j = 0; j < 32; j += 4)
+                    *reinterpret_cast<uint4*>(so + lane * kTcStageRow + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int r = i * 4 + rr, n = c0 + cc;
+                    if (r < rows && n < n_hi) {
+                        const float4 f = *reinterpret_cast<const float4*>(so + r * kTcStageRow + cc);
+                        float o[4] = {f.x, f.y, f.z, f.w};
+                        if (a.out_gate != nullptr) {
+#pragma unroll
+                            for (int e = 0; e < 4; ++e)
+                                if (n + e < n_hi) o[e] = finish_gate(a, o[e], w.g, grow + r, w.n0 * kOut + n + e);
+                        }
+                        TC* p = C + (int64_t)r * a.ldc + n;
+                        if (t.vec_c && n + 4 <= n_hi) {
+                            if constexpr (sizeof(TC) == 4) {
+                                *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]);
+                            } else {
+                                __nv_bfloat162 lo = __floats2bfloat162_rn(o[0], o[1]), hi = __floats2bfloat162_rn(o[2], o[3]);
+                                *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+                            }
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 4; ++e)
+                                if (n + e < n_hi) p[e] = from_f32<TC>(o[e]);
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+        }
+    } else if (!A_TMA) {
+        // a warp's eight lanes copy a row's 128 bytes of the k step, 128 / 16 rows per thread; the image is the one a
+        // 128-byte-swizzled TMA box would leave
+        const int tid = threadIdx.x - 192, ch = tid & 7, r0 = tid >> 3;
+        const __nv_bfloat16* A = (const __nv_bfloat16*)a.A + ch * 8;
+        uint32_t s = 0, ph = 1, done = 0, issued = 0;
+        const uint32_t dst0 = r0 * 128 + ((ch ^ (r0 & 7)) << 4);        // r0 + 16 i keeps r0's place inside its group of eight rows
+        bool ok = true;
+        auto publish = [&]() {
+            umb::fence_proxy_async_smem();                  // the copies of this thread are complete: show them to the tensor core
+            __syncwarp();
+            if (lane == 0) umb::mbar_arrive(full + done % kStages);
+            ++done;
+        };
+        while (ok && w.step()) {
+            int64_t row[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int r = w.m0 + r0 + 16 * i, p = w.row_lo + r;
+                row[i] = r < w.rows ? (int64_t)(a.row_src ? a.row_src[p] : p) * a.lda + (t.a_grouped ? (int64_t)w.g * a.a_goff : 0) : -1;
+            }
+            for (int k = 0; k < t.k_steps; ++k) {
+                if (!(ok = tc_wait(empty + s, ph, quit))) break;
+                const uint32_t dst = smem_u32(smem + s * Cfg::kStage) + dst0;
+                const int kc = k * kTcK + ch * 8;
+                const int bytes = kc < a.K ? 16 : 0;        // behind the last column: zeros (K is a multiple of 8)
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (row[i] >= 0)                        // a row that is not there keeps what the stage held: its sums are not stored
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + i * 2048),
+                                     "l"(A + row[i] + (bytes ? k * kTcK : 0)), "r"(bytes) : "memory");
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                if (++s == kStages) { s = 0; ph ^= 1; }
+                if (++issued > kTcLag) {
+                    asm volatile("cp.async.wait_group %0;" ::"n"(kTcLag) : "memory");
+                    publish();
+                }
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        while (done < issued) publish();
+    }
+    __syncthreads();
+    if (*quit) {                                            // gave up: let copies and products in flight end before the memory goes
+        for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+        __syncthreads();
+    }
+    if (warp == 1) {
+        umb::tc_fence_after();
+        umb::tmem_dealloc(tmem, 2 * BN);
+    }
+}
+
+// ------------------------------------------------------------------------------------------------ host side
+typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static EncodeTiled encode_tiled() {
+    static const EncodeTiled fn = [] {
+        void* sym = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &q) == cudaSuccess &&
+                       q == cudaDriverEntryPointSuccess ? (EncodeTiled)sym : nullptr;
+    }();
+    return fn;
+}
+
+// bf16 [groups][rows][cols] with row stride ld and group stride gs (elements): boxes of 64 columns x box_rows rows, 128-byte swizzle
+static int encode_map(CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows, uint64_t groups, uint64_t ld, uint64_t gs,
+                      uint32_t box_rows) {
+    const EncodeTiled enc = encode_tiled();
+    if (enc == nullptr) return UMB_ERR_DRIVER;
+    const cuuint64_t dims[3] = {cols, rows, groups}, strides[2] = {ld * 2, (groups > 1 ? gs : ld * rows) * 2};
+    const cuuint32_t box[3] = {64, box_rows, 1}, one[3] = {1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
+               ? 0 : UMB_ERR_DRIVER;
+}
+
+template <int BN, bool DUAL, bool A_TMA, typename TC>
+static int launch_tc(const GemmArgs& a, TcArgs t, int sms, cudaStream_t st) {
+    using Cfg = TcCfg<BN, DUAL>;
+    t.n_tiles = (a.N + Cfg::kOut - 1) / Cfg::kOut;
+    t.k_steps = (a.K + kTcK - 1) / kTcK;
+    const int ga = a.a_goff != 0 ? t.groups : 1, gw = a.w_gstride != 0 ? t.groups : 1;
+    t.a_grouped = ga > 1;
+    t.w_grouped = gw > 1;
+    CUtensorMap ma{}, mw;
+    int rc = encode_map(&mw, a.W, a.K, (uint64_t)a.N * (DUAL ? 2 : 1), gw, a.ldw, a.w_gstride, Cfg::kOut);
+    if (rc == 0 && A_TMA) rc = encode_map(&ma, a.A, a.K, a.M, ga, a.lda, a.a_goff, kTcRows);
+    if (rc != 0) return rc;
+    auto kernel = gemm_tc_kernel<BN, DUAL, A_TMA, TC>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
+    if (e != cudaSuccess) return (int)e;
+    const int64_t tiles = (int64_t)t.groups * t.m_tiles * t.n_tiles;            // (sorted by expert: at most)
+    kernel<<<(int)(tiles < sms ? tiles : sms), A_TMA ? 192 : 320, Cfg::kSmem, st>>>(ma, mw, a, t);
+    return 0;
+}
+
+template <int BN>
+static int launch_tc_any(const GemmArgs& a, const TcArgs& t, bool dual, bool c_f32, int sms, cudaStream_t st) {
+    const bool sorted = a.grp_off != nullptr || a.row_src != nullptr;
+#define UMBS_TC(D, S) (c_f32 ? launch_tc<BN, D, S, float>(a, t, sms, st) : launch_tc<BN, D, S, __nv_bfloat16>(a, t, sms, st))
+    if (dual) return sorted ? UMBS_TC(true, false) : UMBS_TC(true, true);
+    return sorted ? UMBS_TC(false, false) : UMBS_TC(false, true);
+#undef UMBS_TC
+}
+
+int launch_gemm_tc(const GemmArgs& a, int groups, bool dual, bool c_f32, cudaStream_t st) {
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return (int)e;
+    TcArgs t{};
+    t.groups = groups;
+    t.m_tiles = (a.M + kTcRows - 1) / kTcRows;
+    const int es = c_f32 ? 4 : 2;
+    t.vec_c = (uintptr_t)a.C % (4 * es) == 0 && a.ldc % 4 == 0 && a.c_goff % 4 == 0;
+    // The widest tile that still gives every SM one: 256 columns need the least shared-memory traffic per product.  (Rows
+    // sorted by expert: how they fall is only known on the device; spread evenly is the guess.)
+    const int64_t m = a.grp_off != nullptr ? (int64_t)groups * ((a.M + groups * kTcRows - 1) / (groups * kTcRows)) : (int64_t)groups * t.m_tiles;
+    auto enough = [&](int bn) { const int out = dual ? bn / 2 : bn; return m * ((a.N + out - 1) / out) >= sms; };
+    if (enough(256)) return launch_tc_any<256>(a, t, dual, c_f32, sms, st);
+    if (enough(128)) return launch_tc_any<128>(a, t, dual, c_f32, sms, st);
+    return launch_tc_any<64>(a, t, dual, c_f32, sms, st);
+}
+
+}  // namespace umbs
+
+extern "C" unsigned int umbs_kernel_timeouts(void) {
+    unsigned int n = 0;
+    return cudaMemcpyFromSymbol(&n, umbs::g_tc_timeouts, sizeof n) == cudaSuccess ? n : ~0u;
+}
