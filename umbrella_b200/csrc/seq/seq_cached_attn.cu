@@ -23,53 +23,12 @@
 #include <algorithm>
 #include <stdint.h>
 
-#include "seq_internal.h"
+#include "seq_attn.h"
 
 namespace umbs {
 
 constexpr int kCaQ = 64, kCaK = 64, kCaS = 68;        // rows and keys per tile; row stride of the [d][row] tiles
 constexpr int kCaD = 64;                              // dimensions of a key tile held at a time
-
-struct CachedAttnArgs {
-    const void* q; const void* kv; const void* kv_cache; const void* pool_cache;
-    int kv_len, pool_len;
-    int heads, kv_heads, dim, vdim, window, pool;
-    float scale;
-    const float* head_bias; const float* gate; int64_t ldg; int gate_per_head;
-    void* out;
-    // score options
-    float softcap; const float* r1; const float* r2; int chunk, maps, vheads; float* raw;
-    const float* sink;                                // [heads] or NULL: the sink's score per head (NULL: 0)
-};
-__device__ __forceinline__ float sink_score(const CachedAttnArgs& a, int h) { return a.sink != nullptr ? a.sink[h] : 0.f; }
-
-// What a virtual head reads: its query's offset in a q row, its keys' and values' offsets in a key/value row.
-struct VHead { int h, qoff, koff, voff, row_kv, qstride, nv; };
-__device__ __forceinline__ VHead virtual_head(const CachedAttnArgs& a, int vh) {
-    const int C = a.vheads, M = a.maps;
-    const int cv = vh % C, hm = vh / C, mp = hm % M, h = hm / M, g = h / (a.heads / a.kv_heads);
-    const int kdim = a.kv_heads * M * a.dim;
-    VHead v;
-    v.h = h; v.qoff = hm * a.dim; v.koff = (g * M + mp) * a.dim; v.voff = kdim + (C > 1 ? cv : g) * a.vdim;
-    v.row_kv = kdim + a.kv_heads * a.vdim; v.qstride = a.heads * M * a.dim; v.nv = a.heads * M * C;
-    return v;
-}
-
-// scale, cap and distance penalty of a raw dot product; dist = row position - key position
-__device__ __forceinline__ float shaped_score(const CachedAttnArgs& a, float dot, float r1h, float r2h, int dist) {
-    float sv = dot * a.scale;
-    if (a.softcap > 0.f) sv = a.softcap * tanhf(sv / a.softcap);
-    if (a.r1 != nullptr) sv -= r1h * log1pf(r2h * (float)dist);
-    return sv;
-}
-
-__device__ __forceinline__ float sigmoidf_(float z) { return 1.f / (1.f + expf(-z)); }
-
-// blocks of `pool` tokens that lie wholly before the window of the row at position p
-__device__ __forceinline__ int pooled_visible(int p, int window, int pool) {
-    const int lim = p - window + 1;                   // tokens [0, lim) have left the window
-    return (pool > 0 && lim >= pool) ? lim / pool : 0;
-}
 
 template <typename T, int VC, int MODE>
 __global__ void __launch_bounds__(256) cached_attention_kernel(CachedAttnArgs a, Batch b) {
@@ -584,7 +543,8 @@ extern "C" int umbs_cached_attention_ex(int dtype, int mode, const void* q, cons
         count_launches(n_split > 1 ? 2 : 1);
         return (int)cudaGetLastError();
     }
-    if (dtype == UMBS_BF16) rc = launch_any<__nv_bfloat16>(mode, a, *batch, st);
+    if (dtype == UMBS_BF16 && attention_tc_fits(a, nullptr)) rc = launch_attention_tc(mode, a, nullptr, *batch, st);
+    else if (dtype == UMBS_BF16) rc = launch_any<__nv_bfloat16>(mode, a, *batch, st);
     else if (dtype == UMBS_F32) rc = launch_any<float>(mode, a, *batch, st);
     else return UMB_ERR_ARG;
     if (rc) return rc;

@@ -16,11 +16,10 @@
 // top 2, 4096 tokens of width 2048 with the routing around it: 808 -> 435 us; 64 tokens: 212 -> 152 us.
 #include <cuda.h>
 
-#include "../common.cuh"
 #include "seq_gemm.h"
+#include "seq_tc.cuh"
 
 namespace umbs {
-using umb::smem_u32;
 
 constexpr int kTcRows = 128, kTcK = 64, kTcLag = 3;         // tile rows; k per ring stage; stages in flight per copying thread
 constexpr int kTcStageRow = 36;                             // fp32 row stride of an epilogue warp's 32 x 32 staging block
@@ -31,44 +30,9 @@ struct TcArgs {
     int a_grouped, w_grouped;                               // the group coordinate of the tensor maps is used
 };
 
-__device__ unsigned int g_tc_timeouts;                      // launches that gave up on a wait (umbs_kernel_timeouts)
-
-// Every wait is bounded (about a second): a block that gives up raises the flag, and every role of it leaves its loop.
-__device__ __forceinline__ bool tc_give_up(volatile int* quit) {
-    if (!*quit) {
-        *quit = 1;
-        atomicAdd(&g_tc_timeouts, 1u);
-    }
-    return false;
-}
-__device__ __forceinline__ bool tc_spin(uint64_t* bar, uint32_t parity, volatile int* quit) {
-    for (int i = 0; i < (1 << 25); ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-        if (ok) return true;
-        if ((i & 1023) == 1023 && *quit) return false;
-    }
-    return tc_give_up(quit);
-}
-__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* quit) {
-    for (int i = 0; i < (1 << 20); ++i) {
-        if (umb::mbar_try_wait(bar, parity)) return true;   // (parks the thread for about a microsecond)
-        if (*quit) return false;
-    }
-    return tc_give_up(quit);
-}
-
 __device__ __forceinline__ void tma_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                  ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar)) : "memory");
-}
-
-__host__ __device__ constexpr uint32_t tc_idesc(uint32_t M, uint32_t N) {       // kind::f16, bf16 x bf16 -> fp32, both operands K-major
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
 // The tiles of a block, in the order every role visits them: rows fastest, then columns, then groups.
@@ -288,10 +252,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         while (done < issued) publish();
     }
     __syncthreads();
-    if (*quit) {                                            // gave up: let copies and products in flight end before the memory goes
-        for (int i = 0; i < 1000; ++i) __nanosleep(1000);
-        __syncthreads();
-    }
+    tc_settle(quit);
     if (warp == 1) {
         umb::tc_fence_after();
         umb::tmem_dealloc(tmem, 2 * BN);
@@ -374,7 +335,4 @@ int launch_gemm_tc(const GemmArgs& a, int groups, bool dual, bool c_f32, cudaStr
 
 }  // namespace umbs
 
-extern "C" unsigned int umbs_kernel_timeouts(void) {
-    unsigned int n = 0;
-    return cudaMemcpyFromSymbol(&n, umbs::g_tc_timeouts, sizeof n) == cudaSuccess ? n : ~0u;
-}
+extern "C" unsigned int umbs_kernel_timeouts(void) { return umbs::tc_timeouts() + umbs::attention_tc_timeouts(); }

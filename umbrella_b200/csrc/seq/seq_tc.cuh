@@ -1,0 +1,69 @@
+// Bounded mbarrier waits of the tensor-core kernels of the sequence-state decoders.
+#pragma once
+#include "../common.cuh"
+
+namespace umbs {
+using umb::smem_u32;
+
+static __device__ unsigned int g_tc_timeouts;               // blocks of this file's kernels that gave up on a wait
+
+// Every wait is bounded (about a second): a block that gives up raises its flag, and every role of it leaves its loop.
+__device__ __forceinline__ bool tc_give_up(volatile int* quit) {
+    if (!*quit) {
+        *quit = 1;
+        atomicAdd(&g_tc_timeouts, 1u);
+    }
+    return false;
+}
+__device__ __forceinline__ bool tc_test(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
+// polling: for one thread on a critical path (a parked thread comes back about a microsecond later)
+__device__ __forceinline__ bool tc_spin(uint64_t* bar, uint32_t parity, volatile int* quit) {
+    for (int i = 0; i < (1 << 25); ++i) {
+        if (tc_test(bar, parity)) return true;
+        if ((i & 1023) == 1023 && *quit) return false;
+    }
+    return tc_give_up(quit);
+}
+// polling with a short sleep in between: for warps that share a scheduler with working ones
+__device__ __forceinline__ bool tc_poll(uint64_t* bar, uint32_t parity, volatile int* quit) {
+    for (int i = 0; i < (1 << 24); ++i) {
+        if (tc_test(bar, parity)) return true;
+        __nanosleep(20);
+        if ((i & 255) == 255 && *quit) return false;
+    }
+    return tc_give_up(quit);
+}
+// parked: for waits that may be long
+__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* quit) {
+    for (int i = 0; i < (1 << 20); ++i) {
+        if (umb::mbar_try_wait(bar, parity)) return true;
+        if (*quit) return false;
+    }
+    return tc_give_up(quit);
+}
+// Behind the last barrier of a kernel that gave up: copies and products in flight end before their memory goes.
+__device__ __forceinline__ void tc_settle(volatile int* quit) {
+    if (!*quit) return;
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+    __syncthreads();
+}
+
+__host__ __device__ constexpr uint32_t tc_idesc(uint32_t M, uint32_t N, bool w_mn_major = false) {   // kind::f16, bf16 x bf16 -> fp32
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((w_mn_major ? 1u : 0u) << 16) | ((N >> 3) << 17) | ((M >> 4) << 24);
+}
+
+static inline unsigned int tc_timeouts() {
+    unsigned int n = 0;
+    return cudaMemcpyFromSymbol(&n, g_tc_timeouts, sizeof n) == cudaSuccess ? n : ~0u;
+}
+unsigned int attention_tc_timeouts();                       // seq_attn_tc.cu
+
+}  // namespace umbs

@@ -14,7 +14,7 @@
 #include <math.h>
 #include <stdint.h>
 
-#include "seq_internal.h"
+#include "seq_attn.h"
 
 namespace umbs {
 
@@ -225,7 +225,13 @@ extern "C" int umbs_window_attention_gated(int dtype, const void* q, int64_t ldq
     const WindowExtra x{k_shared, ldks, dim, mode == UMBS_ATTN_SOFTMAX_SINK, sink, gate, ldg, gate_per_head != 0};
     const int dq = dim + shared_dim;
     int rc;
-    if (dtype == UMBS_BF16) {
+    CachedAttnArgs a{};
+    a.heads = heads; a.kv_heads = heads; a.dim = dq; a.vdim = vdim; a.window = window; a.scale = scale;
+    a.gate = gate; a.ldg = ldg; a.gate_per_head = gate_per_head != 0; a.maps = a.vheads = 1; a.sink = sink;
+    const StepKeys keys{q, ldq, k, ldk, dim, k_shared, ldks, v, ldv, out, ldo};
+    if (dtype == UMBS_BF16 && attention_tc_fits(a, &keys)) {
+        rc = launch_attention_tc(mode, a, &keys, *batch, st);
+    } else if (dtype == UMBS_BF16) {
         rc = vdim <= 64 ? launch_window_attention<__nv_bfloat16, 4>(q, ldq, k, ldk, v, ldv, *batch, heads, dq, vdim, window, scale, out, ldo, x, st)
                         : launch_window_attention<__nv_bfloat16, 8>(q, ldq, k, ldk, v, ldv, *batch, heads, dq, vdim, window, scale, out, ldo, x, st);
     } else if (dtype == UMBS_F32) {
