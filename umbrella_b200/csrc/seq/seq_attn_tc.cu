@@ -3,12 +3,11 @@
 //
 // A block = 128 consecutive query rows of one (sequence, virtual head) = the 128 lanes of tensor memory; two blocks share an
 // SM, so that one multiplies while the other works its weights out.  Per tile of 64 keys:
-//   warps 5-6  copy key and value rows with 16-byte cp.async, each from where it lives (step, ring, block table), into the
-//              128-byte-swizzled images the tensor core reads; a key tile is fetched while the weights of the one before it
-//              are worked out, a value tile while the scores are;
-//   warp 4     one thread issues S = Q K^T and O += P V, accumulators in tensor memory;
-//   warps 0-3  a thread per row: scores to weights in fp32 in the base-2 domain, an online reference that only moves when a
-//              score passes it by 2^8 (then O is rescaled), the row's sum.
+//   warps 9-10 copy key and value rows with 16-byte cp.async, each from where it lives (step, ring, block table), into the
+//              128-byte-swizzled images the tensor core reads, a tile ahead where two fit;
+//   warp 8     one thread issues S = Q K^T and O += P V, accumulators in tensor memory;
+//   warps 0-7  two threads per row, 32 keys each: scores to weights in fp32 in the base-2 domain, an online reference that
+//              only moves when a score passes it by 2^8 (then the pair agrees on it and O is rescaled), the row's sum.
 // Weights stay 32-bit: an fp32 weight is the sum of three bf16 numbers (8 + 8 + 8 significant bits, cut off one after the
 // other, so exactly), and P V is three products against the same values.  Products of bf16 operands are exact in the tensor
 // core and its sums are fp32.
@@ -21,10 +20,10 @@
 namespace umbs {
 
 constexpr int kTaQ = 128, kTaK = 64;
-constexpr int kTaThreads = 224;                            // 4 warps of rows, 1 of products, 2 of copies
+constexpr int kTaThreads = 352;                             // 8 warps of weights, 1 of products, 2 of copies
 constexpr float kTaLazy = 8.f;                              // how far (in powers of two) a score may pass the reference
 
-struct TaDims { int q_atoms, k_steps, v_atoms; };           // 64-wide pieces of a query row, 16-wide k steps, 64-wide pieces of a value row
+struct TaDims { int q_atoms, k_steps, v_atoms, nk, nv; };   // 64-wide pieces of a query row, 16-wide k steps, 64-wide pieces of a value row; tiles held
 
 __device__ __forceinline__ float ex2(float x) {
     float y;
@@ -54,13 +53,19 @@ struct KeyTiles {
     __device__ int last(int i) const { return i < tiles_pool ? n_pool - 1 : p_hi; }
 };
 
+#define UMBS_TMEM_ST_X8(taddr, r)                                                                            \
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"                      \
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory")
+
 template <int MODE, bool SHAPED, bool STEP>
 __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const CachedAttnArgs a, const StepKeys x, const Batch b, const TaDims z) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ uint64_t bars[5];
+    __shared__ uint64_t bars[11];
     __shared__ uint32_t s_tmem;
     __shared__ int s_quit;
-    uint64_t *k_full = bars, *v_full = bars + 1, *s_full = bars + 2, *p_full = bars + 3, *o_full = bars + 4;
+    __shared__ float s_pair[2][kTaQ];
+    __shared__ int s_move[2][8];                            // per tile parity and warp: a row of it wants its reference moved
+    uint64_t *k_full = bars, *v_full = bars + 2, *k_empty = bars + 4, *v_empty = bars + 6, *s_full = bars + 8, *p_full = bars + 9, *o_full = bars + 10;
     volatile int* quit = &s_quit;
     const int s = blockIdx.z, vh = blockIdx.y, q0 = (int)(gridDim.x - 1 - blockIdx.x) * kTaQ;     // the rows that see most start first
     const int len = b.seq_len[s], start = b.seq_start[s], pos0 = STEP ? 0 : b.seq_pos0[s], slot = STEP ? 0 : b.seq_slot[s];
@@ -71,20 +76,25 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const Cache
     const int h = vhd.h, window = a.window > 0 ? a.window : (1 << 30);
     const KeyTiles kt(a, window, pos0, q0, len);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int k_bytes = z.q_atoms * (kTaK * 128), v_bytes = z.v_atoms * (kTaK * 128);
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    unsigned char* s_k = smem + z.q_atoms * (kTaQ * 128);   // Q [q_atoms][128 rows][128 B], K [q_atoms][64][128 B], V [v_atoms][64][128 B]
-    unsigned char* s_v = s_k + z.q_atoms * (kTaK * 128);
+    unsigned char* s_k = smem + z.q_atoms * (kTaQ * 128);   // Q [q_atoms][128 rows][128 B], nk K [q_atoms][64][128 B], nv V [v_atoms][64][128 B]
+    unsigned char* s_v = s_k + z.nk * k_bytes;
 
     if (threadIdx.x == 0) {
-        umb::mbar_init(k_full, 2);
-        umb::mbar_init(v_full, 2);
+        for (int i = 0; i < 2; ++i) {
+            umb::mbar_init(k_full + i, 2);
+            umb::mbar_init(v_full + i, 2);
+            umb::mbar_init(k_empty + i, 1);
+            umb::mbar_init(v_empty + i, 1);
+        }
         umb::mbar_init(s_full, 1);
-        umb::mbar_init(p_full, 4);
+        umb::mbar_init(p_full, 8);
         umb::mbar_init(o_full, 1);
         s_quit = 0;
         umb::fence_barrier_init();
     }
-    if (warp == 4) {
+    if (warp == 8) {
         umb::tmem_alloc(&s_tmem, 256);
         umb::tmem_relinquish();
     }
@@ -93,16 +103,16 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const Cache
     umb::tc_fence_after();
     const uint32_t tmem = s_tmem;
 
-    if (warp > 4) {
+    if (warp > 8) {
         // ------------------------------------------------------------------------------------ copies: 8 threads per 128-byte row piece
-        const int tid = threadIdx.x - 160, ch = tid & 7, r0 = tid >> 3;
+        const int tid = threadIdx.x - 288, ch = tid & 7, r0 = tid >> 3;
         const uint32_t sw = (uint32_t)((ch ^ (r0 & 7)) << 4);               // r0 + 8 p keeps r0's place inside its group of eight rows
         const __nv_bfloat16* q = (const __nv_bfloat16*)(STEP ? x.q : a.q);
         const int64_t ldq = STEP ? x.ldq : vhd.qstride;
         for (int at = 0; at < z.q_atoms; ++at) {
             const int d = at * 64 + ch * 8;
             if (d >= z.k_steps * 16) continue;
-#pragma unroll
+#pragma unroll 4
             for (int p = 0; p < 16; ++p) {
                 const int r = r0 + 8 * p;
                 const bool in = q0 + r < len && d < a.dim;
@@ -110,27 +120,26 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const Cache
             }
         }
         auto publish = [&](uint64_t* bar) {
-            asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-            umb::fence_proxy_async_smem();
+            umb::fence_proxy_async_smem();                  // this thread's copies are complete: show them to the tensor core
             __syncwarp();
             if (lane == 0) umb::mbar_arrive(bar);
         };
         for (int i = 0; i < kt.n; ++i) {
-            const int base = kt.base(i), last = kt.last(i);
-            const __nv_bfloat16 *kp[8], *sp[8], *vp[8];     // this thread's rows: own key part, shared part, values
-            bool in[8];
+            const int base = kt.base(i), last = kt.last(i), ks = i % z.nk, vs = i % z.nv;
+            const __nv_bfloat16 *kp[8], *vp[8];             // this thread's rows: keys, values
+            uint32_t in = 0;
 #pragma unroll
             for (int p = 0; p < 8; ++p) {
                 const int j = base + r0 + 8 * p;
-                in[p] = j <= last;
+                const bool ok = j <= last;
+                in |= (uint32_t)ok << p;
                 if (STEP) {
-                    const int64_t t = start + (in[p] ? j : base);
+                    const int64_t t = start + (ok ? j : base);
                     kp[p] = (const __nv_bfloat16*)x.k + t * x.ldk + (int64_t)vh * x.kdim;
-                    sp[p] = (const __nv_bfloat16*)x.ks + t * x.ldks - x.kdim;
                     vp[p] = (const __nv_bfloat16*)x.v + t * x.ldv + (int64_t)vh * a.vdim;
                 } else {
                     const __nv_bfloat16* row = (const __nv_bfloat16*)a.kv;
-                    if (in[p])
+                    if (ok)
                         row = kt.pooled(i) ? (const __nv_bfloat16*)a.pool_cache + ((int64_t)slot * a.pool_len + j) * vhd.row_kv
                             : j >= pos0 ? (const __nv_bfloat16*)a.kv + (int64_t)(start + j - pos0) * vhd.row_kv
                                         : (const __nv_bfloat16*)a.kv_cache + ((int64_t)slot * a.kv_len + j % a.kv_len) * vhd.row_kv;
@@ -138,45 +147,55 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const Cache
                     vp[p] = row + vhd.voff;
                 }
             }
-            if (i > 0 && !tc_poll(s_full, (i - 1) & 1, quit)) break;        // the scores before have been taken: the key tile is free
+            if (i >= z.nk && !tc_poll(k_empty + ks, (i / z.nk - 1) & 1, quit)) break;
+            const uint32_t kd = smem_u32(s_k) + ks * k_bytes + r0 * 128 + sw, vd = smem_u32(s_v) + vs * v_bytes + r0 * 128 + sw;
             for (int at = 0; at < z.q_atoms; ++at) {
                 const int d = at * 64 + ch * 8;
                 if (d >= z.k_steps * 16) continue;
+                const bool own = !STEP || d < x.kdim, dok = d < a.dim;      // (a part all heads share follows a head's own)
 #pragma unroll
                 for (int p = 0; p < 8; ++p) {
-                    const bool ok = in[p] && d < a.dim;
-                    cp16(smem_u32(s_k) + at * (kTaK * 128) + (r0 + 8 * p) * 128 + sw,
-                         ok ? (STEP && d >= x.kdim ? sp[p] : kp[p]) + d : kp[p], ok ? 16 : 0);
+                    const __nv_bfloat16* src = kp[p] + d;
+                    if (STEP && !own) src = (const __nv_bfloat16*)x.ks + (int64_t)(start + ((in >> p & 1) ? base + r0 + 8 * p : base)) * x.ldks + (d - x.kdim);
+                    const bool ok = (in >> p & 1) && dok;
+                    cp16(kd + at * (kTaK * 128) + p * 1024, ok ? src : kp[p], ok ? 16 : 0);
                 }
             }
-            publish(k_full);
-            if (i > 0 && !tc_poll(o_full, (i - 1) & 1, quit)) break;        // the value tile is free
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (i >= z.nv && !tc_poll(v_empty + vs, (i / z.nv - 1) & 1, quit)) break;
             for (int at = 0; at < z.v_atoms; ++at) {
                 const int c = at * 64 + ch * 8;
 #pragma unroll
                 for (int p = 0; p < 8; ++p) {
-                    const bool ok = in[p] && c < a.vdim;                    // rows that no query sees: zeros, their weights are 0
-                    cp16(smem_u32(s_v) + at * (kTaK * 128) + (r0 + 8 * p) * 128 + sw, ok ? vp[p] + c : vp[p], ok ? 16 : 0);
+                    const bool ok = (in >> p & 1) && c < a.vdim;            // rows that no query sees: zeros, their weights are 0
+                    cp16(vd + at * (kTaK * 128) + p * 1024, ok ? vp[p] + c : vp[p], ok ? 16 : 0);
                 }
             }
-            publish(v_full);
+            asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 1;" ::: "memory");
+            publish(k_full + ks);
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            publish(v_full + vs);
         }
-    } else if (warp == 4) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else if (warp == 8) {
         // ------------------------------------------------------------------------------------ products
         if (lane == 0) {
             const uint32_t idesc_s = tc_idesc(kTaQ, kTaK), idesc_o = tc_idesc(kTaQ, 64, true) + ((z.v_atoms - 1) * (64u >> 3) << 17);
-            const uint64_t qd = umb::umma_smem_desc_sw128(smem_u32(smem)), kd = umb::umma_smem_desc_sw128(smem_u32(s_k));
+            const uint64_t qd = umb::umma_smem_desc_sw128(smem_u32(smem)), kd0 = umb::umma_smem_desc_sw128(smem_u32(s_k));
             // values: keys down the rows, so the operand is MN-major; its 64-wide pieces are 8192 bytes apart, groups of eight keys 1024
-            const uint64_t vd = (umb::umma_smem_desc_sw128(smem_u32(s_v)) & ~((uint64_t)0x3fff << 16)) | ((uint64_t)(8192 >> 4) << 16);
+            const uint64_t vd0 = (umb::umma_smem_desc_sw128(smem_u32(s_v)) & ~((uint64_t)0x3fff << 16)) | ((uint64_t)(8192 >> 4) << 16);
             for (int i = 0; i < kt.n; ++i) {
-                if (!tc_spin(k_full, i & 1, quit)) break;
+                const int ks = i % z.nk, vs = i % z.nv;
+                if (!tc_spin(k_full + ks, (i / z.nk) & 1, quit)) break;
                 if (i > 0 && !tc_spin(o_full, (i - 1) & 1, quit)) break;    // the weights lie over the scores
                 umb::tc_fence_after();
+                const uint64_t kd = kd0 + ((ks * k_bytes) >> 4), vd = vd0 + ((vs * v_bytes) >> 4);
                 for (int k = 0; k < z.k_steps; ++k)
                     umb::umma_ss_f16(tmem, qd + (k >> 2) * (kTaQ * 128 >> 4) + (k & 3) * 2, kd + (k >> 2) * (kTaK * 128 >> 4) + (k & 3) * 2,
                                      idesc_s, k ? 1u : 0u);
                 umb::umma_commit(s_full);
-                if (!tc_spin(v_full, i & 1, quit)) break;
+                umb::umma_commit(k_empty + ks);
+                if (!tc_spin(v_full + vs, (i / z.nv) & 1, quit)) break;
                 if (!tc_spin(p_full, i & 1, quit)) break;
                 umb::tc_fence_after();
                 const uint32_t part[3] = {tmem + 64, tmem + 96, tmem + 32};
@@ -186,96 +205,108 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const Cache
                     for (int k = 0; k < kTaK / 16; ++k)
                         umb::umma_ts_f16(tmem + 128, part[e] + k * 8, vd + k * (2048 >> 4), idesc_o, (i | e | k) ? 1u : 0u);
                 umb::umma_commit(o_full);
+                umb::umma_commit(v_empty + vs);
             }
         }
     } else {
-        // ------------------------------------------------------------------------------------ weights: a thread per row
-        const int r = q0 + warp * 32 + lane, rp = pos0 + r;                 // the row's place in the step and its position
-        const uint32_t t0 = tmem + ((uint32_t)(warp * 32) << 16);
+        // ------------------------------------------------------------------------------------ weights: two threads per row
+        // (The two warps of a row meet at named barrier 1 + quarter, once per tile and once more when a reference moves.  Both
+        // walk every tile, also when a wait has given up, so they always meet.)
+        const int half = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane, pair_id = 1 + quarter;
+        const int r = q0 + row, rp = pos0 + r;                              // the row's place in the step and its position
+        const uint32_t t0 = tmem + ((uint32_t)(quarter * 32) << 16);
         constexpr float kLog2e = 1.4426950408889634f;
         const float c = SHAPED ? kLog2e : a.scale * kLog2e;
-        const float sk = MODE == UMBS_ATTN_SOFTMAX_SINK ? sink_score(a, h) * kLog2e : -INFINITY;
         const float hb = (MODE == UMBS_ATTN_SIGMOID && a.head_bias) ? a.head_bias[h] : 0.f;
         const float r1h = SHAPED && a.r1 ? a.r1[h] : 0.f, r2h = SHAPED && a.r1 ? a.r2[h] : 0.f;
-        float m = sk, l = MODE == UMBS_ATTN_SOFTMAX_SINK ? 1.f : 0.f;       // the sink: a key of this score without a value
+        float m = MODE == UMBS_ATTN_SOFTMAX_SINK ? sink_score(a, h) * kLog2e : -INFINITY;      // the sink: a key of this score ...
+        float l = MODE == UMBS_ATTN_SOFTMAX_SINK && half == 0 ? 1.f : 0.f;                     // ... without a value
         const int tok_lo = max(rp - window + 1, a.chunk > 0 ? rp / a.chunk * a.chunk : 0);
         const int pool_hi = pooled_visible(rp, window, a.pool);
         bool ok = true;
         for (int i = 0; i < kt.n; ++i) {
-            const int base = kt.base(i);
-            // keys [lo, hi) of the tile are visible to this row
+            const int base = kt.base(i) + half * 32;        // this thread's keys: base .. base + 31, of which [lo, hi) are visible to its row
             const int lo = kt.pooled(i) ? 0 : max(tok_lo - base, 0);
-            const int hi = r >= len ? 0 : min(kt.pooled(i) ? pool_hi - base : rp + 1 - base, kTaK);
-            const bool whole = __all_sync(0xffffffffu, lo == 0 && hi == kTaK);
-            if (!(ok = tc_poll(s_full, i & 1, quit))) break;
+            const int hi = r >= len ? 0 : min((kt.pooled(i) ? pool_hi : rp + 1) - base, 32);
+            const bool whole = __all_sync(0xffffffffu, lo == 0 && hi == 32);
+            ok = __all_sync(0xffffffffu, ok && tc_poll(s_full, i & 1, quit));
             umb::tc_fence_after();
             uint32_t v[32];
-            auto score = [&](int half, int jj) -> float {
-                const float sv = __uint_as_float(v[jj]);
-                return SHAPED ? shaped_score(a, sv, r1h, r2h, rp - (base + half * 32 + jj)) : sv;
-            };
-            auto seen = [&](int k) { return whole || (k >= lo && k < hi); };
+            UMB_TMEM_LD_X32(t0 + half * 32, v);
+            umb::tc_wait_ld();
+            if (SHAPED) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(shaped_score(a, __uint_as_float(v[j]), r1h, r2h, rp - (base + j)));
+            }
+            float mx = -INFINITY;
             if (MODE != UMBS_ATTN_SIGMOID) {
-                float mx = -INFINITY;
+                if (!whole) {
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    UMB_TMEM_LD_X32(t0 + half * 32, v);
-                    umb::tc_wait_ld();
-                    float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-                    for (int jj = 0; jj < 32; ++jj) m4[jj & 3] = fmaxf(m4[jj & 3], seen(half * 32 + jj) ? score(half, jj) * c : -INFINITY);
-                    mx = fmaxf(mx, fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])));
+                    for (int j = 0; j < 32; ++j)
+                        if (j < lo || j >= hi) v[j] = 0x7fffffffu;          // (a maximum passes a NaN by)
                 }
-                const bool move = mx > m + (i == 0 ? 0.f : kTaLazy) || (m == -INFINITY && mx > -INFINITY);
-                if (i == 0) {
-                    if (move) {
-                        l *= ex2(m - mx);                                   // (m = -inf: l is 0)
-                        m = mx;
-                    }
-                } else if (__any_sync(0xffffffffu, move)) {                 // rare: the reference of some row moves
-                    const float f = move ? ex2(m - mx) : 1.f;
-                    if (move) m = mx;
-                    l *= f;
-                    for (int c0 = 0; c0 < z.v_atoms * 64; c0 += 32) {
-                        UMB_TMEM_LD_X32(t0 + 128 + c0, v);
-                        umb::tc_wait_ld();
+                float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-                        for (int jj = 0; jj < 32; ++jj) v[jj] = __float_as_uint(__uint_as_float(v[jj]) * f);
-                        UMB_TMEM_ST_X32(t0 + 128 + c0, v);
+                for (int j = 0; j < 32; ++j) m4[j & 3] = fmaxf(m4[j & 3], __uint_as_float(v[j]) * c);
+                mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+                const bool want = __any_sync(0xffffffffu, i == 0 || mx > m + kTaLazy || (m == -INFINITY && mx > -INFINITY));
+                s_pair[half][row] = mx;
+                if (lane == 0) s_move[i & 1][warp] = want;
+            }
+            // behind this both warps have read their scores (the weights' last part goes over them)
+            __syncwarp();
+            umb::named_bar_sync(pair_id, 64);
+            if (MODE != UMBS_ATTN_SIGMOID) {
+                const float other = s_pair[half ^ 1][row];
+                const bool move = (s_move[i & 1][warp] | s_move[i & 1][warp ^ 4]) != 0;
+                __syncwarp();
+                umb::named_bar_sync(pair_id, 64);           // (s_pair may be written again)
+                if (move) {
+                    mx = fmaxf(mx, other);
+                    const float f = mx > m ? ex2(m - mx) : 1.f;
+                    l *= f;                                 // (m = -inf: l is 0)
+                    if (i > 0) {
+                        for (int c0 = half * 32; c0 < z.v_atoms * 64; c0 += 64) {
+                            for (int e = 0; e < 32; e += 16) {
+                                uint32_t o[16];
+                                UMB_TMEM_LD_X16(t0 + 128 + c0 + e, o);
+                                umb::tc_wait_ld();
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
+                                UMB_TMEM_ST_X16(t0 + 128 + c0 + e, o);
+                            }
+                        }
                     }
-                    UMB_TMEM_LD_X32(t0 + 32, v);                            // the scores again
-                    umb::tc_wait_ld();
+                    m = fmaxf(m, mx);
                 }
             }
             const float ref = m == -INFINITY ? 0.f : m;
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+                v[j] = __float_as_uint(MODE == UMBS_ATTN_SIGMOID ? sigmoidf_(__uint_as_float(v[j]) * a.scale + hb)
+                                                                 : ex2(fmaf(__uint_as_float(v[j]), c, -ref)));
+            if (!whole) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                    if (j < lo || j >= hi) v[j] = 0u;
+            }
             float l4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int half = 1; half >= 0; --half) {                         // (the second half is at hand)
-                if (half == 0 || MODE == UMBS_ATTN_SIGMOID) {
-                    UMB_TMEM_LD_X32(t0 + half * 32, v);
-                    umb::tc_wait_ld();
-                }
-                uint32_t hi_[16], mid_[16], lo_[16];
+            for (int e = 0; e < 2; ++e) {
+                uint32_t ph[8], pm[8], pl[8];
 #pragma unroll
-                for (int jj = 0; jj < 32; jj += 2) {
-                    float p[2];
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        if (MODE == UMBS_ATTN_SIGMOID) {
-                            p[e] = seen(half * 32 + jj + e) ? sigmoidf_(__uint_as_float(v[jj + e]) * a.scale + hb) : 0.f;
-                        } else {
-                            p[e] = seen(half * 32 + jj + e) ? ex2(fmaf(score(half, jj + e), c, -ref)) : 0.f;
-                            l4[(jj + e) & 3] += p[e];
-                        }
-                    }
-                    const float ra = p[0] - cut(p[0]), rb = p[1] - cut(p[1]);
-                    hi_[jj >> 1] = hi_pair(p[0], p[1]);
-                    mid_[jj >> 1] = hi_pair(ra, rb);
-                    lo_[jj >> 1] = hi_pair(ra - cut(ra), rb - cut(rb));
+                for (int j = 0; j < 8; ++j) {
+                    const float p = __uint_as_float(v[e * 16 + 2 * j]), p1 = __uint_as_float(v[e * 16 + 2 * j + 1]);
+                    l4[(2 * j) & 3] += p;
+                    l4[(2 * j + 1) & 3] += p1;
+                    const float ra = p - cut(p), rb = p1 - cut(p1);
+                    ph[j] = hi_pair(p, p1);
+                    pm[j] = hi_pair(ra, rb);
+                    pl[j] = hi_pair(ra - cut(ra), rb - cut(rb));
                 }
-                UMB_TMEM_ST_X16(t0 + 64 + half * 16, hi_);
-                UMB_TMEM_ST_X16(t0 + 96 + half * 16, mid_);
-                UMB_TMEM_ST_X16(t0 + 32 + half * 16, lo_);
+                UMBS_TMEM_ST_X8(t0 + 64 + half * 16 + e * 8, ph);
+                UMBS_TMEM_ST_X8(t0 + 96 + half * 16 + e * 8, pm);
+                UMBS_TMEM_ST_X8(t0 + 32 + half * 16 + e * 8, pl);
             }
             l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
             umb::tc_wait_st();
@@ -283,63 +314,78 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const Cache
             __syncwarp();
             if (lane == 0) umb::mbar_arrive(p_full);
         }
-        if (ok && tc_poll(o_full, (kt.n - 1) & 1, quit)) {
-            umb::tc_fence_after();
+        ok = __all_sync(0xffffffffu, ok && tc_poll(o_full, (kt.n - 1) & 1, quit));
+        umb::tc_fence_after();
+        s_pair[half][row] = l;
+        umb::named_bar_sync(pair_id, 64);
+        l += s_pair[half ^ 1][row];
+        if (ok) {
             const float inv = MODE == UMBS_ATTN_SIGMOID ? 1.f : 1.f / l;
             const int64_t t = start + r;
             const float* grow = a.gate ? a.gate + t * a.ldg + (a.gate_per_head ? h : h * a.vdim) : nullptr;
             const float gh = (grow && a.gate_per_head && r < len) ? sigmoidf_(grow[0]) : 1.f;
-            const bool gvec = grow && !a.gate_per_head && ((uintptr_t)a.gate & 15) == 0 && a.ldg % 4 == 0;
+            const bool gvec = grow && !a.gate_per_head && ((uintptr_t)grow & 15) == 0;
             float* rrow = a.raw ? a.raw + (t * vhd.nv + vh) * a.vdim : nullptr;
             __nv_bfloat16* orow = STEP ? (__nv_bfloat16*)x.out + t * x.ldo + (int64_t)h * a.vdim
                                        : (__nv_bfloat16*)a.out + t * a.heads * a.vdim + (int64_t)h * a.vdim;
-            for (int c0 = 0; c0 < a.vdim; c0 += 32) {
+            for (int c0 = half * 32; c0 < a.vdim; c0 += 64) {
                 uint32_t v[32];
                 UMB_TMEM_LD_X32(t0 + 128 + c0, v);
                 umb::tc_wait_ld();
-                if (r >= len) continue;
+                if (r < len) {
 #pragma unroll
-                for (int e = 0; e < 32; e += 8) {
-                    if (c0 + e >= a.vdim) break;                            // (vdim is a multiple of 8)
-                    float o[8];
+                    for (int e = 0; e < 32; e += 8) {
+                        if (c0 + e < a.vdim) {                              // (vdim is a multiple of 8)
+                            float o[8];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) o[u] = __uint_as_float(v[e + u]) * inv;
-                    if (rrow) {
-                        *reinterpret_cast<float4*>(rrow + c0 + e) = make_float4(o[0], o[1], o[2], o[3]);
-                        *reinterpret_cast<float4*>(rrow + c0 + e + 4) = make_float4(o[4], o[5], o[6], o[7]);
-                        continue;
-                    }
-                    if (grow) {
-                        float g[8];
-                        if (gvec) {
-                            *reinterpret_cast<float4*>(g) = *reinterpret_cast<const float4*>(grow + c0 + e);
-                            *reinterpret_cast<float4*>(g + 4) = *reinterpret_cast<const float4*>(grow + c0 + e + 4);
+                            for (int u = 0; u < 8; ++u) o[u] = __uint_as_float(v[e + u]) * inv;
+                            if (rrow) {
+                                *reinterpret_cast<float4*>(rrow + c0 + e) = make_float4(o[0], o[1], o[2], o[3]);
+                                *reinterpret_cast<float4*>(rrow + c0 + e + 4) = make_float4(o[4], o[5], o[6], o[7]);
+                                continue;
+                            }
+                            if (grow) {
+                                float g[8];
+                                if (gvec) {
+                                    *reinterpret_cast<float4*>(g) = *reinterpret_cast<const float4*>(grow + c0 + e);
+                                    *reinterpret_cast<float4*>(g + 4) = *reinterpret_cast<const float4*>(grow + c0 + e + 4);
+                                }
+#pragma unroll
+                                for (int u = 0; u < 8; ++u)
+                                    o[u] *= a.gate_per_head ? gh : sigmoidf_(gvec ? g[u] : grow[c0 + e + u]);
+                            }
+                            uint32_t w[4];
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                const __nv_bfloat162 pr = __floats2bfloat162_rn(o[2 * u], o[2 * u + 1]);
+                                w[u] = *reinterpret_cast<const uint32_t*>(&pr);
+                            }
+                            *reinterpret_cast<uint4*>(orow + c0 + e) = make_uint4(w[0], w[1], w[2], w[3]);
                         }
-#pragma unroll
-                        for (int u = 0; u < 8; ++u)
-                            o[u] *= a.gate_per_head ? gh : sigmoidf_(gvec ? g[u] : grow[c0 + e + u]);
                     }
-                    uint32_t w[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const __nv_bfloat162 pr = __floats2bfloat162_rn(o[2 * u], o[2 * u + 1]);
-                        w[u] = *reinterpret_cast<const uint32_t*>(&pr);
-                    }
-                    *reinterpret_cast<uint4*>(orow + c0 + e) = make_uint4(w[0], w[1], w[2], w[3]);
                 }
+                __syncwarp();
             }
         }
     }
+    __syncwarp();
     umb::tc_fence_before();
     __syncthreads();
     tc_settle(quit);
-    if (warp == 4) {
+    if (warp == 8) {
         umb::tc_fence_after();
         umb::tmem_dealloc(tmem, 256);
     }
 }
 
-static TaDims ta_dims(const CachedAttnArgs& a) { return TaDims{(a.dim + 63) / 64, (a.dim + 15) / 16, (a.vdim + 63) / 64}; }
+// Two key tiles and two value tiles where two blocks of that size fit on an SM (228 KB, 1 KB of it per block the system's).
+static TaDims ta_dims(const CachedAttnArgs& a) {
+    TaDims z{(a.dim + 63) / 64, (a.dim + 15) / 16, (a.vdim + 63) / 64, 2, 2};
+    const int room = 110 * 1024 - z.q_atoms * (kTaQ * 128), k = z.q_atoms * (kTaK * 128), v = z.v_atoms * (kTaK * 128);
+    if (2 * k + 2 * v > room) z.nk = 1;
+    if (k * z.nk + 2 * v > room) z.nv = 1;
+    return z;
+}
 
 // Every row piece is copied in 16-byte pieces and a block's tiles and tensor memory leave room for a second one on the SM:
 // sizes in eights, queries and keys of up to 192, values of up to 128 numbers.
@@ -355,7 +401,7 @@ bool attention_tc_fits(const CachedAttnArgs& a, const StepKeys* s) {
 template <int MODE, bool SHAPED, bool STEP>
 static int launch_ta(const CachedAttnArgs& a, const StepKeys& x, const Batch& b, cudaStream_t st) {
     const TaDims z = ta_dims(a);
-    const int smem = 1024 + z.q_atoms * (kTaQ + kTaK) * 128 + z.v_atoms * kTaK * 128;
+    const int smem = 1024 + (z.q_atoms * (kTaQ + z.nk * kTaK) + z.nv * z.v_atoms * kTaK) * 128;
     auto kernel = attention_tc_kernel<MODE, SHAPED, STEP>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;

@@ -152,7 +152,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int rr = lane >> 3, cc = (lane & 7) * 4;
         for (uint32_t it = 0; w.step(); ++it) {
             const uint32_t acc = it & 1;
-            if (!tc_wait(acc_full + acc, (it >> 1) & 1, quit)) break;
+            if (!__all_sync(0xffffffffu, tc_wait(acc_full + acc, (it >> 1) & 1, quit))) break;      // (and the warp is one again)
             umb::tc_fence_after();
             const uint32_t src = tmem + acc * BN + ((uint32_t)(q * 32) << 16);
             const int rows = w.rows - w.m0 - q * 32, n_hi = a.N - w.n0 * kOut;      // rows of this quarter, columns of the tile
@@ -231,7 +231,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 row[i] = r < w.rows ? (int64_t)(a.row_src ? a.row_src[p] : p) * a.lda + (t.a_grouped ? (int64_t)w.g * a.a_goff : 0) : -1;
             }
             for (int k = 0; k < t.k_steps; ++k) {
-                if (!(ok = tc_wait(empty + s, ph, quit))) break;
+                if (!(ok = __all_sync(0xffffffffu, tc_wait(empty + s, ph, quit)))) break;
                 const uint32_t dst = smem_u32(smem + s * Cfg::kStage) + dst0;
                 const int kc = k * kTcK + ch * 8;
                 const int bytes = kc < a.K ? 16 : 0;        // behind the last column: zeros (K is a multiple of 8)
