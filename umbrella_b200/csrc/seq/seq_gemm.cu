@@ -86,40 +86,38 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(GemmArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------------ few rows (decode)
-// Up to 16 activation rows per group: the product is a stream over the weights.  A warp owns four weight rows (with
-// DUAL: the gate and up rows of two outputs) and walks k with one 16-byte load per lane and row, every row's load in
-// flight at once; the few activation rows come through L1.  Lanes keep fp32 partial sums per (weight row, activation
-// row) and a shuffle tree adds them at the end.  A group without rows returns before touching its weights, so a decode
-// step reads only the experts that were chosen.
+// Up to 16 activation rows per group: the product is a stream over the weights, and with few rows what it waits for is the
+// latency of a row's loads, one after the other.  So a weight row is split over KW warps (k in pieces of 256, warp after
+// warp), a thread takes four weight rows (with DUAL: the gate and up rows of two outputs) and has the 16-byte loads of two
+// of its pieces in flight; a block of four warps covers 4 / KW such sets of rows.  Sums are kept as even and odd halves (one
+// instruction for both), added over the lanes by a tree that hands every lane fewer values at each level, then over the
+// warps in order: the order depends on K alone, so a row's result does not depend on the other rows.  A group without rows
+// returns before touching its weights, so a decode step reads only the experts that were chosen.
 constexpr int SK_ROWS = 4, SK_WARPS = 4;
 
-__device__ __forceinline__ void bf16x8_to_f32(const uint4& v, float (&f)[8]) {
+__device__ __forceinline__ void bf16x8_to_f32x2(const uint4& v, f32x2 (&f)[4]) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        f[2 * i] = __uint_as_float(w[i] << 16);
-        f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-    }
+    for (int i = 0; i < 4; ++i) f[i] = pack2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
 }
 
-template <typename TC, bool DUAL, int MT>
+template <typename TC, bool DUAL, int MT, int KW>
 __global__ void __launch_bounds__(32 * SK_WARPS) gemm_skinny_kernel(GemmArgs a) {
+    constexpr int OUTS = DUAL ? SK_ROWS / 2 : SK_ROWS, SETS = SK_WARPS / KW, V = SK_ROWS * MT;      // outputs per set; sums per thread
+    __shared__ float part[SK_WARPS][V];
     const int g = blockIdx.z;
     int row_lo = 0, rows = a.M;
     if (a.grp_off != nullptr) { row_lo = a.grp_off[g]; rows = a.grp_off[g + 1] - row_lo; }
     const int m0 = blockIdx.y * MT;
     if (m0 >= rows) return;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int OUTS = DUAL ? SK_ROWS / 2 : SK_ROWS;           // outputs per warp
-    const int n0 = (blockIdx.x * SK_WARPS + warp) * OUTS;
-    if (n0 >= a.N) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, set = warp / KW, kw = warp % KW;
+    const int n0 = (blockIdx.x * SETS + set) * OUTS;
     const __nv_bfloat16* A = (const __nv_bfloat16*)a.A + (int64_t)g * a.a_goff;
     const __nv_bfloat16* W = (const __nv_bfloat16*)a.W + (int64_t)g * a.w_gstride;
     const __nv_bfloat16* wrow[SK_ROWS];
 #pragma unroll
     for (int i = 0; i < SK_ROWS; ++i) {
-        int n = DUAL ? (n0 + (i >> 1)) : (n0 + i);
-        n = min(n, a.N - 1);                                      // a tail warp recomputes the last row; it is not stored
+        const int n = min(DUAL ? (n0 + (i >> 1)) : (n0 + i), a.N - 1);      // behind the last row: the last row again, not stored
         wrow[i] = W + (int64_t)(DUAL ? ((i & 1) * a.N + n) : n) * a.ldw;
     }
     const __nv_bfloat16* arow[MT];
@@ -128,60 +126,100 @@ __global__ void __launch_bounds__(32 * SK_WARPS) gemm_skinny_kernel(GemmArgs a) 
         const int p = row_lo + min(m0 + m, rows - 1);
         arow[m] = A + (int64_t)(a.row_src ? a.row_src[p] : p) * a.lda;
     }
-    float acc[SK_ROWS][MT] = {};
-    for (int k = lane * 8; k < a.K; k += 256) {
-        uint4 wv[SK_ROWS];
-#pragma unroll
-        for (int i = 0; i < SK_ROWS; ++i) wv[i] = __ldg(reinterpret_cast<const uint4*>(wrow[i] + k));
-        float wf[SK_ROWS][8];
-#pragma unroll
-        for (int i = 0; i < SK_ROWS; ++i) bf16x8_to_f32(wv[i], wf[i]);
-#pragma unroll
-        for (int m = 0; m < MT; ++m) {
-            float af[8];
-            bf16x8_to_f32(*reinterpret_cast<const uint4*>(arow[m] + k), af);
-#pragma unroll
-            for (int i = 0; i < SK_ROWS; ++i)
-#pragma unroll
-                for (int e = 0; e < 8; ++e) acc[i][m] = fmaf(af[e], wf[i][e], acc[i][m]);
-        }
-    }
+    f32x2 acc[SK_ROWS][MT];
 #pragma unroll
     for (int i = 0; i < SK_ROWS; ++i)
 #pragma unroll
-        for (int m = 0; m < MT; ++m)
+        for (int m = 0; m < MT; ++m) acc[i][m] = 0ull;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    for (int k = (kw * 32 + lane) * 8; k < a.K; k += 2 * KW * 256) {
+        const int k2 = k + KW * 256;
+        uint4 wv[2][SK_ROWS];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc[i][m] += __shfl_xor_sync(0xffffffffu, acc[i][m], o);
-    TC* C = (TC*)a.C + (int64_t)g * a.c_goff;
-    if (lane == 0) {
+        for (int i = 0; i < SK_ROWS; ++i) wv[0][i] = __ldg(reinterpret_cast<const uint4*>(wrow[i] + k));
 #pragma unroll
-        for (int o = 0; o < OUTS; ++o) {
-            if (n0 + o >= a.N) continue;
+        for (int i = 0; i < SK_ROWS; ++i) wv[1][i] = k2 < a.K ? __ldg(reinterpret_cast<const uint4*>(wrow[i] + k2)) : zero;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            f32x2 wf[SK_ROWS][4];
+#pragma unroll
+            for (int i = 0; i < SK_ROWS; ++i) bf16x8_to_f32x2(wv[u][i], wf[i]);
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
-                if (m0 + m >= rows) continue;
-                const float v = finish<DUAL>(a, DUAL ? acc[2 * o][m] : acc[o][m], acc[DUAL ? 2 * o + 1 : o][m], g, row_lo + m0 + m, n0 + o);
-                C[(int64_t)(row_lo + m0 + m) * a.ldc + n0 + o] = from_f32<TC>(v);
+                f32x2 af[4];
+                bf16x8_to_f32x2(u == 0 || k2 < a.K ? *reinterpret_cast<const uint4*>(arow[m] + (u ? k2 : k)) : zero, af);
+#pragma unroll
+                for (int i = 0; i < SK_ROWS; ++i)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[i][m] = fma2(af[e], wf[i][e], acc[i][m]);
             }
         }
     }
+    float v[V];
+#pragma unroll
+    for (int i = 0; i < SK_ROWS; ++i)
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            const float2 h = unpack2(acc[i][m]);
+            v[i * MT + m] = h.x + h.y;
+        }
+    // the lanes' sums: a lane keeps half of its values at each level while it has several
+#pragma unroll
+    for (int o = 16, c = V; o > 0; o >>= 1) {
+        if (c > 1) {
+            c >>= 1;
+#pragma unroll
+            for (int i = 0; i < V / 2; ++i) {
+                if (i >= c) continue;
+                const float send = (lane & o) ? v[i] : v[i + c], keep = (lane & o) ? v[i + c] : v[i];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+    constexpr int per = 32 / V;                                             // lanes that hold the same value
+    if (lane % per == 0) part[warp][lane / per] = v[0];
+    __syncthreads();
+    TC* C = (TC*)a.C + (int64_t)g * a.c_goff;
+    for (int i = threadIdx.x; i < SETS * OUTS * MT; i += 32 * SK_WARPS) {
+        const int st = i / (OUTS * MT), o = i % (OUTS * MT) / MT, m = i % MT, n = (blockIdx.x * SETS + st) * OUTS + o;
+        if (n >= a.N || m0 + m >= rows) continue;
+        float s = 0.f, s2 = 0.f;
+#pragma unroll
+        for (int q = 0; q < KW; ++q) {
+            s += part[st * KW + q][(DUAL ? 2 * o : o) * MT + m];
+            if (DUAL) s2 += part[st * KW + q][(2 * o + 1) * MT + m];
+        }
+        const int64_t row = row_lo + m0 + m;
+        C[row * a.ldc + n] = from_f32<TC>(finish<DUAL>(a, s, s2, g, row, n));
+    }
 }
 
+// K alone chooses how many warps share a row: with one the loop over k is the critical path from 512 on.
 template <typename TC>
 static void launch_skinny(const GemmArgs& a, int groups, bool dual, cudaStream_t st) {
-    const int outs_per_block = SK_WARPS * (dual ? SK_ROWS / 2 : SK_ROWS);
+    const int kw = a.K >= 1024 ? 4 : (a.K >= 512 ? 2 : 1);
+    const int outs_per_block = SK_WARPS / kw * (dual ? SK_ROWS / 2 : SK_ROWS);
     const int mt = a.M <= 1 ? 1 : (a.M <= 2 ? 2 : (a.M <= 4 ? 4 : 8));
     const dim3 grid((a.N + outs_per_block - 1) / outs_per_block, (a.M + mt - 1) / mt, groups), block(32 * SK_WARPS);
+#define UMBS_SK2(MT, KW)                                                              \
+    do {                                                                              \
+        if (dual) gemm_skinny_kernel<TC, true, MT, KW><<<grid, block, 0, st>>>(a);    \
+        else gemm_skinny_kernel<TC, false, MT, KW><<<grid, block, 0, st>>>(a);        \
+    } while (0)
 #define UMBS_SK(MT)                                                                   \
     do {                                                                              \
-        if (dual) gemm_skinny_kernel<TC, true, MT><<<grid, block, 0, st>>>(a);        \
-        else gemm_skinny_kernel<TC, false, MT><<<grid, block, 0, st>>>(a);            \
+        if (kw == 4) UMBS_SK2(MT, 4);                                                 \
+        else if (kw == 2) UMBS_SK2(MT, 2);                                            \
+        else UMBS_SK2(MT, 1);                                                         \
     } while (0)
     if (mt == 1) UMBS_SK(1);
     else if (mt == 2) UMBS_SK(2);
     else if (mt == 4) UMBS_SK(4);
     else UMBS_SK(8);
 #undef UMBS_SK
+#undef UMBS_SK2
 }
 
 template <typename TA, typename TC>
