@@ -21,7 +21,7 @@
 
 namespace umbs {
 
-constexpr int kTcRows = 128, kTcK = 64, kTcLag = 3;         // tile rows; k per ring stage; stages in flight per copying thread
+constexpr int kTcRows = 128, kTcK = 64;                     // tile rows; k per ring stage
 constexpr int kTcStageRow = 36;                             // fp32 row stride of an epilogue warp's 32 x 32 staging block
 
 struct TcArgs {
@@ -63,13 +63,56 @@ struct TileWalk {
 template <int BN, bool DUAL>
 struct TcCfg {
     static constexpr int kStages = BN == 256 ? 4 : (BN == 128 ? 6 : 8);
+    // Rows copied by threads: every stage of the ring has its own warps, which fill it, wait for their copies and publish it.
+    // (Warps that serve the stages in turn publish one only when they come back for another: 1.5 us per k step, a round trip
+    // between the tensor core and the copies.)
+    static constexpr int kWarpsPerStage = BN == 256 ? 2 : 1, kCopyWarps = kStages * kWarpsPerStage;
+    static constexpr int threads(bool a_tma) { return a_tma ? 192 : 192 + 32 * kCopyWarps; }
     static constexpr int kABytes = kTcRows * 128, kWBytes = BN * 128, kStage = kABytes + kWBytes;
     static constexpr int kOut = DUAL ? BN / 2 : BN;         // output columns of a tile
-    static constexpr int kSmem = 1024 + kStages * kStage + 4 * 32 * kTcStageRow * 4 + 256;
+    static constexpr int kSmem = 1024 + kStages * kStage + 4 * 32 * kTcStageRow * 4 + 256 + kCopyWarps * kTcRows * 4;
 };
 
+// Bias and activation of 32 neighbouring columns of a row, v (and u, the up half) in place.  One choice of activation in
+// front of a loop over independent elements: chosen element by element, every exponential and every quotient waited for the
+// one before it (25 to 40 us for a tile's 128 x 128 outputs, several times its products).  Quotients are within two units in
+// the last place here; the sums they scale carry the tensor core's error, an order of magnitude more.  ((1 + tanh(z)) / 2 is
+// the sigmoid of 2 z.)
+__device__ __forceinline__ float tc_sigmoid(float z) { return __fdividef(1.f, 1.f + expf(-z)); }
+template <bool DUAL>
+__device__ __forceinline__ void tc_finish(const GemmArgs& a, uint32_t (&v)[32], uint32_t (&u)[DUAL ? 32 : 1], int n0) {
+#define UMBS_F(x) __uint_as_float(x)
+#define UMBS_EACH(expr)                                                                     \
+    _Pragma("unroll") for (int j = 0; j < 32; ++j) {                                        \
+        const float x = UMBS_F(v[j]), y = DUAL ? UMBS_F(u[DUAL ? j : 0]) : 0.f;              \
+        v[j] = __float_as_uint(expr);                                                       \
+        (void)y;                                                                            \
+    }
+    if (a.bias != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const int n = min(n0 + j, a.N - 1);
+            v[j] = __float_as_uint(UMBS_F(v[j]) + a.bias[n]);
+            if (DUAL) u[DUAL ? j : 0] = __float_as_uint(UMBS_F(u[DUAL ? j : 0]) + a.bias[a.N + n]);
+        }
+    }
+    if (DUAL) {
+        if (a.act == UMBS_ACT_GELU_TANH) UMBS_EACH(x * tc_sigmoid(1.5957691216057308f * (x + 0.044715f * x * x * x)) * y)
+        else if (a.act == UMBS_ACT_SILU) UMBS_EACH(x * tc_sigmoid(x) * y)
+        else UMBS_EACH(fminf(x, a.limit) * tc_sigmoid(1.702f * fminf(x, a.limit)) * (fminf(fmaxf(y, -a.limit), a.limit) + 1.f))
+    } else if (a.unary && n0 + 32 <= a.unary_cols && (a.unary == UMBS_UNARY_SILU || a.unary == UMBS_UNARY_RELU2 || a.unary == UMBS_UNARY_SCALE)) {
+        if (a.unary == UMBS_UNARY_SILU) UMBS_EACH(x * tc_sigmoid(x))
+        else if (a.unary == UMBS_UNARY_RELU2) UMBS_EACH(fmaxf(x, 0.f) * fmaxf(x, 0.f))
+        else UMBS_EACH(a.p0 * x)
+    } else if (a.unary) {
+        UMBS_EACH(n0 + j < a.unary_cols ? unary_act(x, a.unary, a.p0, a.p1) : x)
+    }
+#undef UMBS_EACH
+#undef UMBS_F
+}
+
 template <int BN, bool DUAL, bool A_TMA, typename TC>
-__global__ void __launch_bounds__(A_TMA ? 192 : 320, 1)
+__global__ void __launch_bounds__(TcCfg<BN, DUAL>::threads(A_TMA), 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const GemmArgs a, const TcArgs t) {
     using Cfg = TcCfg<BN, DUAL>;
     constexpr int kStages = Cfg::kStages, kOut = Cfg::kOut;
@@ -86,7 +129,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         umb::tma_prefetch_desc(&map_w);
         if (A_TMA) umb::tma_prefetch_desc(&map_a);
         for (int i = 0; i < kStages; ++i) {
-            umb::mbar_init(full + i, A_TMA ? 1 : 5);        // the TMA thread, and the four copying warps
+            umb::mbar_init(full + i, A_TMA ? 1 : 1 + Cfg::kWarpsPerStage);          // the TMA thread, and the stage's copying warps
             umb::mbar_init(empty + i, 1);
         }
         for (int i = 0; i < 2; ++i) {
@@ -152,7 +195,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int rr = lane >> 3, cc = (lane & 7) * 4;
         for (uint32_t it = 0; w.step(); ++it) {
             const uint32_t acc = it & 1;
-            if (!__all_sync(0xffffffffu, tc_wait(acc_full + acc, (it >> 1) & 1, quit))) break;      // (and the warp is one again)
+            if (!__all_sync(0xffffffffu, tc_poll(acc_full + acc, (it >> 1) & 1, quit))) break;      // (and the warp is one again)
             umb::tc_fence_after();
             const uint32_t src = tmem + acc * BN + ((uint32_t)(q * 32) << 16);
             const int rows = w.rows - w.m0 - q * 32, n_hi = a.N - w.n0 * kOut;      // rows of this quarter, columns of the tile
@@ -170,12 +213,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     if (lane == 0) umb::mbar_arrive(acc_empty + acc);
                 }
                 if (c0 >= n_hi || rows <= 0) continue;
-                if (DUAL || a.bias != nullptr || a.unary) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        v[j] = __float_as_uint(finish_sum<DUAL>(a, __uint_as_float(v[j]), DUAL ? __uint_as_float(u[DUAL ? j : 0]) : 0.f,
-                                                                min(w.n0 * kOut + c0 + j, a.N - 1)));
-                }
+                if (DUAL || a.bias != nullptr || a.unary) tc_finish<DUAL>(a, v, u, w.n0 * kOut + c0);
 #pragma unroll
                 for (int j = 0; j < 32; j += 4)
                     *reinterpret_cast<uint4*>(so + lane * kTcStageRow + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
@@ -210,46 +248,41 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
         }
     } else if (!A_TMA) {
-        // a warp's eight lanes copy a row's 128 bytes of the k step, 128 / 16 rows per thread; the image is the one a
-        // 128-byte-swizzled TMA box would leave
-        const int tid = threadIdx.x - 192, ch = tid & 7, r0 = tid >> 3;
+        // eight lanes copy a row's 128 bytes of the k step; the image is the one a 128-byte-swizzled TMA box would leave
+        constexpr int PW = Cfg::kWarpsPerStage, RS = 4 * PW;                // rows a stage's warps copy side by side
+        const int cw = warp - 6, st = cw / PW, ch = lane & 7, r0 = (cw % PW) * 4 + (lane >> 3);
+        int* src = reinterpret_cast<int*>(bars + 32) + cw * kTcRows;        // this warp's list of the tile's source rows
         const __nv_bfloat16* A = (const __nv_bfloat16*)a.A + ch * 8;
-        uint32_t s = 0, ph = 1, done = 0, issued = 0;
-        const uint32_t dst0 = r0 * 128 + ((ch ^ (r0 & 7)) << 4);        // r0 + 16 i keeps r0's place inside its group of eight rows
+        const uint32_t base = smem_u32(smem + st * Cfg::kStage);
+        uint32_t uses = 0;
+        int unit = 0;                                       // k steps of the tiles before, modulo the ring
         bool ok = true;
-        auto publish = [&]() {
-            umb::fence_proxy_async_smem();                  // the copies of this thread are complete: show them to the tensor core
-            __syncwarp();
-            if (lane == 0) umb::mbar_arrive(full + done % kStages);
-            ++done;
-        };
         while (ok && w.step()) {
-            int64_t row[8];
+            __syncwarp();
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int r = w.m0 + r0 + 16 * i, p = w.row_lo + r;
-                row[i] = r < w.rows ? (int64_t)(a.row_src ? a.row_src[p] : p) * a.lda + (t.a_grouped ? (int64_t)w.g * a.a_goff : 0) : -1;
+            for (int i = 0; i < kTcRows / 32; ++i) {
+                const int r = w.m0 + i * 32 + lane;
+                src[i * 32 + lane] = r < w.rows ? (a.row_src ? a.row_src[w.row_lo + r] : w.row_lo + r) : -1;
             }
-            for (int k = 0; k < t.k_steps; ++k) {
-                if (!(ok = __all_sync(0xffffffffu, tc_wait(empty + s, ph, quit)))) break;
-                const uint32_t dst = smem_u32(smem + s * Cfg::kStage) + dst0;
+            __syncwarp();
+            const int rows = min(kTcRows, w.rows - w.m0);
+            const __nv_bfloat16* Ag = A + (t.a_grouped ? (int64_t)w.g * a.a_goff : 0);
+            for (int k = (st - unit + kStages) % kStages; k < t.k_steps; k += kStages, ++uses) {
+                if (!(ok = __all_sync(0xffffffffu, tc_poll(empty + st, (uses & 1) ^ 1, quit)))) break;
                 const int kc = k * kTcK + ch * 8;
                 const int bytes = kc < a.K ? 16 : 0;        // behind the last column: zeros (K is a multiple of 8)
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    if (row[i] >= 0)                        // a row that is not there keeps what the stage held: its sums are not stored
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + i * 2048),
-                                     "l"(A + row[i] + (bytes ? k * kTcK : 0)), "r"(bytes) : "memory");
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                if (++s == kStages) { s = 0; ph ^= 1; }
-                if (++issued > kTcLag) {
-                    asm volatile("cp.async.wait_group %0;" ::"n"(kTcLag) : "memory");
-                    publish();
-                }
+                // (rows that are not there keep what the stage held: their sums are not stored)
+#pragma unroll 8
+                for (int r = r0; r < rows; r += RS)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + r * 128 + ((ch ^ (r & 7)) << 4)),
+                                 "l"(Ag + (int64_t)src[r] * a.lda + (bytes ? k * kTcK : 0)), "r"(bytes) : "memory");
+                asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+                umb::fence_proxy_async_smem();              // the copies of this thread are complete: show them to the tensor core
+                __syncwarp();
+                if (lane == 0) umb::mbar_arrive(full + st);
             }
+            unit = (unit + t.k_steps) % kStages;
         }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        while (done < issued) publish();
     }
     __syncthreads();
     tc_settle(quit);
@@ -301,7 +334,7 @@ static int launch_tc(const GemmArgs& a, TcArgs t, int sms, cudaStream_t st) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
     if (e != cudaSuccess) return (int)e;
     const int64_t tiles = (int64_t)t.groups * t.m_tiles * t.n_tiles;            // (sorted by expert: at most)
-    kernel<<<(int)(tiles < sms ? tiles : sms), A_TMA ? 192 : 320, Cfg::kSmem, st>>>(ma, mw, a, t);
+    kernel<<<(int)(tiles < sms ? tiles : sms), Cfg::threads(A_TMA), Cfg::kSmem, st>>>(ma, mw, a, t);
     return 0;
 }
 
@@ -324,12 +357,18 @@ int launch_gemm_tc(const GemmArgs& a, int groups, bool dual, bool c_f32, cudaStr
     t.m_tiles = (a.M + kTcRows - 1) / kTcRows;
     const int es = c_f32 ? 4 : 2;
     t.vec_c = (uintptr_t)a.C % (4 * es) == 0 && a.ldc % 4 == 0 && a.c_goff % 4 == 0;
-    // The widest tile that still gives every SM one: 256 columns need the least shared-memory traffic per product.  (Rows
-    // sorted by expert: how they fall is only known on the device; spread evenly is the guess.)
+    // The tile width with the shortest longest walk: rounds of tiles over the SMs times a k step's cost, which is the tensor
+    // core's 128 clocks for 256 columns and more than half, a quarter of that for 128 and 64 (the activation tile is fetched
+    // and read from shared memory for fewer products).  (Rows sorted by expert: how they fall is only known on the device;
+    // spread evenly is the guess.)
     const int64_t m = a.grp_off != nullptr ? (int64_t)groups * ((a.M + groups * kTcRows - 1) / (groups * kTcRows)) : (int64_t)groups * t.m_tiles;
-    auto enough = [&](int bn) { const int out = dual ? bn / 2 : bn; return m * ((a.N + out - 1) / out) >= sms; };
-    if (enough(256)) return launch_tc_any<256>(a, t, dual, c_f32, sms, st);
-    if (enough(128)) return launch_tc_any<128>(a, t, dual, c_f32, sms, st);
+    auto cost = [&](int bn, int step) {
+        const int out = dual ? bn / 2 : bn;
+        return (m * ((a.N + out - 1) / out) + sms - 1) / sms * step;
+    };
+    const int64_t c256 = cost(256, 128), c128 = cost(128, 72), c64 = cost(64, 52);
+    if (c256 <= c128 && c256 <= c64) return launch_tc_any<256>(a, t, dual, c_f32, sms, st);
+    if (c128 <= c64) return launch_tc_any<128>(a, t, dual, c_f32, sms, st);
     return launch_tc_any<64>(a, t, dual, c_f32, sms, st);
 }
 
