@@ -295,6 +295,48 @@ static void launch_add_norm_vec(float* x, const umbs_delta_t& d, const int32_t* 
 #undef UMBS_ANV
 }
 
+// add_rms_norm_kernel in 16-byte pieces, everything a row needs in flight before its sum: KEEP4 pieces per thread, by the
+// width alone (so that a row's sum is the same tree in every step).  A decode step's rows are as many blocks and nothing but
+// latency: 4 rows of 1024 took 7.0 us as scalar loads, the weight fetched behind the sum.
+template <typename T, int KEEP4>
+__global__ void __launch_bounds__(512) add_rms_norm_vec_kernel(float* __restrict__ x, const float* __restrict__ delta, const int32_t* __restrict__ rows,
+                                                               const float* __restrict__ w, float w_offset, int width, float eps,
+                                                               T* __restrict__ y, float* __restrict__ copy) {
+    __shared__ float red[32];
+    const int r = blockIdx.x, n4 = width / 4;
+    const int64_t src = rows ? rows[r] : r;
+    float4* xr = reinterpret_cast<float4*>(x + src * width);
+    float4 v[KEEP4], g[KEEP4];
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < KEEP4; ++i) {
+        const int e = threadIdx.x + i * blockDim.x;
+        v[i] = g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (e < n4) {
+            v[i] = xr[e];
+            if (w != nullptr) g[i] = reinterpret_cast<const float4*>(w)[e];
+            if (delta != nullptr) {
+                const float4 d = reinterpret_cast<const float4*>(delta + src * width)[e];
+                v[i] = make_float4(v[i].x + d.x, v[i].y + d.y, v[i].z + d.z, v[i].w + d.w);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < KEEP4; ++i)
+        sum = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, fmaf(v[i].w, v[i].w, sum))));
+    const float inv = 1.f / sqrtf(block_sum_one_barrier(sum, red) / (float)width + eps);
+#pragma unroll
+    for (int i = 0; i < KEEP4; ++i) {
+        const int e = threadIdx.x + i * blockDim.x;
+        if (e >= n4) continue;
+        if (rows == nullptr && delta != nullptr) xr[e] = v[i];
+        if (copy != nullptr) reinterpret_cast<float4*>(copy + (int64_t)r * width)[e] = v[i];
+        if (y != nullptr)
+            store4(y + (int64_t)r * width + 4 * e, make_float4(v[i].x * inv * (w_offset + g[i].x), v[i].y * inv * (w_offset + g[i].y),
+                                                               v[i].z * inv * (w_offset + g[i].z), v[i].w * inv * (w_offset + g[i].w)));
+    }
+}
+
 // One block per token: the embedding row through an RMS norm, in fp32 and (for a product that reads it) as T.
 template <typename T>
 __global__ void embedding_norm_kernel(const int32_t* __restrict__ ids, const T* __restrict__ table, float scale, const float* __restrict__ w,
@@ -486,8 +528,10 @@ __global__ void attention_prep_kernel(const float* __restrict__ proj, int64_t ld
         }
 }
 
-// One block per (block of tokens completed by the step, sequence, 256 columns): the fp32 mean, in position order, of the
-// block's kv rows as the cache holds them.  Eight rows are loaded ahead of the additions, which stay in position order.
+// One block per (block of tokens completed by the step, sequence, 128 columns): the fp32 mean, in position order, of the
+// block's kv rows as the cache holds them.  Sixteen rows are loaded ahead of the additions, which stay in position order; a
+// row's place in the ring is the one before it plus one.  (Eight at a time with a division per row: 34 us for the blocks that
+// 64 decoding sequences complete, all of it latency.)
 template <typename T>
 __global__ void kv_pool_kernel(const T* __restrict__ kv, const T* __restrict__ kv_cache, int kv_len, T* __restrict__ pool_cache,
                                int pool_len, Batch b, int row, int pool) {
@@ -496,21 +540,26 @@ __global__ void kv_pool_kernel(const T* __restrict__ kv, const T* __restrict__ k
     if ((int64_t)(blk + 1) * pool > (int64_t)pos0 + len || blk >= pool_len) return;
     const int c = blockIdx.z * blockDim.x + threadIdx.x;
     if (c >= row) return;
-    auto at = [&](int j) -> float {
-        const T* src = j >= pos0 ? kv + (int64_t)(start + j - pos0) * row : kv_cache + ((int64_t)slot * kv_len + j % kv_len) * row;
-        return to_f32(src[c]);
-    };
-    float acc = 0.f;
     const int j0 = blk * pool;
-    int j = 0;
-    for (; j + 8 <= pool; j += 8) {
-        float x[8];
+    const T* step = kv + ((int64_t)start - pos0) * row + c;      // row j of the step's own rows at step + j row
+    const T* ring = kv_cache + (int64_t)slot * kv_len * row + c;
+    int at = j0 % kv_len;                                        // row j0 + j of the ring
+    float acc = 0.f;
+    constexpr int U = 16;
+    for (int j = 0; j < pool; j += U) {
+        float x[U];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) x[u] = at(j0 + j + u);
+        for (int u = 0; u < U; ++u) {
+            if (j + u < pool) {
+                const int p = j0 + j + u;
+                x[u] = to_f32(p >= pos0 ? step[(int64_t)p * row] : ring[(int64_t)at * row]);
+                at = at + 1 == kv_len ? 0 : at + 1;
+            }
+        }
 #pragma unroll
-        for (int u = 0; u < 8; ++u) acc += x[u];
+        for (int u = 0; u < U; ++u)
+            if (j + u < pool) acc += x[u];
     }
-    for (; j < pool; ++j) acc += at(j0 + j);
     pool_cache[((int64_t)slot * pool_len + blk) * row + c] = from_f32<T>(acc / (float)pool);
 }
 
@@ -530,8 +579,18 @@ extern "C" int umbs_add_rms_norm(int dtype, float* x, const float* delta, const 
     if (n <= 0) return 0;
     if (x == nullptr || width <= 0 || (y != nullptr && w == nullptr)) return UMB_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
-    const int threads = width >= 2048 ? 256 : (width >= 512 ? 128 : 64);
-    UMBS_DISPATCH_T(dtype, add_rms_norm_kernel<T><<<n, threads, 0, st>>>(x, delta, rows, w, w_offset, width, eps, (T*)y, copy));
+    const uintptr_t ptrs = (uintptr_t)x | (uintptr_t)delta | (uintptr_t)w | (uintptr_t)copy | (uintptr_t)y;
+    if (width % 4 == 0 && width <= 8192 && ptrs % 16 == 0) {
+        const int n4 = width / 4, keep = n4 <= 256 ? 1 : (n4 <= 1024 ? 2 : 4), vt = ((n4 + keep - 1) / keep + 31) / 32 * 32;
+#define UMBS_ARN(K) UMBS_DISPATCH_T(dtype, (add_rms_norm_vec_kernel<T, K><<<n, vt, 0, st>>>(x, delta, rows, w, w_offset, width, eps, (T*)y, copy)))
+        if (keep == 1) UMBS_ARN(1);
+        else if (keep == 2) UMBS_ARN(2);
+        else UMBS_ARN(4);
+#undef UMBS_ARN
+    } else {
+        const int threads = width >= 2048 ? 256 : (width >= 512 ? 128 : 64);
+        UMBS_DISPATCH_T(dtype, add_rms_norm_kernel<T><<<n, threads, 0, st>>>(x, delta, rows, w, w_offset, width, eps, (T*)y, copy));
+    }
     count_launches(1);
     return (int)cudaGetLastError();
 }
@@ -682,8 +741,8 @@ extern "C" int umbs_kv_pool(int dtype, const void* kv, const void* kv_cache, int
     if (batch->n_tokens <= 0 || pool <= 0) return 0;
     if (kv_len < pool) return UMB_ERR_ARG;               // a block's older tokens must still sit in the cache
     cudaStream_t st = (cudaStream_t)stream;
-    const dim3 grid(batch->max_seq_len / pool + 1, batch->n_seqs, (row + 255) / 256);
-    UMBS_DISPATCH_T(dtype, kv_pool_kernel<T><<<grid, 256, 0, st>>>((const T*)kv, (const T*)kv_cache, kv_len, (T*)pool_cache,
+    const dim3 grid(batch->max_seq_len / pool + 1, batch->n_seqs, (row + 127) / 128);
+    UMBS_DISPATCH_T(dtype, kv_pool_kernel<T><<<grid, 128, 0, st>>>((const T*)kv, (const T*)kv_cache, kv_len, (T*)pool_cache,
                                                                    pool_len, *batch, row, pool));
     count_launches(1);
     return (int)cudaGetLastError();
