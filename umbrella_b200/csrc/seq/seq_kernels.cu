@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 #include <algorithm>
+#include <type_traits>
 #include <stdint.h>
 
 #include "seq_internal.h"
@@ -564,19 +565,99 @@ __global__ void ring_append_kernel(const T* __restrict__ c, T* __restrict__ ring
     const int t = blockIdx.x, s = b.tok_seq[t], pos = b.tok_pos[t];
     if (pos < b.seq_pos0[s] + b.seq_len[s] - ring_len) return;     // a later token of this step takes the row
     T* dst = ring + ((int64_t)b.seq_slot[s] * ring_len + pos % ring_len) * R;
-    for (int r = threadIdx.x; r < R; r += blockDim.x) dst[r] = c[(int64_t)t * R + r];
+    const T* src = c + (int64_t)t * R;
+    constexpr int V = 16 / sizeof(T);
+    if (R % V == 0 && (((uintptr_t)c | (uintptr_t)ring) & 15) == 0) {
+        for (int r = threadIdx.x * V; r < R; r += blockDim.x * V) *reinterpret_cast<uint4*>(dst + r) = *reinterpret_cast<const uint4*>(src + r);
+    } else {
+        for (int r = threadIdx.x; r < R; r += blockDim.x) dst[r] = src[r];
+    }
 }
 
 // ------------------------------------------------------------------------------------------------ routing
 // A router logit: fp32 dot product of one token's activations with one expert's row, lanes striding over the width and
 // a shuffle tree at the end.  Both routing kernels below use this one function, so a token's logits -- and with them its
 // experts -- do not depend on which of the two ran.
+// four neighbouring numbers as they are stored, and as fp32
+template <typename T> struct Raw4;
+template <> struct Raw4<float> { typedef float4 type; };
+template <> struct Raw4<__nv_bfloat16> { typedef uint2 type; };
+__device__ __forceinline__ void widen4(const float4& v, float (&f)[4]) { f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w; }
+__device__ __forceinline__ void widen4(const uint2& v, float (&f)[4]) {
+    f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xffff0000u);
+    f[2] = __uint_as_float(v.y << 16); f[3] = __uint_as_float(v.y & 0xffff0000u);
+}
+// Router logits of TT tokens x EE experts by one warp: a lane takes four neighbouring numbers of every 128 (vec: every row
+// can be read four numbers at a time; else one of every 32).  A logit is the same chain of
+// additions whatever TT and EE are, so a token's experts do not depend on the kernel that routes it.
+template <int TT, int EE, typename T>
+__device__ __forceinline__ void router_logits(const T* const (&hr)[TT], const float* const (&w)[EE], int width, bool vec, int lane, float (&s)[TT][EE]) {
+#pragma unroll
+    for (int t = 0; t < TT; ++t)
+#pragma unroll
+        for (int e = 0; e < EE; ++e) s[t][e] = 0.f;
+    if (vec) {
+        // several pieces of 128 in flight at a time: a step of few tokens is a chain of load latencies (64 tokens, 16 experts of
+        // width 2048: 23.6 us a piece at a time, 13.7 us four; with eight tokens to a warp two are what the registers hold)
+        auto pieces = [&](auto count, int k0) {
+            constexpr int U = decltype(count)::value;
+            typename Raw4<T>::type hr4[U][TT];
+            float4 w4[U][EE];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+#pragma unroll
+                for (int t = 0; t < TT; ++t) hr4[u][t] = *reinterpret_cast<const typename Raw4<T>::type*>(hr[t] + k0 + 128 * u);
+#pragma unroll
+                for (int e = 0; e < EE; ++e) w4[u][e] = *reinterpret_cast<const float4*>(w[e] + k0 + 128 * u);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                float hv[TT][4], wv[EE][4];
+#pragma unroll
+                for (int t = 0; t < TT; ++t) widen4(hr4[u][t], hv[t]);
+#pragma unroll
+                for (int e = 0; e < EE; ++e) widen4(w4[u][e], wv[e]);
+#pragma unroll
+                for (int t = 0; t < TT; ++t)
+#pragma unroll
+                    for (int e = 0; e < EE; ++e)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) s[t][e] = fmaf(hv[t][i], wv[e][i], s[t][e]);
+            }
+        };
+        int k = lane * 4;
+        constexpr int U = TT <= 4 ? 4 : 2;
+        for (; k + 128 * (U - 1) < width; k += 128 * U) pieces(std::integral_constant<int, U>{}, k);
+        for (; k < width; k += 128) pieces(std::integral_constant<int, 1>{}, k);
+    } else {
+        for (int k = lane; k < width; k += 32) {
+            float hv[TT], wv[EE];
+#pragma unroll
+            for (int t = 0; t < TT; ++t) hv[t] = to_f32(hr[t][k]);
+#pragma unroll
+            for (int e = 0; e < EE; ++e) wv[e] = w[e][k];
+#pragma unroll
+            for (int t = 0; t < TT; ++t)
+#pragma unroll
+                for (int e = 0; e < EE; ++e) s[t][e] = fmaf(hv[t], wv[e], s[t][e]);
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < TT; ++t)
+#pragma unroll
+        for (int e = 0; e < EE; ++e) s[t][e] = warp_sum(s[t][e]);
+}
 template <typename T>
-__device__ __forceinline__ float router_logit(const T* __restrict__ hr, const float* __restrict__ w, int width, int lane) {
-    float s = 0.f;
-#pragma unroll 8
-    for (int k = lane; k < width; k += 32) s = fmaf(to_f32(hr[k]), w[k], s);
-    return warp_sum(s);
+__host__ __device__ __forceinline__ bool rows_vec(const void* h, const void* w, const void* gate_w, int width) {
+    return width % 4 == 0 && (uintptr_t)h % (4 * sizeof(T)) == 0 && (((uintptr_t)w | (uintptr_t)gate_w) & 15) == 0;
+}
+template <typename T>
+__device__ __forceinline__ float router_logit(const T* hr, const float* w, int width, bool vec, int lane) {
+    const T* const h1[1] = {hr};
+    const float* const w1[1] = {w};
+    float s[1][1];
+    router_logits<1, 1>(h1, w1, width, vec, lane, s);
+    return s[0][0];
 }
 
 // `top` rounds of arg-max over z (lowest index wins a tie; z is consumed) and the softmax over the chosen logits.
@@ -643,28 +724,44 @@ __device__ __forceinline__ void route_choose(float* z, int experts, int top, int
     for (int k = 0; k < top; ++k) w_out[k] = w_out[k] / den * wscale;
 }
 
-// One block per token: the warps share the experts' logits, then one thread chooses.
-template <typename T>
-__global__ void __launch_bounds__(256) moe_router_kernel(const T* __restrict__ h, int n, int width, const float* __restrict__ wr,
+// One block per kRtTok tokens: a warp works out the logits of kRtExp experts for all of them, so that a router weight is
+// fetched once per kRtTok tokens and a token's number once per kRtExp experts; then a thread per token chooses.  (A block per
+// token read all weights for each token: 512 MB through L2 for 4096 tokens, 16 experts of width 2048, 112 us.)
+constexpr int kRtExp = 4;
+
+template <typename T, int kRtTok>
+__global__ void __launch_bounds__(256, kRtTok > 4 ? 2 : 1) moe_router_kernel(const T* __restrict__ h, int n, int width, const float* __restrict__ wr,
                                                          int experts, int top, int mode, int groups, int keep, float wscale,
                                                          float* __restrict__ sel_w, int32_t* __restrict__ sel_e,
                                                          int32_t* __restrict__ counts, const float* __restrict__ gate_w,
                                                          float* __restrict__ gate_out) {
-    extern __shared__ float z[];           // [experts]
+    extern __shared__ float z[];           // [kRtTok][experts]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int t = blockIdx.x;
-    const T* hr = h + (int64_t)t * width;
-    for (int e = warp; e < experts + (gate_w != nullptr ? 1 : 0); e += nw) {
-        // one more row for the token's gate (the shared expert's factor): sigmoid of its logit
-        const float s = router_logit(hr, e < experts ? wr + (int64_t)e * width : gate_w, width, lane);
-        if (lane == 0) {
-            if (e < experts) z[e] = s;
-            else gate_out[t] = 1.f / (1.f + expf(-s));
-        }
+    const bool vec = rows_vec<T>(h, wr, gate_w, width);
+    const int t0 = blockIdx.x * kRtTok, rows = experts + (gate_w != nullptr ? 1 : 0);      // one more row for the tokens' gate
+    const T* hr[kRtTok];
+#pragma unroll
+    for (int t = 0; t < kRtTok; ++t) hr[t] = h + (int64_t)min(t0 + t, n - 1) * width;
+    for (int e0 = warp * kRtExp; e0 < rows; e0 += nw * kRtExp) {
+        const float* w[kRtExp];
+#pragma unroll
+        for (int e = 0; e < kRtExp; ++e) w[e] = e0 + e < experts ? wr + (int64_t)(e0 + e) * width : (e0 + e < rows ? gate_w : wr);
+        float s[kRtTok][kRtExp];
+        router_logits<kRtTok, kRtExp>(hr, w, width, vec, lane, s);
+#pragma unroll
+        for (int t = 0; t < kRtTok; ++t)
+#pragma unroll
+            for (int e = 0; e < kRtExp; ++e) {
+                const float v = s[t][e];
+                if (lane != 0 || t0 + t >= n || e0 + e >= rows) continue;
+                if (e0 + e < experts) z[t * experts + e0 + e] = v;
+                else gate_out[t0 + t] = 1.f / (1.f + expf(-v));             // the shared expert's factor: sigmoid of its logit
+            }
     }
     __syncthreads();
-    if (threadIdx.x == 0)
-        route_choose(z, experts, top, mode, groups, keep, wscale, sel_w + (int64_t)t * top, sel_e + (int64_t)t * top, counts);
+    const int t = t0 + threadIdx.x;
+    if (threadIdx.x < kRtTok && t < n)
+        route_choose(z + threadIdx.x * experts, experts, top, mode, groups, keep, wscale, sel_w + (int64_t)t * top, sel_e + (int64_t)t * top, counts);
 }
 
 // The whole routing of a small step (a decode step) in one block: logits of every (token, expert) pair, the choice per
@@ -683,14 +780,15 @@ __global__ void __launch_bounds__(1024) moe_route_small_kernel(const T* __restri
     int32_t* offs = counts + experts;                // [experts + 1]
     int32_t* chosen = offs + experts + 1;            // [n top]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const bool vec = rows_vec<T>(h, wr, gate_w, width);
     for (int i = threadIdx.x; i < experts; i += blockDim.x) counts[i] = 0;
     for (int i = warp; i < n * experts; i += nw) {
         const int t = i / experts, e = i - t * experts;
-        const float s = router_logit(h + (int64_t)t * width, wr + (int64_t)e * width, width, lane);
+        const float s = router_logit(h + (int64_t)t * width, wr + (int64_t)e * width, width, vec, lane);
         if (lane == 0) zs[i] = s;
     }
     for (int t = warp; gate_w != nullptr && t < n; t += nw) {
-        const float s = router_logit(h + (int64_t)t * width, gate_w, width, lane);
+        const float s = router_logit(h + (int64_t)t * width, gate_w, width, vec, lane);
         if (lane == 0) gate_out[t] = 1.f / (1.f + expf(-s));
     }
     __syncthreads();
@@ -800,7 +898,7 @@ template <typename T>
 __global__ void token_gate_kernel(const T* __restrict__ h, int n, int width, const float* __restrict__ w, float* __restrict__ g) {
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (t >= n) return;
-    const float s = router_logit(h + (int64_t)t * width, w, width, threadIdx.x & 31);
+    const float s = router_logit(h + (int64_t)t * width, w, width, rows_vec<T>(h, w, nullptr, width), threadIdx.x & 31);
     if ((threadIdx.x & 31) == 0) g[t] = 1.f / (1.f + expf(-s));
 }
 
@@ -1137,10 +1235,21 @@ extern "C" int umbs_moe_route_scaled(int dtype, const void* h, int n, int width,
     int32_t* sel_e = scratch + 2 * experts;    // [n top]
     cudaError_t e = cudaMemsetAsync(counts, 0, experts * sizeof(int32_t), st);
     if (e != cudaSuccess) return (int)e;
-    const int rthreads = experts >= 8 ? 256 : 32 * experts;
-    UMBS_DISPATCH_T(dtype, moe_router_kernel<T><<<n, rthreads, (size_t)experts * sizeof(float), st>>>(
-                               (const T*)h, n, width, w_router, experts, top, mode, groups, keep, weight_scale, sel_w, sel_e, counts,
-                               gate_w, gate_out));
+    const int rthreads = 32 * std::min(8, (experts + (gate_w != nullptr) + kRtExp - 1) / kRtExp);
+    // (more tokens to a block once there are blocks enough; thousands of experts need the larger shared memory)
+#define UMBS_ROUTER(TT)                                                                                                          \
+    UMBS_DISPATCH_T(dtype, {                                                                                                     \
+        const size_t smem = (size_t)TT * experts * sizeof(float);                                                                \
+        if (smem > 48 * 1024) {                                                                                                  \
+            e = cudaFuncSetAttribute(moe_router_kernel<T, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
+            if (e != cudaSuccess) return (int)e;                                                                                 \
+        }                                                                                                                        \
+        moe_router_kernel<T, TT><<<(n + TT - 1) / TT, rthreads, smem, st>>>((const T*)h, n, width, w_router, experts, top, mode, groups, keep, \
+                                                                            weight_scale, sel_w, sel_e, counts, gate_w, gate_out); \
+    })
+    if (n > 1024 && experts <= 1024) UMBS_ROUTER(8);
+    else UMBS_ROUTER(4);
+#undef UMBS_ROUTER
     moe_offsets_kernel<<<1, 32, 0, st>>>(counts, experts, grp_off, cursor);
     const int pairs = n * top;
     moe_scatter_kernel<<<(pairs + 255) / 256, 256, 0, st>>>(sel_e, pairs, top, grp_off, cursor, pair_tok, pair_pos);
