@@ -69,7 +69,9 @@ def gemm(a: torch.Tensor, w: torch.Tensor, *, out_f32: bool = False, groups: int
     N = (w3.shape[1] // (2 if dual else 1)) if n is None else n
     M = a.shape[0] if rows is None else rows
     cols = N if (groups == 1 or grp_off is not None) else groups * c_goff        # expert groups share the columns
-    out = torch.zeros((M, cols), dtype=torch.float32 if out_f32 else a.dtype, device=a.device)
+    # (zeros only where the product may leave gaps: rows behind the last group's, columns between the groups')
+    make = torch.empty if groups == 1 and grp_off is None else torch.zeros
+    out = make((M, cols), dtype=torch.float32 if out_f32 else a.dtype, device=a.device)
     S.check(S.load().umbs_gemm(mode, _p(a), a.stride(0), a_goff, _p(w3), w3.stride(1), w3.stride(0), _p(out), out.stride(0),
                                c_goff, int(out_f32), M if max_rows is None else max_rows, N, K, groups, _p(grp_off),
                                _p(row_src), int(dual), float(limit), _stream()), "gemm")
@@ -246,7 +248,8 @@ def gemm_ex(a: torch.Tensor, w: torch.Tensor, *, out_f32: bool = False, groups: 
     K = w3.shape[2] if k is None else k
     N = (w3.shape[1] // (2 if act else 1)) if n is None else n
     M = a.shape[0]
-    out = torch.zeros((M, N if groups == 1 else groups * c_goff), dtype=torch.float32 if out_f32 else a.dtype, device=a.device)
+    make = torch.empty if groups == 1 else torch.zeros
+    out = make((M, N if groups == 1 else groups * c_goff), dtype=torch.float32 if out_f32 else a.dtype, device=a.device)
     S.check(S.load().umbs_gemm_ex(mode, _p(a), a.stride(0), a_goff, _p(w3), w3.stride(1), w3.stride(0), _p(out), out.stride(0),
                                   c_goff, int(out_f32), M, N, K, groups, None, None, int(act), float(limit), _p(bias),
                                   _p(out_gate), out_gate.stride(0) if out_gate is not None else 0, gate_goff, _stream()),
