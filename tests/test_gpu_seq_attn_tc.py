@@ -39,7 +39,7 @@ def _cached(ops, dt, seqs, heads, kv_heads, dim, vdim, seed=3, ring=512, pool=0,
     head = torch.randn(heads, generator=g, device=DEV)
     batch = ops.RaggedBatch(seqs, DEV)
     if pool:
-        kw.update(pool=pool, pool_cache=_r(g, 3, ring // pool + 1, row).to(dt))
+        kw.update(pool=pool, pool_cache=_r(g, 3, 704 // pool + 1, row).to(dt))       # every position of the steps below
     if "sink" in opts:
         kw["sink"] = head
     if "bias" in opts:
@@ -127,3 +127,31 @@ def test_keys_of_the_step(ops, dim, shared, vdim):
         got, ref = (ops.window_attention_shared(q.to(dt), kv[:, :Hh * dim].to(dt), ks.to(dt) if shared else None, kv[:, Hh * dim:].to(dt), batch,
                                                 Hh, (dim + shared) ** -0.5, **kw) for dt in (torch.bfloat16, torch.float32))
         assert H.rel_err(got, ref.cpu()) < TOL
+
+
+# ---------------------------------------------------------------------------------------------- decode steps
+# one token per sequence: the first token, a tile of 32 keys and its edges, several tiles per warp, splits, a ring that wraps
+DECODE = [[(0, 1, 0, 0), (1, 1, 31, 0), (2, 1, 32, 0)], [(1, 1, 127, 0)], [(0, 1, 128, 0), (2, 1, 510, 0)], [(2, 1, 700, 0), (0, 1, 33, 0)]]
+
+
+@pytest.mark.parametrize("heads,kv_heads", [(1, 1), (4, 2), (6, 2), (16, 2), (10, 2)])
+@pytest.mark.parametrize("dim,vdim", [(128, 128), (64, 40), (8, 8), (104, 72)])
+def test_decode_sizes(ops, heads, kv_heads, dim, vdim):
+    for step in DECODE:
+        _both(ops, step, heads, kv_heads, dim, vdim, window=0 if step[0][2] < 600 else 500)
+
+
+@pytest.mark.parametrize("window,pool", [(1, 4), (33, 16), (300, 0)])
+def test_decode_masks_and_outputs(ops, window, pool):
+    from umbrella_b200 import _lib_seq as S
+    for step in DECODE:
+        _both(ops, step, 8, 2, 64, 64, window=window, pool=pool, mode=S.UMBS_ATTN_SOFTMAX_SINK, opts=("sink", "gate_head"))
+        _both(ops, step, 8, 2, 64, 64, window=window, pool=pool, mode=S.UMBS_ATTN_SIGMOID, opts=("bias", "gate"))
+        _both(ops, step, 8, 2, 64, 64, window=window, pool=pool, mode=S.UMBS_ATTN_SOFTMAX_SINK, opts=("sink",), split=False)
+
+
+@pytest.mark.parametrize("kw,opts", [(dict(softcap=5.0), ("dist",)), (dict(chunk=48), ("gate",)), (dict(maps=2, diff_lambda=0.4, unit_norm=True), ("gate",)),
+                                     (dict(softcap=20.0), ("dist", "talk"))])
+def test_decode_score_options(ops, kw, opts):
+    for step in DECODE[:3]:
+        _both(ops, step, 4, 2, 64, 32, opts=opts + ("scored",), **kw)

@@ -9,7 +9,7 @@
 // from transposed fp32 tiles in shared memory, the weights go back through shared memory for the value product.  The key
 // tile holds 64 dimensions at a time (larger heads add their scores up over several passes), which keeps two blocks on an
 // SM for heads of 128.
-// Decode kernel (one token per sequence): one block = (sequence, head, split); a warp takes every 8th key of the block's
+// Decode kernels (one token per sequence): cached_attention_decode_group_kernel for bf16 rows of up to 128 numbers; else one block = (sequence, head, split); a warp takes every 8th key of the block's
 // share, lanes striding over the head's dimensions; partial (max, sum, output) triples are merged per block and, with more
 // than one split, by a second kernel.
 // Score options (umbs_attn_opts_t): a tanh cap, a penalty r1 ln(1 + r2 distance) per head, a chunked mask, several maps per
@@ -369,6 +369,253 @@ __global__ void __launch_bounds__(32 * kCdWarps) cached_attention_decode_kernel(
     }
 }
 
+// Decode steps over bf16 rows: the query heads that share a key/value head together, so that a key and a value are fetched
+// once for all of them.  One block = (split, up to eight heads of a key/value head, sequence), four warps that each take every
+// fourth tile of 32 keys of the split, with running (maximum, sum, output) of their own.  A tile's rows come to shared memory
+// by 16-byte copies, keys and values as groups of their own, the next tile's while this one is worked on.  Both products are
+// 16 x 8 x 16 warp-level tensor-core products with the heads as rows (half of the 16 are empty: the step is bound by its
+// bytes, and these take a tenth of the instructions that FMAs would): bf16 products are exact, a product's sums are added up
+// by ordinary fp32 additions from one k step and one tile to the next (the tensor core would cut them off), and the fp32
+// weights go in as three bf16 numbers that add up to them exactly.  The warps' triples are merged in warp order, splits by
+// cached_attention_merge_kernel as before.
+// 64 sequences x 1040 keys, 16 heads over 4 of 128 (136 MB): a warp per (head, key) took 407 us, heads together with FMAs 65 us,
+// this 51 us.
+constexpr int kCgWarps = 4, kCgKeys = 32, kCgHeads = 8;
+
+struct GroupSizes { int ks16, vs16, warp_bytes; };          // 16-byte pieces between key rows and between value rows (odd: no bank conflicts)
+__host__ __device__ __forceinline__ GroupSizes group_sizes(int dim, int vdim) {
+    GroupSizes z;
+    z.ks16 = ((dim + 15) / 16 * 2) | 1;
+    z.vs16 = (vdim / 8) | 1;
+    z.warp_bytes = kCgKeys * (z.ks16 + z.vs16) * 16;
+    return z;
+}
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], unsigned addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], unsigned addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+// d += a b with the lower eight rows of a empty
+__device__ __forceinline__ void mma_top(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%6,%5,%6}, {%7,%8}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(32 * kCgWarps, 3) cached_attention_decode_group_kernel(CachedAttnArgs a, Batch b, int n_split, float* __restrict__ part) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int dim = a.dim, vdim = a.vdim, G = a.heads / a.kv_heads, chunks = (G + kCgHeads - 1) / kCgHeads;
+    const GroupSizes z = group_sizes(dim, vdim);
+    const int split = blockIdx.x, s = blockIdx.z, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int gc = blockIdx.y % chunks, gv = blockIdx.y / chunks;           // which eight of the group's heads; (key/value head, map, value head)
+    const int C = a.vheads, M = a.maps, cv = gv % C, mp = gv / C % M, kvh = gv / C / M;
+    const int h0 = kvh * G + gc * kCgHeads, nh = min(kCgHeads, G - gc * kCgHeads);
+    auto vhead = [&](int i) { return ((h0 + i) * M + mp) * C + cv; };
+    const VHead v0 = virtual_head(a, vhead(0));
+    const int t = b.seq_start[s], p = b.seq_pos0[s], slot = b.seq_slot[s];
+    const int window = a.window > 0 ? a.window : (1 << 30);
+    const int n_pool = pooled_visible(p, window, a.pool);
+    const int j_lo = max(max(0, p - window + 1), a.chunk > 0 ? p / a.chunk * a.chunk : 0);
+    const int n_keys = n_pool + (p - j_lo + 1);
+    const int per = ((n_keys + n_split - 1) / n_split + kCgKeys - 1) / kCgKeys * kCgKeys, lo = split * per, hi = min(n_keys, lo + per);
+    unsigned char* s_k = smem + w * z.warp_bytes;
+    unsigned char* s_v = s_k + kCgKeys * z.ks16 * 16;
+    const unsigned kaddr = (unsigned)__cvta_generic_to_shared(s_k), vaddr = (unsigned)__cvta_generic_to_shared(s_v);
+    const __nv_bfloat16* own = (const __nv_bfloat16*)a.kv + (int64_t)t * v0.row_kv;
+
+    // this lane's key of the tile at k0 (behind the run: the row itself, whose weight is then 0)
+    auto row_of = [&](int k0) -> const __nv_bfloat16* {
+        const int k = k0 + lane;
+        if (k >= hi) return own;
+        if (k < n_pool) return (const __nv_bfloat16*)a.pool_cache + ((int64_t)slot * a.pool_len + k) * v0.row_kv;
+        const int j = j_lo + (k - n_pool);
+        return j >= p ? own : (const __nv_bfloat16*)a.kv_cache + ((int64_t)slot * a.kv_len + j % a.kv_len) * v0.row_kv;
+    };
+    // the tile's keys or values: a row's 16-byte pieces side by side over the lanes, as many rows at a time as fit.  `even`: the
+    // 32 rows lie one after the other behind the first (a tile of the ring without its end), so no lane has to be asked.
+    auto fetch = [&](const __nv_bfloat16* row, bool even, int off, int n8, unsigned dst, int stride) {
+        const int rpi = 32 / n8, r = lane / n8, c = lane - r * n8;          // (n8 <= 16)
+        const unsigned out = dst + c * 16;
+        if (even) {
+            const __nv_bfloat16* src = (const __nv_bfloat16*)__shfl_sync(0xffffffffu, (unsigned long long)row, 0) + off + c * 8;
+            if (r < rpi)
+#pragma unroll 4
+                for (int k = r; k < kCgKeys; k += rpi)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(out + k * stride), "l"(src + (int64_t)k * v0.row_kv) : "memory");
+        } else {
+            for (int k = 0; k < kCgKeys; k += rpi) {
+                const int kk = min(k + r, kCgKeys - 1);
+                const __nv_bfloat16* src = (const __nv_bfloat16*)__shfl_sync(0xffffffffu, (unsigned long long)row, kk);
+                if (r < rpi && k + r < kCgKeys)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(out + kk * stride), "l"(src + off + c * 8) : "memory");
+            }
+        }
+        __syncwarp();
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto is_even = [&](int k0) {
+        const int j = j_lo + (k0 - n_pool);                                 // the first key's position
+        return k0 >= n_pool && k0 + kCgKeys <= hi && j + kCgKeys <= p && j % a.kv_len + kCgKeys <= a.kv_len;
+    };
+    const int step = kCgWarps * kCgKeys;
+    int k0 = lo + w * kCgKeys;
+    if (k0 < hi) {
+        const __nv_bfloat16* row = row_of(k0);
+        const bool even = is_even(k0);
+        fetch(row, even, v0.koff, dim / 8, kaddr, z.ks16 * 16);
+        fetch(row, even, v0.voff, vdim / 8, vaddr, z.vs16 * 16);
+    }
+    if (dim % 16) *reinterpret_cast<uint4*>(s_k + lane * z.ks16 * 16 + dim * 2) = make_uint4(0, 0, 0, 0);      // the last k step's second half
+    // rows of the products: head hr; a lane's places in a row's pairs of numbers: 2 qd, 2 qd + 1
+    const int hr = lane >> 2, qd = lane & 3, h = h0 + min(hr, nh - 1), ksteps = (dim + 15) / 16, nvt = vdim / 8;
+    uint32_t qa[8][2];
+    const __nv_bfloat16* qrow = (const __nv_bfloat16*)a.q + (int64_t)t * v0.qstride + (h * M + mp) * dim;
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int d = ks * 16 + e * 8 + qd * 2;
+            qa[ks][e] = hr < nh && d < dim ? *reinterpret_cast<const uint32_t*>(qrow + d) : 0u;
+        }
+    const float hb = MODE == UMBS_ATTN_SIGMOID && a.head_bias ? a.head_bias[h] : 0.f;
+    const float r1h = a.r1 ? a.r1[h] : 0.f, r2h = a.r1 ? a.r2[h] : 0.f;
+    float m = -INFINITY, l = 0.f, o[16][2];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) o[j][0] = o[j][1] = 0.f;
+    for (; k0 < hi; k0 += step) {
+        const bool more = k0 + step < hi, even = more && is_even(k0 + step);
+        const __nv_bfloat16* next = more ? row_of(k0 + step) : own;
+        asm volatile("cp.async.wait_group 1;" ::: "memory");                // the keys are here (the values may not be)
+        __syncwarp();
+        float sc[4][2] = {};
+#pragma unroll
+        for (int kp = 0; kp < 4; ++kp) {
+            if (kp * 2 >= ksteps) break;
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                uint32_t r[4];
+                ldsm4(r, kaddr + (nt * 8 + (lane & 7)) * z.ks16 * 16 + kp * 64 + (lane >> 3) * 16);
+                float d[2][4] = {};
+                mma_top(d[0], qa[2 * kp][0], qa[2 * kp][1], r[0], r[1]);
+                if (2 * kp + 1 < ksteps) mma_top(d[1], qa[2 * kp + 1][0], qa[2 * kp + 1][1], r[2], r[3]);
+                sc[nt][0] += d[0][0] + d[1][0];
+                sc[nt][1] += d[0][1] + d[1][1];
+            }
+        }
+        __syncwarp();
+        if (more) fetch(next, even, v0.koff, dim / 8, kaddr, z.ks16 * 16);  // (the key tile has been read)
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+        float pw[4][2];
+        float mx = -INFINITY;
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int k = k0 + nt * 8 + qd * 2 + e;
+                if (MODE == UMBS_ATTN_SIGMOID) {
+                    pw[nt][e] = k < hi ? sigmoidf_(sc[nt][e] * a.scale + hb) : 0.f;
+                } else {
+                    pw[nt][e] = k < hi ? shaped_score(a, sc[nt][e], r1h, r2h, k < n_pool ? 0 : p - (j_lo + k - n_pool)) : -INFINITY;
+                    mx = fmaxf(mx, pw[nt][e]);
+                }
+            }
+        if (MODE != UMBS_ATTN_SIGMOID) {
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            const float mn = fmaxf(m, mx), ref = mn > -INFINITY ? mn : 0.f, corr = expf(m - ref);      // (m = -inf the first time: corr = 0)
+            float ls = 0.f;
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    pw[nt][e] = expf(pw[nt][e] - ref);
+                    ls += pw[nt][e];
+                }
+            l = l * corr + ls;                                              // (a lane's own keys; added up at the end)
+            m = mn;
+            if (__any_sync(0xffffffffu, corr != 1.f)) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    o[j][0] *= corr;
+                    o[j][1] *= corr;
+                }
+            }
+        }
+        // the weights' three parts as row fragments of the second product, for keys 0-15 and 16-31
+        uint32_t pa[3][2][2];
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+            float x = pw[nt][0], y = pw[nt][1];
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                pa[e][nt >> 1][nt & 1] = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+                x -= __uint_as_float(__float_as_uint(x) & 0xffff0000u);
+                y -= __uint_as_float(__float_as_uint(y) & 0xffff0000u);
+            }
+        }
+        asm volatile("cp.async.wait_group 1;" ::: "memory");                // the values
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            if (j >= nvt) break;
+            uint32_t r[4];
+            ldsm4t(r, vaddr + lane * z.vs16 * 16 + j * 16);
+            float d[4] = {};
+#pragma unroll
+            for (int e = 2; e >= 0; --e) {
+                mma_top(d, pa[e][0][0], pa[e][0][1], r[0], r[1]);
+                mma_top(d, pa[e][1][0], pa[e][1][1], r[2], r[3]);
+            }
+            o[j][0] += d[0];
+            o[j][1] += d[1];
+        }
+        __syncwarp();
+        if (more) fetch(next, even, v0.voff, vdim / 8, vaddr, z.vs16 * 16);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    // merge: the warps' triples over the tiles' memory
+    float* s_o = reinterpret_cast<float*>(smem);                            // [warps][heads][vdim]
+    float* s_ml = s_o + kCgWarps * kCgHeads * vdim;                         // [warps][heads][2]
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+        if (j < nvt) *reinterpret_cast<float2*>(s_o + (w * kCgHeads + hr) * vdim + j * 8 + qd * 2) = make_float2(o[j][0], o[j][1]);
+    if (qd == 0) { s_ml[(w * kCgHeads + hr) * 2] = m; s_ml[(w * kCgHeads + hr) * 2 + 1] = l; }
+    __syncthreads();
+    for (int i = threadIdx.x; i < nh * vdim; i += 32 * kCgWarps) {
+        const int g = i / vdim, c = i - g * vdim, hh = h0 + g, vh = vhead(g);
+        float Mx = -INFINITY, L = 0.f, O = 0.f;
+        if (MODE == UMBS_ATTN_SIGMOID) {
+            for (int ww = 0; ww < kCgWarps; ++ww) O += s_o[(ww * kCgHeads + g) * vdim + c];
+        } else {
+            const float sk = (n_split == 1 && MODE == UMBS_ATTN_SOFTMAX_SINK) ? sink_score(a, hh) : -INFINITY;
+            for (int ww = 0; ww < kCgWarps; ++ww) Mx = fmaxf(Mx, s_ml[(ww * kCgHeads + g) * 2]);
+            Mx = fmaxf(Mx, sk);
+            for (int ww = 0; ww < kCgWarps; ++ww) {
+                const float mw = s_ml[(ww * kCgHeads + g) * 2], f = mw > -INFINITY ? expf(mw - Mx) : 0.f;
+                L = fmaf(s_ml[(ww * kCgHeads + g) * 2 + 1], f, L);
+                O = fmaf(s_o[(ww * kCgHeads + g) * vdim + c], f, O);
+            }
+            if (n_split == 1 && MODE == UMBS_ATTN_SOFTMAX_SINK) L += expf(sk - Mx);
+        }
+        if (n_split > 1) {
+            float* pr = part + (((int64_t)t * v0.nv + vh) * n_split + split) * (vdim + 2);
+            pr[c] = O;
+            if (c == 0) { pr[vdim] = Mx; pr[vdim + 1] = L; }
+            continue;
+        }
+        const float inv = MODE == UMBS_ATTN_SIGMOID ? 1.f : 1.f / L;
+        if (a.raw != nullptr) { a.raw[((int64_t)t * v0.nv + vh) * vdim + c] = O * inv; continue; }
+        float gt = 1.f;
+        if (a.gate) gt = sigmoidf_(a.gate[(int64_t)t * a.ldg + (a.gate_per_head ? hh : hh * vdim + c)]);
+        ((__nv_bfloat16*)a.out)[(int64_t)t * a.heads * vdim + (int64_t)hh * vdim + c] = __float2bfloat16_rn(O * inv * gt);
+    }
+}
+
 // One block per (token, head): the splits' triples, in split order, then the sink, the division and the output gate.
 template <typename T, int MODE>
 __global__ void cached_attention_merge_kernel(CachedAttnArgs a, int n_split, const float* __restrict__ part) {
@@ -404,6 +651,38 @@ static int launch_decode(const CachedAttnArgs& a, const Batch& b, int n_split, f
     cached_attention_decode_kernel<T, MODE><<<dim3(n_split, nv, b.n_seqs), 32 * kCdWarps, 0, st>>>(a, b, n_split, part);
     if (n_split > 1) cached_attention_merge_kernel<T, MODE><<<b.n_tokens * nv, a.vdim <= 128 ? 128 : 256, 0, st>>>(a, n_split, part);
     return 0;
+}
+
+// Sizes the grouped kernel takes: rows in 16-byte pieces, at most 128 numbers (eight k steps, sixteen value tiles in registers).
+static bool group_fits(const CachedAttnArgs& a) {
+    auto al = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
+    return a.dim % 8 == 0 && a.vdim % 8 == 0 && a.dim <= 128 && a.vdim <= 128 && al(a.q) && al(a.kv) && al(a.kv_cache) &&
+           (a.pool <= 0 || al(a.pool_cache));
+}
+static int group_blocks(const CachedAttnArgs& a) {
+    return a.kv_heads * a.maps * a.vheads * ((a.heads / a.kv_heads + kCgHeads - 1) / kCgHeads);
+}
+
+template <int MODE>
+static int launch_group(const CachedAttnArgs& a, const Batch& b, int n_split, float* part, cudaStream_t st) {
+    const int tiles = kCgWarps * group_sizes(a.dim, a.vdim).warp_bytes, merge = kCgWarps * kCgHeads * (a.vdim + 2) * 4, smem = tiles > merge ? tiles : merge;
+    auto kernel = cached_attention_decode_group_kernel<MODE>;
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return (int)e;
+    }
+    kernel<<<dim3(n_split, group_blocks(a), b.n_seqs), 32 * kCgWarps, smem, st>>>(a, b, n_split, part);
+    const int nv = a.heads * a.maps * a.vheads;
+    if (n_split > 1) cached_attention_merge_kernel<__nv_bfloat16, MODE><<<b.n_tokens * nv, a.vdim <= 128 ? 128 : 256, 0, st>>>(a, n_split, part);
+    return 0;
+}
+static int launch_group_any(int mode, const CachedAttnArgs& a, const Batch& b, int n_split, float* part, cudaStream_t st) {
+    switch (mode) {
+        case UMBS_ATTN_SOFTMAX: return launch_group<UMBS_ATTN_SOFTMAX>(a, b, n_split, part, st);
+        case UMBS_ATTN_SOFTMAX_SINK: return launch_group<UMBS_ATTN_SOFTMAX_SINK>(a, b, n_split, part, st);
+        case UMBS_ATTN_SIGMOID: return launch_group<UMBS_ATTN_SIGMOID>(a, b, n_split, part, st);
+    }
+    return UMB_ERR_ARG;
 }
 
 template <typename T>
@@ -528,15 +807,29 @@ extern "C" int umbs_cached_attention_ex(int dtype, int mode, const void* q, cons
         int keys = window > 0 ? (batch->max_pos0 < window ? batch->max_pos0 + 1 : window + (pool > 0 ? batch->max_pos0 / pool : 0))
                               : batch->max_pos0 + 1;
         if (a.chunk > 0 && keys > a.chunk) keys = a.chunk;
-        int n_split = (keys + 255) / 256;
+        const bool group = dtype == UMBS_BF16 && group_fits(a);
         const int rows = batch->n_seqs * heads;
-        n_split = n_split < 1 ? 1 : (n_split > 32 ? 32 : n_split);
-        if (n_split > (296 + rows - 1) / rows) n_split = (296 + rows - 1) / rows;
+        int n_split = 1;
+        if (group) {
+            // heads that share a key/value head in one block, three blocks on an SM, 128 keys a round of its warps: the split with
+            // the fewest rounds from first to last block, one more per block for its start and end
+            const int64_t blocks = (int64_t)batch->n_seqs * group_blocks(a);
+            int64_t best = INT64_MAX;
+            for (int n = 1; n <= 32 && (n == 1 || (n - 1) * 128 < keys); ++n) {
+                const int64_t cost = (blocks * n + 443) / 444 * ((keys + n * 128 - 1) / (n * 128) + 1) + (n > 1);
+                if (cost < best) { best = cost; n_split = n; }
+            }
+        } else {
+            n_split = (keys + 255) / 256;
+            n_split = n_split < 1 ? 1 : (n_split > 32 ? 32 : n_split);
+            if (n_split > (296 + rows - 1) / rows) n_split = (296 + rows - 1) / rows;
+        }
         const size_t per_split = (size_t)rows * (vdim + 2) * sizeof(float);
         if (split_scratch == nullptr || per_split == 0) n_split = 1;
         else if ((size_t)n_split * per_split > split_bytes) n_split = (int)(split_bytes / per_split);
         if (n_split < 1) n_split = 1;
-        if (dtype == UMBS_BF16) rc = launch_decode_any<__nv_bfloat16>(mode, a, *batch, n_split, split_scratch, st);
+        if (group) rc = launch_group_any(mode, a, *batch, n_split, split_scratch, st);
+        else if (dtype == UMBS_BF16) rc = launch_decode_any<__nv_bfloat16>(mode, a, *batch, n_split, split_scratch, st);
         else if (dtype == UMBS_F32) rc = launch_decode_any<float>(mode, a, *batch, n_split, split_scratch, st);
         else return UMB_ERR_ARG;
         if (rc) return rc;

@@ -543,23 +543,22 @@ __global__ void kv_pool_kernel(const T* __restrict__ kv, const T* __restrict__ k
     const int j0 = blk * pool;
     const T* step = kv + ((int64_t)start - pos0) * row + c;      // row j of the step's own rows at step + j row
     const T* ring = kv_cache + (int64_t)slot * kv_len * row + c;
-    int at = j0 % kv_len;                                        // row j0 + j of the ring
+    const int at = j0 % kv_len;                                  // row j0 + j of the ring: at + j, less its length behind its end
+    auto place = [&](int j) -> const T* {
+        const int r = at + j;
+        return j0 + j >= pos0 ? step + (int64_t)(j0 + j) * row : ring + (int64_t)(r >= kv_len ? r - kv_len : r) * row;
+    };
     float acc = 0.f;
     constexpr int U = 16;
-    for (int j = 0; j < pool; j += U) {
-        float x[U];
+    int j = 0;
+    for (; j + U <= pool; j += U) {
+        T x[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (j + u < pool) {
-                const int p = j0 + j + u;
-                x[u] = to_f32(p >= pos0 ? step[(int64_t)p * row] : ring[(int64_t)at * row]);
-                at = at + 1 == kv_len ? 0 : at + 1;
-            }
-        }
+        for (int u = 0; u < U; ++u) x[u] = *place(j + u);
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (j + u < pool) acc += x[u];
+        for (int u = 0; u < U; ++u) acc += to_f32(x[u]);
     }
+    for (; j < pool; ++j) acc += to_f32(*place(j));
     pool_cache[((int64_t)slot * pool_len + blk) * row + c] = from_f32<T>(acc / (float)pool);
 }
 
