@@ -1,0 +1,71 @@
+"""Recurrences taken 32 tokens at a time (csrc/seq/seq_chunk.cu; steps whose longest sequence has 64 tokens or more) against
+the walk token by token: the same sequences fed in steps of fewer than 64 tokens.
+
+Tolerance: both add the same fp32 products in another order, over sums that the decays keep to some hundreds of terms; random
+signs give about sqrt(500) 2^-24 = 1.3e-6 of a row's norm, 1e-5 leaves room for rows that nearly cancel."""
+import pytest
+import torch
+
+import seq_helpers as H
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+LENS = [(64,), (65, 1), (95, 200, 31), (500,), (129, 128, 127)]
+
+
+def _feed(fn, lens, size, x):
+    """The sequences' tokens (rows of x, one sequence after the other) in steps of at most `size` per sequence; -> rows in x's order."""
+    from umbrella_b200 import ops_seq as K
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    out, at = [None] * len(lens), [0] * len(lens)
+    while any(a < n for a, n in zip(at, lens)):
+        desc, rows = [], []
+        for s, n in enumerate(lens):
+            m = min(size, n - at[s])
+            if m:
+                desc.append((s, m, at[s], 0))
+                rows.append(torch.arange(starts[s] + at[s], starts[s] + at[s] + m))
+        idx = torch.cat(rows)
+        y, o = fn(x[idx.to(DEV)].contiguous(), K.RaggedBatch(desc, DEV)), 0
+        for s, m, _, _ in desc:
+            out[s] = y[o:o + m] if out[s] is None else torch.cat([out[s], y[o:o + m]])
+            o += m
+            at[s] += m
+    return torch.cat(out)
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("dim,vdim,rot", [(64, 128, 64), (32, 64, 12), (4, 4, 0), (60, 132, 60)])
+def test_retention(lens, dim, vdim, rot):
+    from umbrella_b200 import ops_seq as K
+    heads = 3
+    g = torch.Generator().manual_seed(sum(lens) + dim)
+    x = torch.randn(sum(lens), 2 * heads * (dim + vdim), generator=g).to(DEV)
+    decay = torch.tensor([0.97, 0.999, 0.5], device=DEV)
+    freq = (1e4 ** (-torch.arange(0, max(rot, 2), 2) / max(rot, 2))).float().to(DEV)
+    got = []
+    for size in (40, 10 ** 6, 70):
+        state = torch.full((len(lens), heads, dim, vdim), 3.0, device=DEV)           # dirty: a fresh sequence must not read it
+        y = _feed(lambda r, b: K.retention(r, b, heads, dim, vdim, rot, freq, decay, 1e-6, state), lens, size, x)
+        got.append((y, state.clone()))
+    for y, state in got[1:]:
+        assert H.rel_err(y, got[0][0]) < 1e-5 and H.rel_err(state, got[0][1]) < 1e-5
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("dim,vdim", [(64, 128), (32, 64), (4, 4), (60, 132)])
+def test_mlstm(lens, dim, vdim):
+    from umbrella_b200 import ops_seq as K
+    heads = 2
+    g = torch.Generator().manual_seed(sum(lens) + dim)
+    x = torch.randn(sum(lens), 2 * heads * dim + 2 * heads * vdim + 2 * heads, generator=g)
+    x[:, -2 * heads:] *= 4                                # gates that open and shut
+    x, bias = x.to(DEV), torch.tensor([0.0, -2.0, 3.0, 1.0], device=DEV)
+    norm = torch.ones(heads * vdim, device=DEV)
+    got = []
+    for size in (40, 10 ** 6, 70):
+        state = torch.full((len(lens), heads, dim * (vdim + 1) + 1), 3.0, device=DEV)
+        y = _feed(lambda r, b: K.mlstm(r, bias, b, heads, dim, vdim, 15.0, 1e-6, norm, state), lens, size, x)
+        got.append((y, state.clone()))
+    for y, state in got[1:]:
+        assert H.rel_err(y, got[0][0]) < 1e-5 and H.rel_err(state, got[0][1]) < 1e-5

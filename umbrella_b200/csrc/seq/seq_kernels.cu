@@ -9,7 +9,7 @@
 #include <type_traits>
 #include <stdint.h>
 
-#include "seq_internal.h"
+#include "seq_chunk.h"
 
 namespace umbs {
 
@@ -1056,10 +1056,14 @@ extern "C" int umbs_retention_ex(int dtype, const float* qkvg, int64_t ld, const
     // passes (local end states from zero, chained into start states, then the outputs).  Twice the arithmetic of the
     // recurrence for n_seg times the blocks; the result differs from the single walk by fp32 rounding only.
     int n_seg = 1, seg_len = batch->max_seq_len;
+    const size_t fit = seg_scratch != nullptr ? seg_bytes / ((size_t)batch->n_seqs * heads * dim * vdim * sizeof(float)) : 0;
+    // Steps with long sequences take their tokens 32 at a time (seq_chunk.cu); a chunk costs what the walk takes for about 40.
+    const bool chunks = batch->max_seq_len >= 64 && chunk_memory_fits(dim, vdim);
     const int base_blocks = batch->n_seqs * heads * ((vdim + 31) / 32);
-    if (seg_scratch != nullptr && base_blocks <= 148 && batch->max_seq_len >= 128) {     // less than a block per SM
+    if (chunks) {
+        n_seg = chunk_segments(chunk_base_blocks(batch->n_seqs, heads, vdim), batch->max_seq_len, fit, &seg_len);
+    } else if (seg_scratch != nullptr && base_blocks <= 148 && batch->max_seq_len >= 128) {     // less than a block per SM
         int want = std::min((592 + base_blocks - 1) / base_blocks, batch->max_seq_len / 64);
-        const size_t fit = seg_bytes / ((size_t)batch->n_seqs * heads * dim * vdim * sizeof(float));
         want = (int)std::min<size_t>(want, fit);
         if (want >= 2) {
             seg_len = ((batch->max_seq_len + want - 1) / want + 15) & ~15;
@@ -1067,6 +1071,11 @@ extern "C" int umbs_retention_ex(int dtype, const float* qkvg, int64_t ld, const
         }
     }
     auto run = [&](int pass) -> int {
+        if (chunks) {
+            ChunkMemory m{qkvg, ld, 0, heads * dim, 2 * heads * dim, heads, dim, vdim, 1.f, kscale, rot_dims, rot_tab, decay, nullptr, 0,
+                          state, (int64_t)dim * vdim, o_scratch, seg_len, n_seg, pass, seg_scratch, nullptr};
+            return launch_chunk_memory(m, *batch, st);
+        }
         if (dim <= 32) return launch_retention<8, 16>(qkvg, ld, *batch, heads, dim, vdim, rot_dims, rot_tab, inv_freq, decay, state, o_scratch, kscale, seg_len, n_seg, pass, seg_scratch, st);
         if (dim <= 128) return launch_retention<16, 16>(qkvg, ld, *batch, heads, dim, vdim, rot_dims, rot_tab, inv_freq, decay, state, o_scratch, kscale, seg_len, n_seg, pass, seg_scratch, st);
         if (dim <= 512) return launch_retention<32, 8>(qkvg, ld, *batch, heads, dim, vdim, rot_dims, rot_tab, inv_freq, decay, state, o_scratch, kscale, seg_len, n_seg, pass, seg_scratch, st);

@@ -14,7 +14,7 @@
 #include <algorithm>
 #include <stdint.h>
 
-#include "seq_internal.h"
+#include "seq_chunk.h"
 
 namespace umbs {
 
@@ -277,7 +277,10 @@ extern "C" int umbs_mlstm(int dtype, const float* proj, int64_t ld, const float*
     const int base_blocks = batch->n_seqs * heads * ((V1 + 31) / 32);
     const size_t per_seg = (size_t)batch->n_seqs * heads * ((size_t)dim * V1 + 1) * sizeof(float);      // states + decay products
     // about four blocks per SM run side by side; two passes pay from three segments on (2 / n_seg of the single walk)
-    if (seg_scratch != nullptr && base_blocks * 3 <= 592 && batch->max_seq_len >= 192) {
+    const bool chunks = batch->max_seq_len >= 64 && chunk_memory_fits(dim, vdim);       // 32 tokens at a time: seq_chunk.cu
+    if (chunks) {
+        n_seg = chunk_segments(chunk_base_blocks(batch->n_seqs, heads, vdim), batch->max_seq_len, seg_scratch != nullptr ? seg_bytes / per_seg : 0, &seg_len);
+    } else if (seg_scratch != nullptr && base_blocks * 3 <= 592 && batch->max_seq_len >= 192) {
         int want = std::min(592 / base_blocks, batch->max_seq_len / 64);
         want = (int)std::min<size_t>(want, seg_bytes / per_seg);
         if (want >= 3) {
@@ -287,6 +290,11 @@ extern "C" int umbs_mlstm(int dtype, const float* proj, int64_t ld, const float*
     }
     float* seg_decay = n_seg > 1 ? seg_scratch + (size_t)batch->n_seqs * n_seg * heads * dim * V1 : nullptr;
     auto run = [&](int pass) -> int {
+        if (chunks) {
+            ChunkMemory m{proj, ld, 0, heads * dim, 2 * heads * dim, heads, dim, vdim, 1.f / sqrtf((float)dim), 1.f, 0, nullptr, nullptr, gates_scratch, 1,
+                          state, stride, o_scratch, seg_len, n_seg, pass, seg_scratch, seg_decay};
+            return launch_chunk_memory(m, *batch, st);
+        }
         if (dim <= 32) return launch_mlstm<8, 16>(proj, ld, *batch, heads, dim, vdim, gates_scratch, state, stride, o_scratch, seg_len, n_seg, pass, seg_scratch, seg_decay, st);
         if (dim <= 128) return launch_mlstm<16, 16>(proj, ld, *batch, heads, dim, vdim, gates_scratch, state, stride, o_scratch, seg_len, n_seg, pass, seg_scratch, seg_decay, st);
         if (dim <= 512) return launch_mlstm<32, 8>(proj, ld, *batch, heads, dim, vdim, gates_scratch, state, stride, o_scratch, seg_len, n_seg, pass, seg_scratch, seg_decay, st);
