@@ -88,3 +88,17 @@ def test_rows_sorted_by_expert(ops, sizes, K):
         assert H.rel_err(y[at:at + m], (g * torch.sigmoid(1.702 * g) * (u + 1)).cpu()) < BF16_TOL
         assert H.rel_err(o[at:at + m], (y[at:at + m].double() @ down[e].double().T).cpu()) < F32_TOL
         at += m
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 5), (63, 65, 17), (64, 64, 16), (65, 130, 100), (200, 31, 1000)])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_true_32_bit_tiles(ops, M, N, K, dt):
+    """The fp32 kernel (and what no tensor-core tile takes: K not a multiple of 32) at the edges of its 64 x 64 x 16 tiles, rows that no
+    16-byte load may take, gated pairs."""
+    g = torch.Generator().manual_seed(M)
+    a, w = torch.randn(M, K + 1, generator=g).to(dt).to(DEV)[:, 1:], torch.randn(2 * N, K, generator=g).to(dt).to(DEV)
+    z = a.double() @ w.double().T
+    assert H.rel_err(ops.gemm(a, w, out_f32=True), z.cpu()) < 2e-6                        # sqrt(1000) 2^-24
+    got = ops.gemm(a, w, n=N, dual=True, limit=7.0, out_f32=True)
+    gate, up = z[:, :N].clamp(max=7.0), z[:, N:].clamp(-7.0, 7.0)
+    assert H.rel_err(got, (gate * torch.sigmoid(1.702 * gate) * (up + 1)).cpu()) < 4e-6   # a product of two such sums

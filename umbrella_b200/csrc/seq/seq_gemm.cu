@@ -19,68 +19,122 @@
 namespace umbs {
 
 // ------------------------------------------------------------------------------------------------ SIMT
-constexpr int BM = 64, BN = 64, BK = 16;
+// 64 x 64 outputs per block of 64 threads, 8 x 8 a thread (with DUAL: 8 rows x 4 gate and the same 4 up columns), k in steps of
+// 16 through two shared-memory stages, the next step's numbers on their way in registers.  Per k a thread reads four 16-byte
+// pieces for 64 multiply-adds, two of them an instruction; an output is one chain of additions over k, so it has the same bits
+// in every tiling.  Bound: fp32 multiply-adds.  Blocks are small so that a step of some hundred rows spreads evenly: 777 x 1024
+// -> 3088 are 637 of them.  16 x 16 threads with 4 x 4 outputs and 4-byte loads took 257 us for it (19 TFLOP/s), this
+// takes 178.
+constexpr int BM = 64, BN = 64, BK = 16, BP = BM + 4;
+
+template <typename T> __device__ __forceinline__ void load_k4(const T* p, int left, bool vec, float (&f)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) f[i] = i < left ? to_f32(p[i]) : 0.f;
+}
+template <> __device__ __forceinline__ void load_k4<float>(const float* p, int left, bool vec, float (&f)[4]) {
+    if (vec && left >= 4) {
+        const float4 v = *reinterpret_cast<const float4*>(p);
+        f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) f[i] = i < left ? p[i] : 0.f;
+    }
+}
 
 template <typename TA, typename TC, bool DUAL>
-__global__ void __launch_bounds__(256) gemm_simt_kernel(GemmArgs a) {
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Ws[DUAL ? 2 : 1][BK][BN + 4];
+__global__ void __launch_bounds__(64) gemm_simt_kernel(GemmArgs a, int vec, int vec_c) {
+    __shared__ __align__(16) float As[2][BK][BP], Ws[2][BK][BP];
     const int g = blockIdx.z;
     int row_lo = 0, rows = a.M;
     if (a.grp_off != nullptr) { row_lo = a.grp_off[g]; rows = a.grp_off[g + 1] - row_lo; }
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    constexpr int OUT = DUAL ? BN / 2 : BN;                 // output columns of a block
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * OUT;
     if (m0 >= rows) return;
     const TA* A = (const TA*)a.A + (int64_t)g * a.a_goff;
     const TA* W = (const TA*)a.W + (int64_t)g * a.w_gstride;
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    // loader mapping: 256 threads x 4 elements = a 64 x 16 tile; thread -> (row = tid / 4, k = (tid % 4) * 4 ..)
+    const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
+    // loader: a thread takes four k of rows lr, lr + 16, lr + 32, lr + 48 of both tiles
     const int lr = tid >> 2, lk = (tid & 3) * 4;
-    int64_t a_row = -1;
-    if (m0 + lr < rows) {
-        const int p = row_lo + m0 + lr;
-        a_row = a.row_src ? a.row_src[p] : p;
+    const TA *ap[4], *wp[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = lr + 16 * i;
+        ap[i] = wp[i] = nullptr;
+        if (m0 + r < rows) {
+            const int p = row_lo + m0 + r;
+            ap[i] = A + (int64_t)(a.row_src ? a.row_src[p] : p) * a.lda + lk;
+        }
+        const int n = n0 + (DUAL ? r % OUT : r);            // (DUAL: 32 gate rows, then the 32 up rows)
+        if (n < a.N) wp[i] = W + (int64_t)(DUAL && r >= OUT ? a.N + n : n) * a.ldw + lk;
     }
-    const int wn = n0 + lr;
-    float acc[4][4] = {}, acc2[DUAL ? 4 : 1][4] = {};
-    for (int k0 = 0; k0 < a.K; k0 += BK) {
+    float ra[4][4], rw[4][4];
+    auto fetch = [&](int k0) {
+        const int left = a.K - k0 - lk;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int k = k0 + lk + i;
-            As[lk + i][lr] = (a_row >= 0 && k < a.K) ? to_f32(A[a_row * a.lda + k]) : 0.f;
-            Ws[0][lk + i][lr] = (wn < a.N && k < a.K) ? to_f32(W[(int64_t)wn * a.ldw + k]) : 0.f;
-            if (DUAL) Ws[DUAL ? 1 : 0][lk + i][lr] = (wn < a.N && k < a.K) ? to_f32(W[(int64_t)(a.N + wn) * a.ldw + k]) : 0.f;
+            load_k4<TA>(ap[i] + k0, ap[i] != nullptr ? left : 0, vec, ra[i]);
+            load_k4<TA>(wp[i] + k0, wp[i] != nullptr ? left : 0, vec, rw[i]);
         }
-        __syncthreads();
+    };
+    auto stash = [&](int st) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                As[st][lk + e][lr + 16 * i] = ra[i][e];
+                Ws[st][lk + e][lr + 16 * i] = rw[i][e];
+            }
+    };
+    f32x2 acc[8][4] = {};                                   // rows ty 4 .. + 3 and 32 + ty 4 ..; columns tx 4 .. + 3 and 32 + tx 4 .., in pairs
+    fetch(0);
+    stash(0);
+    __syncthreads();
+    int st = 0;
+    for (int k0 = 0; k0 < a.K; k0 += BK, st ^= 1) {
+        const bool more = k0 + BK < a.K;
+        if (more) fetch(k0 + BK);
 #pragma unroll
         for (int k = 0; k < BK; ++k) {
-            float av[4], wv[4], wv2[4];
+            const float4 a0 = *reinterpret_cast<const float4*>(&As[st][k][ty * 4]), a1 = *reinterpret_cast<const float4*>(&As[st][k][32 + ty * 4]);
+            const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(&Ws[st][k][tx * 4]), w1 = *reinterpret_cast<const ulonglong2*>(&Ws[st][k][32 + tx * 4]);
+            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { av[i] = As[k][ty * 4 + i]; wv[i] = Ws[0][k][tx * 4 + i]; }
-            if (DUAL) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) wv2[i] = Ws[DUAL ? 1 : 0][k][tx * 4 + i];
+            for (int i = 0; i < 8; ++i) {
+                const f32x2 aa = pack2(av[i], av[i]);
+                acc[i][0] = fma2(aa, w0.x, acc[i][0]);
+                acc[i][1] = fma2(aa, w0.y, acc[i][1]);
+                acc[i][2] = fma2(aa, w1.x, acc[i][2]);
+                acc[i][3] = fma2(aa, w1.y, acc[i][3]);
             }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
-                    if (DUAL) acc2[DUAL ? i : 0][j] = fmaf(av[i], wv2[j], acc2[DUAL ? i : 0][j]);
-                }
         }
-        __syncthreads();
+        if (more) {
+            stash(st ^ 1);                                  // the other stage was last read in front of the barrier before
+            __syncthreads();
+        }
     }
     TC* C = (TC*)a.C + (int64_t)g * a.c_goff;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + ty * 4 + i;
+    for (int i = 0; i < 8; ++i) {
+        const int m = m0 + (i >> 2) * 32 + ty * 4 + (i & 3);
         if (m >= rows) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx * 4 + j;
+        for (int half = 0; half < (DUAL ? 1 : 2); ++half) {
+            const int n = n0 + half * 32 + tx * 4;
             if (n >= a.N) continue;
-            const float v = finish<DUAL>(a, acc[i][j], acc2[DUAL ? i : 0][j], g, row_lo + m, n);
-            C[(int64_t)(row_lo + m) * a.ldc + n] = from_f32<TC>(v);
+            const float2 u0 = unpack2(acc[i][half * 2]), u1 = unpack2(acc[i][half * 2 + 1]), p0 = unpack2(acc[i][2]), p1 = unpack2(acc[i][3]);
+            const float s1[4] = {u0.x, u0.y, u1.x, u1.y}, s2[4] = {p0.x, p0.y, p1.x, p1.y};
+            float v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (n + e < a.N) v[e] = finish<DUAL>(a, s1[e], DUAL ? s2[e] : 0.f, g, row_lo + m, n + e);
+            TC* out = C + (int64_t)(row_lo + m) * a.ldc + n;
+            if (sizeof(TC) == 4 && vec_c && n + 4 <= a.N) {
+                *reinterpret_cast<float4*>(out) = make_float4(v[0], v[1], v[2], v[3]);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (n + e < a.N) out[e] = from_f32<TC>(v[e]);
+            }
         }
     }
 }
@@ -224,9 +278,12 @@ static void launch_skinny(const GemmArgs& a, int groups, bool dual, cudaStream_t
 
 template <typename TA, typename TC>
 static void launch_simt(const GemmArgs& a, int groups, bool dual, cudaStream_t st) {
-    const dim3 grid((a.N + BN - 1) / BN, (a.M + BM - 1) / BM, groups);
-    if (dual) gemm_simt_kernel<TA, TC, true><<<grid, 256, 0, st>>>(a);
-    else gemm_simt_kernel<TA, TC, false><<<grid, 256, 0, st>>>(a);
+    const int out = dual ? BN / 2 : BN;
+    const dim3 grid((a.N + out - 1) / out, (a.M + BM - 1) / BM, groups);
+    const bool vec = a.lda % 4 == 0 && a.ldw % 4 == 0 && a.a_goff % 4 == 0 && a.w_gstride % 4 == 0 && (((uintptr_t)a.A | (uintptr_t)a.W) & 15) == 0;
+    const bool vec_c = a.ldc % 4 == 0 && a.c_goff % 4 == 0 && ((uintptr_t)a.C & 15) == 0;
+    if (dual) gemm_simt_kernel<TA, TC, true><<<grid, 64, 0, st>>>(a, vec, vec_c);
+    else gemm_simt_kernel<TA, TC, false><<<grid, 64, 0, st>>>(a, vec, vec_c);
 }
 
 }  // namespace umbs
