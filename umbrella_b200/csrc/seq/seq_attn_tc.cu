@@ -2,28 +2,32 @@
 // seq_cached_attn.cu and seq_window_attn.cu for the sizes and addresses it takes.
 //
 // A block = 128 consecutive query rows of one (sequence, virtual head) = the 128 lanes of tensor memory; two blocks share an
-// SM, so that one multiplies while the other works its weights out.  Per tile of 64 keys:
-//   warps 9-10 copy key and value rows with 16-byte cp.async, each from where it lives (step, ring, block table), into the
-//              128-byte-swizzled images the tensor core reads, a tile ahead where two fit;
-//   warp 8     one thread issues S = Q K^T and O += P V, accumulators in tensor memory;
-//   warps 0-7  two threads per row, 32 keys each: scores to weights in fp32 in the base-2 domain, an online reference that
-//              only moves when a score passes it by 2^8 (then the pair agrees on it and O is rescaled), the row's sum.
+// SM.  Tiles of 32 keys run through three stages that overlap:
+//   warps 5-6  bring key and value rows into the 128-byte-swizzled images the tensor core reads, several tiles ahead: with TMA
+//              where the 32 rows are neighbours in the step and heads are whole pieces of 64 numbers, else with 16-byte
+//              cp.async, each row from where it lives (step, ring, block table), zeros where there is none;
+//   warp 4     one thread issues S = Q K^T of the next tile, then O += P V of this one, accumulators in tensor memory;
+//   warps 0-3  a thread per row: scores to weights in fp32 in the base-2 domain, an online reference that only moves when a
+//              score passes it by 2^8 (then O is rescaled), the row's sum.
 // Weights stay 32-bit: an fp32 weight is the sum of three bf16 numbers (8 + 8 + 8 significant bits, cut off one after the
 // other, so exactly), and P V is three products against the same values.  Products of bf16 operands are exact in the tensor
 // core and its sums are fp32.
 //
-// Tensor memory, 256 columns: scores 0-63, weights' parts lo 32-63 (over scores that have been read), hi 64-95, mid 96-127,
-// output 128-255.
+// Tensor memory, 256 columns: two score tiles 0-31 and 32-63, the weights' parts 64-79, 80-95, 96-111, output 128-255.  With
+// 64 keys to a tile only one score tile fits beside the output of 128 columns, and scores, weights and output products take
+// turns: 5800 clocks per 64 keys and block, of which the tensor core works 1160 (measured with clock64 stamps; 128 x 64 x 16
+// takes it 48 clocks, 128 x 128 x 16 takes 64).
 #include "seq_attn.h"
 #include "seq_tc.cuh"
 
 namespace umbs {
 
-constexpr int kTaQ = 128, kTaK = 64;
-constexpr int kTaThreads = 352;                             // 8 warps of weights, 1 of products, 2 of copies
+constexpr int kTaQ = 128, kTaK = 32;
+constexpr int kTaThreads = 224;                             // 4 warps of weights, 1 of products, 2 of copies
+constexpr int kTaStages = 4;                                // key and value tiles held, at most
 constexpr float kTaLazy = 8.f;                              // how far (in powers of two) a score may pass the reference
 
-struct TaDims { int q_atoms, k_steps, v_atoms, nk, nv; };   // 64-wide pieces of a query row, 16-wide k steps, 64-wide pieces of a value row; tiles held
+struct TaDims { int q_atoms, k_steps, v_atoms, stages, tma; };   // 64-wide pieces of a query row, 16-wide k steps, 64-wide pieces of a value row; tiles held
 
 __device__ __forceinline__ float ex2(float x) {
     float y;
@@ -53,19 +57,15 @@ struct KeyTiles {
     __device__ int last(int i) const { return i < tiles_pool ? n_pool - 1 : p_hi; }
 };
 
-#define UMBS_TMEM_ST_X8(taddr, r)                                                                            \
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"                      \
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory")
-
 template <int MODE, bool SHAPED, bool STEP>
-__global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const CachedAttnArgs a, const StepKeys x, const Batch b, const TaDims z) {
+__global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_s, const __grid_constant__ CUtensorMap map_v,
+                                                                        const CachedAttnArgs a, const StepKeys x, const Batch b, const TaDims z) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ uint64_t bars[11];
+    __shared__ uint64_t bars[4 * kTaStages + 4];
     __shared__ uint32_t s_tmem;
     __shared__ int s_quit;
-    __shared__ float s_pair[2][kTaQ];
-    __shared__ int s_move[2][8];                            // per tile parity and warp: a row of it wants its reference moved
-    uint64_t *k_full = bars, *v_full = bars + 2, *k_empty = bars + 4, *v_empty = bars + 6, *s_full = bars + 8, *p_full = bars + 9, *o_full = bars + 10;
+    uint64_t *k_full = bars, *v_full = bars + kTaStages, *k_empty = bars + 2 * kTaStages, *v_empty = bars + 3 * kTaStages,
+             *s_full = bars + 4 * kTaStages, *p_full = s_full + 2, *o_full = s_full + 3;
     volatile int* quit = &s_quit;
     const int s = blockIdx.z, vh = blockIdx.y, q0 = (int)(gridDim.x - 1 - blockIdx.x) * kTaQ;     // the rows that see most start first
     const int len = b.seq_len[s], start = b.seq_start[s], pos0 = STEP ? 0 : b.seq_pos0[s], slot = STEP ? 0 : b.seq_slot[s];
@@ -78,23 +78,24 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const Cache
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k_bytes = z.q_atoms * (kTaK * 128), v_bytes = z.v_atoms * (kTaK * 128);
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    unsigned char* s_k = smem + z.q_atoms * (kTaQ * 128);   // Q [q_atoms][128 rows][128 B], nk K [q_atoms][64][128 B], nv V [v_atoms][64][128 B]
-    unsigned char* s_v = s_k + z.nk * k_bytes;
+    unsigned char* s_k = smem + z.q_atoms * (kTaQ * 128);   // Q [q_atoms][128 rows][128 B], stages of K [q_atoms][32][128 B], of V [v_atoms][32][128 B]
+    unsigned char* s_v = s_k + z.stages * k_bytes;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < kTaStages; ++i) {
             umb::mbar_init(k_full + i, 2);
             umb::mbar_init(v_full + i, 2);
             umb::mbar_init(k_empty + i, 1);
             umb::mbar_init(v_empty + i, 1);
         }
         umb::mbar_init(s_full, 1);
-        umb::mbar_init(p_full, 8);
+        umb::mbar_init(s_full + 1, 1);
+        umb::mbar_init(p_full, 4);
         umb::mbar_init(o_full, 1);
         s_quit = 0;
         umb::fence_barrier_init();
     }
-    if (warp == 8) {
+    if (warp == 4) {
         umb::tmem_alloc(&s_tmem, 256);
         umb::tmem_relinquish();
     }
@@ -103,9 +104,9 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const Cache
     umb::tc_fence_after();
     const uint32_t tmem = s_tmem;
 
-    if (warp > 8) {
+    if (warp > 4) {
         // ------------------------------------------------------------------------------------ copies: 8 threads per 128-byte row piece
-        const int tid = threadIdx.x - 288, ch = tid & 7, r0 = tid >> 3;
+        const int tid = threadIdx.x - 160, ch = tid & 7, r0 = tid >> 3, stages = z.stages;
         const uint32_t sw = (uint32_t)((ch ^ (r0 & 7)) << 4);               // r0 + 8 p keeps r0's place inside its group of eight rows
         const __nv_bfloat16* q = (const __nv_bfloat16*)(STEP ? x.q : a.q);
         const int64_t ldq = STEP ? x.ldq : vhd.qstride;
@@ -119,17 +120,55 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const Cache
                 cp16(smem_u32(smem) + at * (kTaQ * 128) + r * 128 + sw, in ? q + (int64_t)(start + q0 + r) * ldq + vhd.qoff + d : q, in ? 16 : 0);
             }
         }
-        auto publish = [&](uint64_t* bar) {
+        // A tile's copies are published when the tile behind it has been asked for: two are in flight.  (Publishing waits for the
+        // stage of that next tile, which is free long before: there are three stages or four.)
+        auto publish = [&](int i) {
             umb::fence_proxy_async_smem();                  // this thread's copies are complete: show them to the tensor core
             __syncwarp();
-            if (lane == 0) umb::mbar_arrive(bar);
+            if (lane == 0) {
+                umb::mbar_arrive(k_full + i % stages);
+                umb::mbar_arrive(v_full + i % stages);
+            }
         };
-        for (int i = 0; i < kt.n; ++i) {
-            const int base = kt.base(i), last = kt.last(i), ks = i % z.nk, vs = i % z.nv;
-            const __nv_bfloat16 *kp[8], *vp[8];             // this thread's rows: keys, values
+        int i = 0, pending = 0;                             // pending: the tile before has been asked for but not published
+        for (; i < kt.n; ++i) {
+            const int base = kt.base(i), last = kt.last(i), st = i % stages;
+            bool free = true;
+            if (i >= stages) free = tc_poll(k_empty + st, (i / stages - 1) & 1, quit) && tc_poll(v_empty + st, (i / stages - 1) & 1, quit);
+            if (!__all_sync(0xffffffffu, free)) break;
+            if (z.tma && !kt.pooled(i) && base >= pos0 && base + kTaK - 1 <= last) {
+                if (i == 0 || pending) {                    // (the queries come with the first tile)
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+                    if (pending) publish(i - 1);
+                    else umb::fence_proxy_async_smem();
+                    __syncwarp();
+                    pending = 0;
+                }
+                if (umb::elect_one()) {
+                    const int row = start + base - pos0;
+                    if (warp == 5) {
+                        umb::mbar_arrive_expect_tx(k_full + st, (uint32_t)k_bytes);
+                        for (int at = 0; at < z.q_atoms; ++at) {
+                            unsigned char* dst = s_k + st * k_bytes + at * (kTaK * 128);
+                            if (!STEP) tma_3d(dst, &map_k, vhd.koff + at * 64, row, 0, k_full + st);
+                            else if (at * 64 < x.kdim) tma_3d(dst, &map_k, vh * x.kdim + at * 64, row, 0, k_full + st);
+                            else tma_3d(dst, &map_s, at * 64 - x.kdim, row, 0, k_full + st);
+                        }
+                        umb::mbar_arrive(v_full + st);
+                    } else {
+                        umb::mbar_arrive_expect_tx(v_full + st, (uint32_t)v_bytes);
+                        for (int at = 0; at < z.v_atoms; ++at)
+                            tma_3d(s_v + st * v_bytes + at * (kTaK * 128), &map_v, (STEP ? vh * a.vdim : vhd.voff) + at * 64, row, 0, v_full + st);
+                        umb::mbar_arrive(k_full + st);
+                    }
+                }
+                __syncwarp();
+                continue;
+            }
+            const __nv_bfloat16 *kp[4], *vp[4];             // this thread's rows: keys, values
             uint32_t in = 0;
 #pragma unroll
-            for (int p = 0; p < 8; ++p) {
+            for (int p = 0; p < 4; ++p) {
                 const int j = base + r0 + 8 * p;
                 const bool ok = j <= last;
                 in |= (uint32_t)ok << p;
@@ -147,98 +186,101 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const Cache
                     vp[p] = row + vhd.voff;
                 }
             }
-            if (i >= z.nk && !tc_poll(k_empty + ks, (i / z.nk - 1) & 1, quit)) break;
-            const uint32_t kd = smem_u32(s_k) + ks * k_bytes + r0 * 128 + sw, vd = smem_u32(s_v) + vs * v_bytes + r0 * 128 + sw;
+            const uint32_t kd = smem_u32(s_k) + st * k_bytes + r0 * 128 + sw, vd = smem_u32(s_v) + st * v_bytes + r0 * 128 + sw;
             for (int at = 0; at < z.q_atoms; ++at) {
                 const int d = at * 64 + ch * 8;
                 if (d >= z.k_steps * 16) continue;
                 const bool own = !STEP || d < x.kdim, dok = d < a.dim;      // (a part all heads share follows a head's own)
 #pragma unroll
-                for (int p = 0; p < 8; ++p) {
+                for (int p = 0; p < 4; ++p) {
                     const __nv_bfloat16* src = kp[p] + d;
                     if (STEP && !own) src = (const __nv_bfloat16*)x.ks + (int64_t)(start + ((in >> p & 1) ? base + r0 + 8 * p : base)) * x.ldks + (d - x.kdim);
-                    const bool ok = (in >> p & 1) && dok;
-                    cp16(kd + at * (kTaK * 128) + p * 1024, ok ? src : kp[p], ok ? 16 : 0);
+                    const bool go = (in >> p & 1) && dok;
+                    cp16(kd + at * (kTaK * 128) + p * 1024, go ? src : kp[p], go ? 16 : 0);
                 }
             }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            if (i >= z.nv && !tc_poll(v_empty + vs, (i / z.nv - 1) & 1, quit)) break;
             for (int at = 0; at < z.v_atoms; ++at) {
                 const int c = at * 64 + ch * 8;
 #pragma unroll
-                for (int p = 0; p < 8; ++p) {
-                    const bool ok = (in >> p & 1) && c < a.vdim;            // rows that no query sees: zeros, their weights are 0
-                    cp16(vd + at * (kTaK * 128) + p * 1024, ok ? vp[p] + c : vp[p], ok ? 16 : 0);
+                for (int p = 0; p < 4; ++p) {
+                    const bool go = (in >> p & 1) && c < a.vdim;            // rows that no query sees: zeros, their weights are 0
+                    cp16(vd + at * (kTaK * 128) + p * 1024, go ? vp[p] + c : vp[p], go ? 16 : 0);
                 }
             }
             asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 1;" ::: "memory");
-            publish(k_full + ks);
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-            publish(v_full + vs);
+            if (pending) publish(i - 1);
+            pending = 1;
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
-    } else if (warp == 8) {
+        if (i == kt.n && pending) publish(kt.n - 1);
+    } else if (warp == 4) {
         // ------------------------------------------------------------------------------------ products
-        if (lane == 0) {
-            const uint32_t idesc_s = tc_idesc(kTaQ, kTaK), idesc_o = tc_idesc(kTaQ, 64, true) + ((z.v_atoms - 1) * (64u >> 3) << 17);
-            const uint64_t qd = umb::umma_smem_desc_sw128(smem_u32(smem)), kd0 = umb::umma_smem_desc_sw128(smem_u32(s_k));
-            // values: keys down the rows, so the operand is MN-major; its 64-wide pieces are 8192 bytes apart, groups of eight keys 1024
-            const uint64_t vd0 = (umb::umma_smem_desc_sw128(smem_u32(s_v)) & ~((uint64_t)0x3fff << 16)) | ((uint64_t)(8192 >> 4) << 16);
-            for (int i = 0; i < kt.n; ++i) {
-                const int ks = i % z.nk, vs = i % z.nv;
-                if (!tc_spin(k_full + ks, (i / z.nk) & 1, quit)) break;
-                if (i > 0 && !tc_spin(o_full, (i - 1) & 1, quit)) break;    // the weights lie over the scores
-                umb::tc_fence_after();
-                const uint64_t kd = kd0 + ((ks * k_bytes) >> 4), vd = vd0 + ((vs * v_bytes) >> 4);
+        const uint32_t idesc_s = tc_idesc(kTaQ, kTaK), idesc_o = tc_idesc(kTaQ, 64, true) + ((z.v_atoms - 1) * (64u >> 3) << 17);
+        const uint64_t qd = umb::umma_smem_desc_sw128(smem_u32(smem)), kd0 = umb::umma_smem_desc_sw128(smem_u32(s_k));
+        // values: keys down the rows, so the operand is MN-major; its 64-wide pieces are 4096 bytes apart, groups of eight keys 1024
+        const uint64_t vd0 = (umb::umma_smem_desc_sw128(smem_u32(s_v)) & ~((uint64_t)0x3fff << 16)) | ((uint64_t)(kTaK * 128 >> 4) << 16);
+        auto scores = [&](int i) -> bool {                  // the tile's score columns were read two tiles ago, in front of weights already waited for
+            const int st = i % z.stages;
+            if (!tc_spin_warp(k_full + st, (i / z.stages) & 1, quit)) return false;
+            umb::tc_fence_after();
+            const uint64_t kd = kd0 + ((st * k_bytes) >> 4);
+            if (umb::elect_one()) {
                 for (int k = 0; k < z.k_steps; ++k)
-                    umb::umma_ss_f16(tmem, qd + (k >> 2) * (kTaQ * 128 >> 4) + (k & 3) * 2, kd + (k >> 2) * (kTaK * 128 >> 4) + (k & 3) * 2,
+                    umb::umma_ss_f16(tmem + (i & 1) * kTaK, qd + (k >> 2) * (kTaQ * 128 >> 4) + (k & 3) * 2, kd + (k >> 2) * (kTaK * 128 >> 4) + (k & 3) * 2,
                                      idesc_s, k ? 1u : 0u);
-                umb::umma_commit(s_full);
-                umb::umma_commit(k_empty + ks);
-                if (!tc_spin(v_full + vs, (i / z.nv) & 1, quit)) break;
-                if (!tc_spin(p_full, i & 1, quit)) break;
-                umb::tc_fence_after();
-                const uint32_t part[3] = {tmem + 64, tmem + 96, tmem + 32};
+                umb::umma_commit(s_full + (i & 1));
+                umb::umma_commit(k_empty + st);
+            }
+            __syncwarp();
+            return true;
+        };
+        bool ok = scores(0);
+        for (int i = 0; ok && i < kt.n; ++i) {
+            const int st = i % z.stages;
+            if (i + 1 < kt.n && !scores(i + 1)) break;
+            if (!tc_spin_warp(v_full + st, (i / z.stages) & 1, quit)) break;
+            if (!tc_spin_warp(p_full, i & 1, quit)) break;
+            umb::tc_fence_after();
+            const uint64_t vd = vd0 + ((st * v_bytes) >> 4);
+            if (umb::elect_one()) {
 #pragma unroll
                 for (int e = 0; e < 3; ++e)
 #pragma unroll
                     for (int k = 0; k < kTaK / 16; ++k)
-                        umb::umma_ts_f16(tmem + 128, part[e] + k * 8, vd + k * (2048 >> 4), idesc_o, (i | e | k) ? 1u : 0u);
+                        umb::umma_ts_f16(tmem + 128, tmem + 64 + e * 16 + k * 8, vd + k * (2048 >> 4), idesc_o, (i | e | k) ? 1u : 0u);
                 umb::umma_commit(o_full);
-                umb::umma_commit(v_empty + vs);
+                umb::umma_commit(v_empty + st);
             }
+            __syncwarp();
         }
     } else {
-        // ------------------------------------------------------------------------------------ weights: two threads per row
-        // (The two warps of a row meet at named barrier 1 + quarter, once per tile and once more when a reference moves.  Both
-        // walk every tile, also when a wait has given up, so they always meet.)
-        const int half = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane, pair_id = 1 + quarter;
-        const int r = q0 + row, rp = pos0 + r;                              // the row's place in the step and its position
-        const uint32_t t0 = tmem + ((uint32_t)(quarter * 32) << 16);
+        // ------------------------------------------------------------------------------------ weights: a thread per row
+        const int r = q0 + warp * 32 + lane, rp = pos0 + r;                 // the row's place in the step and its position
+        const uint32_t t0 = tmem + ((uint32_t)(warp * 32) << 16);
         constexpr float kLog2e = 1.4426950408889634f;
         const float c = SHAPED ? kLog2e : a.scale * kLog2e;
         const float hb = (MODE == UMBS_ATTN_SIGMOID && a.head_bias) ? a.head_bias[h] : 0.f;
         const float r1h = SHAPED && a.r1 ? a.r1[h] : 0.f, r2h = SHAPED && a.r1 ? a.r2[h] : 0.f;
         float m = MODE == UMBS_ATTN_SOFTMAX_SINK ? sink_score(a, h) * kLog2e : -INFINITY;      // the sink: a key of this score ...
-        float l = MODE == UMBS_ATTN_SOFTMAX_SINK && half == 0 ? 1.f : 0.f;                     // ... without a value
+        float l = MODE == UMBS_ATTN_SOFTMAX_SINK ? 1.f : 0.f;                                  // ... without a value
         const int tok_lo = max(rp - window + 1, a.chunk > 0 ? rp / a.chunk * a.chunk : 0);
         const int pool_hi = pooled_visible(rp, window, a.pool);
         bool ok = true;
         for (int i = 0; i < kt.n; ++i) {
-            const int base = kt.base(i) + half * 32;        // this thread's keys: base .. base + 31, of which [lo, hi) are visible to its row
+            const int base = kt.base(i);                    // keys base .. base + 31, of which [lo, hi) are visible to this row
             const int lo = kt.pooled(i) ? 0 : max(tok_lo - base, 0);
-            const int hi = r >= len ? 0 : min((kt.pooled(i) ? pool_hi : rp + 1) - base, 32);
-            const bool whole = __all_sync(0xffffffffu, lo == 0 && hi == 32);
-            ok = __all_sync(0xffffffffu, ok && tc_poll(s_full, i & 1, quit));
+            const int hi = r >= len ? 0 : min((kt.pooled(i) ? pool_hi : rp + 1) - base, kTaK);
+            const bool whole = __all_sync(0xffffffffu, lo == 0 && hi == kTaK);
+            if (!(ok = __all_sync(0xffffffffu, tc_spin(s_full + (i & 1), (i >> 1) & 1, quit)))) break;
             umb::tc_fence_after();
             uint32_t v[32];
-            UMB_TMEM_LD_X32(t0 + half * 32, v);
+            UMB_TMEM_LD_X32(t0 + (i & 1) * kTaK, v);
             umb::tc_wait_ld();
             if (SHAPED) {
 #pragma unroll
                 for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(shaped_score(a, __uint_as_float(v[j]), r1h, r2h, rp - (base + j)));
             }
-            float mx = -INFINITY;
+            bool waited = i == 0;                           // the weights' columns are free (the products of the tile before are done)
             if (MODE != UMBS_ATTN_SIGMOID) {
                 if (!whole) {
 #pragma unroll
@@ -248,36 +290,25 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const Cache
                 float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
                 for (int j = 0; j < 32; ++j) m4[j & 3] = fmaxf(m4[j & 3], __uint_as_float(v[j]) * c);
-                mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-                const bool want = __any_sync(0xffffffffu, i == 0 || mx > m + kTaLazy || (m == -INFINITY && mx > -INFINITY));
-                s_pair[half][row] = mx;
-                if (lane == 0) s_move[i & 1][warp] = want;
-            }
-            // behind this both warps have read their scores (the weights' last part goes over them)
-            __syncwarp();
-            umb::named_bar_sync(pair_id, 64);
-            if (MODE != UMBS_ATTN_SIGMOID) {
-                const float other = s_pair[half ^ 1][row];
-                const bool move = (s_move[i & 1][warp] | s_move[i & 1][warp ^ 4]) != 0;
-                __syncwarp();
-                umb::named_bar_sync(pair_id, 64);           // (s_pair may be written again)
-                if (move) {
-                    mx = fmaxf(mx, other);
-                    const float f = mx > m ? ex2(m - mx) : 1.f;
+                const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+                const bool move = mx > m + (i == 0 ? 0.f : kTaLazy) || (m == -INFINITY && mx > -INFINITY);
+                if (__any_sync(0xffffffffu, move)) {        // rare behind the first tiles: the reference of some row moves
+                    const float f = move ? ex2(m - mx) : 1.f;
+                    if (move) m = mx;
                     l *= f;                                 // (m = -inf: l is 0)
                     if (i > 0) {
-                        for (int c0 = half * 32; c0 < z.v_atoms * 64; c0 += 64) {
-                            for (int e = 0; e < 32; e += 16) {
-                                uint32_t o[16];
-                                UMB_TMEM_LD_X16(t0 + 128 + c0 + e, o);
-                                umb::tc_wait_ld();
+                        if (!(ok = __all_sync(0xffffffffu, tc_spin(o_full, (i - 1) & 1, quit)))) break;
+                        umb::tc_fence_after();
+                        waited = true;
+                        for (int c0 = 0; c0 < z.v_atoms * 64; c0 += 32) {
+                            uint32_t o[32];
+                            UMB_TMEM_LD_X32(t0 + 128 + c0, o);
+                            umb::tc_wait_ld();
 #pragma unroll
-                                for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
-                                UMB_TMEM_ST_X16(t0 + 128 + c0 + e, o);
-                            }
+                            for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
+                            UMB_TMEM_ST_X32(t0 + 128 + c0, o);
                         }
                     }
-                    m = fmaxf(m, mx);
                 }
             }
             const float ref = m == -INFINITY ? 0.f : m;
@@ -291,35 +322,33 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const Cache
                     if (j < lo || j >= hi) v[j] = 0u;
             }
             float l4[4] = {0.f, 0.f, 0.f, 0.f};
+            uint32_t ph[16], pm[16];
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                uint32_t ph[8], pm[8], pl[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const float p = __uint_as_float(v[e * 16 + 2 * j]), p1 = __uint_as_float(v[e * 16 + 2 * j + 1]);
-                    l4[(2 * j) & 3] += p;
-                    l4[(2 * j + 1) & 3] += p1;
-                    const float ra = p - cut(p), rb = p1 - cut(p1);
-                    ph[j] = hi_pair(p, p1);
-                    pm[j] = hi_pair(ra, rb);
-                    pl[j] = hi_pair(ra - cut(ra), rb - cut(rb));
-                }
-                UMBS_TMEM_ST_X8(t0 + 64 + half * 16 + e * 8, ph);
-                UMBS_TMEM_ST_X8(t0 + 96 + half * 16 + e * 8, pm);
-                UMBS_TMEM_ST_X8(t0 + 32 + half * 16 + e * 8, pl);
+            for (int j = 0; j < 16; ++j) {
+                const float p = __uint_as_float(v[2 * j]), p1 = __uint_as_float(v[2 * j + 1]);
+                l4[(2 * j) & 3] += p;
+                l4[(2 * j + 1) & 3] += p1;
+                const float ra = p - cut(p), rb = p1 - cut(p1);
+                ph[j] = hi_pair(p, p1);
+                pm[j] = hi_pair(ra, rb);
+                v[j] = hi_pair(ra - cut(ra), rb - cut(rb));                 // (v[2 j] and v[2 j + 1] have been used)
             }
             l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
+            if (!waited) {
+                if (!(ok = __all_sync(0xffffffffu, tc_spin(o_full, (i - 1) & 1, quit)))) break;
+                umb::tc_fence_after();
+            }
+            UMB_TMEM_ST_X16(t0 + 64, ph);
+            UMB_TMEM_ST_X16(t0 + 80, pm);
+            UMB_TMEM_ST_X16(t0 + 96, v);
             umb::tc_wait_st();
             umb::tc_fence_before();
             __syncwarp();
             if (lane == 0) umb::mbar_arrive(p_full);
         }
-        ok = __all_sync(0xffffffffu, ok && tc_poll(o_full, (kt.n - 1) & 1, quit));
-        umb::tc_fence_after();
-        s_pair[half][row] = l;
-        umb::named_bar_sync(pair_id, 64);
-        l += s_pair[half ^ 1][row];
+        if (ok) ok = __all_sync(0xffffffffu, tc_spin(o_full, (kt.n - 1) & 1, quit));
         if (ok) {
+            umb::tc_fence_after();
             const float inv = MODE == UMBS_ATTN_SIGMOID ? 1.f : 1.f / l;
             const int64_t t = start + r;
             const float* grow = a.gate ? a.gate + t * a.ldg + (a.gate_per_head ? h : h * a.vdim) : nullptr;
@@ -328,7 +357,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const Cache
             float* rrow = a.raw ? a.raw + (t * vhd.nv + vh) * a.vdim : nullptr;
             __nv_bfloat16* orow = STEP ? (__nv_bfloat16*)x.out + t * x.ldo + (int64_t)h * a.vdim
                                        : (__nv_bfloat16*)a.out + t * a.heads * a.vdim + (int64_t)h * a.vdim;
-            for (int c0 = half * 32; c0 < a.vdim; c0 += 64) {
+            for (int c0 = 0; c0 < a.vdim; c0 += 32) {
                 uint32_t v[32];
                 UMB_TMEM_LD_X32(t0 + 128 + c0, v);
                 umb::tc_wait_ld();
@@ -372,18 +401,17 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const Cache
     umb::tc_fence_before();
     __syncthreads();
     tc_settle(quit);
-    if (warp == 8) {
+    if (warp == 4) {
         umb::tc_fence_after();
         umb::tmem_dealloc(tmem, 256);
     }
 }
 
-// Two key tiles and two value tiles where two blocks of that size fit on an SM (228 KB, 1 KB of it per block the system's).
+// As many key and value tiles as leave room for a second block on the SM (228 KB, 1 KB of it per block the system's): four, or
+// three beside queries of more than 128 numbers.
 static TaDims ta_dims(const CachedAttnArgs& a) {
-    TaDims z{(a.dim + 63) / 64, (a.dim + 15) / 16, (a.vdim + 63) / 64, 2, 2};
-    const int room = 110 * 1024 - z.q_atoms * (kTaQ * 128), k = z.q_atoms * (kTaK * 128), v = z.v_atoms * (kTaK * 128);
-    if (2 * k + 2 * v > room) z.nk = 1;
-    if (k * z.nk + 2 * v > room) z.nv = 1;
+    TaDims z{(a.dim + 63) / 64, (a.dim + 15) / 16, (a.vdim + 63) / 64, kTaStages, 0};
+    while (z.stages > 3 && z.q_atoms * (kTaQ * 128) + z.stages * (z.q_atoms + z.v_atoms) * (kTaK * 128) > 110 * 1024) --z.stages;
     return z;
 }
 
@@ -400,12 +428,28 @@ bool attention_tc_fits(const CachedAttnArgs& a, const StepKeys* s) {
 
 template <int MODE, bool SHAPED, bool STEP>
 static int launch_ta(const CachedAttnArgs& a, const StepKeys& x, const Batch& b, cudaStream_t st) {
-    const TaDims z = ta_dims(a);
-    const int smem = 1024 + (z.q_atoms * (kTaQ + z.nk * kTaK) + z.nv * z.v_atoms * kTaK) * 128;
+    TaDims z = ta_dims(a);
+    // heads that are whole pieces of 64 numbers: the step's rows as tensor maps
+    CUtensorMap mk{}, ms{}, mv{};
+    z.tma = a.dim % 64 == 0 && a.vdim % 64 == 0 && (!STEP || x.kdim % 64 == 0);
+    if (z.tma) {
+        int rc;
+        if (STEP) {
+            rc = encode_map(&mk, x.k, (uint64_t)a.heads * x.kdim, b.n_tokens, 1, x.ldk, 0, kTaK);
+            if (rc == 0 && x.kdim < a.dim) rc = encode_map(&ms, x.ks, a.dim - x.kdim, b.n_tokens, 1, x.ldks, 0, kTaK);
+            if (rc == 0) rc = encode_map(&mv, x.v, (uint64_t)a.heads * a.vdim, b.n_tokens, 1, x.ldv, 0, kTaK);
+        } else {
+            const uint64_t row = (uint64_t)a.kv_heads * (a.maps * a.dim + a.vdim);
+            rc = encode_map(&mk, a.kv, row, b.n_tokens, 1, row, 0, kTaK);
+            mv = mk;
+        }
+        if (rc != 0) return rc;
+    }
+    const int smem = 1024 + (z.q_atoms * (kTaQ + z.stages * kTaK) + z.stages * z.v_atoms * kTaK) * 128;
     auto kernel = attention_tc_kernel<MODE, SHAPED, STEP>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
-    kernel<<<dim3((b.max_seq_len + kTaQ - 1) / kTaQ, a.heads * a.maps * a.vheads, b.n_seqs), kTaThreads, smem, st>>>(a, x, b, z);
+    kernel<<<dim3((b.max_seq_len + kTaQ - 1) / kTaQ, a.heads * a.maps * a.vheads, b.n_seqs), kTaThreads, smem, st>>>(mk, ms, mv, a, x, b, z);
     return 0;
 }
 

@@ -30,11 +30,6 @@ struct TcArgs {
     int a_grouped, w_grouped;                               // the group coordinate of the tensor maps is used
 };
 
-__device__ __forceinline__ void tma_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                 ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar)) : "memory");
-}
-
 // The tiles of a block, in the order every role visits them: rows fastest, then columns, then groups.
 struct TileWalk {
     const GemmArgs& a; const TcArgs& t;
@@ -150,43 +145,45 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     TileWalk w(a, t);
 
     if (warp == 0) {
-        if (lane == 0) {
-            uint32_t s = 0, ph = 1;
-            bool ok = true;
-            while (ok && w.step()) {
-                for (int k = 0; k < t.k_steps; ++k) {
-                    if (!(ok = tc_spin(empty + s, ph, quit))) break;
-                    unsigned char* st = smem + s * Cfg::kStage;
+        uint32_t s = 0, ph = 1;
+        bool ok = true;
+        while (ok && w.step()) {
+            const int gw = t.w_grouped ? w.g : 0, ga = t.a_grouped ? w.g : 0, n0 = w.n0 * kOut;
+            for (int k = 0; k < t.k_steps; ++k) {
+                if (!(ok = tc_spin_warp(empty + s, ph, quit))) break;
+                unsigned char* st = smem + s * Cfg::kStage;
+                if (umb::elect_one()) {
                     umb::mbar_arrive_expect_tx(full + s, (A_TMA ? Cfg::kABytes : 0) + Cfg::kWBytes);
-                    if (A_TMA) tma_3d(st, &map_a, k * kTcK, w.m0, t.a_grouped ? w.g : 0, full + s);
-                    const int gw = t.w_grouped ? w.g : 0, n0 = w.n0 * kOut;
+                    if (A_TMA) tma_3d(st, &map_a, k * kTcK, w.m0, ga, full + s);
                     tma_3d(st + Cfg::kABytes, &map_w, k * kTcK, n0, gw, full + s);
                     if (DUAL) tma_3d(st + Cfg::kABytes + kOut * 128, &map_w, k * kTcK, a.N + n0, gw, full + s);
-                    if (++s == kStages) { s = 0; ph ^= 1; }
                 }
+                __syncwarp();
+                if (++s == kStages) { s = 0; ph ^= 1; }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = tc_idesc(kTcRows, BN);
-            uint32_t s = 0, ph = 0, it = 0;
-            bool ok = true;
-            for (; ok && w.step(); ++it) {
-                const uint32_t acc = it & 1, d = tmem + acc * BN;
-                if (!(ok = tc_spin(acc_empty + acc, ((it >> 1) & 1) ^ 1, quit))) break;
+        constexpr uint32_t idesc = tc_idesc(kTcRows, BN);
+        uint32_t s = 0, ph = 0, it = 0;
+        bool ok = true;
+        for (; ok && w.step(); ++it) {
+            const uint32_t acc = it & 1, d = tmem + acc * BN;
+            if (!(ok = tc_spin_warp(acc_empty + acc, ((it >> 1) & 1) ^ 1, quit))) break;
+            umb::tc_fence_after();
+            for (int k = 0; k < t.k_steps; ++k) {
+                if (!(ok = tc_spin_warp(full + s, ph, quit))) break;
                 umb::tc_fence_after();
-                for (int k = 0; k < t.k_steps; ++k) {
-                    if (!(ok = tc_spin(full + s, ph, quit))) break;
-                    umb::tc_fence_after();
-                    const uint32_t st = smem_u32(smem + s * Cfg::kStage);
-                    const uint64_t ad = umb::umma_smem_desc_sw128(st), wd = umb::umma_smem_desc_sw128(st + Cfg::kABytes);
+                const uint32_t st = smem_u32(smem + s * Cfg::kStage);
+                const uint64_t ad = umb::umma_smem_desc_sw128(st), wd = umb::umma_smem_desc_sw128(st + Cfg::kABytes);
+                if (umb::elect_one()) {
 #pragma unroll
                     for (int kk = 0; kk < kTcK / 16; ++kk)
                         umb::umma_ss_f16(d, ad + kk * 2, wd + kk * 2, idesc, (k | kk) ? 1u : 0u);
                     umb::umma_commit(empty + s);
-                    if (++s == kStages) { s = 0; ph ^= 1; }
+                    if (k + 1 == t.k_steps) umb::umma_commit(acc_full + acc);
                 }
-                if (ok) umb::umma_commit(acc_full + acc);
+                __syncwarp();
+                if (++s == kStages) { s = 0; ph ^= 1; }
             }
         }
     } else if (warp < 6) {
@@ -306,8 +303,7 @@ static EncodeTiled encode_tiled() {
     return fn;
 }
 
-// bf16 [groups][rows][cols] with row stride ld and group stride gs (elements): boxes of 64 columns x box_rows rows, 128-byte swizzle
-static int encode_map(CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows, uint64_t groups, uint64_t ld, uint64_t gs,
+int encode_map(CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows, uint64_t groups, uint64_t ld, uint64_t gs,
                       uint32_t box_rows) {
     const EncodeTiled enc = encode_tiled();
     if (enc == nullptr) return UMB_ERR_DRIVER;

@@ -1,5 +1,7 @@
 // Bounded mbarrier waits of the tensor-core kernels of the sequence-state decoders.
 #pragma once
+#include <cuda.h>
+
 #include "../common.cuh"
 
 namespace umbs {
@@ -31,6 +33,13 @@ __device__ __forceinline__ bool tc_spin(uint64_t* bar, uint32_t parity, volatile
         if ((i & 1023) == 1023 && *quit) return false;
     }
     return tc_give_up(quit);
+}
+// The same by a whole warp, which is one again behind it.  The warps that issue copies and products run their loops whole and
+// elect a thread for the instructions themselves: inside a branch that one thread takes, operands leave the uniform registers
+// and every tcgen05 instruction and every passed wait costs hundreds of clocks (measured with clock64 stamps: 8 products of
+// 128 x 32 x 16 and a passed wait 1740 clocks, a wait for a finished barrier 370).
+__device__ __forceinline__ bool tc_spin_warp(uint64_t* bar, uint32_t parity, volatile int* quit) {
+    return __all_sync(0xffffffffu, tc_spin(bar, parity, quit));
 }
 // polling with a short sleep in between: for warps that share a scheduler with working ones
 __device__ __forceinline__ bool tc_poll(uint64_t* bar, uint32_t parity, volatile int* quit) {
@@ -65,5 +74,14 @@ static inline unsigned int tc_timeouts() {
     return cudaMemcpyFromSymbol(&n, g_tc_timeouts, sizeof n) == cudaSuccess ? n : ~0u;
 }
 unsigned int attention_tc_timeouts();                       // seq_attn_tc.cu
+
+// seq_gemm_tc.cu: bf16 [groups][rows][cols] with row stride ld and group stride gs (elements) as a tensor map of boxes of 64
+// columns x box_rows rows, 128-byte swizzle, zeros outside
+int encode_map(CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows, uint64_t groups, uint64_t ld, uint64_t gs, uint32_t box_rows);
+
+__device__ __forceinline__ void tma_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar)) : "memory");
+}
 
 }  // namespace umbs
