@@ -257,25 +257,37 @@ __device__ __forceinline__ unsigned long long gtimer() {
 
 template <int MPAD>
 struct GemmCfg {
-    static constexpr int kDq = MPAD == 16 ? UMB_DQ_GROUPS_16 : kDqGroups;           // dequant groups per CTA (AWQ)
-    static constexpr int kThreadsAwq = 96 + 128 * (kDq + 1) + (UMB_X_PRODUCER ? 32 : 0);
+    // 128 rows (AWQ): weight records and x slabs in rings of their own.  A shared ring holds four units of 41 KB, and a unit
+    // occupies its place from the request over the dequantisation to the product.  The records' ring is free as soon as they
+    // are in registers, so dequantisation runs ahead of the slabs: 500 rows through a layer of width 4096 and its head
+    // 887 -> 849 us; with the heads of split tiles reduced by every group of warps (below) 683.
+    static constexpr bool kSplit = MPAD >= 128;
+    // dequant groups per CTA (AWQ).  kSplit takes two: every ring depth is a multiple of it, so a stage always comes back to
+    // the group that used it last, which the parity waits need there (see the dequant warps' note)
+    static constexpr int kDq = MPAD == 16 ? UMB_DQ_GROUPS_16 : (kSplit ? 2 : kDqGroups);
+    static constexpr bool kXWarp = UMB_X_PRODUCER || kSplit;                        // x slabs are requested by their own warp
+    static constexpr int kWStages = 6;                                              // records held with kSplit
+    static constexpr int kThreadsAwq = 96 + 128 * (kDq + 1) + (kXWarp ? 32 : 0);
     static constexpr int kStagesAwq = MPAD == 16 ? 10 : (MPAD == 32 ? 8 : (MPAD == 64 ? 6 : 4));
     static constexpr int kStagesF16 = MPAD <= 32 ? 8 : (MPAD == 64 ? 6 : 4);
     static constexpr int kXBytesAwq = MPAD * 256;           // [2 atoms][MPAD][128 B]
     static constexpr int kXBytesF16 = MPAD * 128;           // [MPAD][128 B]
     static constexpr int kWBytesF16 = kTileN * 128;         // [128][128 B]
     static constexpr int kPackedStride = 8576;              // record padded to a 128-byte multiple
-    static constexpr int kExchBytes = MPAD * 64 * 2 < 3 * 16 * 128 * 2 ? 3 * 16 * 128 * 2 : MPAD * 64 * 2;   // epilogue staging: output tile + cos / sin rows (RoPE)
+    // epilogue staging: output tile + cos / sin rows (RoPE), for each group of warps that finishes tiles
+    static constexpr int kExchBytes = 3 * 16 * 128 * 2;
+    static constexpr int kExchGroups = kSplit ? kDq + 1 : 1;
     // Independent fp32 accumulators in TMEM (columns a * MPAD): consecutive k-steps rotate through them so
     // that back-to-back tcgen05.mma never wait on each other's accumulate (a dependent 128xNx16 MMA chain
     // runs at its ~150-cycle latency, not at its 8-cycle issue rate); the epilogue sums them.
     static constexpr int kNumAcc = MPAD <= 16 ? 8 : (MPAD == 32 ? 4 : 2);
     static constexpr int kTmemACol0 = kNumAcc * MPAD < 128 ? 128 : kNumAcc * MPAD;   // A operand stages start here
     static constexpr int kTmemAStages = (kTmemCols - kTmemACol0) / 64;             // 6 (4 at MPAD = 128)
-    static constexpr int kBarBytes = 512;
+    static constexpr int kBarBytes = 576;
     static constexpr int smem_bytes(bool awq, int stages) {
-        return 1024 /*align slack*/ + kBarBytes + kExchBytes +
-               stages * (awq ? (kXBytesAwq + kPackedStride) : (kXBytesF16 + kWBytesF16));
+        return 1024 /*align slack*/ + kBarBytes + kExchGroups * kExchBytes +
+               (awq && kSplit ? stages * kXBytesAwq + kWStages * kPackedStride
+                              : stages * (awq ? (kXBytesAwq + kPackedStride) : (kXBytesF16 + kWBytesF16)));
     }
 };
 
@@ -285,10 +297,11 @@ __device__ __forceinline__ unsigned int orderable_f32_g(float f) {
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-// Epilogue of 16 token columns [m0, m0 + 16) for feature lane `fl` (0..127) of tile `tile`.
+// Epilogue of 16 token columns [m0, m0 + 16) for feature lane `fl` (0..127) of tile `tile`.  The four warps that run it
+// share the staging rows `exch` and the named barrier `bar`.
 template <int MPAD>
 __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int tile, int fl, int m0, const float (&v)[16],
-                                               __half* exch) {
+                                               __half* exch, uint32_t bar = 2) {
     const int n = tile * kTileN + fl;
     if (p.mode == UMB_EPI_SILU_MUL) {
         // lanes 0..63 hold `gate`, lanes 64..127 `up` of output features tile*64 + (fl & 63).  Both halves of the
@@ -301,7 +314,7 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int tile, in
 #pragma unroll
             for (int j = 0; j < 16; ++j) dst[j * 64] = __float2half_rn(v[j]);
         }
-        named_bar_sync(2, 128);
+        named_bar_sync(bar, 128);
         {
             const int col = fl & 63, r0 = fl >> 6;
 #pragma unroll
@@ -312,7 +325,7 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int tile, in
                 g_t[r * 64 + col] = __hmul(sl, u_t[r * 64 + col]);
             }
         }
-        named_bar_sync(2, 128);
+        named_bar_sync(bar, 128);
         {
             const int row = fl >> 3, seg = (fl & 7) * 8;
             const int no = tile * 64 + seg;
@@ -326,7 +339,7 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int tile, in
                 }
             }
         }
-        named_bar_sync(2, 128);
+        named_bar_sync(bar, 128);
         return;
     }
     if (p.mode == UMB_EPI_ROPE_QKV) {
@@ -367,7 +380,7 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int tile, in
                         *reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(r.sin) + off);
                 }
             }
-            named_bar_sync(2, 128);
+            named_bar_sync(bar, 128);
             const int head = n / D, d = n - head * D;
             const bool rot = n_ok && head < r.num_q_heads + r.num_kv_heads;
             __half o[16];
@@ -380,10 +393,10 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int tile, in
                     o[j] = __hadd_rn(__hmul_rn(h[j], cos_t[j * D + d]), __hmul_rn(d < half_d ? __hneg(pr) : pr, sin_t[j * D + d]));
                 }
             }
-            named_bar_sync(2, 128);                  // every partner value has been read
+            named_bar_sync(bar, 128);                  // every partner value has been read
 #pragma unroll
             for (int j = 0; j < 16; ++j) exch[j * kTileN + fl] = o[j];
-            named_bar_sync(2, 128);
+            named_bar_sync(bar, 128);
 #pragma unroll
             for (int it = 0; it < 2; ++it) {
                 const int sidx = fl + it * 128, row = sidx >> 4, c0 = (sidx & 15) * 8;
@@ -402,10 +415,10 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int tile, in
                     *reinterpret_cast<uint4*>(dst + d0) = *reinterpret_cast<const uint4*>(exch + row * kTileN + c0);
                 }
             }
-            named_bar_sync(2, 128);
+            named_bar_sync(bar, 128);
             return;
         }
-        named_bar_sync(2, 128);
+        named_bar_sync(bar, 128);
         if (n_ok) {
             const int head = n / D, d = n - head * D;
             const bool rot = head < r.num_q_heads + r.num_kv_heads;
@@ -434,7 +447,7 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int tile, in
                 dst[d] = o;
             }
         }
-        named_bar_sync(2, 128);
+        named_bar_sync(bar, 128);
         return;
     }
     const bool n_ok = n < p.N_total;
@@ -461,7 +474,7 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int tile, in
                 if (ok[i])
                     *reinterpret_cast<uint4*>(exch + row[i] * kTileN + col[i]) = *reinterpret_cast<const uint4*>(
                         p.residual + (int64_t)(m0 + row[i]) * p.ld_residual + tile * kTileN + col[i]);
-            named_bar_sync(2, 128);
+            named_bar_sync(bar, 128);
         }
         const __half bb = (p.bias && n_ok) ? p.bias[n] : __float2half_rn(0.f);
         __half h[16];
@@ -471,16 +484,16 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int tile, in
             if (p.bias) h[j] = __hadd(h[j], bb);
             if (resid) h[j] = __hadd(exch[j * kTileN + fl], h[j]);
         }
-        if (resid) named_bar_sync(2, 128);            // every thread has read its residual column
+        if (resid) named_bar_sync(bar, 128);            // every thread has read its residual column
 #pragma unroll
         for (int j = 0; j < 16; ++j) exch[j * kTileN + fl] = h[j];
-        named_bar_sync(2, 128);
+        named_bar_sync(bar, 128);
 #pragma unroll
         for (int i = 0; i < 2; ++i)
             if (ok[i])
                 *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(p.y) + (int64_t)(m0 + row[i]) * p.ldy + tile * kTileN + col[i]) =
                     *reinterpret_cast<const uint4*>(exch + row[i] * kTileN + col[i]);
-        named_bar_sync(2, 128);                       // the staging tile is free for the next chunk
+        named_bar_sync(bar, 128);                       // the staging tile is free for the next chunk
         return;
     }
     if (!n_ok && !(p.mode == UMB_EPI_LOGITS && p.argmax)) return;
@@ -549,6 +562,8 @@ __device__ __forceinline__ void load_acc_sum(uint32_t taddr, float (&v)[16], int
 //                 soon as a weight record has landed, also before the predecessor kernel has finished
 //   last 4 warps  epilogue only (AWQ: warps 15..18, fp16: warps 3..6): the partial-tile fix-up is a chain of
 //                 global round trips and must not stall the dequant stream
+//   65..128 rows  (AWQ) two dequant groups, warps 3..10, which also reduce when they have no units left; epilogue warps
+//                 11..14; warp 15 requests the x slabs
 template <int MPAD, bool kAwq>
 __global__ void __launch_bounds__(kAwq ? GemmCfg<MPAD>::kThreadsAwq : kGemmThreadsF16, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
@@ -569,14 +584,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
     // the MMA warps take alternate units, so a ring stage must always come back to the same warp (parity waits, see the
     // dequant warps' note): both rings need an even depth
     static_assert(!kAwq || (kAStages % 2 == 0 && Cfg::kStagesAwq % 2 == 0), "ring depths must be even");
+    constexpr bool kSplit = kAwq && Cfg::kSplit, kXWarp = kAwq && Cfg::kXWarp;
+    static_assert(!kSplit || (kAStages % Cfg::kDq == 0 && Cfg::kWStages % Cfg::kDq == 0 && Cfg::kStagesAwq == kAStages),
+                  "the rings of separate records must return each stage to its dequant group");
+    const int kWRing = kSplit ? Cfg::kWStages : kStages;        // depth of the weight records' ring
     constexpr int kDq = Cfg::kDq;                               // dequant groups of this CTA
+    constexpr int kFinish = kSplit ? Cfg::kExchGroups : 1;      // groups of warps that reduce the head of a split tile
 
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* s_x = smem;                                   // kStages x kXBytes   (1024-aligned slabs)
     unsigned char* s_w = s_x + kStages * kXBytes;                // kStages x kWStride
-    __half* s_exch = reinterpret_cast<__half*>(s_w + kStages * kWStride);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(s_exch) + Cfg::kExchBytes);
+    __half* s_exch = reinterpret_cast<__half*>(s_w + kWRing * kWStride);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(s_exch) + Cfg::kExchGroups * Cfg::kExchBytes);
     uint64_t* full_w = bars;                  // [kStages]   weight record / tile landed
     uint64_t* full_x = bars + 16;             // [kStages]   x slab landed
     uint64_t* done = bars + 32;               // [kStages]   every MMA of the unit in this stage has retired
@@ -584,7 +604,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
     uint64_t* acc_full = bars + 56;
     uint64_t* acc_empty = bars + 57;
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 58);
-    int* s_flag = reinterpret_cast<int*>(bars + 59);
+    uint64_t* last_full = bars + 59;          //             kSplit: the last segment's accumulators are complete
+    uint64_t* w_empty = bars + 60;            // [kWStages]  kSplit: the record in this stage is in the dequant group's registers
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) UMB_TRACE(0);
@@ -598,12 +619,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
         tma_prefetch_desc(&tmap_x);
         if (!kAwq || UMB_X_3D) tma_prefetch_desc(&tmap_w);
         for (int i = 0; i < kStages; ++i) {
-            mbar_init(full_w + i, 1);
+            if (!kSplit) mbar_init(full_w + i, 1);
             mbar_init(full_x + i, 1);
             mbar_init(done + i, 1);
         }
+        for (int i = 0; kSplit && i < kWRing; ++i) {
+            mbar_init(full_w + i, 1);
+            mbar_init(w_empty + i, 4);
+        }
         for (int i = 0; i < kAStages; ++i) mbar_init(a_full + i, 4);
         mbar_init(acc_full, 2);
+        if (kSplit) mbar_init(last_full, 2);
         mbar_init(acc_empty, 4);
         fence_barrier_init();
     }
@@ -622,7 +648,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
         // ===================== TMA producer (whole warp runs the loop, one elected lane issues) =====================
         const uint64_t pol_w = l2_policy_evict_first(), pol_x = l2_policy_evict_last();
         const unsigned char* src = p.packed + (kAwq ? u_begin * kRecordStride : 0);
-        const int n_pre = n_units < kStages ? n_units : kStages;
+        const int n_pre = n_units < kWRing ? n_units : kWRing;
         // The weight copies of the whole ring are requested before griddepcontrol.wait (they never depend on the
         // stream predecessor), the x slabs after it.  (Requesting only a few records early, so that the first x
         // slab does not queue behind ~85 KB of weights, starts the first MMA 2 us sooner but measured no faster:
@@ -637,7 +663,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                 tma_tensor2d_g2s(s_w + stage * kWStride, &tmap_w, g * 64, tile * kTileN, full_w + stage, pol_w);
         };
         auto issue_x = [&](int stage, int gk) {
-            if (kAwq && UMB_X_PRODUCER) return;                   // requested by the x-producer warp
+            if (kXWarp) return;                                   // requested by the x-producer warp
             mbar_arrive_expect_tx(full_x + stage, (uint32_t)kXBytes);
             unsigned char* xs = s_x + stage * kXBytes;
             if constexpr (kAwq && UMB_X_3D) {
@@ -726,19 +752,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
         Ring r;
         r.phase = 1;                                             // every stage has been used once
         for (int i = n_pre; i < n_units; ++i) {
-            UMB_WAIT(done + r.stage, r.phase ^ 1);              // the unit that last used this stage has retired
+            // the unit that last used this stage has retired (kSplit: its record has been read)
+            if constexpr (kSplit) UMB_WAIT(w_empty + r.stage, r.phase ^ 1);
+            else UMB_WAIT(done + r.stage, r.phase ^ 1);
             if (elect_one()) {
                 issue_w(r.stage);
                 issue_x(r.stage, g);
             }
             __syncwarp();
             advance_w();
-            r.advance(kStages);
+            r.advance(kWRing);
         }
         }
         if (lane == 0) UMB_TRACE(10);
-    } else if (kAwq && UMB_X_PRODUCER && warp == GemmCfg<MPAD>::kThreadsAwq / 32 - 1) {
-        // ===================== x-slab producer (AWQ, UMB_X_PRODUCER): two tensor copies per unit =====================
+    } else if (kXWarp && warp == GemmCfg<MPAD>::kThreadsAwq / 32 - 1) {
+        // ===================== x-slab producer (AWQ, kXWarp) =====================
         const uint64_t pol_x = l2_policy_evict_last();
         pdl_wait();                                              // x is the predecessor's output
         int gx = in_tile0, stage = 0, use = 0;
@@ -797,6 +825,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                         }
                         umma_commit(done + st);
                         if (last) umma_commit(acc_full);
+                        if (kSplit && last && seg_end == n_units) umma_commit(last_full);
                     }
                 } else {
                     const uint32_t ws = smem_u32(s_w + st * kWStride);
@@ -824,7 +853,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                 }
             }
             if (first) {                     // this warp had no unit in the segment: plain arrival
-                if (elect_one()) mbar_arrive(acc_full);
+                if (elect_one()) {
+                    mbar_arrive(acc_full);
+                    if (kSplit && seg_end == n_units) mbar_arrive(last_full);
+                }
                 __syncwarp();
             }
             seg_begin = seg_end;
@@ -838,10 +870,82 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
         const bool is_epi = kAwq ? (grp == kDq) : true;
         const int fl = q * 32 + lane;                // feature lane 0..127
         const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
+        // acc[j] += the partial sums the other CTAs of `tile_` published for token columns [m0, m0 + 16), in
+        // ascending CTA order (deterministic); the polled words are stored back as zeros.
+        auto reduce_others = [&](float (&acc)[16], int m0, int tile_, int c_first, int n_other) {
+            const int mcols = p.M - m0;
+            uint32_t* sl0 = reinterpret_cast<uint32_t*>(p.slots) +
+                            ((size_t)tile_ + c_first + 1) * (MPAD * kTileN) + m0 * kTileN + fl;
+            if (mcols <= 4) {
+                // few token rows (draft levels): 8 slots in flight per round trip
+                for (int c0 = 0; c0 < n_other; c0 += 8) {
+                    uint32_t t[8][4];
+                    bool pending;
+                    do {
+                        pending = false;
+#pragma unroll
+                        for (int cc = 0; cc < 8; ++cc)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const bool need = c0 + cc < n_other && j < mcols;
+                                t[cc][j] = need ? ld_relaxed_gpu_u32(sl0 + (size_t)(c0 + cc) * (MPAD * kTileN) + j * kTileN) : 0x80000000u;
+                            }
+#pragma unroll
+                        for (int cc = 0; cc < 8; ++cc)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) pending |= t[cc][j] == 0u;
+                    } while (pending);
+#pragma unroll
+                    for (int cc = 0; cc < 8; ++cc)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            acc[j] += __uint_as_float(t[cc][j]);
+                            if (c0 + cc < n_other && j < mcols) sl0[(size_t)(c0 + cc) * (MPAD * kTileN) + j * kTileN] = 0u;
+                        }
+                }
+            } else if (mcols > 0) {
+                for (int c0 = 0; c0 < n_other; c0 += 2) {
+                    uint32_t t[2][16];
+                    bool pending;
+                    do {
+                        pending = false;
+#pragma unroll
+                        for (int cc = 0; cc < 2; ++cc)
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) {
+                                const bool need = c0 + cc < n_other && j < mcols;
+                                t[cc][j] = need ? ld_relaxed_gpu_u32(sl0 + (size_t)(c0 + cc) * (MPAD * kTileN) + j * kTileN) : 0x80000000u;
+                            }
+#pragma unroll
+                        for (int cc = 0; cc < 2; ++cc)
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) pending |= t[cc][j] == 0u;
+                    } while (pending);
+#pragma unroll
+                    for (int cc = 0; cc < 2; ++cc)
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            acc[j] += __uint_as_float(t[cc][j]);
+                            if (c0 + cc < n_other && j < mcols) sl0[(size_t)(c0 + cc) * (MPAD * kTileN) + j * kTileN] = 0u;
+                        }
+                }
+            }
+        };
+        // The reducer's share of a tile: chunks of 16 token columns m_first, m_first + m_step, ...
+        auto reduce_tile = [&](int m_first, int m_step, int tile_, int c_first, int c_last, int use_mask, __half* ex, uint32_t bar) {
+#pragma unroll 1
+            for (int m0 = m_first; m0 < MPAD; m0 += m_step) {
+                if (!(m0 < p.M || p.mode == UMB_EPI_SILU_MUL || p.mode == UMB_EPI_ROPE_QKV)) break;
+                float v[16];
+                load_acc_sum<kAccUsed, MPAD>(tmem_base + lane_addr + m0, v, use_mask);
+                reduce_others(v, m0, tile_, c_first, c_last - c_first);
+                epilogue_chunk<MPAD>(p, tile_, fl, m0, v, ex, bar);
+            }
+        };
         if (!is_epi) {
             // ===================== dequant warps (AWQ): group g takes CTA-local units g, g + kDqGroups, ... =====================
             if constexpr (kAwq) {
-                int dq_st = grp % kStages, dq_ph = 0, dq_ts = grp % kAStages;      // ring positions of unit `mine`
+                int dq_st = grp % kWRing, dq_ph = 0, dq_ts = grp % kAStages;      // ring positions of unit `mine`
                 int w_first = grp;                                                 // first unit of this group that re-uses a TMEM stage
                 while (w_first < kAStages) w_first += kDq;
                 int w_st = (w_first - kAStages) % kStages, w_ph = 0;               // ring position of unit `mine - kAStages`
@@ -859,12 +963,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                     UMB_WAIT(full_w + (kPair ? (dq_st & ~1) : dq_st), dq_ph);
                     if (grp == 0 && q == 0 && lane == 0) UMB_TRACE(4);
                     fetch(dq_st);
+                    if constexpr (kSplit) {
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(w_empty + dq_st);
+                    }
                 }
                 for (int mine = grp; mine < n_units; mine += kDq) {
                     const int ts = dq_ts;
                     dq_st += kDq;
-                    if (dq_st >= kStages) {
-                        dq_st -= kStages;
+                    if (dq_st >= kWRing) {
+                        dq_st -= kWRing;
                         dq_ph ^= 1;
                     }
                     dq_ts += kDq;
@@ -900,6 +1008,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                         //     done[v - kAStages] implies done[v - kStages]: both ring depths are even, so the two units were
                         //     issued and committed, in order, by the same MMA thread; a retired occupant has landed, so
                         //     full_w is at most one use behind.  (v < kAStages: first use of both stages, nothing to wait for.)
+                        //     kSplit: the producer no longer orders the records behind done, so (1) itself has to know that
+                        //     done[v - 2 kAStages] is over, and (2) that record v - kWStages was read: this group has waited
+                        //     for both itself, both depths being multiples of the number of groups.
                         if (mine + kDq >= kAStages) {
                             UMB_WAIT(done + w_st, w_ph);
                             tc_fence_after();
@@ -911,6 +1022,29 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                         }
                         UMB_WAIT(full_w + (kPair ? (dq_st & ~1) : dq_st), dq_ph);
                         fetch(dq_st);
+                        if constexpr (kSplit) {
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(w_empty + dq_st);
+                        }
+                    }
+                }
+                if constexpr (kSplit) {
+                    // The head of a split tile is reduced by all groups of warps, one chunk of 16 columns each in turn: a chunk
+                    // waits for two or three round trips to the other CTAs' sums, 24 of them in series with one group
+                    // when five CTAs share a tile (849 -> 683 us, see kSplit; four sums in flight a thread instead of two
+                    // spill registers: 753).
+                    const int tile_ = (int)((u_end - 1) / p.units_per_tile);
+                    const long long tile_u0 = (long long)tile_ * p.units_per_tile;
+                    const int c_first = sk_owner(tile_u0, U, P), c_last = sk_owner(tile_u0 + p.units_per_tile - 1, U, P);
+                    if (n_units > 0 && c_first == (int)blockIdx.x && c_last != c_first) {
+                        const int begin = tile_u0 > u_begin ? (int)(tile_u0 - u_begin) : 0;       // CTA-local first unit of the segment
+                        const int n_odd = (n_units >> 1) - (begin >> 1);
+                        const int use_mask = ((n_units - begin - n_odd) > 0 ? 1 : 0) | (n_odd > 0 ? 2 : 0);
+                        pdl_wait();
+                        UMB_WAIT_LONG(last_full, 0);
+                        tc_fence_after();
+                        reduce_tile(16 * (grp + 1), 16 * kFinish, tile_, c_first, c_last, use_mask,
+                                    s_exch + (grp + 1) * (Cfg::kExchBytes / 2), 3 + grp);
                     }
                 }
             }
@@ -920,67 +1054,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
             pdl_wait();                                  // residual / workspace / y belong to the predecessors
             if (ew == 0 && lane == 0) UMB_TRACE(11);
             int seg = 0, seg_begin = 0, in_tile = in_tile0, tile = tile0;
-            // acc[j] += the partial sums the other CTAs of `tile_` published for token columns [m0, m0 + 16), in
-            // ascending CTA order (deterministic); the polled words are stored back as zeros.
-            auto reduce_others = [&](float (&acc)[16], int m0, int tile_, int c_first, int n_other) {
-                const int mcols = p.M - m0;
-                uint32_t* sl0 = reinterpret_cast<uint32_t*>(p.slots) +
-                                ((size_t)tile_ + c_first + 1) * (MPAD * kTileN) + m0 * kTileN + fl;
-                if (mcols <= 4) {
-                    // few token rows (draft levels): 8 slots in flight per round trip
-                    for (int c0 = 0; c0 < n_other; c0 += 8) {
-                        uint32_t t[8][4];
-                        bool pending;
-                        do {
-                            pending = false;
-#pragma unroll
-                            for (int cc = 0; cc < 8; ++cc)
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    const bool need = c0 + cc < n_other && j < mcols;
-                                    t[cc][j] = need ? ld_relaxed_gpu_u32(sl0 + (size_t)(c0 + cc) * (MPAD * kTileN) + j * kTileN) : 0x80000000u;
-                                }
-#pragma unroll
-                            for (int cc = 0; cc < 8; ++cc)
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) pending |= t[cc][j] == 0u;
-                        } while (pending);
-#pragma unroll
-                        for (int cc = 0; cc < 8; ++cc)
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                acc[j] += __uint_as_float(t[cc][j]);
-                                if (c0 + cc < n_other && j < mcols) sl0[(size_t)(c0 + cc) * (MPAD * kTileN) + j * kTileN] = 0u;
-                            }
-                    }
-                } else if (mcols > 0) {
-                    for (int c0 = 0; c0 < n_other; c0 += 2) {
-                        uint32_t t[2][16];
-                        bool pending;
-                        do {
-                            pending = false;
-#pragma unroll
-                            for (int cc = 0; cc < 2; ++cc)
-#pragma unroll
-                                for (int j = 0; j < 16; ++j) {
-                                    const bool need = c0 + cc < n_other && j < mcols;
-                                    t[cc][j] = need ? ld_relaxed_gpu_u32(sl0 + (size_t)(c0 + cc) * (MPAD * kTileN) + j * kTileN) : 0x80000000u;
-                                }
-#pragma unroll
-                            for (int cc = 0; cc < 2; ++cc)
-#pragma unroll
-                                for (int j = 0; j < 16; ++j) pending |= t[cc][j] == 0u;
-                        } while (pending);
-#pragma unroll
-                        for (int cc = 0; cc < 2; ++cc)
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                acc[j] += __uint_as_float(t[cc][j]);
-                                if (c0 + cc < n_other && j < mcols) sl0[(size_t)(c0 + cc) * (MPAD * kTileN) + j * kTileN] = 0u;
-                            }
-                    }
-                }
-            };
             while (seg_begin < n_units) {
                 const int seg_end = seg_begin + min(n_units - seg_begin, p.units_per_tile - in_tile);
                 const int seg_len = seg_end - seg_begin;
@@ -1035,22 +1108,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                                 }
                         }
                     } else {
-                        const int n_other = c_last - c_first;
-#pragma unroll 1
-                        for (int m0 = 0; m0 < MPAD; m0 += 16) {
-                            float v[16];
-                            load_acc_sum<kAccUsed, MPAD>(tmem_base + lane_addr + m0, v, use_mask);
-                            if (m0 + 16 >= MPAD) {
-                                tc_fence_before();
-                                __syncwarp();
-                                if (lane == 0) mbar_arrive(acc_empty);
-                            }
-                            if (!(m0 < p.M || p.mode == UMB_EPI_SILU_MUL || p.mode == UMB_EPI_ROPE_QKV)) continue;
-                            if (ew == 0 && lane == 0 && m0 == 0) UMB_TRACE(14);
-                            reduce_others(v, m0, tile, c_first, n_other);
-                            if (ew == 0 && lane == 0 && m0 == 0) UMB_TRACE(15);
-                            epilogue_chunk<MPAD>(p, tile, fl, m0, v, s_exch);
-                        }
+                        // always the CTA's last segment: the accumulators are not handed back
+                        if (ew == 0 && lane == 0) UMB_TRACE(14);
+                        reduce_tile(0, 16 * kFinish, tile, c_first, c_last, use_mask, s_exch, 2);
+                        if (ew == 0 && lane == 0) UMB_TRACE(15);
                     }
                 }
                 seg_begin = seg_end;
@@ -1330,7 +1391,7 @@ static int launch_gemm(const CUtensorMap& tx, const CUtensorMap& tw, GemmParams 
             const char* e = getenv("UMB_GEMM_STAGES");
             env_stages = e ? atoi(e) : 0;
         }
-        if (env_stages > 0 && env_stages <= 16 && (env_stages % 2) == 0 && GemmCfg<MPAD>::smem_bytes(kAwq, env_stages) <= 227 * 1024)
+        if (env_stages > 0 && env_stages <= 16 && (env_stages % 2) == 0 && !(kAwq && GemmCfg<MPAD>::kSplit) && GemmCfg<MPAD>::smem_bytes(kAwq, env_stages) <= 227 * 1024)
             p.stages = env_stages;                                   // even: see the static_assert on the ring depths
     }
     p.trace = trace_for_this_launch();
