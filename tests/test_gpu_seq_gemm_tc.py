@@ -35,6 +35,15 @@ def test_plain(ops, M, N, K):
     assert H.rel_err(ops.gemm(a, w), ref.cpu()) < BF16_TOL
 
 
+def test_overlapping_rows_are_taken(ops):
+    a, w = _mat(41, 1, 64), _mat(42, 40, 64)
+    ref = a.double() @ w.double().T
+    assert H.rel_err(ops.gemm(a.expand(33, 64), w, out_f32=True), ref.expand(33, 40).cpu()) < F32_TOL
+    x = _mat(43, 600)                                            # row i starts at number 8 i
+    rows = x.as_strided((60, 64), (8, 1))
+    assert H.rel_err(ops.gemm(rows, w, out_f32=True), (rows.double() @ w.double().T).cpu()) < F32_TOL
+
+
 def test_rows_are_bitwise_the_same_in_every_tile_width(ops):
     a, w = _mat(3, 2100, 512), _mat(4, 2048, 512)               # 17 x 8 tiles of 256 columns; 64 rows alone: tiles of 64
     full = ops.gemm(a, w, out_f32=True)

@@ -4,7 +4,7 @@
 //
 // Three kernels share one argument block:
 //   * gemm_simt_kernel  -- fp32 FMA chains over shared-memory tiles; the UMBS_F32 mode (true 32-bit) and every shape
-//                          the tensor-core kernel does not take (K not a multiple of 16, unaligned rows);
+//                          the tensor-core kernel does not take (K not a multiple of 32, unaligned rows);
 //   * gemm_tc_kernel    -- bf16 operands through tcgen05 with fp32 accumulators (seq_gemm_tc.cu);
 //   * gemm_skinny_kernel -- bf16, at most 16 rows (decoding): a weight stream with the rows' partial sums in registers.
 // In each of them an output element is one fp32 sum over k in an order that does not depend on the other rows, so a
@@ -350,7 +350,8 @@ static int gemm_run(int dtype, const void* A, int64_t lda, int a_goff, const voi
         // 16-byte loads: every row start and group offset must sit on a 16-byte boundary
         const bool vec = (K % 8 == 0) && (lda % 8 == 0) && (ldw % 8 == 0) && (a_goff % 8 == 0) && (w_gstride % 8 == 0) &&
                          ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
-        const bool tc = vec && (K % 32 == 0);
+        // (rows that overlap, one row repeated among them: not described by a tensor map, they take the general kernel)
+        const bool tc = vec && (K % 32 == 0) && lda >= K && ldw >= K;
         if (vec && M <= 16) {
             if (c_f32) launch_skinny<float>(a, groups, dual != 0, st);
             else launch_skinny<__nv_bfloat16>(a, groups, dual != 0, st);
