@@ -17,6 +17,10 @@
 // 64 keys to a tile only one score tile fits beside the output of 128 columns, and scores, weights and output products take
 // turns: 5800 clocks per 64 keys and block, of which the tensor core works 1160 (measured with clock64 stamps; 128 x 64 x 16
 // takes it 48 clocks, 128 x 128 x 16 takes 64).
+//
+// Bound: the weights (an exponential and three bf16 parts of each score by the row's own thread) between products they wait
+// for.  4096 tokens, 16 heads of 128 over 4 key/value heads, window 1024, pooled blocks: 2250 us on fp32 multiply-adds,
+// 141 us here; two prompts of 2000 tokens, 16 heads of 128 + 64 shared: 2652 -> 187 us.
 #include "seq_attn.h"
 #include "seq_tc.cuh"
 
@@ -354,7 +358,6 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
             const float* grow = a.gate ? a.gate + t * a.ldg + (a.gate_per_head ? h : h * a.vdim) : nullptr;
             const float gh = (grow && a.gate_per_head && r < len) ? sigmoidf_(grow[0]) : 1.f;
             const bool gvec = grow && !a.gate_per_head && ((uintptr_t)grow & 15) == 0;
-            float* rrow = a.raw ? a.raw + (t * vhd.nv + vh) * a.vdim : nullptr;
             __nv_bfloat16* orow = STEP ? (__nv_bfloat16*)x.out + t * x.ldo + (int64_t)h * a.vdim
                                        : (__nv_bfloat16*)a.out + t * a.heads * a.vdim + (int64_t)h * a.vdim;
             for (int c0 = 0; c0 < a.vdim; c0 += 32) {
@@ -368,11 +371,6 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
                             float o[8];
 #pragma unroll
                             for (int u = 0; u < 8; ++u) o[u] = __uint_as_float(v[e + u]) * inv;
-                            if (rrow) {
-                                *reinterpret_cast<float4*>(rrow + c0 + e) = make_float4(o[0], o[1], o[2], o[3]);
-                                *reinterpret_cast<float4*>(rrow + c0 + e + 4) = make_float4(o[4], o[5], o[6], o[7]);
-                                continue;
-                            }
                             if (grow) {
                                 float g[8];
                                 if (gvec) {
@@ -417,13 +415,16 @@ static TaDims ta_dims(const CachedAttnArgs& a) {
 
 // Every row piece is copied in 16-byte pieces and a block's tiles and tensor memory leave room for a second one on the SM:
 // sizes in eights, queries and keys of up to 192, values of up to 128 numbers.
+// bf16 results only: the tensor core cuts its running sums off instead of rounding them, which leaves an fp32 result 1.2e-6
+// from float64 (in the norm, 600 keys) where the fp32 kernel leaves 4e-7, so results handed out in fp32 keep that kernel.
 bool attention_tc_fits(const CachedAttnArgs& a, const StepKeys* s) {
+    if (s == nullptr && a.raw != nullptr) return false;
     auto al = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
     if (a.dim % 8 || a.vdim % 8 || a.dim > 192 || a.vdim > 128 || a.dim < 8 || a.vdim < 8) return false;
     if (s != nullptr)
         return s->kdim % 8 == 0 && al(s->q) && al(s->k) && al(s->v) && al(s->out) && s->ldq % 8 == 0 && s->ldk % 8 == 0 && s->ldv % 8 == 0 &&
                s->ldo % 8 == 0 && (s->kdim == a.dim || (al(s->ks) && s->ldks % 8 == 0));
-    return al(a.q) && al(a.kv) && al(a.kv_cache) && (a.pool <= 0 || al(a.pool_cache)) && (a.raw != nullptr ? al(a.raw) : al(a.out));
+    return al(a.q) && al(a.kv) && al(a.kv_cache) && (a.pool <= 0 || al(a.pool_cache)) && al(a.out);
 }
 
 template <int MODE, bool SHAPED, bool STEP>

@@ -4,7 +4,8 @@
 // slot's cache rows (position p at row p mod kv_len), pooled blocks from the slot's block table -- so a prompt in one
 // piece, in portions, and token-by-token decoding all walk the same keys in the same order.
 //
-// Tile kernel (any step): one block = 64 consecutive query rows of one (sequence, head); 256 threads as 16 x 16, a thread
+// Steps with several tokens per sequence, bf16, of the sizes and addresses that seq_attn_tc.cu takes: its kernel.
+// Tile kernel (any other such step): one block = 64 consecutive query rows of one (sequence, head); 256 threads as 16 x 16, a thread
 // owns 4 rows x 4 keys of the score tile and 4 rows x VC value columns of the output; per tile of 64 keys the scores come
 // from transposed fp32 tiles in shared memory, the weights go back through shared memory for the value product.  The key
 // tile holds 64 dimensions at a time (larger heads add their scores up over several passes), which keeps two blocks on an
@@ -609,7 +610,6 @@ __global__ void __launch_bounds__(32 * kCgWarps, 3) cached_attention_decode_grou
             continue;
         }
         const float inv = MODE == UMBS_ATTN_SIGMOID ? 1.f : 1.f / L;
-        if (a.raw != nullptr) { a.raw[((int64_t)t * v0.nv + vh) * vdim + c] = O * inv; continue; }
         float gt = 1.f;
         if (a.gate) gt = sigmoidf_(a.gate[(int64_t)t * a.ldg + (a.gate_per_head ? hh : hh * vdim + c)]);
         ((__nv_bfloat16*)a.out)[(int64_t)t * a.heads * vdim + (int64_t)hh * vdim + c] = __float2bfloat16_rn(O * inv * gt);
@@ -654,9 +654,10 @@ static int launch_decode(const CachedAttnArgs& a, const Batch& b, int n_split, f
 }
 
 // Sizes the grouped kernel takes: rows in 16-byte pieces, at most 128 numbers (eight k steps, sixteen value tiles in registers).
+// fp32 results stay with the fp32 kernel: at 64 dimensions its error to float64 is 2.2e-7, the tensor path's 2.9e-7.
 static bool group_fits(const CachedAttnArgs& a) {
     auto al = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
-    return a.dim % 8 == 0 && a.vdim % 8 == 0 && a.dim <= 128 && a.vdim <= 128 && al(a.q) && al(a.kv) && al(a.kv_cache) &&
+    return a.raw == nullptr && a.dim % 8 == 0 && a.vdim % 8 == 0 && a.dim <= 128 && a.vdim <= 128 && al(a.q) && al(a.kv) && al(a.kv_cache) &&
            (a.pool <= 0 || al(a.pool_cache));
 }
 static int group_blocks(const CachedAttnArgs& a) {

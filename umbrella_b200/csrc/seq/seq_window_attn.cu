@@ -8,7 +8,8 @@
 //   scores   Q K^T from transposed fp32 tiles in shared memory (two 16-byte loads per 16 multiply-adds),
 //   softmax  running maximum / sum per row in fp32, reduced over the 16 threads that share the row,
 //   values   P V with P handed over through shared memory.
-// Everything is fp32 arithmetic; T is the storage type of q, k, v and the output.
+// Everything is fp32 arithmetic; T is the storage type of q, k, v and the output.  bf16 rows of the sizes and addresses that
+// seq_attn_tc.cu takes go there instead.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math.h>
