@@ -69,3 +69,17 @@ def test_mlstm(lens, dim, vdim):
         got.append((y, state.clone()))
     for y, state in got[1:]:
         assert H.rel_err(y, got[0][0]) < 1e-5 and H.rel_err(state, got[0][1]) < 1e-5
+
+
+@pytest.mark.parametrize("vdim", [255, 256, 257, 600])
+def test_mlstm_rows_around_a_lanes_columns(vdim):
+    """The last kernel takes 256 columns at a time.  Tolerance: fp32 sums of a few dozen terms and one division, as in the
+    operator's own tests."""
+    from test_gpu_zed_ops import f32, mlstm_reference, rnd
+    from umbrella_b200 import ops_seq as K
+    heads, dim, n = 2, 16, 3
+    proj, bias, norm = rnd(n, 2 * heads * (dim + vdim + 1), seed=60), rnd(2 * heads, seed=61), 1.0 + rnd(heads * vdim, seed=62, scale=0.2)
+    state = torch.zeros(1, heads, dim * (vdim + 1) + 1, device=DEV)
+    out = K.mlstm(f32(proj), f32(bias), K.RaggedBatch([(0, n, 0, 0)], DEV), heads, dim, vdim, 10.0, 1e-5, f32(norm), state)
+    ref = mlstm_reference(proj, bias, heads, dim, vdim, 10.0, 1e-5, norm)
+    assert float((out.double().cpu() - ref.double()).abs().max() / ref.double().abs().max()) < 2e-5

@@ -213,6 +213,9 @@ __global__ void mlstm_chain_kernel(Batch b, int heads, int dim, int V1, const fl
     }
 }
 
+// A warp per (token, head).  Bound in a decode step: the latency of its reads, so a lane asks for 8 columns of all three rows
+// before it uses one (a batch of four through 8 layers, one prompt and 8 decoded tokens: 3480 -> 3443 us).
+constexpr int kMfCols = 8;
 template <typename T>
 __global__ void mlstm_finish_kernel(const float* __restrict__ o, const float* __restrict__ gates, const float* __restrict__ proj,
                                     int64_t ld, int off_g, int n, int heads, int vdim, float eps,
@@ -222,17 +225,41 @@ __global__ void mlstm_finish_kernel(const float* __restrict__ o, const float* __
     const int t = w / heads, h = w - t * heads, V1 = vdim + 1;
     const float* orow = o + (int64_t)w * V1;
     const float* grow = proj + (int64_t)t * ld + off_g + h * vdim;
+    const float* nrow = norm_w + h * vdim;
+    auto fetch = [&](const float* row, int e0, float (&r)[kMfCols]) {
+#pragma unroll
+        for (int i = 0; i < kMfCols; ++i) r[i] = e0 + 32 * i < vdim ? row[e0 + 32 * i] : 0.f;
+    };
+    float v[kMfCols], g[kMfCols], nw[kMfCols];
+    fetch(orow, lane, v);
+    fetch(grow, lane, g);
+    fetch(nrow, lane, nw);
     const float den = fmaxf(fabsf(orow[vdim]), gates[(int64_t)w * 3 + 2]) + 1e-6f;
     float ss = 0.f;
-    for (int e = lane; e < vdim; e += 32) {
-        const float v = orow[e] / den;
-        ss = fmaf(v, v, ss);
+    for (int e0 = lane; e0 < vdim; e0 += 32 * kMfCols) {
+        if (e0 != lane) fetch(orow, e0, v);
+#pragma unroll
+        for (int i = 0; i < kMfCols; ++i) {
+            v[i] /= den;                                            // (columns past the end: 0)
+            ss = fmaf(v[i], v[i], ss);
+        }
     }
     ss = warp_sum_ml(ss);
     const float inv = 1.f / sqrtf(ss / (float)vdim + eps);
-    for (int e = lane; e < vdim; e += 32) {
-        const float g = 1.f / (1.f + expf(-grow[e]));
-        out[(int64_t)t * heads * vdim + h * vdim + e] = from_f32<T>(orow[e] / den * inv * norm_w[h * vdim + e] * g);
+    for (int e0 = lane; e0 < vdim; e0 += 32 * kMfCols) {
+        if (vdim > 32 * kMfCols) {
+            fetch(orow, e0, v);
+            fetch(grow, e0, g);
+            fetch(nrow, e0, nw);
+#pragma unroll
+            for (int i = 0; i < kMfCols; ++i) v[i] /= den;
+        }
+#pragma unroll
+        for (int i = 0; i < kMfCols; ++i)
+            if (e0 + 32 * i < vdim) {
+                const float s = 1.f / (1.f + expf(-g[i]));
+                out[(int64_t)t * heads * vdim + h * vdim + e0 + 32 * i] = from_f32<T>(v[i] * inv * nw[i] * s);
+            }
     }
 }
 
