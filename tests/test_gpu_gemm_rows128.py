@@ -1,5 +1,5 @@
-"""The AWQ product with 65 to 128 token rows: weight records and x slabs in rings of their own, and the head of a split
-tile reduced by all groups of warps in turn.  K from one unit of 128 (fewer units than a ring is deep) to many tiles a
+"""The AWQ product with 33 to 128 token rows, where the head of a split tile is reduced by all groups of warps in turn, and
+beyond 64 rows with weight records and x slabs in rings of their own.  K from one unit of 128 (fewer units than a ring is deep) to many tiles a
 block shares, rows at the edges of the 16-row chunks, every epilogue that stages rows."""
 import numpy as np
 import pytest
@@ -18,8 +18,8 @@ def _near(out, ref, slack):
 
 
 @pytest.mark.parametrize("M,K,N", [(65, 128, 128), (80, 512, 640), (81, 4096, 4096), (112, 14336, 512), (113, 1024, 2048),
-                                   (127, 2048, 128), (128, 4096, 6144)])
-def test_rows_65_to_128(M, K, N):
+                                   (127, 2048, 128), (128, 4096, 6144), (33, 4096, 4096), (49, 1024, 640), (64, 14336, 512)])
+def test_rows_33_to_128(M, K, N):
     from umbrella_b200 import ops
     rng = np.random.default_rng(M + K + N)
     packed = ops.awq_repack(*(torch.from_numpy(t).to(DEV) for t in oawq.random_awq(K, N, 128, rng)))

@@ -276,7 +276,10 @@ struct GemmCfg {
     static constexpr int kPackedStride = 8576;              // record padded to a 128-byte multiple
     // epilogue staging: output tile + cos / sin rows (RoPE), for each group of warps that finishes tiles
     static constexpr int kExchBytes = 3 * 16 * 128 * 2;
-    static constexpr int kExchGroups = kSplit ? kDq + 1 : 1;
+    // (AWQ) all of them reduce the head of a split tile.  From four chunks of 16 columns on (a layer of width 4096 and its head:
+    // 40 rows 254 -> 237 us, 64 rows 262 -> 239); up to 32 rows are one or two chunks, hardly more than one group's turn.
+    static constexpr bool kShare = MPAD >= 64;
+    static constexpr int kExchGroups = kShare ? kDq + 1 : 1;
     // Independent fp32 accumulators in TMEM (columns a * MPAD): consecutive k-steps rotate through them so
     // that back-to-back tcgen05.mma never wait on each other's accumulate (a dependent 128xNx16 MMA chain
     // runs at its ~150-cycle latency, not at its 8-cycle issue rate); the epilogue sums them.
@@ -584,12 +587,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
     // the MMA warps take alternate units, so a ring stage must always come back to the same warp (parity waits, see the
     // dequant warps' note): both rings need an even depth
     static_assert(!kAwq || (kAStages % 2 == 0 && Cfg::kStagesAwq % 2 == 0), "ring depths must be even");
-    constexpr bool kSplit = kAwq && Cfg::kSplit, kXWarp = kAwq && Cfg::kXWarp;
+    constexpr bool kSplit = kAwq && Cfg::kSplit, kShare = kAwq && Cfg::kShare, kXWarp = kAwq && Cfg::kXWarp;
     static_assert(!kSplit || (kAStages % Cfg::kDq == 0 && Cfg::kWStages % Cfg::kDq == 0 && Cfg::kStagesAwq == kAStages),
                   "the rings of separate records must return each stage to its dequant group");
     const int kWRing = kSplit ? Cfg::kWStages : kStages;        // depth of the weight records' ring
     constexpr int kDq = Cfg::kDq;                               // dequant groups of this CTA
-    constexpr int kFinish = kSplit ? Cfg::kExchGroups : 1;      // groups of warps that reduce the head of a split tile
+    constexpr int kFinish = kShare ? Cfg::kExchGroups : 1;      // groups of warps that reduce the head of a split tile
 
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -604,7 +607,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
     uint64_t* acc_full = bars + 56;
     uint64_t* acc_empty = bars + 57;
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 58);
-    uint64_t* last_full = bars + 59;          //             kSplit: the last segment's accumulators are complete
+    uint64_t* last_full = bars + 59;          //             kShare: the last segment's accumulators are complete
     uint64_t* w_empty = bars + 60;            // [kWStages]  kSplit: the record in this stage is in the dequant group's registers
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -629,7 +632,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
         }
         for (int i = 0; i < kAStages; ++i) mbar_init(a_full + i, 4);
         mbar_init(acc_full, 2);
-        if (kSplit) mbar_init(last_full, 2);
+        if (kShare) mbar_init(last_full, 2);
         mbar_init(acc_empty, 4);
         fence_barrier_init();
     }
@@ -825,7 +828,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                         }
                         umma_commit(done + st);
                         if (last) umma_commit(acc_full);
-                        if (kSplit && last && seg_end == n_units) umma_commit(last_full);
+                        if (kShare && last && seg_end == n_units) umma_commit(last_full);
                     }
                 } else {
                     const uint32_t ws = smem_u32(s_w + st * kWStride);
@@ -855,7 +858,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
             if (first) {                     // this warp had no unit in the segment: plain arrival
                 if (elect_one()) {
                     mbar_arrive(acc_full);
-                    if (kSplit && seg_end == n_units) mbar_arrive(last_full);
+                    if (kShare && seg_end == n_units) mbar_arrive(last_full);
                 }
                 __syncwarp();
             }
@@ -1028,7 +1031,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                         }
                     }
                 }
-                if constexpr (kSplit) {
+                if constexpr (kShare) {
                     // The head of a split tile is reduced by all groups of warps, one chunk of 16 columns each in turn: a chunk
                     // waits for two or three round trips to the other CTAs' sums, 24 of them in series with one group
                     // when five CTAs share a tile (849 -> 683 us, see kSplit; four sums in flight a thread instead of two
