@@ -1,7 +1,10 @@
 """Tiny driver for ncu: the four AWQ GEMMs of one Llama-3.1-70B layer at M rows (default 13), the fp16 lm_head
 GEMM, the tree attention, the accept kernel and the KV gather -- two launches each (the second is profiled warm).
 
-    ncu --set full --clock-control none --import-source on -o gpurun_out/kernels_full -f python scripts/ncu_gemm.py
+    ncu --section SpeedOfLight --section MemoryWorkloadAnalysis --clock-control none -k regex:<one kernel> -s 1 -c 1 -o kernel -f \
+        python scripts/ncu_gemm.py
+
+Capture one kernel at a time, and only after the same command has run without ncu.
 """
 import os, sys
 import torch

@@ -1,4 +1,4 @@
-"""kernels_full.ncu-rep (scripts/ncu_gemm.py under `ncu --set full`) -> per-kernel summary text + the DRAM traffic
+"""kernels_full.ncu-rep (scripts/ncu_gemm.py under ncu) -> per-kernel summary text + the DRAM traffic
 per AWQ GEMM launch that bench.py reports as roofline.traffic.   python scripts/ncu_traffic.py REP OUT_TXT OUT_JSON"""
 import csv, io, json, subprocess, sys
 rep, out_txt, out_json = sys.argv[1:4]
@@ -22,7 +22,7 @@ for r in rows[2:]:
                  f"fma% {float(r[idx[cols[4]]]):5.1f} alu% {float(r[idx[cols[5]]]):5.1f} regs {r[idx[cols[6]]]} grid {r[idx[cols[7]]]} block {r[idx[cols[8]]]}")
     if "gemm_kernel<16, 1>" in name:
         awq.append((rd, wr))
-open(out_txt, "w").write("ncu --set full --clock-control none (cold caches, serialised): python scripts/ncu_gemm.py, M = 13\n"
+open(out_txt, "w").write("ncu --clock-control none (cold caches, serialised): python scripts/ncu_gemm.py, M = 13\n"
                          "AWQ launches in order: q|k|v x2, o x2, gate|up x2, down x2; then lm_head x2, tree attention x2, (accept, gather) x2\n"
                          + "\n".join(lines) + "\n")
 second = awq[1::2]                                   # the second launch of each shape
