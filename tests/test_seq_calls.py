@@ -1,0 +1,32 @@
+"""What the tensor-level calls and the model do around the native library, on the CPU with a library that only records."""
+import pytest
+import torch
+
+from umbrella_b200 import _lib_seq as S
+from umbrella_b200 import ops_seq as K
+
+
+class Recorder:
+    """Every entry point returns 0 and writes nothing."""
+
+    def __getattr__(self, name):
+        return lambda *a: 0
+
+
+@pytest.fixture
+def recorder(monkeypatch):
+    lib = Recorder()
+    monkeypatch.setattr(S, "load", lambda *a, **k: lib)
+    monkeypatch.setattr(K, "_stream", lambda: 0)
+    monkeypatch.setattr(K, "_mode", lambda t: S.UMBS_BF16)
+    dirty = lambda *a, **k: torch.full(a[0], 7.0, **k)               # memory that something else has used
+    monkeypatch.setattr(K.torch, "empty", dirty)
+    return lib
+
+
+@pytest.mark.parametrize("max_rows,cleared", [(None, False), (6, False), (5, True), (0, True)])
+def test_rows_that_a_product_is_told_to_leave_out_are_zero(recorder, max_rows, cleared):
+    a, w = torch.ones(6, 8, dtype=torch.bfloat16), torch.ones(4, 8, dtype=torch.bfloat16)
+    out = K.gemm(a, w, max_rows=max_rows)
+    assert bool((out == 0).all()) == cleared
+    assert K.gemm(a, w, rows=3, max_rows=2).eq(0).all()              # of the rows asked for, not of a's

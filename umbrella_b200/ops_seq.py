@@ -69,8 +69,8 @@ def gemm(a: torch.Tensor, w: torch.Tensor, *, out_f32: bool = False, groups: int
     N = (w3.shape[1] // (2 if dual else 1)) if n is None else n
     M = a.shape[0] if rows is None else rows
     cols = N if (groups == 1 or grp_off is not None) else groups * c_goff        # expert groups share the columns
-    # (zeros only where the product may leave gaps: rows behind the last group's, columns between the groups')
-    make = torch.empty if groups == 1 and grp_off is None else torch.zeros
+    # (zeros only where the product may leave gaps: rows behind max_rows or the last group's, columns between the groups')
+    make = torch.empty if groups == 1 and grp_off is None and (max_rows is None or max_rows >= M) else torch.zeros
     out = make((M, cols), dtype=torch.float32 if out_f32 else a.dtype, device=a.device)
     S.check(S.load().umbs_gemm(mode, _p(a), a.stride(0), a_goff, _p(w3), w3.stride(1), w3.stride(0), _p(out), out.stride(0),
                                c_goff, int(out_f32), M if max_rows is None else max_rows, N, K, groups, _p(grp_off),
