@@ -1,8 +1,8 @@
 #!/usr/bin/env python
-"""The reference's own GPU path timed on this box (SURVEY.md 8d, BASELINE.md 4) -- MEASUREMENT HARNESS ONLY.
+"""The reference's own GPU path timed on this box -- MEASUREMENT HARNESS ONLY.
 
 Runs the UNMODIFIED reference package from baseline/_ref (``pip install --no-index --no-deps --target baseline/_ref
-<copy of /root/reference>``, git-ignored, travels to the GPU box) through its own public classes
+<copy of the reference>``, git-ignored) through its own public classes
 (``StaticSpeculationEngine`` / ``AutoModelLM`` / ``LlamaAwq`` / ``LlamaCudagraph`` / ``KV_Cache``) on the same synthetic
 weights, prompt, tree and scripted acceptance as bench.py's own arm.  Nothing of umbrella_b200's engine, models or
 kernels is on the timed path; from this repo only the synthetic-weight generator, the growmap data and the scripted
@@ -21,9 +21,9 @@ packages, none of them touches reference source:
      built from the synthetic weights (tensor holders shaped like the HF modules the reference reads from)
   6. the tokenizer / GenerationConfig need hub files     -> token-id entry points only, eos list empty
 
-Variants (BASELINE.md 4): C = static engine, resident ``LlamaAwq`` target + ``LlamaCudagraph`` draft (the strongest
+Variants: C = static engine, resident ``LlamaAwq`` target + ``LlamaCudagraph`` draft (the strongest
 reference configuration on a 180 GB GPU).  A = ``LlamaAwqOffload`` with ``num_cache_layers = 0`` is reported by
-bench.py from our own paged model only (the reference's copy loop needs 35.6 GB of pinned host weights; see DESIGN.md).
+bench.py from our own paged model only (the reference's copy loop needs 35.6 GB of pinned host weights).
 """
 from __future__ import annotations
 

@@ -4,7 +4,7 @@
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference] [--workload NAME]
                     [--no-reference-gpu] [--with-offload]
 
-Workloads (BASELINE.json ``configs``) -- synthetic seeded weights of the real shapes, synthetic prompts,
+Workloads -- synthetic seeded weights of the real shapes, synthetic prompts,
 scripted acceptance with the reference's DEFAULT_ACC (random weights make draft and target uncorrelated):
 
   static70b      (default; the configuration the metric is quoted on, configs[2] / greedy_config_48gb.json)

@@ -1,4 +1,4 @@
-"""The request API over several GPUs (the reference's app/api.py runs one engine behind one port; SURVEY.md 8e / 8f-4:
+"""The request API over several GPUs (the reference's app/api.py runs one engine behind one port:
 one replica per GPU behind one front, no data-path collective).
 
     python examples/api_replicas.py --server --gpus 8 --port 65432 [--config configs/greedy_config_48gb.json]

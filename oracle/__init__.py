@@ -21,7 +21,7 @@ What is restated (all citations relative to the reference project's root, UMbreL
 * ``oracle.llama``      -- RMSNorm, RoPE, the Llama verify forward
                            (umbrella/models/llama.py:262-322, umbrella/models/model_utils.py:17-64)
 
-Pinning status (see DESIGN.md "Oracle"):
+Pinning status:
 
 * tree / accept / gather / mask / RoPE / attention: PINNED against outputs of the
   reference's own Python run on CPU in the build container
@@ -31,5 +31,5 @@ Pinning status (see DESIGN.md "Oracle"):
   ``vllm`` re-implementation of the AutoAWQ packer; the GEMM *arithmetic* of
   ``awq_ext.gemm_forward_cuda`` has no golden vector anywhere in the reference
   -> "parity unpinned" for that one function (restated from its published
-  algorithm; checked on the GPU box against vLLM's build of the same kernel).
+  algorithm; checked on a GPU against vLLM's build of the same kernel).
 """

@@ -9,7 +9,7 @@ The reference call site is ``AwqLinear.apply`` (umbrella/quantization/awq_utils.
 
 ``awq_ext`` is the un-vendored dependency autoawq-kernels==0.0.8 (requirements.txt:7); the tensor
 layout is defined by autoawq==0.2.7.post3 ``WQLinear_GEMM`` (requirements.txt:6).  Neither is in
-/root/reference, and the reference holds no golden vector for them -> the *arithmetic* below is
+the reference, and it holds no golden vector for them -> the *arithmetic* below is
 "parity unpinned": it restates the published algorithm
 
     W[k, 8c + j] = (nib(qweight[k, c], p_j) - nib(qzeros[k // g, c], p_j)) * scales[k // g, 8c + j]
@@ -110,7 +110,7 @@ def gemm_reference_emulated(x: np.ndarray, qweight, qzeros, scales, group: int,
 
 
 def random_awq(k: int, n: int, group: int, rng: np.random.Generator, scale: float = 0.003):
-    """Synthetic AWQ triplet with the statistics SURVEY.md 8(d) prescribes: uniform nibbles,
+    """Synthetic AWQ triplet with the usual statistics: uniform nibbles,
     scales = scale * (0.5 + U[0,1)) in fp16."""
     qw = rng.integers(0, 16, size=(k, n), dtype=np.int64)
     qz = rng.integers(0, 16, size=(k // group, n), dtype=np.int64)
@@ -122,7 +122,7 @@ def dequantize_torch(qweight, qzeros, scales, group: int, exact: bool = False):
     """Device-agnostic torch twin of ``dequantize`` (same nibble order): fp32 [K, N] holding either the
     fp16-rounded weights fp16((q - z) * s) -- what both upstream kernels feed their MMAs -- or, with
     ``exact=True``, the unrounded product (exact in fp32: a 5-bit integer times an 11-bit mantissa).
-    Used where the numpy version is too slow (70B-shape parity tests run the oracle on the GPU box)."""
+    Used where the numpy version is too slow (70B-shape parity tests run the oracle on a GPU)."""
     import torch
     shifts = torch.tensor([4 * int(p) for p in AWQ_NIBBLE_OF_COL], dtype=torch.int32, device=qweight.device)
     q = ((qweight.unsqueeze(-1) >> shifts) & 0xF).reshape(qweight.shape[0], -1)            # [K, N]

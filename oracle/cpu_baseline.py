@@ -10,7 +10,7 @@ umbrella/models/llama.py:262-303, umbrella/quantization/awq_utils.py:63-86).  Th
 over them with unit stride, a 16-entry fp16((q - z) * s) table per column and group, pthreads over column
 blocks; no dequantised matrix is materialised); RMSNorm, RoPE, masked GQA attention over the prefix and SiLU
 are torch CPU ops.  The reference itself has no CPU path (it is GPU compute with optional host-RAM weight
-paging, SURVEY.md 8d); this port is the closest CPU statement of the same arithmetic.  A full verify is 80
+paging); this port is the closest CPU statement of the same arithmetic.  A full verify is 80
 such layers + the fp16 lm_head; the sample is ONE layer (+ a 1/80 share of the lm_head), scaled by 80 and
 stated as such.
 """

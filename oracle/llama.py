@@ -3,7 +3,7 @@ points), plus a seeded synthetic-weight generator shared by tests and bench.
 
 TEST INFRASTRUCTURE ONLY -- see oracle/__init__.py.
 
-Restates (paths relative to /root/reference):
+Restates (paths within the reference project):
   * ``layer_norm`` -> flashinfer.rmsnorm          umbrella/models/model_utils.py:54-64
   * ``apply_rotary_pos_emb`` / ``rotate_half``    umbrella/models/model_utils.py:17-52
   * cos/sin tables                               umbrella/models/llama.py:237-249
@@ -116,7 +116,7 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
 
 
 # --------------------------------------------------------------------------------------
-# synthetic weights (SURVEY.md 8d): seeded, real shapes, value-independent timing
+# synthetic weights: seeded, real shapes, value-independent timing
 # --------------------------------------------------------------------------------------
 LINEAR_NAMES = ("wq", "wk", "wv", "wo", "gate_proj", "up_proj", "down_proj")
 
@@ -169,7 +169,7 @@ def dequant_fp16(qweight: torch.Tensor, qzeros: torch.Tensor, scales: torch.Tens
 
 # --------------------------------------------------------------------------------------
 # one decoder layer, functional and device-agnostic (the 70B-shape parity tests stream the layers
-# through it on the GPU box; OracleLlama below calls it with its own caches)
+# through it on a GPU; OracleLlama below calls it with its own caches)
 # --------------------------------------------------------------------------------------
 def _linear(x16: torch.Tensor, w32: torch.Tensor) -> torch.Tensor:
     return (x16.float() @ w32).to(torch.float16)

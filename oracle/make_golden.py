@@ -2,10 +2,10 @@
 """Generate tests/golden/* by running the REFERENCE's own Python on CPU.
 
 TEST INFRASTRUCTURE ONLY -- see oracle/__init__.py.  Run in the build container only
-(``python oracle/make_golden.py``): /root/reference does not exist on the GPU box, which is why
+(``python oracle/make_golden.py``): the reference is not there when the GPU tests run, which is why
 the outputs are committed as small fixtures.
 
-What is driven, unmodified, from /root/reference (read-only import, nothing copied):
+What is driven, unmodified, from the reference (read-only import, nothing copied):
   * umbrella.sequoia_utils.generate_sequoia_tree / successor_list_to_mask and the six shipped
     growmap JSONs                                                    -> trees.json
   * StaticSpeculationEngine.initialize/_prefill/build_tree/verify    -> accept_static.json
@@ -16,7 +16,7 @@ What is driven, unmodified, from /root/reference (read-only import, nothing copi
   * transformers' LlamaRotaryEmbedding (what llama.py:45-46 reads)   -> rope.npz (inv_freq)
   * vLLM's restatement of the AutoAWQ packer (awq_pack)              -> awq_pack.npz
 
-Shims needed to import the reference in this image (SURVEY.md 8c): ``awq``, ``awq_ext``,
+Shims needed to import the reference in this image: ``awq``, ``awq_ext``,
 ``matplotlib`` stubs; fake LMs ("bigram tables") stand in for the HF models; CUDA-graph helpers are
 replaced by their un-graphed bodies; device is "cpu".
 """

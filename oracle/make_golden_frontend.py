@@ -1,5 +1,5 @@
 """TEST INFRASTRUCTURE.  Front-end fixtures made by the reference's own code, so the product can be pinned byte for byte on
-a box without /root/reference:
+a machine without the reference:
   tests/golden/templates.json   the chat-template tables (umbrella/templates.py:1-47)
   tests/golden/wire.bin         what the reference's send_data (umbrella/api/api_utils.py:3-7) puts on a socket for the
                                 messages in tests/golden/wire.json (a request, a response, the greeting, terminate)

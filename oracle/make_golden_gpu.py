@@ -1,13 +1,13 @@
-"""Golden vectors for the AWQ arithmetic from the UPSTREAM KERNEL, generated on a GPU box.
+"""Golden vectors for the AWQ arithmetic from the UPSTREAM KERNEL, generated on a GPU.
 
 TEST INFRASTRUCTURE ONLY.  The reference calls ``awq_ext.gemm_forward_cuda`` / ``dequantize_weights_cuda``
 (umbrella/quantization/awq_utils.py:67-77) from autoawq-kernels==0.0.8, which is not in this image.  vLLM 0.22
 ships a build of the same upstream CUDA sources (device symbols ``vllm::awq::gemm_forward_4bit_cuda_m16nXk32``,
 ``vllm::awq::dequantize_weights``; python entry points ``vllm._custom_ops.awq_gemm / awq_dequantize``, same
 argument order and ``split_k_iters = 8`` as the reference's call).  This script runs those kernels on seeded AWQ
-triplets and writes ``gpurun_out/awq_upstream.npz``; the file is committed as ``tests/golden/awq_upstream.npz``:
+triplets and writes ``awq_upstream.npz`` into the folder that it is given; it is committed in tests/golden:
 
-    gpurun -- 'python oracle/make_golden_gpu.py'  &&  cp gpurun_out/awq_upstream.npz tests/golden/
+    python oracle/make_golden_gpu.py tests/golden
 """
 import os
 import sys
@@ -39,9 +39,9 @@ def main():
         out[pre + "qweight"], out[pre + "qzeros"], out[pre + "scales"], out[pre + "x"] = qweight, qzeros, scales, x
         out[pre + "dequant"] = deq.cpu().numpy()
         out[pre + "y"] = y.cpu().numpy()
-    os.makedirs("gpurun_out", exist_ok=True)
-    np.savez_compressed("gpurun_out/awq_upstream.npz", **out)
-    print("wrote gpurun_out/awq_upstream.npz", len(out), "arrays")
+    path = os.path.join(sys.argv[1] if len(sys.argv) > 1 else ".", "awq_upstream.npz")
+    np.savez_compressed(path, **out)
+    print("wrote", path, len(out), "arrays")
 
 
 if __name__ == "__main__":

@@ -3,7 +3,7 @@ tree node) in numpy float64.
 
 TEST INFRASTRUCTURE ONLY -- see oracle/__init__.py.
 
-Restates (paths relative to /root/reference):
+Restates (paths within the reference project):
 
   * ``apply_repetition_penalty``  umbrella/speculation/speculation_utils.py:340-345
   * ``apply_topk``                umbrella/speculation/speculation_utils.py:347-352
@@ -42,7 +42,7 @@ renormalised nucleus) -- same distribution, deterministic given the uniforms.  T
 deliberate difference and is what the product implements as well.
 
 No golden vector exists for either flashinfer function in the reference -> "parity unpinned" for the sampling
-arithmetic; the distribution is pinned on the GPU box against flashinfer 0.6.11's own
+arithmetic; the distribution is pinned on a GPU against flashinfer 0.6.11's own
 ``top_k_top_p_sampling_from_logits`` / ``top_p_renorm_probs`` (tests/test_gpu_sampling.py).
 """
 from __future__ import annotations
@@ -155,7 +155,7 @@ def argmax_penalised(logits: np.ndarray, penalty_ids, penalty: float) -> np.ndar
 def exact_distribution(logits_row: np.ndarray, temperature: float, top_k: int, top_p: float) -> np.ndarray:
     """The distribution both engines sample from (up to the static engine's bounded rejection rounds): the
     top-p nucleus of softmax(top-k(logits) / T), renormalised.  Used to pin the algorithm against flashinfer's own
-    samplers on the GPU box."""
+    samplers on a GPU."""
     probs = softmax(top_k_mask(np.asarray(logits_row, dtype=np.float64)[None] / temperature, top_k))[0]
     keep = nucleus(probs, top_p)
     pr = np.where(keep, probs, 0.0)

@@ -3,7 +3,7 @@
 TEST INFRASTRUCTURE ONLY -- see oracle/__init__.py.
 
 Every function cites the reference lines it restates (paths relative to
-/root/reference).  Everything here is integer / boolean work and must be
+the reference project).  Everything here is integer / boolean work and must be
 bit-exact with the reference; ``tests/test_oracle_tree.py`` pins it against
 fixtures produced by running the reference's own Python on CPU
 (``oracle/make_golden.py``).
@@ -305,7 +305,7 @@ def kv_gather(cache: np.ndarray, indices: np.ndarray, offset: int, seq_axis: int
 
 
 # --------------------------------------------------------------------------------------
-# scripted acceptance (benchmark input generator; SURVEY.md 8d) -- not a reference function
+# scripted acceptance (benchmark input generator) -- not a reference function
 # --------------------------------------------------------------------------------------
 def scripted_samples(successors: list[list[int]], spec_tokens: np.ndarray, rng: np.random.Generator,
                      acc=DEFAULT_ACC, vocab_hi: int = 30000) -> np.ndarray:

@@ -1,4 +1,4 @@
-"""What the request API costs on top of the engine: the default bench workload (70B-AWQ target + 1B
+"""What the request API costs on top of the engine (the default bench workload (70B-AWQ target + 1B
 draft, 3x4 tree, scripted acceptance, prompt 512 / generation 256) served over the socket -- APIClient -> ReplicaFront ->
 APIServer (engine on the server's worker thread) -- against the same requests through a direct engine.generate().
 

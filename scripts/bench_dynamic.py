@@ -1,4 +1,4 @@
-"""Dynamic (SpecExec) engine at full scale on one B200 -- BASELINE.json config 3 shapes:
+"""Dynamic (SpecExec) engine at full scale on one B200 -- the shapes of the dynamic configuration:
 Llama-3.1-70B-AWQ target + Llama-3.1-8B-AWQ draft, tree width x depth (+1) nodes, synthetic weights.
 Reports time per phase -- build_tree (depth + 1 draft forwards + tree growth kernels) and verify (chunked target
 forward over N rows + accept + gathers) -- and accepted tokens/s under scripted acceptance: random weights make draft

@@ -1,5 +1,5 @@
 """Pre-build the flashinfer JIT modules the reference-kernel comparator (tests/refkernels.py) and the reference
-arm of bench.py call, for sm_100a, into baseline/fi_ws (git-ignored, travels to the GPU box with the snapshot).
+arm of bench.py call, for sm_100a, into baseline/fi_ws (git-ignored).
 nvcc cross-compiles them without a GPU.  Run once per container:
 
     python scripts/build_flashinfer_modules.py

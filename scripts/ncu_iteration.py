@@ -5,7 +5,7 @@ profiled (the synthetic-weight generation is not).  LAYERS trims the target's de
 to keep the capture short; the per-layer kernel sequence is what is being listed.
 
     ncu --profile-from-start off --metrics gpu__time_duration.sum --clock-control none --csv \
-        --log-file gpurun_out/launches.csv python scripts/ncu_iteration.py
+        --log-file launches.csv python scripts/ncu_iteration.py
 """
 import os
 import sys

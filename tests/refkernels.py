@@ -1,6 +1,6 @@
 """The reference's OWN GPU kernels, op by op -- the second comparator of the forward parity tests.
 
-TEST INFRASTRUCTURE ONLY (GPU box).  The reference forward (umbrella/models/llama.py:262-322) is plain
+TEST INFRASTRUCTURE ONLY.  The reference forward (umbrella/models/llama.py:262-322) is plain
 torch glue around three third-party kernels; this module restates that glue and calls the same kernels:
 
   * ``AwqLinear.apply`` (umbrella/quantization/awq_utils.py:63-86) -> ``awq_ext.gemm_forward_cuda(x, qweight,
@@ -15,7 +15,7 @@ torch glue around three third-party kernels; this module restates that glue and 
   * RoPE, SiLU, residual adds, lm_head: the reference's own torch fp16 ops, restated verbatim.
 
 flashinfer JIT-compiles its modules; they are pre-built for sm_100a into baseline/fi_ws (git-ignored, travels to
-the GPU box) by scripts/build_flashinfer_modules.py, and FLASHINFER_WORKSPACE_BASE points there.
+the GPU machine) by scripts/build_flashinfer_modules.py, and FLASHINFER_WORKSPACE_BASE points there.
 """
 from __future__ import annotations
 

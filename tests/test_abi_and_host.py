@@ -69,7 +69,7 @@ def test_no_cpu_fallback_and_no_oracle_in_product():
 
 
 def test_reference_import_paths():
-    """`umbrella` resolves to this package with the reference's module layout (SURVEY.md 8b)."""
+    """`umbrella` resolves to this package with the reference's module layout."""
     import umbrella
     from umbrella.models.auto_model import AutoModelLM                                # noqa: F401
     from umbrella.sequoia_utils import generate_sequoia_tree                            # noqa: F401
@@ -141,7 +141,7 @@ def test_product_sequoia_utils_match_reference_fixtures():
 
 
 def test_engines_refuse_states_without_room_for_the_tree():
-    """the kernels write tree_size rows past num_nodes (505 for the shipped dynamic config), far more
+    """The kernels write tree_size rows past num_nodes (505 for the shipped dynamic config), far more
     than safe_buffer; validate_status / _prefill / _append must refuse such states on the host."""
     from umbrella_b200.speculation.dynamic_speculation_engine import DynamicSpeculationEngine
     from umbrella_b200.speculation.static_speculation_engine import StaticSpeculationEngine
@@ -168,7 +168,7 @@ def test_engines_refuse_states_without_room_for_the_tree():
 def test_checkpoint_reader_round_trip(tmp_path):
     """models/checkpoint.py: a synthetic model written in the Hugging Face / AutoAWQ safetensors layout reads back
     tensor-for-tensor, config.json gives the shape back, and a model without a checkpoint refuses to allocate
-    unless synthetic weights are asked for (ADVICE r1)."""
+    unless synthetic weights are asked for."""
     import torch
     from umbrella_b200.models import checkpoint as ck
     from umbrella_b200.models import llama as L
@@ -226,7 +226,7 @@ def test_budget_tree_is_the_best_tree_of_its_size():
     assert same_depth["size"] == 16 and max(same_depth["depth"]) == max(shipped["depth"])   # same number of draft levels
     assert expected_accept_length(same_depth) > expected_accept_length(shipped) * 1.06
     assert expected_accept_length(generate_budget_tree(13, 4)) >= expected_accept_length(generate_sequoia_tree(3, 4))
-    # the packaged tuned tree is the optimum of the measured two-parameter cost model (DESIGN.md 5): one level fewer
+    # the packaged tuned tree is the optimum of the measured two-parameter cost model: one level fewer
     tuned, rate = tune_budget_tree(16, fixed_ms=10.0, draft_forward_ms=1.05)
     assert load_growmap("b200_sequoia_tree-16.json")["Successors"] == tuned["Successors"]
     assert tuned["size"] == 16 and max(tuned["depth"]) == 3
@@ -449,7 +449,7 @@ def test_graph_inference_surface():
 
 
 def test_packaged_configs_build_engines():
-    """configs/*.json (the BASELINE workloads in the reference's config schema) go through AutoEngine.from_config; the
+    """configs/*.json (the workloads in the reference's config schema) go through AutoEngine.from_config; the
     trees they name are packaged."""
     import glob
     import json

@@ -1,4 +1,4 @@
-"""Request API (SURVEY.md 8b "API wire", 8f-4 multi-replica front): wire format against the reference's byte layout,
+"""Request API : wire format against the reference's byte layout,
 server / client behaviour, placement over replicas.  CPU only: the engines here are stand-ins with the engine's
 ``generate(**api_args) -> dict`` contract (umbrella/speculation/static_speculation_engine.py:429-434)."""
 import json
@@ -271,7 +271,7 @@ def test_text_colors_and_logger():
 
 
 def test_reference_import_paths_resolve():
-    """every ``umbrella`` import statement of the reference's app/*.py and examples/*.py."""
+    """Every ``umbrella`` import statement of the reference's app/*.py and examples/*.py."""
     statements = [
         "from umbrella.api.client import APIClient",
         "from umbrella.api.server import APIServer",

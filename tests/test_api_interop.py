@@ -1,5 +1,5 @@
-"""Interoperation with the reference's own API code (SURVEY.md 8b "API wire"): its client against this server, this
-client and the replica front against its server.  The reference runs in subprocesses from /root/reference (read-only,
+"""Interoperation with the reference's own API code : its client against this server, this
+client and the replica front against its server.  The reference runs in subprocesses from its own folder (read-only,
 present in the build container only -- skipped elsewhere); engines are stand-ins on both sides."""
 import json
 import os

@@ -1,6 +1,6 @@
 """GPU parity: the static speculative-decoding engine end to end on small synthetic models.
 
-Losslessness KAT (SURVEY.md 8c): greedy speculative decoding must emit exactly the tokens of plain
+Losslessness KAT: greedy speculative decoding must emit exactly the tokens of plain
 greedy autoregressive decoding of the target model -- checked bit-exactly against an AR loop over
 the same CUDA forward, and against the CPU oracle model wherever the oracle's top-2 margin is safe.
 Also replays scripted acceptance and checks accept lengths against the oracle's verify_step."""
@@ -192,7 +192,7 @@ def test_lazy_leaf_kv_keeps_draft_quality():
 
 
 def test_append_after_lazily_skipped_leaf_row():
-    """with lazy_leaf_kv the draft K/V row of an accepted last-level node is written by the NEXT
+    """With lazy_leaf_kv the draft K/V row of an accepted last-level node is written by the NEXT
     build_tree; a multi-turn ``_append`` in between must re-derive it.  After appends that follow leaf accepts, every
     committed row of the draft cache must equal (fp16 noise) what a fresh causal pass over the same tokens gives --
     a stale row (never written, or holding another tree node's K/V) is far outside that tolerance."""

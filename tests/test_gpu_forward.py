@@ -2,7 +2,7 @@
   * the oracle (oracle/llama.py: the reference's op order, fp32 maths, the reference's fp16 rounding points), run on
     the device through the same streaming helper as the 70B-shape test, and
   * the reference's own kernels (tests/refkernels.py).
-north_star tolerance: target logits within 1e-3 -- read relative to max|logit| (one fp16 ulp of the top logit is
+Tolerance: target logits within 1e-3 -- read relative to max|logit| (one fp16 ulp of the top logit is
 already 4.9e-4 .. 9.8e-4 of it) -- or, where the reference's own kernels sit farther than that from the same oracle on the
 same inputs, their measured distance; arg-max equal wherever the oracle's top-2 margin exceeds twice the bound."""
 import json

@@ -2,7 +2,7 @@
 (oracle/awq.py).  Tolerances: the kernel rounds (q - z) * s to fp16 exactly like the reference
 kernels (bit-exact, checked through the unpack), accumulates in fp32 in tensor memory and rounds the
 result once to fp16, so it must sit within a few fp16 ulps of ``gemm_fp16_weights`` -- far inside
-north_star's 1e-3."""
+the 1e-3 that is asked for."""
 import os
 
 import numpy as np

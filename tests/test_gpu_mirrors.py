@@ -1,4 +1,4 @@
-"""GPU parity through the reference's own class surface: ``AwqLinear`` (umbrella/quantization/
+"""GPU parity through the reference's own class surface : ``AwqLinear`` (umbrella/quantization/
 awq_utils.py:5-86) and ``KV_Cache`` (umbrella/attn/cache.py:5-96) used the way LlamaAwq.layer_compute uses them,
 checked against the oracle -- including the edge cases the seams imply (bias, > 128 rows, paging through
 ``copy``, empty accept path, append semantics that ignore the values of storage_ids)."""
@@ -101,14 +101,14 @@ def test_kv_cache_class_seams():
     for layer in range(3):
         ref = oattn.masked_gqa_attention(q[0], k_all[layer], v_all[layer], mask[:, :P + N])
         assert np.abs(outs[layer] - ref).max() <= 2e-3 * max(1.0, np.abs(ref).max())
-    # accept path [0, 2, 6]: overlapping source / destination rows (SURVEY.md 9.5), then the tail is zeroed
+    # accept path [0, 2, 6]: overlapping source / destination rows, then the tail is zeroed
     want_k = cache.k_cache.cpu().numpy().copy()
     idx = np.array([P + 0, P + 2, P + 6])
     new_off = otree.kv_gather(want_k, idx, P)
     cache.gather_kv_incremental(torch.from_numpy(idx).to(DEV), P)
     assert cache.kv_offset == new_off == P + 3
     assert np.array_equal(cache.k_cache.cpu().numpy(), want_k)
-    # empty accept path (EOS at the root, SURVEY.md 9.7)
+    # empty accept path (EOS at the root)
     cache.gather_kv_incremental(torch.zeros(0, dtype=torch.int64, device=DEV), cache.kv_offset)
     assert cache.kv_offset == P + 3
     cache.clear()

@@ -1,4 +1,4 @@
-"""GPU parity at the BASELINE shape: the native verify forward at Llama-3.1-70B dimensions
+"""GPU parity at the headline shape: the native verify forward at Llama-3.1-70B dimensions
 (H = 8192, I = 28672, 64 / 8 heads, V = 128256) against
 
   (b) the fp32 oracle (oracle/llama.py: the reference's op order, fp32 maths, the reference's fp16 rounding
@@ -6,9 +6,9 @@
   (c) the reference's own kernels on the same inputs (tests/refkernels.py: vLLM's build of the upstream AWQ GEMM,
       flashinfer single_prefill_with_kv_cache(custom_mask) and flashinfer.rmsnorm, glued as llama.py:262-322).
 
-north_star tolerance: logits within 1e-3, read relative to max|logit| -- or, where the reference's own
+Tolerance: logits within 1e-3, read relative to max|logit| -- or, where the reference's own
 kernels sit farther than that from the fp32 oracle, the measured reference noise (both distances are printed and
-written to gpurun_out/parity70b_<layers>.json).
+written to parity70b_<layers>.json).
 
 Also here: every fused full-width GEMM of a 70B layer (q|k|v N = 10240, gate|up N = 57344 with the SiLU epilogue,
 o, down) against the oracle's dequantiser (validated against the numpy oracle on CPU), not against the kernel's
@@ -28,7 +28,7 @@ from oracle import tree as otree
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 GOLDEN = os.path.join(os.path.dirname(__file__), "golden")
-TOL = 1e-3                      # north_star: "target logits matching the reference within 1e-3 fp16"
+TOL = 1e-3                      # target logits match the reference within 1e-3 (fp16)
 
 
 def _tree():
@@ -85,7 +85,7 @@ def test_70b_shape_logits_vs_oracle_and_reference_kernels(layers):
     json.dump(rec, open(f"gpurun_out/parity70b_{layers}.json", "w"), indent=1)
 
     # yardstick: the fp32 oracle with the reference's rounding points (fp16-rounded weights, as both the upstream kernel
-    # and the product feed their MMAs); bar: north_star's 1e-3 or, where the reference's own kernels sit farther than that
+    # and the product feed their MMAs); bar: the 1e-3 that is asked for or, where the reference's own kernels sit farther than that
     # from the same oracle, their measured distance.  (The exact-weight oracle's distances are in the record too.)
     bound = max(TOL, rec.get("reference_kernels_vs_fp32_oracle", 0.0))
     assert rec["ours_vs_fp32_oracle"] <= bound, rec

@@ -133,7 +133,7 @@ def test_kv_gather(layout):
         offset = int(rng.integers(1, 40))
         m = int(rng.integers(0, 20))
         idx = np.sort(rng.choice(np.arange(offset, offset + 40), size=m, replace=False)).astype(np.int64)
-        # includes the hazard of SURVEY 9-5 when idx[k] == offset + j for k < j
+        # includes the hazard of overlapping rows when idx[k] == offset + j for k < j
         zero_tail = trial % 2 == 0
         k_ref, v_ref = k.copy(), v.copy()
         otree.kv_gather(k_ref, idx, offset, seq_axis, zero_tail)

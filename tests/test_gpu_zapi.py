@@ -1,4 +1,4 @@
-"""GPU: the request API in front of a real engine (SURVEY.md 8b "API wire", 8f-4).  A request served over the socket
+"""GPU: the request API in front of a real engine .  A request served over the socket
 by ``APIServer`` -- engine built and driven on the server's worker thread, CUDA graph of the iteration captured there --
 must return exactly the tokens of a direct ``engine.generate`` call, also through the replica front."""
 import pytest

@@ -107,7 +107,7 @@ def _greedy_ar(model, prompt, steps):
 
 def test_tree_verify_is_lossless_on_oracle_model(golden_dir):
     """KAT for the whole path: verify over a Sequoia tree whose nodes hold arbitrary tokens accepts
-    exactly the greedy continuation (SURVEY.md 8c 'losslessness')."""
+    exactly the greedy continuation ."""
     import json
     succ = json.load(open(os.path.join(golden_dir, "trees.json")))["shipped"]["sequoia_tree-3x4.json"]["Successors"]
     parents = T.successors_to_parents(succ)
@@ -163,7 +163,7 @@ def test_awq_oracle_matches_upstream_kernel(golden_dir):
     emulation of its rounding and the exact-accumulation form both sit within fp16 noise of it."""
     path = os.path.join(golden_dir, "awq_upstream.npz")
     if not os.path.exists(path):
-        pytest.skip("awq_upstream.npz not generated yet (needs a GPU box)")
+        pytest.skip("awq_upstream.npz not generated yet (needs a GPU)")
     z = np.load(path)
     ci = 0
     while "c%d_meta" % ci in z:

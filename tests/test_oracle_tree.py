@@ -40,7 +40,7 @@ def test_generate_sequoia_tree_matches_reference(trees):
             g = T.generate_sequoia_tree(w, d)
         assert g["Successors"] == ref["Successors"], key
         assert canon_hash(g) == ref["all_sha256"], key
-    # the shipped 3x4 growmap is exactly generate_sequoia_tree(3, 4) (SURVEY.md 4)
+    # the shipped 3x4 growmap is exactly generate_sequoia_tree(3, 4)
     assert canon_hash(T.generate_sequoia_tree(3, 4)) == trees["shipped"]["sequoia_tree-3x4.json"]["all_sha256"]
 
 
@@ -193,7 +193,7 @@ def test_mask_windows_equal_compact_form(trees):
 
 
 def test_gather_overlap_hazard():
-    """path [0,2,6] -> row n+2 is both a source (for slot 1) and a destination."""
+    """Path [0,2,6] -> row n+2 is both a source (for slot 1) and a destination."""
     cache = np.arange(2 * 32, dtype=np.float64).reshape(2, 32, 1, 1)
     ref = cache.copy()
     n = 10

@@ -1,4 +1,4 @@
-"""Drop-in alias: ``import umbrella...`` resolves to ``umbrella_b200...`` (SURVEY.md 8b -- the reference's
+"""Drop-in alias: ``import umbrella...`` resolves to ``umbrella_b200...`` (the reference's
 front-ends import ``umbrella.speculation.auto_engine.AutoEngine`` etc.).  No code lives here."""
 import importlib
 import importlib.abc

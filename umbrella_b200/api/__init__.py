@@ -1,2 +1,2 @@
 """Request front of the engines: the reference's socket protocol (umbrella/api/) and, above it, a front that spreads
-independent requests over one engine per GPU (SURVEY.md 8e / 8f-4: replicas only, no data-path collective)."""
+independent requests over one engine per GPU (replicas only, no data-path collective)."""

@@ -1,4 +1,4 @@
-"""Multi-replica request front (SURVEY.md 8e / 8f-4): N independent engines, one per GPU, behind one port.
+"""Multi-replica request front: N independent engines, one per GPU, behind one port.
 
 A request's speculative-decoding loop is a sequential chain over private state and the reference never shards inside a
 request (umbrella/api/server.py:43-49 serialises requests on its one engine), so an 8-GPU box serves eight requests at a

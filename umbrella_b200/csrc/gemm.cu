@@ -1381,7 +1381,7 @@ static unsigned long long* trace_for_this_launch() {
     return (want < 0 || idx == want) ? buf : nullptr;
 }
 
-// Rows one launch takes (internal.h: UMB_MAX_ROWS; 64 splits 65..128 rows into two launches as round 1 did).
+// Rows one launch takes (internal.h: UMB_MAX_ROWS; 64 splits 65..128 rows into two launches).
 constexpr int kMaxRowsPerLaunch = UMB_MAX_ROWS;
 static int mpad_of(int M) { return M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128)); }
 

@@ -1,5 +1,5 @@
 // Fused target-side sampling of verify(): repetition penalty + top-k + softmax(T) + top-p + one sample per tree
-// node, one CTA per node, straight from the fp32 logits the lm_head GEMM wrote (SURVEY.md 8f-3).
+// node, one CTA per node, straight from the fp32 logits the lm_head GEMM wrote.
 //
 // Replaces (reference paths):
 //   apply_repetition_penalty            umbrella/speculation/speculation_utils.py:340-345

@@ -1,10 +1,10 @@
 """AutoModelLM: name -> model class (mirror of reference umbrella/models/auto_model.py:9-182 for the
-Llama entries; the Qwen/Mistral/Gemma tables are out of scope, SURVEY.md 2.1 #6).
+Llama entries; the Qwen/Mistral/Gemma tables are out of scope).
 
 ``alloc()`` loads the model's safetensors checkpoint (fp16 or AutoAWQ INT4) from a local directory or the Hugging
 Face cache through models/checkpoint.py -- no ``autoawq`` / ``gptqmodel`` needed -- and raises ``CheckpointNotFound``
 when there is none.  Synthetic seeded weights of the architecture (there are no real weights and no network in this
-environment; SURVEY.md 8d) are strictly opt-in: ``alloc(synthetic=True)`` or a ``"synthetic": true`` /
+environment) are strictly opt-in: ``alloc(synthetic=True)`` or a ``"synthetic": true`` /
 ``"synthetic_seed": N`` key in the engine config.  ``model_name`` may also be a checkpoint directory of a Llama
 architecture that is not in the table (its config.json supplies the shape).
 """

@@ -1,4 +1,4 @@
-"""Host-resident KV pages: the K/V planes of the upper ``kv_host_layers`` decoder
+"""Host-resident KV pages : the K/V planes of the upper ``kv_host_layers`` decoder
 layers live in pinned host memory and are streamed through two device staging planes, layer by layer, with
 ``cudaMemcpyAsync`` on a side stream ordered by events -- the weight pager's scheme (models/offload.py) applied to the
 cache.  The reference keeps the whole cache on the device (umbrella/attn/cache.py:18-34: ``[L, S, Hkv, D]`` per K / V,

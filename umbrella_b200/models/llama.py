@@ -6,8 +6,8 @@ Host-side mirror of the reference's ``Llama`` / ``LlamaAwq`` (umbrella/models/ll
 (``layer_compute``) is gone: one C call enqueues the whole forward on the current stream.
 
 Weights come from one of two sources:
-  * synthetic, seeded, real shapes (there are no checkpoints and no network in this environment;
-    SURVEY.md 8d) -- ``SyntheticLlama``;
+  * synthetic, seeded, real shapes (there are no checkpoints and no network in this environment)
+    -- ``SyntheticLlama``;
   * tensors handed in by a loader (``load_awq_layer`` / ``load_fp16_layer``), the seam where
     ``LlamaAwqLayer.init_parameters`` (umbrella/models/llama_layer.py:165-218) plugs in.
 """
@@ -363,7 +363,7 @@ class LlamaAwq(Llama):
 
 
 # --------------------------------------------------------------------------------------------
-# synthetic weights (SURVEY.md 8d): seeded, real shapes; value-independent timing
+# synthetic weights: seeded, real shapes; value-independent timing
 # --------------------------------------------------------------------------------------------
 LINEAR_NAMES = ("wq", "wk", "wv", "wo", "gate_proj", "up_proj", "down_proj")
 

@@ -1,4 +1,4 @@
-"""Weight paging: host-resident layers streamed through device staging slabs.
+"""Weight paging: host-resident layers streamed through device staging slabs .
 
 Host-side mirror of the reference's ``LlamaOffload`` / ``LlamaAwqOffload`` (umbrella/models/llama.py:
 145-219, 324-409; umbrella/models/llama_layer.py:220-258; umbrella/quantization/awq_utils.py:24-26,

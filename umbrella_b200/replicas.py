@@ -1,9 +1,9 @@
-"""One replica per GPU (SURVEY.md 8e): request stream i -> rank i % world, no data-path collective.
+"""One replica per GPU: request stream i -> rank i % world, no data-path collective.
 
 A request's speculative-decoding loop is a strictly sequential chain over private state, and the
 reference never shards inside a request, so N GPUs run N independent engines.  ``torch.distributed``
 is plumbing here: a barrier around the timed region and the reduction of the per-rank timings
-(MAX of times, SUM of token counts) -- the same code under ``nccl`` on the GPU box and ``gloo`` in
+(MAX of times, SUM of token counts) -- the same code under ``nccl`` on a GPU and ``gloo`` in
 the CPU tests.
 """
 from __future__ import annotations
@@ -45,7 +45,7 @@ def reduce_over_replicas(times: list[float], counts: list[float], device=None):
 
 
 def gather_over_replicas(values: list[float], device=None) -> list[list[float]]:
-    """Every replica's ``values`` (one list per rank, rank order) -- the per-replica min / max SURVEY.md 8e asks for."""
+    """Every replica's ``values`` (one list per rank, rank order) -- the per-replica min / max a report of the spread needs."""
     import torch
     import torch.distributed as dist
     if not (dist.is_available() and dist.is_initialized()) or dist.get_world_size() == 1:

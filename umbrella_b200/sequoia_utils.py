@@ -124,7 +124,7 @@ def tune_budget_tree(budget: int, fixed_ms: float, draft_forward_ms: float, acc:
     draft forward of ``draft_forward_ms`` per level below the root that is fed to the draft model (the leaf level is
     not, with the lazily computed leaf K/V).  Returns (growmap, predicted tokens per second).
 
-    Measured on a B200 for the 70B-AWQ target + 1B draft: fixed 10.0 ms, 1.05 ms per draft forward ->
+    Measured on a B200 for the 70B-AWQ target + 1B draft : fixed 10.0 ms, 1.05 ms per draft forward ->
     depth 3, ``b200_sequoia_tree-16.json`` (packaged): 3.43 expected tokens per verify in 13.2 ms against 3.36 in 14.2 ms
     for ``sequoia_tree-3x4.json`` (13 nodes, depth 4)."""
     best, best_rate = None, -1.0

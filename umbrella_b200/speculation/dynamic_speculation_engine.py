@@ -1,7 +1,7 @@
 """DynamicSpeculationEngine: SpecExec-style dynamic-tree speculative decoding on the sm_100a verify path.
 
 Host-side mirror of reference umbrella/speculation/dynamic_speculation_engine.py (same constructor
-kwargs ``width / num_beams / depth``, same BaseEngine surface, same bookkeeping), SURVEY.md 8a row a2:
+kwargs ``width / num_beams / depth``, same BaseEngine surface, same bookkeeping):
 
   * build_tree() (dynamic...:215-248): ``depth + 1`` draft forwards (1 row, then ``width`` rows per
     level); after each one the draft's top-``num_beams`` logits go through ONE kernel
@@ -47,7 +47,7 @@ class DynamicSpeculationEngine(BaseEngine):
         self.tree_width = kwargs.pop("width", 16)
         self.tree_depth = kwargs.pop("depth", 24)
         self.config = kwargs
-        self.acceptance_script = None      # benchmark hook: callable(engine, sampled) -> sampled (SURVEY.md 8d)
+        self.acceptance_script = None      # benchmark hook: callable(engine, sampled) -> sampled
         self.draft_model = None
         self.target_model = None
         self.stats = {"verify_calls": 0}

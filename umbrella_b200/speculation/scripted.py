@@ -1,4 +1,4 @@
-"""Scripted acceptance for benchmarks on synthetic weights (SURVEY.md 8d).
+"""Scripted acceptance for benchmarks on synthetic weights.
 
 Random-init draft and target models are uncorrelated, so "accepted tokens/sec" would degenerate to
 one token per verify.  The script replaces the target's sampled token at every tree node, AFTER the

@@ -2,7 +2,7 @@
 
 Host-side mirror of reference umbrella/speculation/static_speculation_engine.py (same constructor
 kwargs, same 13-method BaseEngine surface, same return values and bookkeeping), with the inner loop
-replaced (SURVEY.md 8a, rows a1/a12-a15):
+replaced:
 
   * verify(): one native target forward over the token tree (umb_llama_forward: AWQ tcgen05 GEMMs,
     tree attention with (prefix_len, ancestor bitmask) instead of the O(S^2) master mask, arg-max
@@ -44,7 +44,7 @@ class StaticSpeculationEngine(BaseEngine):
         self.repetition_penalty = kwargs.pop("repetition_penalty", 1.0)
         self.topk = kwargs.pop("topk", 32)
         self.config = kwargs
-        self.acceptance_script = None      # benchmark hook: callable(engine, sampled) -> sampled (SURVEY.md 8d)
+        self.acceptance_script = None      # benchmark hook: callable(engine, sampled) -> sampled
         # One CUDA graph per speculative-decoding iteration (all draft levels + verify + accept + gathers):
         # the reference graphs only the draft forward (llama.py:505-533); here the whole iteration is one
         # launch and the host reads back 3 ints.  Greedy decoding only; other settings run eagerly.
