@@ -665,8 +665,18 @@ __device__ __forceinline__ float router_logit(const T* hr, const float* w, int w
 // arg-max over the groups mark the eligible ones; `top` rounds of arg-max over the eligible scores; weights = score / sum.
 // UMBS_ROUTE_SOFTMAX_ALL: the softmax's sum runs over every expert, the chosen scores are not renormalised.
 // Every weight is multiplied by wscale at the end.
+// A score that compares with nothing (a token with a NaN, or what is left is all -infinity) is chosen last: the lowest place
+// that has not been chosen, so that every choice is an expert of its own whatever the token holds.
+__device__ __forceinline__ int lowest_not_in(const int32_t* chosen, int n, int lo, int hi) {
+    for (int e = lo; e < hi; ++e) {
+        bool taken = false;
+        for (int i = 0; i < n; ++i) taken |= chosen[i] == e;
+        if (!taken) return e;
+    }
+    return -1;
+}
 __device__ __forceinline__ void route_choose(float* z, int experts, int top, int mode, int groups, int keep, float wscale,
-                                             float* __restrict__ w_out, int32_t* __restrict__ e_out, int32_t* counts) {
+                                             float* __restrict__ w_out, int32_t* e_out, int32_t* counts) {
     if (mode == UMBS_ROUTE_SIGMOID_GROUPS) {
         const int per = experts / groups;
         for (int e = 0; e < experts; ++e) z[e] = 1.f / (1.f + expf(-z[e]));
@@ -685,6 +695,8 @@ __device__ __forceinline__ void route_choose(float* z, int experts, int top, int
                 const float gs = per > 1 ? a + b2 : a;
                 if (gs > bv) { bv = gs; best = g; }
             }
+            for (int g = 0; best < 0 && g < groups; ++g)
+                if (!((kept >> g) & 1ull)) best = g;
             if (best >= 0) kept |= 1ull << best;
         }
         float den = 0.f;
@@ -693,6 +705,12 @@ __device__ __forceinline__ void route_choose(float* z, int experts, int top, int
             float bv = -INFINITY;
             for (int e = 0; e < experts; ++e)
                 if (((kept >> (e / per)) & 1ull) && z[e] > bv) { bv = z[e]; best = e; }
+            if (best < 0) {
+                for (int g = 0; best < 0 && g < groups; ++g)
+                    if ((kept >> g) & 1ull) best = lowest_not_in(e_out, k, g * per, (g + 1) * per);
+                if (best < 0) best = lowest_not_in(e_out, k, 0, experts);
+                bv = z[best];                                          // (a NaN: the token's weights are)
+            }
             e_out[k] = best;
             w_out[k] = bv;
             den += bv;
@@ -709,10 +727,11 @@ __device__ __forceinline__ void route_choose(float* z, int experts, int top, int
         for (int e = 0; e < experts; ++e) den += expf(z[e] - zmax);
     }
     for (int k = 0; k < top; ++k) {
-        int best = 0;
+        int best = -1;
         float bv = -INFINITY;
         for (int e = 0; e < experts; ++e)
             if (z[e] > bv) { bv = z[e]; best = e; }
+        if (best < 0) best = lowest_not_in(e_out, k, 0, experts);
         if (k == 0 && mode != UMBS_ROUTE_SOFTMAX_ALL) zmax = bv;
         const float p = expf(bv - zmax);
         e_out[k] = best;
