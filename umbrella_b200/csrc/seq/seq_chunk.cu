@@ -161,8 +161,8 @@ __global__ void __launch_bounds__(256, 2) chunk_memory_kernel(const ChunkMemory 
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
                     const int far = ti + i - (tj + j);
-                    const float f = GATES ? sh.p[tj + j][ti + i] : (far < 0 ? 0.f : (far == 0 ? 1.f : sh.lam[far - 1]));
-                    sh.p[tj + j][ti + i] = acc[i][j] * f;
+                    const float f = GATES ? sh.p[tj + j][ti + i] : (far <= 0 ? 1.f : sh.lam[far - 1]);
+                    sh.p[tj + j][ti + i] = far < 0 ? 0.f : acc[i][j] * f;   // (chosen, not multiplied by 0: a later token's NaN stays its own)
                 }
         }
         __syncthreads();
@@ -188,15 +188,26 @@ __global__ void __launch_bounds__(256, 2) chunk_memory_kernel(const ChunkMemory 
                     acc[i][0] = mul2(acc[i][0], pack2(f, f));
                     acc[i][1] = mul2(acc[i][1], pack2(f, f));
                 }
-                const int jn = min(nb, i0 + 4);
 #pragma unroll 4
-                for (int j = 0; j < jn; ++j) {
+                for (int j = 0; j < i0; ++j) {                          // tokens that all four rows see
                     const float4 pv4 = *reinterpret_cast<const float4*>(&sh.p[j][i0]);
                     const ulonglong2 vv = ld2(&sh.v[j][c]);
                     const float pp[4] = {pv4.x, pv4.y, pv4.z, pv4.w};
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const f32x2 q2 = pack2(pp[i], pp[i]);
+                        acc[i][0] = fma2(q2, vv.x, acc[i][0]);
+                        acc[i][1] = fma2(q2, vv.y, acc[i][1]);
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {                           // the rows' own tokens: seen by themselves and the rows behind
+                    if (i0 + e >= nb) break;
+                    const ulonglong2 vv = ld2(&sh.v[i0 + e][c]);
+#pragma unroll
+                    for (int i = e; i < 4; ++i) {
+                        const float w = sh.p[i0 + e][i0 + i];
+                        const f32x2 q2 = pack2(w, w);
                         acc[i][0] = fma2(q2, vv.x, acc[i][0]);
                         acc[i][1] = fma2(q2, vv.y, acc[i][1]);
                     }
