@@ -39,6 +39,7 @@ typedef void* umb_stream_t; /* cudaStream_t */
 #define UMB_ERR_UNSUPPORTED (-2) /* shape or option outside what the kernels implement */
 #define UMB_ERR_WORKSPACE (-3)   /* workspace too small */
 #define UMB_ERR_DRIVER (-4)      /* driver entry point (cuTensorMapEncodeTiled) unavailable */
+#define UMB_ERR_TIMEOUT (-5)     /* an earlier kernel gave up on a bounded wait: results since then are not to be used */
 
 const char* umb_version(void);
 const char* umb_error_string(int code);

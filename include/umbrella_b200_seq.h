@@ -305,6 +305,11 @@ unsigned long long umbs_launch_count(void);
  * results are not to be used).  Synchronises. */
 unsigned int umbs_kernel_timeouts(void);
 
+/* Whether such a block has reported so far (1 or 0).  Does not synchronise: behind a synchronisation it covers all work in front
+ * of it.  From then on the calls that launch such kernels return UMB_ERR_TIMEOUT: caches and results written since are not to be
+ * used, and the process is to be started again.  (The first such call allocates the report's 4 bytes of host memory.) */
+unsigned int umbs_give_ups_seen(void);
+
 /* Bytes of scratch umbs_forward needs for a step of up to max_tokens tokens of which up to max_want want logits. */
 size_t umbs_workspace_bytes(const umbs_model_t* model, int max_tokens, int max_want);
 

@@ -30,3 +30,28 @@ def test_rows_that_a_product_is_told_to_leave_out_are_zero(recorder, max_rows, c
     out = K.gemm(a, w, max_rows=max_rows)
     assert bool((out == 0).all()) == cleared
     assert K.gemm(a, w, rows=3, max_rows=2).eq(0).all()              # of the rows asked for, not of a's
+
+
+# ---------------------------------------------------------------------------------------------- a kernel that gave up
+def test_a_give_up_is_raised_before_anything_is_made_of_the_results(monkeypatch):
+    """The library reports it as a word that needs no synchronisation; the model looks before a step, the engine behind the copy
+    of the sampled tokens."""
+    from umbrella_b200.models import seq_model
+    from umbrella_b200.speculation import batch_engine
+    seen = [0]
+    monkeypatch.setattr(S, "load", lambda *a, **k: type("Lib", (), {"umbs_give_ups_seen": staticmethod(lambda: seen[0])})())
+    model = seq_model.SeqStateModel.__new__(seq_model.SeqStateModel)
+    model.spec = seq_model.SeqModelSpec(width=8, vocab=5, layers=[])
+    model.cache, model.device, model.max_length = None, torch.device("cpu"), None
+    assert model.forward([]).shape == (0, 5)
+    engine = batch_engine.BatchDecodingEngine.__new__(batch_engine.BatchDecodingEngine)
+    engine.model = model
+    engine.sample = lambda logits: logits.argmax(-1)
+    assert engine._take(torch.eye(3)) == [0, 1, 2]
+    seen[0] = 1
+    with pytest.raises(RuntimeError, match="gave up"):
+        engine._take(torch.eye(3))
+    with pytest.raises(RuntimeError, match="gave up"):
+        model.forward([])
+    with pytest.raises(RuntimeError, match="gave up"):
+        S.check(-5, "forward")

@@ -129,6 +129,7 @@ SIGNATURES = {
     "umbs_version": (C.c_char_p, []),
     "umbs_launch_count": (C.c_ulonglong, []),
     "umbs_kernel_timeouts": (C.c_uint, []),
+    "umbs_give_ups_seen": (C.c_uint, []),
     "umbs_workspace_bytes": (c_size_t, [C.POINTER(Model), c_int, c_int]),
     "umbs_forward": (c_int, [C.POINTER(Model), _BP, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
     "umbs_gemm": (c_int, [c_int, c_void_p, c_int64, c_int, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int, c_int,
@@ -247,10 +248,21 @@ def load() -> C.CDLL:
     return lib
 
 
+GAVE_UP = "an earlier kernel gave up on a wait: results since then, cached states among them, are not to be used"
+
+
+def raise_if_given_up() -> None:
+    """Raise if a kernel has reported that it gave up on a bounded wait.  Does not synchronise: called behind a copy to the
+    host it covers everything the copy waited for."""
+    if load().umbs_give_ups_seen():
+        raise RuntimeError("umbrella_b200_seq: " + GAVE_UP)
+
+
 def check(rc: int, what: str = "") -> None:
     if rc != 0:
         from . import _lib as core
-        msg = {-1: "invalid argument", -2: "shape or option not supported", -3: "workspace too small"}.get(rc)
+        msg = {-1: "invalid argument", -2: "shape or option not supported", -3: "workspace too small",
+               -5: GAVE_UP}.get(rc)
         if msg is None:
             try:
                 msg = core.load().umb_error_string(rc).decode()

@@ -64,6 +64,7 @@ extern "C" const char* umb_error_string(int code) {
         case UMB_ERR_UNSUPPORTED: return "shape or option not supported by the sm_100a kernels";
         case UMB_ERR_WORKSPACE: return "workspace too small";
         case UMB_ERR_DRIVER: return "CUDA driver entry point unavailable (cuTensorMapEncodeTiled)";
+        case UMB_ERR_TIMEOUT: return "an earlier kernel gave up on a wait: results since then are not to be used";
         default: break;
     }
     if (code > 0) return cudaGetErrorString((cudaError_t)code);

@@ -31,7 +31,8 @@ constexpr int kTaThreads = 224;                             // 4 warps of weight
 constexpr int kTaStages = 4;                                // key and value tiles held, at most
 constexpr float kTaLazy = 8.f;                              // how far (in powers of two) a score may pass the reference
 
-struct TaDims { int q_atoms, k_steps, v_atoms, stages, tma; };   // 64-wide pieces of a query row, 16-wide k steps, 64-wide pieces of a value row; tiles held
+// 64-wide pieces of a query row, 16-wide k steps, 64-wide pieces of a value row; tiles held; give_up_word()
+struct TaDims { int q_atoms, k_steps, v_atoms, stages, tma; unsigned int* report; };
 
 __device__ __forceinline__ float ex2(float x) {
     float y;
@@ -398,7 +399,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
     __syncwarp();
     umb::tc_fence_before();
     __syncthreads();
-    tc_settle(quit);
+    tc_settle(quit, z.report);
     if (warp == 4) {
         umb::tc_fence_after();
         umb::tmem_dealloc(tmem, 256);
@@ -408,7 +409,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
 // As many key and value tiles as leave room for a second block on the SM (228 KB, 1 KB of it per block the system's): four, or
 // three beside queries of more than 128 numbers.
 static TaDims ta_dims(const CachedAttnArgs& a) {
-    TaDims z{(a.dim + 63) / 64, (a.dim + 15) / 16, (a.vdim + 63) / 64, kTaStages, 0};
+    TaDims z{(a.dim + 63) / 64, (a.dim + 15) / 16, (a.vdim + 63) / 64, kTaStages, 0, nullptr};
     while (z.stages > 3 && z.q_atoms * (kTaQ * 128) + z.stages * (z.q_atoms + z.v_atoms) * (kTaK * 128) > 110 * 1024) --z.stages;
     return z;
 }
@@ -430,11 +431,13 @@ bool attention_tc_fits(const CachedAttnArgs& a, const StepKeys* s) {
 template <int MODE, bool SHAPED, bool STEP>
 static int launch_ta(const CachedAttnArgs& a, const StepKeys& x, const Batch& b, cudaStream_t st) {
     TaDims z = ta_dims(a);
+    int rc = give_up_word(&z.report);
+    if (rc == 0) rc = give_up_status();
+    if (rc != 0) return rc;
     // heads that are whole pieces of 64 numbers: the step's rows as tensor maps
     CUtensorMap mk{}, ms{}, mv{};
     z.tma = a.dim % 64 == 0 && a.vdim % 64 == 0 && (!STEP || x.kdim % 64 == 0);
     if (z.tma) {
-        int rc;
         if (STEP) {
             rc = encode_map(&mk, x.k, (uint64_t)a.heads * x.kdim, b.n_tokens, 1, x.ldk, 0, kTaK);
             if (rc == 0 && x.kdim < a.dim) rc = encode_map(&ms, x.ks, a.dim - x.kdim, b.n_tokens, 1, x.ldks, 0, kTaK);

@@ -224,6 +224,7 @@ extern "C" int umbs_forward(const umbs_model_t* m, const umbs_batch_t* b, float*
     if (m == nullptr || b == nullptr || workspace == nullptr) return UMB_ERR_ARG;
     const int T = b->n_tokens, W = m->width, dt = m->dtype;
     if (T <= 0) return 0;
+    if (const int gave_up = give_up_status()) return gave_up;
     if ((uintptr_t)workspace % 256 != 0) return UMB_ERR_ARG;
     Scratch s;
     if (carve(m, T, b->n_want, (char*)workspace, &s) > workspace_bytes) return UMB_ERR_WORKSPACE;

@@ -16,6 +16,8 @@
 // cleared first), 109 us here (947 TFLOP/s).  16 experts, top 2, 4096 tokens of width 2048 with the routing around it:
 // 808 -> 229 us; 64 tokens: 213 -> 98 us.
 #include <cuda.h>
+#include <atomic>
+#include <mutex>
 
 #include "seq_gemm.h"
 #include "seq_tc.cuh"
@@ -29,6 +31,7 @@ struct TcArgs {
     int groups, n_tiles, m_tiles, k_steps;
     int vec_c;                                              // rows of C take 16-byte (fp32) / 8-byte (bf16) stores of 4 columns
     int a_grouped, w_grouped;                               // the group coordinate of the tensor maps is used
+    unsigned int* report;                                   // give_up_word()
 };
 
 // The tiles of a block, in the order every role visits them: rows fastest, then columns, then groups.
@@ -283,7 +286,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
     }
     __syncthreads();
-    tc_settle(quit);
+    tc_settle(quit, t.report);
     if (warp == 1) {
         umb::tc_fence_after();
         umb::tmem_dealloc(tmem, 2 * BN);
@@ -291,6 +294,33 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 }
 
 // ------------------------------------------------------------------------------------------------ host side
+static std::atomic<unsigned int*> g_give_up{nullptr};       // 4 bytes for the process, shared by its devices, streams and threads
+
+int give_up_word(unsigned int** word) {
+    static std::mutex making;
+    unsigned int* w = g_give_up.load(std::memory_order_acquire);
+    if (w == nullptr) {
+        std::lock_guard<std::mutex> lock(making);
+        w = g_give_up.load(std::memory_order_acquire);
+        if (w == nullptr) {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // (the first call may be inside a capture)
+            cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+            if (e != cudaSuccess) return (int)e;
+            e = cudaHostAlloc((void**)&w, sizeof *w, cudaHostAllocPortable | cudaHostAllocMapped);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            if (e != cudaSuccess) return (int)e;
+            *w = 0u;
+            g_give_up.store(w, std::memory_order_release);
+        }
+    }
+    *word = w;
+    return 0;
+}
+int give_up_status() {
+    const volatile unsigned int* w = g_give_up.load(std::memory_order_acquire);
+    return w != nullptr && *w != 0u ? UMB_ERR_TIMEOUT : 0;
+}
+
 typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -350,6 +380,9 @@ int launch_gemm_tc(const GemmArgs& a, int groups, bool dual, bool c_f32, cudaStr
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return (int)e;
     TcArgs t{};
+    int rc = give_up_word(&t.report);
+    if (rc == 0) rc = give_up_status();
+    if (rc != 0) return rc;
     t.groups = groups;
     t.m_tiles = (a.M + kTcRows - 1) / kTcRows;
     const int es = c_f32 ? 4 : 2;
@@ -371,4 +404,5 @@ int launch_gemm_tc(const GemmArgs& a, int groups, bool dual, bool c_f32, cudaStr
 
 }  // namespace umbs
 
+extern "C" unsigned int umbs_give_ups_seen(void) { return umbs::give_up_status() != 0; }
 extern "C" unsigned int umbs_kernel_timeouts(void) { return umbs::tc_timeouts() + umbs::attention_tc_timeouts(); }

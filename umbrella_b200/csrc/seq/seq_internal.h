@@ -41,4 +41,9 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
 }
 
 void count_launches(unsigned n);
+
+// seq_gemm_tc.cu: a word of host memory that the kernels can write, set by a block that gave up.  Every call that launches such
+// a kernel looks at it first (no synchronisation) and refuses once it is set: results since then are not to be used.
+int give_up_word(unsigned int** word);                      // made on the first call; an error of the runtime, or 0
+int give_up_status();                                       // 0, or UMB_ERR_TIMEOUT
 }  // namespace umbs

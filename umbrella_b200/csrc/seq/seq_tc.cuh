@@ -3,6 +3,7 @@
 #include <cuda.h>
 
 #include "../common.cuh"
+#include "seq_internal.h"
 
 namespace umbs {
 using umb::smem_u32;
@@ -58,9 +59,14 @@ __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile
     }
     return tc_give_up(quit);
 }
-// Behind the last barrier of a kernel that gave up: copies and products in flight end before their memory goes.
-__device__ __forceinline__ void tc_settle(volatile int* quit) {
+// Behind the last barrier of a kernel that gave up: the host learns of it (give_up_word), and copies and products in flight end
+// before their memory goes.
+__device__ __forceinline__ void tc_settle(volatile int* quit, volatile unsigned int* report) {
     if (!*quit) return;
+    if (threadIdx.x == 0) {
+        *report = 1u;
+        __threadfence_system();
+    }
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);
     __syncthreads();
 }

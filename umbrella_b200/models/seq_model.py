@@ -693,7 +693,10 @@ class SeqStateModel:
     def forward(self, entries, layer_out: bool = False):
         """``entries``: [(slot, tokens, want)], the next tokens of every sequence of the step and the indices among
         them whose logits are wanted.  Returns fp32 logits [sum of wants, vocab] in entry order (and, with
-        ``layer_out``, the residual stream after every layer run, [runs, tokens, width]).  The slots' positions advance."""
+        ``layer_out``, the residual stream after every layer run, [runs, tokens, width]).  The slots' positions advance.
+        Raises if a kernel of an earlier step gave up on a wait; ``check_results`` says so of this step once the logits are on
+        the host."""
+        S.raise_if_given_up()                 # (a replayed graph does not pass the library's own look at it)
         cache = self.cache
         ids, tok_seq, tok_pos, want = [], [], [], []
         slot, start, length, pos0, parity = [], [], [], [], []
@@ -750,6 +753,10 @@ class SeqStateModel:
         for s, n in zip(slot, length):
             cache.advance(s, n)
         return (logits, layers) if layer_out else logits
+
+    def check_results(self):
+        """Behind a copy of the logits to the host: raise if a kernel of their step gave up, so that nothing is made of them."""
+        S.raise_if_given_up()
 
     def _graph_step(self, key, host, describe, enqueue):
         """Replay (capturing first, on the third step of this shape) the CUDA graph of a decode step; None = run eagerly."""

@@ -112,6 +112,14 @@ class BatchDecodingEngine(BaseEngine):
         return ops.sample(logits, ops.UMB_SAMPLE_DYNAMIC, temperature=self.temperature, top_k=self.topk, top_p=self.topp,
                           uniforms=u)
 
+    def _take(self, logits: torch.Tensor) -> list:
+        """The sampled tokens on the host, once it is known that the step's kernels came to their end."""
+        tokens = self.sample(logits).tolist()
+        check = getattr(self.model, "check_results", None)
+        if check is not None:
+            check()
+        return tokens
+
     # ------------------------------------------------------------------ batches of requests
     def submit(self, rid, input_ids, max_new_tokens: int = 128):
         self.queue.append({"id": rid, "prompt": [int(t) for t in input_ids], "max_new": int(max_new_tokens), "out": []})
@@ -133,7 +141,7 @@ class BatchDecodingEngine(BaseEngine):
             live = self._form_batch()
             logits = self.step([{"id": r["id"], "tokens": r["prompt"], "want": [len(r["prompt"]) - 1]} for r in live])
             while live:
-                nxt = self.sample(logits).tolist()
+                nxt = self._take(logits)
                 still, ended = [], []
                 for r, t in zip(live, nxt):
                     r["out"].append(t)
@@ -182,8 +190,9 @@ class BatchDecodingEngine(BaseEngine):
         if self.max_length is not None and len(toks) + len(ids) >= self.max_length:
             return False
         logits = self.step([{"id": rid, "tokens": ids, "want": [len(ids) - 1]}])
+        nxt = self._take(logits)[0]
         toks += ids
-        toks.append(int(self.sample(logits)[0]))          # the first committed token, fed by the next verify()
+        toks.append(nxt)                                  # the first committed token, fed by the next verify()
         return True
 
     def build_tree(self):
@@ -194,7 +203,7 @@ class BatchDecodingEngine(BaseEngine):
         if toks[-1] in self.eos_tokens:
             return False
         logits = self.step([{"id": rid, "tokens": [toks[-1]], "want": [0]}])
-        toks.append(int(self.sample(logits)[0]))
+        toks.append(self._take(logits)[0])
         return toks[-1] not in self.eos_tokens
 
     def speculative_decoding(self, max_new_tokens=128):
