@@ -169,3 +169,17 @@ def test_decode_masks_and_outputs(ops, window, pool):
 def test_decode_score_options(ops, kw, opts):
     for step in DECODE[:3]:
         _both(ops, step, 4, 2, 64, 32, opts=opts + ("scored",), **kw)
+
+
+@pytest.mark.parametrize("which", ["k", "v", "ks", "same"])
+def test_overlapping_rows_of_a_steps_keys_are_taken(ops, which):
+    """Rows that share memory (each a few numbers behind the one before it, or one row for every token) give what copies of them give."""
+    heads, dim, shared, vdim, T = 2, 64, 64, 64, 150
+    g = torch.Generator(device=DEV).manual_seed(5)
+    rows = dict(q=_r(g, T, heads * (dim + shared), s=1.5), k=_r(g, T, heads * dim), ks=_r(g, T, shared), v=_r(g, T, heads * vdim))
+    for name in ("k", "v") if which == "same" else (which,):
+        n = rows[name].shape[1]
+        rows[name] = rows[name][:1].expand(T, n) if which == "same" else _r(g, 8 * T + n).as_strided((T, n), (8, 1))
+    batch = ops.RaggedBatch([(0, T - 20, 0, 0), (1, 20, 0, 0)], DEV)
+    run = lambda q, k, ks, v: ops.window_attention_shared(q, k, ks, v, batch, heads, (dim + shared) ** -0.5)
+    assert torch.equal(run(**rows), run(**{n: t.contiguous() for n, t in rows.items()}))

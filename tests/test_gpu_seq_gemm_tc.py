@@ -111,3 +111,11 @@ def test_true_32_bit_tiles(ops, M, N, K, dt):
     got = ops.gemm(a, w, n=N, dual=True, limit=7.0, out_f32=True)
     gate, up = z[:, :N].clamp(max=7.0), z[:, N:].clamp(-7.0, 7.0)
     assert H.rel_err(got, (gate * torch.sigmoid(1.702 * gate) * (up + 1)).cpu()) < 4e-6   # a product of two such sums
+
+
+def test_groups_that_run_backwards_are_taken(ops):
+    """A negative step between the groups' columns: no tensor map describes it."""
+    x, w = _mat(51, 40, 3 * 64), _mat(52, 3, 48, 64)
+    got = ops.gemm(x[:, 128:], w, out_f32=True, groups=3, a_goff=-64, c_goff=48)
+    ref = torch.cat([x[:, 128 - 64 * i:192 - 64 * i].double() @ w[i].double().T for i in range(3)], 1)
+    assert H.rel_err(got, ref.cpu()) < F32_TOL

@@ -434,9 +434,11 @@ static int launch_ta(const CachedAttnArgs& a, const StepKeys& x, const Batch& b,
     int rc = give_up_word(&z.report);
     if (rc == 0) rc = give_up_status();
     if (rc != 0) return rc;
-    // heads that are whole pieces of 64 numbers: the step's rows as tensor maps
+    // heads that are whole pieces of 64 numbers: the step's rows as tensor maps.  Rows that overlap (a row repeated among them)
+    // and whatever else a map does not describe are copied row by row like the other sizes.
     CUtensorMap mk{}, ms{}, mv{};
-    z.tma = a.dim % 64 == 0 && a.vdim % 64 == 0 && (!STEP || x.kdim % 64 == 0);
+    z.tma = a.dim % 64 == 0 && a.vdim % 64 == 0 && (!STEP || (x.kdim % 64 == 0 && x.ldk >= (int64_t)a.heads * x.kdim && x.ldv >= (int64_t)a.heads * a.vdim &&
+                                                              (x.kdim == a.dim || x.ldks >= a.dim - x.kdim)));
     if (z.tma) {
         if (STEP) {
             rc = encode_map(&mk, x.k, (uint64_t)a.heads * x.kdim, b.n_tokens, 1, x.ldk, 0, kTaK);
@@ -447,7 +449,7 @@ static int launch_ta(const CachedAttnArgs& a, const StepKeys& x, const Batch& b,
             rc = encode_map(&mk, a.kv, row, b.n_tokens, 1, row, 0, kTaK);
             mv = mk;
         }
-        if (rc != 0) return rc;
+        z.tma = rc == 0;
     }
     const int smem = 1024 + (z.q_atoms * (kTaQ + z.stages * kTaK) + z.stages * z.v_atoms * kTaK) * 128;
     auto kernel = attention_tc_kernel<MODE, SHAPED, STEP>;

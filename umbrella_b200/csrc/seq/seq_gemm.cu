@@ -355,12 +355,14 @@ static int gemm_run(int dtype, const void* A, int64_t lda, int a_goff, const voi
         if (vec && M <= 16) {
             if (c_f32) launch_skinny<float>(a, groups, dual != 0, st);
             else launch_skinny<__nv_bfloat16>(a, groups, dual != 0, st);
-        } else if (tc) {
-            const int rc = launch_gemm_tc(a, groups, dual != 0, c_f32 != 0, st);
-            if (rc != 0) return rc;
         } else {
-            if (c_f32) launch_simt<__nv_bfloat16, float>(a, groups, dual != 0, st);
-            else launch_simt<__nv_bfloat16, __nv_bfloat16>(a, groups, dual != 0, st);
+            const int rc = tc ? launch_gemm_tc(a, groups, dual != 0, c_f32 != 0, st) : UMB_ERR_DRIVER;
+            if (rc == UMB_ERR_DRIVER) {                     // (also strides that no tensor map describes: groups that run backwards)
+                if (c_f32) launch_simt<__nv_bfloat16, float>(a, groups, dual != 0, st);
+                else launch_simt<__nv_bfloat16, __nv_bfloat16>(a, groups, dual != 0, st);
+            } else if (rc != 0) {
+                return rc;
+            }
         }
     } else {
         return UMB_ERR_ARG;
