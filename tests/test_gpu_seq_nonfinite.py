@@ -69,3 +69,84 @@ def test_tokens_in_front_of_a_nan_keep_their_bits(kind, n, what):
         out = run(y)
         assert torch.equal(out[:j], want[:j]), j
         assert not torch.isfinite(out[j]).any(), j
+
+
+# ---------------------------------------------------------------------------------------------- attention
+def seen_only(q, keys, values, visible, scale, sink):
+    """float64: every row over the keys it sees and no others.  q [n, d], keys [m, d], values [m, e], visible [n, m]."""
+    rows = []
+    for i in range(q.shape[0]):
+        at = visible[i].nonzero().flatten()
+        z = (keys[at] @ q[i]) * scale
+        m = torch.maximum(z.max(), sink)
+        p = torch.exp(z - m)
+        rows.append((p[:, None] * values[at]).sum(0) / (p.sum() + torch.exp(sink - m)))
+    return torch.stack(rows)
+
+
+def assert_same(got, want):
+    """NaN where it is NaN, infinite where it is infinite, else within the rounding of a bf16 result (2^-8 of the row's largest)."""
+    got, want = got.double().cpu(), want.cpu()
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    assert torch.equal(got[torch.isinf(want)], want[torch.isinf(want)]) and torch.equal(torch.isinf(got), torch.isinf(want))
+    ok = torch.isfinite(want)
+    big = torch.where(ok, want, torch.zeros_like(want)).abs().amax(-1, keepdim=True).expand_as(want)
+    assert bool(((got - want).abs()[ok] <= 2.0 ** -8 * big[ok] + 1e-6).all())
+
+
+BAD = {"value": lambda row, kdim: row[kdim + 3:kdim + 4].fill_(float("inf")),
+       "both signs": lambda row, kdim: (row[kdim + 3:kdim + 4].fill_(float("inf")), row[kdim + 5:kdim + 6].fill_(float("-inf"))),
+       "token": lambda row, kdim: row.fill_(float("nan"))}
+
+
+@pytest.mark.parametrize("what", list(BAD))
+@pytest.mark.parametrize("tokens,past", [(150, 0), (40, 90), (1, 300), (1, 2000)])           # a prompt, a later portion of one, decode steps
+@pytest.mark.parametrize("dim,window", [(64, 0), (72, 50), (128, 100)])
+def test_attention_over_a_cache(what, tokens, past, dim, window):
+    from umbrella_b200 import _lib_seq as S, ops_seq as K
+    heads, kv_heads, n = 4, 2, past + tokens
+    kdim = kv_heads * dim
+    q = rnd(tokens, heads * dim, seed=1).bfloat16()
+    rows = rnd(n, 2 * kdim, seed=2).bfloat16()
+    bad = n - 1 if tokens == 1 and window else max(n - 30, past + tokens // 2) if tokens > 1 else n // 2
+    for at in sorted({bad, max(bad - 17, 0)}):
+        for g in range(kv_heads):
+            part = rows[at] if what == "token" else rows[at, kdim + g * dim:kdim + (g + 1) * dim]
+            BAD[what](part, 0)
+        if what == "token":
+            break
+    sink = rnd(heads, seed=3)
+    cache = torch.zeros(1, max(n, 1), 2 * kdim, dtype=torch.bfloat16)
+    cache[0, :past] = rows[:past]
+    out = K.cached_attention(q.to(DEV), rows[past:].contiguous().to(DEV), cache.to(DEV), K.RaggedBatch([(0, tokens, past, 0)], DEV), heads, kv_heads,
+                             dim, dim, dim ** -0.5, mode=S.UMBS_ATTN_SOFTMAX_SINK, window=window, sink=sink.to(DEV), append=False)
+    pos, j = torch.arange(past, n)[:, None], torch.arange(n)[None]
+    visible = (j <= pos) & (j > pos - (window or 1 << 30))
+    for h in range(heads):
+        g = h // (heads // kv_heads)
+        want = seen_only(q[:, h * dim:(h + 1) * dim].double(), rows[:, g * dim:(g + 1) * dim].double(), rows[:, kdim + g * dim:kdim + (g + 1) * dim].double(),
+                         visible, float(torch.tensor(dim ** -0.5)), sink[h].double())
+        assert_same(out[:, h * dim:(h + 1) * dim], want)
+
+
+@pytest.mark.parametrize("what", list(BAD))
+@pytest.mark.parametrize("shared,window", [(0, 0), (64, 40)])
+def test_attention_of_a_steps_own_keys(what, shared, window):
+    from umbrella_b200 import ops_seq as K
+    heads, dim, n = 2, 64, 150
+    q, k, v = rnd(n, heads * (dim + shared), seed=1).bfloat16(), rnd(n, heads * dim, seed=2).bfloat16(), rnd(n, heads * dim, seed=3).bfloat16()
+    ks = rnd(n, shared, seed=4).bfloat16() if shared else None
+    for h in range(heads):
+        BAD[what](v[100, h * dim:(h + 1) * dim], 0)
+    if what == "token":
+        k[100] = float("nan")
+    sink = rnd(heads, seed=5)
+    out = K.window_attention_shared(q.to(DEV), k.to(DEV), ks.to(DEV) if shared else None, v.to(DEV), K.RaggedBatch([(0, n, 0, 0)], DEV), heads,
+                                    (dim + shared) ** -0.5, window=window, sink=sink.to(DEV))
+    i = torch.arange(n)
+    visible = (i[None] <= i[:, None]) & (i[None] > i[:, None] - (window or 1 << 30))
+    for h in range(heads):
+        keys = torch.cat([k[:, h * dim:(h + 1) * dim]] + ([ks] if shared else []), 1).double()
+        want = seen_only(q[:, h * (dim + shared):(h + 1) * (dim + shared)].double(), keys, v[:, h * dim:(h + 1) * dim].double(), visible,
+                         float(torch.tensor((dim + shared) ** -0.5)), sink[h].double())
+        assert_same(out[:, h * dim:(h + 1) * dim], want)

@@ -41,6 +41,51 @@ __device__ __forceinline__ float shaped_score(const CachedAttnArgs& a, float dot
 
 __device__ __forceinline__ float sigmoidf_(float z) { return 1.f / (1.f + expf(-z)); }
 
+// One query row in plain fp32 by a whole warp, a key at a time.  The tensor-core kernels hand a row to it whose result is not
+// finite: a key that the row does not see sits in its tile with a weight of 0, and 0 times a NaN value is NaN; the parts that a
+// weight is split into are often 0, and 0 times an infinite value is no infinity.  Bound: a load latency per key; it is not there
+// for speed.
+struct PlainRow { float q[6], o[4], m, l; };          // a lane's numbers: dimensions lane + 32 i (up to 192), value columns (up to 128)
+__device__ __forceinline__ void plain_start(PlainRow& s, const __nv_bfloat16* q, int dim, float m, float l) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) s.q[i] = lane + 32 * i < dim ? to_f32(q[lane + 32 * i]) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s.o[i] = 0.f;
+    s.m = m;
+    s.l = l;
+}
+// one key: its first `own` dimensions at k, the others at k_shared; false once every column is NaN for good
+template <int MODE>
+__device__ __forceinline__ bool plain_key(PlainRow& s, const CachedAttnArgs& a, const __nv_bfloat16* k, int own, const __nv_bfloat16* k_shared,
+                                          const __nv_bfloat16* v, int h, int dist) {
+    const int lane = threadIdx.x & 31;
+    float dot = 0.f;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        const int d = lane + 32 * i;
+        if (d < a.dim) dot = fmaf(s.q[i], to_f32(d < own ? k[d] : k_shared[d - own]), dot);
+    }
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, w);
+    float p;
+    if (MODE == UMBS_ATTN_SIGMOID) {
+        p = sigmoidf_(dot * a.scale + (a.head_bias ? a.head_bias[h] : 0.f));
+    } else {
+        const float sc = shaped_score(a, dot, a.r1 ? a.r1[h] : 0.f, a.r1 ? a.r2[h] : 0.f, dist);
+        const float mn = fmaxf(s.m, sc), ref = mn > -INFINITY ? mn : 0.f, corr = expf(s.m - ref);       // (m = -inf: corr = 0)
+        p = expf(sc - ref);
+        s.l = s.l * corr + p;
+        s.m = mn;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s.o[i] *= corr;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (lane + 32 * i < a.vdim) s.o[i] = fmaf(p, to_f32(v[lane + 32 * i]), s.o[i]);
+    return MODE == UMBS_ATTN_SIGMOID ? p == p : s.l == s.l;
+}
+
 // blocks of `pool` tokens that lie wholly before the window of the row at position p
 __device__ __forceinline__ int pooled_visible(int p, int window, int pool) {
     const int lim = p - window + 1;                   // tokens [0, lim) have left the window

@@ -62,9 +62,48 @@ struct KeyTiles {
     __device__ int last(int i) const { return i < tiles_pool ? n_pool - 1 : p_hi; }
 };
 
+// Row r of (sequence s, virtual head vh) in plain fp32, by a whole warp: the keys it sees, in order, as the kernel below ends.
+template <int MODE, bool STEP>
+__device__ __noinline__ void plain_row(const CachedAttnArgs& a, const StepKeys& x, const Batch& b, int s, int vh, int r) {
+    const int lane = threadIdx.x & 31, start = b.seq_start[s], pos0 = STEP ? 0 : b.seq_pos0[s], slot = STEP ? 0 : b.seq_slot[s], rp = pos0 + r;
+    const int window = a.window > 0 ? a.window : (1 << 30);
+    const int64_t t = start + r;
+    VHead v;
+    if (STEP) { v.h = vh; v.qoff = vh * a.dim; }
+    else v = virtual_head(a, vh);
+    PlainRow p;
+    plain_start(p, STEP ? (const __nv_bfloat16*)x.q + t * x.ldq + v.qoff : (const __nv_bfloat16*)a.q + t * v.qstride + v.qoff, a.dim,
+                MODE == UMBS_ATTN_SOFTMAX_SINK ? sink_score(a, v.h) : -INFINITY, MODE == UMBS_ATTN_SOFTMAX_SINK ? 1.f : 0.f);
+    const int n_pool = STEP ? 0 : pooled_visible(rp, window, a.pool), lo = max(max(0, rp - window + 1), a.chunk > 0 ? rp / a.chunk * a.chunk : 0);
+    bool go = true;
+    for (int i = 0; go && i < n_pool; ++i) {
+        const __nv_bfloat16* row = (const __nv_bfloat16*)a.pool_cache + ((int64_t)slot * a.pool_len + i) * v.row_kv;
+        go = plain_key<MODE>(p, a, row + v.koff, a.dim, nullptr, row + v.voff, v.h, rp - i);
+    }
+    for (int j = lo; go && j <= rp; ++j) {
+        if (STEP) {
+            const int64_t key = start + j;
+            go = plain_key<MODE>(p, a, (const __nv_bfloat16*)x.k + key * x.ldk + (int64_t)vh * x.kdim, x.kdim, (const __nv_bfloat16*)x.ks + key * x.ldks,
+                                 (const __nv_bfloat16*)x.v + key * x.ldv + (int64_t)vh * a.vdim, v.h, rp - j);
+        } else {
+            const __nv_bfloat16* row = j >= pos0 ? (const __nv_bfloat16*)a.kv + (int64_t)(start + j - pos0) * v.row_kv
+                                                 : (const __nv_bfloat16*)a.kv_cache + ((int64_t)slot * a.kv_len + j % a.kv_len) * v.row_kv;
+            go = plain_key<MODE>(p, a, row + v.koff, a.dim, nullptr, row + v.voff, v.h, rp - j);
+        }
+    }
+    const float inv = MODE == UMBS_ATTN_SIGMOID ? 1.f : 1.f / p.l;
+    const float* grow = a.gate ? a.gate + t * a.ldg + (a.gate_per_head ? v.h : v.h * a.vdim) : nullptr;
+    __nv_bfloat16* orow = STEP ? (__nv_bfloat16*)x.out + t * x.ldo + (int64_t)v.h * a.vdim : (__nv_bfloat16*)a.out + t * a.heads * a.vdim + (int64_t)v.h * a.vdim;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int c = lane + 32 * i;
+        if (c < a.vdim) orow[c] = from_f32<__nv_bfloat16>(p.o[i] * inv * (grow ? sigmoidf_(grow[a.gate_per_head ? 0 : c]) : 1.f));
+    }
+}
+
 template <int MODE, bool SHAPED, bool STEP>
 __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_s, const __grid_constant__ CUtensorMap map_v,
-                                                                        const CachedAttnArgs a, const StepKeys x, const Batch b, const TaDims z) {
+                                                                        const __grid_constant__ CachedAttnArgs a, const __grid_constant__ StepKeys x, const __grid_constant__ Batch b, const TaDims z) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ uint64_t bars[4 * kTaStages + 4];
     __shared__ uint32_t s_tmem;
@@ -361,6 +400,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
             const bool gvec = grow && !a.gate_per_head && ((uintptr_t)grow & 15) == 0;
             __nv_bfloat16* orow = STEP ? (__nv_bfloat16*)x.out + t * x.ldo + (int64_t)h * a.vdim
                                        : (__nv_bfloat16*)a.out + t * a.heads * a.vdim + (int64_t)h * a.vdim;
+            float odd = 0.f;                                // stays 0 while the row's sums are finite
             for (int c0 = 0; c0 < a.vdim; c0 += 32) {
                 uint32_t v[32];
                 UMB_TMEM_LD_X32(t0 + 128 + c0, v);
@@ -371,7 +411,10 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
                         if (c0 + e < a.vdim) {                              // (vdim is a multiple of 8)
                             float o[8];
 #pragma unroll
-                            for (int u = 0; u < 8; ++u) o[u] = __uint_as_float(v[e + u]) * inv;
+                            for (int u = 0; u < 8; ++u) {
+                                o[u] = __uint_as_float(v[e + u]) * inv;
+                                odd = fmaf(o[u], 0.f, odd);
+                            }
                             if (grow) {
                                 float g[8];
                                 if (gvec) {
@@ -394,6 +437,8 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
                 }
                 __syncwarp();
             }
+            for (uint32_t rows = __ballot_sync(0xffffffffu, odd != 0.f); rows != 0; rows &= rows - 1)
+                plain_row<MODE, STEP>(a, x, b, s, vh, q0 + warp * 32 + __ffs(rows) - 1);
         }
     }
     __syncwarp();

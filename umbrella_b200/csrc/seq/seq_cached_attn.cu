@@ -403,8 +403,30 @@ __device__ __forceinline__ void mma_top(float (&d)[4], uint32_t a0, uint32_t a2,
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
 }
 
+// A warp's triple of one head in plain fp32: every fourth tile of the keys [lo, hi) from the warp's own, key after key.
 template <int MODE>
-__global__ void __launch_bounds__(32 * kCgWarps, 3) cached_attention_decode_group_kernel(CachedAttnArgs a, Batch b, int n_split, float* __restrict__ part) {
+__device__ __noinline__ void plain_part(const CachedAttnArgs& a, const VHead& v, const __nv_bfloat16* q, int h, const __nv_bfloat16* own, int slot, int p, int n_pool,
+                                        int j_lo, int first, int hi, float* s_o, float* s_ml) {
+    const int lane = threadIdx.x & 31;
+    PlainRow s;
+    plain_start(s, q, a.dim, -INFINITY, 0.f);
+    bool go = true;
+    for (int k0 = first; go && k0 < hi; k0 += kCgWarps * kCgKeys)
+        for (int k = k0; go && k < min(k0 + kCgKeys, hi); ++k) {
+            const int j = j_lo + (k - n_pool);
+            const __nv_bfloat16* row = k < n_pool ? (const __nv_bfloat16*)a.pool_cache + ((int64_t)slot * a.pool_len + k) * v.row_kv
+                                     : j >= p ? own : (const __nv_bfloat16*)a.kv_cache + ((int64_t)slot * a.kv_len + j % a.kv_len) * v.row_kv;
+            go = plain_key<MODE>(s, a, row + v.koff, a.dim, nullptr, row + v.voff, h, k < n_pool ? 0 : p - j);
+        }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (lane + 32 * i < a.vdim) s_o[lane + 32 * i] = s.o[i];
+    if (lane == 0) { s_ml[0] = s.m; s_ml[1] = s.l; }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(32 * kCgWarps, 3) cached_attention_decode_group_kernel(const __grid_constant__ CachedAttnArgs a, const __grid_constant__ Batch b,
+                                                                                         int n_split, float* __restrict__ part) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int dim = a.dim, vdim = a.vdim, G = a.heads / a.kv_heads, chunks = (G + kCgHeads - 1) / kCgHeads;
     const GroupSizes z = group_sizes(dim, vdim);
@@ -586,6 +608,15 @@ __global__ void __launch_bounds__(32 * kCgWarps, 3) cached_attention_decode_grou
     for (int j = 0; j < 16; ++j)
         if (j < nvt) *reinterpret_cast<float2*>(s_o + (w * kCgHeads + hr) * vdim + j * 8 + qd * 2) = make_float2(o[j][0], o[j][1]);
     if (qd == 0) { s_ml[(w * kCgHeads + hr) * 2] = m; s_ml[(w * kCgHeads + hr) * 2 + 1] = l; }
+    float odd = 0.f;                                                        // stays 0 while the sums are finite
+#pragma unroll
+    for (int j = 0; j < 16; ++j) odd = fmaf(o[j][0], 0.f, fmaf(o[j][1], 0.f, odd));
+    if (__any_sync(0xffffffffu, hr < nh && odd != 0.f)) {
+        __syncwarp();
+        for (int g = 0; g < nh; ++g)
+            plain_part<MODE>(a, v0, (const __nv_bfloat16*)a.q + (int64_t)t * v0.qstride + ((h0 + g) * M + mp) * dim, h0 + g, own, slot, p, n_pool, j_lo,
+                             lo + w * kCgKeys, hi, s_o + (w * kCgHeads + g) * vdim, s_ml + (w * kCgHeads + g) * 2);
+    }
     __syncthreads();
     for (int i = threadIdx.x; i < nh * vdim; i += 32 * kCgWarps) {
         const int g = i / vdim, c = i - g * vdim, hh = h0 + g, vh = vhead(g);
