@@ -1,7 +1,7 @@
 // Attention of a step with several tokens per sequence on the 5th-generation tensor cores, bf16 storage: the tile kernels of
 // seq_cached_attn.cu and seq_window_attn.cu for the sizes and addresses it takes.
 //
-// A block = 128 consecutive query rows of one (sequence, virtual head) = the 128 lanes of tensor memory; two blocks share an
+// A block = 128 consecutive query rows of one (sequence, head) = the 128 lanes of tensor memory; two blocks share an
 // SM.  Tiles of 32 keys run through three stages that overlap:
 //   warps 5-6  bring key and value rows into the 128-byte-swizzled images the tensor core reads, several tiles ahead: with TMA
 //              where the 32 rows are neighbours in the step and heads are whole pieces of 64 numbers, else with 16-byte
@@ -490,7 +490,7 @@ static int launch_ta(const CachedAttnArgs& a, const StepKeys& x, const Batch& b,
             if (rc == 0 && x.kdim < a.dim) rc = encode_map(&ms, x.ks, a.dim - x.kdim, b.n_tokens, 1, x.ldks, 0, kTaK);
             if (rc == 0) rc = encode_map(&mv, x.v, (uint64_t)a.heads * a.vdim, b.n_tokens, 1, x.ldv, 0, kTaK);
         } else {
-            const uint64_t row = (uint64_t)a.kv_heads * (a.maps * a.dim + a.vdim);
+            const uint64_t row = (uint64_t)a.kv_heads * (a.dim + a.vdim);
             rc = encode_map(&mk, a.kv, row, b.n_tokens, 1, row, 0, kTaK);
             mv = mk;
         }
@@ -500,7 +500,7 @@ static int launch_ta(const CachedAttnArgs& a, const StepKeys& x, const Batch& b,
     auto kernel = attention_tc_kernel<MODE, SHAPED, STEP>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
-    kernel<<<dim3((b.max_seq_len + kTaQ - 1) / kTaQ, a.heads * a.maps * a.vheads, b.n_seqs), kTaThreads, smem, st>>>(mk, ms, mv, a, x, b, z);
+    kernel<<<dim3((b.max_seq_len + kTaQ - 1) / kTaQ, a.heads, b.n_seqs), kTaThreads, smem, st>>>(mk, ms, mv, a, x, b, z);
     return 0;
 }
 

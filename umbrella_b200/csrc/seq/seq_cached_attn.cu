@@ -431,11 +431,9 @@ __global__ void __launch_bounds__(32 * kCgWarps, 3) cached_attention_decode_grou
     const int dim = a.dim, vdim = a.vdim, G = a.heads / a.kv_heads, chunks = (G + kCgHeads - 1) / kCgHeads;
     const GroupSizes z = group_sizes(dim, vdim);
     const int split = blockIdx.x, s = blockIdx.z, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int gc = blockIdx.y % chunks, gv = blockIdx.y / chunks;           // which eight of the group's heads; (key/value head, map, value head)
-    const int C = a.vheads, M = a.maps, cv = gv % C, mp = gv / C % M, kvh = gv / C / M;
+    const int gc = blockIdx.y % chunks, kvh = blockIdx.y / chunks;          // which eight of the group's heads
     const int h0 = kvh * G + gc * kCgHeads, nh = min(kCgHeads, G - gc * kCgHeads);
-    auto vhead = [&](int i) { return ((h0 + i) * M + mp) * C + cv; };
-    const VHead v0 = virtual_head(a, vhead(0));
+    const VHead v0 = virtual_head(a, h0);                                   // (one map, one value head: the rule asks for a bf16 result)
     const int t = b.seq_start[s], p = b.seq_pos0[s], slot = b.seq_slot[s];
     const int window = a.window > 0 ? a.window : (1 << 30);
     const int n_pool = pooled_visible(p, window, a.pool);
@@ -493,7 +491,7 @@ __global__ void __launch_bounds__(32 * kCgWarps, 3) cached_attention_decode_grou
     // rows of the products: head hr; a lane's places in a row's pairs of numbers: 2 qd, 2 qd + 1
     const int hr = lane >> 2, qd = lane & 3, h = h0 + min(hr, nh - 1), ksteps = (dim + 15) / 16, nvt = vdim / 8;
     uint32_t qa[8][2];
-    const __nv_bfloat16* qrow = (const __nv_bfloat16*)a.q + (int64_t)t * v0.qstride + (h * M + mp) * dim;
+    const __nv_bfloat16* qrow = (const __nv_bfloat16*)a.q + (int64_t)t * v0.qstride + h * dim;
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks)
 #pragma unroll
@@ -614,12 +612,12 @@ __global__ void __launch_bounds__(32 * kCgWarps, 3) cached_attention_decode_grou
     if (__any_sync(0xffffffffu, hr < nh && odd != 0.f)) {
         __syncwarp();
         for (int g = 0; g < nh; ++g)
-            plain_part<MODE>(a, v0, (const __nv_bfloat16*)a.q + (int64_t)t * v0.qstride + ((h0 + g) * M + mp) * dim, h0 + g, own, slot, p, n_pool, j_lo,
+            plain_part<MODE>(a, v0, (const __nv_bfloat16*)a.q + (int64_t)t * v0.qstride + (h0 + g) * dim, h0 + g, own, slot, p, n_pool, j_lo,
                              lo + w * kCgKeys, hi, s_o + (w * kCgHeads + g) * vdim, s_ml + (w * kCgHeads + g) * 2);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < nh * vdim; i += 32 * kCgWarps) {
-        const int g = i / vdim, c = i - g * vdim, hh = h0 + g, vh = vhead(g);
+        const int g = i / vdim, c = i - g * vdim, hh = h0 + g;
         float Mx = -INFINITY, L = 0.f, O = 0.f;
         if (MODE == UMBS_ATTN_SIGMOID) {
             for (int ww = 0; ww < kCgWarps; ++ww) O += s_o[(ww * kCgHeads + g) * vdim + c];
@@ -635,7 +633,7 @@ __global__ void __launch_bounds__(32 * kCgWarps, 3) cached_attention_decode_grou
             if (n_split == 1 && MODE == UMBS_ATTN_SOFTMAX_SINK) L += expf(sk - Mx);
         }
         if (n_split > 1) {
-            float* pr = part + (((int64_t)t * v0.nv + vh) * n_split + split) * (vdim + 2);
+            float* pr = part + (((int64_t)t * a.heads + hh) * n_split + split) * (vdim + 2);
             pr[c] = O;
             if (c == 0) { pr[vdim] = Mx; pr[vdim + 1] = L; }
             continue;
@@ -692,7 +690,7 @@ static bool group_fits(const CachedAttnArgs& a) {
            (a.pool <= 0 || al(a.pool_cache));
 }
 static int group_blocks(const CachedAttnArgs& a) {
-    return a.kv_heads * a.maps * a.vheads * ((a.heads / a.kv_heads + kCgHeads - 1) / kCgHeads);
+    return a.kv_heads * ((a.heads / a.kv_heads + kCgHeads - 1) / kCgHeads);
 }
 
 template <int MODE>
@@ -704,8 +702,7 @@ static int launch_group(const CachedAttnArgs& a, const Batch& b, int n_split, fl
         if (e != cudaSuccess) return (int)e;
     }
     kernel<<<dim3(n_split, group_blocks(a), b.n_seqs), 32 * kCgWarps, smem, st>>>(a, b, n_split, part);
-    const int nv = a.heads * a.maps * a.vheads;
-    if (n_split > 1) cached_attention_merge_kernel<__nv_bfloat16, MODE><<<b.n_tokens * nv, a.vdim <= 128 ? 128 : 256, 0, st>>>(a, n_split, part);
+    if (n_split > 1) cached_attention_merge_kernel<__nv_bfloat16, MODE><<<b.n_tokens * a.heads, a.vdim <= 128 ? 128 : 256, 0, st>>>(a, n_split, part);
     return 0;
 }
 static int launch_group_any(int mode, const CachedAttnArgs& a, const Batch& b, int n_split, float* part, cudaStream_t st) {

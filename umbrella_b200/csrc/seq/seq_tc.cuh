@@ -51,14 +51,6 @@ __device__ __forceinline__ bool tc_poll(uint64_t* bar, uint32_t parity, volatile
     }
     return tc_give_up(quit);
 }
-// parked: for waits that may be long
-__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* quit) {
-    for (int i = 0; i < (1 << 20); ++i) {
-        if (umb::mbar_try_wait(bar, parity)) return true;
-        if (*quit) return false;
-    }
-    return tc_give_up(quit);
-}
 // Behind the last barrier of a kernel that gave up: the host learns of it (give_up_word), and copies and products in flight end
 // before their memory goes.
 __device__ __forceinline__ void tc_settle(volatile int* quit, volatile unsigned int* report) {
