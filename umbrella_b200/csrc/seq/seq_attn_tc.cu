@@ -453,9 +453,10 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
 
 // As many key and value tiles as leave room for a second block on the SM (228 KB, 1 KB of it per block the system's): four, or
 // three beside queries of more than 128 numbers.
+constexpr int kTaTiles = 110 * 1024, kTaSmem = 1024 + kTaTiles;     // the largest of them
 static TaDims ta_dims(const CachedAttnArgs& a) {
     TaDims z{(a.dim + 63) / 64, (a.dim + 15) / 16, (a.vdim + 63) / 64, kTaStages, 0, nullptr};
-    while (z.stages > 3 && z.q_atoms * (kTaQ * 128) + z.stages * (z.q_atoms + z.v_atoms) * (kTaK * 128) > 110 * 1024) --z.stages;
+    while (z.stages > 3 && z.q_atoms * (kTaQ * 128) + z.stages * (z.q_atoms + z.v_atoms) * (kTaK * 128) > kTaTiles) --z.stages;
     return z;
 }
 
@@ -498,7 +499,8 @@ static int launch_ta(const CachedAttnArgs& a, const StepKeys& x, const Batch& b,
     }
     const int smem = 1024 + (z.q_atoms * (kTaQ + z.stages * kTaK) + z.stages * z.v_atoms * kTaK) * 128;
     auto kernel = attention_tc_kernel<MODE, SHAPED, STEP>;
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // (always the same limit: another thread may be between setting it and its launch)
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTaSmem);
     if (e != cudaSuccess) return (int)e;
     kernel<<<dim3((b.max_seq_len + kTaQ - 1) / kTaQ, a.heads, b.n_seqs), kTaThreads, smem, st>>>(mk, ms, mv, a, x, b, z);
     return 0;

@@ -697,8 +697,8 @@ template <int MODE>
 static int launch_group(const CachedAttnArgs& a, const Batch& b, int n_split, float* part, cudaStream_t st) {
     const int tiles = kCgWarps * group_sizes(a.dim, a.vdim).warp_bytes, merge = kCgWarps * kCgHeads * (a.vdim + 2) * 4, smem = tiles > merge ? tiles : merge;
     auto kernel = cached_attention_decode_group_kernel<MODE>;
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (smem > 48 * 1024) {                                 // (always the same limit: another thread may be between setting it and its launch)
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCgWarps * group_sizes(128, 128).warp_bytes);
         if (e != cudaSuccess) return (int)e;
     }
     kernel<<<dim3(n_split, group_blocks(a), b.n_seqs), 32 * kCgWarps, smem, st>>>(a, b, n_split, part);

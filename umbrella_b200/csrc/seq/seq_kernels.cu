@@ -1269,8 +1269,8 @@ extern "C" int umbs_moe_route_scaled(int dtype, const void* h, int n, int width,
 #define UMBS_ROUTER(TT)                                                                                                          \
     UMBS_DISPATCH_T(dtype, {                                                                                                     \
         const size_t smem = (size_t)TT * experts * sizeof(float);                                                                \
-        if (smem > 48 * 1024) {                                                                                                  \
-            e = cudaFuncSetAttribute(moe_router_kernel<T, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
+        if (smem > 48 * 1024) {     /* always the same limit: another thread may be between setting it and its launch */          \
+            e = cudaFuncSetAttribute(moe_router_kernel<T, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);          \
             if (e != cudaSuccess) return (int)e;                                                                                 \
         }                                                                                                                        \
         moe_router_kernel<T, TT><<<(n + TT - 1) / TT, rthreads, smem, st>>>((const T*)h, n, width, w_router, experts, top, mode, groups, keep, \
