@@ -838,25 +838,23 @@ extern "C" int umbs_cached_attention_ex(int dtype, int mode, const void* q, cons
         if (a.chunk > 0 && keys > a.chunk) keys = a.chunk;
         const bool group = dtype == UMBS_BF16 && group_fits(a);
         const int rows = batch->n_seqs * heads;
+        const size_t per_split = (size_t)rows * (vdim + 2) * sizeof(float);
+        const int room = split_scratch == nullptr || per_split == 0 ? 1 : (int)std::clamp<size_t>(split_bytes / per_split, 1, 32);
         int n_split = 1;
         if (group) {
             // heads that share a key/value head in one block, three blocks on an SM, 128 keys a round of its warps: the split with
             // the fewest rounds from first to last block, one more per block for its start and end
             const int64_t blocks = (int64_t)batch->n_seqs * group_blocks(a);
             int64_t best = INT64_MAX;
-            for (int n = 1; n <= 32 && (n == 1 || (n - 1) * 128 < keys); ++n) {
+            for (int n = 1; n <= room && (n == 1 || (n - 1) * 128 < keys); ++n) {
                 const int64_t cost = (blocks * n + 443) / 444 * ((keys + n * 128 - 1) / (n * 128) + 1) + (n > 1);
                 if (cost < best) { best = cost; n_split = n; }
             }
         } else {
             n_split = (keys + 255) / 256;
             n_split = n_split < 1 ? 1 : (n_split > 32 ? 32 : n_split);
-            if (n_split > (296 + rows - 1) / rows) n_split = (296 + rows - 1) / rows;
+            n_split = std::min(n_split, std::min((296 + rows - 1) / rows, room));
         }
-        const size_t per_split = (size_t)rows * (vdim + 2) * sizeof(float);
-        if (split_scratch == nullptr || per_split == 0) n_split = 1;
-        else if ((size_t)n_split * per_split > split_bytes) n_split = (int)(split_bytes / per_split);
-        if (n_split < 1) n_split = 1;
         if (group) rc = launch_group_any(mode, a, *batch, n_split, split_scratch, st);
         else if (dtype == UMBS_BF16) rc = launch_decode_any<__nv_bfloat16>(mode, a, *batch, n_split, split_scratch, st);
         else if (dtype == UMBS_F32) rc = launch_decode_any<float>(mode, a, *batch, n_split, split_scratch, st);
