@@ -405,7 +405,7 @@ __device__ __forceinline__ void mma_top(float (&d)[4], uint32_t a0, uint32_t a2,
 
 // A warp's triple of one head in plain fp32: every fourth tile of the keys [lo, hi) from the warp's own, key after key.
 template <int MODE>
-__device__ __noinline__ void plain_part(const CachedAttnArgs& a, const VHead& v, const __nv_bfloat16* q, int h, const __nv_bfloat16* own, int slot, int p, int n_pool,
+__device__ __forceinline__ void plain_part(const CachedAttnArgs& a, const VHead& v, const __nv_bfloat16* q, int h, const __nv_bfloat16* own, int slot, int p, int n_pool,
                                         int j_lo, int first, int hi, float* s_o, float* s_ml) {
     const int lane = threadIdx.x & 31;
     PlainRow s;
