@@ -676,7 +676,7 @@ __device__ __forceinline__ int lowest_not_in(const int32_t* chosen, int n, int l
     return -1;
 }
 __device__ __forceinline__ void route_choose(float* z, int experts, int top, int mode, int groups, int keep, float wscale,
-                                             float* __restrict__ w_out, int32_t* e_out, int32_t* counts) {
+                                             float* __restrict__ w_out, int32_t* __restrict__ e_out, int32_t* counts) {
     if (mode == UMBS_ROUTE_SIGMOID_GROUPS) {
         const int per = experts / groups;
         for (int e = 0; e < experts; ++e) z[e] = 1.f / (1.f + expf(-z[e]));
