@@ -119,3 +119,27 @@ def test_groups_that_run_backwards_are_taken(ops):
     got = ops.gemm(x[:, 128:], w, out_f32=True, groups=3, a_goff=-64, c_goff=48)
     ref = torch.cat([x[:, 128 - 64 * i:192 - 64 * i].double() @ w[i].double().T for i in range(3)], 1)
     assert H.rel_err(got, ref.cpu()) < F32_TOL
+
+
+@pytest.mark.parametrize("act", ["CLAMPED_GLU", "GELU_TANH", "SILU"])
+@pytest.mark.parametrize("M", [17, 300])
+def test_activations_are_those_of_the_fp32_kernels(ops, act, M):
+    """Weight rows with a single one make every sum a bf16 number exactly, so the results show the activation alone.  They are those of
+    the fp32 kernel bit for bit (a sigmoid below 2^-126 is 0 here and a subnormal number there: 1e-35 covers it times a number of the
+    row), and within 1e-6 of float64 in the norm (a tanh or an exponential of two units in the last place, an argument rounded three
+    times)."""
+    from umbrella_b200 import _lib_seq as S
+    K, N = 64, 32
+    a = _mat(61, M, K, scale=3.0)
+    a[0, :8] = torch.tensor([0.0, 1e-30, 88.0, -88.0, 100.0, -100.0, 3e38, -3e38], dtype=torch.bfloat16)
+    w = torch.zeros(2 * N, K, dtype=torch.bfloat16, device=DEV)
+    w[torch.arange(2 * N), torch.arange(2 * N) % K] = 1.0                 # gate n reads number n, up n reads number 32 + n
+    run = lambda x, y: ops.gemm_ex(x, y, out_f32=True, act=getattr(S, "UMBS_ACT_" + act), limit=7.0)
+    got, f32 = run(a, w), run(a.float(), w.float())
+    assert bool(((got == f32) | ((got - f32).abs() < 1e-35)).all())
+    g, u = a[1:, :N].double(), a[1:, N:].double()
+    if act == "CLAMPED_GLU":
+        g, u = g.clamp(max=7.0), u.clamp(-7.0, 7.0) + 1
+    f = {"CLAMPED_GLU": lambda t: t * torch.sigmoid(1.702 * t), "SILU": torch.nn.functional.silu,
+         "GELU_TANH": lambda t: torch.nn.functional.gelu(t, approximate="tanh")}[act]
+    assert H.rel_err(got[1:], (f(g) * u).cpu()) < 1e-6

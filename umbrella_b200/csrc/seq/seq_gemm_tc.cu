@@ -11,7 +11,9 @@
 // the rest of the batch; against float64 it is as far off as the mma.sync tiles that this replaced (2.1e-6 at K = 2048, in
 // both the tensor core's own accumulation).
 //
-// Bound: L2 for dense prompts (48 KB of tiles per 512 clocks of products on every SM, 13 TB/s over the chip).  4096 x 2048 -> 6144
+// Bound for dense prompts: bringing the tiles from L2, and the last round.  A k step is 48 KB for 512 clocks of products on every
+// SM, 26 TB/s over the chip if the products never waited; 4096 x 2048 -> 6144 passes 1.21 GB of them in 109 us, 11 TB/s, and its 768
+// tiles are 5.2 rounds of the 148 SMs run as 6.  That product
 // (fp32 out): 650 us on 128 x 64 mma.sync tiles (159 TFLOP/s, fragments fetched from shared memory by every warp, 100 MB
 // cleared first), 109 us here (947 TFLOP/s).  16 experts, top 2, 4096 tokens of width 2048 with the routing around it:
 // 808 -> 229 us; 64 tokens: 213 -> 98 us.
@@ -74,10 +76,14 @@ struct TcCfg {
 
 // Bias and activation of 32 neighbouring columns of a row, v (and u, the up half) in place.  One choice of activation in
 // front of a loop over independent elements: chosen element by element, every exponential and every quotient waited for the
-// one before it (25 to 40 us for a tile's 128 x 128 outputs, several times its products).  Quotients are within two units in
-// the last place here; the sums they scale carry the tensor core's error, an order of magnitude more.  ((1 + tanh(z)) / 2 is
-// the sigmoid of 2 z.)
-__device__ __forceinline__ float tc_sigmoid(float z) { return __fdividef(1.f, 1.f + expf(-z)); }
+// one before it (25 to 40 us for a tile's 128 x 128 outputs, several times its products).
+// The sigmoids' quotient without the rounded division's branch, which costs 12 us of 50 over 4096 rows of 2 x 2048 sums: the
+// hardware's approximate reciprocal and one Newton-Raphson step, r (2 - x r) with the residual in one rounding.  Behind 2^126 the
+// quotient is below the smallest normal number and becomes 0.
+__device__ __forceinline__ float tc_sigmoid(float z) {
+    const float x = 1.f + expf(-z), r = __fdividef(1.f, x);
+    return x >= 0x1p126f ? 0.f : fmaf(r, fmaf(-x, r, 1.f), r);
+}
 template <bool DUAL>
 __device__ __forceinline__ void tc_finish(const GemmArgs& a, uint32_t (&v)[32], uint32_t (&u)[DUAL ? 32 : 1], int n0) {
 #define UMBS_F(x) __uint_as_float(x)
@@ -96,13 +102,13 @@ __device__ __forceinline__ void tc_finish(const GemmArgs& a, uint32_t (&v)[32], 
         }
     }
     if (DUAL) {
-        if (a.act == UMBS_ACT_GELU_TANH) UMBS_EACH(x * tc_sigmoid(1.5957691216057308f * (x + 0.044715f * x * x * x)) * y)
+        if (a.act == UMBS_ACT_GELU_TANH) UMBS_EACH(gated_act(x, y, a.limit, UMBS_ACT_GELU_TANH))
         else if (a.act == UMBS_ACT_SILU) UMBS_EACH(x * tc_sigmoid(x) * y)
         else UMBS_EACH(fminf(x, a.limit) * tc_sigmoid(1.702f * fminf(x, a.limit)) * (fminf(fmaxf(y, -a.limit), a.limit) + 1.f))
     } else if (a.unary && n0 + 32 <= a.unary_cols && (a.unary == UMBS_UNARY_SILU || a.unary == UMBS_UNARY_RELU2 || a.unary == UMBS_UNARY_SCALE)) {
         if (a.unary == UMBS_UNARY_SILU) UMBS_EACH(x * tc_sigmoid(x))
-        else if (a.unary == UMBS_UNARY_RELU2) UMBS_EACH(fmaxf(x, 0.f) * fmaxf(x, 0.f))
-        else UMBS_EACH(a.p0 * x)
+        else if (a.unary == UMBS_UNARY_RELU2) UMBS_EACH(unary_act(x, UMBS_UNARY_RELU2, a.p0, a.p1))
+        else UMBS_EACH(unary_act(x, UMBS_UNARY_SCALE, a.p0, a.p1))
     } else if (a.unary) {
         UMBS_EACH(n0 + j < a.unary_cols ? unary_act(x, a.unary, a.p0, a.p1) : x)
     }
@@ -387,9 +393,9 @@ int launch_gemm_tc(const GemmArgs& a, int groups, bool dual, bool c_f32, cudaStr
     t.m_tiles = (a.M + kTcRows - 1) / kTcRows;
     const int es = c_f32 ? 4 : 2;
     t.vec_c = (uintptr_t)a.C % (4 * es) == 0 && a.ldc % 4 == 0 && a.c_goff % 4 == 0;
-    // The tile width with the shortest longest walk: rounds of tiles over the SMs times a k step's cost, which is the tensor
-    // core's 128 clocks for 256 columns and more than half, a quarter of that for 128 and 64 (the activation tile is fetched
-    // and read from shared memory for fewer products).  (Rows sorted by expert: how they fall is only known on the device;
+    // The tile width with the shortest longest walk: rounds of tiles over the SMs times what 16 of k cost, which is the tensor
+    // core's 128 clocks for 256 columns and more than half, a quarter of that for 128 and 64: 72 and 52 (the activation tile is
+    // fetched and read from shared memory for fewer products).  (Rows sorted by expert: how they fall is only known on the device;
     // spread evenly is the guess.)
     const int64_t m = a.grp_off != nullptr ? (int64_t)groups * ((a.M + groups * kTcRows - 1) / (groups * kTcRows)) : (int64_t)groups * t.m_tiles;
     auto cost = [&](int bn, int step) {
