@@ -19,13 +19,13 @@
 namespace umbs {
 
 // ------------------------------------------------------------------------------------------------ SIMT
-// 64 x 64 outputs per block of 64 threads, 8 x 8 a thread (with DUAL: 8 rows x 4 gate and the same 4 up columns), k in steps of
+// 64 x 64 outputs per block of 64 threads, 8 x 8 a thread (or, for small products, 16 x 64 and 2 x 8; with DUAL: 8 rows x 4 gate and the same 4 up columns), k in steps of
 // 16 through two shared-memory stages, the next step's numbers on their way in registers.  Per k a thread reads four 16-byte
 // pieces for 64 multiply-adds, two of them an instruction; an output is one chain of additions over k, so it has the same bits
-// in every tiling.  Bound: fp32 multiply-adds.  Blocks are small so that a step of some hundred rows spreads evenly: 777 x 1024
+// in every tiling.  Bound: those loads from shared memory, 2.7 times the time of the multiply-adds.  Blocks are small so that a step of some hundred rows spreads evenly: 777 x 1024
 // -> 3088 are 637 of them.  16 x 16 threads with 4 x 4 outputs and 4-byte loads took 257 us for it (19 TFLOP/s), this
 // takes 178.
-constexpr int BM = 64, BN = 64, BK = 16, BP = BM + 4;
+constexpr int BN = 64, BK = 16;
 
 template <typename T> __device__ __forceinline__ void load_k4(const T* p, int left, bool vec, float (&f)[4]) {
 #pragma unroll
@@ -41,9 +41,10 @@ template <> __device__ __forceinline__ void load_k4<float>(const float* p, int l
     }
 }
 
-template <typename TA, typename TC, bool DUAL>
+template <typename TA, typename TC, bool DUAL, int RT>
 __global__ void __launch_bounds__(64) gemm_simt_kernel(GemmArgs a, int vec, int vec_c) {
-    __shared__ __align__(16) float As[2][BK][BP], Ws[2][BK][BP];
+    constexpr int BM = 8 * RT, LA = BM / 16;                // RT rows a thread; LA: rows of A a thread loads
+    __shared__ __align__(16) float As[2][BK][BM + 4], Ws[2][BK][BN + 4];
     const int g = blockIdx.z;
     int row_lo = 0, rows = a.M;
     if (a.grp_off != nullptr) { row_lo = a.grp_off[g]; rows = a.grp_off[g + 1] - row_lo; }
@@ -55,37 +56,37 @@ __global__ void __launch_bounds__(64) gemm_simt_kernel(GemmArgs a, int vec, int 
     const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
     // loader: a thread takes four k of rows lr, lr + 16, lr + 32, lr + 48 of both tiles
     const int lr = tid >> 2, lk = (tid & 3) * 4;
-    const TA *ap[4], *wp[4];
+    const TA *ap[LA], *wp[4];
+#pragma unroll
+    for (int i = 0; i < LA; ++i) {
+        const int r = lr + 16 * i, p = row_lo + m0 + r;
+        ap[i] = m0 + r < rows ? A + (int64_t)(a.row_src ? a.row_src[p] : p) * a.lda + lk : nullptr;
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int r = lr + 16 * i;
-        ap[i] = wp[i] = nullptr;
-        if (m0 + r < rows) {
-            const int p = row_lo + m0 + r;
-            ap[i] = A + (int64_t)(a.row_src ? a.row_src[p] : p) * a.lda + lk;
-        }
+        wp[i] = nullptr;
         const int n = n0 + (DUAL ? r % OUT : r);            // (DUAL: 32 gate rows, then the 32 up rows)
         if (n < a.N) wp[i] = W + (int64_t)(DUAL && r >= OUT ? a.N + n : n) * a.ldw + lk;
     }
-    float ra[4][4], rw[4][4];
+    float ra[LA][4], rw[4][4];
     auto fetch = [&](int k0) {
         const int left = a.K - k0 - lk;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            load_k4<TA>(ap[i] + k0, ap[i] != nullptr ? left : 0, vec, ra[i]);
-            load_k4<TA>(wp[i] + k0, wp[i] != nullptr ? left : 0, vec, rw[i]);
-        }
+        for (int i = 0; i < LA; ++i) load_k4<TA>(ap[i] + k0, ap[i] != nullptr ? left : 0, vec, ra[i]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) load_k4<TA>(wp[i] + k0, wp[i] != nullptr ? left : 0, vec, rw[i]);
     };
     auto stash = [&](int st) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                As[st][lk + e][lr + 16 * i] = ra[i][e];
+                if (i < LA) As[st][lk + e][lr + 16 * i] = ra[i < LA ? i : 0][e];
                 Ws[st][lk + e][lr + 16 * i] = rw[i][e];
             }
     };
-    f32x2 acc[8][4] = {};                                   // rows ty 4 .. + 3 and 32 + ty 4 ..; columns tx 4 .. + 3 and 32 + tx 4 .., in pairs
+    f32x2 acc[RT][4] = {};                                  // rows ty 4 .. + 3 and 32 + ty 4 .. (RT = 2: 2 ty, + 1); columns tx 4 .. + 3 and 32 + tx 4 .., in pairs
     fetch(0);
     stash(0);
     __syncthreads();
@@ -95,11 +96,16 @@ __global__ void __launch_bounds__(64) gemm_simt_kernel(GemmArgs a, int vec, int 
         if (more) fetch(k0 + BK);
 #pragma unroll
         for (int k = 0; k < BK; ++k) {
-            const float4 a0 = *reinterpret_cast<const float4*>(&As[st][k][ty * 4]), a1 = *reinterpret_cast<const float4*>(&As[st][k][32 + ty * 4]);
+            float av[RT];
+            if constexpr (RT == 8) {
+                *reinterpret_cast<float4*>(av) = *reinterpret_cast<const float4*>(&As[st][k][ty * 4]);
+                *reinterpret_cast<float4*>(av + 4) = *reinterpret_cast<const float4*>(&As[st][k][32 + ty * 4]);
+            } else {
+                *reinterpret_cast<float2*>(av) = *reinterpret_cast<const float2*>(&As[st][k][ty * 2]);
+            }
             const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(&Ws[st][k][tx * 4]), w1 = *reinterpret_cast<const ulonglong2*>(&Ws[st][k][32 + tx * 4]);
-            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < RT; ++i) {
                 const f32x2 aa = pack2(av[i], av[i]);
                 acc[i][0] = fma2(aa, w0.x, acc[i][0]);
                 acc[i][1] = fma2(aa, w0.y, acc[i][1]);
@@ -114,8 +120,8 @@ __global__ void __launch_bounds__(64) gemm_simt_kernel(GemmArgs a, int vec, int 
     }
     TC* C = (TC*)a.C + (int64_t)g * a.c_goff;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int m = m0 + (i >> 2) * 32 + ty * 4 + (i & 3);
+    for (int i = 0; i < RT; ++i) {
+        const int m = m0 + (RT == 8 ? (i >> 2) * 32 + ty * 4 + (i & 3) : ty * 2 + i);
         if (m >= rows) continue;
 #pragma unroll
         for (int half = 0; half < (DUAL ? 1 : 2); ++half) {
@@ -276,14 +282,24 @@ static void launch_skinny(const GemmArgs& a, int groups, bool dual, cudaStream_t
 #undef UMBS_SK2
 }
 
+template <typename TA, typename TC, int RT>
+static void launch_simt_rows(const GemmArgs& a, int groups, bool dual, cudaStream_t st) {
+    const int out = dual ? BN / 2 : BN;
+    const dim3 grid((a.N + out - 1) / out, (a.M + 8 * RT - 1) / (8 * RT), groups);
+    const bool vec = a.lda % 4 == 0 && a.ldw % 4 == 0 && a.a_goff % 4 == 0 && a.w_gstride % 4 == 0 && (((uintptr_t)a.A | (uintptr_t)a.W) & 15) == 0;
+    const bool vec_c = a.ldc % 4 == 0 && a.c_goff % 4 == 0 && ((uintptr_t)a.C & 15) == 0;
+    if (dual) gemm_simt_kernel<TA, TC, true, RT><<<grid, 64, 0, st>>>(a, vec, vec_c);
+    else gemm_simt_kernel<TA, TC, false, RT><<<grid, 64, 0, st>>>(a, vec, vec_c);
+}
+// Tiles of 64 rows where they give every SM a block, else of 16: with few blocks a tile's own length counts, whether its rows are
+// there or not (us with 4 x 4 outputs a thread over 256 threads, as before the 8 x 8 tiles / 64 rows / 16 rows; K = 1024: 1 row to
+// 3088 columns 71 / 74 / 47, 64 rows to 1024 columns 82 / 85 / 45, 64 rows of 16 groups, K = 64: 11 / 29 / 9; 100 rows to 8192
+// columns, 256 blocks: 109 / 89 / 114).
 template <typename TA, typename TC>
 static void launch_simt(const GemmArgs& a, int groups, bool dual, cudaStream_t st) {
     const int out = dual ? BN / 2 : BN;
-    const dim3 grid((a.N + out - 1) / out, (a.M + BM - 1) / BM, groups);
-    const bool vec = a.lda % 4 == 0 && a.ldw % 4 == 0 && a.a_goff % 4 == 0 && a.w_gstride % 4 == 0 && (((uintptr_t)a.A | (uintptr_t)a.W) & 15) == 0;
-    const bool vec_c = a.ldc % 4 == 0 && a.c_goff % 4 == 0 && ((uintptr_t)a.C & 15) == 0;
-    if (dual) gemm_simt_kernel<TA, TC, true><<<grid, 64, 0, st>>>(a, vec, vec_c);
-    else gemm_simt_kernel<TA, TC, false><<<grid, 64, 0, st>>>(a, vec, vec_c);
+    if ((int64_t)((a.N + out - 1) / out) * ((a.M + 63) / 64) * groups < 148) launch_simt_rows<TA, TC, 2>(a, groups, dual, st);
+    else launch_simt_rows<TA, TC, 8>(a, groups, dual, st);
 }
 
 }  // namespace umbs
