@@ -35,7 +35,7 @@ def _feed(fn, lens, size, x):
 
 
 @pytest.mark.parametrize("lens", LENS)
-@pytest.mark.parametrize("dim,vdim,rot", [(64, 128, 64), (32, 64, 12), (4, 4, 0), (60, 132, 60)])
+@pytest.mark.parametrize("dim,vdim,rot", [(64, 128, 64), (32, 64, 12), (24, 64, 12), (36, 64, 0), (4, 4, 0), (60, 132, 60)])
 def test_retention(lens, dim, vdim, rot):
     from umbrella_b200 import ops_seq as K
     heads = 3
@@ -53,7 +53,7 @@ def test_retention(lens, dim, vdim, rot):
 
 
 @pytest.mark.parametrize("lens", LENS)
-@pytest.mark.parametrize("dim,vdim", [(64, 128), (32, 64), (4, 4), (60, 132)])
+@pytest.mark.parametrize("dim,vdim", [(64, 128), (32, 64), (24, 64), (36, 64), (4, 4), (60, 132)])
 def test_mlstm(lens, dim, vdim):
     from umbrella_b200 import ops_seq as K
     heads = 2

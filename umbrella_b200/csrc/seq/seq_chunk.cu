@@ -288,7 +288,9 @@ __global__ void __launch_bounds__(256, 2) chunk_memory_kernel(const ChunkMemory 
     if (norm && tid < dim) st_out[(int64_t)tid * V1 + vdim] = sh.n[tid];
 }
 
-bool chunk_memory_fits(int dim, int vdim) { return dim % 4 == 0 && dim <= kChD && vdim % 4 == 0; }
+// Keys of 28 and 32 numbers walk: the walk's smallest form holds up to 32 of them and a piece's products grow with them (16 sequences
+// of 512 tokens, 4 heads, mLSTM, walked / in pieces: 24 x 32 165 / 159 us, 32 x 32 138 / 164; retention of 64 tokens, 32 x 32: 18 / 21).
+bool chunk_memory_fits(int dim, int vdim) { return dim % 4 == 0 && dim <= kChD && (dim <= 24 || dim > 32) && vdim % 4 == 0; }
 int chunk_base_blocks(int n_seqs, int heads, int vdim) { return n_seqs * heads * ((vdim + kChV - 1) / kChV); }
 
 int chunk_segments(int base_blocks, int max_seq_len, size_t fit, int* seg_len) {

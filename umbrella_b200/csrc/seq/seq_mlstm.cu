@@ -304,9 +304,13 @@ extern "C" int umbs_mlstm(int dtype, const float* proj, int64_t ld, const float*
     const int base_blocks = batch->n_seqs * heads * ((V1 + 31) / 32);
     const size_t per_seg = (size_t)batch->n_seqs * heads * ((size_t)dim * V1 + 1) * sizeof(float);      // states + decay products
     // about four blocks per SM run side by side; two passes pay from three segments on (2 / n_seg of the single walk)
-    const bool chunks = batch->max_seq_len >= 64 && chunk_memory_fits(dim, vdim);       // 32 tokens at a time: seq_chunk.cu
+    // 32 tokens at a time: seq_chunk.cu.  Not where one prompt runs among many decoding sequences: a block of pieces costs its state's
+    // way in and out whatever its tokens (8 heads of 64 x 128, 127 sequences of one token and one of 64, walked / in pieces: 56 / 73 us;
+    // of 4 tokens 63 / 76, of 8 75 / 80; 63 of one token and one of 512 207 / 190).
+    const int chunk_blocks = chunk_base_blocks(batch->n_seqs, heads, vdim);
+    const bool chunks = batch->max_seq_len >= 64 && chunk_memory_fits(dim, vdim) && (chunk_blocks <= 296 || batch->n_tokens >= 10 * (int64_t)batch->n_seqs);
     if (chunks) {
-        n_seg = chunk_segments(chunk_base_blocks(batch->n_seqs, heads, vdim), batch->max_seq_len, seg_scratch != nullptr ? seg_bytes / per_seg : 0, &seg_len);
+        n_seg = chunk_segments(chunk_blocks, batch->max_seq_len, seg_scratch != nullptr ? seg_bytes / per_seg : 0, &seg_len);
     } else if (seg_scratch != nullptr && base_blocks * 3 <= 592 && batch->max_seq_len >= 192) {
         int want = std::min(592 / base_blocks, batch->max_seq_len / 64);
         want = (int)std::min<size_t>(want, seg_bytes / per_seg);
