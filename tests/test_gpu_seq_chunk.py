@@ -71,9 +71,9 @@ def test_mlstm(lens, dim, vdim):
         assert H.rel_err(y, got[0][0]) < 1e-5 and H.rel_err(state, got[0][1]) < 1e-5
 
 
-@pytest.mark.parametrize("vdim", [255, 256, 257, 600])
+@pytest.mark.parametrize("vdim", [1, 32, 33, 64, 65, 128, 129, 255, 256, 257, 600])
 def test_mlstm_rows_around_a_lanes_columns(vdim):
-    """The last kernel takes 256 columns at a time.  Tolerance: fp32 sums of a few dozen terms and one division, as in the
+    """The last kernel takes 32, 64, 128 or 256 columns at a time.  Tolerance: fp32 sums of a few dozen terms and one division, as in the
     operator's own tests."""
     from test_gpu_zed_ops import f32, mlstm_reference, rnd
     from umbrella_b200 import ops_seq as K

@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 #include <algorithm>
+#include <type_traits>
 #include <stdint.h>
 
 #include "seq_chunk.h"
@@ -213,10 +214,10 @@ __global__ void mlstm_chain_kernel(Batch b, int heads, int dim, int V1, const fl
     }
 }
 
-// A warp per (token, head).  Bound in a decode step: the latency of its reads, so a lane asks for 8 columns of all three rows
-// before it uses one (a batch of four through 8 layers, one prompt and 8 decoded tokens: 3480 -> 3443 us).
-constexpr int kMfCols = 8;
-template <typename T>
+// A warp per (token, head).  Bound in a decode step: the latency of its reads, so a lane asks for COLS columns of all three rows
+// before it uses one (a batch of four through 8 layers, one prompt and 8 decoded tokens: 3480 -> 3443 us).  COLS is what the row
+// holds, up to 8: columns that are not there cost their instructions (8192 tokens, 4 heads of 32: 12 us of 150).
+template <typename T, int COLS>
 __global__ void mlstm_finish_kernel(const float* __restrict__ o, const float* __restrict__ gates, const float* __restrict__ proj,
                                     int64_t ld, int off_g, int n, int heads, int vdim, float eps,
                                     const float* __restrict__ norm_w, T* __restrict__ out) {
@@ -226,36 +227,36 @@ __global__ void mlstm_finish_kernel(const float* __restrict__ o, const float* __
     const float* orow = o + (int64_t)w * V1;
     const float* grow = proj + (int64_t)t * ld + off_g + h * vdim;
     const float* nrow = norm_w + h * vdim;
-    auto fetch = [&](const float* row, int e0, float (&r)[kMfCols]) {
+    auto fetch = [&](const float* row, int e0, float (&r)[COLS]) {
 #pragma unroll
-        for (int i = 0; i < kMfCols; ++i) r[i] = e0 + 32 * i < vdim ? row[e0 + 32 * i] : 0.f;
+        for (int i = 0; i < COLS; ++i) r[i] = e0 + 32 * i < vdim ? row[e0 + 32 * i] : 0.f;
     };
-    float v[kMfCols], g[kMfCols], nw[kMfCols];
+    float v[COLS], g[COLS], nw[COLS];
     fetch(orow, lane, v);
     fetch(grow, lane, g);
     fetch(nrow, lane, nw);
     const float den = fmaxf(fabsf(orow[vdim]), gates[(int64_t)w * 3 + 2]) + 1e-6f;
     float ss = 0.f;
-    for (int e0 = lane; e0 < vdim; e0 += 32 * kMfCols) {
+    for (int e0 = lane; e0 < vdim; e0 += 32 * COLS) {
         if (e0 != lane) fetch(orow, e0, v);
 #pragma unroll
-        for (int i = 0; i < kMfCols; ++i) {
+        for (int i = 0; i < COLS; ++i) {
             v[i] /= den;                                            // (columns past the end: 0)
             ss = fmaf(v[i], v[i], ss);
         }
     }
     ss = warp_sum_ml(ss);
     const float inv = 1.f / sqrtf(ss / (float)vdim + eps);
-    for (int e0 = lane; e0 < vdim; e0 += 32 * kMfCols) {
-        if (vdim > 32 * kMfCols) {
+    for (int e0 = lane; e0 < vdim; e0 += 32 * COLS) {
+        if (vdim > 32 * COLS) {
             fetch(orow, e0, v);
             fetch(grow, e0, g);
             fetch(nrow, e0, nw);
 #pragma unroll
-            for (int i = 0; i < kMfCols; ++i) v[i] /= den;
+            for (int i = 0; i < COLS; ++i) v[i] /= den;
         }
 #pragma unroll
-        for (int i = 0; i < kMfCols; ++i)
+        for (int i = 0; i < COLS; ++i)
             if (e0 + 32 * i < vdim) {
                 const float s = 1.f / (1.f + expf(-g[i]));
                 out[(int64_t)t * heads * vdim + h * vdim + e0 + 32 * i] = from_f32<T>(v[i] * inv * nw[i] * s);
@@ -346,12 +347,16 @@ extern "C" int umbs_mlstm(int dtype, const float* proj, int64_t ld, const float*
     }
     if (rc) return rc;
     const int fw = batch->n_tokens * heads;
-    if (dtype == UMBS_BF16)
-        mlstm_finish_kernel<__nv_bfloat16><<<(fw + 3) / 4, 128, 0, st>>>(o_scratch, gates_scratch, proj, ld, off_g, batch->n_tokens,
-                                                                        heads, vdim, eps, out_norm_w, (__nv_bfloat16*)out);
-    else if (dtype == UMBS_F32)
-        mlstm_finish_kernel<float><<<(fw + 3) / 4, 128, 0, st>>>(o_scratch, gates_scratch, proj, ld, off_g, batch->n_tokens, heads,
-                                                                vdim, eps, out_norm_w, (float*)out);
+    auto finish = [&](auto* to) {
+        using T = std::remove_pointer_t<decltype(to)>;
+        auto run = [&](auto kernel) { kernel<<<(fw + 3) / 4, 128, 0, st>>>(o_scratch, gates_scratch, proj, ld, off_g, batch->n_tokens, heads, vdim, eps, out_norm_w, to); };
+        if (vdim <= 32) run(mlstm_finish_kernel<T, 1>);
+        else if (vdim <= 64) run(mlstm_finish_kernel<T, 2>);
+        else if (vdim <= 128) run(mlstm_finish_kernel<T, 4>);
+        else run(mlstm_finish_kernel<T, 8>);
+    };
+    if (dtype == UMBS_BF16) finish((__nv_bfloat16*)out);
+    else if (dtype == UMBS_F32) finish((float*)out);
     else return UMB_ERR_ARG;
     count_launches(launches);
     return (int)cudaGetLastError();
