@@ -146,7 +146,8 @@ def test_keys_of_the_step(ops, dim, shared, vdim):
 
 # ---------------------------------------------------------------------------------------------- decode steps
 # one token per sequence: the first token, a tile of 32 keys and its edges, several tiles per warp, splits, a ring that wraps
-DECODE = [[(0, 1, 0, 0), (1, 1, 31, 0), (2, 1, 32, 0)], [(1, 1, 127, 0)], [(0, 1, 128, 0), (2, 1, 510, 0)], [(2, 1, 700, 0), (0, 1, 33, 0)]]
+DECODE = [[(0, 1, 0, 0), (1, 1, 31, 0), (2, 1, 32, 0)], [(1, 1, 127, 0)], [(0, 1, 128, 0), (2, 1, 510, 0)], [(2, 1, 700, 0), (0, 1, 33, 0)],
+          [(0, 1, 0, 0), (1, 1, 31, 0), (2, 1, 200, 0)]]
 
 
 @pytest.mark.parametrize("heads,kv_heads", [(1, 1), (4, 2), (6, 2), (16, 2), (10, 2)])
@@ -183,3 +184,107 @@ def test_overlapping_rows_of_a_steps_keys_are_taken(ops, which):
     batch = ops.RaggedBatch([(0, T - 20, 0, 0), (1, 20, 0, 0)], DEV)
     run = lambda q, k, ks, v: ops.window_attention_shared(q, k, ks, v, batch, heads, (dim + shared) ** -0.5)
     assert torch.equal(run(**rows), run(**{n: t.contiguous() for n, t in rows.items()}))
+
+
+# ---------------------------------------------------------------------------------------------- against a plain statement in 64 bits
+def _plain64(q, rows, pools, pos0, kv_heads, dim, vdim, heads, window=0, pool=0, mode="softmax", sink=None, bias=None, softcap=0.0, r1=None, r2=None, chunk=0):
+    """One sequence: q [n, heads dim], rows [pos0 + n, kv_heads (dim + vdim)] of positions 0 .., pools [blocks, same].  Everything double."""
+    n, scale, out = q.shape[0], float(torch.tensor(dim ** -0.5)), []
+    pos, j = pos0 + torch.arange(n)[:, None], torch.arange(pos0 + n)[None]
+    see = (j <= pos) & (j > pos - (window or 1 << 30))
+    if chunk:
+        see &= j // chunk == pos // chunk
+    dist, keys = (pos - j).clamp(min=0), rows
+    if pool:
+        keys = torch.cat([rows, pools])
+        see = torch.cat([see, (torch.arange(pools.shape[0])[None] + 1) * pool <= pos - window + 1], 1)
+        dist = torch.cat([dist, torch.zeros(n, pools.shape[0], dtype=torch.long)], 1)
+    for h in range(heads):
+        g = h // (heads // kv_heads)
+        k, v = keys[:, g * dim:(g + 1) * dim], keys[:, kv_heads * dim + g * vdim:kv_heads * dim + (g + 1) * vdim]
+        z = q[:, h * dim:(h + 1) * dim] @ k.T * scale
+        if mode == "sigmoid":
+            out.append((torch.sigmoid(z + bias[h]) * see) @ v)
+            continue
+        if softcap:
+            z = softcap * torch.tanh(z / softcap)
+        if r1 is not None:
+            z = z - r1[h] * torch.log1p(r2[h] * dist)
+        z = z.masked_fill(~see, -float("inf"))
+        z = torch.cat([z, sink[h].expand(n, 1)], 1) if sink is not None else z
+        out.append(torch.softmax(z, 1)[:, :keys.shape[0]] @ v)
+    return torch.cat(out, 1)
+
+
+@pytest.mark.parametrize("seqs", [[(0, 140, 70, 0), (2, 3, 0, 0)], [(1, 300, 0, 0)], [(0, 1, 200, 0), (1, 1, 5, 0)]])
+@pytest.mark.parametrize("dim,vdim", [(128, 128), (72, 40)])
+@pytest.mark.parametrize("kw", [dict(), dict(window=50, pool=16, sink=True), dict(window=70, mode="sigmoid"), dict(softcap=5.0, dist=True), dict(chunk=48)],
+                         ids=lambda k: "-".join(k) or "plain")
+def test_against_float64(ops, seqs, dim, vdim, kw):
+    from umbrella_b200 import _lib_seq as S
+    kw, heads, kv_heads, ring = dict(kw), 4, 2, 320
+    g = torch.Generator(device=DEV).manual_seed(dim)
+    T, row = sum(s[1] for s in seqs), kv_heads * (dim + vdim)
+    q, kv, cache = _r(g, T, heads * dim, s=1.5), _r(g, T, row), _r(g, 3, ring, row)
+    head = torch.randn(heads, generator=g, device=DEV)
+    plain = {k: v for k, v in kw.items() if k in ("window", "pool", "mode", "softcap", "chunk")}
+    before, batch, pools = cache.clone(), ops.RaggedBatch(seqs, DEV), None
+    if kw.get("pool"):
+        p = kw["pool"]
+        pools = cache.reshape(3, ring // p, p, row).float().mean(2).bfloat16()             # what earlier steps left
+    if kw.get("softcap") or kw.get("chunk"):
+        r = dict(r1=head.abs(), r2=head.abs() * 0.1) if kw.pop("dist", False) else {}
+        plain.update({n: t.double().cpu() for n, t in r.items()})
+        got = _scored(ops, q, kv, cache, batch, heads, kv_heads, dim, vdim, dim ** -0.5, **kw, **r)
+    else:
+        extra = dict(sink=head) if kw.pop("sink", False) else dict(head_bias=head) if kw.get("mode") else {}
+        plain.update({"sink" if "sink" in extra else "bias": head.double().cpu()} if extra else {})
+        mode = {"sigmoid": S.UMBS_ATTN_SIGMOID, None: S.UMBS_ATTN_SOFTMAX_SINK if "sink" in extra else S.UMBS_ATTN_SOFTMAX}[kw.pop("mode", None)]
+        got = ops.cached_attention(q, kv, cache, batch, heads, kv_heads, dim, vdim, dim ** -0.5, mode=mode, pool_cache=pools, append=False, **extra, **kw)
+    at = 0
+    for slot, n, pos0, _ in seqs:
+        rows = torch.cat([before[slot, :pos0], kv[at:at + n]]).double().cpu()
+        blocks = (pos0 + n) // kw["pool"] if kw.get("pool") else 0
+        ref = _plain64(q[at:at + n].double().cpu(), rows, pools[slot, :blocks].double().cpu() if blocks else rows[:0], pos0, kv_heads, dim, vdim, heads, **plain)
+        assert H.rel_err(got[at:at + n], ref) < TOL
+        at += n
+
+
+def test_decode_split_is_one_that_the_scratch_holds(ops):
+    """64 sequences of 1055 keys, 16 heads over 4: three splits cost less than one and two cost more (rounds of blocks on the chip), so
+    with room for two the step is not split (one launch), with room for three it is (the second launch merges)."""
+    from umbrella_b200 import _lib_seq as S
+    n, heads, kv_heads, dim = 64, 16, 4, 64
+    g = torch.Generator(device=DEV).manual_seed(9)
+    q, kv, cache = _r(g, n, heads * dim), _r(g, n, 2 * kv_heads * dim), _r(g, n, 1055, 2 * kv_heads * dim)
+    batch, p, lib, outs = ops.RaggedBatch([(i, 1, 1054, 0) for i in range(n)], DEV), ops._p, S.load(), []
+    part = torch.empty(3 * n * heads * (dim + 2), device=DEV)
+    for room, launches in ((0, 1), (1, 1), (2, 1), (3, 2)):
+        out, before = torch.empty(n, heads * dim, dtype=torch.bfloat16, device=DEV), lib.umbs_launch_count()
+        S.check(lib.umbs_cached_attention(S.UMBS_BF16, S.UMBS_ATTN_SOFTMAX, p(q), p(kv), p(cache), 1055, None, 0, ctypes.byref(batch.c), heads, kv_heads, dim, dim,
+                                          0, 0, dim ** -0.5, None, None, 0, 0, p(part) if room else None, 4 * room * n * heads * (dim + 2), p(out), ops._stream()))
+        assert lib.umbs_launch_count() - before == launches, room
+        outs.append(out)
+    for out in outs[1:]:
+        assert H.rel_err(out, outs[0].cpu()) < TOL
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim", [(16, 4, 128), (16, 4, 64), (8, 8, 64)])
+@pytest.mark.parametrize("keys", [1, 16, 17, 32, 33, 64, 65])
+def test_decode_steps_of_few_keys(ops, heads, kv_heads, dim, keys):
+    """Both kernels on either side of the line between them, and a step captured with few keys whose graph is replayed with many."""
+    for n in (1, 3):
+        _both(ops, [(i, 1, keys - 1 - i if keys > i else 0, 0) for i in range(n)], heads, kv_heads, dim, dim)
+    g = torch.Generator(device=DEV).manual_seed(11)
+    q, kv, cache = _r(g, 2, heads * dim, s=1.5), _r(g, 2, 2 * kv_heads * dim), _r(g, 2, 512, 2 * kv_heads * dim)
+    short, far = ops.RaggedBatch([(0, 1, keys - 1, 0), (1, 1, 0, 0)], DEV), ops.RaggedBatch([(0, 1, 300, 0), (1, 1, 511, 0)], DEV)
+    run = lambda b: ops.cached_attention(q, kv, cache, b, heads, kv_heads, dim, dim, dim ** -0.5, append=False)
+    want = [run(short), run(far)]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = run(short)
+    for b, ref in zip((short, far), want):
+        for name, t in b.t.items():
+            short.t[name].copy_(t)
+        graph.replay()
+        assert H.rel_err(out, ref.cpu()) < TOL

@@ -689,6 +689,19 @@ static bool group_fits(const CachedAttnArgs& a) {
     return a.raw == nullptr && a.dim % 8 == 0 && a.vdim % 8 == 0 && a.dim <= 128 && a.vdim <= 128 && al(a.q) && al(a.kv) && al(a.kv_cache) &&
            (a.pool <= 0 || al(a.pool_cache));
 }
+// Few keys: a block of the grouped kernel is a chain of copies and products as long for one key as for 128, 6 us at 64 dimensions and
+// 8 at 128; a block per head takes 4 us for up to 32 keys and 2 for every 32 more, while its blocks are few (16 heads over 4 of
+// 128, us per head / grouped: 8 sequences of 11 keys 4.3 / 8.4, of 64 6.9 / 8.2, of 81 8.4 / 8.2; 32 of 11 8.0 / 8.4; 64 of 11 13.7 / 9.0; heads on their
+// own, 64 sequences of 21 keys: 8.6 / 14.5).  A captured step keeps the grouped kernel: its graph is replayed for longer contexts.
+static bool few_keys(const CachedAttnArgs& a, int keys, int rows) {
+    if (a.heads == a.kv_heads && keys <= 32) return true;
+    if (a.dim > 64 && rows <= 512 && keys <= 16) return true;
+    return rows <= 256 && keys <= (a.dim > 64 ? 64 : 32);
+}
+static bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone;
+}
 static int group_blocks(const CachedAttnArgs& a) {
     return a.kv_heads * ((a.heads / a.kv_heads + kCgHeads - 1) / kCgHeads);
 }
@@ -836,8 +849,8 @@ extern "C" int umbs_cached_attention_ex(int dtype, int mode, const void* q, cons
         int keys = window > 0 ? (batch->max_pos0 < window ? batch->max_pos0 + 1 : window + (pool > 0 ? batch->max_pos0 / pool : 0))
                               : batch->max_pos0 + 1;
         if (a.chunk > 0 && keys > a.chunk) keys = a.chunk;
-        const bool group = dtype == UMBS_BF16 && group_fits(a);
         const int rows = batch->n_seqs * heads;
+        const bool group = dtype == UMBS_BF16 && group_fits(a) && !(few_keys(a, keys, rows) && !capturing(st));
         const size_t per_split = (size_t)rows * (vdim + 2) * sizeof(float);
         const int room = split_scratch == nullptr || per_split == 0 ? 1 : (int)std::clamp<size_t>(split_bytes / per_split, 1, 32);
         int n_split = 1;
