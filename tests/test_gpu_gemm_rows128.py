@@ -44,3 +44,46 @@ def test_rows_33_to_128(M, K, N):
     for _ in range(5):
         assert torch.equal(ops.awq_gemm(x, packed, K, N, workspace=ws), out)
     assert int(ws.view(torch.int32).abs().max()) == 0                    # the workspace is handed on clean
+
+
+@pytest.mark.parametrize("M", [33, 49, 64, 65, 128])
+def test_rope_rows_33_to_128(M):
+    """The rotary epilogue stages its output and the rows of cos and sin in each group's own rows: the bits of the product followed by
+    umb_rope_append_f16, with K long enough that tiles are split over blocks."""
+    from umbrella_b200 import ops
+    Hq, Hkv, D, K, S, off = 16, 4, 128, 4096, 256, 77
+    rng = np.random.default_rng(M)
+    N = (Hq + 2 * Hkv) * D
+    x = torch.from_numpy((rng.standard_normal((M, K)) * 0.5).astype(np.float16)).to(DEV)
+    packed = ops.awq_repack(*(torch.from_numpy(t).to(DEV) for t in oawq.random_awq(K, N, 128, rng, scale=0.02)))
+    pos = torch.from_numpy(rng.integers(0, S, M)).to(DEV)
+    ang = torch.rand(S, D, device=DEV) * 6.28
+    cos, sin = ang.cos().to(torch.float16), ang.sin().to(torch.float16)
+    outs = []
+    for fused in (False, True):
+        q = torch.zeros(M, Hq, D, dtype=torch.float16, device=DEV)
+        k = torch.zeros(S, Hkv, D, dtype=torch.float16, device=DEV)
+        v = torch.zeros_like(k)
+        if fused:
+            rope = ops.make_rope_epilogue(q, k, v, cos, sin, pos, Hq, Hkv, D, off)
+            ops.awq_gemm(x, packed, K, N, mode=ops.UMB_EPI_ROPE_QKV, rope=rope, out=torch.zeros(M, N, dtype=torch.float16, device=DEV))
+        else:
+            ops.rope_append(ops.awq_gemm(x, packed, K, N), q, k, v, cos, sin, pos, Hq, Hkv, D, off)
+        outs.append((q, k, v))
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
+    assert outs[1][1][off:off + M].abs().sum() > 0
+
+
+@pytest.mark.parametrize("M", [33, 64, 65, 128])
+def test_logits_with_their_largest_rows_33_to_128(M):
+    """The fp32 results of an AWQ head are the fp16 products' numbers, and the keys name each row's largest."""
+    from umbrella_b200 import ops
+    K, N = 4096, 3072
+    rng = np.random.default_rng(M)
+    packed = ops.awq_repack(*(torch.from_numpy(t).to(DEV) for t in oawq.random_awq(K, N, 128, rng, scale=0.02)))
+    x = torch.from_numpy((rng.standard_normal((M, K)) * 0.5).astype(np.float16)).to(DEV)
+    keys = torch.zeros(M, dtype=torch.int64, device=DEV)
+    logits = ops.awq_gemm(x, packed, K, N, mode=ops.UMB_EPI_LOGITS, argmax=keys)
+    assert logits.dtype == torch.float32 and torch.equal(logits, ops.awq_gemm(x, packed, K, N).float())
+    assert torch.equal(ops.argmax_keys_to_ids(keys).cpu(), logits.cpu().argmax(-1))

@@ -83,3 +83,30 @@ def test_mlstm_rows_around_a_lanes_columns(vdim):
     out = K.mlstm(f32(proj), f32(bias), K.RaggedBatch([(0, n, 0, 0)], DEV), heads, dim, vdim, 10.0, 1e-5, f32(norm), state)
     ref = mlstm_reference(proj, bias, heads, dim, vdim, 10.0, 1e-5, norm)
     assert float((out.double().cpu() - ref.double()).abs().max() / ref.double().abs().max()) < 2e-5
+
+
+# ---------------------------------------------------------------------------------------------- against the plain recurrences in 64 bits
+# (tolerances as in the operators' own tests of shorter steps, test_gpu_seq_ops.py and test_gpu_zed_ops.py)
+@pytest.mark.parametrize("dim,vdim,rot,n", [(64, 128, 64, 200), (60, 132, 12, 64), (4, 4, 0, 97)])
+def test_retention_against_float64(dim, vdim, rot, n):
+    from test_gpu_seq_ops import _ret_inputs, _ret_ref
+    from umbrella_b200 import ops_seq as K
+    from umbrella_b200.models.seq_model import rotary_inv_freq
+    heads, decay, base = 2, [0.93, 0.9995], 50.0
+    qkvg, q, k, v, gate = _ret_inputs(n, heads, dim, vdim, 21)
+    state = torch.full((1, heads, dim, vdim), 5.0, device=DEV)
+    out = K.retention(qkvg.to(DEV), K.RaggedBatch([(0, n, 0, 0)], DEV), heads, dim, vdim, rot, (rotary_inv_freq(rot, base) if rot else torch.zeros(1)).to(DEV),
+                      torch.tensor(decay, device=DEV), 1e-4, state)
+    assert H.row_err(out, _ret_ref(q, k, v, gate, dim, rot, base, decay, 1e-4)) < 2e-5
+
+
+@pytest.mark.parametrize("dim,vdim,n", [(64, 128, 200), (60, 132, 64), (4, 4, 97)])
+def test_mlstm_against_float64(dim, vdim, n):
+    from test_gpu_zed_ops import f32, mlstm_reference, rnd
+    from umbrella_b200 import ops_seq as K
+    heads = 2
+    proj, bias, norm = rnd(n, 2 * heads * (dim + vdim + 1), seed=70), rnd(2 * heads, seed=71), 1.0 + rnd(heads * vdim, seed=72, scale=0.2)
+    state = torch.full((1, heads, dim * (vdim + 1) + 1), 2.5, device=DEV)
+    out = K.mlstm(f32(proj), f32(bias), K.RaggedBatch([(0, n, 0, 0)], DEV), heads, dim, vdim, 10.0, 1e-5, f32(norm), state)
+    ref = mlstm_reference(proj, bias, heads, dim, vdim, 10.0, 1e-5, norm)
+    assert float((out.double().cpu() - ref.double()).abs().max() / ref.double().abs().max()) < 2e-5
