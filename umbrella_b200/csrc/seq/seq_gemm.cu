@@ -22,7 +22,8 @@ namespace umbs {
 // 64 x 64 outputs per block of 64 threads, 8 x 8 a thread (or, for small products, 16 x 64 and 2 x 8; with DUAL: 8 rows x 4 gate and the same 4 up columns), k in steps of
 // 16 through two shared-memory stages, the next step's numbers on their way in registers.  Per k a thread reads four 16-byte
 // pieces for 64 multiply-adds, two of them an instruction; an output is one chain of additions over k, so it has the same bits
-// in every tiling.  Bound: those loads from shared memory, 2.7 times the time of the multiply-adds.  Blocks are small so that a step of some hundred rows spreads evenly: 777 x 1024
+// in every tiling.  Bound: two warps a scheduler (162 registers) that wait on their own
+// chains: issue slots 39 % taken, shared memory 52 %, 2.7 times the time of the multiply-adds alone.  Blocks are small so that a step of some hundred rows spreads evenly: 777 x 1024
 // -> 3088 are 637 of them.  16 x 16 threads with 4 x 4 outputs and 4-byte loads took 257 us for it (19 TFLOP/s), this
 // takes 178.
 constexpr int BN = 64, BK = 16;

@@ -11,12 +11,11 @@
 // the rest of the batch; against float64 it is as far off as the mma.sync tiles that this replaced (2.1e-6 at K = 2048, in
 // both the tensor core's own accumulation).
 //
-// Bound for dense prompts: bringing the tiles from L2, and the last round.  A k step is 48 KB for 512 clocks of products on every
-// SM, 26 TB/s over the chip if the products never waited; 4096 x 2048 -> 6144 passes 1.21 GB of them in 109 us, 11 TB/s, and its 768
-// tiles are 5.2 rounds of the 148 SMs run as 6.  That product
-// (fp32 out): 650 us on 128 x 64 mma.sync tiles (159 TFLOP/s, fragments fetched from shared memory by every warp, 100 MB
+// Bound for dense prompts: the way of a stage from L2, and the last round.  4096 x 2048 -> 6144 has the tensor pipe 61 % active and L2 at
+// 30 % of its throughput; a ring holds four k steps of 48 KB, 512 clocks of products each, and its 768 tiles are 5.2 rounds of the
+// 148 SMs run as 6.  That product (fp32 out): 650 us on 128 x 64 mma.sync tiles (159 TFLOP/s, fragments fetched from shared memory by every warp, 100 MB
 // cleared first), 109 us here (947 TFLOP/s).  16 experts, top 2, 4096 tokens of width 2048 with the routing around it:
-// 808 -> 229 us; 64 tokens: 213 -> 98 us.
+// 808 -> 234 us (gate|up: tensor pipe 42 % active, the copying warps' loads the longest wait); 64 tokens: 213 -> 102 to 110 us.
 #include <cuda.h>
 #include <atomic>
 #include <mutex>
