@@ -158,3 +158,43 @@ def test_general_kernel_rows_have_the_same_bits_in_both_tile_heights(ops, dtype)
     x, v = a[:, :64].contiguous(), w[:48, :32].reshape(2, 24, 32).contiguous()               # groups, a step between them
     got = ops.gemm(x[:17], v, out_f32=True, groups=2, a_goff=32, c_goff=24)
     assert H.rel_err(got, torch.cat([x[:17, 32 * i:32 * i + 32].double() @ v[i].double().T for i in range(2)], 1).cpu()) < F32_TOL
+
+
+# few rows: both forms (multiply-add: 32-bit; tensor core: tiles of 8 and of 16 weight rows, pieces of 16 and of 32 bytes), columns and k that end inside a tile, a piece, a warp's share.  A sum is rounded at most 24 times: pieces, lanes, warps.
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(1, 8), (19, 40), (130, 520), (1030, 1032), (2050, 1304), (515, 4104)])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_few_rows(ops, M, N, K, dt):
+    a, w = _mat(51, M, K).to(dt), _mat(52, N, K).to(dt)
+    if dt == torch.float32:
+        a, w = a + 2.0 ** -9 * _mat(53, M, K).float(), w + 2.0 ** -9 * _mat(54, N, K).float()
+    ref = a.double() @ w.double().T
+    assert H.rel_err(ops.gemm(a, w, out_f32=True), ref.cpu()) < 24 * 2.0 ** -24
+    assert H.rel_err(ops.gemm(a, w), ref.cpu()) < (BF16_TOL if dt == torch.bfloat16 else 24 * 2.0 ** -24)
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("K", [64, 1032, 2048])
+def test_few_rows_sorted_by_expert(ops, dt, K):
+    from umbrella_b200 import _lib_seq as S
+    sizes, ff = (3, 0, 16, 1, 9), 37
+    off = torch.tensor([0, 3, 3, 19, 20, 29], dtype=torch.int32, device=DEV)
+    a, w = _mat(55, 40, K).to(dt), _mat(56, 5, 2 * ff, K, scale=K ** -0.5).to(dt)
+    src = torch.randperm(40, generator=torch.Generator().manual_seed(57))[:29].int().to(DEV)
+    got = ops.gemm(a, w, groups=5, n=ff, dual=True, limit=3.0, grp_off=off, row_src=src, rows=29, max_rows=16)
+    lo = 0
+    for g, n in enumerate(sizes):
+        x = a[src[lo:lo + n].long()].double()
+        gate, up = (x @ w[g, :ff].double().T).clamp(max=3.0), (x @ w[g, ff:].double().T).clamp(-3.0, 3.0)
+        ref = gate * torch.sigmoid(1.702 * gate) * (up + 1)
+        if n:
+            assert H.rel_err(got[lo:lo + n], ref.cpu()) < (BF16_TOL if dt == torch.bfloat16 else 1e-6)
+        lo += n
+
+
+@pytest.mark.parametrize("N,K", [(100, 512), (1030, 2048), (6144, 1024)])
+def test_few_rows_do_not_depend_on_the_others(ops, N, K):
+    a, w = _mat(58, 16, K), _mat(59, N, K)
+    full = ops.gemm(a, w, out_f32=True)
+    for m in (1, 4, 8, 11):
+        assert torch.equal(ops.gemm(a[:m].contiguous(), w, out_f32=True), full[:m])

@@ -2,13 +2,14 @@
 // experts), optionally over expert-sorted gathered rows, optionally with the gated feed-forward activation fused
 // into the epilogue of a gate|up pair of products.
 //
-// Three kernels share one argument block:
+// Four kernels share one argument block:
 //   * gemm_simt_kernel  -- fp32 FMA chains over shared-memory tiles; the UMBS_F32 mode (true 32-bit) and every shape
 //                          the tensor-core kernel does not take (K not a multiple of 32, unaligned rows);
 //   * gemm_tc_kernel    -- bf16 operands through tcgen05 with fp32 accumulators (seq_gemm_tc.cu);
-//   * gemm_skinny_kernel -- bf16, at most 16 rows (decoding): a weight stream with the rows' partial sums in registers.
+//   * gemm_skinny_kernel, gemm_rows_kernel -- few rows (decoding), bf16 and fp32: a weight stream with the rows' partial sums in
+//                          registers.
 // In each of them an output element is one fp32 sum over k in an order that does not depend on the other rows, so a
-// row's result is the same whatever else is in the batch; which kernel runs depends on the row count, and the three
+// row's result is the same whatever else is in the batch; which kernel runs depends on the row count, and they
 // differ from each other by rounding only.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -147,24 +148,189 @@ __global__ void __launch_bounds__(64) gemm_simt_kernel(GemmArgs a, int vec, int 
 }
 
 // ------------------------------------------------------------------------------------------------ few rows (decode)
-// Up to 16 activation rows per group: the product is a stream over the weights, and with few rows what it waits for is the
-// latency of a row's loads, one after the other.  So a weight row is split over KW warps (k in pieces of 256, warp after
+// Up to 16 bf16 activation rows per group: the product is a stream over the weights.  A warp owns R weight rows (with DUAL: R / 2 gate
+// rows and their up rows) and a share of k.  mma.m16n8k16 takes the weights as its 16-row operand and the activations as its 8-column
+// one, or (R = 8) the other way round.  Which k sits where in a product does not matter as long as both operands agree, so a lane
+// fetches 8 V neighbouring k of its weight rows and of its activation rows, straight into the registers that the products read, and U
+// such steps are in flight before the first is used.  KW warps of a block share a tile's k.
+// Sums: every product starts from zero, a step's products are added in fp32 pair by pair, the steps in order, the warps in fp64: no chain
+// runs through the tensor core, which cuts its sums off (5 to 7e-8 from float64 for K = 384 to 4096, 6 to 8e-8 as chains of
+// multiply-adds).  The order depends on the weight's sizes alone: a row's result does not depend on the other rows.  A group without
+// rows returns before touching its weights, so a decode step reads only the experts that were chosen.
+// Bound: a launch, a load's way from HBM and the reduction, one after the other: 8 rows of 2048 to 6144 columns 14.8 -> 6.7 us (3.8 TB/s;
+// the multiply-adds that this replaced unpacked every weight for every row), of 1024 to 1024 3.9 -> 2.5, 16 rows 23.9 -> 9.3.
+// V 16-byte pieces that follow one another: weights, which no other block reads, and activations
+template <int V> __device__ __forceinline__ void load_weights(uint4 (&v)[V], const __nv_bfloat16* p) {
+    if constexpr (V == 2)
+        asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(v[0].x), "=r"(v[0].y), "=r"(v[0].z), "=r"(v[0].w), "=r"(v[1].x), "=r"(v[1].y), "=r"(v[1].z), "=r"(v[1].w) : "l"(p));
+    else
+        asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0].x), "=r"(v[0].y), "=r"(v[0].z), "=r"(v[0].w) : "l"(p));
+}
+template <int V> __device__ __forceinline__ void load_rows(uint4 (&v)[V], const __nv_bfloat16* p) {
+    if constexpr (V == 2)
+        asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(v[0].x), "=r"(v[0].y), "=r"(v[0].z), "=r"(v[0].w), "=r"(v[1].x), "=r"(v[1].y), "=r"(v[1].z), "=r"(v[1].w) : "l"(p));
+    else
+        v[0] = *reinterpret_cast<const uint4*>(p);
+}
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <typename TC, bool DUAL, int R, int NT, int KW, int U, int V>
+__global__ void __launch_bounds__(32 * KW) gemm_skinny_kernel(const GemmArgs a) {
+    constexpr int OUT = DUAL ? R / 2 : R, WR = R / 8;       // output columns of a block; weight rows of a lane
+    __shared__ float part[KW][NT * 8][R + 1];
+    const int g = blockIdx.y;
+    int row_lo = 0, rows = a.M;
+    if (a.grp_off != nullptr) { row_lo = a.grp_off[g]; rows = a.grp_off[g + 1] - row_lo; }
+    if (rows <= 0) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane >> 2, k8 = (lane & 3) * 8 * V, n0 = blockIdx.x * OUT;
+    const __nv_bfloat16* A = (const __nv_bfloat16*)a.A + (int64_t)g * a.a_goff;
+    const __nv_bfloat16* W = (const __nv_bfloat16*)a.W + (int64_t)g * a.w_gstride;
+    const __nv_bfloat16 *w[WR], *x[NT];                     // rows q and q + 8 of the tile, of the activations
+#pragma unroll
+    for (int i = 0; i < WR; ++i) {
+        const int r = q + 8 * i, n = min(n0 + r % OUT, a.N - 1);            // (behind the last row: the last row again, not stored)
+        w[i] = W + (int64_t)(DUAL && r >= OUT ? a.N + n : n) * a.ldw;
+    }
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+        const int m = q + 8 * i;
+        x[i] = m < rows ? A + (int64_t)(a.row_src ? a.row_src[row_lo + m] : row_lo + m) * a.lda : nullptr;
+    }
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    float sum[R == 16 ? NT : 1][4] = {};
+    for (int s = warp * U; s * 32 * V < a.K; s += KW * U) {
+        uint4 wv[WR][U][V], xv[NT][U][V];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int i = 0; i < WR; ++i) {
+                const int k = (s + u) * 32 * V + k8;
+#pragma unroll
+                for (int e = 0; e < V; ++e) wv[i][u][e] = zero;
+                if (k < a.K) load_weights<V>(wv[i][u], w[i] + k);           // (K is a multiple of 8 V)
+            }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int i = 0; i < NT; ++i) {
+                const int k = (s + u) * 32 * V + k8;
+#pragma unroll
+                for (int e = 0; e < V; ++e) xv[i][u][e] = zero;
+                if (x[i] != nullptr && k < a.K) load_rows<V>(xv[i][u], x[i] + k);
+            }
+#pragma unroll
+        for (int i = 0; i < (R == 16 ? NT : 1); ++i) {
+            float d[2 * U * V][4] = {};
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int e = 0; e < V; ++e) {
+                    float (&d0)[4] = d[2 * (u * V + e)], (&d1)[4] = d[2 * (u * V + e) + 1];
+                    const uint4 xl = xv[i][u][e], w0 = wv[0][u][e];
+                    if constexpr (R == 16) {
+                        const uint4 w1 = wv[WR - 1][u][e];
+                        mma_16816(d0, w0.x, w1.x, w0.y, w1.y, xl.x, xl.y);
+                        mma_16816(d1, w0.z, w1.z, w0.w, w1.w, xl.z, xl.w);
+                    } else {
+                        const uint4 xh = NT == 2 ? xv[NT - 1][u][e] : zero;
+                        mma_16816(d0, xl.x, xh.x, xl.y, xh.y, w0.x, w0.y);
+                        mma_16816(d1, xl.z, xh.z, xl.w, xh.w, w0.z, w0.w);
+                    }
+                }
+#pragma unroll
+            for (int h = U * V; h > 0; h >>= 1)
+#pragma unroll
+                for (int c = 0; c < h; ++c)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) d[c][e] += d[c + h][e];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sum[i][e] += d[0][e];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < (R == 16 ? NT : 1); ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int lo = (lane & 3) * 2 + (e & 1), hi = q + (e >> 1) * 8;
+            if (R == 16) part[warp][i * 8 + lo][hi] = sum[i][e];
+            else if (hi < NT * 8) part[warp][hi][lo] = sum[i][e];
+        }
+    __syncthreads();
+    TC* C = (TC*)a.C + (int64_t)g * a.c_goff;
+    for (int i = threadIdx.x; i < OUT * NT * 8; i += 32 * KW) {
+        const int m = i / OUT, o = i % OUT, n = n0 + o;
+        if (n >= a.N || m >= rows) continue;
+        double s[4] = {}, s2[4] = {};
+#pragma unroll
+        for (int p = 0; p < KW; ++p) {
+            s[p & 3] += (double)part[p][m][o];
+            if (DUAL) s2[p & 3] += (double)part[p][m][o + OUT];
+        }
+        const int64_t row = row_lo + m;
+        C[row * a.ldc + n] = from_f32<TC>(finish<DUAL>(a, (float)((s[0] + s[1]) + (s[2] + s[3])), (float)((s2[0] + s2[1]) + (s2[2] + s2[3])), g, row, n));
+    }
+}
+
+// The weight's sizes choose the order of the sums: warps that share a tile's k so that each has its pieces in flight at once, up to
+// what the SMs hold.  Tiles of 8 weight rows (the activations are the 16-row operand then) where tiles of 16 would leave SMs idle, and
+// for 9 to 16 activation rows, whose pieces the registers hold beside one weight row's.  (us, weights not in L2, 8 rows, tiles of
+// 16 / 8 rows: 1024 x 1024 2.8 / 2.7, 2048 x 1024 3.1 / 3.2, 8192 x 1024 5.8 / 6.8; 6144 x 2048 by 4 / 8 / 16 warps 9.0 / 7.3 / 9.3.)
+// The weight's sizes choose the order of the sums: warps that share a tile's k so that each has all or half of its pieces in flight at
+// once, up to what the SMs hold.  Tiles of 8 weight rows (the activations are the 16-row operand then) where tiles of 16 would leave SMs
+// idle, and for 9 to 16 activation rows, whose pieces the registers hold beside one weight row's; the sums are the same in both.
+// us, weights of 50 to 200 MB in turn, 8 rows, the best of the others / the chosen one: 1024 x 1024 2.4 / 2.5, 2048 x 1024 2.6 / 2.6,
+// 8192 x 1024 5.3 / 5.5, 1024 x 2048 2.9 / 2.7, 6144 x 2048 7.3 / 6.7, 1024 x 4096 5.2 / 5.0, 3088 x 4096 9.2 / 7.9.
+template <typename TC, bool DUAL, int NT, int KW, int U, int V>
+static void launch_skinny_tiles(const GemmArgs& a, int groups, int64_t tiles, cudaStream_t st) {
+    if (NT == 1 && tiles >= 128) gemm_skinny_kernel<TC, DUAL, 16, 1, KW, U, V><<<dim3((a.N + (DUAL ? 7 : 15)) / (DUAL ? 8 : 16), groups), 32 * KW, 0, st>>>(a);
+    else gemm_skinny_kernel<TC, DUAL, 8, NT, KW, U, V><<<dim3((a.N + (DUAL ? 3 : 7)) / (DUAL ? 4 : 8), groups), 32 * KW, 0, st>>>(a);
+}
+template <typename TC, bool DUAL, int NT, int V>
+static void launch_skinny_rows(const GemmArgs& a, int groups, cudaStream_t st) {
+    const int64_t tiles = (int64_t)((a.N + (DUAL ? 7 : 15)) / (DUAL ? 8 : 16)) * groups;
+    constexpr int U = 2 / V;                                // steps of 64 k
+    if (a.K <= 512 || (a.K <= 1024 && tiles >= 400)) launch_skinny_tiles<TC, DUAL, NT, 8, U, V>(a, groups, tiles, st);
+    else if (a.K <= 1024 || tiles > 200) launch_skinny_tiles<TC, DUAL, NT, 8, 2 * U, V>(a, groups, tiles, st);
+    else if (tiles > 100) launch_skinny_tiles<TC, DUAL, NT, 16, U, V>(a, groups, tiles, st);
+    else launch_skinny_tiles<TC, DUAL, NT, 16, 2 * U, V>(a, groups, tiles, st);
+}
+template <typename TC, int V>
+static void launch_skinny_pieces(const GemmArgs& a, int groups, bool dual, cudaStream_t st) {
+    if (dual) a.M <= 8 ? launch_skinny_rows<TC, true, 1, V>(a, groups, st) : launch_skinny_rows<TC, true, 2, V>(a, groups, st);
+    else a.M <= 8 ? launch_skinny_rows<TC, false, 1, V>(a, groups, st) : launch_skinny_rows<TC, false, 2, V>(a, groups, st);
+}
+// 32-byte pieces where every row of both operands starts on such a boundary: a load then takes whole lines of eight rows, not halves
+// (2048 x 1024 2.9 -> 2.6, 1024 x 2048 3.7 -> 2.7).
+template <typename TC>
+static void launch_skinny(const GemmArgs& a, int groups, bool dual, cudaStream_t st) {
+    const bool wide = a.K % 16 == 0 && a.lda % 16 == 0 && a.ldw % 16 == 0 && a.a_goff % 16 == 0 && a.w_gstride % 16 == 0 &&
+                      (((uintptr_t)a.A | (uintptr_t)a.W) & 31) == 0;
+    if (wide) launch_skinny_pieces<TC, 2>(a, groups, dual, st);
+    else launch_skinny_pieces<TC, 1>(a, groups, dual, st);
+}
+
+// Few rows of 32-bit operands, on the multiply-add pipe.  What it waits for is the latency of a
+// row's loads, one after the other, so a weight row is split over KW warps (k in pieces of 16 bytes a lane, warp after
 // warp), a thread takes four weight rows (with DUAL: the gate and up rows of two outputs) and has the 16-byte loads of two
 // of its pieces in flight; a block of four warps covers 4 / KW such sets of rows.  Sums are kept as even and odd halves (one
 // instruction for both), added over the lanes by a tree that hands every lane fewer values at each level, then over the
-// warps in order: the order depends on K alone, so a row's result does not depend on the other rows.  A group without rows
-// returns before touching its weights, so a decode step reads only the experts that were chosen.
+// warps in order: the order depends on K alone, so a row's result does not depend on the other rows.
 constexpr int SK_ROWS = 4, SK_WARPS = 4;
 
-__device__ __forceinline__ void bf16x8_to_f32x2(const uint4& v, f32x2 (&f)[4]) {
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) f[i] = pack2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
+__device__ __forceinline__ void unpack_piece(const uint4& v, f32x2 (&f)[2]) {
+    f[0] = (f32x2)v.y << 32 | v.x;
+    f[1] = (f32x2)v.w << 32 | v.z;
 }
 
-template <typename TC, bool DUAL, int MT, int KW>
-__global__ void __launch_bounds__(32 * SK_WARPS) gemm_skinny_kernel(GemmArgs a) {
+template <bool DUAL, int MT, int KW>
+__global__ void __launch_bounds__(32 * SK_WARPS) gemm_rows_kernel(GemmArgs a) {
     constexpr int OUTS = DUAL ? SK_ROWS / 2 : SK_ROWS, SETS = SK_WARPS / KW, V = SK_ROWS * MT;      // outputs per set; sums per thread
+    constexpr int PV = 4, STEP = KW * 32 * PV;              // numbers of a piece; k of the warps' pieces together
     __shared__ float part[SK_WARPS][V];
     const int g = blockIdx.z;
     int row_lo = 0, rows = a.M;
@@ -173,15 +339,15 @@ __global__ void __launch_bounds__(32 * SK_WARPS) gemm_skinny_kernel(GemmArgs a) 
     if (m0 >= rows) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, set = warp / KW, kw = warp % KW;
     const int n0 = (blockIdx.x * SETS + set) * OUTS;
-    const __nv_bfloat16* A = (const __nv_bfloat16*)a.A + (int64_t)g * a.a_goff;
-    const __nv_bfloat16* W = (const __nv_bfloat16*)a.W + (int64_t)g * a.w_gstride;
-    const __nv_bfloat16* wrow[SK_ROWS];
+    const float* A = (const float*)a.A + (int64_t)g * a.a_goff;
+    const float* W = (const float*)a.W + (int64_t)g * a.w_gstride;
+    const float* wrow[SK_ROWS];
 #pragma unroll
     for (int i = 0; i < SK_ROWS; ++i) {
         const int n = min(DUAL ? (n0 + (i >> 1)) : (n0 + i), a.N - 1);      // behind the last row: the last row again, not stored
         wrow[i] = W + (int64_t)(DUAL ? ((i & 1) * a.N + n) : n) * a.ldw;
     }
-    const __nv_bfloat16* arow[MT];
+    const float* arow[MT];
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
         const int p = row_lo + min(m0 + m, rows - 1);
@@ -193,8 +359,8 @@ __global__ void __launch_bounds__(32 * SK_WARPS) gemm_skinny_kernel(GemmArgs a) 
 #pragma unroll
         for (int m = 0; m < MT; ++m) acc[i][m] = 0ull;
     const uint4 zero = make_uint4(0, 0, 0, 0);
-    for (int k = (kw * 32 + lane) * 8; k < a.K; k += 2 * KW * 256) {
-        const int k2 = k + KW * 256;
+    for (int k = (kw * 32 + lane) * PV; k < a.K; k += 2 * STEP) {
+        const int k2 = k + STEP;
         uint4 wv[2][SK_ROWS];
 #pragma unroll
         for (int i = 0; i < SK_ROWS; ++i) wv[0][i] = __ldg(reinterpret_cast<const uint4*>(wrow[i] + k));
@@ -202,17 +368,17 @@ __global__ void __launch_bounds__(32 * SK_WARPS) gemm_skinny_kernel(GemmArgs a) 
         for (int i = 0; i < SK_ROWS; ++i) wv[1][i] = k2 < a.K ? __ldg(reinterpret_cast<const uint4*>(wrow[i] + k2)) : zero;
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-            f32x2 wf[SK_ROWS][4];
+            f32x2 wf[SK_ROWS][PV / 2];
 #pragma unroll
-            for (int i = 0; i < SK_ROWS; ++i) bf16x8_to_f32x2(wv[u][i], wf[i]);
+            for (int i = 0; i < SK_ROWS; ++i) unpack_piece(wv[u][i], wf[i]);
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
-                f32x2 af[4];
-                bf16x8_to_f32x2(u == 0 || k2 < a.K ? *reinterpret_cast<const uint4*>(arow[m] + (u ? k2 : k)) : zero, af);
+                f32x2 af[PV / 2];
+                unpack_piece(u == 0 || k2 < a.K ? *reinterpret_cast<const uint4*>(arow[m] + (u ? k2 : k)) : zero, af);
 #pragma unroll
                 for (int i = 0; i < SK_ROWS; ++i)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[i][m] = fma2(af[e], wf[i][e], acc[i][m]);
+                    for (int e = 0; e < PV / 2; ++e) acc[i][m] = fma2(af[e], wf[i][e], acc[i][m]);
             }
         }
     }
@@ -242,7 +408,7 @@ __global__ void __launch_bounds__(32 * SK_WARPS) gemm_skinny_kernel(GemmArgs a) 
     constexpr int per = 32 / V;                                             // lanes that hold the same value
     if (lane % per == 0) part[warp][lane / per] = v[0];
     __syncthreads();
-    TC* C = (TC*)a.C + (int64_t)g * a.c_goff;
+    float* C = (float*)a.C + (int64_t)g * a.c_goff;
     for (int i = threadIdx.x; i < SETS * OUTS * MT; i += 32 * SK_WARPS) {
         const int st = i / (OUTS * MT), o = i % (OUTS * MT) / MT, m = i % MT, n = (blockIdx.x * SETS + st) * OUTS + o;
         if (n >= a.N || m0 + m >= rows) continue;
@@ -253,21 +419,20 @@ __global__ void __launch_bounds__(32 * SK_WARPS) gemm_skinny_kernel(GemmArgs a) 
             if (DUAL) s2 += part[st * KW + q][(2 * o + 1) * MT + m];
         }
         const int64_t row = row_lo + m0 + m;
-        C[row * a.ldc + n] = from_f32<TC>(finish<DUAL>(a, s, s2, g, row, n));
+        C[row * a.ldc + n] = finish<DUAL>(a, s, s2, g, row, n);
     }
 }
 
-// K alone chooses how many warps share a row: with one the loop over k is the critical path from 512 on.
-template <typename TC>
-static void launch_skinny(const GemmArgs& a, int groups, bool dual, cudaStream_t st) {
-    const int kw = a.K >= 1024 ? 4 : (a.K >= 512 ? 2 : 1);
+// K alone chooses how many warps share a row: with one the loop over k is the critical path from 64 pieces on.
+static void launch_rows(const GemmArgs& a, int groups, bool dual, cudaStream_t st) {
+    const int pieces = a.K / 4, kw = pieces >= 128 ? 4 : (pieces >= 64 ? 2 : 1);
     const int outs_per_block = SK_WARPS / kw * (dual ? SK_ROWS / 2 : SK_ROWS);
     const int mt = a.M <= 1 ? 1 : (a.M <= 2 ? 2 : (a.M <= 4 ? 4 : 8));
     const dim3 grid((a.N + outs_per_block - 1) / outs_per_block, (a.M + mt - 1) / mt, groups), block(32 * SK_WARPS);
-#define UMBS_SK2(MT, KW)                                                              \
-    do {                                                                              \
-        if (dual) gemm_skinny_kernel<TC, true, MT, KW><<<grid, block, 0, st>>>(a);    \
-        else gemm_skinny_kernel<TC, false, MT, KW><<<grid, block, 0, st>>>(a);        \
+#define UMBS_SK2(MT, KW)                                                                  \
+    do {                                                                                  \
+        if (dual) gemm_rows_kernel<true, MT, KW><<<grid, block, 0, st>>>(a);              \
+        else gemm_rows_kernel<false, MT, KW><<<grid, block, 0, st>>>(a);                  \
     } while (0)
 #define UMBS_SK(MT)                                                                   \
     do {                                                                              \
@@ -361,8 +526,13 @@ static int gemm_run(int dtype, const void* A, int64_t lda, int a_goff, const voi
     GemmArgs a{A, lda, a_goff, W, ldw, w_gstride, C, ldc, c_goff, M, N, K, grp_off, row_src, limit,
                (dual == UMBS_ACT_GELU_TANH || dual == UMBS_ACT_SILU) ? dual : UMBS_ACT_CLAMPED_GLU,
                bias, out_gate, ld_gate, gate_goff, gate_n, unary, p0, p1, unary_cols};
-    if (dtype == UMBS_F32) {
-        launch_simt<float, float>(a, groups, dual != 0, st);          // activations are fp32 too: c_f32 changes nothing
+    if (dtype == UMBS_F32) {                                              // activations are fp32 too: c_f32 changes nothing
+        const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) && (a_goff % 4 == 0) && (w_gstride % 4 == 0) &&
+                         ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
+        // (us, tiles of 16 or 64 rows / rows streamed, 48 rows of 1024 to 1024, 3088 and 8192 columns: 44 / 10, 51 / 25, 60 / 60; one row 43 / 2.3,
+        // 54 / 4.6, 51 / 8; a sum's distance from float64 5.7e-7 / 0.9e-7: lanes and warps hold parts of it)
+        if (vec && M <= 48) launch_rows(a, groups, dual != 0, st);
+        else launch_simt<float, float>(a, groups, dual != 0, st);
     } else if (dtype == UMBS_BF16) {
         // 16-byte loads: every row start and group offset must sit on a 16-byte boundary
         const bool vec = (K % 8 == 0) && (lda % 8 == 0) && (ldw % 8 == 0) && (a_goff % 8 == 0) && (w_gstride % 8 == 0) &&
