@@ -198,3 +198,62 @@ def test_few_rows_do_not_depend_on_the_others(ops, N, K):
     full = ops.gemm(a, w, out_f32=True)
     for m in (1, 4, 8, 11):
         assert torch.equal(ops.gemm(a[:m].contiguous(), w, out_f32=True), full[:m])
+
+
+# 32-bit operands as three bf16 parts: tiles of 128 rows and of 32 to 160 columns, k in steps of 64 (sums of two steps are added up), the
+# edges of each.  A product's dropped terms are below 2^-25 of it; sums: 16 terms cut off 8 times in a row (2^-23 each at most), then
+# K / 128 rounded additions; random signs: 1e-6 covers K = 1000.
+F32_SPLIT_TOL = 1e-6
+
+
+def _mat32(seed, *shape, scale=1.0):
+    return (torch.randn(*shape, generator=torch.Generator().manual_seed(seed)) * scale).to(DEV)
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 1028, 1000), (129, 1990, 68), (1200, 33, 516), (777, 513, 128), (300, 5000, 132), (40, 9001, 64)])
+def test_split_products(ops, M, N, K):
+    from umbrella_b200 import _lib_seq as S
+    a, w = _mat32(81, M, K), _mat32(82, N, K)
+    assert H.rel_err(ops.gemm(a, w), (a.double() @ w.double().T).cpu()) < F32_SPLIT_TOL
+    w2, bias, gate = _mat32(83, 2 * N, K, scale=K ** -0.5), _mat32(84, 2 * N), _mat32(85, M, N)
+    z = a.double() @ w2.double().T + bias.double()
+    ref = torch.nn.functional.silu(z[:, :N]) * z[:, N:] * torch.sigmoid(gate.double())
+    assert H.rel_err(ops.gemm_ex(a, w2, act=S.UMBS_ACT_SILU, bias=bias, out_gate=gate), ref.cpu()) < 2 * F32_SPLIT_TOL
+    got = ops.gemm_unary(a, w2[:N].contiguous(), S.UMBS_UNARY_SILU, cols=N // 2)
+    z = a.double() @ w2[:N].double().T
+    assert H.rel_err(got, torch.cat([torch.nn.functional.silu(z[:, :N // 2]), z[:, N // 2:]], 1).cpu()) < 2 * F32_SPLIT_TOL
+
+
+def test_split_products_sorted_by_expert(ops):
+    sizes, ff, K = (130, 0, 3, 260, 1), 200, 196
+    off = torch.tensor([0, 130, 130, 133, 393, 394], dtype=torch.int32, device=DEV)
+    a, w = _mat32(86, 300, K), _mat32(87, 5, 2 * ff, K, scale=K ** -0.5)
+    src = torch.randint(0, 300, (394,), generator=torch.Generator().manual_seed(88)).int().to(DEV)
+    got = ops.gemm(a, w, groups=5, n=ff, dual=True, limit=3.0, grp_off=off, row_src=src, rows=394, max_rows=300)
+    lo = 0
+    for g, n in enumerate(sizes):
+        x = a[src[lo:lo + n].long()].double()
+        gate, up = (x @ w[g, :ff].double().T).clamp(max=3.0), (x @ w[g, ff:].double().T).clamp(-3.0, 3.0)
+        if n:
+            assert H.rel_err(got[lo:lo + n], (gate * torch.sigmoid(1.702 * gate) * (up + 1)).cpu()) < 2 * F32_SPLIT_TOL
+        lo += n
+
+
+def test_split_products_of_numbers_at_the_ends_of_the_range(ops):
+    """Infinite and NaN operands, numbers that round to infinity in bf16, and rows so small that their low parts vanish there."""
+    M, N, K = 200, 2000, 64
+    a, w = _mat32(91, M, K), _mat32(92, N, K)
+    a[0, 3], a[1, 5], a[2, 7], w[9, 11] = float("inf"), float("nan"), 3.4e38, float("-inf")
+    a[3], w[10] = a[3] * 2.0 ** -120, w[10] * 2.0 ** -100
+    w[:, 7] = w[:, 7] * 2.0 ** -20                                   # (the sums of row 2 stay in range)
+    got, ref = ops.gemm(a, w), a.double() @ w.double().T
+    fin = torch.isfinite(ref.float())
+    assert torch.equal(torch.isfinite(got), fin) and torch.equal(torch.isnan(got), torch.isnan(ref))
+    assert torch.equal(got[~fin & ~torch.isnan(ref)], ref[~fin & ~torch.isnan(ref)].float())
+    keep = torch.ones(N, dtype=torch.bool, device=DEV)
+    keep[9] = False
+    for rows in (slice(2, 3), slice(3, 4), slice(4, M)):
+        x, y = got[rows][:, keep].double(), ref[rows][:, keep]
+        assert ((x - y).norm() / y.norm()).item() < F32_SPLIT_TOL
+    x, y = got[4:, 10].double(), ref[4:, 10]
+    assert ((x - y).norm() / y.norm()).item() < F32_SPLIT_TOL

@@ -2,9 +2,10 @@
 // experts), optionally over expert-sorted gathered rows, optionally with the gated feed-forward activation fused
 // into the epilogue of a gate|up pair of products.
 //
-// Four kernels share one argument block:
-//   * gemm_simt_kernel  -- fp32 FMA chains over shared-memory tiles; the UMBS_F32 mode (true 32-bit) and every shape
-//                          the tensor-core kernel does not take (K not a multiple of 32, unaligned rows);
+// Five kernels share one argument block:
+//   * gemm_simt_kernel  -- fp32 FMA chains over shared-memory tiles: every shape that the others do not take (unaligned rows; bf16
+//                          with K not a multiple of 32);
+//   * gemm_split_kernel -- fp32 operands (true 32-bit) as sums of bf16 numbers through tcgen05 (seq_gemm_split.cu);
 //   * gemm_tc_kernel    -- bf16 operands through tcgen05 with fp32 accumulators (seq_gemm_tc.cu);
 //   * gemm_skinny_kernel, gemm_rows_kernel -- few rows (decoding), bf16 and fp32: a weight stream with the rows' partial sums in
 //                          registers.
@@ -529,10 +530,17 @@ static int gemm_run(int dtype, const void* A, int64_t lda, int a_goff, const voi
     if (dtype == UMBS_F32) {                                              // activations are fp32 too: c_f32 changes nothing
         const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) && (a_goff % 4 == 0) && (w_gstride % 4 == 0) &&
                          ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
-        // (us, tiles of 16 or 64 rows / rows streamed, 48 rows of 1024 to 1024, 3088 and 8192 columns: 44 / 10, 51 / 25, 60 / 60; one row 43 / 2.3,
-        // 54 / 4.6, 51 / 8; a sum's distance from float64 5.7e-7 / 0.9e-7: lanes and warps hold parts of it)
-        if (vec && M <= 48) launch_rows(a, groups, dual != 0, st);
-        else launch_simt<float, float>(a, groups, dual != 0, st);
+        // Streamed rows take 2 us and one for 6.5 million products, tiles on the tensor core 6 us and 1.3 for each 64 of k.  (us, multiply-add
+        // tiles / streamed / tensor core, K = 1024: one row of 3088 columns 54 / 4.6 / 29, 64 rows of 1024 45 / 12 / 25, of 3088 51 / 32 / 28, of
+        // 8192 73 / 78 / 31; 200 rows of 3088 85 / - / 32; 128 rows, K = 4096, to 1024 columns 184 / 60 / 90.)
+        if (vec && (M <= 16 || (int64_t)M * N * (dual ? 2 : 1) * groups * K <= (int64_t)8500000 * (K / 64 + 4))) {
+            launch_rows(a, groups, dual != 0, st);
+        } else if (vec) {
+            const int rc = launch_gemm_split(a, groups, dual != 0, st);
+            if (rc != 0) return rc;
+        } else {
+            launch_simt<float, float>(a, groups, dual != 0, st);
+        }
     } else if (dtype == UMBS_BF16) {
         // 16-byte loads: every row start and group offset must sit on a 16-byte boundary
         const bool vec = (K % 8 == 0) && (lda % 8 == 0) && (ldw % 8 == 0) && (a_goff % 8 == 0) && (w_gstride % 8 == 0) &&

@@ -20,45 +20,11 @@
 #include <atomic>
 #include <mutex>
 
-#include "seq_gemm.h"
-#include "seq_tc.cuh"
+#include "seq_gemm_walk.cuh"
 
 namespace umbs {
 
-constexpr int kTcRows = 128, kTcK = 64;                     // tile rows; k per ring stage
 constexpr int kTcStageRow = 36;                             // fp32 row stride of an epilogue warp's 32 x 32 staging block
-
-struct TcArgs {
-    int groups, n_tiles, m_tiles, k_steps;
-    int vec_c;                                              // rows of C take 16-byte (fp32) / 8-byte (bf16) stores of 4 columns
-    int a_grouped, w_grouped;                               // the group coordinate of the tensor maps is used
-    unsigned int* report;                                   // give_up_word()
-};
-
-// The tiles of a block, in the order every role visits them: rows fastest, then columns, then groups.
-struct TileWalk {
-    const GemmArgs& a; const TcArgs& t;
-    int next, g, first, m_tiles, row_lo, rows, m0, n0;
-    __device__ TileWalk(const GemmArgs& a_, const TcArgs& t_) : a(a_), t(t_), next(blockIdx.x), g(-1), first(0), m_tiles(0), row_lo(0), rows(a_.M), m0(0), n0(0) {}
-    __device__ bool step() {
-        while (next >= first + m_tiles * t.n_tiles) {
-            if (++g >= t.groups) return false;
-            first += m_tiles * t.n_tiles;
-            if (a.grp_off != nullptr) {
-                row_lo = a.grp_off[g];
-                rows = a.grp_off[g + 1] - row_lo;
-                m_tiles = (rows + kTcRows - 1) / kTcRows;
-            } else {
-                m_tiles = t.m_tiles;
-            }
-        }
-        const int i = next - first;
-        m0 = i % m_tiles * kTcRows;
-        n0 = i / m_tiles;                                   // in tiles: the caller knows their width
-        next += gridDim.x;
-        return true;
-    }
-};
 
 template <int BN, bool DUAL>
 struct TcCfg {
@@ -410,4 +376,4 @@ int launch_gemm_tc(const GemmArgs& a, int groups, bool dual, bool c_f32, cudaStr
 }  // namespace umbs
 
 extern "C" unsigned int umbs_give_ups_seen(void) { return umbs::give_up_status() != 0; }
-extern "C" unsigned int umbs_kernel_timeouts(void) { return umbs::tc_timeouts() + umbs::attention_tc_timeouts(); }
+extern "C" unsigned int umbs_kernel_timeouts(void) { return umbs::tc_timeouts() + umbs::attention_tc_timeouts() + umbs::split_timeouts(); }
