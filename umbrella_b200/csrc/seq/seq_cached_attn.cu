@@ -255,6 +255,7 @@ __global__ void __launch_bounds__(32 * kCdWarps) cached_attention_decode_kernel(
                                                                                 float* __restrict__ part) {
     __shared__ float sm_o[kCdWarps][32 * kCdMaxPerLane];
     __shared__ float sm_ml[kCdWarps][2];
+    chain_wait();
     const int split = blockIdx.x, vh = blockIdx.y, s = blockIdx.z;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int dim = a.dim, vdim = a.vdim;
@@ -428,6 +429,7 @@ template <int MODE>
 __global__ void __launch_bounds__(32 * kCgWarps, 3) cached_attention_decode_group_kernel(const __grid_constant__ CachedAttnArgs a, const __grid_constant__ Batch b,
                                                                                          int n_split, float* __restrict__ part) {
     extern __shared__ __align__(16) unsigned char smem[];
+    chain_wait();
     const int dim = a.dim, vdim = a.vdim, G = a.heads / a.kv_heads, chunks = (G + kCgHeads - 1) / kCgHeads;
     const GroupSizes z = group_sizes(dim, vdim);
     const int split = blockIdx.x, s = blockIdx.z, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -648,6 +650,7 @@ __global__ void __launch_bounds__(32 * kCgWarps, 3) cached_attention_decode_grou
 // One block per (token, head): the splits' triples, in split order, then the sink, the division and the output gate.
 template <typename T, int MODE>
 __global__ void cached_attention_merge_kernel(CachedAttnArgs a, int n_split, const float* __restrict__ part) {
+    chain_wait();
     const int nv = a.heads * a.maps * a.vheads;
     const int th = blockIdx.x, t = th / nv, h = th - t * nv, vdim = a.vdim, c = threadIdx.x;      // (without options h is the head)
     const float* pr = part + (int64_t)th * n_split * (vdim + 2);
@@ -677,8 +680,8 @@ __global__ void cached_attention_merge_kernel(CachedAttnArgs a, int n_split, con
 template <typename T, int MODE>
 static int launch_decode(const CachedAttnArgs& a, const Batch& b, int n_split, float* part, cudaStream_t st) {
     const int nv = a.heads * a.maps * a.vheads;
-    cached_attention_decode_kernel<T, MODE><<<dim3(n_split, nv, b.n_seqs), 32 * kCdWarps, 0, st>>>(a, b, n_split, part);
-    if (n_split > 1) cached_attention_merge_kernel<T, MODE><<<b.n_tokens * nv, a.vdim <= 128 ? 128 : 256, 0, st>>>(a, n_split, part);
+    chain_launch(cached_attention_decode_kernel<T, MODE>, dim3(n_split, nv, b.n_seqs), 32 * kCdWarps, 0, st, a, b, n_split, part);
+    if (n_split > 1) chain_launch(cached_attention_merge_kernel<T, MODE>, b.n_tokens * nv, a.vdim <= 128 ? 128 : 256, 0, st, a, n_split, part);
     return 0;
 }
 
@@ -714,8 +717,8 @@ static int launch_group(const CachedAttnArgs& a, const Batch& b, int n_split, fl
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCgWarps * group_sizes(128, 128).warp_bytes);
         if (e != cudaSuccess) return (int)e;
     }
-    kernel<<<dim3(n_split, group_blocks(a), b.n_seqs), 32 * kCgWarps, smem, st>>>(a, b, n_split, part);
-    if (n_split > 1) cached_attention_merge_kernel<__nv_bfloat16, MODE><<<b.n_tokens * a.heads, a.vdim <= 128 ? 128 : 256, 0, st>>>(a, n_split, part);
+    chain_launch(kernel, dim3(n_split, group_blocks(a), b.n_seqs), 32 * kCgWarps, smem, st, a, b, n_split, part);
+    if (n_split > 1) chain_launch(cached_attention_merge_kernel<__nv_bfloat16, MODE>, b.n_tokens * a.heads, a.vdim <= 128 ? 128 : 256, 0, st, a, n_split, part);
     return 0;
 }
 static int launch_group_any(int mode, const CachedAttnArgs& a, const Batch& b, int n_split, float* part, cudaStream_t st) {

@@ -11,6 +11,11 @@ namespace umbs {
 static std::atomic<unsigned long long> g_launches{0};
 void count_launches(unsigned n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
+static thread_local int g_chain_depth = 0;
+ChainScope::ChainScope() { ++g_chain_depth; }
+ChainScope::~ChainScope() { --g_chain_depth; }
+bool in_chain() { return g_chain_depth > 0; }
+
 struct Arena {
     char* base;
     size_t used, cap;
@@ -228,6 +233,7 @@ extern "C" int umbs_forward(const umbs_model_t* m, const umbs_batch_t* b, float*
     if ((uintptr_t)workspace % 256 != 0) return UMB_ERR_ARG;
     Scratch s;
     if (carve(m, T, b->n_want, (char*)workspace, &s) > workspace_bytes) return UMB_ERR_WORKSPACE;
+    const ChainScope chain;
     const int64_t plane = (int64_t)T * W;
     const float embed_scale = m->embed_scale != 0.f ? m->embed_scale : 1.f;
     const size_t es = dt == UMBS_F32 ? 4 : 2;

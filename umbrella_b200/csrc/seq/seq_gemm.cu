@@ -184,11 +184,7 @@ template <typename TC, bool DUAL, int R, int NT, int KW, int U, int V>
 __global__ void __launch_bounds__(32 * KW) gemm_skinny_kernel(const GemmArgs a) {
     constexpr int OUT = DUAL ? R / 2 : R, WR = R / 8;       // output columns of a block; weight rows of a lane
     __shared__ float part[KW][NT * 8][R + 1];
-    const int g = blockIdx.y;
-    int row_lo = 0, rows = a.M;
-    if (a.grp_off != nullptr) { row_lo = a.grp_off[g]; rows = a.grp_off[g + 1] - row_lo; }
-    if (rows <= 0) return;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane >> 2, k8 = (lane & 3) * 8 * V, n0 = blockIdx.x * OUT;
+    const int g = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane >> 2, k8 = (lane & 3) * 8 * V, n0 = blockIdx.x * OUT;
     const __nv_bfloat16* A = (const __nv_bfloat16*)a.A + (int64_t)g * a.a_goff;
     const __nv_bfloat16* W = (const __nv_bfloat16*)a.W + (int64_t)g * a.w_gstride;
     const __nv_bfloat16 *w[WR], *x[NT];                     // rows q and q + 8 of the tile, of the activations
@@ -197,15 +193,9 @@ __global__ void __launch_bounds__(32 * KW) gemm_skinny_kernel(const GemmArgs a) 
         const int r = q + 8 * i, n = min(n0 + r % OUT, a.N - 1);            // (behind the last row: the last row again, not stored)
         w[i] = W + (int64_t)(DUAL && r >= OUT ? a.N + n : n) * a.ldw;
     }
-#pragma unroll
-    for (int i = 0; i < NT; ++i) {
-        const int m = q + 8 * i;
-        x[i] = m < rows ? A + (int64_t)(a.row_src ? a.row_src[row_lo + m] : row_lo + m) * a.lda : nullptr;
-    }
     const uint4 zero = make_uint4(0, 0, 0, 0);
-    float sum[R == 16 ? NT : 1][4] = {};
-    for (int s = warp * U; s * 32 * V < a.K; s += KW * U) {
-        uint4 wv[WR][U][V], xv[NT][U][V];
+    uint4 wv[WR][U][V];
+    auto fetch = [&](int s) {
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
@@ -215,6 +205,24 @@ __global__ void __launch_bounds__(32 * KW) gemm_skinny_kernel(const GemmArgs a) 
                 for (int e = 0; e < V; ++e) wv[i][u][e] = zero;
                 if (k < a.K) load_weights<V>(wv[i][u], w[i] + k);           // (K is a multiple of 8 V)
             }
+    };
+    // (a model's weights: on their way while the kernel in front of this one ends.  Not where experts without rows are left out)
+    const bool early = a.weights_ready && a.grp_off == nullptr;
+    if (early) fetch(warp * U);
+    chain_wait();
+    int row_lo = 0, rows = a.M;
+    if (a.grp_off != nullptr) { row_lo = a.grp_off[g]; rows = a.grp_off[g + 1] - row_lo; }
+    if (rows <= 0) return;
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+        const int m = q + 8 * i;
+        x[i] = m < rows ? A + (int64_t)(a.row_src ? a.row_src[row_lo + m] : row_lo + m) * a.lda : nullptr;
+    }
+    if (!early) fetch(warp * U);
+    float sum[R == 16 ? NT : 1][4] = {};
+    for (int s = warp * U; s * 32 * V < a.K; s += KW * U) {
+        uint4 xv[NT][U][V];
+        if (s != warp * U) fetch(s);
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
@@ -288,8 +296,8 @@ __global__ void __launch_bounds__(32 * KW) gemm_skinny_kernel(const GemmArgs a) 
 // 8192 x 1024 5.3 / 5.5, 1024 x 2048 2.9 / 2.7, 6144 x 2048 7.3 / 6.7, 1024 x 4096 5.2 / 5.0, 3088 x 4096 9.2 / 7.9.
 template <typename TC, bool DUAL, int NT, int KW, int U, int V>
 static void launch_skinny_tiles(const GemmArgs& a, int groups, int64_t tiles, cudaStream_t st) {
-    if (NT == 1 && tiles >= 128) gemm_skinny_kernel<TC, DUAL, 16, 1, KW, U, V><<<dim3((a.N + (DUAL ? 7 : 15)) / (DUAL ? 8 : 16), groups), 32 * KW, 0, st>>>(a);
-    else gemm_skinny_kernel<TC, DUAL, 8, NT, KW, U, V><<<dim3((a.N + (DUAL ? 3 : 7)) / (DUAL ? 4 : 8), groups), 32 * KW, 0, st>>>(a);
+    if (NT == 1 && tiles >= 128) chain_launch(gemm_skinny_kernel<TC, DUAL, 16, 1, KW, U, V>, dim3((a.N + (DUAL ? 7 : 15)) / (DUAL ? 8 : 16), groups), 32 * KW, 0, st, a);
+    else chain_launch(gemm_skinny_kernel<TC, DUAL, 8, NT, KW, U, V>, dim3((a.N + (DUAL ? 3 : 7)) / (DUAL ? 4 : 8), groups), 32 * KW, 0, st, a);
 }
 template <typename TC, bool DUAL, int NT, int V>
 static void launch_skinny_rows(const GemmArgs& a, int groups, cudaStream_t st) {
@@ -333,6 +341,7 @@ __global__ void __launch_bounds__(32 * SK_WARPS) gemm_rows_kernel(GemmArgs a) {
     constexpr int OUTS = DUAL ? SK_ROWS / 2 : SK_ROWS, SETS = SK_WARPS / KW, V = SK_ROWS * MT;      // outputs per set; sums per thread
     constexpr int PV = 4, STEP = KW * 32 * PV;              // numbers of a piece; k of the warps' pieces together
     __shared__ float part[SK_WARPS][V];
+    chain_wait();
     const int g = blockIdx.z;
     int row_lo = 0, rows = a.M;
     if (a.grp_off != nullptr) { row_lo = a.grp_off[g]; rows = a.grp_off[g + 1] - row_lo; }
@@ -432,8 +441,8 @@ static void launch_rows(const GemmArgs& a, int groups, bool dual, cudaStream_t s
     const dim3 grid((a.N + outs_per_block - 1) / outs_per_block, (a.M + mt - 1) / mt, groups), block(32 * SK_WARPS);
 #define UMBS_SK2(MT, KW)                                                                  \
     do {                                                                                  \
-        if (dual) gemm_rows_kernel<true, MT, KW><<<grid, block, 0, st>>>(a);              \
-        else gemm_rows_kernel<false, MT, KW><<<grid, block, 0, st>>>(a);                  \
+        if (dual) chain_launch(gemm_rows_kernel<true, MT, KW>, grid, block, 0, st, a);    \
+        else chain_launch(gemm_rows_kernel<false, MT, KW>, grid, block, 0, st, a);        \
     } while (0)
 #define UMBS_SK(MT)                                                                   \
     do {                                                                              \
@@ -526,7 +535,8 @@ static int gemm_run(int dtype, const void* A, int64_t lda, int a_goff, const voi
     cudaStream_t st = (cudaStream_t)stream;
     GemmArgs a{A, lda, a_goff, W, ldw, w_gstride, C, ldc, c_goff, M, N, K, grp_off, row_src, limit,
                (dual == UMBS_ACT_GELU_TANH || dual == UMBS_ACT_SILU) ? dual : UMBS_ACT_CLAMPED_GLU,
-               bias, out_gate, ld_gate, gate_goff, gate_n, unary, p0, p1, unary_cols};
+               bias, out_gate, ld_gate, gate_goff, gate_n, unary, p0, p1, unary_cols,
+               in_chain()};                                 // (a model's products: W is a layer's weight)
     if (dtype == UMBS_F32) {                                              // activations are fp32 too: c_f32 changes nothing
         const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) && (a_goff % 4 == 0) && (w_gstride % 4 == 0) &&
                          ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);

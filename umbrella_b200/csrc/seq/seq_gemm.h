@@ -21,6 +21,7 @@ struct GemmArgs {
     int unary;        // UMBS_UNARY_* of a plain product's first unary_cols columns, with its two numbers
     float p0, p1;
     int unary_cols;
+    int weights_ready;       // W was there before the chain of launches began: it may be read ahead of chain_wait
 };
 
 __device__ __forceinline__ float unary_act(float z, int unary, float p0, float p1) {

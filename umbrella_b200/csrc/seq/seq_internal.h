@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 #include "../../../include/umbrella_b200.h"      // UMB_ERR_*
 #include "../../../include/umbrella_b200_seq.h"
 
@@ -41,6 +43,37 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
 }
 
 void count_launches(unsigned n);
+
+// The launches of one umbs_forward are a chain: a kernel of it may be brought onto the SMs while the one in front of it still runs,
+// and waits there (chain_wait, ahead of everything it reads or writes but the model's weights) until that one is done and its
+// results are visible.  Every block waits, so a kernel is done only after all those in front of it are.  A decode step is some 80 kernels
+// of 2 to 6 us each; launched one behind the other, 1.2 us of each are its launch.
+class ChainScope {                                          // this thread's launches until the scope ends
+public:
+    ChainScope();
+    ~ChainScope();
+    ChainScope(const ChainScope&) = delete;
+    ChainScope& operator=(const ChainScope&) = delete;
+};
+bool in_chain();
+template <typename... P, typename... A>
+int chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &early;
+    c.numAttrs = in_chain() ? 1 : 0;
+    return (int)cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+}
+// (no operation in a kernel that was launched otherwise)
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // seq_gemm_tc.cu: a word of host memory that the kernels can write, set by a block that gave up.  Every call that launches such
 // a kernel looks at it first (no synchronisation) and refuses once it is set: results since then are not to be used.

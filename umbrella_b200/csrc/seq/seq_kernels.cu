@@ -44,6 +44,7 @@ __device__ float block_sum(float v, float* red) {   // red: >= 33 floats of shar
 template <typename T>
 __global__ void embedding_kernel(const int32_t* __restrict__ ids, const T* __restrict__ table, float* __restrict__ y,
                                  T* __restrict__ y2, int width, float scale, const int32_t* __restrict__ tok_pos, const float* __restrict__ pos_freq) {
+    chain_wait();
     const int t = blockIdx.x;
     const T* row = table + (int64_t)ids[t] * width;
     const float pos = pos_freq != nullptr ? (float)tok_pos[t] : 0.f;
@@ -562,6 +563,7 @@ __global__ void latent_merge_kernel(const float* __restrict__ part, int nsplit, 
 
 template <typename T>
 __global__ void ring_append_kernel(const T* __restrict__ c, T* __restrict__ ring, int ring_len, Batch b, int R) {
+    chain_wait();
     const int t = blockIdx.x, s = b.tok_seq[t], pos = b.tok_pos[t];
     if (pos < b.seq_pos0[s] + b.seq_len[s] - ring_len) return;     // a later token of this step takes the row
     T* dst = ring + ((int64_t)b.seq_slot[s] * ring_len + pos % ring_len) * R;
@@ -795,6 +797,7 @@ __global__ void __launch_bounds__(1024) moe_route_small_kernel(const T* __restri
                                                               int32_t* __restrict__ pair_pos, const float* __restrict__ gate_w,
                                                               float* __restrict__ gate_out) {
     extern __shared__ float zs[];                    // [n][experts] logits, then [experts] counts, [n top] chosen experts
+    chain_wait();
     int32_t* counts = reinterpret_cast<int32_t*>(zs + n * experts);
     int32_t* offs = counts + experts;                // [experts + 1]
     int32_t* chosen = offs + experts + 1;            // [n top]
@@ -986,8 +989,8 @@ extern "C" int umbs_embedding_rows(int dtype, const int32_t* ids, const int32_t*
     if (n <= 0) return 0;
     if (pos_freq != nullptr && tok_pos == nullptr) return UMB_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
-    UMBS_DISPATCH_T(dtype, embedding_kernel<T><<<n, threads_for(width), 0, st>>>(ids, (const T*)table, y, (T*)y2, width, scale, tok_pos,
-                                                                              pos_freq));
+    UMBS_DISPATCH_T(dtype, chain_launch(embedding_kernel<T>, n, threads_for(width), 0, st, ids, (const T*)table, y, (T*)y2, width, scale,
+                                        tok_pos, pos_freq));
     count_launches(1);
     return (int)cudaGetLastError();
 }
@@ -1215,8 +1218,7 @@ extern "C" int umbs_ring_append(int dtype, const void* c, void* ring, int ring_l
                                 umbs_stream_t stream) {
     if (batch->n_tokens <= 0) return 0;
     cudaStream_t st = (cudaStream_t)stream;
-    UMBS_DISPATCH_T(dtype, ring_append_kernel<T><<<batch->n_tokens, 64, 0, st>>>((const T*)c, (T*)ring, ring_len, *batch,
-                                                                              kv_rank));
+    UMBS_DISPATCH_T(dtype, chain_launch(ring_append_kernel<T>, batch->n_tokens, 64, 0, st, (const T*)c, (T*)ring, ring_len, *batch, kv_rank));
     count_launches(1);
     return (int)cudaGetLastError();
 }
@@ -1253,9 +1255,9 @@ extern "C" int umbs_moe_route_scaled(int dtype, const void* h, int n, int width,
     if ((size_t)n * experts <= 256 && (size_t)n * top <= 1024) {
         // a small step (decoding): one block does the logits, the choice, the offsets and the sorted pair list
         const size_t smem = ((size_t)n * experts + 2 * (size_t)experts + 1 + (size_t)n * top) * sizeof(float);
-        UMBS_DISPATCH_T(dtype, moe_route_small_kernel<T><<<1, 1024, smem, st>>>((const T*)h, n, width, w_router, experts, top,
-                                                                              mode, groups, keep, weight_scale, sel_w, scratch + 2 * experts,
-                                                                              grp_off, pair_tok, pair_pos, gate_w, gate_out));
+        UMBS_DISPATCH_T(dtype, chain_launch(moe_route_small_kernel<T>, 1, 1024, smem, st, (const T*)h, n, width, w_router, experts, top,
+                                            mode, groups, keep, weight_scale, sel_w, scratch + 2 * experts, grp_off, pair_tok, pair_pos,
+                                            gate_w, gate_out));
         count_launches(1);
         return (int)cudaGetLastError();
     }

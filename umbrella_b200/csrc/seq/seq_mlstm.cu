@@ -31,6 +31,7 @@ __device__ __forceinline__ float log_sigmoid(float z) { return fminf(z, 0.f) - l
 __global__ void mlstm_gates_kernel(const float* __restrict__ proj, int64_t ld, int off_i, int off_f,
                                    const float* __restrict__ gate_bias, Batch b, int heads, float cap, float* __restrict__ state,
                                    int64_t state_stride, int m_off, float* __restrict__ gates) {
+    chain_wait();
     const int wid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (wid >= b.n_seqs * heads) return;
     const int s = wid / heads, h = wid - s * heads;
@@ -79,6 +80,7 @@ __global__ void mlstm_kernel(const float* __restrict__ proj, int64_t ld, Batch b
                              float* __restrict__ o_out, int seg_len, int n_seg, int pass, float* __restrict__ seg_state,
                              float* __restrict__ seg_decay) {
     extern __shared__ __align__(16) float sm[];
+    chain_wait();
     const int DS = blockDim.y, dimP = DS * DPT, nthr = 32 * DS, V1 = vdim + 1;
     float* qs = sm;                          // [TB][dimP]
     float* ks = qs + TB * dimP;              // [TB][dimP]   keys times the token's input weight
@@ -221,6 +223,7 @@ template <typename T, int COLS>
 __global__ void mlstm_finish_kernel(const float* __restrict__ o, const float* __restrict__ gates, const float* __restrict__ proj,
                                     int64_t ld, int off_g, int n, int heads, int vdim, float eps,
                                     const float* __restrict__ norm_w, T* __restrict__ out) {
+    chain_wait();
     const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (w >= n * heads) return;
     const int t = w / heads, h = w - t * heads, V1 = vdim + 1;
@@ -277,8 +280,8 @@ static int launch_mlstm(const float* proj, int64_t ld, const Batch& b, int heads
         if (e != cudaSuccess) return (int)e;
         set = smem;
     }
-    mlstm_kernel<DPT, TB><<<grid, block, smem, st>>>(proj, ld, b, heads, dim, vdim, gates, state, stride, o, seg_len, n_seg, pass,
-                                                     seg_state, seg_decay);
+    chain_launch(mlstm_kernel<DPT, TB>, grid, block, smem, st, proj, ld, b, heads, dim, vdim, gates, state, stride, o, seg_len, n_seg, pass,
+                 seg_state, seg_decay);
     return 0;
 }
 
@@ -296,7 +299,7 @@ extern "C" int umbs_mlstm(int dtype, const float* proj, int64_t ld, const float*
     const int64_t stride = (int64_t)dim * (vdim + 1) + 1;
     const int off_g = 2 * heads * dim + heads * vdim, off_i = off_g + heads * vdim, off_f = off_i + heads;
     const int warps = batch->n_seqs * heads;
-    mlstm_gates_kernel<<<(warps + 3) / 4, 128, 0, st>>>(proj, ld, off_i, off_f, gate_bias, *batch, heads, gate_cap, state, stride,
+    chain_launch(mlstm_gates_kernel, (warps + 3) / 4, 128, 0, st, proj, ld, off_i, off_f, gate_bias, *batch, heads, gate_cap, state, stride,
                                                         dim * (vdim + 1), gates_scratch);
     // Few blocks and long sequences (one long prompt): cut the sequences into segments that run side by side in two passes.
     // Twice the arithmetic of the recurrence for n_seg times the blocks; differs from the single walk by fp32 rounding only.
@@ -349,7 +352,7 @@ extern "C" int umbs_mlstm(int dtype, const float* proj, int64_t ld, const float*
     const int fw = batch->n_tokens * heads;
     auto finish = [&](auto* to) {
         using T = std::remove_pointer_t<decltype(to)>;
-        auto run = [&](auto kernel) { kernel<<<(fw + 3) / 4, 128, 0, st>>>(o_scratch, gates_scratch, proj, ld, off_g, batch->n_tokens, heads, vdim, eps, out_norm_w, to); };
+        auto run = [&](auto kernel) { chain_launch(kernel, (fw + 3) / 4, 128, 0, st, (const float*)o_scratch, (const float*)gates_scratch, proj, ld, off_g, batch->n_tokens, heads, vdim, eps, out_norm_w, to); };
         if (vdim <= 32) run(mlstm_finish_kernel<T, 1>);
         else if (vdim <= 64) run(mlstm_finish_kernel<T, 2>);
         else if (vdim <= 128) run(mlstm_finish_kernel<T, 4>);

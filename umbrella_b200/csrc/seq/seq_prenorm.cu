@@ -214,6 +214,7 @@ __global__ void add_norm_vec_kernel(float* __restrict__ x, const float* __restri
                                     const int32_t* __restrict__ rows, const float* __restrict__ w, float w_offset, int width, float eps,
                                     T* __restrict__ y, int64_t ldy, float* __restrict__ copy) {
     __shared__ float red[2][32];
+    chain_wait();
     const int r = blockIdx.x, n4 = width / 4;
     const int64_t src = rows ? rows[r] : r;
     float4* xr = reinterpret_cast<float4*>(x + src * width);
@@ -288,7 +289,7 @@ static void launch_add_norm_vec(float* x, const umbs_delta_t& d, const int32_t* 
     const int n4 = width / 4, keep = n <= 148 ? (n4 <= 1024 ? 1 : 2) : 4;
     const int threads = ((n4 + keep - 1) / keep + 31) / 32 * 32;
     const float* delta = ROUTED ? d.pair_out : d.delta;
-#define UMBS_ANV(K) add_norm_vec_kernel<T, K, ROUTED><<<n, threads, 0, st>>>(x, delta, d.sel_w, d.pair_pos, d.top, d.norm_w, d.mult, rows, w, w_offset, width, eps, y, ldy, copy)
+#define UMBS_ANV(K) chain_launch(add_norm_vec_kernel<T, K, ROUTED>, n, threads, 0, st, x, delta, d.sel_w, d.pair_pos, d.top, d.norm_w, d.mult, rows, w, w_offset, width, eps, y, ldy, copy)
     if (keep == 1) UMBS_ANV(1);
     else if (keep == 2) UMBS_ANV(2);
     else UMBS_ANV(4);
@@ -303,6 +304,7 @@ __global__ void __launch_bounds__(512) add_rms_norm_vec_kernel(float* __restrict
                                                                const float* __restrict__ w, float w_offset, int width, float eps,
                                                                T* __restrict__ y, float* __restrict__ copy) {
     __shared__ float red[32];
+    chain_wait();
     const int r = blockIdx.x, n4 = width / 4;
     const int64_t src = rows ? rows[r] : r;
     float4* xr = reinterpret_cast<float4*>(x + src * width);
@@ -410,6 +412,7 @@ __global__ void latent_prep_kernel(umbs_latent_prep_t p, Batch b) {
 }
 
 __global__ void softcap_kernel(float* __restrict__ z, int64_t n, float cap) {
+    chain_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) z[i] = cap * tanhf(z[i] / cap);
 }
@@ -427,6 +430,7 @@ __global__ void attention_prep_kernel(const float* __restrict__ proj, int64_t ld
     const int Cq = heads * maps * dim, Ck = kv_heads * maps * dim, C = Cq + Ck, Cv = kv_heads * vdim;
     float* y = sm;
     float* cs = sm + C;
+    chain_wait();
     const int t = blockIdx.x, s = b.tok_seq[t], pos = b.tok_pos[t];
     const int start = b.seq_start[s], len = b.seq_len[s], pos0 = b.seq_pos0[s], slot = b.seq_slot[s], par = b.seq_parity[s];
     const int keep = taps - 1;
@@ -535,6 +539,7 @@ __global__ void attention_prep_kernel(const float* __restrict__ proj, int64_t ld
 template <typename T>
 __global__ void kv_pool_kernel(const T* __restrict__ kv, const T* __restrict__ kv_cache, int kv_len, T* __restrict__ pool_cache,
                                int pool_len, Batch b, int row, int pool) {
+    chain_wait();
     const int s = blockIdx.y, pos0 = b.seq_pos0[s], len = b.seq_len[s], start = b.seq_start[s], slot = b.seq_slot[s];
     const int blk = pos0 / pool + blockIdx.x;                    // first block whose last token is in the step, onwards
     if ((int64_t)(blk + 1) * pool > (int64_t)pos0 + len || blk >= pool_len) return;
@@ -581,7 +586,7 @@ extern "C" int umbs_add_rms_norm(int dtype, float* x, const float* delta, const 
     const uintptr_t ptrs = (uintptr_t)x | (uintptr_t)delta | (uintptr_t)w | (uintptr_t)copy | (uintptr_t)y;
     if (width % 4 == 0 && width <= 8192 && ptrs % 16 == 0) {
         const int n4 = width / 4, keep = n4 <= 256 ? 1 : (n4 <= 1024 ? 2 : 4), vt = ((n4 + keep - 1) / keep + 31) / 32 * 32;
-#define UMBS_ARN(K) UMBS_DISPATCH_T(dtype, (add_rms_norm_vec_kernel<T, K><<<n, vt, 0, st>>>(x, delta, rows, w, w_offset, width, eps, (T*)y, copy)))
+#define UMBS_ARN(K) UMBS_DISPATCH_T(dtype, (chain_launch(add_rms_norm_vec_kernel<T, K>, n, vt, 0, st, x, delta, rows, w, w_offset, width, eps, (T*)y, copy)))
         if (keep == 1) UMBS_ARN(1);
         else if (keep == 2) UMBS_ARN(2);
         else UMBS_ARN(4);
@@ -684,7 +689,7 @@ extern "C" int umbs_latent_prep_parts(int dtype, const umbs_latent_prep_t* p, co
 extern "C" int umbs_softcap(float* z, int64_t n, float cap, umbs_stream_t stream) {
     if (n <= 0) return 0;
     if (!(cap > 0.f)) return UMB_ERR_ARG;
-    softcap_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(z, n, cap);
+    chain_launch(softcap_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, z, n, cap);
     count_launches(1);
     return (int)cudaGetLastError();
 }
@@ -728,7 +733,7 @@ extern "C" int umbs_attention_prep_opts(int dtype, const float* proj, int64_t ld
     if (smem > 48 * 1024) return UMB_ERR_UNSUPPORTED;
     // a small step (decoding) has few blocks: spread a token's channels over up to 1024 threads
     const int threads = batch->n_tokens <= 64 ? std::min(1024, (C + 31) / 32 * 32) : (C >= 1024 ? 256 : 128);
-    UMBS_DISPATCH_T(dtype, attention_prep_kernel<T><<<batch->n_tokens, threads, smem, st>>>(
+    UMBS_DISPATCH_T(dtype, chain_launch(attention_prep_kernel<T>, batch->n_tokens, threads, smem, st,
                                proj, ld, bias, *batch, heads, kv_heads, dim, vdim, values_are_keys, taps, conv_w, conv_state, slots,
                                rot_dims, inv_freq, rot_mag, maps, q_norm_w, k_norm_w, eps, po, (T*)q, (T*)kv));
     count_launches(1);
@@ -741,7 +746,7 @@ extern "C" int umbs_kv_pool(int dtype, const void* kv, const void* kv_cache, int
     if (kv_len < pool) return UMB_ERR_ARG;               // a block's older tokens must still sit in the cache
     cudaStream_t st = (cudaStream_t)stream;
     const dim3 grid(batch->max_seq_len / pool + 1, batch->n_seqs, (row + 127) / 128);
-    UMBS_DISPATCH_T(dtype, kv_pool_kernel<T><<<grid, 128, 0, st>>>((const T*)kv, (const T*)kv_cache, kv_len, (T*)pool_cache,
+    UMBS_DISPATCH_T(dtype, chain_launch(kv_pool_kernel<T>, grid, 128, 0, st, (const T*)kv, (const T*)kv_cache, kv_len, (T*)pool_cache,
                                                                    pool_len, *batch, row, pool));
     count_launches(1);
     return (int)cudaGetLastError();
