@@ -269,6 +269,21 @@ def test_mlstm_whole_portions_and_batches(H, D, V, cap):
                 assert err(torch.cat(got[s]), refs[s][:at[s]]) < 2e-5, (s, len(lengths))
 
 
+# one token per sequence runs in one kernel: key sizes around a warp's 8 and 16 state rows, value sizes around its columns
+@pytest.mark.parametrize("H,D,V", [(1, 1, 1), (2, 8, 31), (3, 32, 63), (2, 33, 64), (2, 64, 128), (1, 128, 159), (2, 100, 40)])
+def test_mlstm_single_tokens_have_the_bits_of_longer_steps(H, D, V):
+    from umbrella_b200 import ops_seq as K
+    rows = 2 * H * D + 2 * H * V + 2 * H
+    x, bias, norm_w = f32(rnd(5, rows, seed=35)), f32(rnd(2 * H, seed=36)), f32(1.0 + rnd(H * V, seed=37, scale=0.2))
+    for pos in (0, 3):
+        state = f32(rnd(3, H, D * (V + 1) + 1, seed=38))
+        alone, beside = state.clone(), state.clone()
+        one = K.mlstm(x[:2].contiguous(), bias, K.RaggedBatch([(0, 1, pos, 0), (1, 1, 4, 0)], DEV), H, D, V, 9.0, 1e-5, norm_w, alone)
+        two = K.mlstm(x, bias, K.RaggedBatch([(0, 1, pos, 0), (1, 1, 4, 0), (2, 3, 0, 0)], DEV), H, D, V, 9.0, 1e-5, norm_w, beside)
+        assert torch.equal(one, two[:2]) and torch.equal(alone[:2], beside[:2])
+        assert torch.equal(alone[2], state[2])
+
+
 def test_mlstm_long_sequences_cut_into_segments():
     """A step of few long sequences runs as segments side by side (two passes, chained states): a long prompt that starts
     from a carried state, with a short neighbour and one whose last segment is a single token, against the single walk

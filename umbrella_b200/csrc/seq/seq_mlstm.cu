@@ -267,6 +267,111 @@ __global__ void mlstm_finish_kernel(const float* __restrict__ o, const float* __
     }
 }
 
+// One token per sequence: gates, recurrence and finish of a (sequence, head) in one block of DS = ceil(dim / DPT) warps, with the
+// arithmetic of the three kernels above and below (a warp's DPT state rows in one chain, the warps' sums in order, the row's
+// finish by one warp), so a step's results do not depend on which of them ran.  A lane has the state's columns lane, lane + 32, ..., and asks for
+// all of them, every row of the step and the old maximum before it uses one.
+// Bound: launches and a load's latency; three kernels of 2.5 to 5 us behind one another, this one 3 (4 and 64 sequences, 8 heads of 64 x 128:
+// see launch_mlstm_decode).
+template <typename T, int DPT, int CL>
+__global__ void mlstm_decode_kernel(const float* __restrict__ proj, int64_t ld, const float* __restrict__ gate_bias, const Batch b,
+                                    int heads, int dim, int vdim, float cap, float eps, const float* __restrict__ norm_w,
+                                    float* __restrict__ state, int64_t state_stride, T* __restrict__ out) {
+    extern __shared__ __align__(16) float part[];           // [DS][32 CL]
+    chain_wait();
+    const int s = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, w = threadIdx.x >> 5, DS = blockDim.x >> 5, V1 = vdim + 1, d0 = w * DPT;
+    const int64_t t = b.seq_start[s];
+    const bool have = b.seq_pos0[s] > 0;
+    float* st = state + ((int64_t)b.seq_slot[s] * heads + h) * state_stride;
+    if (b.seq_len[s] == 0) {                                // (a new sequence's maximum starts at 0 as in a step with tokens)
+        if (threadIdx.x == 0 && !have) st[(int64_t)dim * V1] = 0.f;
+        return;
+    }
+    const float* row = proj + t * ld;
+    const float* vrow = row + 2 * heads * dim + h * vdim;
+    const float* grow = row + 2 * heads * dim + heads * vdim + h * vdim;
+    const int off_i = 2 * heads * (dim + vdim), off_f = off_i + heads;
+    float S[DPT][CL], v[CL];
+#pragma unroll
+    for (int i = 0; i < DPT; ++i)
+#pragma unroll
+        for (int c = 0; c < CL; ++c) {
+            const int j = lane + 32 * c;
+            S[i][c] = have && d0 + i < dim && j < V1 ? st[(int64_t)(d0 + i) * V1 + j] : 0.f;
+        }
+#pragma unroll
+    for (int c = 0; c < CL; ++c) {
+        const int j = lane + 32 * c;
+        v[c] = j < vdim ? vrow[j] : (j == vdim ? 1.f : 0.f);
+    }
+    // lane i: the row's query and key numbers d0 + i
+    const bool dl = lane < DPT && d0 + lane < dim;
+    const float qn = dl ? row[h * dim + d0 + lane] * (1.f / sqrtf((float)dim)) : 0.f;
+    float kn = dl ? row[heads * dim + h * dim + d0 + lane] : 0.f;
+    const float m_in = have ? st[(int64_t)dim * V1] : 0.f;
+    const float bi = gate_bias ? gate_bias[h] : 0.f, bf = gate_bias ? gate_bias[heads + h] : 0.f;
+    const float il = cap * tanhf((row[off_i + h] + bi) / cap), fl = log_sigmoid(cap * tanhf((row[off_f + h] + bf) / cap));
+    const float m = fmaxf(m_in + fl, il), dec = expf(fl + m_in - m), low = expf(-m);
+    kn *= expf(il - m);
+    float acc[CL] = {};
+#pragma unroll
+    for (int i = 0; i < DPT; ++i) {
+        const float qv = __shfl_sync(0xffffffffu, qn, i), kv = __shfl_sync(0xffffffffu, kn, i);
+#pragma unroll
+        for (int c = 0; c < CL; ++c) {
+            S[i][c] = fmaf(dec, S[i][c], kv * v[c]);
+            acc[c] = fmaf(S[i][c], qv, acc[c]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < DPT; ++i)
+#pragma unroll
+        for (int c = 0; c < CL; ++c) {
+            const int j = lane + 32 * c;
+            if (d0 + i < dim && j < V1) st[(int64_t)(d0 + i) * V1 + j] = S[i][c];
+        }
+#pragma unroll
+    for (int c = 0; c < CL; ++c) part[w * 32 * CL + lane + 32 * c] = acc[c];
+    __syncthreads();                                        // (and every warp has read the old maximum)
+    if (w != 0) return;
+    if (lane == 0) st[(int64_t)dim * V1] = m;
+    float nq = 0.f, o[CL], ss = 0.f;
+    for (int ww = 0; ww < DS; ++ww) nq += part[ww * 32 * CL + vdim];
+    const float den = fmaxf(fabsf(nq), low) + 1e-6f;
+#pragma unroll
+    for (int c = 0; c < CL; ++c) {
+        const int j = lane + 32 * c;
+        o[c] = 0.f;
+        if (j >= vdim) continue;
+        for (int ww = 0; ww < DS; ++ww) o[c] += part[ww * 32 * CL + j];
+        o[c] /= den;
+        ss = fmaf(o[c], o[c], ss);
+    }
+    ss = warp_sum_ml(ss);
+    const float inv = 1.f / sqrtf(ss / (float)vdim + eps);
+#pragma unroll
+    for (int c = 0; c < CL; ++c) {
+        const int j = lane + 32 * c;
+        if (j >= vdim) continue;
+        const float g = 1.f / (1.f + expf(-grow[j]));
+        out[t * heads * vdim + h * vdim + j] = from_f32<T>(o[c] * inv * norm_w[h * vdim + j] * g);
+    }
+}
+
+// Keys of up to 128 and values of up to 159 numbers: what a lane's registers hold.
+static bool mlstm_decode_fits(int dim, int vdim) { return dim <= 128 && vdim < 160; }
+template <typename T>
+static void launch_mlstm_decode(const float* proj, int64_t ld, const float* gate_bias, const Batch& b, int heads, int dim, int vdim, float cap,
+                                float eps, const float* norm_w, float* state, int64_t stride, T* out, cudaStream_t st) {
+    auto run = [&](auto kernel, int dpt, int cl) {
+        const int ds = (dim + dpt - 1) / dpt;
+        chain_launch(kernel, dim3(b.n_seqs, heads), 32 * ds, (size_t)ds * 32 * cl * sizeof(float), st, proj, ld, gate_bias, b, heads, dim, vdim, cap,
+                     eps, norm_w, state, stride, out);
+    };
+    if (dim <= 32) vdim < 64 ? run(mlstm_decode_kernel<T, 8, 2>, 8, 2) : run(mlstm_decode_kernel<T, 8, 5>, 8, 5);
+    else vdim < 64 ? run(mlstm_decode_kernel<T, 16, 2>, 16, 2) : run(mlstm_decode_kernel<T, 16, 5>, 16, 5);
+}
+
 template <int DPT, int TB>
 static int launch_mlstm(const float* proj, int64_t ld, const Batch& b, int heads, int dim, int vdim, const float* gates,
                         float* state, int64_t stride, float* o, int seg_len, int n_seg, int pass, float* seg_state,
@@ -298,6 +403,13 @@ extern "C" int umbs_mlstm(int dtype, const float* proj, int64_t ld, const float*
     cudaStream_t st = (cudaStream_t)stream;
     const int64_t stride = (int64_t)dim * (vdim + 1) + 1;
     const int off_g = 2 * heads * dim + heads * vdim, off_i = off_g + heads * vdim, off_f = off_i + heads;
+    if (batch->max_seq_len == 1 && mlstm_decode_fits(dim, vdim)) {
+        if (dtype == UMBS_BF16) launch_mlstm_decode(proj, ld, gate_bias, *batch, heads, dim, vdim, gate_cap, eps, out_norm_w, state, stride, (__nv_bfloat16*)out, st);
+        else if (dtype == UMBS_F32) launch_mlstm_decode(proj, ld, gate_bias, *batch, heads, dim, vdim, gate_cap, eps, out_norm_w, state, stride, (float*)out, st);
+        else return UMB_ERR_ARG;
+        count_launches(1);
+        return (int)cudaGetLastError();
+    }
     const int warps = batch->n_seqs * heads;
     chain_launch(mlstm_gates_kernel, (warps + 3) / 4, 128, 0, st, proj, ld, off_i, off_f, gate_bias, *batch, heads, gate_cap, state, stride,
                                                         dim * (vdim + 1), gates_scratch);
