@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
     uint64_t *k_full = bars, *v_full = bars + kTaStages, *k_empty = bars + 2 * kTaStages, *v_empty = bars + 3 * kTaStages,
              *s_full = bars + 4 * kTaStages, *p_full = s_full + 2, *o_full = s_full + 3;
     volatile int* quit = &s_quit;
+    chain_wait();
     const int s = blockIdx.z, vh = blockIdx.y, q0 = (int)(gridDim.x - 1 - blockIdx.x) * kTaQ;     // the rows that see most start first
     const int len = b.seq_len[s], start = b.seq_start[s], pos0 = STEP ? 0 : b.seq_pos0[s], slot = STEP ? 0 : b.seq_slot[s];
     if (q0 >= len) return;
@@ -502,8 +503,7 @@ static int launch_ta(const CachedAttnArgs& a, const StepKeys& x, const Batch& b,
     // (always the same limit: another thread may be between setting it and its launch)
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTaSmem);
     if (e != cudaSuccess) return (int)e;
-    kernel<<<dim3((b.max_seq_len + kTaQ - 1) / kTaQ, a.heads, b.n_seqs), kTaThreads, smem, st>>>(mk, ms, mv, a, x, b, z);
-    return 0;
+    return chain_launch(kernel, dim3((b.max_seq_len + kTaQ - 1) / kTaQ, a.heads, b.n_seqs), kTaThreads, smem, st, mk, ms, mv, a, x, b, z);
 }
 
 int launch_attention_tc(int mode, const CachedAttnArgs& a, const StepKeys* keys, const Batch& b, cudaStream_t st) {

@@ -35,6 +35,7 @@ template <bool GATES>
 __global__ void __launch_bounds__(256, 2) chunk_memory_kernel(const ChunkMemory x, const Batch b) {
     extern __shared__ __align__(16) unsigned char smem[];
     ChunkShared& sh = *reinterpret_cast<ChunkShared*>(smem);
+    chain_wait();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int s = blockIdx.x / x.n_seg, seg = blockIdx.x - s * x.n_seg, h = blockIdx.y, c0 = blockIdx.z * kChV;
     const int seq_len = b.seq_len[s], t_first = seg * x.seg_len;
@@ -308,8 +309,7 @@ int launch_chunk_memory(const ChunkMemory& m, const Batch& b, cudaStream_t st) {
     auto run = [&](auto kernel) -> int {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ChunkShared));
         if (e != cudaSuccess) return (int)e;
-        kernel<<<grid, 256, sizeof(ChunkShared), st>>>(m, b);
-        return 0;
+        return chain_launch(kernel, grid, 256, sizeof(ChunkShared), st, m, b);
     };
     return m.gates != nullptr ? run(chunk_memory_kernel<true>) : run(chunk_memory_kernel<false>);
 }

@@ -117,6 +117,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     __syncthreads();
     umb::tc_fence_after();
     const uint32_t tmem = *s_tmem;
+    chain_wait();
     TileWalk w(a, t);
 
     if (warp == 0) {
@@ -332,8 +333,7 @@ static int launch_tc(const GemmArgs& a, TcArgs t, int sms, cudaStream_t st) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
     if (e != cudaSuccess) return (int)e;
     const int64_t tiles = (int64_t)t.groups * t.m_tiles * t.n_tiles;            // (sorted by expert: at most)
-    kernel<<<(int)(tiles < sms ? tiles : sms), Cfg::threads(A_TMA), Cfg::kSmem, st>>>(ma, mw, a, t);
-    return 0;
+    return chain_launch(kernel, (int)(tiles < sms ? tiles : sms), Cfg::threads(A_TMA), Cfg::kSmem, st, ma, mw, a, t);
 }
 
 template <int BN>

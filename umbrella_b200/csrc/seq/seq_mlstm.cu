@@ -1,6 +1,6 @@
 // mLSTM: a matrix memory per head with exponential input gates, sigmoid forget gates and a running maximum that keeps
 // the exponentials in range (see umbs_mlstm in include/umbrella_b200_seq.h).  Three kernels per step:
-//   gates       one warp per (sequence, head): the log gates of 32 tokens at a time, the running maximum by a warp scan
+//   gates       one block per (sequence, head): the log gates of 32 tokens a warp, the running maximum by a warp scan
 //               of the maps m -> max(m + f, i) (they compose: (f1, i1) then (f2, i2) = (f1 + f2, max(i1 + f2, i2))), and
 //               from it each token's decay e^(f + m' - m), input weight e^(i - m) and floor e^(-m);
 //   recurrence  one block per (sequence, head, 32 columns) walking the tokens in order with its slice of the state in
@@ -27,21 +27,23 @@ __device__ __forceinline__ float warp_sum_ml(float v) {
 
 __device__ __forceinline__ float log_sigmoid(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
 
-// gates[t, h] = (decay, input weight, floor)
+// gates[t, h] = (decay, input weight, floor).  A block per (sequence, head), a warp per 32 of its next 32 WARPS tokens: the scans side by
+// side, then every warp takes the maximum through the whole runs in front of its own, one after the other as a walk would.  (One warp
+// for all of a sequence's tokens waited for their loads 32 at a time: 29 us for prompts of 146 to 256 tokens, this 5.)
 __global__ void mlstm_gates_kernel(const float* __restrict__ proj, int64_t ld, int off_i, int off_f,
                                    const float* __restrict__ gate_bias, Batch b, int heads, float cap, float* __restrict__ state,
                                    int64_t state_stride, int m_off, float* __restrict__ gates) {
+    __shared__ float run_a[32], run_b[32], s_m;
     chain_wait();
-    const int wid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (wid >= b.n_seqs * heads) return;
-    const int s = wid / heads, h = wid - s * heads;
+    const int s = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int start = b.seq_start[s], len = b.seq_len[s];
     float* m_state = state + ((int64_t)b.seq_slot[s] * heads + h) * state_stride + m_off;
     float m_in = b.seq_pos0[s] > 0 ? *m_state : 0.f;
     const float bi = gate_bias ? gate_bias[h] : 0.f, bf = gate_bias ? gate_bias[heads + h] : 0.f;
-    for (int t0 = 0; t0 < len; t0 += 32) {
-        const bool ok = t0 + lane < len;
-        const int64_t t = start + t0 + lane;
+    for (int t0 = 0; t0 < len; t0 += 32 * warps) {
+        const int at = t0 + warp * 32 + lane;
+        const bool ok = at < len;
+        const int64_t t = start + at;
         float fl = 0.f, il = -INFINITY;                            // the identity map for lanes past the end
         if (ok) {
             il = cap * tanhf((proj[t * ld + off_i + h] + bi) / cap);
@@ -53,6 +55,9 @@ __global__ void mlstm_gates_kernel(const float* __restrict__ proj, int64_t ld, i
             const float Ae = __shfl_up_sync(0xffffffffu, A, d), Be = __shfl_up_sync(0xffffffffu, B, d);
             if (lane >= d) { B = fmaxf(Be + A, B); A = Ae + A; }
         }
+        if (lane == 31) { run_a[warp] = A; run_b[warp] = B; }
+        __syncthreads();
+        for (int w = 0; w < warp; ++w) m_in = fmaxf(m_in + run_a[w], run_b[w]);
         const float m = fmaxf(m_in + A, B);
         float m_prev = __shfl_up_sync(0xffffffffu, m, 1);
         if (lane == 0) m_prev = m_in;
@@ -62,9 +67,11 @@ __global__ void mlstm_gates_kernel(const float* __restrict__ proj, int64_t ld, i
             g[1] = expf(il - m);
             g[2] = expf(-m);
         }
-        m_in = __shfl_sync(0xffffffffu, m, 31);                     // lanes past the end carry the last token's maximum
+        if (threadIdx.x == blockDim.x - 1) s_m = m;                 // lanes past the end carry the last token's maximum
+        __syncthreads();
+        m_in = s_m;
     }
-    if (lane == 0) *m_state = m_in;
+    if (threadIdx.x == 0) *m_state = m_in;
 }
 
 // See retention_kernel (seq_kernels.cu) for the walk; here V1 = vdim + 1 columns (the last one is n), per-token factors.
@@ -199,6 +206,7 @@ __global__ void mlstm_kernel(const float* __restrict__ proj, int64_t ld, Batch b
 // overwrites L_g with the state segment g + 1 starts from; entry n_seg - 1 (never an end state) takes segment 0's start.
 __global__ void mlstm_chain_kernel(Batch b, int heads, int dim, int V1, const float* __restrict__ state, int64_t state_stride,
                                    int seg_len, int n_seg, float* __restrict__ seg_state, const float* __restrict__ seg_decay) {
+    chain_wait();
     const int64_t plane = (int64_t)heads * dim * V1;
     const int s = blockIdx.y;
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -410,8 +418,8 @@ extern "C" int umbs_mlstm(int dtype, const float* proj, int64_t ld, const float*
         count_launches(1);
         return (int)cudaGetLastError();
     }
-    const int warps = batch->n_seqs * heads;
-    chain_launch(mlstm_gates_kernel, (warps + 3) / 4, 128, 0, st, proj, ld, off_i, off_f, gate_bias, *batch, heads, gate_cap, state, stride,
+    const int warps = std::max(1, std::min(32, (batch->max_seq_len + 31) / 32));
+    chain_launch(mlstm_gates_kernel, dim3(batch->n_seqs, heads), 32 * warps, 0, st, proj, ld, off_i, off_f, gate_bias, *batch, heads, gate_cap, state, stride,
                                                         dim * (vdim + 1), gates_scratch);
     // Few blocks and long sequences (one long prompt): cut the sequences into segments that run side by side in two passes.
     // Twice the arithmetic of the recurrence for n_seg times the blocks; differs from the single walk by fp32 rounding only.
@@ -453,8 +461,8 @@ extern "C" int umbs_mlstm(int dtype, const float* proj, int64_t ld, const float*
         rc = run(1);
         if (rc) return rc;
         const int64_t plane = (int64_t)heads * dim * V1;
-        mlstm_chain_kernel<<<dim3((unsigned)((plane + 255) / 256), batch->n_seqs), 256, 0, st>>>(*batch, heads, dim, V1, state, stride,
-                                                                                             seg_len, n_seg, seg_scratch, seg_decay);
+        chain_launch(mlstm_chain_kernel, dim3((unsigned)((plane + 255) / 256), batch->n_seqs), 256, 0, st, *batch, heads, dim, V1, (const float*)state,
+                     stride, seg_len, n_seg, seg_scratch, (const float*)seg_decay);
         launches += 2;
         rc = run(2);
     } else {
