@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
     else vhd = virtual_head(a, vh);
     const int h = vhd.h, window = a.window > 0 ? a.window : (1 << 30);
     const KeyTiles kt(a, window, pos0, q0, len);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int k_bytes = z.q_atoms * (kTaK * 128), v_bytes = z.v_atoms * (kTaK * 128);
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* s_k = smem + z.q_atoms * (kTaQ * 128);   // Q [q_atoms][128 rows][128 B], stages of K [q_atoms][32][128 B], of V [v_atoms][32][128 B]
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
             const int lo = kt.pooled(i) ? 0 : max(tok_lo - base, 0);
             const int hi = r >= len ? 0 : min((kt.pooled(i) ? pool_hi : rp + 1) - base, kTaK);
             const bool whole = __all_sync(0xffffffffu, lo == 0 && hi == kTaK);
-            if (!(ok = __all_sync(0xffffffffu, tc_spin(s_full + (i & 1), (i >> 1) & 1, quit)))) break;
+            if (!(ok = tc_spin_warp(s_full + (i & 1), (i >> 1) & 1, quit))) break;
             umb::tc_fence_after();
             uint32_t v[32];
             UMB_TMEM_LD_X32(t0 + (i & 1) * kTaK, v);
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
                     if (move) m = mx;
                     l *= f;                                 // (m = -inf: l is 0)
                     if (i > 0) {
-                        if (!(ok = __all_sync(0xffffffffu, tc_spin(o_full, (i - 1) & 1, quit)))) break;
+                        if (!(ok = tc_spin_warp(o_full, (i - 1) & 1, quit))) break;
                         umb::tc_fence_after();
                         waited = true;
                         for (int c0 = 0; c0 < z.v_atoms * 64; c0 += 32) {
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
             }
             l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
             if (!waited) {
-                if (!(ok = __all_sync(0xffffffffu, tc_spin(o_full, (i - 1) & 1, quit)))) break;
+                if (!(ok = tc_spin_warp(o_full, (i - 1) & 1, quit))) break;
                 umb::tc_fence_after();
             }
             UMB_TMEM_ST_X16(t0 + 64, ph);
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
             __syncwarp();
             if (lane == 0) umb::mbar_arrive(p_full);
         }
-        if (ok) ok = __all_sync(0xffffffffu, tc_spin(o_full, (kt.n - 1) & 1, quit));
+        if (ok) ok = tc_spin_warp(o_full, (kt.n - 1) & 1, quit);
         if (ok) {
             umb::tc_fence_after();
             const float inv = MODE == UMBS_ATTN_SIGMOID ? 1.f : 1.f / l;

@@ -93,7 +93,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     uint64_t *full = bars, *empty = bars + kStages, *acc_full = bars + 2 * kStages, *acc_empty = acc_full + 2;
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* quit = reinterpret_cast<volatile int*>(s_tmem + 1);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         umb::tma_prefetch_desc(&map_w);
@@ -122,32 +122,39 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
     if (warp == 0) {
         uint32_t s = 0, ph = 1;
-        bool ok = true;
+        bool ok = true, ready = false;
         while (ok && w.step()) {
             const int gw = t.w_grouped ? w.g : 0, ga = t.a_grouped ? w.g : 0, n0 = w.n0 * kOut;
             for (int k = 0; k < t.k_steps; ++k) {
-                if (!(ok = tc_spin_warp(empty + s, ph, quit))) break;
+                if (!ready && !(ok = tc_spin_warp(empty + s, ph, quit))) break;
                 unsigned char* st = smem + s * Cfg::kStage;
+                const uint32_t s2 = s + 1 == kStages ? 0 : s + 1, ph2 = s + 1 == kStages ? ph ^ 1 : ph;
+                const bool next = tc_test(empty + s2, ph2);             // (known behind the copies: no wait of its own where it is free)
                 if (umb::elect_one()) {
                     umb::mbar_arrive_expect_tx(full + s, (A_TMA ? Cfg::kABytes : 0) + Cfg::kWBytes);
                     if (A_TMA) tma_3d(st, &map_a, k * kTcK, w.m0, ga, full + s);
                     tma_3d(st + Cfg::kABytes, &map_w, k * kTcK, n0, gw, full + s);
                     if (DUAL) tma_3d(st + Cfg::kABytes + kOut * 128, &map_w, k * kTcK, a.N + n0, gw, full + s);
                 }
-                __syncwarp();
-                if (++s == kStages) { s = 0; ph ^= 1; }
+                ready = __all_sync(0xffffffffu, next);
+                s = s2;
+                ph = ph2;
             }
         }
     } else if (warp == 1) {
         constexpr uint32_t idesc = tc_idesc(kTcRows, BN);
+        // Whether the next step's operands are there is asked in front of this step's products and known behind them: a wait for a
+        // barrier that is through costs 300 clocks, and the tensor core has no more than two products in hand.
         uint32_t s = 0, ph = 0, it = 0;
-        bool ok = true;
+        bool ok = true, ready = false;
         for (; ok && w.step(); ++it) {
             const uint32_t acc = it & 1, d = tmem + acc * BN;
             if (!(ok = tc_spin_warp(acc_empty + acc, ((it >> 1) & 1) ^ 1, quit))) break;
             umb::tc_fence_after();
             for (int k = 0; k < t.k_steps; ++k) {
-                if (!(ok = tc_spin_warp(full + s, ph, quit))) break;
+                if (!ready && !(ok = tc_spin_warp(full + s, ph, quit))) break;
+                const uint32_t s2 = s + 1 == kStages ? 0 : s + 1, ph2 = s + 1 == kStages ? ph ^ 1 : ph;
+                const bool next = tc_test(full + s2, ph2);
                 umb::tc_fence_after();
                 const uint32_t st = smem_u32(smem + s * Cfg::kStage);
                 const uint64_t ad = umb::umma_smem_desc_sw128(st), wd = umb::umma_smem_desc_sw128(st + Cfg::kABytes);
@@ -158,8 +165,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     umb::umma_commit(empty + s);
                     if (k + 1 == t.k_steps) umb::umma_commit(acc_full + acc);
                 }
-                __syncwarp();
-                if (++s == kStages) { s = 0; ph ^= 1; }
+                ready = __all_sync(0xffffffffu, next);
+                s = s2;
+                ph = ph2;
             }
         }
     } else if (warp < 6) {

@@ -35,12 +35,21 @@ __device__ __forceinline__ bool tc_spin(uint64_t* bar, uint32_t parity, volatile
     }
     return tc_give_up(quit);
 }
-// The same by a whole warp, which is one again behind it.  The warps that issue copies and products run their loops whole and
+// The same by a whole warp, which is one again behind it (the loop as one statement: as C++ its exits cost 100 clocks a wait).  The warps that issue copies and products run their loops whole and
 // elect a thread for the instructions themselves: inside a branch that one thread takes, operands leave the uniform registers
 // and every tcgen05 instruction and every passed wait costs hundreds of clocks (measured with clock64 stamps: 8 products of
 // 128 x 32 x 16 and a passed wait 1740 clocks, a wait for a finished barrier 370).
 __device__ __forceinline__ bool tc_spin_warp(uint64_t* bar, uint32_t parity, volatile int* quit) {
-    return __all_sync(0xffffffffu, tc_spin(bar, parity, quit));
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, 0;\n\t"
+        "AGAIN_%=:\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra DONE_%=;\n\t"
+        "add.u32 n, n, 1;\n\tsetp.lt.u32 q, n, 33554432;\n\t@q bra AGAIN_%=;\n\t"
+        "DONE_%=:\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return __all_sync(0xffffffffu, ok) || tc_give_up(quit);
 }
 // polling with a short sleep in between: for warps that share a scheduler with working ones
 __device__ __forceinline__ bool tc_poll(uint64_t* bar, uint32_t parity, volatile int* quit) {
