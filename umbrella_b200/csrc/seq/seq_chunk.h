@@ -26,4 +26,10 @@ int chunk_segments(int base_blocks, int max_seq_len, size_t fit, int* seg_len);
 int chunk_base_blocks(int n_seqs, int heads, int vdim);
 int launch_chunk_memory(const ChunkMemory& m, const Batch& b, cudaStream_t st);
 
+// seq_chunk_tc.cu, one decay per head: the 128-token pieces of the longest sequence if the tensor-core kernels take these sizes and
+// addresses and `fit` states per sequence are room enough, else 0.  launch_chunk_tc (m.n_seg: that number): norm_dtype UMBS_*: every
+// head's unit norm and silu gate too, results in `out`; -1: plain results in m.out.
+int chunk_tc_count(const ChunkMemory& m, const Batch& b, const void* out, size_t fit);
+int launch_chunk_tc(const ChunkMemory& m, const Batch& b, int norm_dtype, float eps, void* out, cudaStream_t st);
+
 }  // namespace umbs

@@ -1,0 +1,516 @@
+// Matrix memories with one decay per head (seq_chunk.h, retention) on the 5th-generation tensor cores: a prompt's tokens 128 at a time,
+// every 128 of them in blocks of their own.  With D[i][j] = decay^(i - j) for j <= i, else 0, and S the state in front of the 128:
+//     states   L = (diag(decay^(n - 1 - j)) K)^T V                      a block per 128 tokens, head and 128 value columns
+//     chain    S <- decay^n S + L, from the slot's state to the slot's state, every S kept: a thread per element
+//     outputs  O = diag(decay^(i + 1)) Q S + ((Q K^T) o D) V            a block as for the states; then the head's norm and gate
+// Every operand is 32-bit and taken as three bf16 parts in six products (seq_gemm_split.cu); a product's leading part is summed over at
+// most 128 of k and apart from the small ones, so no chain through the tensor core is longer than eight.  Sums whose parts are no
+// numbers (infinite or NaN operands, or beyond bf16) are worked out again in plain fp32.
+//
+// Bound: what a block does one after the other (rows in, split, products, weights split again, products, out: 6 us for states, 10 for
+// outputs), 512 blocks of each on 148 SMs; outputs hold 192 KB of shared memory, states 72 KB three to an SM.
+#include <math.h>
+
+#include "seq_chunk.h"
+#include "seq_tc.cuh"
+
+namespace umbs {
+
+constexpr int kCtT = 128;                                   // tokens of a block
+constexpr int kCtStates = 1024 + 3 * (64 * 128 * 2 + 64 * 128);             // V and K of 64 tokens
+constexpr int kCtOutputs = 1024 + 3 * (128 * 128 + 128 * 128 + 128 * 256);  // Q, K (then the state), V
+
+__device__ __forceinline__ void ld8(const float* p, float (&f)[8]) {
+    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+    f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
+    f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+}
+// Numbers d .. d + 7 of a token's query or key row, scaled and turned (d, dim, half of rot_dims: multiples of 8; zeros behind dim).
+__device__ __forceinline__ void turned8(const ChunkMemory& x, int64_t tok, int off, float scale, int d, float (&f)[8]) {
+    if (d >= x.dim) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = 0.f;
+        return;
+    }
+    const float* row = x.x + tok * x.ld + off;
+    ld8(row + d, f);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] *= scale;
+    if (d >= x.rot_dims) return;
+    const int half = x.rot_dims / 2;
+    const bool low = d < half;
+    const float* tab = x.rot_tab + tok * x.rot_dims + (low ? d : d - half);
+    float g[8], c[8], s[8];
+    ld8(row + (low ? d + half : d - half), g);
+    ld8(tab, c);
+    ld8(tab + half, s);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] = low ? f[e] * c[e] - g[e] * scale * s[e] : f[e] * c[e] + g[e] * scale * s[e];
+}
+__device__ __forceinline__ float turned(const ChunkMemory& x, int64_t tok, int off, float scale, int d) {
+    float f[8];
+    turned8(x, tok, off, scale, d & ~7, f);
+    float r = f[0];
+#pragma unroll
+    for (int e = 1; e < 8; ++e) r = (d & 7) == e ? f[e] : r;
+    return r;
+}
+__device__ __forceinline__ void st_parts(uint32_t at, uint32_t step, const float (&f)[8]) {
+    uint4 v[3];
+    split8(f, v);
+#pragma unroll
+    for (int e = 0; e < 3; ++e)
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(at + e * step), "r"(v[e].x), "r"(v[e].y), "r"(v[e].z), "r"(v[e].w) : "memory");
+}
+__device__ __forceinline__ bool no_number(float v) { return !(fabsf(v) <= 3.402823466e38f); }
+// an operand whose k runs down the rows: its 64-wide pieces are `piece` bytes apart, groups of eight rows 1024
+__device__ __forceinline__ uint64_t mn_desc(uint32_t addr, uint32_t piece) {
+    return (umb::umma_smem_desc_sw128(addr) & ~((uint64_t)0x3fff << 16)) | ((uint64_t)(piece >> 4) << 16);
+}
+
+// element (d, c) of L, token by token
+__device__ __noinline__ float plain_state(const ChunkMemory& x, int64_t tok, int nb, int h, int d, int c, float dec) {
+    float s = 0.f;
+    for (int j = 0; j < nb; ++j)
+        s = fmaf(s, dec, turned(x, tok + j, x.koff + h * x.dim, x.kscale, d) * x.x[(tok + j) * x.ld + x.voff + h * x.vdim + c]);
+    return s;
+}
+// element (i, c) of O, token by token; st: the state in front of the tokens
+__device__ float plain_output(const ChunkMemory& x, int64_t tok, int i, int h, int c, float dec, const float* st) {
+    float o = 0.f;
+    for (int d = 0; d < x.dim; ++d) o = fmaf(turned(x, tok + i, x.qoff + h * x.dim, x.qscale, d), st[(int64_t)d * x.vdim + c], o);
+    o *= powf(dec, (float)(i + 1));
+    for (int j = 0; j <= i; ++j) {
+        float w = 0.f;
+        for (int d = 0; d < x.dim; ++d)
+            w = fmaf(turned(x, tok + i, x.qoff + h * x.dim, x.qscale, d), turned(x, tok + j, x.koff + h * x.dim, x.kscale, d), w);
+        o = fmaf(w * powf(dec, (float)(i - j)), x.x[(tok + j) * x.ld + x.voff + h * x.vdim + c], o);
+    }
+    return o;
+}
+
+// columns c0 + e of row i for the bits e of odd
+__device__ __noinline__ void plain_outputs(const ChunkMemory& x, int64_t tok, int i, int h, int c0, float dec, const float* st, uint32_t odd, float* o) {
+    for (; odd; odd &= odd - 1) o[__ffs(odd) - 1] = plain_output(x, tok, i, h, c0 + __ffs(odd) - 1, dec, st);
+}
+
+__global__ void __launch_bounds__(256, 3) chunk_states_kernel(const __grid_constant__ ChunkMemory x, const __grid_constant__ Batch b, unsigned int* report) {
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ uint64_t done;
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_quit;
+    __shared__ float keep[kCtT];
+    volatile int* quit = &s_quit;
+    unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    chain_wait();
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int s = blockIdx.x / x.n_seg, c = blockIdx.x - s * x.n_seg, h = blockIdx.y, c0 = blockIdx.z * 128;
+    const int t0 = c * kCtT, nb = min(kCtT, b.seq_len[s] - t0);
+    if (nb <= 0) return;
+    const int64_t tok = b.seq_start[s] + t0;
+    const int nv = min(128, x.vdim - c0);
+    const float dec = x.decay[h];
+    if (tid < kCtT) keep[tid] = tid < nb ? powf(dec, (float)(nb - 1 - tid)) : 0.f;
+    if (tid == 0) {
+        umb::mbar_init(&done, 1);
+        s_quit = 0;
+        umb::fence_barrier_init();
+    }
+    if (warp == 0) {
+        umb::tmem_alloc(&s_tmem, 128);
+        umb::tmem_relinquish();
+    }
+    umb::tc_fence_before();
+    __syncthreads();
+    umb::tc_fence_after();
+    const uint32_t tmem = s_tmem, s_v = smem_u32(smem), s_k = s_v + 3 * 16384;
+    constexpr uint32_t idesc = tc_idesc(128, 64, true) | (1u << 15);
+    bool ok = true;
+    for (int half = 0; half < 2 && half * 64 < nb && ok; ++half) {
+        if (half == 1 && !(ok = __syncthreads_and(tc_spin_warp(&done, 0, quit)))) break;
+        const int ch = tid & 7, r8 = tid >> 3, cv = tid & 15, r16 = tid >> 4;
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const int r = r8 + 32 * p, j = half * 64 + r;
+            float f[8] = {};
+            if (j < nb) {
+                turned8(x, tok + j, x.koff + h * x.dim, x.kscale, ch * 8, f);
+                const float w = keep[j];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) f[e] *= w;
+            }
+            st_parts(s_k + r * 128 + ((ch ^ (r & 7)) << 4), 8192, f);
+        }
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const int r = r16 + 16 * p, j = half * 64 + r;
+            float f[8] = {};
+            if (j < nb && cv * 8 < nv) ld8(x.x + (tok + j) * x.ld + x.voff + h * x.vdim + c0 + cv * 8, f);
+            st_parts(s_v + (cv >> 3) * 8192 + r * 128 + (((cv & 7) ^ (r & 7)) << 4), 16384, f);
+        }
+        umb::fence_proxy_async_smem();
+        __syncthreads();
+        if (warp == 0) {
+            const uint64_t vd = mn_desc(s_v, 8192), kd = mn_desc(s_k, 8192);
+            const uint32_t more = half ? 1u : 0u;
+            if (umb::elect_one()) {
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+#pragma unroll
+                    for (int j = 0; j < 3 - i; ++j)
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                            umb::umma_ss_f16(tmem + (i + j ? 64 : 0), vd + i * (16384 >> 4) + kk * (2048 >> 4), kd + j * (8192 >> 4) + kk * (2048 >> 4), idesc,
+                                             kk > 0 || i > 0 || j > 1 ? 1u : more);
+                umb::umma_commit(&done);
+            }
+            __syncwarp();
+        }
+    }
+    if (ok) ok = __syncthreads_and(tc_spin_warp(&done, nb > 64 ? 1 : 0, quit));
+    if (ok) {
+        umb::tc_fence_after();
+        // lane: value column; 32 dimensions a warp
+        const int q = warp & 3, d0 = (warp >> 2) * 32, col = q * 32 + lane;
+        const uint32_t at = tmem + ((uint32_t)(q * 32) << 16) + d0;
+        uint32_t u[32], v[32];
+        UMB_TMEM_LD_X32(at, u);
+        UMB_TMEM_LD_X32(at + 64, v);
+        umb::tc_wait_ld();
+        float* out = x.seg_state + (((int64_t)s * x.n_seg + c) * x.heads + h) * x.dim * x.vdim + c0 + col;
+        uint32_t odd = 0;
+        if (col < nv)
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+                if (d0 + i < x.dim) {
+                    const float l = __uint_as_float(u[i]) + __uint_as_float(v[i]);
+                    odd |= (uint32_t)no_number(l) << i;
+                    out[(int64_t)(d0 + i) * x.vdim] = l;
+                }
+        for (; odd; odd &= odd - 1) {
+            const int d = d0 + __ffs(odd) - 1;
+            out[(int64_t)d * x.vdim] = plain_state(x, tok, nb, h, d, c0 + col, dec);
+        }
+    }
+    __syncwarp();
+    umb::tc_fence_before();
+    __syncthreads();
+    tc_settle(quit, report);
+    if (warp == 0) {
+        umb::tc_fence_after();
+        umb::tmem_dealloc(tmem, 128);
+    }
+}
+
+// A thread per state element: every L is replaced by the state in front of its tokens; eight of them are on their way at a time.
+__global__ void chunk_chain_kernel(const ChunkMemory x, const Batch b) {
+    chain_wait();
+    const int64_t plane = (int64_t)x.heads * x.dim * x.vdim, e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int s = blockIdx.y, len = b.seq_len[s];
+    if (e >= plane || len <= 0) return;
+    const float dec = x.decay[(int)(e / ((int64_t)x.dim * x.vdim))], whole = powf(dec, (float)kCtT);
+    const int n = (len + kCtT - 1) / kCtT;
+    float* slot = x.state + (int64_t)b.seq_slot[s] * plane + e;
+    float* p = x.seg_state + (int64_t)s * x.n_seg * plane + e;
+    float S = b.seq_pos0[s] > 0 ? *slot : 0.f;
+    for (int c = 0; c < n; c += 8) {
+        float l[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) l[i] = c + i < n ? p[(c + i) * plane] : 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (c + i >= n) continue;
+            p[(c + i) * plane] = S;
+            S = fmaf(c + i + 1 < n ? whole : powf(dec, (float)(len - (n - 1) * kCtT)), S, l[i]);
+        }
+    }
+    *slot = S;
+}
+
+// T: the result's type; float with NORM false: o as it is, for a norm over several heads
+template <typename T, bool NORM>
+__global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_constant__ ChunkMemory x, const __grid_constant__ Batch b, float eps, T* __restrict__ out,
+                                                               unsigned int* report) {
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ uint64_t done;
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_quit, s_bad;
+    __shared__ float lam[kCtT + 1], red[4][kCtT];
+    volatile int* quit = &s_quit;
+    unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    chain_wait();
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int s = blockIdx.x / x.n_seg, c = blockIdx.x - s * x.n_seg, h = blockIdx.y, c0 = blockIdx.z * 128;
+    const int t0 = c * kCtT, nb = min(kCtT, b.seq_len[s] - t0);
+    if (nb <= 0) return;
+    const int64_t tok = b.seq_start[s] + t0;
+    const int nv = min(128, x.vdim - c0);
+    const float dec = x.decay[h];
+    if (tid <= kCtT) lam[tid] = powf(dec, (float)tid);
+    if (tid == 0) {
+        umb::mbar_init(&done, 1);
+        s_quit = 0;
+        s_bad = kCtT;
+        umb::fence_barrier_init();
+    }
+    if (warp == 0) {
+        umb::tmem_alloc(&s_tmem, 512);
+        umb::tmem_relinquish();
+    }
+    const uint32_t s_q = smem_u32(smem), s_k = s_q + 3 * 16384, s_v = s_k + 3 * 16384;
+    const int ch = tid & 7, r8 = tid >> 3, cv = tid & 15, r16 = tid >> 4;
+    // values and state are asked for first, and are there when their turn comes
+    const float* st = x.seg_state + (((int64_t)s * x.n_seg + c) * x.heads + h) * x.dim * x.vdim;
+    float vf[4][8] = {}, sf[2][8] = {};
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const int r = r16 + 32 * p;
+        if (r < nb && cv * 8 < nv) ld8(x.x + (tok + r) * x.ld + x.voff + h * x.vdim + c0 + cv * 8, vf[p]);
+    }
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const int d = r16 + 32 * p;
+        if (d < x.dim && cv * 8 < nv) ld8(st + (int64_t)d * x.vdim + c0 + cv * 8, sf[p]);
+    }
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const int r = r8 + 64 * p;
+        const uint32_t at = r * 128 + ((ch ^ (r & 7)) << 4);
+        float f[8] = {}, g[8] = {};
+        if (r < nb) {
+            turned8(x, tok + r, x.qoff + h * x.dim, x.qscale, ch * 8, f);
+            turned8(x, tok + r, x.koff + h * x.dim, x.kscale, ch * 8, g);
+        }
+        st_parts(s_q + at, 16384, f);
+        st_parts(s_k + at, 16384, g);
+    }
+    umb::fence_proxy_async_smem();
+    umb::tc_fence_before();
+    __syncthreads();
+    umb::tc_fence_after();
+    // tensor memory: scores 0-127 and their small terms 128-255, later the weights' parts 0-63, 64-127, 128-191; results 256-383, 384-511
+    const uint32_t tmem = s_tmem;
+    if (warp == 0) {
+        const uint64_t qd = umb::umma_smem_desc_sw128(s_q), kd = umb::umma_smem_desc_sw128(s_k);
+        if (umb::elect_one()) {
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3 - i; ++j)
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+                        umb::umma_ss_f16(tmem + (i + j ? 128 : 0), qd + i * (16384 >> 4) + kk * 2, kd + j * (16384 >> 4) + kk * 2, tc_idesc(128, 128),
+                                         kk > 0 || i > 0 || j > 1 ? 1u : 0u);
+            umb::umma_commit(&done);
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const int r = r16 + 32 * p;
+        // a weight of 0 times a value that is no number is none either: such values stay out of the product, and the rows from their token
+        // on are worked out in plain fp32 (the rows in front of it keep their bits)
+        bool bad = false;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const bool no = !(fabsf(vf[p][e]) <= 0x1.fep127f);
+            bad |= no;
+            vf[p][e] = no ? 0.f : vf[p][e];
+        }
+        if (bad) atomicMin(&s_bad, r);
+        st_parts(s_v + (cv >> 3) * 16384 + r * 128 + (((cv & 7) ^ (r & 7)) << 4), 32768, vf[p]);
+    }
+    // row i: the row of this thread, of which it has 32 columns
+    const int q = warp & 3, part = (warp >> 2) * 32, i = q * 32 + lane;
+    const uint32_t row = tmem + ((uint32_t)(q * 32) << 16);
+    float o[32];
+    bool ok = __syncthreads_and(tc_spin_warp(&done, 0, quit));
+    if (ok) {
+        umb::tc_fence_after();
+        uint32_t u[32], v[32];
+        UMB_TMEM_LD_X32(row + part, u);
+        UMB_TMEM_LD_X32(row + 128 + part, v);
+        umb::tc_wait_ld();
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {                       // the keys have been read: the state takes their place
+            const int d = r16 + 32 * p;
+            st_parts(s_k + (cv >> 3) * 8192 + d * 128 + (((cv & 7) ^ (d & 7)) << 4), 16384, sf[p]);
+        }
+        umb::fence_proxy_async_smem();
+        umb::tc_fence_before();
+        __syncthreads();                                    // (and every thread has read its scores)
+        if (warp == 0) {
+            umb::tc_fence_after();
+            const uint64_t qd = umb::umma_smem_desc_sw128(s_q), sd = mn_desc(s_k, 8192);
+            if (umb::elect_one()) {
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+#pragma unroll
+                    for (int j = 0; j < 3 - a; ++j)
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                            umb::umma_ss_f16(tmem + (a + j ? 384 : 256), qd + a * (16384 >> 4) + kk * 2, sd + j * (16384 >> 4) + kk * (2048 >> 4),
+                                             tc_idesc(128, 128, true), kk > 0 || a > 0 || j > 1 ? 1u : 0u);
+                umb::umma_commit(&done);
+            }
+            __syncwarp();
+        }
+        uint32_t w0[16], w1[16], w2[16];                    // weights of two tokens each, in three parts
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+            float p[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int far = i - (part + 2 * e + k);
+                const float z = __uint_as_float(u[2 * e + k]) + __uint_as_float(v[2 * e + k]);
+                p[k] = far >= 0 ? z * lam[far >= 0 ? far : 0] : 0.f;        // (chosen: a later token's NaN stays its own)
+            }
+            uint32_t* to[3] = {&w0[e], &w1[e], &w2[e]};
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const __nv_bfloat162 r = __floats2bfloat162_rn(p[0], p[1]);
+                const uint32_t bits = *reinterpret_cast<const uint32_t*>(&r);
+                *to[k] = bits;
+                p[0] -= __uint_as_float(bits << 16);
+                p[1] -= __uint_as_float(bits & 0xffff0000u);
+            }
+        }
+        UMB_TMEM_ST_X16(row + part / 2, w0);
+        UMB_TMEM_ST_X16(row + 64 + part / 2, w1);
+        UMB_TMEM_ST_X16(row + 128 + part / 2, w2);
+        umb::tc_wait_st();
+        ok = __syncthreads_and(tc_spin_warp(&done, 1, quit));
+    }
+    if (ok) {
+        umb::tc_fence_after();
+        uint32_t u[32], v[32];
+        UMB_TMEM_LD_X32(row + 256 + part, u);
+        UMB_TMEM_LD_X32(row + 384 + part, v);
+        umb::tc_wait_ld();
+        const float f = lam[i + 1];
+#pragma unroll
+        for (int e = 0; e < 32; ++e) o[e] = f * (__uint_as_float(u[e]) + __uint_as_float(v[e]));
+        umb::tc_fence_before();
+        __syncthreads();
+        if (warp == 0) {
+            umb::tc_fence_after();
+            const uint64_t vd = mn_desc(s_v, 16384);
+            if (umb::elect_one()) {
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+#pragma unroll
+                    for (int j = 0; j < 3 - a; ++j)
+#pragma unroll
+                        for (int kk = 0; kk < 8; ++kk)
+                            umb::umma_ts_f16(tmem + (a + j ? 384 : 256), tmem + a * 64 + kk * 8, vd + j * (32768 >> 4) + kk * (2048 >> 4), tc_idesc(128, 128, true),
+                                             kk > 0 || a > 0 || j > 1 ? 1u : 0u);
+                umb::umma_commit(&done);
+            }
+            __syncwarp();
+        }
+        if (NORM && i < nb && part < nv)                    // the gate's row, for the end
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(x.x + (tok + i) * x.ld + x.voff + x.heads * x.vdim + (int64_t)h * x.vdim + c0 + part));
+        ok = __syncthreads_and(tc_spin_warp(&done, 0, quit));
+    }
+    if (ok) {
+        umb::tc_fence_after();
+        uint32_t u[32], v[32];
+        UMB_TMEM_LD_X32(row + 256 + part, u);
+        UMB_TMEM_LD_X32(row + 384 + part, v);
+        umb::tc_wait_ld();
+        const int n0 = c0 + part;                           // this thread's first column
+        uint32_t odd = 0;
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+            o[e] += __uint_as_float(u[e]) + __uint_as_float(v[e]);
+            odd |= (uint32_t)((i >= s_bad || no_number(o[e])) && i < nb && part + e < nv) << e;
+        }
+        if (odd) {
+            float f[32];
+#pragma unroll
+            for (int e = 0; e < 32; ++e) f[e] = o[e];
+            plain_outputs(x, tok, i, h, n0, dec, st, odd, f);
+#pragma unroll
+            for (int e = 0; e < 32; ++e) o[e] = f[e];
+        }
+        float ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < 32; ++e) ss = fmaf(o[e], o[e], ss);             // (columns that are not there: 0)
+        const int hv = x.heads * x.vdim;
+        T* orow = out + (tok + i) * hv + (int64_t)h * x.vdim + n0;
+        float inv = 1.f;
+        if (NORM) {                                         // o / rms(o) over the head, times silu(g)
+            red[warp >> 2][i] = ss;
+            __syncthreads();
+            inv = 1.f / sqrtf(((red[0][i] + red[1][i]) + (red[2][i] + red[3][i])) / (float)x.vdim + eps);
+        }
+        if (i < nb) {
+            const float* g = x.x + (tok + i) * x.ld + x.voff + hv + (int64_t)h * x.vdim + n0;
+#pragma unroll
+            for (int e = 0; e < 32; e += 8) {
+                if (part + e >= nv) continue;               // (vdim is a multiple of 8)
+                float r[8], gv[8];
+                if (NORM) ld8(g + e, gv);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) r[k] = NORM ? o[e + k] * inv * (gv[k] / (1.f + expf(-gv[k]))) : o[e + k];
+                if constexpr (sizeof(T) == 4) {
+                    *reinterpret_cast<float4*>(orow + e) = make_float4(r[0], r[1], r[2], r[3]);
+                    *reinterpret_cast<float4*>(orow + e + 4) = make_float4(r[4], r[5], r[6], r[7]);
+                } else {
+                    uint32_t wds[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const __nv_bfloat162 pr = __floats2bfloat162_rn(r[2 * k], r[2 * k + 1]);
+                        wds[k] = *reinterpret_cast<const uint32_t*>(&pr);
+                    }
+                    *reinterpret_cast<uint4*>(orow + e) = make_uint4(wds[0], wds[1], wds[2], wds[3]);
+                }
+            }
+        }
+    }
+    __syncwarp();
+    umb::tc_fence_before();
+    __syncthreads();
+    tc_settle(quit, report);
+    if (warp == 0) {
+        umb::tc_fence_after();
+        umb::tmem_dealloc(tmem, 512);
+    }
+}
+
+int chunk_tc_count(const ChunkMemory& m, const Batch& b, const void* out, size_t fit) {
+    const int n = (b.max_seq_len + kCtT - 1) / kCtT;
+    auto al = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
+    if (m.gates != nullptr || m.normaliser || m.dim % 8 || m.dim > 64 || m.vdim % 8 || m.rot_dims % 16 || b.max_seq_len < kCtT || (size_t)n > fit) return 0;
+    if (m.ld % 4 || m.qoff % 4 || m.koff % 4 || m.voff % 4 || !al(m.x) || !al(m.seg_state) || !al(out) || (m.rot_dims > 0 && !al(m.rot_tab))) return 0;
+    return n;
+}
+
+template <typename T, bool NORM>
+static int launch_outputs(const ChunkMemory& m, const Batch& b, const dim3& grid, float eps, T* out, unsigned int* report, cudaStream_t st) {
+    auto kernel = chunk_outputs_kernel<T, NORM>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCtOutputs);
+    return e != cudaSuccess ? (int)e : chain_launch(kernel, grid, 512, kCtOutputs, st, m, b, eps, out, report);
+}
+
+int launch_chunk_tc(const ChunkMemory& m, const Batch& b, int norm_dtype, float eps, void* out, cudaStream_t st) {
+    unsigned int* report = nullptr;
+    int rc = give_up_word(&report);
+    if (rc == 0) rc = give_up_status();
+    if (rc != 0) return rc;
+    const dim3 grid(b.n_seqs * m.n_seg, m.heads, (m.vdim + 127) / 128);
+    const cudaError_t e = cudaFuncSetAttribute(chunk_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCtStates);
+    if (e != cudaSuccess) return (int)e;
+    rc = chain_launch(chunk_states_kernel, grid, 256, kCtStates, st, m, b, report);
+    if (rc != 0) return rc;
+    const int64_t plane = (int64_t)m.heads * m.dim * m.vdim;
+    rc = chain_launch(chunk_chain_kernel, dim3((unsigned)((plane + 255) / 256), b.n_seqs), 256, 0, st, m, b);
+    if (rc != 0) return rc;
+    if (norm_dtype == UMBS_BF16) return launch_outputs<__nv_bfloat16, true>(m, b, grid, eps, (__nv_bfloat16*)out, report, st);
+    if (norm_dtype == UMBS_F32) return launch_outputs<float, true>(m, b, grid, eps, (float*)out, report, st);
+    return launch_outputs<float, false>(m, b, grid, eps, m.out, report, st);
+}
+
+unsigned int chunk_tc_timeouts() { return tc_timeouts(); }
+
+}  // namespace umbs

@@ -27,23 +27,6 @@ constexpr int kSpThreads = 32 * (kSpConv + kSpSum + 1);
 constexpr int kSpSmem = 1024 + kSpStages * 3 * (kTcRows + kSpMaxN) * 128;
 constexpr int kSpChunk = 2;                                 // k steps whose a0 w0 the tensor core sums
 
-// eight numbers to three rows of eight bf16
-__device__ __forceinline__ void split8(const float (&f)[8], uint4 (&p)[3]) {
-    uint32_t* o[3] = {&p[0].x, &p[1].x, &p[2].x};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        float a = f[2 * i], b = f[2 * i + 1];
-#pragma unroll
-        for (int e = 0; e < 3; ++e) {
-            const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-            const uint32_t u = *reinterpret_cast<const uint32_t*>(&h);
-            o[e][i] = u;
-            a -= __uint_as_float(u << 16);
-            b -= __uint_as_float(u & 0xffff0000u);
-        }
-    }
-}
-
 __device__ __forceinline__ bool odd_sum(float s) { return !(fabsf(s) <= 3.402823466e38f) || (s != 0.f && fabsf(s) < 0x1p-90f); }
 
 // What 16 neighbouring sums of a row become, in place (DUAL: u the up half).  Sums that the parts do not give are worked out again in

@@ -384,4 +384,4 @@ int launch_gemm_tc(const GemmArgs& a, int groups, bool dual, bool c_f32, cudaStr
 }  // namespace umbs
 
 extern "C" unsigned int umbs_give_ups_seen(void) { return umbs::give_up_status() != 0; }
-extern "C" unsigned int umbs_kernel_timeouts(void) { return umbs::tc_timeouts() + umbs::attention_tc_timeouts() + umbs::split_timeouts(); }
+extern "C" unsigned int umbs_kernel_timeouts(void) { return umbs::tc_timeouts() + umbs::attention_tc_timeouts() + umbs::split_timeouts() + umbs::chunk_tc_timeouts(); }

@@ -1066,6 +1066,19 @@ extern "C" int umbs_retention_ex(int dtype, const float* qkvg, int64_t ld, const
     if (rot_dims < 0 || rot_dims > dim || (rot_dims & 1)) return UMB_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     unsigned launches = 2;
+    auto gate = [&](unsigned launches) -> int {
+        if (opts != nullptr && opts->norm_w != nullptr) {
+            count_launches(launches - 1);
+            const int hv = heads * vdim;
+            return umbs_gated_norm_ex(dtype, o_scratch, qkvg + 2 * (int64_t)heads * dim + hv, ld, batch->n_tokens, hv, opts->norm_parts,
+                                      opts->norm_w, hv, 0, opts->gate_act, eps, out, stream);
+        }
+        const int warps = batch->n_tokens * heads;
+        UMBS_DISPATCH_T(dtype, retention_gate_kernel<T><<<(warps + 3) / 4, 128, 0, st>>>(o_scratch, qkvg, ld, batch->n_tokens,
+                                                                                       heads, dim, vdim, eps, (T*)out));
+        count_launches(launches);
+        return (int)cudaGetLastError();
+    };
     // a step with several tokens per sequence shares one cos | sin table between heads and column blocks; a decode step
     // works the few values out inside the recurrence kernel
     const float* rot_tab = nullptr;
@@ -1079,6 +1092,22 @@ extern "C" int umbs_retention_ex(int dtype, const float* qkvg, int64_t ld, const
     // recurrence for n_seg times the blocks; the result differs from the single walk by fp32 rounding only.
     int n_seg = 1, seg_len = batch->max_seq_len;
     const size_t fit = seg_scratch != nullptr ? seg_bytes / ((size_t)batch->n_seqs * heads * dim * vdim * sizeof(float)) : 0;
+    const bool heads_norm = opts == nullptr || opts->norm_w == nullptr;     // (vdim > 128: a head's norm spans blocks)
+    {
+        ChunkMemory m{qkvg, ld, 0, heads * dim, 2 * heads * dim, heads, dim, vdim, 1.f, kscale, rot_dims, rot_tab, decay, nullptr, 0,
+                      state, (int64_t)dim * vdim, o_scratch, kChunkTokens, 1, 0, seg_scratch, nullptr};
+        const bool fused = heads_norm && vdim <= 128;
+        m.n_seg = chunk_tc_count(m, *batch, fused ? out : (void*)o_scratch, fit);
+        if (m.n_seg > 0) {
+            if (const int rc = launch_chunk_tc(m, *batch, fused ? dtype : -1, eps, out, st)) return rc;
+            launches += 2;
+            if (fused) {
+                count_launches(launches);
+                return (int)cudaGetLastError();
+            }
+            return gate(launches);
+        }
+    }
     // Steps with long sequences take their tokens 32 at a time (seq_chunk.cu); 16 sequences of 63, 64, 128 tokens take
     // 58, 58, 98 us walked and 42, 62 us in chunks (64, 128); below 64 tokens one sequence alone gains nothing (38 us both ways).
     const bool chunks = batch->max_seq_len >= 64 && chunk_memory_fits(dim, vdim);
@@ -1117,17 +1146,7 @@ extern "C" int umbs_retention_ex(int dtype, const float* qkvg, int64_t ld, const
         rc = run(0);
     }
     if (rc) return rc;
-    if (opts != nullptr && opts->norm_w != nullptr) {
-        count_launches(launches - 1);
-        const int hv = heads * vdim;
-        return umbs_gated_norm_ex(dtype, o_scratch, qkvg + 2 * (int64_t)heads * dim + hv, ld, batch->n_tokens, hv, opts->norm_parts,
-                                  opts->norm_w, hv, 0, opts->gate_act, eps, out, stream);
-    }
-    const int warps = batch->n_tokens * heads;
-    UMBS_DISPATCH_T(dtype, retention_gate_kernel<T><<<(warps + 3) / 4, 128, 0, st>>>(o_scratch, qkvg, ld, batch->n_tokens,
-                                                                                   heads, dim, vdim, eps, (T*)out));
-    count_launches(launches);
-    return (int)cudaGetLastError();
+    return gate(launches);
 }
 
 extern "C" int umbs_latent_norm(int dtype, const float* x, int n, int q_rank, int kv_rank, const float* q_norm,

@@ -76,12 +76,30 @@ __host__ __device__ constexpr uint32_t tc_idesc(uint32_t M, uint32_t N, bool w_m
     return (1u << 4) | (1u << 7) | (1u << 10) | ((w_mn_major ? 1u : 0u) << 16) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
+// eight fp32 numbers as three rows of eight bf16, rounded to nearest one after the other: their sum, exactly, where all are finite
+__device__ __forceinline__ void split8(const float (&f)[8], uint4 (&p)[3]) {
+    uint32_t* o[3] = {&p[0].x, &p[1].x, &p[2].x};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float a = f[2 * i], b = f[2 * i + 1];
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+            const uint32_t u = *reinterpret_cast<const uint32_t*>(&h);
+            o[e][i] = u;
+            a -= __uint_as_float(u << 16);
+            b -= __uint_as_float(u & 0xffff0000u);
+        }
+    }
+}
+
 static inline unsigned int tc_timeouts() {
     unsigned int n = 0;
     return cudaMemcpyFromSymbol(&n, g_tc_timeouts, sizeof n) == cudaSuccess ? n : ~0u;
 }
 unsigned int attention_tc_timeouts();                       // seq_attn_tc.cu
 unsigned int split_timeouts();                              // seq_gemm_split.cu
+unsigned int chunk_tc_timeouts();                           // seq_chunk_tc.cu
 
 // seq_gemm_tc.cu: bf16 [groups][rows][cols] with row stride ld and group stride gs (elements) as a tensor map of boxes of 64
 // columns x box_rows rows, 128-byte swizzle, zeros outside
