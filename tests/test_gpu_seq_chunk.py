@@ -52,6 +52,31 @@ def test_retention(lens, dim, vdim, rot):
         assert H.rel_err(y, got[0][0]) < 1e-5 and H.rel_err(state, got[0][1]) < 1e-5
 
 
+# pieces of 128 tokens (csrc/seq/seq_chunk_tc.cu): key and value sizes in eights and rotations in sixteens; a piece's edges, values in
+# one block of 128 columns and in two, a norm per head (in the kernel where a head is one block) and over all heads
+@pytest.mark.parametrize("lens", [(128,), (300, 1, 128), (255, 257, 383)])
+@pytest.mark.parametrize("dim,vdim,rot", [(8, 8, 0), (64, 72, 48), (40, 136, 32), (64, 128, 64)])
+@pytest.mark.parametrize("all_heads", [False, True])
+def test_retention_in_pieces_of_128(lens, dim, vdim, rot, all_heads):
+    from umbrella_b200 import ops_seq as K
+    heads = 3
+    g = torch.Generator().manual_seed(sum(lens) + dim)
+    x = torch.randn(sum(lens), 2 * heads * (dim + vdim), generator=g).to(DEV)
+    decay = torch.tensor([0.97, 0.9995, 0.1], device=DEV)
+    freq = (1e4 ** (-torch.arange(0, max(rot, 2), 2) / max(rot, 2))).float().to(DEV)
+    w = (1 + 0.1 * torch.randn(heads * vdim, generator=g)).to(DEV) if all_heads else None
+    got = []
+    for size in (40, 10 ** 6, 150):
+        state = torch.full((len(lens), heads, dim, vdim), 3.0, device=DEV)
+        y = _feed(lambda r, b: K.retention(r, b, heads, dim, vdim, rot, freq, decay, 1e-6, state, norm_w=w), lens, size, x)
+        got.append((y, state.clone()))
+    for y, state in got[1:]:
+        assert H.rel_err(y, got[0][0]) < 1e-5 and H.rel_err(state, got[0][1]) < 1e-5
+    bf = K.retention(x, K.RaggedBatch([(i, n, 0, 0) for i, n in enumerate(lens)], DEV), heads, dim, vdim, rot, freq, decay, 1e-6, state,
+                     dtype=torch.bfloat16, norm_w=w)
+    assert H.rel_err(bf, got[0][0]) < 2.0 ** -8
+
+
 @pytest.mark.parametrize("lens", LENS)
 @pytest.mark.parametrize("dim,vdim", [(64, 128), (32, 64), (24, 64), (36, 64), (4, 4), (60, 132)])
 def test_mlstm(lens, dim, vdim):

@@ -7,8 +7,11 @@
 // most 128 of k and apart from the small ones, so no chain through the tensor core is longer than eight.  Sums whose parts are no
 // numbers (infinite or NaN operands, or beyond bf16) are worked out again in plain fp32.
 //
-// Bound: what a block does one after the other (rows in, split, products, weights split again, products, out: 6 us for states, 10 for
-// outputs), 512 blocks of each on 148 SMs; outputs hold 192 KB of shared memory, states 72 KB three to an SM.
+// Bound: what a block does one after the other (rows in, split, products, weights split again, products, out), four warps a scheduler
+// in step: outputs 33,000 clocks a block, of which the products take 6,000, three and a half blocks to an SM (192 KB of shared memory
+// and all of tensor memory each); states three blocks to an SM (72 KB).  4096 tokens of 16 heads 64 x 128: 238 us in pieces of 32
+// tokens on the multiply-add pipe with a norm-and-gate kernel behind, 117 here (states 29, chain 9, outputs 75, cold).  Distance from
+// float64 2.1e-7 -> 1.1e-7 (fp32 results of 128 to 1500 tokens), states 1.7e-7 -> 0.9e-7.
 #include <math.h>
 
 #include "seq_chunk.h"
@@ -16,7 +19,7 @@
 
 namespace umbs {
 
-constexpr int kCtT = 128;                                   // tokens of a block
+constexpr int kCtT = 128, kCtStride = 132;                  // tokens of a block; floats between rows of results
 constexpr int kCtStates = 1024 + 3 * (64 * 128 * 2 + 64 * 128);             // V and K of 64 tokens
 constexpr int kCtOutputs = 1024 + 3 * (128 * 128 + 128 * 128 + 128 * 256);  // Q, K (then the state), V
 
@@ -46,6 +49,23 @@ __device__ __forceinline__ void turned8(const ChunkMemory& x, int64_t tok, int o
     ld8(tab + half, s);
 #pragma unroll
     for (int e = 0; e < 8; ++e) f[e] = low ? f[e] * c[e] - g[e] * scale * s[e] : f[e] * c[e] + g[e] * scale * s[e];
+}
+// The same for numbers 8 ch .. 8 ch + 7 of a row whose pieces the eight lanes of a row hold in f, with the turn's cos and sin.
+__device__ __forceinline__ void load_turn(const ChunkMemory& x, int64_t tok, int ch, float (&c)[8], float (&s)[8]) {
+    const int hc = x.rot_dims / 16;
+    if (ch >= 2 * hc) return;
+    const float* tab = x.rot_tab + tok * x.rot_dims + (ch < hc ? ch : ch - hc) * 8;
+    ld8(tab, c);
+    ld8(tab + x.rot_dims / 2, s);
+}
+__device__ __forceinline__ void turn_row(const ChunkMemory& x, int ch, float (&f)[8], const float (&c)[8], const float (&s)[8]) {
+    const int hc = x.rot_dims / 16, lane = threadIdx.x & 31;
+    const int from = (lane & ~7) | (ch < hc ? ch + hc : (ch < 2 * hc ? ch - hc : ch));
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const float g = __shfl_sync(0xffffffffu, f[e], from);
+        if (ch < 2 * hc) f[e] = ch < hc ? f[e] * c[e] - g * s[e] : f[e] * c[e] + g * s[e];
+    }
 }
 __device__ __forceinline__ float turned(const ChunkMemory& x, int64_t tok, int off, float scale, int d) {
     float f[8];
@@ -106,10 +126,10 @@ __global__ void __launch_bounds__(256, 3) chunk_states_kernel(const __grid_const
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int s = blockIdx.x / x.n_seg, c = blockIdx.x - s * x.n_seg, h = blockIdx.y, c0 = blockIdx.z * 128;
     const int t0 = c * kCtT, nb = min(kCtT, b.seq_len[s] - t0);
-    if (nb <= 0) return;
     const int64_t tok = b.seq_start[s] + t0;
-    const int nv = min(128, x.vdim - c0);
     const float dec = x.decay[h];
+    if (nb <= 0) return;
+    const int nv = min(128, x.vdim - c0);
     if (tid < kCtT) keep[tid] = tid < nb ? powf(dec, (float)(nb - 1 - tid)) : 0.f;
     if (tid == 0) {
         umb::mbar_init(&done, 1);
@@ -127,25 +147,31 @@ __global__ void __launch_bounds__(256, 3) chunk_states_kernel(const __grid_const
     constexpr uint32_t idesc = tc_idesc(128, 64, true) | (1u << 15);
     bool ok = true;
     for (int half = 0; half < 2 && half * 64 < nb && ok; ++half) {
-        if (half == 1 && !(ok = __syncthreads_and(tc_spin_warp(&done, 0, quit)))) break;
         const int ch = tid & 7, r8 = tid >> 3, cv = tid & 15, r16 = tid >> 4;
+        float kf[2][8] = {}, cf[2][8], sf[2][8];            // asked for ahead of the wait
 #pragma unroll
         for (int p = 0; p < 2; ++p) {
-            const int r = r8 + 32 * p, j = half * 64 + r;
-            float f[8] = {};
-            if (j < nb) {
-                turned8(x, tok + j, x.koff + h * x.dim, x.kscale, ch * 8, f);
-                const float w = keep[j];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) f[e] *= w;
+            const int j = half * 64 + r8 + 32 * p;
+            if (j < nb && ch * 8 < x.dim) {
+                ld8(x.x + (tok + j) * x.ld + x.koff + h * x.dim + ch * 8, kf[p]);
+                load_turn(x, tok + j, ch, cf[p], sf[p]);
             }
-            st_parts(s_k + r * 128 + ((ch ^ (r & 7)) << 4), 8192, f);
+        }
+        if (half == 1 && !(ok = __syncthreads_and(tc_spin_warp(&done, 0, quit)))) break;
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const int r = r8 + 32 * p;
+            turn_row(x, ch, kf[p], cf[p], sf[p]);
+            const float w = keep[half * 64 + r];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) kf[p][e] = w == 0.f ? 0.f : kf[p][e] * x.kscale * w;     // (tokens that are not there, or forgotten: nothing)
+            st_parts(s_k + r * 128 + ((ch ^ (r & 7)) << 4), 8192, kf[p]);
         }
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
-            const int r = r16 + 16 * p, j = half * 64 + r;
+            const int r = r16 + 16 * p;
             float f[8] = {};
-            if (j < nb && cv * 8 < nv) ld8(x.x + (tok + j) * x.ld + x.voff + h * x.vdim + c0 + cv * 8, f);
+            if (half * 64 + r < nb && cv * 8 < nv) ld8(x.x + (tok + half * 64 + r) * x.ld + x.voff + h * x.vdim + c0 + cv * 8, f);
             st_parts(s_v + (cv >> 3) * 8192 + r * 128 + (((cv & 7) ^ (r & 7)) << 4), 16384, f);
         }
         umb::fence_proxy_async_smem();
@@ -208,21 +234,27 @@ __global__ void chunk_chain_kernel(const ChunkMemory x, const Batch b) {
     const int64_t plane = (int64_t)x.heads * x.dim * x.vdim, e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int s = blockIdx.y, len = b.seq_len[s];
     if (e >= plane || len <= 0) return;
-    const float dec = x.decay[(int)(e / ((int64_t)x.dim * x.vdim))], whole = powf(dec, (float)kCtT);
     const int n = (len + kCtT - 1) / kCtT;
+    const float dec = x.decay[(int)e / (x.dim * x.vdim)], whole = powf(dec, (float)kCtT), rest = powf(dec, (float)(len - (n - 1) * kCtT));
     float* slot = x.state + (int64_t)b.seq_slot[s] * plane + e;
     float* p = x.seg_state + (int64_t)s * x.n_seg * plane + e;
-    float S = b.seq_pos0[s] > 0 ? *slot : 0.f;
-    for (int c = 0; c < n; c += 8) {
-        float l[8];
+    float S = b.seq_pos0[s] > 0 ? *slot : 0.f, l[8];
+    auto fetch = [&](int c) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) l[i] = c + i < n ? p[(c + i) * plane] : 0.f;
+    };
+    fetch(0);
+    for (int c = 0; c < n; c += 8) {
+        float f[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            if (c + i >= n) continue;
-            p[(c + i) * plane] = S;
-            S = fmaf(c + i + 1 < n ? whole : powf(dec, (float)(len - (n - 1) * kCtT)), S, l[i]);
-        }
+        for (int i = 0; i < 8; ++i) f[i] = l[i];
+        if (c + 8 < n) fetch(c + 8);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (c + i < n) {
+                p[(c + i) * plane] = S;
+                S = fmaf(c + i + 1 < n ? whole : rest, S, f[i]);
+            }
     }
     *slot = S;
 }
@@ -235,17 +267,17 @@ __global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_cons
     __shared__ uint64_t done;
     __shared__ uint32_t s_tmem;
     __shared__ int s_quit, s_bad;
-    __shared__ float lam[kCtT + 1], red[4][kCtT];
+    __shared__ float lam[kCtT + 1];
     volatile int* quit = &s_quit;
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     chain_wait();
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int s = blockIdx.x / x.n_seg, c = blockIdx.x - s * x.n_seg, h = blockIdx.y, c0 = blockIdx.z * 128;
     const int t0 = c * kCtT, nb = min(kCtT, b.seq_len[s] - t0);
-    if (nb <= 0) return;
     const int64_t tok = b.seq_start[s] + t0;
-    const int nv = min(128, x.vdim - c0);
     const float dec = x.decay[h];
+    if (nb <= 0) return;
+    const int nv = min(128, x.vdim - c0);
     if (tid <= kCtT) lam[tid] = powf(dec, (float)tid);
     if (tid == 0) {
         umb::mbar_init(&done, 1);
@@ -259,7 +291,34 @@ __global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_cons
     }
     const uint32_t s_q = smem_u32(smem), s_k = s_q + 3 * 16384, s_v = s_k + 3 * 16384;
     const int ch = tid & 7, r8 = tid >> 3, cv = tid & 15, r16 = tid >> 4;
-    // values and state are asked for first, and are there when their turn comes
+    {
+        float qf[2][8] = {}, kf[2][8] = {}, cf[2][8], sf[2][8];
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const int r = r8 + 64 * p;
+            if (r < nb && ch * 8 < x.dim) {
+                const float* row = x.x + (tok + r) * x.ld + h * x.dim + ch * 8;
+                ld8(row + x.qoff, qf[p]);
+                ld8(row + x.koff, kf[p]);
+                load_turn(x, tok + r, ch, cf[p], sf[p]);
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const int r = r8 + 64 * p;
+            const uint32_t at = r * 128 + ((ch ^ (r & 7)) << 4);
+            turn_row(x, ch, qf[p], cf[p], sf[p]);
+            turn_row(x, ch, kf[p], cf[p], sf[p]);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                qf[p][e] *= x.qscale;
+                kf[p][e] *= x.kscale;
+            }
+            st_parts(s_q + at, 16384, qf[p]);
+            st_parts(s_k + at, 16384, kf[p]);
+        }
+    }
+    // values and state, while the scores are worked out
     const float* st = x.seg_state + (((int64_t)s * x.n_seg + c) * x.heads + h) * x.dim * x.vdim;
     float vf[4][8] = {}, sf[2][8] = {};
 #pragma unroll
@@ -271,18 +330,6 @@ __global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_cons
     for (int p = 0; p < 2; ++p) {
         const int d = r16 + 32 * p;
         if (d < x.dim && cv * 8 < nv) ld8(st + (int64_t)d * x.vdim + c0 + cv * 8, sf[p]);
-    }
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-        const int r = r8 + 64 * p;
-        const uint32_t at = r * 128 + ((ch ^ (r & 7)) << 4);
-        float f[8] = {}, g[8] = {};
-        if (r < nb) {
-            turned8(x, tok + r, x.qoff + h * x.dim, x.qscale, ch * 8, f);
-            turned8(x, tok + r, x.koff + h * x.dim, x.kscale, ch * 8, g);
-        }
-        st_parts(s_q + at, 16384, f);
-        st_parts(s_k + at, 16384, g);
     }
     umb::fence_proxy_async_smem();
     umb::tc_fence_before();
@@ -408,8 +455,6 @@ __global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_cons
             }
             __syncwarp();
         }
-        if (NORM && i < nb && part < nv)                    // the gate's row, for the end
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(x.x + (tok + i) * x.ld + x.voff + x.heads * x.vdim + (int64_t)h * x.vdim + c0 + part));
         ok = __syncthreads_and(tc_spin_warp(&done, 0, quit));
     }
     if (ok) {
@@ -433,38 +478,51 @@ __global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_cons
 #pragma unroll
             for (int e = 0; e < 32; ++e) o[e] = f[e];
         }
-        float ss = 0.f;
+        // rows leave by whole warps, four columns a lane, from where the values were (a thread's own row, 16 bytes of it at a time beside 31
+        // others, took 15,000 clocks of 35,000)
+        float* so = reinterpret_cast<float*>(smem + 6 * 16384);
 #pragma unroll
-        for (int e = 0; e < 32; ++e) ss = fmaf(o[e], o[e], ss);             // (columns that are not there: 0)
-        const int hv = x.heads * x.vdim;
-        T* orow = out + (tok + i) * hv + (int64_t)h * x.vdim + n0;
+        for (int e = 0; e < 32; e += 4) *reinterpret_cast<float4*>(so + i * kCtStride + part + e) = make_float4(o[e], o[e + 1], o[e + 2], o[e + 3]);
+        __syncthreads();
+        const int hv = x.heads * x.vdim, rows = min(8, nb - warp * 8);
+        const float* g = x.x + (tok + warp * 8) * x.ld + x.voff + hv + (int64_t)h * x.vdim + c0 + lane * 4;
+        T* orow = out + (tok + warp * 8) * hv + (int64_t)h * x.vdim + c0 + lane * 4;
+        float4 gv[8];
+        if (NORM && lane * 4 < nv)
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                if (r < rows) gv[r] = *reinterpret_cast<const float4*>(g + r * x.ld);
+        float4 f[8];
         float inv = 1.f;
-        if (NORM) {                                         // o / rms(o) over the head, times silu(g)
-            red[warp >> 2][i] = ss;
-            __syncthreads();
-            inv = 1.f / sqrtf(((red[0][i] + red[1][i]) + (red[2][i] + red[3][i])) / (float)x.vdim + eps);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) f[r] = *reinterpret_cast<const float4*>(so + (warp * 8 + r) * kCtStride + lane * 4);     // (columns that are not there: 0)
+        if (NORM) {                                         // o / rms(o) over the head, times silu(g): lane r has row r's factor
+            float ss = 0.f;
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                float z = fmaf(f[r].x, f[r].x, fmaf(f[r].y, f[r].y, fmaf(f[r].z, f[r].z, f[r].w * f[r].w)));
+#pragma unroll
+                for (int w = 16; w > 0; w >>= 1) z += __shfl_xor_sync(0xffffffffu, z, w);
+                if (lane == r) ss = z;
+            }
+            inv = 1.f / sqrtf(ss / (float)x.vdim + eps);
         }
-        if (i < nb) {
-            const float* g = x.x + (tok + i) * x.ld + x.voff + hv + (int64_t)h * x.vdim + n0;
 #pragma unroll
-            for (int e = 0; e < 32; e += 8) {
-                if (part + e >= nv) continue;               // (vdim is a multiple of 8)
-                float r[8], gv[8];
-                if (NORM) ld8(g + e, gv);
+        for (int r = 0; r < 8; ++r) {
+            if (r >= rows) continue;
+            float z[4] = {f[r].x, f[r].y, f[r].z, f[r].w};
+            if (NORM) {
+                const float by = __shfl_sync(0xffffffffu, inv, r), ga[4] = {gv[r].x, gv[r].y, gv[r].z, gv[r].w};
 #pragma unroll
-                for (int k = 0; k < 8; ++k) r[k] = NORM ? o[e + k] * inv * (gv[k] / (1.f + expf(-gv[k]))) : o[e + k];
-                if constexpr (sizeof(T) == 4) {
-                    *reinterpret_cast<float4*>(orow + e) = make_float4(r[0], r[1], r[2], r[3]);
-                    *reinterpret_cast<float4*>(orow + e + 4) = make_float4(r[4], r[5], r[6], r[7]);
-                } else {
-                    uint32_t wds[4];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const __nv_bfloat162 pr = __floats2bfloat162_rn(r[2 * k], r[2 * k + 1]);
-                        wds[k] = *reinterpret_cast<const uint32_t*>(&pr);
-                    }
-                    *reinterpret_cast<uint4*>(orow + e) = make_uint4(wds[0], wds[1], wds[2], wds[3]);
-                }
+                for (int k = 0; k < 4; ++k) z[k] = z[k] * by * (ga[k] * tc_sigmoid(ga[k]));
+            }
+            if (lane * 4 >= nv) continue;
+            T* to = orow + (int64_t)r * hv;
+            if constexpr (sizeof(T) == 4) {
+                *reinterpret_cast<float4*>(to) = make_float4(z[0], z[1], z[2], z[3]);
+            } else {
+                const __nv_bfloat162 a = __floats2bfloat162_rn(z[0], z[1]), d = __floats2bfloat162_rn(z[2], z[3]);
+                *reinterpret_cast<uint2*>(to) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&d));
             }
         }
     }

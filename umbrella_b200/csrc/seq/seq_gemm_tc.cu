@@ -42,13 +42,6 @@ struct TcCfg {
 // Bias and activation of 32 neighbouring columns of a row, v (and u, the up half) in place.  One choice of activation in
 // front of a loop over independent elements: chosen element by element, every exponential and every quotient waited for the
 // one before it (25 to 40 us for a tile's 128 x 128 outputs, several times its products).
-// The sigmoids' quotient without the rounded division's branch, which costs 12 us of 50 over 4096 rows of 2 x 2048 sums: the
-// hardware's approximate reciprocal and one Newton-Raphson step, r (2 - x r) with the residual in one rounding.  Behind 2^126 the
-// quotient is below the smallest normal number and becomes 0.
-__device__ __forceinline__ float tc_sigmoid(float z) {
-    const float x = 1.f + expf(-z), r = __fdividef(1.f, x);
-    return x >= 0x1p126f ? 0.f : fmaf(r, fmaf(-x, r, 1.f), r);
-}
 template <bool DUAL>
 __device__ __forceinline__ void tc_finish(const GemmArgs& a, uint32_t (&v)[32], uint32_t (&u)[DUAL ? 32 : 1], int n0) {
 #define UMBS_F(x) __uint_as_float(x)

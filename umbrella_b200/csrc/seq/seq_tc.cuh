@@ -76,6 +76,13 @@ __host__ __device__ constexpr uint32_t tc_idesc(uint32_t M, uint32_t N, bool w_m
     return (1u << 4) | (1u << 7) | (1u << 10) | ((w_mn_major ? 1u : 0u) << 16) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
+// The sigmoids' quotient without the rounded division's branch, which costs 12 us of 50 over 4096 rows of 2 x 2048 sums: the
+// hardware's approximate reciprocal and one Newton-Raphson step, r (2 - x r) with the residual in one rounding.  Behind 2^126 the
+// quotient is below the smallest normal number and becomes 0.
+__device__ __forceinline__ float tc_sigmoid(float z) {
+    const float x = 1.f + expf(-z), r = __fdividef(1.f, x);
+    return x >= 0x1p126f ? 0.f : fmaf(r, fmaf(-x, r, 1.f), r);
+}
 // eight fp32 numbers as three rows of eight bf16, rounded to nearest one after the other: their sum, exactly, where all are finite
 __device__ __forceinline__ void split8(const float (&f)[8], uint4 (&p)[3]) {
     uint32_t* o[3] = {&p[0].x, &p[1].x, &p[2].x};
