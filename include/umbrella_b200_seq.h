@@ -679,6 +679,12 @@ int umbs_gated_norm(int dtype, const float* o, const float* gate, int64_t ldg, i
 int umbs_gated_norm_ex(int dtype, const float* o, const float* gate, int64_t ldg, int n, int width, int parts, const float* w, int w_len,
                        int gate_first, int gate_act, float eps, void* out, umbs_stream_t stream);
 
+/* umbs_gemm over rows sorted by group (grp_off, row_src as there) that defines all `rows` rows of C: those of no group, and those of a
+ * group that are left out, are zeros. */
+int umbs_gemm_sorted(int dtype, const void* A, int64_t lda, const void* W, int64_t ldw, int64_t w_gstride, void* C, int64_t ldc,
+                     int c_f32, int M, int rows, int N, int K, int groups, const int32_t* grp_off, const int32_t* row_src, int dual,
+                     float limit, umbs_stream_t stream);
+
 /* umbs_gemm_ex for a plain product followed by a unary activation (UMBS_UNARY_*, with its two numbers). */
 int umbs_gemm_unary(int dtype, const void* A, int64_t lda, int a_goff, const void* W, int64_t ldw, int64_t w_gstride, void* C,
                     int64_t ldc, int c_goff, int c_f32, int M, int N, int K, int groups, const float* bias, int unary,

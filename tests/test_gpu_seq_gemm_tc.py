@@ -257,3 +257,21 @@ def test_split_products_of_numbers_at_the_ends_of_the_range(ops):
         assert ((x - y).norm() / y.norm()).item() < F32_SPLIT_TOL
     x, y = got[4:, 10].double(), ref[4:, 10]
     assert ((x - y).norm() / y.norm()).item() < F32_SPLIT_TOL
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("K,max_rows", [(64, 200), (64, 16), (40, 200)])          # tensor-core tiles, few rows, neither
+def test_sorted_rows_of_no_group_are_zero(ops, dt, K, max_rows):
+    """Rows behind the last group's, into memory that something else has used; a_goff is not used by sorted rows."""
+    sizes = (9, 0, 13)
+    off = torch.tensor([0, 9, 9, 22], dtype=torch.int32, device=DEV)
+    a, w = _mat(101, 30, K).to(dt), _mat(102, 3, 50, K).to(dt)
+    junk = [torch.full((30, 50), float("nan"), device=DEV) for _ in range(8)]
+    del junk
+    got = ops.gemm(a, w, groups=3, grp_off=off, rows=30, max_rows=max_rows, out_f32=True)
+    assert bool((got[22:] == 0).all())
+    lo = 0
+    for g, n in enumerate(sizes):
+        if n:
+            assert H.rel_err(got[lo:lo + n], (a[lo:lo + n].double() @ w[g].double().T).cpu()) < F32_TOL
+        lo += n

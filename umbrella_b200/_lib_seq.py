@@ -134,6 +134,8 @@ SIGNATURES = {
     "umbs_forward": (c_int, [C.POINTER(Model), _BP, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
     "umbs_gemm": (c_int, [c_int, c_void_p, c_int64, c_int, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int, c_int,
                           c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_float, c_void_p]),
+    "umbs_gemm_sorted": (c_int, [c_int, c_void_p, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int, c_int, c_int, c_int,
+                                 c_int, c_int, c_void_p, c_void_p, c_int, c_float, c_void_p]),
     "umbs_gemm_ex": (c_int, [c_int, c_void_p, c_int64, c_int, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int, c_int,
                              c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_float, c_void_p, c_void_p, c_int64, c_int,
                              c_void_p]),

@@ -486,13 +486,22 @@ static int gemm_run(int dtype, const void* A, int64_t lda, int a_goff, const voi
                     void* C, int64_t ldc, int c_goff, int c_f32, int M, int N, int K, int groups,
                     const int32_t* grp_off, const int32_t* row_src, int dual, float limit, const float* bias,
                     const float* out_gate, int64_t ld_gate, int gate_goff, int gate_n, int unary, float p0, float p1, int unary_cols,
-                    umbs_stream_t stream);
+                    umbs_stream_t stream, int rows_total = 0);
 
 extern "C" int umbs_gemm(int dtype, const void* A, int64_t lda, int a_goff, const void* W, int64_t ldw, int64_t w_gstride,
                          void* C, int64_t ldc, int c_goff, int c_f32, int M, int N, int K, int groups,
                          const int32_t* grp_off, const int32_t* row_src, int dual, float limit, umbs_stream_t stream) {
     return umbs_gemm_ex(dtype, A, lda, a_goff, W, ldw, w_gstride, C, ldc, c_goff, c_f32, M, N, K, groups, grp_off, row_src, dual,
                         limit, nullptr, nullptr, 0, 0, stream);
+}
+
+extern "C" int umbs_gemm_sorted(int dtype, const void* A, int64_t lda, const void* W, int64_t ldw, int64_t w_gstride, void* C, int64_t ldc,
+                                int c_f32, int M, int rows, int N, int K, int groups, const int32_t* grp_off, const int32_t* row_src, int dual,
+                                float limit, umbs_stream_t stream) {
+    if (rows <= 0 || N <= 0) return 0;
+    if (C == nullptr || grp_off == nullptr || ldc < N) return UMB_ERR_ARG;
+    return gemm_run(dtype, A, lda, 0, W, ldw, w_gstride, C, ldc, 0, c_f32, M, N, K, groups, grp_off, row_src, dual, limit, nullptr, nullptr, 0, 0,
+                    1, 0, 0.f, 0.f, 0, stream, rows);
 }
 
 extern "C" int umbs_gemm_ex(int dtype, const void* A, int64_t lda, int a_goff, const void* W, int64_t ldw, int64_t w_gstride,
@@ -529,15 +538,22 @@ static int gemm_run(int dtype, const void* A, int64_t lda, int a_goff, const voi
                     void* C, int64_t ldc, int c_goff, int c_f32, int M, int N, int K, int groups,
                     const int32_t* grp_off, const int32_t* row_src, int dual, float limit, const float* bias,
                     const float* out_gate, int64_t ld_gate, int gate_goff, int gate_n, int unary, float p0, float p1, int unary_cols,
-                    umbs_stream_t stream) {
-    if (M <= 0 || N <= 0 || groups <= 0) return 0;
-    if (K <= 0 || A == nullptr || W == nullptr || C == nullptr) return UMB_ERR_ARG;
+                    umbs_stream_t stream, int rows_total) {
     cudaStream_t st = (cudaStream_t)stream;
+    // (the tensor-core tiles take every row of every group and clear what is left themselves: two products of a prompt's 8192 sorted
+    // rows, 18 us of clearing first)
+    auto clear = [&]() -> cudaError_t {
+        const size_t es = dtype == UMBS_F32 || c_f32 ? 4 : 2;
+        return rows_total > 0 ? cudaMemset2DAsync(C, ldc * es, 0, N * es, rows_total, st) : cudaSuccess;
+    };
+    if (M <= 0 || N <= 0 || groups <= 0) return (int)clear();
+    if (K <= 0 || A == nullptr || W == nullptr || C == nullptr) return UMB_ERR_ARG;
     GemmArgs a{A, lda, a_goff, W, ldw, w_gstride, C, ldc, c_goff, M, N, K, grp_off, row_src, limit,
                (dual == UMBS_ACT_GELU_TANH || dual == UMBS_ACT_SILU) ? dual : UMBS_ACT_CLAMPED_GLU,
-               bias, out_gate, ld_gate, gate_goff, gate_n, unary, p0, p1, unary_cols,
+               bias, out_gate, ld_gate, gate_goff, gate_n, unary, p0, p1, unary_cols, rows_total,
                in_chain()};                                 // (a model's products: W is a layer's weight)
     if (dtype == UMBS_F32) {                                              // activations are fp32 too: c_f32 changes nothing
+        if (const cudaError_t e = clear()) return (int)e;
         const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) && (a_goff % 4 == 0) && (w_gstride % 4 == 0) &&
                          ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
         // Streamed rows take 2 us and one for 6.5 million products, tiles on the tensor core 6 us and 1.3 for each 64 of k.  (us, multiply-add
@@ -558,11 +574,13 @@ static int gemm_run(int dtype, const void* A, int64_t lda, int a_goff, const voi
         // (rows that overlap, one row repeated among them: not described by a tensor map, they take the general kernel)
         const bool tc = vec && (K % 32 == 0) && lda >= K && ldw >= K;
         if (vec && M <= 16) {
+            if (const cudaError_t e = clear()) return (int)e;
             if (c_f32) launch_skinny<float>(a, groups, dual != 0, st);
             else launch_skinny<__nv_bfloat16>(a, groups, dual != 0, st);
         } else {
             const int rc = tc ? launch_gemm_tc(a, groups, dual != 0, c_f32 != 0, st) : UMB_ERR_DRIVER;
-            if (rc == UMB_ERR_DRIVER) {                     // (also strides that no tensor map describes: groups that run backwards)
+            if (rc == UMB_ERR_DRIVER) {
+                if (const cudaError_t e = clear()) return (int)e;         // (also strides that no tensor map describes: groups that run backwards)
                 if (c_f32) launch_simt<__nv_bfloat16, float>(a, groups, dual != 0, st);
                 else launch_simt<__nv_bfloat16, __nv_bfloat16>(a, groups, dual != 0, st);
             } else if (rc != 0) {

@@ -258,6 +258,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             unit = (unit + t.k_steps) % kStages;
         }
     }
+    if (!A_TMA && warp >= 2 && warp < 6 && a.rows_total > 0)               // rows of no group
+        for (int64_t r = a.grp_off[t.groups] + (int64_t)blockIdx.x * 4 + warp - 2; r < a.rows_total; r += (int64_t)gridDim.x * 4)
+            for (int n = lane; n < a.N; n += 32) ((TC*)a.C)[r * a.ldc + n] = from_f32<TC>(0.f);
     __syncthreads();
     tc_settle(quit, t.report);
     if (warp == 1) {

@@ -72,9 +72,16 @@ def gemm(a: torch.Tensor, w: torch.Tensor, *, out_f32: bool = False, groups: int
     N = (ws[-2] // (2 if dual else 1)) if n is None else n
     M = a.shape[0] if rows is None else rows
     cols = N if (groups == 1 or grp_off is not None) else groups * c_goff        # expert groups share the columns
+    dt = torch.float32 if out_f32 else a.dtype
+    if grp_off is not None and a_goff == 0 and c_goff == 0:
+        out = torch.empty((M, cols), dtype=dt, device=a.device)
+        S.check(S.load().umbs_gemm_sorted(mode, _p(a), a.stride(0), _p(w), ws[-1], ws[-2] * ws[-1], _p(out), cols, int(out_f32),
+                                          M if max_rows is None else max_rows, M, N, K, groups, _p(grp_off), _p(row_src), int(dual),
+                                          float(limit), _stream()), "gemm")
+        return out
     # (zeros only where the product may leave gaps: rows behind max_rows or the last group's, columns between the groups')
-    make = a.new_empty if groups == 1 and grp_off is None and (max_rows is None or max_rows >= M) else a.new_zeros
-    out = make((M, cols), dtype=torch.float32 if out_f32 else a.dtype)
+    make = torch.empty if groups == 1 and grp_off is None and (max_rows is None or max_rows >= M) else torch.zeros
+    out = make((M, cols), dtype=dt, device=a.device)
     S.check(S.load().umbs_gemm(mode, _p(a), a.stride(0), a_goff, _p(w), ws[-1], ws[-2] * ws[-1], _p(out), cols,
                                c_goff, int(out_f32), M if max_rows is None else max_rows, N, K, groups, _p(grp_off),
                                _p(row_src), int(dual), float(limit), _stream()), "gemm")
