@@ -749,14 +749,17 @@ __device__ __forceinline__ void route_choose(float* z, int experts, int top, int
 // fetched once per kRtTok tokens and a token's number once per kRtExp experts; then a thread per token chooses.  (A block per
 // token read all weights for each token: 512 MB through L2 for 4096 tokens, 16 experts of width 2048, 112 us.)
 constexpr int kRtExp = 4;
+constexpr int kRtPairs = 1024;         // up to so many pairs are handed out by the router's last block
 
 template <typename T, int kRtTok>
 __global__ void __launch_bounds__(256, kRtTok > 4 ? 2 : 1) moe_router_kernel(const T* __restrict__ h, int n, int width, const float* __restrict__ wr,
                                                          int experts, int top, int mode, int groups, int keep, float wscale,
                                                          float* __restrict__ sel_w, int32_t* __restrict__ sel_e,
                                                          int32_t* __restrict__ counts, const float* __restrict__ gate_w,
-                                                         float* __restrict__ gate_out) {
+                                                         float* __restrict__ gate_out, int32_t* __restrict__ cursor, int32_t* __restrict__ grp_off,
+                                                         int32_t* __restrict__ pair_tok, int32_t* __restrict__ pair_pos) {
     extern __shared__ float z[];           // [kRtTok][experts]
+    __shared__ int last;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const bool vec = rows_vec<T>(h, wr, gate_w, width);
     const int t0 = blockIdx.x * kRtTok, rows = experts + (gate_w != nullptr ? 1 : 0);      // one more row for the tokens' gate
@@ -783,6 +786,41 @@ __global__ void __launch_bounds__(256, kRtTok > 4 ? 2 : 1) moe_router_kernel(con
     const int t = t0 + threadIdx.x;
     if (threadIdx.x < kRtTok && t < n)
         route_choose(z + threadIdx.x * experts, experts, top, mode, groups, keep, wscale, sel_w + (int64_t)t * top, sel_e + (int64_t)t * top, counts);
+    // The block that is done last adds the counts up and, for a step of few pairs, hands the pairs out.  (Launches of their own for both:
+    // 64 tokens, 16 experts, top 2: see kRtPairs.)  cursor[0] counts the blocks until then.
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(cursor, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    int* next = reinterpret_cast<int*>(z);                  // [experts] the experts' next free places
+    if (warp == 0) {
+        int base = 0;
+        for (int e0 = 0; e0 < experts; e0 += 32) {
+            const int e = e0 + lane, c = e < experts ? __ldcg(counts + e) : 0;
+            int inc = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += up;
+            }
+            if (e < experts) {
+                grp_off[e] = next[e] = base + inc - c;
+                cursor[e] = 0;
+            }
+            base += __shfl_sync(0xffffffffu, inc, 31);
+        }
+        if (lane == 0) grp_off[experts] = base;
+    }
+    __syncthreads();
+    const int pairs = n * top;
+    if (pairs > kRtPairs) return;                           // moe_scatter_kernel's
+    for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
+        const int p = atomicAdd(next + __ldcg(sel_e + i), 1);
+        pair_tok[p] = i / top;
+        pair_pos[i] = p;
+    }
 }
 
 // The whole routing of a small step (a decode step) in one block: logits of every (token, expert) pair, the choice per
@@ -830,15 +868,6 @@ __global__ void __launch_bounds__(1024) moe_route_small_kernel(const T* __restri
             if (chosen[i] == e) { pair_tok[p] = i / top; pair_pos[i] = p; ++p; }
     }
     for (int i = threadIdx.x; i < n * top; i += blockDim.x) sel_e[i] = chosen[i];
-}
-
-__global__ void moe_offsets_kernel(const int32_t* __restrict__ counts, int experts, int32_t* __restrict__ grp_off,
-                                   int32_t* __restrict__ cursor) {
-    if (threadIdx.x == 0) {
-        int s = 0;
-        for (int e = 0; e < experts; ++e) { grp_off[e] = s; cursor[e] = 0; s += counts[e]; }
-        grp_off[experts] = s;
-    }
 }
 
 __global__ void moe_scatter_kernel(const int32_t* __restrict__ sel_e, int n_pairs, int top,
@@ -1283,7 +1312,7 @@ extern "C" int umbs_moe_route_scaled(int dtype, const void* h, int n, int width,
     int32_t* counts = scratch;                 // [experts]
     int32_t* cursor = scratch + experts;       // [experts]
     int32_t* sel_e = scratch + 2 * experts;    // [n top]
-    cudaError_t e = cudaMemsetAsync(counts, 0, experts * sizeof(int32_t), st);
+    cudaError_t e = cudaMemsetAsync(counts, 0, (experts + 1) * sizeof(int32_t), st);         // (and cursor[0])
     if (e != cudaSuccess) return (int)e;
     const int rthreads = 32 * std::min(8, (experts + (gate_w != nullptr) + kRtExp - 1) / kRtExp);
     // (more tokens to a block once there are blocks enough; thousands of experts need the larger shared memory)
@@ -1295,15 +1324,14 @@ extern "C" int umbs_moe_route_scaled(int dtype, const void* h, int n, int width,
             if (e != cudaSuccess) return (int)e;                                                                                 \
         }                                                                                                                        \
         moe_router_kernel<T, TT><<<(n + TT - 1) / TT, rthreads, smem, st>>>((const T*)h, n, width, w_router, experts, top, mode, groups, keep, \
-                                                                            weight_scale, sel_w, sel_e, counts, gate_w, gate_out); \
+                                                                            weight_scale, sel_w, sel_e, counts, gate_w, gate_out, cursor, grp_off, pair_tok, pair_pos); \
     })
     if (n > 1024 && experts <= 1024) UMBS_ROUTER(8);
     else UMBS_ROUTER(4);
 #undef UMBS_ROUTER
-    moe_offsets_kernel<<<1, 32, 0, st>>>(counts, experts, grp_off, cursor);
     const int pairs = n * top;
-    moe_scatter_kernel<<<(pairs + 255) / 256, 256, 0, st>>>(sel_e, pairs, top, grp_off, cursor, pair_tok, pair_pos);
-    count_launches(3);
+    if (pairs > kRtPairs) moe_scatter_kernel<<<(pairs + 255) / 256, 256, 0, st>>>(sel_e, pairs, top, grp_off, cursor, pair_tok, pair_pos);
+    count_launches(pairs > kRtPairs ? 2 : 1);
     return (int)cudaGetLastError();
 }
 
