@@ -275,3 +275,26 @@ def test_sorted_rows_of_no_group_are_zero(ops, dt, K, max_rows):
         if n:
             assert H.rel_err(got[lo:lo + n], (a[lo:lo + n].double() @ w[g].double().T).cpu()) < F32_TOL
         lo += n
+
+
+# pairs of SMs: tiles of 256 rows x 256 columns (gate|up: 128 of each), rows and columns that end in either half; groups
+@pytest.mark.parametrize("M,N,K", [(1000, 3100, 1056), (1537, 2049, 64), (4096, 1100, 96), (1290, 6144, 512)])
+def test_pairs_of_blocks(ops, M, N, K):
+    from umbrella_b200 import _lib_seq as S
+    a, w, w2 = _mat(111, M, K), _mat(112, N, K), _mat(113, 2 * N, K, scale=K ** -0.5)
+    ref = a.double() @ w.double().T
+    got = ops.gemm(a, w, out_f32=True)
+    assert H.rel_err(got, ref.cpu()) < F32_TOL
+    assert H.rel_err(ops.gemm(a, w), ref.cpu()) < BF16_TOL
+    assert torch.equal(ops.gemm(a[-100:].contiguous(), w, out_f32=True), got[-100:])              # (single blocks)
+    bias = torch.randn(2 * N, device=DEV)
+    z = a.double() @ w2.double().T + bias.double()
+    ref = torch.nn.functional.silu(z[:, :N]) * z[:, N:]
+    assert H.rel_err(ops.gemm_ex(a, w2, act=S.UMBS_ACT_SILU, bias=bias, out_f32=True), ref.cpu()) < F32_TOL
+
+
+def test_pairs_of_blocks_over_heads(ops):
+    M, heads, n, k = 700, 5, 520, 128
+    a, w = _mat(114, M, heads * k), _mat(115, heads, n, k)
+    ref = torch.einsum("mhk,hnk->mhn", a.double().view(M, heads, k), w.double()).reshape(M, heads * n)
+    assert H.rel_err(ops.gemm(a, w, out_f32=True, groups=heads, a_goff=k, c_goff=n), ref.cpu()) < F32_TOL

@@ -24,8 +24,6 @@
 
 namespace umbs {
 
-constexpr int kTcStageRow = 36;                             // fp32 row stride of an epilogue warp's 32 x 32 staging block
-
 template <int BN, bool DUAL>
 struct TcCfg {
     static constexpr int kStages = BN == 256 ? 4 : (BN == 128 ? 6 : 8);
@@ -38,41 +36,6 @@ struct TcCfg {
     static constexpr int kOut = DUAL ? BN / 2 : BN;         // output columns of a tile
     static constexpr int kSmem = 1024 + kStages * kStage + 4 * 32 * kTcStageRow * 4 + 256 + kCopyWarps * kTcRows * 4;
 };
-
-// Bias and activation of 32 neighbouring columns of a row, v (and u, the up half) in place.  One choice of activation in
-// front of a loop over independent elements: chosen element by element, every exponential and every quotient waited for the
-// one before it (25 to 40 us for a tile's 128 x 128 outputs, several times its products).
-template <bool DUAL>
-__device__ __forceinline__ void tc_finish(const GemmArgs& a, uint32_t (&v)[32], uint32_t (&u)[DUAL ? 32 : 1], int n0) {
-#define UMBS_F(x) __uint_as_float(x)
-#define UMBS_EACH(expr)                                                                     \
-    _Pragma("unroll") for (int j = 0; j < 32; ++j) {                                        \
-        const float x = UMBS_F(v[j]), y = DUAL ? UMBS_F(u[DUAL ? j : 0]) : 0.f;              \
-        v[j] = __float_as_uint(expr);                                                       \
-        (void)y;                                                                            \
-    }
-    if (a.bias != nullptr) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            const int n = min(n0 + j, a.N - 1);
-            v[j] = __float_as_uint(UMBS_F(v[j]) + a.bias[n]);
-            if (DUAL) u[DUAL ? j : 0] = __float_as_uint(UMBS_F(u[DUAL ? j : 0]) + a.bias[a.N + n]);
-        }
-    }
-    if (DUAL) {
-        if (a.act == UMBS_ACT_GELU_TANH) UMBS_EACH(gated_act(x, y, a.limit, UMBS_ACT_GELU_TANH))
-        else if (a.act == UMBS_ACT_SILU) UMBS_EACH(x * tc_sigmoid(x) * y)
-        else UMBS_EACH(fminf(x, a.limit) * tc_sigmoid(1.702f * fminf(x, a.limit)) * (fminf(fmaxf(y, -a.limit), a.limit) + 1.f))
-    } else if (a.unary && n0 + 32 <= a.unary_cols && (a.unary == UMBS_UNARY_SILU || a.unary == UMBS_UNARY_RELU2 || a.unary == UMBS_UNARY_SCALE)) {
-        if (a.unary == UMBS_UNARY_SILU) UMBS_EACH(x * tc_sigmoid(x))
-        else if (a.unary == UMBS_UNARY_RELU2) UMBS_EACH(unary_act(x, UMBS_UNARY_RELU2, a.p0, a.p1))
-        else UMBS_EACH(unary_act(x, UMBS_UNARY_SCALE, a.p0, a.p1))
-    } else if (a.unary) {
-        UMBS_EACH(n0 + j < a.unary_cols ? unary_act(x, a.unary, a.p0, a.p1) : x)
-    }
-#undef UMBS_EACH
-#undef UMBS_F
-}
 
 template <int BN, bool DUAL, bool A_TMA, typename TC>
 __global__ void __launch_bounds__(TcCfg<BN, DUAL>::threads(A_TMA), 1)
@@ -166,60 +129,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     } else if (warp < 6) {
         const int q = warp & 3;                             // the quarter of tensor-memory lanes this warp may read
         float* so = s_out + (warp - 2) * 32 * kTcStageRow;
-        const int rr = lane >> 3, cc = (lane & 7) * 4;
         for (uint32_t it = 0; w.step(); ++it) {
             const uint32_t acc = it & 1;
             if (!__all_sync(0xffffffffu, tc_poll(acc_full + acc, (it >> 1) & 1, quit))) break;      // (and the warp is one again)
             umb::tc_fence_after();
-            const uint32_t src = tmem + acc * BN + ((uint32_t)(q * 32) << 16);
-            const int rows = w.rows - w.m0 - q * 32, n_hi = a.N - w.n0 * kOut;      // rows of this quarter, columns of the tile
-            TC* C = (TC*)a.C + (int64_t)w.g * a.c_goff + (int64_t)(w.row_lo + w.m0 + q * 32) * a.ldc + w.n0 * kOut;
-            const int64_t grow = w.row_lo + w.m0 + q * 32;
-#pragma unroll 1
-            for (int c0 = 0; c0 < kOut; c0 += 32) {
-                uint32_t v[32], u[DUAL ? 32 : 1];
-                UMB_TMEM_LD_X32(src + c0, v);
-                if (DUAL) UMB_TMEM_LD_X32(src + kOut + c0, u);
-                umb::tc_wait_ld();
-                if (c0 + 32 >= kOut) {                      // read to the end: the next tile but one may be summed here
-                    umb::tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) umb::mbar_arrive(acc_empty + acc);
-                }
-                if (c0 >= n_hi || rows <= 0) continue;
-                if (DUAL || a.bias != nullptr || a.unary) tc_finish<DUAL>(a, v, u, w.n0 * kOut + c0);
-#pragma unroll
-                for (int j = 0; j < 32; j += 4)
-                    *reinterpret_cast<uint4*>(so + lane * kTcStageRow + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                __syncwarp();
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int r = i * 4 + rr, n = c0 + cc;
-                    if (r < rows && n < n_hi) {
-                        const float4 f = *reinterpret_cast<const float4*>(so + r * kTcStageRow + cc);
-                        float o[4] = {f.x, f.y, f.z, f.w};
-                        if (a.out_gate != nullptr) {
-#pragma unroll
-                            for (int e = 0; e < 4; ++e)
-                                if (n + e < n_hi) o[e] = finish_gate(a, o[e], w.g, grow + r, w.n0 * kOut + n + e);
-                        }
-                        TC* p = C + (int64_t)r * a.ldc + n;
-                        if (t.vec_c && n + 4 <= n_hi) {
-                            if constexpr (sizeof(TC) == 4) {
-                                *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]);
-                            } else {
-                                __nv_bfloat162 lo = __floats2bfloat162_rn(o[0], o[1]), hi = __floats2bfloat162_rn(o[2], o[3]);
-                                *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
-                            }
-                        } else {
-#pragma unroll
-                            for (int e = 0; e < 4; ++e)
-                                if (n + e < n_hi) p[e] = from_f32<TC>(o[e]);
-                        }
-                    }
-                }
-                __syncwarp();
-            }
+            tc_store_tile<kOut, kOut, DUAL, TC>(a, t.vec_c, tmem + acc * BN + ((uint32_t)(q * 32) << 16), so, w.g, w.row_lo + w.m0 + q * 32,
+                                          w.rows - w.m0 - q * 32, w.n0 * kOut, [&] { umb::mbar_arrive(acc_empty + acc); });
         }
     } else if (!A_TMA) {
         // eight lanes copy a row's 128 bytes of the k step; the image is the one a 128-byte-swizzled TMA box would leave
@@ -362,16 +277,26 @@ int launch_gemm_tc(const GemmArgs& a, int groups, bool dual, bool c_f32, cudaStr
     t.m_tiles = (a.M + kTcRows - 1) / kTcRows;
     const int es = c_f32 ? 4 : 2;
     t.vec_c = (uintptr_t)a.C % (4 * es) == 0 && a.ldc % 4 == 0 && a.c_goff % 4 == 0;
-    // The tile width with the shortest longest walk: rounds of tiles over the SMs times what 16 of k cost, which is the tensor
-    // core's 128 clocks for 256 columns and more than half, a quarter of that for 128 and 64: 72 and 52 (the activation tile is
-    // fetched and read from shared memory for fewer products).  (Rows sorted by expert: how they fall is only known on the device;
-    // spread evenly is the guess.)
+    // The tile width with the shortest longest walk.  Dense rows, in ns: what a launch, a tile's first operands and its last results take,
+    // and a k step of a round of tiles (measured, loaded chip; pairs of SMs: seq_gemm_pair.cu).  us, single blocks / pairs: 803 rows, K =
+    // 1024, to 1024 / 3088 columns 8.6 / 12.1, 15.2 / 13.3; 1500, K = 2048, to 6144 34.9 / 31.0; 4096 90.0 / 80.1; 4096, K = 1024, to 4096
+    // 41.8 / 34.1.
+    // Rows sorted by expert (how they fall is only known on the device; spread evenly is the guess): rounds of tiles times what 16 of k
+    // cost, the tensor core's 128 clocks for 256 columns and more than half, a quarter of that for 128 and 64: 72 and 52 (the activation
+    // tile is fetched and read from shared memory for fewer products).
+    const bool dense = a.grp_off == nullptr && a.row_src == nullptr;
     const int64_t m = a.grp_off != nullptr ? (int64_t)groups * ((a.M + groups * kTcRows - 1) / (groups * kTcRows)) : (int64_t)groups * t.m_tiles;
-    auto cost = [&](int bn, int step) {
+    const int64_t steps = dense ? (a.K + kTcK - 1) / kTcK : 1;
+    auto cost = [&](int bn, int step, int once) {
         const int out = dual ? bn / 2 : bn;
-        return (m * ((a.N + out - 1) / out) + sms - 1) / sms * step;
+        return (m * ((a.N + out - 1) / out) + sms - 1) / sms * steps * step + (dense ? once : 0);
     };
-    const int64_t c256 = cost(256, 128), c128 = cost(128, 72), c64 = cost(64, 52);
+    const int64_t c256 = cost(256, dense ? 410 : 128, 8300), c128 = cost(128, dense ? 275 : 72, 6000), c64 = cost(64, dense ? 250 : 52, 4300);
+    if (dense && a.M > kTcRows) {
+        const int out = dual ? 128 : 256;
+        const int64_t tiles = (int64_t)groups * ((a.M + 255) / 256) * ((a.N + out - 1) / out), pair = (tiles + sms / 2 - 1) / (sms / 2) * steps * 370 + 6800;
+        if (pair < c256 && pair < c128 && pair < c64) return launch_gemm_pair(a, t, dual, c_f32, sms, st);
+    }
     if (c256 <= c128 && c256 <= c64) return launch_tc_any<256>(a, t, dual, c_f32, sms, st);
     if (c128 <= c64) return launch_tc_any<128>(a, t, dual, c_f32, sms, st);
     return launch_tc_any<64>(a, t, dual, c_f32, sms, st);
@@ -380,4 +305,4 @@ int launch_gemm_tc(const GemmArgs& a, int groups, bool dual, bool c_f32, cudaStr
 }  // namespace umbs
 
 extern "C" unsigned int umbs_give_ups_seen(void) { return umbs::give_up_status() != 0; }
-extern "C" unsigned int umbs_kernel_timeouts(void) { return umbs::tc_timeouts() + umbs::attention_tc_timeouts() + umbs::split_timeouts() + umbs::chunk_tc_timeouts(); }
+extern "C" unsigned int umbs_kernel_timeouts(void) { return umbs::tc_timeouts() + umbs::attention_tc_timeouts() + umbs::split_timeouts() + umbs::pair_timeouts() + umbs::chunk_tc_timeouts(); }

@@ -107,6 +107,7 @@ static inline unsigned int tc_timeouts() {
 unsigned int attention_tc_timeouts();                       // seq_attn_tc.cu
 unsigned int split_timeouts();                              // seq_gemm_split.cu
 unsigned int chunk_tc_timeouts();                           // seq_chunk_tc.cu
+unsigned int pair_timeouts();                               // seq_gemm_pair.cu
 
 // seq_gemm_tc.cu: bf16 [groups][rows][cols] with row stride ld and group stride gs (elements) as a tensor map of boxes of 64
 // columns x box_rows rows, 128-byte swizzle, zeros outside
