@@ -44,10 +44,11 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
 
 void count_launches(unsigned n);
 
-// The launches of one umbs_forward are a chain: a kernel of it may be brought onto the SMs while the one in front of it still runs,
-// and waits there (chain_wait, ahead of everything it reads or writes but the model's weights) until that one is done and its
-// results are visible.  Every block waits, so a kernel is done only after all those in front of it are.  A decode step is some 80 kernels
-// of 2 to 6 us each; launched one behind the other, 1.2 us of each are its launch.
+// Kernels that follow one another: one may be brought onto the SMs while the one in front of it still runs, and waits there (chain_wait,
+// ahead of everything it reads or writes but a model's weights) until that one is done and its results are visible.  Every block
+// waits, so a kernel is done only after all those in front of it are.  A decode step is some 80 kernels of 2 to 6 us each; launched
+// one behind the other, 1.2 us of each are its launch.
+// A ChainScope says that the launches are one umbs_forward's, whose products' weights were there before its first kernel.
 class ChainScope {                                          // this thread's launches until the scope ends
 public:
     ChainScope();
@@ -57,7 +58,7 @@ public:
 };
 bool in_chain();
 template <typename... P, typename... A>
-int chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+int chain_launch_if(bool early_too, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
     cudaLaunchAttribute early{};
     early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     early.val.programmaticStreamSerializationAllowed = 1;
@@ -67,10 +68,13 @@ int chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaS
     c.dynamicSmemBytes = smem;
     c.stream = st;
     c.attrs = &early;
-    c.numAttrs = in_chain() ? 1 : 0;
+    c.numAttrs = early_too ? 1 : 0;
     return (int)cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
 }
-// (no operation in a kernel that was launched otherwise)
+template <typename... P, typename... A>
+int chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    return chain_launch_if(true, kernel, grid, block, smem, st, std::forward<A>(args)...);
+}
 __device__ __forceinline__ void chain_wait() {
     asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
 }

@@ -144,6 +144,7 @@ __global__ void group_norm_rows_kernel(const float* __restrict__ x, const int32_
 // cos / sin of every (token, frequency) pair of the step, once for all heads: tab[t] = cos[half] | sin[half]
 __global__ void rotary_table_kernel(const int32_t* __restrict__ tok_pos, const float* __restrict__ inv_freq, int half,
                                     float* __restrict__ tab) {
+    chain_wait();
     const int t = blockIdx.x;
     const float p = (float)tok_pos[t];
     for (int i = threadIdx.x; i < half; i += blockDim.x) {
@@ -760,6 +761,7 @@ __global__ void __launch_bounds__(256, kRtTok > 4 ? 2 : 1) moe_router_kernel(con
                                                          int32_t* __restrict__ pair_tok, int32_t* __restrict__ pair_pos) {
     extern __shared__ float z[];           // [kRtTok][experts]
     __shared__ int last;
+    chain_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const bool vec = rows_vec<T>(h, wr, gate_w, width);
     const int t0 = blockIdx.x * kRtTok, rows = experts + (gate_w != nullptr ? 1 : 0);      // one more row for the tokens' gate
@@ -873,6 +875,7 @@ __global__ void __launch_bounds__(1024) moe_route_small_kernel(const T* __restri
 __global__ void moe_scatter_kernel(const int32_t* __restrict__ sel_e, int n_pairs, int top,
                                    const int32_t* __restrict__ grp_off, int32_t* __restrict__ cursor,
                                    int32_t* __restrict__ pair_tok, int32_t* __restrict__ pair_pos) {
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_pairs) return;
     const int e = sel_e[i];
@@ -1112,7 +1115,7 @@ extern "C" int umbs_retention_ex(int dtype, const float* qkvg, int64_t ld, const
     // works the few values out inside the recurrence kernel
     const float* rot_tab = nullptr;
     if (rot_dims > 0 && batch->max_seq_len > 1) {
-        rotary_table_kernel<<<batch->n_tokens, 64, 0, st>>>(batch->tok_pos, inv_freq, rot_dims / 2, rot_scratch);
+        chain_launch(rotary_table_kernel, batch->n_tokens, 64, 0, st, batch->tok_pos, inv_freq, rot_dims / 2, rot_scratch);
         rot_tab = rot_scratch;
         ++launches;
     }
@@ -1323,14 +1326,14 @@ extern "C" int umbs_moe_route_scaled(int dtype, const void* h, int n, int width,
             e = cudaFuncSetAttribute(moe_router_kernel<T, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);          \
             if (e != cudaSuccess) return (int)e;                                                                                 \
         }                                                                                                                        \
-        moe_router_kernel<T, TT><<<(n + TT - 1) / TT, rthreads, smem, st>>>((const T*)h, n, width, w_router, experts, top, mode, groups, keep, \
+        chain_launch(moe_router_kernel<T, TT>, (n + TT - 1) / TT, rthreads, smem, st, (const T*)h, n, width, w_router, experts, top, mode, groups, keep, \
                                                                             weight_scale, sel_w, sel_e, counts, gate_w, gate_out, cursor, grp_off, pair_tok, pair_pos); \
     })
     if (n > 1024 && experts <= 1024) UMBS_ROUTER(8);
     else UMBS_ROUTER(4);
 #undef UMBS_ROUTER
     const int pairs = n * top;
-    if (pairs > kRtPairs) moe_scatter_kernel<<<(pairs + 255) / 256, 256, 0, st>>>(sel_e, pairs, top, grp_off, cursor, pair_tok, pair_pos);
+    if (pairs > kRtPairs) chain_launch(moe_scatter_kernel, (pairs + 255) / 256, 256, 0, st, (const int32_t*)sel_e, pairs, top, (const int32_t*)grp_off, cursor, pair_tok, pair_pos);
     count_launches(pairs > kRtPairs ? 2 : 1);
     return (int)cudaGetLastError();
 }
