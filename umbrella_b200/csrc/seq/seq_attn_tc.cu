@@ -44,7 +44,7 @@ __device__ __forceinline__ void cp16(uint32_t dst, const void* src, int bytes) {
 }
 // the top halves of two words: two bf16 numbers, cut off
 __device__ __forceinline__ uint32_t hi_pair(float a, float b) { return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632); }
-__device__ __forceinline__ float cut(float a) { return __uint_as_float(__float_as_uint(a) & 0xffff0000u); }
+__device__ __forceinline__ float minus_cut(float a) { return __uint_as_float((__float_as_uint(a) & 0xffff0000u) ^ 0x80000000u); }
 
 // The key tiles of a block: pooled blocks first, then tokens.
 struct KeyTiles {
@@ -264,9 +264,9 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
         const uint64_t qd = umb::umma_smem_desc_sw128(smem_u32(smem)), kd0 = umb::umma_smem_desc_sw128(smem_u32(s_k));
         // values: keys down the rows, so the operand is MN-major; its 64-wide pieces are 4096 bytes apart, groups of eight keys 1024
         const uint64_t vd0 = (umb::umma_smem_desc_sw128(smem_u32(s_v)) & ~((uint64_t)0x3fff << 16)) | ((uint64_t)(kTaK * 128 >> 4) << 16);
-        auto scores = [&](int i) -> bool {                  // the tile's score columns were read two tiles ago, in front of weights already waited for
+        auto scores = [&](int i, bool ready) -> bool {      // the tile's score columns were read two tiles ago, in front of weights already waited for
             const int st = i % z.stages;
-            if (!tc_spin_warp(k_full + st, (i / z.stages) & 1, quit)) return false;
+            if (!ready && !tc_spin_warp(k_full + st, (i / z.stages) & 1, quit)) return false;
             umb::tc_fence_after();
             const uint64_t kd = kd0 + ((st * k_bytes) >> 4);
             if (umb::elect_one()) {
@@ -279,12 +279,14 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
             __syncwarp();
             return true;
         };
-        bool ok = scores(0);
+        bool ok = scores(0, false), k_ready = false;
         for (int i = 0; ok && i < kt.n; ++i) {
             const int st = i % z.stages;
-            if (i + 1 < kt.n && !scores(i + 1)) break;
-            if (!tc_spin_warp(v_full + st, (i / z.stages) & 1, quit)) break;
+            const bool v_there = tc_test(v_full + st, (i / z.stages) & 1);
+            if (i + 1 < kt.n && !scores(i + 1, k_ready)) break;
+            if (!__all_sync(0xffffffffu, v_there) && !tc_spin_warp(v_full + st, (i / z.stages) & 1, quit)) break;
             if (!tc_spin_warp(p_full, i & 1, quit)) break;
+            const bool k_there = i + 2 < kt.n && tc_test(k_full + (i + 2) % z.stages, ((i + 2) / z.stages) & 1);
             umb::tc_fence_after();
             const uint64_t vd = vd0 + ((st * v_bytes) >> 4);
             if (umb::elect_one()) {
@@ -296,7 +298,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
                 umb::umma_commit(o_full);
                 umb::umma_commit(v_empty + st);
             }
-            __syncwarp();
+            k_ready = __all_sync(0xffffffffu, k_there);
         }
     } else {
         // ------------------------------------------------------------------------------------ weights: a thread per row
@@ -310,13 +312,13 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
         float l = MODE == UMBS_ATTN_SOFTMAX_SINK ? 1.f : 0.f;                                  // ... without a value
         const int tok_lo = max(rp - window + 1, a.chunk > 0 ? rp / a.chunk * a.chunk : 0);
         const int pool_hi = pooled_visible(rp, window, a.pool);
-        bool ok = true;
+        bool ok = true, s_ready = false;
         for (int i = 0; i < kt.n; ++i) {
             const int base = kt.base(i);                    // keys base .. base + 31, of which [lo, hi) are visible to this row
             const int lo = kt.pooled(i) ? 0 : max(tok_lo - base, 0);
             const int hi = r >= len ? 0 : min((kt.pooled(i) ? pool_hi : rp + 1) - base, kTaK);
             const bool whole = __all_sync(0xffffffffu, lo == 0 && hi == kTaK);
-            if (!(ok = tc_spin_warp(s_full + (i & 1), (i >> 1) & 1, quit))) break;
+            if (!s_ready && !(ok = tc_spin_warp(s_full + (i & 1), (i >> 1) & 1, quit))) break;
             umb::tc_fence_after();
             uint32_t v[32];
             UMB_TMEM_LD_X32(t0 + (i & 1) * kTaK, v);
@@ -333,9 +335,16 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
                         if (j < lo || j >= hi) v[j] = 0x7fffffffu;          // (a maximum passes a NaN by)
                 }
                 float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+                float mx;
+                if (SHAPED || c > 0.f) {                    // (the product rounds every score alike: the largest stays the largest)
 #pragma unroll
-                for (int j = 0; j < 32; ++j) m4[j & 3] = fmaxf(m4[j & 3], __uint_as_float(v[j]) * c);
-                const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+                    for (int j = 0; j < 32; ++j) m4[j & 3] = fmaxf(m4[j & 3], __uint_as_float(v[j]));
+                    mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * c;
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) m4[j & 3] = fmaxf(m4[j & 3], __uint_as_float(v[j]) * c);
+                    mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+                }
                 const bool move = mx > m + (i == 0 ? 0.f : kTaLazy) || (m == -INFINITY && mx > -INFINITY);
                 if (__any_sync(0xffffffffu, move)) {        // rare behind the first tiles: the reference of some row moves
                     const float f = move ? ex2(m - mx) : 1.f;
@@ -357,32 +366,45 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
                 }
             }
             const float ref = m == -INFINITY ? 0.f : m;
+            // two numbers an instruction where there is one for two
+            if (MODE == UMBS_ATTN_SIGMOID) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-                v[j] = __float_as_uint(MODE == UMBS_ATTN_SIGMOID ? sigmoidf_(__uint_as_float(v[j]) * a.scale + hb)
-                                                                 : ex2(fmaf(__uint_as_float(v[j]), c, -ref)));
+                for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(sigmoidf_(__uint_as_float(v[j]) * a.scale + hb));
+            } else {
+                const f32x2 cc = pack2(c, c), rr = pack2(-ref, -ref);
+#pragma unroll
+                for (int j = 0; j < 32; j += 2) {
+                    const float2 z = unpack2(fma2(pack2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), cc, rr));
+                    v[j] = __float_as_uint(ex2(z.x));
+                    v[j + 1] = __float_as_uint(ex2(z.y));
+                }
+            }
             if (!whole) {
 #pragma unroll
                 for (int j = 0; j < 32; ++j)
                     if (j < lo || j >= hi) v[j] = 0u;
             }
-            float l4[4] = {0.f, 0.f, 0.f, 0.f};
+            // (asked in front of the parts, known behind them: a wait for a barrier that is through costs 200 to 350 clocks)
+            const bool o_there = !waited && tc_test(o_full, (i - 1) & 1), s_there = i + 1 < kt.n && tc_test(s_full + ((i + 1) & 1), ((i + 1) >> 1) & 1);
+            f32x2 l2[2] = {0ull, 0ull};
             uint32_t ph[16], pm[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
                 const float p = __uint_as_float(v[2 * j]), p1 = __uint_as_float(v[2 * j + 1]);
-                l4[(2 * j) & 3] += p;
-                l4[(2 * j + 1) & 3] += p1;
-                const float ra = p - cut(p), rb = p1 - cut(p1);
+                const f32x2 pp = pack2(p, p1), r = add2(pp, pack2(minus_cut(p), minus_cut(p1)));
+                const float2 ra = unpack2(r), rb = unpack2(add2(r, pack2(minus_cut(ra.x), minus_cut(ra.y))));
+                l2[j & 1] = add2(l2[j & 1], pp);
                 ph[j] = hi_pair(p, p1);
-                pm[j] = hi_pair(ra, rb);
-                v[j] = hi_pair(ra - cut(ra), rb - cut(rb));                 // (v[2 j] and v[2 j + 1] have been used)
+                pm[j] = hi_pair(ra.x, ra.y);
+                v[j] = hi_pair(rb.x, rb.y);                                 // (v[2 j] and v[2 j + 1] have been used)
             }
-            l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
+            const float2 la = unpack2(l2[0]), lb = unpack2(l2[1]);
+            l += (la.x + la.y) + (lb.x + lb.y);
             if (!waited) {
-                if (!(ok = tc_spin_warp(o_full, (i - 1) & 1, quit))) break;
+                if (!__all_sync(0xffffffffu, o_there) && !(ok = tc_spin_warp(o_full, (i - 1) & 1, quit))) break;
                 umb::tc_fence_after();
             }
+            s_ready = __all_sync(0xffffffffu, s_there);
             UMB_TMEM_ST_X16(t0 + 64, ph);
             UMB_TMEM_ST_X16(t0 + 80, pm);
             UMB_TMEM_ST_X16(t0 + 96, v);
