@@ -210,7 +210,8 @@ def _mat32(seed, *shape, scale=1.0):
     return (torch.randn(*shape, generator=torch.Generator().manual_seed(seed)) * scale).to(DEV)
 
 
-@pytest.mark.parametrize("M,N,K", [(128, 1028, 1000), (129, 1990, 68), (1200, 33, 516), (777, 513, 128), (300, 5000, 132), (40, 9001, 64)])
+@pytest.mark.parametrize("M,N,K", [(128, 1028, 1000), (129, 1990, 68), (1200, 33, 516), (777, 513, 128), (300, 5000, 132), (40, 9001, 64),
+                                   (70000, 2, 8)])
 def test_split_products(ops, M, N, K):
     from umbrella_b200 import _lib_seq as S
     a, w = _mat32(81, M, K), _mat32(82, N, K)

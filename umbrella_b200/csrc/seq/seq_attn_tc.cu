@@ -18,9 +18,10 @@
 // turns: 5800 clocks per 64 keys and block, of which the tensor core works 1160 (measured with clock64 stamps; 128 x 64 x 16
 // takes it 48 clocks, 128 x 128 x 16 takes 64).
 //
-// Bound: the weights (an exponential and three bf16 parts of each score by the row's own thread) between products they wait
-// for: issue slots 43 % taken, tensor pipe 30 % active, fixed latencies the longest stall.  4096 tokens, 16 heads of 128 over 4 key/value heads, window 1024, pooled blocks: 2250 us on fp32 multiply-adds,
-// 141 us here; two prompts of 2000 tokens, 16 heads of 128 + 64 shared: 2652 -> 187 us.
+// Bound: the weights (an exponential and three bf16 parts of each score by the row's own thread: 1450 of a tile's 2400 clocks) beside
+// products of 32 keys, and blocks that fill the SMs 1.7 times.  4096 tokens, 16 heads of 128 over 4 key/value heads, window 1024, pooled
+// blocks: 2250 us on fp32 multiply-adds, 141 with waits of 330 clocks for barriers that were through, 115 here; two prompts of 2000
+// tokens, 16 heads of 128 + 64 shared: 2652 -> 188 -> 158 us.
 #include "seq_attn.h"
 #include "seq_tc.cuh"
 

@@ -15,6 +15,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <algorithm>
 
 #include "seq_gemm.h"
 
@@ -26,8 +27,7 @@ namespace umbs {
 // pieces for 64 multiply-adds, two of them an instruction; an output is one chain of additions over k, so it has the same bits
 // in every tiling.  Bound: two warps a scheduler (162 registers) that wait on their own
 // chains: issue slots 39 % taken, shared memory 52 %, 2.7 times the time of the multiply-adds alone.  Blocks are small so that a step of some hundred rows spreads evenly: 777 x 1024
-// -> 3088 are 637 of them.  16 x 16 threads with 4 x 4 outputs and 4-byte loads took 257 us for it (19 TFLOP/s), this
-// takes 178.
+// -> 3088 are 637 of them: 178 us (27.6 TFLOP/s) as fp32 with rows that the tensor-core form does not take.
 constexpr int BN = 64, BK = 16;
 
 template <typename T> __device__ __forceinline__ void load_k4(const T* p, int left, bool vec, float (&f)[4]) {
@@ -559,9 +559,12 @@ static int gemm_run(int dtype, const void* A, int64_t lda, int a_goff, const voi
         // Streamed rows take 2 us and one for 6.5 million products, tiles on the tensor core 6 us and 1.3 for each 64 of k.  (us, multiply-add
         // tiles / streamed / tensor core, K = 1024: one row of 3088 columns 54 / 4.6 / 29, 64 rows of 1024 45 / 12 / 25, of 3088 51 / 32 / 28, of
         // 8192 73 / 78 / 31; 200 rows of 3088 85 / - / 32; 128 rows, K = 4096, to 1024 columns 184 / 60 / 90.)
-        if (vec && (M <= 16 || (int64_t)M * N * (dual ? 2 : 1) * groups * K <= (int64_t)8500000 * (K / 64 + 4))) {
+        // (the tiles count rows in 16-byte pieces of 32 bits: strides forwards, 64 GB; the streamed rows are the grid's second extent)
+        const int64_t w_rows = (int64_t)N * (dual ? 2 : 1);
+        const bool split = vec && lda >= 0 && ldw >= 0 && lda <= UINT32_MAX / std::max(M, 1) && ldw <= UINT32_MAX / w_rows;
+        if (vec && M <= 4096 && (M <= 16 || (double)M * w_rows * groups * K <= 8.5e6 * (K / 64 + 4))) {
             launch_rows(a, groups, dual != 0, st);
-        } else if (vec) {
+        } else if (split) {
             const int rc = launch_gemm_split(a, groups, dual != 0, st);
             if (rc != 0) return rc;
         } else {

@@ -11,11 +11,11 @@
 // the rest of the batch; against float64 it is as far off as the mma.sync tiles that this replaced (2.1e-6 at K = 2048, in
 // both the tensor core's own accumulation).
 //
-// Bound for dense prompts: the way of a stage from L2, and the last round.  4096 x 2048 -> 6144 has the tensor pipe 61 % active and L2 at
-// 30 % of its throughput; a ring holds four k steps of 48 KB, 512 clocks of products each, and its 768 tiles are 5.2 rounds of the
-// 148 SMs run as 6.  That product (fp32 out): 650 us on 128 x 64 mma.sync tiles (159 TFLOP/s, fragments fetched from shared memory by every warp, 100 MB
-// cleared first), 109 us here (947 TFLOP/s).  16 experts, top 2, 4096 tokens of width 2048 with the routing around it:
-// 808 -> 234 us (gate|up: tensor pipe 42 % active, the copying warps' loads the longest wait); 64 tokens: 213 -> 102 to 110 us.
+// Bound for dense prompts: a block's shared memory, 48 KB in and 48 KB out for 512 clocks of products at 256 columns (690 clocks a step); the
+// large ones go to pairs of SMs (seq_gemm_pair.cu).  With few steps: launch, first operands, last results (8.0 us for K = 1024 to 1024
+// columns, 3.8 of them steps).  16 experts, top 2, 4096 tokens of width 2048 with the routing around it: 808 us on mma.sync tiles, 232 here,
+// 207 without clearing the results first (gate|up 890 clocks a step: the copying warps' loads); 64 tokens: 213 -> 99 -> 86 us (gate|up at
+// the memory's rate inside: 134 MB in 23.5 us).
 #include <cuda.h>
 #include <atomic>
 #include <mutex>

@@ -27,15 +27,7 @@ __device__ __forceinline__ bool tc_test(uint64_t* bar, uint32_t parity) {
         : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return ok != 0;
 }
-// polling: for one thread on a critical path (a parked thread comes back about a microsecond later)
-__device__ __forceinline__ bool tc_spin(uint64_t* bar, uint32_t parity, volatile int* quit) {
-    for (int i = 0; i < (1 << 25); ++i) {
-        if (tc_test(bar, parity)) return true;
-        if ((i & 1023) == 1023 && *quit) return false;
-    }
-    return tc_give_up(quit);
-}
-// The same by a whole warp, which is one again behind it (the loop as one statement: as C++ its exits cost 100 clocks a wait).  The warps that issue copies and products run their loops whole and
+// Polling by a whole warp on a critical path (a parked thread comes back about a microsecond later); it is one again behind it (the loop as one statement: as C++ its exits cost 100 clocks a wait).  The warps that issue copies and products run their loops whole and
 // elect a thread for the instructions themselves: inside a branch that one thread takes, operands leave the uniform registers
 // and every tcgen05 instruction and every passed wait costs hundreds of clocks (measured with clock64 stamps: 8 products of
 // 128 x 32 x 16 and a passed wait 1740 clocks, a wait for a finished barrier 370).
