@@ -1,8 +1,8 @@
 """ctypes binding of libumbrella_b200_seq.so (the C ABI declared in include/umbrella_b200_seq.h): the batched step
 of the sequence-state decoders and its building blocks.
 
-The library is compiled in-tree on first use when it is missing or older than its sources (``build.build_seq``: nine
-small translation units, seconds) -- a fresh checkout serves these models without a separate build step.  There is
+The library is compiled in-tree on first use when it is missing or older than its sources (``build.build_seq``:
+small translation units, under a minute) -- a fresh checkout serves these models without a separate build step.  There is
 no PyTorch / CPU fallback behind these calls: without nvcc and without the library, loading is an error.
 """
 from __future__ import annotations

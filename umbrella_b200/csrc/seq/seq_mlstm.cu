@@ -1,5 +1,6 @@
 // mLSTM: a matrix memory per head with exponential input gates, sigmoid forget gates and a running maximum that keeps
-// the exponentials in range (see umbs_mlstm in include/umbrella_b200_seq.h).  Three kernels per step:
+// the exponentials in range (see umbs_mlstm in include/umbrella_b200_seq.h).  One kernel for a step of one token a sequence
+// (mlstm_decode_kernel), else three:
 //   gates       one block per (sequence, head): the log gates of 32 tokens a warp, the running maximum by a warp scan
 //               of the maps m -> max(m + f, i) (they compose: (f1, i1) then (f2, i2) = (f1 + f2, max(i1 + f2, i2))), and
 //               from it each token's decay e^(f + m' - m), input weight e^(i - m) and floor e^(-m);
