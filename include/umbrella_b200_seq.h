@@ -679,6 +679,15 @@ int umbs_gated_norm(int dtype, const float* o, const float* gate, int64_t ldg, i
 int umbs_gated_norm_ex(int dtype, const float* o, const float* gate, int64_t ldg, int n, int width, int parts, const float* w, int w_len,
                        int gate_first, int gate_act, float eps, void* out, umbs_stream_t stream);
 
+/* Which kernel a product of these sizes takes on a GPU of `sms` SMs when every row of its operands starts on a 16-byte boundary and rows
+ * do not overlap (sorted != 0: rows by grp_off and row_src): one of these, or the columns (64, 128, 256) of one block's tensor-core tiles.
+ * No GPU is asked. */
+#define UMBS_GEMM_GENERAL 0          /* multiply-add tiles */
+#define UMBS_GEMM_FEW_ROWS 1         /* a stream over the weights */
+#define UMBS_GEMM_SPLIT 2            /* fp32 operands as three bf16 parts */
+#define UMBS_GEMM_PAIRS 512          /* tiles of 256 x 256 by pairs of SMs */
+int umbs_gemm_kernel(int dtype, int M, int N, int K, int groups, int sorted, int dual, int sms);
+
 /* umbs_gemm over rows sorted by group (grp_off, row_src as there) that defines all `rows` rows of C: those of no group, and those of a
  * group that are left out, are zeros. */
 int umbs_gemm_sorted(int dtype, const void* A, int64_t lda, const void* W, int64_t ldw, int64_t w_gstride, void* C, int64_t ldc,

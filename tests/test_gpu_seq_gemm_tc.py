@@ -210,10 +210,19 @@ def _mat32(seed, *shape, scale=1.0):
     return (torch.randn(*shape, generator=torch.Generator().manual_seed(seed)) * scale).to(DEV)
 
 
-@pytest.mark.parametrize("M,N,K", [(128, 1028, 1000), (129, 1990, 68), (1200, 33, 516), (777, 513, 128), (300, 5000, 132), (40, 9001, 64),
-                                   (70000, 2, 8)])
+def _kernel(dt, M, N, K, **kw):
+    from umbrella_b200 import _lib_seq as S
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    return S.load().umbs_gemm_kernel(S.UMBS_F32 if dt == torch.float32 else S.UMBS_BF16, M, N, K, kw.get("groups", 1), kw.get("sorted", 0), kw.get("dual", 0), sms)
+
+
+# (the first four sizes are few enough products for the streamed rows in some of the calls; the others take the tiles in all)
+@pytest.mark.parametrize("M,N,K", [(128, 1028, 1000), (129, 1990, 68), (1200, 33, 516), (40, 9001, 64), (777, 513, 128), (300, 5000, 132),
+                                   (70000, 2, 8), (128, 8300, 1000), (129, 19900, 68), (4200, 33, 516), (40, 41000, 64)])
 def test_split_products(ops, M, N, K):
     from umbrella_b200 import _lib_seq as S
+    if (M, N, K) not in ((128, 1028, 1000), (129, 1990, 68), (1200, 33, 516), (40, 9001, 64)):
+        assert _kernel(torch.float32, M, N, K) == _kernel(torch.float32, M, N, K, dual=1) == S.UMBS_GEMM_SPLIT
     a, w = _mat32(81, M, K), _mat32(82, N, K)
     assert H.rel_err(ops.gemm(a, w), (a.double() @ w.double().T).cpu()) < F32_SPLIT_TOL
     w2, bias, gate = _mat32(83, 2 * N, K, scale=K ** -0.5), _mat32(84, 2 * N), _mat32(85, M, N)
@@ -240,9 +249,28 @@ def test_split_products_sorted_by_expert(ops):
         lo += n
 
 
-def test_split_products_of_numbers_at_the_ends_of_the_range(ops):
+def test_split_products_of_wider_rows_and_of_groups(ops):
+    from umbrella_b200 import _lib_seq as S
+    M, N, K = 400, 4000, 72
+    assert _kernel(torch.float32, M, N, K) == S.UMBS_GEMM_SPLIT
+    x, w = _mat32(93, M, K + 28), _mat32(94, N, K)
+    a = x[:, 12:12 + K]                                              # rows further apart than they are long, from a 16-byte boundary on
+    assert H.rel_err(ops.gemm(a, w), (a.double() @ w.double().T).cpu()) < F32_SPLIT_TOL
+    heads, n, k = 3, 1500, 68
+    assert _kernel(torch.float32, M, n, k, groups=heads) == S.UMBS_GEMM_SPLIT
+    a, w = _mat32(95, M, heads * k), _mat32(96, heads, n, k)
+    got = ops.gemm(a, w, groups=heads, a_goff=k, c_goff=n + 1)
+    ref = torch.einsum("mhk,hnk->mhn", a.double().view(M, heads, k), w.double())
+    assert H.rel_err(got.view(M, heads, n + 1)[..., :n], ref.cpu()) < F32_SPLIT_TOL
+    assert bool((got.view(M, heads, n + 1)[..., n] == 0).all())
+
+
+@pytest.mark.parametrize("M,N", [(200, 2000), (400, 4000)])          # streamed, tiles
+def test_split_products_of_numbers_at_the_ends_of_the_range(ops, M, N):
     """Infinite and NaN operands, numbers that round to infinity in bf16, and rows so small that their low parts vanish there."""
-    M, N, K = 200, 2000, 64
+    from umbrella_b200 import _lib_seq as S
+    K = 64
+    assert _kernel(torch.float32, M, N, K) == (S.UMBS_GEMM_SPLIT if M == 400 else S.UMBS_GEMM_FEW_ROWS)
     a, w = _mat32(91, M, K), _mat32(92, N, K)
     a[0, 3], a[1, 5], a[2, 7], w[9, 11] = float("inf"), float("nan"), 3.4e38, float("-inf")
     a[3], w[10] = a[3] * 2.0 ** -120, w[10] * 2.0 ** -100
@@ -294,8 +322,33 @@ def test_pairs_of_blocks(ops, M, N, K):
     assert H.rel_err(ops.gemm_ex(a, w2, act=S.UMBS_ACT_SILU, bias=bias, out_f32=True), ref.cpu()) < F32_TOL
 
 
-def test_pairs_of_blocks_over_heads(ops):
-    M, heads, n, k = 700, 5, 520, 128
+# sizes for which the rule takes pairs in every call: one, two and several steps of 64 of k, k that ends inside one, an odd number of
+# columns, last tiles with rows in the first block alone
+@pytest.mark.parametrize("M,N,K,dual", [(1000, 3100, 1056, 0), (6000, 6145, 64, 0), (4200, 4099, 128, 0), (1100, 4098, 736, 0),
+                                        (1290, 6144, 512, 1), (2900, 3071, 96, 1), (6000, 3071, 64, 1)])
+def test_products_that_take_pairs(ops, M, N, K, dual):
+    from umbrella_b200 import _lib_seq as S
+    assert _kernel(torch.bfloat16, M, N, K, dual=dual) == S.UMBS_GEMM_PAIRS
+    assert _kernel(torch.bfloat16, 100, N, K, dual=dual) != S.UMBS_GEMM_PAIRS
+    a, w = _mat(116, M, K), _mat(117, N * (1 + dual), K, scale=K ** -0.5)
+    bias = torch.randn(w.shape[0], device=DEV)
+    run = lambda x, f32: ops.gemm_ex(x, w, act=S.UMBS_ACT_SILU if dual else 0, bias=bias, out_f32=f32)
+    ref = a.double() @ w.double().T + bias.double()
+    if dual:
+        ref = torch.nn.functional.silu(ref[:, :N]) * ref[:, N:]
+    got = run(a, True)
+    assert H.rel_err(got, ref.cpu()) < F32_TOL
+    assert H.rel_err(run(a, False), ref.cpu()) < BF16_TOL
+    assert torch.equal(run(a[-100:].contiguous(), True), got[-100:])                              # (single blocks)
+
+
+@pytest.mark.parametrize("M,heads,n,k", [(700, 5, 520, 128), (1290, 3, 1550, 1056)])             # single blocks, pairs
+@pytest.mark.parametrize("gap", [0, 1])
+def test_pairs_of_blocks_over_heads(ops, M, heads, n, k, gap):
+    from umbrella_b200 import _lib_seq as S
+    assert (_kernel(torch.bfloat16, M, n, k, groups=heads) == S.UMBS_GEMM_PAIRS) == (M == 1290)
     a, w = _mat(114, M, heads * k), _mat(115, heads, n, k)
-    ref = torch.einsum("mhk,hnk->mhn", a.double().view(M, heads, k), w.double()).reshape(M, heads * n)
-    assert H.rel_err(ops.gemm(a, w, out_f32=True, groups=heads, a_goff=k, c_goff=n), ref.cpu()) < F32_TOL
+    ref = torch.einsum("mhk,hnk->mhn", a.double().view(M, heads, k), w.double())
+    got = ops.gemm(a, w, out_f32=True, groups=heads, a_goff=k, c_goff=n + gap).view(M, heads, n + gap)
+    assert H.rel_err(got[..., :n], ref.cpu()) < F32_TOL
+    assert bool((got[..., n:] == 0).all())

@@ -21,6 +21,7 @@ UMBS_MIX_GATED_DELTA, UMBS_MIX_SSD = 5, 6
 UMBS_MEMORY_ADD, UMBS_MEMORY_DELTA = 0, 1
 UMBS_FORM_PARALLEL, UMBS_FORM_PRENORM = 0, 1
 UMBS_ACT_CLAMPED_GLU, UMBS_ACT_GELU_TANH, UMBS_ACT_SILU = 1, 2, 3
+UMBS_GEMM_GENERAL, UMBS_GEMM_FEW_ROWS, UMBS_GEMM_SPLIT, UMBS_GEMM_PAIRS = 0, 1, 2, 512
 UMBS_NORM_RMS, UMBS_NORM_LAYER, UMBS_NORM_DYT = 0, 1, 2
 UMBS_UNARY_TANH, UMBS_UNARY_XIELU, UMBS_UNARY_RELU2, UMBS_UNARY_SILU, UMBS_UNARY_SCALE = 1, 2, 3, 4, 5
 UMBS_GATE_SILU, UMBS_GATE_SIGMOID = 0, 1
@@ -134,6 +135,7 @@ SIGNATURES = {
     "umbs_forward": (c_int, [C.POINTER(Model), _BP, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
     "umbs_gemm": (c_int, [c_int, c_void_p, c_int64, c_int, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int, c_int,
                           c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_float, c_void_p]),
+    "umbs_gemm_kernel": (c_int, [c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int]),
     "umbs_gemm_sorted": (c_int, [c_int, c_void_p, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int, c_int, c_int, c_int,
                                  c_int, c_int, c_void_p, c_void_p, c_int, c_float, c_void_p]),
     "umbs_gemm_ex": (c_int, [c_int, c_void_p, c_int64, c_int, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int, c_int,

@@ -534,6 +534,23 @@ extern "C" int umbs_gemm_head_gate(int dtype, const void* A, int64_t lda, int a_
                     out_gate, ld_gate, 1, 0, 0, 0.f, 0.f, 0, stream);
 }
 
+constexpr int kFewRows = 16;
+// Streamed fp32 rows take 2 us and one for 6.5 million products, tiles on the tensor core 6 us and 1.3 for each 64 of k.  (us, multiply-add
+// tiles / streamed / tensor core, K = 1024: one row of 3088 columns 54 / 4.6 / 29, 64 rows of 1024 45 / 12 / 25, of 3088 51 / 32 / 28, of
+// 8192 73 / 78 / 31; 200 rows of 3088 85 / - / 32; 128 rows, K = 4096, to 1024 columns 184 / 60 / 90.)
+// (the streamed rows are the grid's second extent)
+static bool f32_streams(int M, int64_t w_rows, int K, int groups) {
+    return M <= 4096 && (M <= kFewRows || (double)M * w_rows * groups * K <= 8.5e6 * (K / 64 + 4));
+}
+
+extern "C" int umbs_gemm_kernel(int dtype, int M, int N, int K, int groups, int sorted, int dual, int sms) {
+    if (M <= 0 || N <= 0 || K <= 0 || groups <= 0 || sms <= 0) return UMB_ERR_ARG;
+    if (dtype == UMBS_F32) return K % 4 ? UMBS_GEMM_GENERAL : f32_streams(M, (int64_t)N * (dual ? 2 : 1), K, groups) ? UMBS_GEMM_FEW_ROWS : UMBS_GEMM_SPLIT;
+    if (dtype != UMBS_BF16) return UMB_ERR_ARG;
+    if (K % 8 == 0 && M <= kFewRows) return UMBS_GEMM_FEW_ROWS;
+    return K % 32 ? UMBS_GEMM_GENERAL : tc_tile_columns(M, N, K, groups, dual != 0, sorted != 0, sorted != 0, sms);
+}
+
 static int gemm_run(int dtype, const void* A, int64_t lda, int a_goff, const void* W, int64_t ldw, int64_t w_gstride,
                     void* C, int64_t ldc, int c_goff, int c_f32, int M, int N, int K, int groups,
                     const int32_t* grp_off, const int32_t* row_src, int dual, float limit, const float* bias,
@@ -556,13 +573,10 @@ static int gemm_run(int dtype, const void* A, int64_t lda, int a_goff, const voi
         if (const cudaError_t e = clear()) return (int)e;
         const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) && (a_goff % 4 == 0) && (w_gstride % 4 == 0) &&
                          ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
-        // Streamed rows take 2 us and one for 6.5 million products, tiles on the tensor core 6 us and 1.3 for each 64 of k.  (us, multiply-add
-        // tiles / streamed / tensor core, K = 1024: one row of 3088 columns 54 / 4.6 / 29, 64 rows of 1024 45 / 12 / 25, of 3088 51 / 32 / 28, of
-        // 8192 73 / 78 / 31; 200 rows of 3088 85 / - / 32; 128 rows, K = 4096, to 1024 columns 184 / 60 / 90.)
-        // (the tiles count rows in 16-byte pieces of 32 bits: strides forwards, 64 GB; the streamed rows are the grid's second extent)
+        // (the tiles count rows in 16-byte pieces of 32 bits: strides forwards, 64 GB)
         const int64_t w_rows = (int64_t)N * (dual ? 2 : 1);
         const bool split = vec && lda >= 0 && ldw >= 0 && lda <= UINT32_MAX / std::max(M, 1) && ldw <= UINT32_MAX / w_rows;
-        if (vec && M <= 4096 && (M <= 16 || (double)M * w_rows * groups * K <= 8.5e6 * (K / 64 + 4))) {
+        if (vec && f32_streams(M, w_rows, K, groups)) {
             launch_rows(a, groups, dual != 0, st);
         } else if (split) {
             const int rc = launch_gemm_split(a, groups, dual != 0, st);
@@ -576,7 +590,7 @@ static int gemm_run(int dtype, const void* A, int64_t lda, int a_goff, const voi
                          ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
         // (rows that overlap, one row repeated among them: not described by a tensor map, they take the general kernel)
         const bool tc = vec && (K % 32 == 0) && lda >= K && ldw >= K;
-        if (vec && M <= 16) {
+        if (vec && M <= kFewRows) {
             if (const cudaError_t e = clear()) return (int)e;
             if (c_f32) launch_skinny<float>(a, groups, dual != 0, st);
             else launch_skinny<__nv_bfloat16>(a, groups, dual != 0, st);

@@ -65,6 +65,7 @@ __device__ __forceinline__ float finish(const GemmArgs& a, float s, float s2, in
 
 // seq_gemm_tc.cu: bf16 operands, 16-byte rows (the caller has checked them)
 int launch_gemm_tc(const GemmArgs& a, int groups, bool dual, bool c_f32, cudaStream_t st);
+int tc_tile_columns(int M, int N, int K, int groups, bool dual, bool by_group, bool gathered, int sms);     // columns of its tiles, or UMBS_GEMM_PAIRS
 // seq_gemm_split.cu: fp32 operands, 16-byte rows, K a multiple of 4 (the caller has checked them)
 int launch_gemm_split(const GemmArgs& a, int groups, bool dual, cudaStream_t st);
 

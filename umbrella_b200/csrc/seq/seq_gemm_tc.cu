@@ -264,6 +264,31 @@ static int launch_tc_any(const GemmArgs& a, const TcArgs& t, bool dual, bool c_f
 #undef UMBS_TC
 }
 
+// The tile width with the shortest longest walk.  Dense rows, in ns: what a launch, a tile's first operands and its last results take,
+// and a k step of a round of tiles (measured, loaded chip; pairs of SMs: seq_gemm_pair.cu).  us, single blocks / pairs: 803 rows, K =
+// 1024, to 1024 / 3088 columns 8.6 / 12.1, 15.2 / 13.3; 1500, K = 2048, to 6144 34.9 / 31.0; 4096 90.0 / 80.1; 4096, K = 1024, to 4096
+// 41.8 / 34.1.
+// Rows sorted by expert (how they fall is only known on the device; spread evenly is the guess): rounds of tiles times what 16 of k
+// cost, the tensor core's 128 clocks for 256 columns and more than half, a quarter of that for 128 and 64: 72 and 52 (the activation
+// tile is fetched and read from shared memory for fewer products).
+int tc_tile_columns(int M, int N, int K, int groups, bool dual, bool by_group, bool gathered, int sms) {
+    const bool dense = !by_group && !gathered;
+    const int64_t m = by_group ? (int64_t)groups * ((M + groups * kTcRows - 1) / (groups * kTcRows)) : (int64_t)groups * ((M + kTcRows - 1) / kTcRows);
+    const int64_t steps = dense ? (K + kTcK - 1) / kTcK : 1;
+    auto cost = [&](int bn, int step, int once) {
+        const int out = dual ? bn / 2 : bn;
+        return (m * ((N + out - 1) / out) + sms - 1) / sms * steps * step + (dense ? once : 0);
+    };
+    const int64_t c256 = cost(256, dense ? 410 : 128, 8300), c128 = cost(128, dense ? 275 : 72, 6000), c64 = cost(64, dense ? 250 : 52, 4300);
+    if (dense && M > kTcRows) {
+        const int out = dual ? 128 : 256;
+        const int64_t tiles = (int64_t)groups * ((M + 255) / 256) * ((N + out - 1) / out), pair = (tiles + sms / 2 - 1) / (sms / 2) * steps * 370 + 6800;
+        if (pair < c256 && pair < c128 && pair < c64) return UMBS_GEMM_PAIRS;
+    }
+    if (c256 <= c128 && c256 <= c64) return 256;
+    return c128 <= c64 ? 128 : 64;
+}
+
 int launch_gemm_tc(const GemmArgs& a, int groups, bool dual, bool c_f32, cudaStream_t st) {
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -277,29 +302,12 @@ int launch_gemm_tc(const GemmArgs& a, int groups, bool dual, bool c_f32, cudaStr
     t.m_tiles = (a.M + kTcRows - 1) / kTcRows;
     const int es = c_f32 ? 4 : 2;
     t.vec_c = (uintptr_t)a.C % (4 * es) == 0 && a.ldc % 4 == 0 && a.c_goff % 4 == 0;
-    // The tile width with the shortest longest walk.  Dense rows, in ns: what a launch, a tile's first operands and its last results take,
-    // and a k step of a round of tiles (measured, loaded chip; pairs of SMs: seq_gemm_pair.cu).  us, single blocks / pairs: 803 rows, K =
-    // 1024, to 1024 / 3088 columns 8.6 / 12.1, 15.2 / 13.3; 1500, K = 2048, to 6144 34.9 / 31.0; 4096 90.0 / 80.1; 4096, K = 1024, to 4096
-    // 41.8 / 34.1.
-    // Rows sorted by expert (how they fall is only known on the device; spread evenly is the guess): rounds of tiles times what 16 of k
-    // cost, the tensor core's 128 clocks for 256 columns and more than half, a quarter of that for 128 and 64: 72 and 52 (the activation
-    // tile is fetched and read from shared memory for fewer products).
-    const bool dense = a.grp_off == nullptr && a.row_src == nullptr;
-    const int64_t m = a.grp_off != nullptr ? (int64_t)groups * ((a.M + groups * kTcRows - 1) / (groups * kTcRows)) : (int64_t)groups * t.m_tiles;
-    const int64_t steps = dense ? (a.K + kTcK - 1) / kTcK : 1;
-    auto cost = [&](int bn, int step, int once) {
-        const int out = dual ? bn / 2 : bn;
-        return (m * ((a.N + out - 1) / out) + sms - 1) / sms * steps * step + (dense ? once : 0);
-    };
-    const int64_t c256 = cost(256, dense ? 410 : 128, 8300), c128 = cost(128, dense ? 275 : 72, 6000), c64 = cost(64, dense ? 250 : 52, 4300);
-    if (dense && a.M > kTcRows) {
-        const int out = dual ? 128 : 256;
-        const int64_t tiles = (int64_t)groups * ((a.M + 255) / 256) * ((a.N + out - 1) / out), pair = (tiles + sms / 2 - 1) / (sms / 2) * steps * 370 + 6800;
-        if (pair < c256 && pair < c128 && pair < c64) return launch_gemm_pair(a, t, dual, c_f32, sms, st);
+    switch (tc_tile_columns(a.M, a.N, a.K, groups, dual, a.grp_off != nullptr, a.row_src != nullptr, sms)) {
+        case UMBS_GEMM_PAIRS: return launch_gemm_pair(a, t, dual, c_f32, sms, st);
+        case 256: return launch_tc_any<256>(a, t, dual, c_f32, sms, st);
+        case 128: return launch_tc_any<128>(a, t, dual, c_f32, sms, st);
+        default: return launch_tc_any<64>(a, t, dual, c_f32, sms, st);
     }
-    if (c256 <= c128 && c256 <= c64) return launch_tc_any<256>(a, t, dual, c_f32, sms, st);
-    if (c128 <= c64) return launch_tc_any<128>(a, t, dual, c_f32, sms, st);
-    return launch_tc_any<64>(a, t, dual, c_f32, sms, st);
 }
 
 }  // namespace umbs
