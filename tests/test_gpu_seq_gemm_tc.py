@@ -306,6 +306,24 @@ def test_sorted_rows_of_no_group_are_zero(ops, dt, K, max_rows):
         lo += n
 
 
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("K,max_rows", [(64, 200), (64, 16), (40, 200)])          # tensor-core tiles, few rows, neither
+@pytest.mark.parametrize("f32", [True, False])
+def test_sorted_rows_in_front_of_the_first_group_are_zero(ops, dt, K, max_rows, f32):
+    """A slice of the experts: the offsets begin behind rows of others."""
+    from umbrella_b200 import _lib_seq as S
+    off = torch.tensor([5, 9, 9, 22], dtype=torch.int32, device=DEV)
+    a, w = _mat(103, 30, K).to(dt), _mat(104, 3, 50, K).to(dt)
+    got = torch.full((30, 50), float("nan"), dtype=torch.float32 if f32 else dt, device=DEV)
+    S.check(S.load().umbs_gemm_sorted(ops._mode(a), a.data_ptr(), K, w.data_ptr(), K, 50 * K, got.data_ptr(), 50, int(f32), max_rows, 30, 50, K, 3,
+                                      off.data_ptr(), None, 0, 0.0, ops._stream()), "gemm")
+    assert bool((got[:5] == 0).all()) and bool((got[22:] == 0).all())
+    tol = F32_TOL if got.dtype == torch.float32 else BF16_TOL
+    for g, (lo, hi) in enumerate([(5, 9), (9, 9), (9, 22)]):
+        if hi > lo:
+            assert H.rel_err(got[lo:hi], (a[lo:hi].double() @ w[g].double().T).cpu()) < tol
+
+
 # pairs of SMs: tiles of 256 rows x 256 columns (gate|up: 128 of each), rows and columns that end in either half; groups
 @pytest.mark.parametrize("M,N,K", [(1000, 3100, 1056), (1537, 2049, 64), (4096, 1100, 96), (1290, 6144, 512)])
 def test_pairs_of_blocks(ops, M, N, K):

@@ -21,7 +21,7 @@ struct GemmArgs {
     int unary;        // UMBS_UNARY_* of a plain product's first unary_cols columns, with its two numbers
     float p0, p1;
     int unary_cols;
-    int rows_total;          // of C, rows sorted by group: those behind the last group's are set to zero (0: not asked for)
+    int rows_total;          // of C, rows sorted by group: those of no group are set to zero (0: not asked for)
     int weights_ready;       // W was there before the chain of launches began: it may be read ahead of chain_wait
 };
 

@@ -173,9 +173,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             unit = (unit + t.k_steps) % kStages;
         }
     }
-    if (!A_TMA && warp >= 2 && warp < 6 && a.rows_total > 0)               // rows of no group
-        for (int64_t r = a.grp_off[t.groups] + (int64_t)blockIdx.x * 4 + warp - 2; r < a.rows_total; r += (int64_t)gridDim.x * 4)
+    if (!A_TMA && warp >= 2 && warp < 6 && a.rows_total > 0) {             // rows of no group: in front of the first, behind the last
+        const int64_t lo = min(a.grp_off[0], a.rows_total), gap = a.grp_off[t.groups] - lo;
+        for (int64_t i = (int64_t)blockIdx.x * 4 + warp - 2; i < a.rows_total - gap; i += (int64_t)gridDim.x * 4) {
+            const int64_t r = i < lo ? i : i + gap;
             for (int n = lane; n < a.N; n += 32) ((TC*)a.C)[r * a.ldc + n] = from_f32<TC>(0.f);
+        }
+    }
     __syncthreads();
     tc_settle(quit, t.report);
     if (warp == 1) {
