@@ -135,3 +135,42 @@ def test_mlstm_against_float64(dim, vdim, n):
     out = K.mlstm(f32(proj), f32(bias), K.RaggedBatch([(0, n, 0, 0)], DEV), heads, dim, vdim, 10.0, 1e-5, f32(norm), state)
     ref = mlstm_reference(proj, bias, heads, dim, vdim, 10.0, 1e-5, norm)
     assert float((out.double().cpu() - ref.double()).abs().max() / ref.double().abs().max()) < 2e-5
+
+
+def _retention64(x, heads, dim, vdim, decay, S, eps):
+    """float64, token by token, no rotation, keys as they are; -> gated rows of unit norm, the state behind them"""
+    n, hd, hv = x.shape[0], heads * dim, heads * vdim
+    q, k, v, gate = x.double().split([hd, hd, hv, hv], 1)
+    q, k, v = q.view(n, heads, dim), k.view(n, heads, dim), v.view(n, heads, vdim)
+    S, out, d = S.double(), [], decay.double()[:, None, None]
+    for t in range(n):
+        S = d * S + k[t][:, :, None] * v[t][:, None, :]
+        out.append((q[t][:, :, None] * S).sum(1))
+    o = torch.stack(out)
+    o = o / torch.sqrt((o * o).mean(-1, keepdim=True) + eps)
+    return o.reshape(n, hv) * gate * torch.sigmoid(gate), S
+
+
+def _ratio(a, b):
+    return float((a.double() - b).norm() / b.norm())
+
+
+# Rows of ordinary size, and queries, keys and values times powers of two that leave the products where they were: numbers whose bf16 parts
+# would fall below bf16's smallest, scores beyond 2^79, a fresh and a carried state.  Tolerance: decays by powf (two units in the last
+# place), some 200 rounded products of random signs, the norm and the gate: 2e-6 is ten times what they add up to.
+@pytest.mark.parametrize("n,dim,vdim", [(128, 64, 128), (300, 64, 128), (131, 8, 72), (257, 40, 128)])
+@pytest.mark.parametrize("pos", [0, 37])
+@pytest.mark.parametrize("xq,xk,xv", [(0, 0, 0), (58, -118, 60), (-20, -100, 120), (60, 60, -120), (26, -126, 100)])
+def test_retention_in_pieces_of_128_against_float64(n, dim, vdim, pos, xq, xk, xv):
+    from umbrella_b200 import ops_seq as K
+    heads = 2
+    x = torch.randn(n, 2 * heads * (dim + vdim), generator=torch.Generator().manual_seed(n)).to(DEV)
+    hd = heads * dim
+    x[:, :hd] *= 2.0 ** xq
+    x[:, hd:2 * hd] *= 2.0 ** xk
+    x[:, 2 * hd:2 * hd + heads * vdim] *= 2.0 ** xv
+    decay = torch.tensor([0.93, 0.9995], device=DEV)
+    state = torch.randn(1, heads, dim, vdim, generator=torch.Generator().manual_seed(1)).to(DEV) * 2.0 ** (xk + xv)
+    want, S = _retention64(x, heads, dim, vdim, decay, state[0] * (pos > 0), 1e-6)
+    got = K.retention(x, K.RaggedBatch([(0, n, pos, 0)], DEV), heads, dim, vdim, 0, torch.zeros(1, device=DEV), decay, 1e-6, state, k_scale=1.0)
+    assert _ratio(got, want) < 2e-6 and _ratio(state[0], S) < 2e-6

@@ -265,6 +265,18 @@ def test_split_products_of_wider_rows_and_of_groups(ops):
     assert bool((got.view(M, heads, n + 1)[..., n] == 0).all())
 
 
+# Operands that three bf16 parts in fp32's own scale do not hold (below 2^-110), beside partners that lift the results back into range, on either
+# side; results near and in the subnormal range: one rounding more, 2^-150 for an element.
+@pytest.mark.parametrize("x,y", [(-118, 40), (-124, 60), (-126, 100), (-140, 110), (60, -118), (110, -140), (-60, -66), (-74, -66)])
+def test_split_products_of_small_numbers_beside_large_ones(ops, x, y):
+    from umbrella_b200 import _lib_seq as S
+    M, N, K = 400, 4000, 64
+    assert _kernel(torch.float32, M, N, K) == S.UMBS_GEMM_SPLIT
+    a, w = _mat32(97, M, K) * 2.0 ** x, _mat32(98, N, K) * 2.0 ** y
+    got, ref = ops.gemm(a, w).double(), a.double() @ w.double().T
+    assert float((got - ref).norm() / ref.norm()) < F32_SPLIT_TOL + 2.0 ** -150 * (M * N) ** 0.5 / float(ref.norm())
+
+
 @pytest.mark.parametrize("M,N", [(200, 2000), (400, 4000)])          # streamed, tiles
 def test_split_products_of_numbers_at_the_ends_of_the_range(ops, M, N):
     """Infinite and NaN operands, numbers that round to infinity in bf16, and rows so small that their low parts vanish there."""

@@ -5,7 +5,7 @@
 //     outputs  O = diag(decay^(i + 1)) Q S + ((Q K^T) o D) V            a block as for the states; then the head's norm and gate
 // Every operand is 32-bit and taken as three bf16 parts in six products (seq_gemm_split.cu); a product's leading part is summed over at
 // most 128 of k and apart from the small ones, so no chain through the tensor core is longer than eight.  Sums whose parts are no
-// numbers (infinite or NaN operands, or beyond bf16) are worked out again in plain fp32.
+// numbers (operands infinite, NaN or beyond 2^103; sums beyond 2^79) are worked out again in plain fp32.
 //
 // Bound: what a block does one after the other (rows in, split, products, weights split again, products, out), four warps a scheduler
 // in step: outputs 33,000 clocks a block, of which the products take 6,000, three and a half blocks to an SM (192 KB of shared memory
@@ -75,9 +75,10 @@ __device__ __forceinline__ float turned(const ChunkMemory& x, int64_t tok, int o
     for (int e = 1; e < 8; ++e) r = (d & 7) == e ? f[e] : r;
     return r;
 }
+template <bool SCALED = false>
 __device__ __forceinline__ void st_parts(uint32_t at, uint32_t step, const float (&f)[8]) {
     uint4 v[3];
-    split8(f, v);
+    split8<SCALED>(f, v);
 #pragma unroll
     for (int e = 0; e < 3; ++e)
         asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(at + e * step), "r"(v[e].x), "r"(v[e].y), "r"(v[e].z), "r"(v[e].w) : "memory");
@@ -164,14 +165,16 @@ __global__ void __launch_bounds__(256, 3) chunk_states_kernel(const __grid_const
             turn_row(x, ch, kf[p], cf[p], sf[p]);
             const float w = keep[half * 64 + r];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) kf[p][e] = w == 0.f ? 0.f : kf[p][e] * x.kscale * w;     // (tokens that are not there, or forgotten: nothing)
-            st_parts(s_k + r * 128 + ((ch ^ (r & 7)) << 4), 8192, kf[p]);
+            for (int e = 0; e < 8; ++e) kf[p][e] = w == 0.f ? 0.f : kf[p][e] * (x.kscale * kSplitScale) * w;     // (tokens that are not there, or forgotten: nothing)
+            st_parts<true>(s_k + r * 128 + ((ch ^ (r & 7)) << 4), 8192, kf[p]);
         }
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
             const int r = r16 + 16 * p;
             float f[8] = {};
             if (half * 64 + r < nb && cv * 8 < nv) ld8(x.x + (tok + half * 64 + r) * x.ld + x.voff + h * x.vdim + c0 + cv * 8, f);
+            // (the loads stay apart from the multiplications, which the compiler otherwise waits for load by load: 29.8 -> 25.7 us)
+            asm volatile("" : "+f"(f[0]), "+f"(f[1]), "+f"(f[2]), "+f"(f[3]), "+f"(f[4]), "+f"(f[5]), "+f"(f[6]), "+f"(f[7]));
             st_parts(s_v + (cv >> 3) * 8192 + r * 128 + (((cv & 7) ^ (r & 7)) << 4), 16384, f);
         }
         umb::fence_proxy_async_smem();
@@ -209,7 +212,7 @@ __global__ void __launch_bounds__(256, 3) chunk_states_kernel(const __grid_const
 #pragma unroll
             for (int i = 0; i < 32; ++i)
                 if (d0 + i < x.dim) {
-                    const float l = __uint_as_float(u[i]) + __uint_as_float(v[i]);
+                    const float l = (__uint_as_float(u[i]) + __uint_as_float(v[i])) * kSplitBack;
                     odd |= (uint32_t)no_number(l) << i;
                     out[(int64_t)(d0 + i) * x.vdim] = l;
                 }
@@ -311,11 +314,11 @@ __global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_cons
             turn_row(x, ch, kf[p], cf[p], sf[p]);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                qf[p][e] *= x.qscale;
-                kf[p][e] *= x.kscale;
+                qf[p][e] *= x.qscale * kSplitScale;
+                kf[p][e] *= x.kscale * kSplitScale;
             }
-            st_parts(s_q + at, 16384, qf[p]);
-            st_parts(s_k + at, 16384, kf[p]);
+            st_parts<true>(s_q + at, 16384, qf[p]);
+            st_parts<true>(s_k + at, 16384, kf[p]);
         }
     }
     // values and state, while the scores are worked out
@@ -360,7 +363,7 @@ __global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_cons
         bool bad = false;
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            const bool no = !(fabsf(vf[p][e]) <= 0x1.fep127f);
+            const bool no = !(fabsf(vf[p][e]) <= 0x1.fep103f);
             bad |= no;
             vf[p][e] = no ? 0.f : vf[p][e];
         }
@@ -409,7 +412,7 @@ __global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_cons
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
                 const int far = i - (part + 2 * e + k);
-                const float z = __uint_as_float(u[2 * e + k]) + __uint_as_float(v[2 * e + k]);
+                const float z = (__uint_as_float(u[2 * e + k]) + __uint_as_float(v[2 * e + k])) * (kSplitBack * kSplitScale);    // (as split8: 2^24)
                 p[k] = far >= 0 ? z * lam[far >= 0 ? far : 0] : 0.f;        // (chosen: a later token's NaN stays its own)
             }
             uint32_t* to[3] = {&w0[e], &w1[e], &w2[e]};
@@ -436,7 +439,7 @@ __global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_cons
         umb::tc_wait_ld();
         const float f = lam[i + 1];
 #pragma unroll
-        for (int e = 0; e < 32; ++e) o[e] = f * (__uint_as_float(u[e]) + __uint_as_float(v[e]));
+        for (int e = 0; e < 32; ++e) o[e] = f * ((__uint_as_float(u[e]) + __uint_as_float(v[e])) * kSplitBack);
         umb::tc_fence_before();
         __syncthreads();
         if (warp == 0) {
@@ -467,13 +470,16 @@ __global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_cons
         uint32_t odd = 0;
 #pragma unroll
         for (int e = 0; e < 32; ++e) {
-            o[e] += __uint_as_float(u[e]) + __uint_as_float(v[e]);
-            odd |= (uint32_t)((i >= s_bad || no_number(o[e])) && i < nb && part + e < nv) << e;
+            o[e] += (__uint_as_float(u[e]) + __uint_as_float(v[e])) * kSplitBack;
+            odd |= (uint32_t)((i >= s_bad || no_number(o[e])) && i < nb) << e;
         }
         if (odd) {
-            float f[32];
+            float f[32];                                    // (columns that are not there: 0 times a score beyond the parts is none)
 #pragma unroll
-            for (int e = 0; e < 32; ++e) f[e] = o[e];
+            for (int e = 0; e < 32; ++e) {
+                f[e] = part + e < nv ? o[e] : 0.f;
+                odd &= ~((uint32_t)(part + e >= nv) << e);
+            }
             plain_outputs(x, tok, i, h, n0, dec, st, odd, f);
 #pragma unroll
             for (int e = 0; e < 32; ++e) o[e] = f[e];
@@ -495,7 +501,8 @@ __global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_cons
         float4 f[8];
         float inv = 1.f;
 #pragma unroll
-        for (int r = 0; r < 8; ++r) f[r] = *reinterpret_cast<const float4*>(so + (warp * 8 + r) * kCtStride + lane * 4);     // (columns that are not there: 0)
+        for (int r = 0; r < 8; ++r)                         // (columns that are not there: 0, and NaN beside a score beyond the parts)
+            f[r] = lane * 4 < nv ? *reinterpret_cast<const float4*>(so + (warp * 8 + r) * kCtStride + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
         if (NORM) {                                         // o / rms(o) over the head, times silu(g): lane r has row r's factor
             float ss = 0.f;
 #pragma unroll

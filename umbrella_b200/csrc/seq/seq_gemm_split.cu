@@ -1,8 +1,9 @@
 // Products of 32-bit operands with more than a few rows on the 5th-generation tensor cores: C = A W^T, fp32 in, fp32 out.
 //
-// An fp32 number is the sum of three bf16 numbers, rounded to nearest one after the other (8 significant bits each, the parts behind
-// the first signed): a = a0 + a1 + a2, exactly.  Products of bf16 numbers are exact in the tensor core, so
-//     a w = a0 w0 + (a0 w1 + a1 w0 + a1 w1 + a0 w2 + a2 w0) + terms below 2^-26 of it.
+// An fp32 number times 2^24 (so that no part falls below bf16's smallest number) is the sum of three bf16 numbers, rounded to nearest one
+// after the other (8 significant bits each, the parts behind the first signed): 2^24 a = a0 + a1 + a2, exactly.  Products of bf16 numbers
+// are exact in the tensor core, so
+//     2^48 a w = a0 w0 + (a0 w1 + a1 w0 + a1 w1 + a0 w2 + a2 w0) + terms below 2^-26 of it.
 // The tensor core cuts its running sums off where an fp32 addition rounds, so no long chain runs through it: a0 w0 is summed over
 // 128 of k at a time, in two accumulators in turn, and these sums are added in fp32 registers; the small terms, 2^-8 of the result, have
 // an accumulator of their own.  Distance from float64 at K = 64 / 512 / 1024 / 4096: 0.7 / 1.3 / 1.3 / 1.7e-7, where one chain of fp32
@@ -14,7 +15,7 @@
 // terms', 3 BN of 512 columns.
 //
 // Bound: the splitting: 9 rows of 8 numbers a thread and step, and a step's loads, which nothing covers (2.6 us a step of 64 k at
-// BN = 160, of which the products take 1.2).  777 rows of 1024 to 3088 columns: 177 us on the multiply-add pipe (its own time 66), 48 here; 64 rows
+// BN = 160, of which the products take 1.2).  777 rows of 1024 to 3088 columns: 177 us on the multiply-add pipe (its own time 66), 47 here; 64 rows
 // 50 -> 28.  What the first forms cost: products issued by a splitting warp 100 us, activations unrolled into the kernel 77.
 #include <algorithm>
 
@@ -27,12 +28,11 @@ constexpr int kSpThreads = 32 * (kSpConv + kSpSum + 1);
 constexpr int kSpSmem = 1024 + kSpStages * 3 * (kTcRows + kSpMaxN) * 128;
 constexpr int kSpChunk = 2;                                 // k steps whose a0 w0 the tensor core sums
 
-__device__ __forceinline__ bool odd_sum(float s) { return !(fabsf(s) <= 3.402823466e38f) || (s != 0.f && fabsf(s) < 0x1p-90f); }
+__device__ __forceinline__ bool odd_sum(float s) { return !(fabsf(s) <= 3.402823466e38f); }
 
 // What 16 neighbouring sums of a row become, in place (DUAL: u the up half).  Sums that the parts do not give are worked out again in
-// plain fp32: operands that are not finite or do not fit bf16's range (a part is infinite then, the next NaN), and results so small that
-// parts of their operands were rounded below bf16's smallest number.  Out of line: unrolled into the kernel, its 80 copies were
-// fetched from memory by every block, 40 us of a 77 us product.
+// plain fp32: of operands that are not finite or beyond 2^103 (a part is infinite then, the next NaN), and beyond 2^79 (2^127 in the scale of
+// the parts).  Out of line: unrolled into the kernel, its 80 copies were fetched from memory by every block, 40 us of a 77 us product.
 template <bool DUAL>
 __device__ __noinline__ void finish_chunk(const GemmArgs& a, int g, int64_t row, int n0, float* v, float* u) {
     const float* A = (const float*)a.A + (int64_t)g * a.a_goff + (int64_t)(a.row_src ? a.row_src[row] : row) * a.lda;
@@ -130,6 +130,10 @@ __global__ void __launch_bounds__(kSpThreads, 1) gemm_split_kernel(const __grid_
             if (!ok) break;
             add(2 * bn);                                                   // (the last chunk's barrier stands behind the small terms too)
             if (lane == 0) umb::mbar_arrive(low_empty);
+#pragma unroll
+            for (int c = 0; c < kSpMaxN / 32; ++c)
+#pragma unroll
+                for (int j = 0; j < 16; ++j) acc[c][j] *= kSplitBack;
             const int r = w.m0 + q * 32 + lane;
             if (r < w.rows) {
                 const int64_t grow = w.row_lo + r;

@@ -75,12 +75,17 @@ __device__ __forceinline__ float tc_sigmoid(float z) {
     const float x = 1.f + expf(-z), r = __fdividef(1.f, x);
     return x >= 0x1p126f ? 0.f : fmaf(r, fmaf(-x, r, 1.f), r);
 }
-// eight fp32 numbers as three rows of eight bf16, rounded to nearest one after the other: their sum, exactly, where all are finite
+// Eight fp32 numbers times 2^24 (SCALED: they are that already) as three rows of eight bf16, rounded to nearest one after the other: their sum, exactly, for all numbers up
+// to 2^103.  (bf16 has fp32's range, so the parts of an fp32 number below 2^-110 would end below bf16's smallest, 2^-133; scaled,
+// the lowest bit of the smallest subnormal is 2^-125, a normal number.)  Numbers beyond are infinite or NaN in their parts, and so are the sums
+// they enter.  A product of two such operands is 2^48 times the operands': kSplitBack takes it back, exactly where the result is normal.
+constexpr float kSplitScale = 0x1p24f, kSplitBack = 0x1p-48f;
+template <bool SCALED = false>
 __device__ __forceinline__ void split8(const float (&f)[8], uint4 (&p)[3]) {
     uint32_t* o[3] = {&p[0].x, &p[1].x, &p[2].x};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        float a = f[2 * i], b = f[2 * i + 1];
+        float a = SCALED ? f[2 * i] : f[2 * i] * kSplitScale, b = SCALED ? f[2 * i + 1] : f[2 * i + 1] * kSplitScale;
 #pragma unroll
         for (int e = 0; e < 3; ++e) {
             const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
