@@ -174,3 +174,15 @@ def test_retention_in_pieces_of_128_against_float64(n, dim, vdim, pos, xq, xk, x
     want, S = _retention64(x, heads, dim, vdim, decay, state[0] * (pos > 0), 1e-6)
     got = K.retention(x, K.RaggedBatch([(0, n, pos, 0)], DEV), heads, dim, vdim, 0, torch.zeros(1, device=DEV), decay, 1e-6, state, k_scale=1.0)
     assert _ratio(got, want) < 2e-6 and _ratio(state[0], S) < 2e-6
+
+
+def test_gates_of_pieces_of_128_over_their_range():
+    """Row by row, from gates whose silu is near the smallest normal number (there 1 + e^-g is beyond 2^126) up to ordinary ones.  Tolerance as above."""
+    from umbrella_b200 import ops_seq as K
+    n, heads, dim, vdim = 130, 2, 64, 128
+    x = torch.randn(n, 2 * heads * (dim + vdim), generator=torch.Generator().manual_seed(2)).to(DEV)
+    x[:, -heads * vdim:] = torch.linspace(-88.5, 3.0, n, device=DEV)[:, None]
+    decay, state = torch.tensor([0.93, 0.9995], device=DEV), torch.zeros(1, heads, dim, vdim, device=DEV)
+    want, _ = _retention64(x, heads, dim, vdim, decay, state[0], 1e-6)
+    got = K.retention(x, K.RaggedBatch([(0, n, 0, 0)], DEV), heads, dim, vdim, 0, torch.zeros(1, device=DEV), decay, 1e-6, state, k_scale=1.0).double()
+    assert float(((got - want).norm(dim=1) / want.norm(dim=1)).max()) < 2e-6

@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_cons
             if (NORM) {
                 const float by = __shfl_sync(0xffffffffu, inv, r), ga[4] = {gv[r].x, gv[r].y, gv[r].z, gv[r].w};
 #pragma unroll
-                for (int k = 0; k < 4; ++k) z[k] = z[k] * by * (ga[k] * tc_sigmoid(ga[k]));
+                for (int k = 0; k < 4; ++k) z[k] = z[k] * by * (ga[k] / (1.f + expf(-ga[k])));         // (retention_gate_kernel's)
             }
             if (lane * 4 >= nv) continue;
             T* to = orow + (int64_t)r * hv;
