@@ -1,4 +1,6 @@
 """What the tensor-level calls and the model do around the native library, on the CPU with a library that only records."""
+import ctypes as C
+
 import pytest
 import torch
 
@@ -55,3 +57,19 @@ def test_a_give_up_is_raised_before_anything_is_made_of_the_results(monkeypatch)
         model.forward([])
     with pytest.raises(RuntimeError, match="gave up"):
         S.check(-5, "forward")
+
+
+# ---------------------------------------------------------------------------------------------- what the library refuses
+@pytest.mark.skipif(torch.cuda.is_available(), reason="memory of the host: only where no kernel could follow")
+@pytest.mark.parametrize("tokens", [1, 40, 128])
+@pytest.mark.parametrize("dtype", [-1, 2, 7])
+def test_retention_refuses_types_that_it_does_not_have(tokens, dtype):
+    """Before anything is launched, whichever kernels the step's length would take."""
+    heads, dim, vdim = 1, 8, 8
+    batch = S.Batch()
+    batch.n_tokens, batch.n_seqs, batch.max_seq_len = tokens, 1, tokens
+    keep = [torch.zeros(tokens * 64) for _ in range(6)]
+    p = [t.data_ptr() for t in keep]
+    got = S.load().umbs_retention_ex(dtype, p[0], 2 * heads * (dim + vdim), C.byref(batch), heads, dim, vdim, 0, None, p[1], 1e-6, p[2], p[3], None, p[4],
+                                     tokens * 256, None, p[5], None)
+    assert got == -1                                                 # UMB_ERR_ARG

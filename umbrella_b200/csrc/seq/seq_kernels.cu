@@ -1095,7 +1095,7 @@ extern "C" int umbs_retention_ex(int dtype, const float* qkvg, int64_t ld, const
                                  const umbs_retention_opts_t* opts, void* out, umbs_stream_t stream) {
     if (batch->n_tokens <= 0) return 0;
     const float kscale = (opts != nullptr && opts->k_scale != 0.f) ? opts->k_scale : 1.f / sqrtf((float)dim);
-    if (rot_dims < 0 || rot_dims > dim || (rot_dims & 1)) return UMB_ERR_ARG;
+    if (rot_dims < 0 || rot_dims > dim || (rot_dims & 1) || (dtype != UMBS_BF16 && dtype != UMBS_F32)) return UMB_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     unsigned launches = 2;
     auto gate = [&](unsigned launches) -> int {
