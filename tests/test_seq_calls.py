@@ -73,3 +73,25 @@ def test_retention_refuses_types_that_it_does_not_have(tokens, dtype):
     got = S.load().umbs_retention_ex(dtype, p[0], 2 * heads * (dim + vdim), C.byref(batch), heads, dim, vdim, 0, None, p[1], 1e-6, p[2], p[3], None, p[4],
                                      tokens * 256, None, p[5], None)
     assert got == -1                                                 # UMB_ERR_ARG
+
+
+# ---------------------------------------------------------------------------------------------- kernels that follow one another
+def test_tensor_memory_is_taken_before_the_next_kernel_is_let_in():
+    """A product of the next launch takes its tensor memory ahead of its wait: beside a block that has let it in and has none itself, neither
+    would ever go on.  So in every kernel the allocation stands in front of what lets the next one in."""
+    import glob
+    import os
+    import re
+    seen = 0
+    for path in glob.glob(os.path.join(os.path.dirname(S.__file__), "csrc", "seq", "*.cu")):
+        text = re.sub(r"//[^\n]*", "", open(path).read())
+        for body in text.split("__global__")[1:]:
+            body = body[:re.search(r"^}", body, re.M).end()]
+            alloc = re.search(r"tmem_alloc\(|tcgen05\.alloc", body)
+            let_in = re.search(r"chain_wait\(\)|chain_next\(\)", body)
+            if alloc and let_in:
+                seen += 1
+                assert alloc.start() < let_in.start(), (path, body[:120])
+            if alloc and "chain_wait_only()" in body:
+                assert let_in, path
+    assert seen >= 5

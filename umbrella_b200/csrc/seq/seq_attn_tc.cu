@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
     uint64_t *k_full = bars, *v_full = bars + kTaStages, *k_empty = bars + 2 * kTaStages, *v_empty = bars + 3 * kTaStages,
              *s_full = bars + 4 * kTaStages, *p_full = s_full + 2, *o_full = s_full + 3;
     volatile int* quit = &s_quit;
-    chain_wait();
+    chain_wait_only();
     const int s = blockIdx.z, vh = blockIdx.y, q0 = (int)(gridDim.x - 1 - blockIdx.x) * kTaQ;     // the rows that see most start first
     const int len = b.seq_len[s], start = b.seq_start[s], pos0 = STEP ? 0 : b.seq_pos0[s], slot = STEP ? 0 : b.seq_slot[s];
     if (q0 >= len) return;
@@ -144,6 +144,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
     if (warp == 4) {
         umb::tmem_alloc(&s_tmem, 256);
         umb::tmem_relinquish();
+        chain_next();
     }
     umb::tc_fence_before();
     __syncthreads();

@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(256, 3) chunk_states_kernel(const __grid_const
     __shared__ float keep[kCtT];
     volatile int* quit = &s_quit;
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    chain_wait();
+    chain_wait_only();
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int s = blockIdx.x / x.n_seg, c = blockIdx.x - s * x.n_seg, h = blockIdx.y, c0 = blockIdx.z * 128;
     const int t0 = c * kCtT, nb = min(kCtT, b.seq_len[s] - t0);
@@ -140,6 +140,7 @@ __global__ void __launch_bounds__(256, 3) chunk_states_kernel(const __grid_const
     if (warp == 0) {
         umb::tmem_alloc(&s_tmem, 128);
         umb::tmem_relinquish();
+        chain_next();
     }
     umb::tc_fence_before();
     __syncthreads();
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_cons
     __shared__ float lam[kCtT + 1];
     volatile int* quit = &s_quit;
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    chain_wait();
+    chain_wait_only();
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int s = blockIdx.x / x.n_seg, c = blockIdx.x - s * x.n_seg, h = blockIdx.y, c0 = blockIdx.z * 128;
     const int t0 = c * kCtT, nb = min(kCtT, b.seq_len[s] - t0);
@@ -291,6 +292,7 @@ __global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_cons
     if (warp == 0) {
         umb::tmem_alloc(&s_tmem, 512);
         umb::tmem_relinquish();
+        chain_next();
     }
     const uint32_t s_q = smem_u32(smem), s_k = s_q + 3 * 16384, s_v = s_k + 3 * 16384;
     const int ch = tid & 7, r8 = tid >> 3, cv = tid & 15, r16 = tid >> 4;

@@ -80,8 +80,14 @@ template <typename... P, typename... A>
 int chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
     return chain_launch_if(true, kernel, grid, block, smem, st, std::forward<A>(args)...);
 }
+// The two halves of it, apart in a kernel that takes tensor memory behind the wait: it lets the next one in when it has it (any thread's
+// chain_next counts for its block).  The products take theirs ahead of their wait: one brought onto an SM beside a block that has none yet
+// could hold all of it, and each would wait for the other for good.
+__device__ __forceinline__ void chain_wait_only() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() {
-    asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+    chain_wait_only();
+    chain_next();
 }
 
 // seq_gemm_tc.cu: a word of host memory that the kernels can write, set by a block that gave up.  Every call that launches such
