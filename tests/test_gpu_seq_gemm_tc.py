@@ -277,6 +277,21 @@ def test_split_products_of_small_numbers_beside_large_ones(ops, x, y):
     assert float((got - ref).norm() / ref.norm()) < F32_SPLIT_TOL + 2.0 ** -150 * (M * N) ** 0.5 / float(ref.norm())
 
 
+def test_split_products_of_rows_far_apart(ops):
+    """Gathered rows up to 64 GiB behind the first, where offsets of 32 bits in 16-byte pieces end."""
+    from umbrella_b200 import _lib_seq as S
+    ld, M, N, K = 2 ** 26, 60, 5000, 256
+    if torch.cuda.mem_get_info()[0] < 80 << 30:
+        pytest.skip("65 GiB of memory")
+    assert _kernel(torch.float32, M, N, K) == S.UMBS_GEMM_SPLIT
+    a, w, src = torch.empty(257 * ld, device=DEV).as_strided((257, K), (ld, 1)), _mat32(99, 1, N, K), torch.arange(256, 256 - 4 * M, -4, dtype=torch.int32, device=DEV)
+    a.copy_(_mat32(100, 257, K))
+    got = ops.gemm(a, w, grp_off=torch.tensor([0, M], dtype=torch.int32, device=DEV), row_src=src, rows=M, max_rows=M)
+    assert H.rel_err(got, (a[src.long()].double() @ w[0].double().T).cpu()) < F32_SPLIT_TOL
+    del a
+    torch.cuda.empty_cache()
+
+
 @pytest.mark.parametrize("M,N", [(200, 2000), (400, 4000)])          # streamed, tiles
 def test_split_products_of_numbers_at_the_ends_of_the_range(ops, M, N):
     """Infinite and NaN operands, numbers that round to infinity in bf16, and rows so small that their low parts vanish there."""

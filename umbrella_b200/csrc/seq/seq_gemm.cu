@@ -573,7 +573,7 @@ static int gemm_run(int dtype, const void* A, int64_t lda, int a_goff, const voi
         if (const cudaError_t e = clear()) return (int)e;
         const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) && (a_goff % 4 == 0) && (w_gstride % 4 == 0) &&
                          ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
-        // (the tiles count rows in 16-byte pieces of 32 bits: strides forwards, 64 GB)
+        // (the tiles count rows in 16-byte pieces of 32 bits: strides forwards, 16 GB of dense rows and of weights)
         const int64_t w_rows = (int64_t)N * (dual ? 2 : 1);
         const bool split = vec && lda >= 0 && ldw >= 0 && lda <= UINT32_MAX / std::max(M, 1) && ldw <= UINT32_MAX / w_rows;
         if (vec && f32_streams(M, w_rows, K, groups)) {

@@ -18,6 +18,7 @@
 // BN = 160, of which the products take 1.2).  777 rows of 1024 to 3088 columns: 177 us on the multiply-add pipe (its own time 66), 47 here; 64 rows
 // 50 -> 28.  What the first forms cost: products issued by a splitting warp 100 us, activations unrolled into the kernel 77.
 #include <algorithm>
+#include <math.h>
 
 #include "seq_gemm_walk.cuh"
 
@@ -28,10 +29,18 @@ constexpr int kSpThreads = 32 * (kSpConv + kSpSum + 1);
 constexpr int kSpSmem = 1024 + kSpStages * 3 * (kTcRows + kSpMaxN) * 128;
 constexpr int kSpChunk = 2;                                 // k steps whose a0 w0 the tensor core sums
 
+// Where row r of the activations starts, in 16-byte pieces.  Rows that are gathered or follow other groups' may lie 64 GB and more behind A: the
+// sums are told to work those out in plain fp32.
+constexpr uint32_t kNoRow = 0xffffffffu;
+__device__ __forceinline__ uint32_t piece(const GemmArgs& a, int64_t r) {
+    const int64_t p = (a.row_src ? a.row_src[r] : r) * a.lda >> 2;
+    return p < kNoRow ? (uint32_t)p : kNoRow;
+}
+
 __device__ __forceinline__ bool odd_sum(float s) { return !(fabsf(s) <= 3.402823466e38f); }
 
 // What 16 neighbouring sums of a row become, in place (DUAL: u the up half).  Sums that the parts do not give are worked out again in
-// plain fp32: of operands that are not finite or beyond 2^103 (a part is infinite then, the next NaN), and beyond 2^79 (2^127 in the scale of
+// plain fp32: of rows that piece() does not reach, of operands that are not finite or beyond 2^103 (a part is infinite then, the next NaN), and beyond 2^79 (2^127 in the scale of
 // the parts).  Out of line: unrolled into the kernel, its 80 copies were fetched from memory by every block, 40 us of a 77 us product.
 template <bool DUAL>
 __device__ __noinline__ void finish_chunk(const GemmArgs& a, int g, int64_t row, int n0, float* v, float* u) {
@@ -135,6 +144,12 @@ __global__ void __launch_bounds__(kSpThreads, 1) gemm_split_kernel(const __grid_
 #pragma unroll
                 for (int j = 0; j < 16; ++j) acc[c][j] *= kSplitBack;
             const int r = w.m0 + q * 32 + lane;
+            if (r < w.rows && piece(a, w.row_lo + r) == kNoRow) {          // (nothing was summed for it)
+#pragma unroll
+                for (int c = 0; c < kSpMaxN / 32; ++c)
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) acc[c][j] = NAN;
+            }
             if (r < w.rows) {
                 const int64_t grow = w.row_lo + r;
                 float* crow = (float*)a.C + (int64_t)w.g * a.c_goff + grow * a.ldc;
@@ -179,17 +194,16 @@ __global__ void __launch_bounds__(kSpThreads, 1) gemm_split_kernel(const __grid_
         while (ok && w.step()) {
             const float4* A = (const float4*)((const float*)a.A + (int64_t)w.g * a.a_goff) + ch * 2;
             const float4* W = (const float4*)((const float*)a.W + (int64_t)w.g * a.w_gstride) + ch * 2;
-            constexpr uint32_t kNone = 0xffffffffu;
-            uint32_t off[P];                                               // where a row starts, in 16-byte pieces; kNone: no such row, zeros
+            uint32_t off[P];                                               // where a row starts, in 16-byte pieces; kNoRow: none here, zeros
 #pragma unroll
             for (int p = 0; p < PA; ++p) {
                 const int r = w.m0 + p * kRows + r0;
-                off[p] = r < w.rows ? (uint32_t)((int64_t)(a.row_src ? a.row_src[w.row_lo + r] : w.row_lo + r) * a.lda >> 2) : kNone;
+                off[p] = r < w.rows ? piece(a, w.row_lo + r) : kNoRow;
             }
 #pragma unroll
             for (int p = 0; p < PW; ++p) {
                 const int r = p * kRows + r0, n = w.n0 * out + (DUAL && r >= out ? r - out : r);
-                off[PA + p] = p < pw && n < a.N ? (uint32_t)((int64_t)(DUAL && r >= out ? a.N + n : n) * a.ldw >> 2) : kNone;
+                off[PA + p] = p < pw && n < a.N ? (uint32_t)((int64_t)(DUAL && r >= out ? a.N + n : n) * a.ldw >> 2) : kNoRow;
             }
             float4 buf[P][2];
             auto fetch = [&](int k) {
@@ -199,7 +213,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) gemm_split_kernel(const __grid_
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         buf[p][e] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (off[p] != kNone && left > 4 * e) buf[p][e] = (p < PA ? A : W)[(uint64_t)off[p] + k * (kTcK / 4) + e];
+                        if (off[p] != kNoRow && left > 4 * e) buf[p][e] = (p < PA ? A : W)[(uint64_t)off[p] + k * (kTcK / 4) + e];
                     }
             };
             fetch(0);
