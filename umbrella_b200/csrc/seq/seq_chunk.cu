@@ -9,7 +9,7 @@
 // rows x four columns, of K^T V four rows x eight columns: two or three 16-byte loads for 16 or 32 multiply-adds.
 // Walking tokens: a token's state update is a chain of shared-memory loads that every warp of a block repeats, 0.1 us per token
 // and block; 4096 tokens, 16 heads of 64 x 128 took 822 us in its two passes, these 194 us
-// (retention of that size is seq_chunk_tc.cu's now: 112).
+// (retention of that size is seq_chunk_tc.cu's now: 118 with norm and gate).
 #include <algorithm>
 #include <math.h>
 
@@ -310,7 +310,9 @@ int launch_chunk_memory(const ChunkMemory& m, const Batch& b, cudaStream_t st) {
     auto run = [&](auto kernel) -> int {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ChunkShared));
         if (e != cudaSuccess) return (int)e;
-        return chain_launch(kernel, grid, 256, sizeof(ChunkShared), st, m, b);
+        // (two blocks to an SM, often fewer of them than SMs: brought in while the angles or gates in front are worked out, two heavy ones fell on
+        // one SM.  us, early / not: a sequence of 171 tokens, 16 heads 64 x 128 80 / 63; 113 and 105 tokens, 4 heads 60 x 132 59 / 46)
+        return chain_launch_if(false, kernel, grid, 256, sizeof(ChunkShared), st, m, b);
     };
     return m.gates != nullptr ? run(chunk_memory_kernel<true>) : run(chunk_memory_kernel<false>);
 }
