@@ -292,6 +292,21 @@ def test_split_products_of_rows_far_apart(ops):
     torch.cuda.empty_cache()
 
 
+@pytest.mark.parametrize("value", [1e32, float("nan")])
+def test_split_products_beyond_the_parts_on_every_tile(ops, value):
+    """Several tiles a block, all of whose sums are worked out again, while the other warps wait for the next tile.  Tolerance: chains of 256
+    rounded additions of random signs, sqrt(256) 2^-24 = 1e-6, three times."""
+    from umbrella_b200 import _lib_seq as S
+    M, N, K = 4100, 1610, 256
+    assert _kernel(torch.float32, M, N, K) == S.UMBS_GEMM_SPLIT
+    a, w = _mat32(77, M, K) * value, _mat32(78, N, K)
+    got, ref = ops.gemm(a, w).double(), a.double() @ w.double().T
+    if value == value:
+        assert float((got - ref).norm() / ref.norm()) < 3e-6
+    else:
+        assert bool(torch.isnan(got).all())
+
+
 @pytest.mark.parametrize("M,N", [(200, 2000), (400, 4000)])          # streamed, tiles
 def test_split_products_of_numbers_at_the_ends_of_the_range(ops, M, N):
     """Infinite and NaN operands, numbers that round to infinity in bf16, and rows so small that their low parts vanish there."""

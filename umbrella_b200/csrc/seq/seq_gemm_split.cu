@@ -15,7 +15,7 @@
 // terms', 3 BN of 512 columns.
 //
 // Bound: the splitting: 9 rows of 8 numbers a thread and step, and a step's loads, which nothing covers (2.6 us a step of 64 k at
-// BN = 160, of which the products take 1.2).  777 rows of 1024 to 3088 columns: 177 us on the multiply-add pipe (its own time 66), 47 here; 64 rows
+// BN = 160, of which the products take 1.2).  777 rows of 1024 to 3088 columns: 177 us on the multiply-add pipe (its own time 66), 48 here; 64 rows
 // 50 -> 28.  What the first forms cost: products issued by a splitting warp 100 us, activations unrolled into the kernel 77.
 #include <algorithm>
 #include <math.h>
@@ -42,8 +42,9 @@ __device__ __forceinline__ bool odd_sum(float s) { return !(fabsf(s) <= 3.402823
 // What 16 neighbouring sums of a row become, in place (DUAL: u the up half).  Sums that the parts do not give are worked out again in
 // plain fp32: of rows that piece() does not reach, of operands that are not finite or beyond 2^103 (a part is infinite then, the next NaN), and beyond 2^79 (2^127 in the scale of
 // the parts).  Out of line: unrolled into the kernel, its 80 copies were fetched from memory by every block, 40 us of a 77 us product.
+// again: counts the sums worked out so.
 template <bool DUAL>
-__device__ __noinline__ void finish_chunk(const GemmArgs& a, int g, int64_t row, int n0, float* v, float* u) {
+__device__ __noinline__ void finish_chunk(const GemmArgs& a, int g, int64_t row, int n0, float* v, float* u, int* again) {
     const float* A = (const float*)a.A + (int64_t)g * a.a_goff + (int64_t)(a.row_src ? a.row_src[row] : row) * a.lda;
     const float* W = (const float*)a.W + (int64_t)g * a.w_gstride;
 #pragma unroll 1
@@ -55,9 +56,23 @@ __device__ __noinline__ void finish_chunk(const GemmArgs& a, int g, int64_t row,
             if (!odd_sum(s[h])) continue;
             const float* w = W + (int64_t)(h ? a.N + n : n) * a.ldw;
             s[h] = 0.f;
-            for (int k = 0; k < a.K; ++k) s[h] = fmaf(A[k], w[k], s[h]);
+            for (int k = 0; k < a.K && s[h] == s[h]; k += 64)              // (a NaN stays one)
+                for (int kk = k; kk < min(k + 64, a.K); ++kk) s[h] = fmaf(A[kk], w[kk], s[h]);
+            atomicAdd(again, 1);
         }
         v[j] = finish<DUAL>(a, s[0], s[1], g, row, n);
+    }
+}
+
+// A warp's wait whose time is up.  When all sums of a tile are worked out again, at 7 us for 1024 of k and sum, the warps that wait for these are in
+// time as long as the count goes on: a wait gives up when its time is up once more with none in between.  (In the loops themselves: 49.2 us
+// for 48.4.)
+__device__ __noinline__ bool wait_on(uint64_t* bar, uint32_t parity, volatile int* quit, volatile int* again) {
+    for (int seen = -1;;) {
+        const int now = __shfl_sync(0xffffffffu, *again, 0);
+        if (now == seen || __any_sync(0xffffffffu, *quit)) return tc_give_up(quit);
+        seen = now;
+        if (__all_sync(0xffffffffu, tc_poll_for(bar, parity, quit))) return true;
     }
 }
 
@@ -70,7 +85,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) gemm_split_kernel(const __grid_
     extern __shared__ unsigned char smem_raw[];
     __shared__ uint64_t bars[2 * kSpStages + 5];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_quit;
+    __shared__ int s_quit, s_again;
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t *full = bars, *empty = bars + kSpStages, *main_full = bars + 2 * kSpStages, *main_empty = main_full + 2, *low_empty = main_empty + 2;
     volatile int* quit = &s_quit;
@@ -86,7 +101,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) gemm_split_kernel(const __grid_
             umb::mbar_init(main_empty + i, kSpSum);
         }
         umb::mbar_init(low_empty, kSpSum);
-        s_quit = 0;
+        s_quit = s_again = 0;
         umb::fence_barrier_init();
     }
     if (warp == kSpConv + kSpSum) {
@@ -98,6 +113,10 @@ __global__ void __launch_bounds__(kSpThreads, 1) gemm_split_kernel(const __grid_
     umb::tc_fence_after();
     const uint32_t tmem = s_tmem;
     TileWalk w(a, t);
+    auto poll = [&](uint64_t* bar, uint32_t parity) {
+        return __all_sync(0xffffffffu, tc_poll_for(bar, parity, quit)) || wait_on(bar, parity, quit, &s_again);
+    };
+    auto spin = [&](uint64_t* bar, uint32_t parity) { return tc_spin_for(bar, parity) || wait_on(bar, parity, quit, &s_again); };
 
     if (warp < kSpSum) {
         // ------------------------------------------------------------------------------------ sums: a thread per row and half the columns
@@ -131,7 +150,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) gemm_split_kernel(const __grid_
                 for (int j = 0; j < 16; ++j) acc[c][j] = 0.f;
             for (int k = 0; ok && k < t.k_steps; k += kSpChunk, ++it) {
                 const uint32_t m = it & 1;
-                if (!(ok = __all_sync(0xffffffffu, tc_poll(main_full + m, (it >> 1) & 1, quit)))) break;
+                if (!(ok = poll(main_full + m, (it >> 1) & 1))) break;
                 umb::tc_fence_after();
                 add(m * bn);
                 if (lane == 0) umb::mbar_arrive(main_empty + m);
@@ -167,7 +186,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) gemm_split_kernel(const __grid_
                             o[j] = acc[c][j];
                             if (DUAL) up[j] = nch == 4 ? acc[c + 2][j] : acc[c + 1][j];
                         }
-                        finish_chunk<DUAL>(a, w.g, grow, n0, o, up);
+                        finish_chunk<DUAL>(a, w.g, grow, n0, o, up, &s_again);
 #pragma unroll
                         for (int j = 0; j < 16; ++j) acc[c][j] = o[j];
                     }
@@ -219,7 +238,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) gemm_split_kernel(const __grid_
             fetch(0);
             for (int k = 0; k < t.k_steps; ++k, ++it) {
                 const uint32_t s = it % kSpStages;
-                if (!(ok = __all_sync(0xffffffffu, tc_poll(empty + s, ((it / kSpStages) & 1) ^ 1, quit)))) break;
+                if (!(ok = poll(empty + s, ((it / kSpStages) & 1) ^ 1))) break;
                 const uint32_t dst = base + s * stage;
 #pragma unroll
                 for (int p = 0; p < P; ++p) {
@@ -247,11 +266,11 @@ __global__ void __launch_bounds__(kSpThreads, 1) gemm_split_kernel(const __grid_
         uint32_t it = 0, chunk = 0, tiles = 0;
         bool ok = true;
         for (; ok && w.step(); ++tiles) {
-            if (!(ok = tc_spin_warp(low_empty, (tiles & 1) ^ 1, quit))) break;
+            if (!(ok = spin(low_empty, (tiles & 1) ^ 1))) break;
             for (int k = 0; k < t.k_steps; ++k, ++it) {
                 const uint32_t s = it % kSpStages, m = chunk & 1;
-                if (k % kSpChunk == 0 && !(ok = tc_spin_warp(main_empty + m, ((chunk >> 1) & 1) ^ 1, quit))) break;
-                if (!(ok = tc_spin_warp(full + s, (it / kSpStages) & 1, quit))) break;
+                if (k % kSpChunk == 0 && !(ok = spin(main_empty + m, ((chunk >> 1) & 1) ^ 1))) break;
+                if (!(ok = spin(full + s, (it / kSpStages) & 1))) break;
                 umb::tc_fence_after();
                 const uint32_t st = smem_u32(smem) + s * stage, d_main = tmem + m * bn, go_main = k % kSpChunk ? 1u : 0u, go_low = k ? 1u : 0u;
                 const bool last = k + 1 == t.k_steps || k % kSpChunk == kSpChunk - 1;

@@ -31,7 +31,7 @@ __device__ __forceinline__ bool tc_test(uint64_t* bar, uint32_t parity) {
 // elect a thread for the instructions themselves: inside a branch that one thread takes, operands leave the uniform registers
 // and every tcgen05 instruction and every passed wait costs hundreds of clocks (measured with clock64 stamps: 8 products of
 // 128 x 32 x 16 and a passed wait 1740 clocks, a wait for a finished barrier 370).
-__device__ __forceinline__ bool tc_spin_warp(uint64_t* bar, uint32_t parity, volatile int* quit) {
+__device__ __forceinline__ bool tc_spin_for(uint64_t* bar, uint32_t parity) {      // false: time is up
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, 0;\n\t"
@@ -41,17 +41,19 @@ __device__ __forceinline__ bool tc_spin_warp(uint64_t* bar, uint32_t parity, vol
         "add.u32 n, n, 1;\n\tsetp.lt.u32 q, n, 33554432;\n\t@q bra AGAIN_%=;\n\t"
         "DONE_%=:\n\tselp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return __all_sync(0xffffffffu, ok) || tc_give_up(quit);
+    return __all_sync(0xffffffffu, ok);
 }
+__device__ __forceinline__ bool tc_spin_warp(uint64_t* bar, uint32_t parity, volatile int* quit) { return tc_spin_for(bar, parity) || tc_give_up(quit); }
 // polling with a short sleep in between: for warps that share a scheduler with working ones
-__device__ __forceinline__ bool tc_poll(uint64_t* bar, uint32_t parity, volatile int* quit) {
+__device__ __forceinline__ bool tc_poll_for(uint64_t* bar, uint32_t parity, volatile int* quit) {        // false: time is up, or another role gave up
     for (int i = 0; i < (1 << 24); ++i) {
         if (tc_test(bar, parity)) return true;
         __nanosleep(20);
         if ((i & 255) == 255 && *quit) return false;
     }
-    return tc_give_up(quit);
+    return false;
 }
+__device__ __forceinline__ bool tc_poll(uint64_t* bar, uint32_t parity, volatile int* quit) { return tc_poll_for(bar, parity, quit) || tc_give_up(quit); }
 // Behind the last barrier of a kernel that gave up: the host learns of it (give_up_word), and copies and products in flight end
 // before their memory goes.
 __device__ __forceinline__ void tc_settle(volatile int* quit, volatile unsigned int* report) {
