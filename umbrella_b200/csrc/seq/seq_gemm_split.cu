@@ -15,7 +15,7 @@
 // terms', 3 BN of 512 columns.
 //
 // Bound: the splitting: 9 rows of 8 numbers a thread and step, and a step's loads, which nothing covers (2.6 us a step of 64 k at
-// BN = 160, of which the products take 1.2).  777 rows of 1024 to 3088 columns: 177 us on the multiply-add pipe (its own time 66), 48 here; 64 rows
+// BN = 160, of which the products take 1.2).  777 rows of 1024 to 3088 columns: 177 us on the multiply-add pipe (its own time 66), 49 here; 64 rows
 // 50 -> 28.  What the first forms cost: products issued by a splitting warp 100 us, activations unrolled into the kernel 77.
 #include <algorithm>
 #include <math.h>
@@ -42,31 +42,45 @@ __device__ __forceinline__ bool odd_sum(float s) { return !(fabsf(s) <= 3.402823
 // What 16 neighbouring sums of a row become, in place (DUAL: u the up half).  Sums that the parts do not give are worked out again in
 // plain fp32: of rows that piece() does not reach, of operands that are not finite or beyond 2^103 (a part is infinite then, the next NaN), and beyond 2^79 (2^127 in the scale of
 // the parts).  Out of line: unrolled into the kernel, its 80 copies were fetched from memory by every block, 40 us of a 77 us product.
-// again: counts the sums worked out so.
+// again: counts them, and their way through a long row.  (16 sums side by side: a row's numbers are fetched once for all of them, 4096 rows x 1024 ->
+// 1600 columns with every sum worked out again 28 -> 6.3 ms.)
 template <bool DUAL>
 __device__ __noinline__ void finish_chunk(const GemmArgs& a, int g, int64_t row, int n0, float* v, float* u, int* again) {
     const float* A = (const float*)a.A + (int64_t)g * a.a_goff + (int64_t)(a.row_src ? a.row_src[row] : row) * a.lda;
     const float* W = (const float*)a.W + (int64_t)g * a.w_gstride;
 #pragma unroll 1
-    for (int j = 0; j < 16 && n0 + j < a.N; ++j) {
-        const int n = n0 + j;
-        float s[2] = {v[j], DUAL ? u[j] : 0.f};
+    for (int h = 0; h < (DUAL ? 2 : 1); ++h) {
+        float* o = h ? u : v;
+        uint32_t odd = 0;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) odd |= (uint32_t)(n0 + j < a.N && odd_sum(o[j])) << j;
+        if (odd == 0) continue;
+        const float* w = W + (int64_t)(h ? a.N + n0 : n0) * a.ldw;
+        float s[16] = {};
 #pragma unroll 1
-        for (int h = 0; h < (DUAL ? 2 : 1); ++h) {
-            if (!odd_sum(s[h])) continue;
-            const float* w = W + (int64_t)(h ? a.N + n : n) * a.ldw;
-            s[h] = 0.f;
-            for (int k = 0; k < a.K && s[h] == s[h]; k += 64)              // (a NaN stays one)
-                for (int kk = k; kk < min(k + 64, a.K); ++kk) s[h] = fmaf(A[kk], w[kk], s[h]);
-            atomicAdd(again, 1);
+        for (int k = 0; k < a.K; k += 4) {                  // (K is a multiple of 4, rows start on 16 bytes)
+            const float4 x = *reinterpret_cast<const float4*>(A + k);
+            uint32_t left = 0;                              // sums that are not NaN yet: those stay so
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                if (odd >> j & 1) {
+                    const float4 y = __ldg(reinterpret_cast<const float4*>(w + j * a.ldw + k));
+                    s[j] = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, s[j]))));
+                    left |= (uint32_t)(s[j] == s[j]) << j;
+                }
+            if (left == 0) break;
+            if ((k & 4095) == 0) atomicAdd(again, 1);
         }
-        v[j] = finish<DUAL>(a, s[0], s[1], g, row, n);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) o[j] = odd >> j & 1 ? s[j] : o[j];
     }
+#pragma unroll 1
+    for (int j = 0; j < 16 && n0 + j < a.N; ++j) v[j] = finish<DUAL>(a, v[j], DUAL ? u[j] : 0.f, g, row, n0 + j);
 }
 
-// A warp's wait whose time is up.  When all sums of a tile are worked out again, at 7 us for 1024 of k and sum, the warps that wait for these are in
-// time as long as the count goes on: a wait gives up when its time is up once more with none in between.  (In the loops themselves: 49.2 us
-// for 48.4.)
+// A warp's wait whose time is up.  When all sums of a tile are worked out again, at 0.4 ms for 1024 of k and 16 of them, the warps that wait for these are in
+// time as long as the count goes on: a wait gives up when its time is up once more with none in between.  (In the loops themselves a
+// microsecond of 49.)
 __device__ __noinline__ bool wait_on(uint64_t* bar, uint32_t parity, volatile int* quit, volatile int* again) {
     for (int seen = -1;;) {
         const int now = __shfl_sync(0xffffffffu, *again, 0);
