@@ -71,6 +71,46 @@ def test_tokens_in_front_of_a_nan_keep_their_bits(kind, n, what):
         assert not torch.isfinite(out[j]).any(), j
 
 
+@pytest.mark.parametrize("n", [128, 300])
+@pytest.mark.parametrize("what", ["state", "row", "values"])
+def test_retention_in_pieces_of_128_from_a_carried_state(n, what):
+    """What is not finite in a carried state, a row or a token's values is where float64 has it, in the outputs (rows of the norm) and in the state;
+    the rest is what it is without.  Tolerance as in test_gpu_seq_chunk.py."""
+    from test_gpu_seq_chunk import _ratio, _retention64
+    from umbrella_b200 import ops_seq as K
+    heads, dim, vdim, j = 2, 64, 128, n // 2
+    hd, hv = heads * dim, heads * vdim
+    x, state = rnd(n, 2 * (hd + hv), seed=n).to(DEV), rnd(1, heads, dim, vdim, seed=1).to(DEV)
+    decay = torch.tensor([0.97, 0.999], device=DEV)
+
+    def run(t, S):
+        S = S.clone()
+        out = K.retention(t, K.RaggedBatch([(0, n, 5, 0)], DEV), heads, dim, vdim, 0, torch.zeros(1, device=DEV), decay, 1e-6, S, k_scale=1.0)
+        return out, S[0]
+    clean, clean_state = run(x, state)
+    if what == "state":
+        state[0, 0, 3, 7] = float("inf")
+    elif what == "row":
+        x[j, dim:2 * dim] = float("nan")                                # of queries: head 1's row j alone
+        x[j, hd + 5] = float("nan")                                     # of keys: head 0 from row j on
+    else:
+        x[j, 2 * hd + 9] = float("-inf")                                # a value of head 0
+    out, got = run(x, state)
+    want, S = _retention64(x, heads, dim, vdim, decay, state[0], 1e-6)
+    assert torch.equal(torch.isfinite(got), torch.isfinite(S)) and torch.equal(torch.isnan(got), torch.isnan(S))
+    fin = torch.isfinite(S)
+    assert torch.equal(got[torch.isinf(S)].double(), S[torch.isinf(S)]) and _ratio(got[fin], S[fin]) < 2e-6
+    if what == "values":                                                # (a score times an infinity is one; a state's column of them is NaN: a piece later)
+        assert not bool(torch.isfinite(out[j:, 9]).any()) and _ratio(out[:, vdim:], want[:, vdim:]) < 2e-6
+    else:
+        fin = torch.isfinite(want)
+        assert torch.equal(torch.isfinite(out), fin) and _ratio(out[fin], want[fin]) < 2e-6
+    first = 0 if what == "state" else j
+    assert torch.equal(out[:first], clean[:first])
+    if what != "row":
+        assert torch.equal(out[:, vdim:], clean[:, vdim:]) and torch.equal(got[1], clean_state[1])
+
+
 # ---------------------------------------------------------------------------------------------- attention
 def seen_only(q, keys, values, visible, scale, sink):
     """float64: every row over the keys it sees and no others.  q [n, d], keys [m, d], values [m, e], visible [n, m]."""

@@ -67,14 +67,6 @@ __device__ __forceinline__ void turn_row(const ChunkMemory& x, int ch, float (&f
         if (ch < 2 * hc) f[e] = ch < hc ? f[e] * c[e] - g * s[e] : f[e] * c[e] + g * s[e];
     }
 }
-__device__ __forceinline__ float turned(const ChunkMemory& x, int64_t tok, int off, float scale, int d) {
-    float f[8];
-    turned8(x, tok, off, scale, d & ~7, f);
-    float r = f[0];
-#pragma unroll
-    for (int e = 1; e < 8; ++e) r = (d & 7) == e ? f[e] : r;
-    return r;
-}
 template <bool SCALED = false>
 __device__ __forceinline__ void st_parts(uint32_t at, uint32_t step, const float (&f)[8]) {
     uint4 v[3];
@@ -89,37 +81,79 @@ __device__ __forceinline__ uint64_t mn_desc(uint32_t addr, uint32_t piece) {
     return (umb::umma_smem_desc_sw128(addr) & ~((uint64_t)0x3fff << 16)) | ((uint64_t)(piece >> 4) << 16);
 }
 
-// element (d, c) of L, token by token
-__device__ __noinline__ float plain_state(const ChunkMemory& x, int64_t tok, int nb, int h, int d, int c, float dec) {
-    float s = 0.f;
-    for (int j = 0; j < nb; ++j)
-        s = fmaf(s, dec, turned(x, tok + j, x.koff + h * x.dim, x.kscale, d) * x.x[(tok + j) * x.ld + x.voff + h * x.vdim + c]);
-    return s;
-}
-// element (i, c) of O, token by token; st: the state in front of the tokens
-__device__ float plain_output(const ChunkMemory& x, int64_t tok, int i, int h, int c, float dec, const float* st) {
-    float o = 0.f;
-    for (int d = 0; d < x.dim; ++d) o = fmaf(turned(x, tok + i, x.qoff + h * x.dim, x.qscale, d), st[(int64_t)d * x.vdim + c], o);
-    o *= powf(dec, (float)(i + 1));
-    for (int j = 0; j <= i; ++j) {
-        float w = 0.f;
-        for (int d = 0; d < x.dim; ++d)
-            w = fmaf(turned(x, tok + i, x.qoff + h * x.dim, x.qscale, d), turned(x, tok + j, x.koff + h * x.dim, x.kscale, d), w);
-        o = fmaf(w * powf(dec, (float)(i - j)), x.x[(tok + j) * x.ld + x.voff + h * x.vdim + c], o);
+// What the parts do not give, in plain fp32, by the whole block where one of its sums is no number (prompts of 4096 tokens, 16 heads, all of them
+// NaN from the first tokens on: 0.8 ms; each number by a thread of its own, token by token, took 2400 of them).
+// The turned and scaled rows of the block's tokens, to rows of dim + 1 floats.
+__device__ __forceinline__ void plain_rows(const ChunkMemory& x, int64_t tok, int nb, int off, float scale, float* to) {
+    const int n8 = x.dim / 8;
+    for (int e = threadIdx.x; e < nb * n8; e += blockDim.x) {
+        const int r = e / n8, d = (e - r * n8) * 8;
+        float f[8];
+        turned8(x, tok + r, off, scale, d, f);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) to[r * (x.dim + 1) + d + u] = f[u];
     }
-    return o;
 }
-
-// columns c0 + e of row i for the bits e of odd
-__device__ __noinline__ void plain_outputs(const ChunkMemory& x, int64_t tok, int i, int h, int c0, float dec, const float* st, uint32_t odd, float* o) {
-    for (; odd; odd &= odd - 1) o[__ffs(odd) - 1] = plain_output(x, tok, i, h, c0 + __ffs(odd) - 1, dec, st);
+// L, token by token: dimensions d0 + i of column c for the bits i of odd, to `out` and x.vdim further each
+__device__ __noinline__ void plain_states(const ChunkMemory& x, int64_t tok, int nb, int h, int d0, int c, float dec, float* sm, uint32_t odd, float* out) {
+    plain_rows(x, tok, nb, x.koff + h * x.dim, x.kscale, sm);
+    __syncthreads();
+    if (odd == 0) return;
+    float s[32] = {};
+    const float* v = x.x + tok * x.ld + x.voff + h * x.vdim + c;
+    for (int j = 0; j < nb; ++j, v += x.ld) {
+        const float z = *v;
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+            if (odd >> i & 1) s[i] = fmaf(s[i], dec, sm[j * (x.dim + 1) + d0 + i] * z);
+    }
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+        if (odd >> i & 1) out[(int64_t)i * x.vdim] = s[i];
+}
+// O: columns c + e of row i for the bits e of odd, of `cols` that there are; st: the state in front of the tokens
+__device__ __noinline__ void plain_outputs(const ChunkMemory& x, int64_t tok, int nb, int h, int i, int c, int cols, const float* lam, const float* st, float* sm,
+                                           uint32_t odd, float* o) {
+    const int dp = x.dim + 1;
+    float *q = sm, *k = q + kCtT * dp, *w = k + kCtT * dp;  // rows of q and k, weights in rows of kCtT + 1
+    plain_rows(x, tok, nb, x.qoff + h * x.dim, x.qscale, q);
+    plain_rows(x, tok, nb, x.koff + h * x.dim, x.kscale, k);
+    __syncthreads();
+    for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
+        const int r = e / nb, j = e - r * nb;
+        if (j > r) continue;
+        float z = 0.f;
+        for (int d = 0; d < x.dim; ++d) z = fmaf(q[r * dp + d], k[j * dp + d], z);
+        w[r * (kCtT + 1) + j] = z * lam[r - j];
+    }
+    __syncthreads();
+    if (odd == 0) return;
+    float s[32] = {};
+    auto add = [&](float z, const float* row) {
+#pragma unroll
+        for (int e = 0; e < 32; e += 4)
+            if (e < cols) {
+                const float4 v = *reinterpret_cast<const float4*>(row + e);
+                s[e] = fmaf(z, v.x, s[e]);
+                s[e + 1] = fmaf(z, v.y, s[e + 1]);
+                s[e + 2] = fmaf(z, v.z, s[e + 2]);
+                s[e + 3] = fmaf(z, v.w, s[e + 3]);
+            }
+    };
+    for (int d = 0; d < x.dim; ++d) add(q[i * dp + d], st + (int64_t)d * x.vdim + c);
+#pragma unroll
+    for (int e = 0; e < 32; ++e) s[e] *= lam[i + 1];
+    const float* v = x.x + tok * x.ld + x.voff + h * x.vdim + c;
+    for (int j = 0; j <= i; ++j, v += x.ld) add(w[i * (kCtT + 1) + j], v);
+#pragma unroll
+    for (int e = 0; e < 32; ++e) o[e] = odd >> e & 1 ? s[e] : o[e];
 }
 
 __global__ void __launch_bounds__(256, 3) chunk_states_kernel(const __grid_constant__ ChunkMemory x, const __grid_constant__ Batch b, unsigned int* report) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ uint64_t done;
     __shared__ uint32_t s_tmem;
-    __shared__ int s_quit;
+    __shared__ int s_quit, s_odd;
     __shared__ float keep[kCtT];
     volatile int* quit = &s_quit;
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -134,7 +168,7 @@ __global__ void __launch_bounds__(256, 3) chunk_states_kernel(const __grid_const
     if (tid < kCtT) keep[tid] = tid < nb ? powf(dec, (float)(nb - 1 - tid)) : 0.f;
     if (tid == 0) {
         umb::mbar_init(&done, 1);
-        s_quit = 0;
+        s_quit = s_odd = 0;
         umb::fence_barrier_init();
     }
     if (warp == 0) {
@@ -198,33 +232,31 @@ __global__ void __launch_bounds__(256, 3) chunk_states_kernel(const __grid_const
         }
     }
     if (ok) ok = __syncthreads_and(tc_spin_warp(&done, nb > 64 ? 1 : 0, quit));
+    // lane: value column; 32 dimensions a warp
+    const int q = warp & 3, d0 = (warp >> 2) * 32, col = q * 32 + lane;
+    float* out = x.seg_state + ((((int64_t)s * x.n_seg + c) * x.heads + h) * x.dim + d0) * x.vdim + c0 + col;
+    uint32_t odd = 0;
     if (ok) {
         umb::tc_fence_after();
-        // lane: value column; 32 dimensions a warp
-        const int q = warp & 3, d0 = (warp >> 2) * 32, col = q * 32 + lane;
         const uint32_t at = tmem + ((uint32_t)(q * 32) << 16) + d0;
         uint32_t u[32], v[32];
         UMB_TMEM_LD_X32(at, u);
         UMB_TMEM_LD_X32(at + 64, v);
         umb::tc_wait_ld();
-        float* out = x.seg_state + (((int64_t)s * x.n_seg + c) * x.heads + h) * x.dim * x.vdim + c0 + col;
-        uint32_t odd = 0;
         if (col < nv)
 #pragma unroll
             for (int i = 0; i < 32; ++i)
                 if (d0 + i < x.dim) {
                     const float l = (__uint_as_float(u[i]) + __uint_as_float(v[i])) * kSplitBack;
                     odd |= (uint32_t)no_number(l) << i;
-                    out[(int64_t)(d0 + i) * x.vdim] = l;
+                    out[(int64_t)i * x.vdim] = l;
                 }
-        for (; odd; odd &= odd - 1) {
-            const int d = d0 + __ffs(odd) - 1;
-            out[(int64_t)d * x.vdim] = plain_state(x, tok, nb, h, d, c0 + col, dec);
-        }
+        if (odd) s_odd = 1;
     }
     __syncwarp();
     umb::tc_fence_before();
     __syncthreads();
+    if (s_odd) plain_states(x, tok, nb, h, d0, min(c0 + col, x.vdim - 1), dec, reinterpret_cast<float*>(smem), odd, out);
     tc_settle(quit, report);
     if (warp == 0) {
         umb::tc_fence_after();
@@ -270,7 +302,7 @@ __global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_cons
     extern __shared__ unsigned char smem_raw[];
     __shared__ uint64_t done;
     __shared__ uint32_t s_tmem;
-    __shared__ int s_quit, s_bad;
+    __shared__ int s_quit, s_bad, s_odd;
     __shared__ float lam[kCtT + 1];
     volatile int* quit = &s_quit;
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -285,7 +317,7 @@ __global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_cons
     if (tid <= kCtT) lam[tid] = powf(dec, (float)tid);
     if (tid == 0) {
         umb::mbar_init(&done, 1);
-        s_quit = 0;
+        s_quit = s_odd = 0;
         s_bad = kCtT;
         umb::fence_barrier_init();
     }
@@ -475,23 +507,29 @@ __global__ void __launch_bounds__(512, 1) chunk_outputs_kernel(const __grid_cons
             o[e] += (__uint_as_float(u[e]) + __uint_as_float(v[e])) * kSplitBack;
             odd |= (uint32_t)((i >= s_bad || no_number(o[e])) && i < nb) << e;
         }
-        if (odd) {
+        if (odd) s_odd = 1;
+        // rows leave by whole warps, four columns a lane, from where the values were (a thread's own row, 16 bytes of it at a time beside 31
+        // others, took 15,000 clocks of 35,000)
+        float* so = reinterpret_cast<float*>(smem + 6 * 16384);
+        auto put = [&] {
+#pragma unroll
+            for (int e = 0; e < 32; e += 4) *reinterpret_cast<float4*>(so + i * kCtStride + part + e) = make_float4(o[e], o[e + 1], o[e + 2], o[e + 3]);
+            __syncthreads();
+        };
+        put();
+        if (s_odd) {
             float f[32];                                    // (columns that are not there: 0 times a score beyond the parts is none)
 #pragma unroll
             for (int e = 0; e < 32; ++e) {
                 f[e] = part + e < nv ? o[e] : 0.f;
                 odd &= ~((uint32_t)(part + e >= nv) << e);
             }
-            plain_outputs(x, tok, i, h, n0, dec, st, odd, f);
+            plain_outputs(x, tok, nb, h, i, n0, nv - part, lam, st, reinterpret_cast<float*>(smem), odd, f);
 #pragma unroll
             for (int e = 0; e < 32; ++e) o[e] = f[e];
+            __syncthreads();
+            put();
         }
-        // rows leave by whole warps, four columns a lane, from where the values were (a thread's own row, 16 bytes of it at a time beside 31
-        // others, took 15,000 clocks of 35,000)
-        float* so = reinterpret_cast<float*>(smem + 6 * 16384);
-#pragma unroll
-        for (int e = 0; e < 32; e += 4) *reinterpret_cast<float4*>(so + i * kCtStride + part + e) = make_float4(o[e], o[e + 1], o[e + 2], o[e + 3]);
-        __syncthreads();
         const int hv = x.heads * x.vdim, rows = min(8, nb - warp * 8);
         const float* g = x.x + (tok + warp * 8) * x.ld + x.voff + hv + (int64_t)h * x.vdim + c0 + lane * 4;
         T* orow = out + (tok + warp * 8) * hv + (int64_t)h * x.vdim + c0 + lane * 4;
