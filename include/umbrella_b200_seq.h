@@ -320,8 +320,8 @@ int umbs_forward(const umbs_model_t* model, const umbs_batch_t* batch, float* lo
 
 /* ---- building blocks (dtype: UMBS_BF16 / UMBS_F32 for the `void*` activations and weights) ---- */
 
-/* C[m, g*c_goff + n] = sum_k A[row(m), g*a_goff + k] * W[g*w_gstride + n*ldw + k], fp32 accumulation in k order
- * (a row's result does not depend on the other rows of the call).  groups > 1: batched over g.  grp_off != NULL:
+/* C[m, g*c_goff + n] = sum_k A[row(m), g*a_goff + k] * W[g*w_gstride + n*ldw + k], fp32 accumulation
+ * in an order that does not depend on the other rows of the call, so neither does a row's result.  groups > 1: batched over g.  grp_off != NULL:
  * group g owns rows [grp_off[g], grp_off[g+1]) (device array; M bounds a group's size), row_src != NULL gathers A rows.
  * dual != 0: W holds N gate rows then N up rows per group and C gets the gated activation (see umbs_mlp_t).
  * c_f32 != 0: C is fp32, otherwise of `dtype`. */

@@ -9,7 +9,7 @@
 // rows x four columns, of K^T V four rows x eight columns: two or three 16-byte loads for 16 or 32 multiply-adds.
 // Walking tokens: a token's state update is a chain of shared-memory loads that every warp of a block repeats, 0.1 us per token
 // and block; 4096 tokens, 16 heads of 64 x 128 took 822 us in its two passes, these 194 us
-// (retention of that size is seq_chunk_tc.cu's now: 118 with norm and gate).
+// (retention of that size is seq_chunk_tc.cu's now: 119 with norm and gate).
 #include <algorithm>
 #include <math.h>
 

@@ -10,7 +10,7 @@
 // Bound: what a block does one after the other (rows in, split, products, weights split again, products, out), four warps a scheduler
 // in step: outputs 33,000 clocks a block, of which the products take 6,000, three and a half blocks to an SM (192 KB of shared memory
 // and all of tensor memory each); states three blocks to an SM (72 KB).  4096 tokens of 16 heads 64 x 128: 238 us in pieces of 32
-// tokens on the multiply-add pipe with a norm-and-gate kernel behind, 117 here (states 29, chain 9, outputs 75, cold).  Distance from
+// tokens on the multiply-add pipe with a norm-and-gate kernel behind, 119 here (states 31, chain 9, outputs 77, cold).  Distance from
 // float64 2.1e-7 -> 1.1e-7 (fp32 results of 128 to 1500 tokens), states 1.7e-7 -> 0.9e-7.
 #include <math.h>
 

@@ -9,9 +9,9 @@
 //   * gemm_tc_kernel    -- bf16 operands through tcgen05 with fp32 accumulators (seq_gemm_tc.cu);
 //   * gemm_skinny_kernel, gemm_rows_kernel -- few rows (decoding), bf16 and fp32: a weight stream with the rows' partial sums in
 //                          registers.
-// In each of them an output element is one fp32 sum over k in an order that does not depend on the other rows, so a
-// row's result is the same whatever else is in the batch; which kernel runs depends on the row count, and they
-// differ from each other by rounding only.
+// In each of them the order in which an output element's products are added up (one chain, or shares of k by themselves first) does not
+// depend on the other rows, so a row's result is the same whatever else is in the batch; which kernel runs depends on the row count and
+// the alignment, and they differ from each other by rounding only.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -156,8 +156,8 @@ __global__ void __launch_bounds__(64) gemm_simt_kernel(GemmArgs a, int vec, int 
 // such steps are in flight before the first is used.  KW warps of a block share a tile's k.
 // Sums: every product starts from zero, a step's products are added in fp32 pair by pair, the steps in order, the warps in fp64: no chain
 // runs through the tensor core, which cuts its sums off (5 to 7e-8 from float64 for K = 384 to 4096, 6 to 8e-8 as chains of
-// multiply-adds).  The order depends on the weight's sizes alone: a row's result does not depend on the other rows.  A group without
-// rows returns before touching its weights, so a decode step reads only the experts that were chosen.
+// multiply-adds).  The order depends on the weight's sizes and on whether rows start on 32 bytes or 16 (launch_skinny): a row's result does not
+// depend on the other rows.  A group without rows returns before touching its weights, so a decode step reads only the experts that were chosen.
 // Bound: a launch, a load's way from HBM and the reduction, one after the other: 8 rows of 2048 to 6144 columns 14.8 -> 6.7 us (3.8 TB/s;
 // the multiply-adds that this replaced unpacked every weight for every row), of 1024 to 1024 3.9 -> 2.5, 16 rows 23.9 -> 9.3.
 // V 16-byte pieces that follow one another: weights, which no other block reads, and activations
@@ -285,11 +285,7 @@ __global__ void __launch_bounds__(32 * KW) gemm_skinny_kernel(const GemmArgs a) 
     }
 }
 
-// The weight's sizes choose the order of the sums: warps that share a tile's k so that each has its pieces in flight at once, up to
-// what the SMs hold.  Tiles of 8 weight rows (the activations are the 16-row operand then) where tiles of 16 would leave SMs idle, and
-// for 9 to 16 activation rows, whose pieces the registers hold beside one weight row's.  (us, weights not in L2, 8 rows, tiles of
-// 16 / 8 rows: 1024 x 1024 2.8 / 2.7, 2048 x 1024 3.1 / 3.2, 8192 x 1024 5.8 / 6.8; 6144 x 2048 by 4 / 8 / 16 warps 9.0 / 7.3 / 9.3.)
-// The weight's sizes choose the order of the sums: warps that share a tile's k so that each has all or half of its pieces in flight at
+// The weight's sizes (and V) choose the order of the sums: warps that share a tile's k so that each has all or half of its pieces in flight at
 // once, up to what the SMs hold.  Tiles of 8 weight rows (the activations are the 16-row operand then) where tiles of 16 would leave SMs
 // idle, and for 9 to 16 activation rows, whose pieces the registers hold beside one weight row's; the sums are the same in both.
 // us, weights of 50 to 200 MB in turn, 8 rows, the best of the others / the chosen one: 1024 x 1024 2.4 / 2.5, 2048 x 1024 2.6 / 2.6,

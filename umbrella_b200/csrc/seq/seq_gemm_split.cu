@@ -40,10 +40,10 @@ __device__ __forceinline__ uint32_t piece(const GemmArgs& a, int64_t r) {
 __device__ __forceinline__ bool odd_sum(float s) { return !(fabsf(s) <= 3.402823466e38f); }
 
 // What 16 neighbouring sums of a row become, in place (DUAL: u the up half).  Sums that the parts do not give are worked out again in
-// plain fp32: of rows that piece() does not reach, of operands that are not finite or beyond 2^103 (a part is infinite then, the next NaN), and beyond 2^79 (2^127 in the scale of
-// the parts).  Out of line: unrolled into the kernel, its 80 copies were fetched from memory by every block, 40 us of a 77 us product.
-// again: counts them, and their way through a long row.  (16 sums side by side: a row's numbers are fetched once for all of them, 4096 rows x 1024 ->
-// 1600 columns with every sum worked out again 28 -> 6.3 ms.)
+// plain fp32: of rows that piece() does not reach, of operands that are not finite or beyond 2^103 (a part is infinite then, the next NaN),
+// and sums beyond 2^79 (2^127 in the scale of the parts).  16 side by side, for which a row's numbers are fetched once: all of 4096 rows x
+// 1024 -> 1600 columns 28 -> 6.3 ms.  Out of line: unrolled into the kernel, its 80 copies were fetched from memory by every block, 40 us of
+// a 77 us product.  again: counts them, and their way through a long row.
 template <bool DUAL>
 __device__ __noinline__ void finish_chunk(const GemmArgs& a, int g, int64_t row, int n0, float* v, float* u, int* again) {
     const float* A = (const float*)a.A + (int64_t)g * a.a_goff + (int64_t)(a.row_src ? a.row_src[row] : row) * a.lda;
