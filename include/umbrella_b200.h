@@ -120,6 +120,11 @@ int umb_awq_gemm_f16(const void* x, int64_t ldx, const void* packed, void* y, in
                      int N_total, int group, const umb_epilogue_t* epilogue, void* workspace, size_t workspace_bytes,
                      umb_stream_t stream);
 
+/* The same for up to 512 rows; the workspace holds umb_awq_gemm_rows_ws_bytes() bytes, zero-filled once. */
+size_t umb_awq_gemm_rows_ws_bytes(int M, int K, int N_total);
+int umb_awq_gemm_rows_f16(const void* x, int64_t ldx, const void* packed, void* y, int64_t ldy, int M, int K, int N_total, int group,
+                          const umb_epilogue_t* epilogue, void* workspace, size_t workspace_bytes, umb_stream_t stream);
+
 /* fp16 weights W [N, K] row-major (torch Linear layout): y[M,N] = x . W^T.  Same contract. */
 int umb_gemm_f16(const void* x, int64_t ldx, const void* w, int64_t ldw, void* y, int64_t ldy, int M, int K, int N,
                  const umb_epilogue_t* epilogue, void* workspace, size_t workspace_bytes, umb_stream_t stream);
@@ -317,6 +322,12 @@ int umb_llama_forward(const umb_llama_t* model, const int64_t* input_ids, const 
                       int kv_offset, const umb_attn_mask_t* mask, float* logits, int logits_from_row,
                       unsigned long long* argmax_keys, umb_stream_t stream);
 
+/* The same with passes over the weights of up to rows_per_pass rows (umb_llama_forward: 128).  AWQ layers take up to 512, fp16
+ * layers 128; the model's activations have to hold as many rows.  A prompt of 500 rows is one pass instead of four. */
+int umb_llama_forward_passes(const umb_llama_t* model, int rows_per_pass, const int64_t* input_ids, const int64_t* position_ids, int rows,
+                             int kv_offset, const umb_attn_mask_t* mask, float* logits, int logits_from_row,
+                             unsigned long long* argmax_keys, umb_stream_t stream);
+
 /* Layer-range slice of umb_llama_forward for paged (host-offloaded) weights -- the seam of the
  * reference's LlamaOffload.inference loop (umbrella/models/llama.py:196-219): the caller runs layers
  * [layer_begin, layer_end) of rows <= 128 (hidden state kept in model->hidden between calls), waiting on
@@ -324,6 +335,10 @@ int umb_llama_forward(const umb_llama_t* model, const int64_t* input_ids, const 
  * logits != NULL finishes with the final norm + lm_head (last slice; layer_begin == layer_end ==
  * num_layers runs the head alone). */
 int umb_llama_forward_range(const umb_llama_t* model, const int64_t* input_ids, const int64_t* position_ids, int rows,
+                            int kv_offset, const umb_attn_mask_t* mask, int layer_begin, int layer_end, int do_embed,
+                            float* logits, int logits_from_row, unsigned long long* argmax_keys, umb_stream_t stream);
+/* The same for up to rows_per_pass rows (umb_llama_forward_passes). */
+int umb_llama_forward_range_passes(const umb_llama_t* model, int rows_per_pass, const int64_t* input_ids, const int64_t* position_ids, int rows,
                             int kv_offset, const umb_attn_mask_t* mask, int layer_begin, int layer_end, int do_embed,
                             float* logits, int logits_from_row, unsigned long long* argmax_keys, umb_stream_t stream);
 

@@ -66,6 +66,9 @@ SIGNATURES = {
     "umb_gemm_workspace_bytes": (c_size_t, [c_int, c_int, c_int]),
     "umb_awq_gemm_f16": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_int,
                                  C.POINTER(Epilogue), c_void_p, c_size_t, c_void_p]),
+    "umb_awq_gemm_rows_ws_bytes": (c_size_t, [c_int, c_int, c_int]),
+    "umb_awq_gemm_rows_f16": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_int,
+                                      C.POINTER(Epilogue), c_void_p, c_size_t, c_void_p]),
     "umb_gemm_f16": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_int,
                              C.POINTER(Epilogue), c_void_p, c_size_t, c_void_p]),
     "umb_tree_attn_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
@@ -89,8 +92,12 @@ SIGNATURES = {
     "umb_llama_gemm_ws_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int, c_int]),
     "umb_llama_forward": (c_int, [C.POINTER(LlamaModel), c_void_p, c_void_p, c_int, c_int, C.POINTER(AttnMask),
                                   c_void_p, c_int, c_void_p, c_void_p]),
+    "umb_llama_forward_passes": (c_int, [C.POINTER(LlamaModel), c_int, c_void_p, c_void_p, c_int, c_int, C.POINTER(AttnMask),
+                                         c_void_p, c_int, c_void_p, c_void_p]),
     "umb_llama_forward_range": (c_int, [C.POINTER(LlamaModel), c_void_p, c_void_p, c_int, c_int, C.POINTER(AttnMask),
                                         c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p]),
+    "umb_llama_forward_range_passes": (c_int, [C.POINTER(LlamaModel), c_int, c_void_p, c_void_p, c_int, c_int, C.POINTER(AttnMask),
+                                               c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p]),
     "umb_llama_forward_dyn": (c_int, [C.POINTER(LlamaModel), c_void_p, c_void_p, c_int, c_void_p, c_int, c_int,
                                       c_void_p, c_int, c_void_p, c_void_p, c_void_p]),
     "umb_sample_f32": (c_int, [c_void_p, c_int64, c_int, c_int, c_int, c_float, c_int, c_float, c_void_p, c_int, c_void_p,

@@ -12,13 +12,13 @@ namespace umb {
 static int linear(const umb_llama_t* m, const void* x, int64_t ldx, const void* w, void* y, int64_t ldy, int rows,
                   int K, int N, const umb_epilogue_t* epi, umb_stream_t st) {
     if (m->awq)
-        return umb_awq_gemm_f16(x, ldx, w, y, ldy, rows, K, N, 128, epi, m->gemm_ws, m->gemm_ws_bytes, st);
+        return awq_gemm_rows(x, ldx, w, y, ldy, rows, K, N, epi, m->gemm_ws, m->gemm_ws_bytes, (cudaStream_t)st);
     return umb_gemm_f16(x, ldx, w, K, y, ldy, rows, K, N, epi, m->gemm_ws, m->gemm_ws_bytes, st);
 }
 
 #define UMB_TRY(expr) do { int rc__ = (expr); if (rc__ != UMB_OK) return rc__; } while (0)
 
-constexpr int kChunkRows = UMB_MAX_ROWS;
+constexpr int kChunkRows = 128, kChunkRowsAwq = 512;       // token rows of a pass over the weights, at most
 
 // UMB_FUSE_ROPE=1 runs the q|k|v projection with the fused RoPE + KV-append epilogue (UMB_EPI_ROPE_QKV) instead of
 // the GEMM + rope_append kernel pair.  Off by default: bit-identical, one launch fewer, but measured slower
@@ -106,10 +106,12 @@ static int forward_chunk(const umb_llama_t* m, const int64_t* ids, const int64_t
                                     m->rms_eps, st));
             umb_epilogue_t lg{};
             lg.mode = UMB_EPI_LOGITS;
-            lg.argmax = keys;
             // logits == NULL with keys only is not supported by the epilogue: the fp32 rows are always written
-            UMB_TRY(umb_gemm_f16(m->normed, H, m->lm_head, H, logits, m->vocab, n, H, m->vocab, &lg, m->gemm_ws,
-                                 m->gemm_ws_bytes, st));
+            for (int r0 = 0; r0 < n; r0 += kChunkRows) {
+                lg.argmax = keys ? keys + r0 : nullptr;
+                UMB_TRY(umb_gemm_f16((const __half*)m->normed + (int64_t)r0 * H, H, m->lm_head, H, logits + (int64_t)r0 * m->vocab, m->vocab,
+                                     n - r0 < kChunkRows ? n - r0 : kChunkRows, H, m->vocab, &lg, m->gemm_ws, m->gemm_ws_bytes, st));
+            }
         }
     }
     return UMB_OK;
@@ -124,22 +126,25 @@ extern "C" size_t umb_llama_gemm_ws_bytes(int hidden, int intermediate, int num_
     for (int i = 0; i < 5; ++i) {
         const size_t b = umb_gemm_workspace_bytes(128, hidden, ns[i]);
         best = b > best ? b : best;
+        const size_t wide = umb::awq_wide_ws_bytes(umb::kChunkRowsAwq, ns[i]);        // (the passes of umb_llama_forward_passes)
+        best = i < 4 && wide > best ? wide : best;
     }
     return best;
 }
 
-extern "C" int umb_llama_forward(const umb_llama_t* m, const int64_t* input_ids, const int64_t* position_ids, int rows,
-                                 int kv_offset, const umb_attn_mask_t* mask, float* logits, int logits_from_row,
-                                 unsigned long long* argmax_keys, umb_stream_t stream) {
+extern "C" int umb_llama_forward_passes(const umb_llama_t* m, int rows_per_pass, const int64_t* input_ids, const int64_t* position_ids, int rows,
+                                        int kv_offset, const umb_attn_mask_t* mask, float* logits, int logits_from_row,
+                                        unsigned long long* argmax_keys, umb_stream_t stream) {
     UMB_CHECK_ARG(m && input_ids && position_ids && mask && rows >= 1 && kv_offset >= 0);
     UMB_CHECK_ARG(m->layers && m->embed && m->final_norm && m->cos && m->sin && m->k_cache && m->v_cache);
     UMB_CHECK_ARG(m->hidden && m->normed && m->qkv && m->q_rot && m->attn_out && m->act && m->gemm_ws);
     UMB_CHECK_ARG(kv_offset + rows <= m->max_length);
     UMB_CHECK_ARG(!argmax_keys || logits);
     if (logits) UMB_CHECK_ARG(m->lm_head != nullptr);
-    // rows > 128 (prefill, dynamic trees of 257..505 nodes): equal chunks of <= 128 rows, each a full pass
+    UMB_CHECK_ARG(rows_per_pass >= 1 && rows_per_pass <= (m->awq ? umb::kChunkRowsAwq : umb::kChunkRows));
+    // more rows than a pass takes (prefill, dynamic trees of 257..505 nodes): equal chunks, each a full pass
     // over the weights; later chunks see the KV rows the earlier ones appended.
-    const int n_chunks = (rows + umb::kChunkRows - 1) / umb::kChunkRows;
+    const int n_chunks = (rows + rows_per_pass - 1) / rows_per_pass;
     const int chunk = (rows + n_chunks - 1) / n_chunks;
     for (int r0 = 0; r0 < rows; r0 += chunk) {
         const int n = rows - r0 < chunk ? rows - r0 : chunk;
@@ -168,11 +173,19 @@ extern "C" int umb_llama_forward(const umb_llama_t* m, const int64_t* input_ids,
     return UMB_OK;
 }
 
-extern "C" int umb_llama_forward_range(const umb_llama_t* m, const int64_t* input_ids, const int64_t* position_ids,
-                                       int rows, int kv_offset, const umb_attn_mask_t* mask, int layer_begin,
+extern "C" int umb_llama_forward(const umb_llama_t* m, const int64_t* input_ids, const int64_t* position_ids, int rows,
+                                 int kv_offset, const umb_attn_mask_t* mask, float* logits, int logits_from_row,
+                                 unsigned long long* argmax_keys, umb_stream_t stream) {
+    return umb_llama_forward_passes(m, umb::kChunkRows, input_ids, position_ids, rows, kv_offset, mask, logits, logits_from_row, argmax_keys,
+                                    stream);
+}
+
+extern "C" int umb_llama_forward_range_passes(const umb_llama_t* m, int rows_per_pass, const int64_t* input_ids, const int64_t* position_ids,
+                                              int rows, int kv_offset, const umb_attn_mask_t* mask, int layer_begin,
                                        int layer_end, int do_embed, float* logits, int logits_from_row,
                                        unsigned long long* argmax_keys, umb_stream_t stream) {
-    UMB_CHECK_ARG(m && input_ids && position_ids && mask && rows >= 1 && rows <= 128 && kv_offset >= 0);
+    UMB_CHECK_ARG(m && input_ids && position_ids && mask && rows >= 1 && kv_offset >= 0);
+    UMB_CHECK_ARG(rows <= rows_per_pass && rows_per_pass <= (m->awq ? umb::kChunkRowsAwq : umb::kChunkRows));
     UMB_CHECK_ARG(m->layers && m->embed && m->final_norm && m->cos && m->sin && m->k_cache && m->v_cache);
     UMB_CHECK_ARG(m->hidden && m->normed && m->qkv && m->q_rot && m->attn_out && m->act && m->gemm_ws);
     UMB_CHECK_ARG(kv_offset + rows <= m->max_length);
@@ -181,6 +194,14 @@ extern "C" int umb_llama_forward_range(const umb_llama_t* m, const int64_t* inpu
     if (logits) UMB_CHECK_ARG(m->lm_head != nullptr && logits_from_row >= 0 && logits_from_row < rows);
     return umb::forward_chunk(m, input_ids, position_ids, rows, kv_offset, mask, logits, logits_from_row, argmax_keys,
                               stream, nullptr, layer_begin, layer_end, do_embed != 0);
+}
+
+extern "C" int umb_llama_forward_range(const umb_llama_t* m, const int64_t* input_ids, const int64_t* position_ids,
+                                       int rows, int kv_offset, const umb_attn_mask_t* mask, int layer_begin,
+                                       int layer_end, int do_embed, float* logits, int logits_from_row,
+                                       unsigned long long* argmax_keys, umb_stream_t stream) {
+    return umb_llama_forward_range_passes(m, umb::kChunkRows, input_ids, position_ids, rows, kv_offset, mask, layer_begin, layer_end, do_embed,
+                                          logits, logits_from_row, argmax_keys, stream);
 }
 
 extern "C" int umb_llama_forward_dyn(const umb_llama_t* m, const int64_t* tokens_base, const int64_t* position_base,

@@ -6,7 +6,7 @@
 //
 // Orientation ("swap-AB"): the verify pass multiplies M <= 128 token rows by a huge weight matrix,
 // so the WEIGHTS are the UMMA A operand (128 output features per tile = the 128 TMEM lanes) and the
-// token rows are the UMMA B/N operand (N = M padded to 16/32/64/128):
+// token rows are the UMMA B/N operand (N = M padded to 16/32/64; fp16 weights 128 too, AWQ beyond 64 rows: gemm_wide.cu):
 //     D[128 features, MPAD tokens] (fp32, TMEM) += A[128, k] * B[MPAD, k]^T .
 // Every weight byte is read from HBM exactly once per call.
 //
@@ -29,19 +29,11 @@
 #include <stdlib.h>
 
 #include "common.cuh"
+#include "gemm_core.cuh"
 #include "internal.h"
 
 namespace umb {
 
-constexpr int kTileN = 128;              // output features per tile (UMMA M)
-constexpr int kGroup = 128;              // AWQ group size == k per AWQ unit
-constexpr int kRecordBytes = 8512;       // 8192 nibble bytes + 256 scale bytes + 64 zero bytes (what a TMA copy moves)
-#ifndef UMB_RECORD_STRIDE
-#define UMB_RECORD_STRIDE 8512
-#endif
-constexpr int kRecordStride = UMB_RECORD_STRIDE;   // distance between records in the stream
-constexpr int kRecScaleOff = 8192;
-constexpr int kRecZeroOff = 8448;
 #ifndef UMB_DQ_GROUPS
 #define UMB_DQ_GROUPS 3
 #endif
@@ -61,24 +53,10 @@ constexpr int kTmemCols = 512;
 #define UMB_WAIT(bar, parity) mbar_wait(bar, parity)
 #define UMB_WAIT_LONG(bar, parity) mbar_wait(bar, parity)
 #endif
-#ifndef UMB_X_3D
-#define UMB_X_3D 1                         // 1: one 3-D tensor copy per x slab (both 64-k atoms) instead of two 2-D copies (AWQ)
-#endif
-#ifndef UMB_W_PAIR
-#define UMB_W_PAIR 0                       // 1: the weight producer requests two records per cp.async.bulk (AWQ)
-#endif
-#ifndef UMB_X_PRODUCER
-#define UMB_X_PRODUCER 0                   // 1: the x slabs are requested by their own warp (AWQ), not by the weight producer
-#endif
 // Pipeline variants that were built, measured on B200 and rejected (sleeping mbarrier polls in the idle warps,
 // software-pipelined dequant, x slabs ahead of the weight ring, early residual fetch / early partial-sum
 // reduction, a fourth dequant group) are recorded in profiles/r1_gemm_experiments.txt; none beat this form,
 // whose steady state is bound by the fp16x2 issue rate of the dequant warps (scripts/ubench/pipe_rates.cu).
-
-// nibble position of the i-th of 8 consecutive values inside a 32-bit word: (0,4,1,5,2,6,3,7).
-// Used by the AutoAWQ checkpoint layout (along N) and by our repacked stream (along K): nibbles p
-// and p + 4 hold consecutive values, so (w >> 4p) & 0x000f000f yields an ordered pair.
-__host__ __device__ __forceinline__ int nib_pos(int i) { return (i >> 1) + ((i & 1) << 2); }
 
 // ------------------------------------------------------------------------------------------------
 // repack / dequantize / unpack
@@ -170,78 +148,6 @@ __global__ void awq_unpack_kernel(const unsigned char* __restrict__ packed, int 
     *reinterpret_cast<uint4*>(out + (int64_t)pr * K + k0) = o.u;
 }
 
-// ------------------------------------------------------------------------------------------------
-// stream-K schedule helpers
-// ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ long long sk_begin(long long c, long long U, long long P) { return c * U / P; }
-__device__ __forceinline__ int sk_owner(long long u, long long U, long long P) {
-    long long c = u * P / U;
-    while (c + 1 < P && sk_begin(c + 1, U, P) <= u) ++c;
-    while (c > 0 && sk_begin(c, U, P) > u) --c;
-    return (int)c;
-}
-
-// One 32-bit word of the packed stream = 8 consecutive k of one feature row, nibble i at position
-// (0,4,1,5,2,6,3,7)[i].  Nibbles p and p+4 are extracted together as an fp16 pair:
-//   p = 0: (w      & 0x000f000f) | 0x6400 = 1024 +    q      p = 1: (w      & 0x00f000f0) | 0x6400 = 1024 + 16 q
-//   p = 2: (w >> 8 & 0x000f000f) | 0x6400                     p = 3: (w >> 8 & 0x00f000f0) | 0x6400
-// then   even: (1024 + q) - (1024 + z)        odd: (1024 + 16 q) * (1/16) - (64 + z)
-// are both EXACT (q - z), and one multiply by the group scale rounds once: fp16((q - z) * s).
-template <uint32_t kMask>
-__device__ __forceinline__ uint32_t lop3_and_or(uint32_t a, uint32_t c) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "n"(kMask), "r"(c));
-    return d;
-}
-__device__ __forceinline__ __half2 as_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
-__device__ __forceinline__ uint32_t as_u32(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
-__device__ __forceinline__ void dequant_word(uint32_t w, uint32_t magic, __half2 ce, __half2 neg_co, __half2 s2,
-                                             uint32_t* out) {
-    const __half2 sixteenth = as_h2(0x2C002C00u);                 // 1/16
-    const uint32_t w8 = w >> 8;
-    // (t - ce) and fma(t, 1/16, -co) are exact; the multiply by the scale is the single rounding
-    out[0] = as_u32(__hmul2(__hsub2(as_h2(lop3_and_or<0x000f000fu>(w, magic)), ce), s2));
-    out[1] = as_u32(__hmul2(__hfma2(as_h2(lop3_and_or<0x00f000f0u>(w, magic)), sixteenth, neg_co), s2));
-    out[2] = as_u32(__hmul2(__hsub2(as_h2(lop3_and_or<0x000f000fu>(w8, magic)), ce), s2));
-    out[3] = as_u32(__hmul2(__hfma2(as_h2(lop3_and_or<0x00f000f0u>(w8, magic)), sixteenth, neg_co), s2));
-}
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-    return v;
-}
-__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-    return v;
-}
-__device__ __forceinline__ uint32_t lds16(uint32_t addr) {
-    unsigned short v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
-    return v;
-}
-
-struct GemmParams {
-    const unsigned char* packed;   // AWQ stream (kAwq) -- else unused
-    int M, K, N_total;             // N_total = output features (rows of W)
-    int units_per_tile;            // K / 128 (AWQ) or K / 64 (fp16)
-    int tiles;
-    void* y;
-    int64_t ldy;
-    int mode;
-    const __half* bias;
-    const __half* residual;
-    int64_t ld_residual;
-    int vec_ok;                    // y (and the residual) can be accessed with 16-byte vectors
-    int rope_vec_ok;               // same for q_out / k_cache / v_cache / cos / sin of UMB_EPI_ROPE_QKV
-    unsigned long long* argmax;
-    int* counters;                 // [tiles]
-    float* slots;                  // [tiles + grid][MPAD][128]
-    umb_rope_epilogue_t rope;      // UMB_EPI_ROPE_QKV operands (by value)
-    int stages;                    // depth of the shared-memory ring
-    unsigned long long* trace;     // debug timeline [grid][16] (UMB_GEMM_TRACE=1), else NULL
-};
-
 __device__ __forceinline__ unsigned long long gtimer() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t) : : "memory");
@@ -257,18 +163,9 @@ __device__ __forceinline__ unsigned long long gtimer() {
 
 template <int MPAD>
 struct GemmCfg {
-    // 128 rows (AWQ): weight records and x slabs in rings of their own.  A shared ring holds four units of 41 KB, and a unit
-    // occupies its place from the request over the dequantisation to the product.  The records' ring is free as soon as they
-    // are in registers, so dequantisation runs ahead of the slabs: 500 rows through a layer of width 4096 and its head
-    // 887 -> 849 us; with the heads of split tiles reduced by every group of warps (below) 683.
-    static constexpr bool kSplit = MPAD >= 128;
-    // dequant groups per CTA (AWQ).  kSplit takes two: every ring depth is a multiple of it, so a stage always comes back to
-    // the group that used it last, which the parity waits need there (see the dequant warps' note)
-    static constexpr int kDq = MPAD == 16 ? UMB_DQ_GROUPS_16 : (kSplit ? 2 : kDqGroups);
-    static constexpr bool kXWarp = UMB_X_PRODUCER || kSplit;                        // x slabs are requested by their own warp
-    static constexpr int kWStages = 6;                                              // records held with kSplit
-    static constexpr int kThreadsAwq = 96 + 128 * (kDq + 1) + (kXWarp ? 32 : 0);
-    static constexpr int kStagesAwq = MPAD == 16 ? 10 : (MPAD == 32 ? 8 : (MPAD == 64 ? 6 : 4));
+    static constexpr int kDq = MPAD == 16 ? UMB_DQ_GROUPS_16 : kDqGroups;          // dequant groups per CTA (AWQ)
+    static constexpr int kThreadsAwq = 96 + 128 * (kDq + 1);
+    static constexpr int kStagesAwq = MPAD == 16 ? 10 : (MPAD == 32 ? 8 : 6);
     static constexpr int kStagesF16 = MPAD <= 32 ? 8 : (MPAD == 64 ? 6 : 4);
     static constexpr int kXBytesAwq = MPAD * 256;           // [2 atoms][MPAD][128 B]
     static constexpr int kXBytesF16 = MPAD * 128;           // [MPAD][128 B]
@@ -289,254 +186,9 @@ struct GemmCfg {
     static constexpr int kBarBytes = 576;
     static constexpr int smem_bytes(bool awq, int stages) {
         return 1024 /*align slack*/ + kBarBytes + kExchGroups * kExchBytes +
-               (awq && kSplit ? stages * kXBytesAwq + kWStages * kPackedStride
-                              : stages * (awq ? (kXBytesAwq + kPackedStride) : (kXBytesF16 + kWBytesF16)));
+               stages * (awq ? (kXBytesAwq + kPackedStride) : (kXBytesF16 + kWBytesF16));
     }
 };
-
-__device__ __forceinline__ float silu_f(float f) { return f / (1.f + expf(-f)); }
-__device__ __forceinline__ unsigned int orderable_f32_g(float f) {
-    const unsigned int u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-
-// Epilogue of 16 token columns [m0, m0 + 16) for feature lane `fl` (0..127) of tile `tile`.  The four warps that run it
-// share the staging rows `exch` and the named barrier `bar`.
-template <int MPAD>
-__device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int tile, int fl, int m0, const float (&v)[16],
-                                               __half* exch, uint32_t bar = 2) {
-    const int n = tile * kTileN + fl;
-    if (p.mode == UMB_EPI_SILU_MUL) {
-        // lanes 0..63 hold `gate`, lanes 64..127 `up` of output features tile*64 + (fl & 63).  Both halves of the
-        // 16-row chunk are staged as fp16 (the rounding point of the reference's gate / up tensors), every thread
-        // then finishes 8 of the 16 x 64 outputs in place, and the tile leaves with one 16-byte store per thread.
-        __half* g_t = exch;                    // [16][64] gate, overwritten by the outputs
-        __half* u_t = exch + 16 * 64;          // [16][64] up
-        {
-            __half* dst = (fl < 64 ? g_t : u_t) + (fl & 63);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) dst[j * 64] = __float2half_rn(v[j]);
-        }
-        named_bar_sync(bar, 128);
-        {
-            const int col = fl & 63, r0 = fl >> 6;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int r = r0 + 2 * i;
-                const __half g = g_t[r * 64 + col];
-                const __half sl = __float2half_rn(silu_f(__half2float(g)));
-                g_t[r * 64 + col] = __hmul(sl, u_t[r * 64 + col]);
-            }
-        }
-        named_bar_sync(bar, 128);
-        {
-            const int row = fl >> 3, seg = (fl & 7) * 8;
-            const int no = tile * 64 + seg;
-            if (row < p.M - m0 && no + 8 <= p.N_total / 2) {
-                __half* yp = reinterpret_cast<__half*>(p.y) + (int64_t)(m0 + row) * p.ldy + no;
-                if (p.vec_ok) {
-                    *reinterpret_cast<uint4*>(yp) = *reinterpret_cast<const uint4*>(g_t + row * 64 + seg);
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) yp[c] = g_t[row * 64 + seg + c];
-                }
-            }
-        }
-        named_bar_sync(bar, 128);
-        return;
-    }
-    if (p.mode == UMB_EPI_ROPE_QKV) {
-        // q|k|v projection with RoPE + KV append fused: the rotation partner of feature d is d +- D/2, i.e. lane
-        // fl ^ (D/2) of the same tile (128 % D == 0); the pair is exchanged through shared memory as fp16 -- the
-        // rounding point where the reference holds the fp16 q / k / v tensors.
-        const umb_rope_epilogue_t& r = p.rope;
-        const int D = r.head_dim, half_d = D >> 1;
-        const bool n_ok = n < p.N_total;
-        __half h[16];
-        const bool has_bias = p.bias != nullptr && n_ok;
-        const __half qb = has_bias ? p.bias[n] : __float2half_rn(0.f);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            h[j] = __float2half_rn(v[j]);
-            if (has_bias) h[j] = __hadd(h[j], qb);
-            exch[j * kTileN + fl] = h[j];
-        }
-        const int base = r.n_dev ? r.n_dev[0] : 0;
-        const int mcols = p.M - m0;
-        if (p.rope_vec_ok) {
-            // Staged form: the cos / sin rows of the chunk's 16 positions are fetched with 16-byte loads by the whole
-            // group (two dependent round trips in total instead of three per token through one register), the
-            // rotated tile is finished in shared memory and leaves with two 16-byte stores per thread.
-            __half* cos_t = exch + 16 * kTileN;          // [16][D]
-            __half* sin_t = cos_t + 16 * kTileN;         // [16][D]
-            const int segs = D >> 3;                     // 16-byte segments per table row
-            const int64_t* pid = r.position_ids + (r.n_dev ? base + r.row_offset : 0) + m0;
-#pragma unroll
-            for (int it = 0; it < 2; ++it) {
-                const int sidx = fl + it * 128;
-                const int row = sidx / segs, seg = sidx - row * segs;
-                if (sidx < 16 * segs && row < mcols) {
-                    const int64_t off = pid[row] * D + seg * 8;
-                    *reinterpret_cast<uint4*>(cos_t + row * D + seg * 8) =
-                        *reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(r.cos) + off);
-                    *reinterpret_cast<uint4*>(sin_t + row * D + seg * 8) =
-                        *reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(r.sin) + off);
-                }
-            }
-            named_bar_sync(bar, 128);
-            const int head = n / D, d = n - head * D;
-            const bool rot = n_ok && head < r.num_q_heads + r.num_kv_heads;
-            __half o[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                o[j] = h[j];
-                if (rot && j < mcols) {
-                    const __half pr = exch[j * kTileN + (fl ^ half_d)];
-                    // (x * cos) + (rotate_half(x) * sin): two products and one sum, each rounded (no fma)
-                    o[j] = __hadd_rn(__hmul_rn(h[j], cos_t[j * D + d]), __hmul_rn(d < half_d ? __hneg(pr) : pr, sin_t[j * D + d]));
-                }
-            }
-            named_bar_sync(bar, 128);                  // every partner value has been read
-#pragma unroll
-            for (int j = 0; j < 16; ++j) exch[j * kTileN + fl] = o[j];
-            named_bar_sync(bar, 128);
-#pragma unroll
-            for (int it = 0; it < 2; ++it) {
-                const int sidx = fl + it * 128, row = sidx >> 4, c0 = (sidx & 15) * 8;
-                const int n0 = tile * kTileN + c0;
-                if (row < mcols && n0 + 8 <= p.N_total) {
-                    const int hd = n0 / D, d0 = n0 - hd * D, m = m0 + row;
-                    __half* dst;
-                    if (hd < r.num_q_heads) {
-                        dst = reinterpret_cast<__half*>(r.q_out) + ((int64_t)m * r.num_q_heads + hd) * D;
-                    } else {
-                        const bool is_k = hd < r.num_q_heads + r.num_kv_heads;
-                        const int kvh = hd - r.num_q_heads - (is_k ? 0 : r.num_kv_heads);
-                        dst = reinterpret_cast<__half*>(is_k ? r.k_cache : r.v_cache) +
-                              (int64_t)(base + r.kv_offset + m) * r.kv_tok_stride + (int64_t)kvh * r.kv_head_stride;
-                    }
-                    *reinterpret_cast<uint4*>(dst + d0) = *reinterpret_cast<const uint4*>(exch + row * kTileN + c0);
-                }
-            }
-            named_bar_sync(bar, 128);
-            return;
-        }
-        named_bar_sync(bar, 128);
-        if (n_ok) {
-            const int head = n / D, d = n - head * D;
-            const bool rot = head < r.num_q_heads + r.num_kv_heads;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                if (j >= mcols) continue;
-                const int m = m0 + j;
-                __half o = h[j];
-                if (rot) {
-                    const int64_t pos = r.position_ids[(r.n_dev ? base + r.row_offset : 0) + m];
-                    const __half c = reinterpret_cast<const __half*>(r.cos)[pos * D + d];
-                    const __half sn = reinterpret_cast<const __half*>(r.sin)[pos * D + d];
-                    const __half pr = exch[j * kTileN + (fl ^ half_d)];
-                    // (x * cos) + (rotate_half(x) * sin): two products and one sum, each rounded (no fma)
-                    o = __hadd_rn(__hmul_rn(h[j], c), __hmul_rn(d < half_d ? __hneg(pr) : pr, sn));
-                }
-                __half* dst;
-                if (head < r.num_q_heads) {
-                    dst = reinterpret_cast<__half*>(r.q_out) + ((int64_t)m * r.num_q_heads + head) * D;
-                } else {
-                    const bool is_k = head < r.num_q_heads + r.num_kv_heads;
-                    const int kvh = head - r.num_q_heads - (is_k ? 0 : r.num_kv_heads);
-                    dst = reinterpret_cast<__half*>(is_k ? r.k_cache : r.v_cache) +
-                          (int64_t)(base + r.kv_offset + m) * r.kv_tok_stride + (int64_t)kvh * r.kv_head_stride;
-                }
-                dst[d] = o;
-            }
-        }
-        named_bar_sync(bar, 128);
-        return;
-    }
-    const bool n_ok = n < p.N_total;
-    const int mcols = p.M - m0;                       // valid token columns of this chunk (may exceed 16)
-    // fp16 outputs (plain store / residual add): the 16 x 128 tile goes through shared memory so that global memory
-    // is touched with two independent 16-byte accesses per thread instead of one 2-byte access per token row.
-    // Written as the plain per-row loop the residual loads compile into 13 serialised L2 round trips (4.2 us on the
-    // tail of every o-proj / down-proj launch) and the stores into ~500 dependent instructions
-    // (profiles/r1_gemm_tail_trace.txt).  y may alias the residual: all loads of the tile complete before any store.
-    if ((p.mode == UMB_EPI_STORE || p.mode == UMB_EPI_RESIDUAL) && p.vec_ok) {
-        const bool resid = p.mode == UMB_EPI_RESIDUAL;
-        int row[2], col[2];
-        bool ok[2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int idx = fl + i * 128;
-            row[i] = idx >> 4;
-            col[i] = (idx & 15) * 8;
-            ok[i] = row[i] < mcols && tile * kTileN + col[i] + 8 <= p.N_total;
-        }
-        if (resid) {
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-                if (ok[i])
-                    *reinterpret_cast<uint4*>(exch + row[i] * kTileN + col[i]) = *reinterpret_cast<const uint4*>(
-                        p.residual + (int64_t)(m0 + row[i]) * p.ld_residual + tile * kTileN + col[i]);
-            named_bar_sync(bar, 128);
-        }
-        const __half bb = (p.bias && n_ok) ? p.bias[n] : __float2half_rn(0.f);
-        __half h[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            h[j] = __float2half_rn(v[j]);
-            if (p.bias) h[j] = __hadd(h[j], bb);
-            if (resid) h[j] = __hadd(exch[j * kTileN + fl], h[j]);
-        }
-        if (resid) named_bar_sync(bar, 128);            // every thread has read its residual column
-#pragma unroll
-        for (int j = 0; j < 16; ++j) exch[j * kTileN + fl] = h[j];
-        named_bar_sync(bar, 128);
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-            if (ok[i])
-                *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(p.y) + (int64_t)(m0 + row[i]) * p.ldy + tile * kTileN + col[i]) =
-                    *reinterpret_cast<const uint4*>(exch + row[i] * kTileN + col[i]);
-        named_bar_sync(bar, 128);                       // the staging tile is free for the next chunk
-        return;
-    }
-    if (!n_ok && !(p.mode == UMB_EPI_LOGITS && p.argmax)) return;
-    const __half b = (p.bias && n_ok) ? p.bias[n] : __float2half_rn(0.f);
-    // residual rows first, all loads in flight together: y may alias residual, so a load placed after a
-    // store of the previous row would be serialised behind it (one L2 round trip per token row)
-    __half res[16];
-    if (p.mode == UMB_EPI_RESIDUAL) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-            if (j < mcols) res[j] = p.residual[(int64_t)(m0 + j) * p.ld_residual + n];
-    }
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        if (j >= mcols) continue;
-        const int m = m0 + j;
-        __half h = __float2half_rn(v[j]);
-        if (p.bias) h = __hadd(h, b);
-        if (p.mode == UMB_EPI_RESIDUAL) {
-            h = __hadd(res[j], h);
-            reinterpret_cast<__half*>(p.y)[(int64_t)m * p.ldy + n] = h;
-        } else if (p.mode == UMB_EPI_LOGITS) {
-            const float f = __half2float(h);
-            if (n_ok) reinterpret_cast<float*>(p.y)[(int64_t)m * p.ldy + n] = f;
-            if (p.argmax) {
-                // warp-level max first: one atomic per (warp, token)
-                unsigned long long key =
-                    n_ok ? (((unsigned long long)orderable_f32_g(f) << 32) | (unsigned int)(~n)) : 0ull;
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    const unsigned long long other = __shfl_xor_sync(0xffffffffu, key, o);
-                    key = other > key ? other : key;
-                }
-                if ((threadIdx.x & 31) == 0) atomicMax(p.argmax + m, key);
-            }
-        } else {
-            reinterpret_cast<__half*>(p.y)[(int64_t)m * p.ldy + n] = h;
-        }
-    }
-}
 
 // v[j] = sum over the accumulators of column (m0 + j), in a fixed order (deterministic).  The
 // accumulators are split between the two MMA warps (first / second half); `use_mask` bit w tells
@@ -565,8 +217,6 @@ __device__ __forceinline__ void load_acc_sum(uint32_t taddr, float (&v)[16], int
 //                 soon as a weight record has landed, also before the predecessor kernel has finished
 //   last 4 warps  epilogue only (AWQ: warps 15..18, fp16: warps 3..6): the partial-tile fix-up is a chain of
 //                 global round trips and must not stall the dequant stream
-//   65..128 rows  (AWQ) two dequant groups, warps 3..10, which also reduce when they have no units left; epilogue warps
-//                 11..14; warp 15 requests the x slabs
 template <int MPAD, bool kAwq>
 __global__ void __launch_bounds__(kAwq ? GemmCfg<MPAD>::kThreadsAwq : kGemmThreadsF16, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
@@ -574,9 +224,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
     using Cfg = GemmCfg<MPAD>;
     const int kStages = p.stages;
     constexpr int kXBytes = kAwq ? Cfg::kXBytesAwq : Cfg::kXBytesF16;
-    // paired weight requests: two records of the stream land back to back, so the shared-memory stride is the record's
-    constexpr bool kPair = kAwq && UMB_W_PAIR && kRecordStride == kRecordBytes;
-    constexpr int kWStride = kAwq ? (kPair ? kRecordBytes : Cfg::kPackedStride) : Cfg::kWBytesF16;
+    constexpr int kWStride = kAwq ? Cfg::kPackedStride : Cfg::kWBytesF16;
     constexpr uint32_t kWTxBytes = kAwq ? (uint32_t)kRecordBytes : (uint32_t)Cfg::kWBytesF16;
     constexpr uint32_t kIdesc = umma_idesc_f16(kTileN, MPAD);
     constexpr int kNumAcc = Cfg::kNumAcc;                       // >= 2, even
@@ -587,10 +235,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
     // the MMA warps take alternate units, so a ring stage must always come back to the same warp (parity waits, see the
     // dequant warps' note): both rings need an even depth
     static_assert(!kAwq || (kAStages % 2 == 0 && Cfg::kStagesAwq % 2 == 0), "ring depths must be even");
-    constexpr bool kSplit = kAwq && Cfg::kSplit, kShare = kAwq && Cfg::kShare, kXWarp = kAwq && Cfg::kXWarp;
-    static_assert(!kSplit || (kAStages % Cfg::kDq == 0 && Cfg::kWStages % Cfg::kDq == 0 && Cfg::kStagesAwq == kAStages),
-                  "the rings of separate records must return each stage to its dequant group");
-    const int kWRing = kSplit ? Cfg::kWStages : kStages;        // depth of the weight records' ring
+    constexpr bool kShare = kAwq && Cfg::kShare;
     constexpr int kDq = Cfg::kDq;                               // dequant groups of this CTA
     constexpr int kFinish = kShare ? Cfg::kExchGroups : 1;      // groups of warps that reduce the head of a split tile
 
@@ -598,7 +243,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* s_x = smem;                                   // kStages x kXBytes   (1024-aligned slabs)
     unsigned char* s_w = s_x + kStages * kXBytes;                // kStages x kWStride
-    __half* s_exch = reinterpret_cast<__half*>(s_w + kWRing * kWStride);
+    __half* s_exch = reinterpret_cast<__half*>(s_w + kStages * kWStride);
     uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(s_exch) + Cfg::kExchGroups * Cfg::kExchBytes);
     uint64_t* full_w = bars;                  // [kStages]   weight record / tile landed
     uint64_t* full_x = bars + 16;             // [kStages]   x slab landed
@@ -608,7 +253,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
     uint64_t* acc_empty = bars + 57;
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 58);
     uint64_t* last_full = bars + 59;          //             kShare: the last segment's accumulators are complete
-    uint64_t* w_empty = bars + 60;            // [kWStages]  kSplit: the record in this stage is in the dequant group's registers
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) UMB_TRACE(0);
@@ -620,15 +264,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
 
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(&tmap_x);
-        if (!kAwq || UMB_X_3D) tma_prefetch_desc(&tmap_w);
+        tma_prefetch_desc(&tmap_w);
         for (int i = 0; i < kStages; ++i) {
-            if (!kSplit) mbar_init(full_w + i, 1);
+            mbar_init(full_w + i, 1);
             mbar_init(full_x + i, 1);
             mbar_init(done + i, 1);
-        }
-        for (int i = 0; kSplit && i < kWRing; ++i) {
-            mbar_init(full_w + i, 1);
-            mbar_init(w_empty + i, 4);
         }
         for (int i = 0; i < kAStages; ++i) mbar_init(a_full + i, 4);
         mbar_init(acc_full, 2);
@@ -651,7 +291,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
         // ===================== TMA producer (whole warp runs the loop, one elected lane issues) =====================
         const uint64_t pol_w = l2_policy_evict_first(), pol_x = l2_policy_evict_last();
         const unsigned char* src = p.packed + (kAwq ? u_begin * kRecordStride : 0);
-        const int n_pre = n_units < kWRing ? n_units : kWRing;
+        const int n_pre = n_units < kStages ? n_units : kStages;
         // The weight copies of the whole ring are requested before griddepcontrol.wait (they never depend on the
         // stream predecessor), the x slabs after it.  (Requesting only a few records early, so that the first x
         // slab does not queue behind ~85 KB of weights, starts the first MMA 2 us sooner but measured no faster:
@@ -666,14 +306,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                 tma_tensor2d_g2s(s_w + stage * kWStride, &tmap_w, g * 64, tile * kTileN, full_w + stage, pol_w);
         };
         auto issue_x = [&](int stage, int gk) {
-            if (kXWarp) return;                                   // requested by the x-producer warp
             mbar_arrive_expect_tx(full_x + stage, (uint32_t)kXBytes);
             unsigned char* xs = s_x + stage * kXBytes;
-            if constexpr (kAwq && UMB_X_3D) {
+            if constexpr (kAwq) {
                 tma_tensor3d_g2s(xs, &tmap_w, 0, 0, gk * 2, full_x + stage, pol_x);      // tmap_w = x as [64, rows, K / 64]
-            } else if constexpr (kAwq) {
-                tma_tensor2d_g2s(xs, &tmap_x, gk * kGroup, 0, full_x + stage, pol_x);
-                tma_tensor2d_g2s(xs + MPAD * 128, &tmap_x, gk * kGroup + 64, 0, full_x + stage, pol_x);
             } else {
                 tma_tensor2d_g2s(xs, &tmap_x, gk * 64, 0, full_x + stage, pol_x);
             }
@@ -685,51 +321,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                 ++tile;
             }
         };
-        if constexpr (kPair) {
-            // One request per PAIR of units (17 KB): a thread gets a cp.async.bulk out every ~230 ns whatever its size
-            // (scripts/ubench/tma_rates.cu), so single records cap an SM at 37 GB/s (5.4 TB/s for the chip).  Stages
-            // 2j and 2j + 1 share the barrier full_w[2j]; kStages is even and the ring starts at stage 0, so pairs
-            // never straddle the wrap.
-            auto issue_pair = [&](int stage, int cnt) {
-                mbar_arrive_expect_tx(full_w + stage, (uint32_t)(kRecordBytes * cnt));
-                tma_bulk_g2s(s_w + stage * kWStride, src, (uint32_t)(kRecordBytes * cnt), full_w + stage, pol_w);
-            };
-            for (int i = 0; i < n_pre; i += 2) {                 // weights first: independent of the predecessor
-                const int cnt = n_pre - i >= 2 ? 2 : 1;
-                if (elect_one()) issue_pair(i, cnt);
-                __syncwarp();
-                src += (size_t)kRecordStride * cnt;
-            }
-            if (lane == 0) UMB_TRACE(2);
-            pdl_wait();                                          // x is the predecessor's output
-            if (lane == 0) UMB_TRACE(3);
-            int gx = in_tile0;
-            for (int i = 0; i < n_pre; ++i) {
-                if (elect_one()) issue_x(i, gx);
-                __syncwarp();
-                if (++gx == p.units_per_tile) gx = 0;
-            }
-            int stage = 0, use = 1;
-            for (int i = n_pre; i < n_units; i += 2) {
-                const int cnt = n_units - i >= 2 ? 2 : 1;
-                UMB_WAIT(done + stage, (use - 1) & 1);          // the units that last used these stages have retired
-                if (cnt == 2) UMB_WAIT(done + stage + 1, (use - 1) & 1);
-                if (elect_one()) {
-                    issue_pair(stage, cnt);
-                    issue_x(stage, gx);
-                    if (cnt == 2) issue_x(stage + 1, gx + 1 == p.units_per_tile ? 0 : gx + 1);
-                }
-                __syncwarp();
-                src += (size_t)kRecordStride * cnt;
-                for (int c = 0; c < cnt; ++c)
-                    if (++gx == p.units_per_tile) gx = 0;
-                stage += 2;
-                if (stage >= kStages) {
-                    stage = 0;
-                    ++use;
-                }
-            }
-        } else {
         for (int i = 0; i < n_early; ++i) {                      // weights first: independent of the predecessor
             if (elect_one()) issue_w(i);
             __syncwarp();
@@ -755,43 +346,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
         Ring r;
         r.phase = 1;                                             // every stage has been used once
         for (int i = n_pre; i < n_units; ++i) {
-            // the unit that last used this stage has retired (kSplit: its record has been read)
-            if constexpr (kSplit) UMB_WAIT(w_empty + r.stage, r.phase ^ 1);
-            else UMB_WAIT(done + r.stage, r.phase ^ 1);
+            UMB_WAIT(done + r.stage, r.phase ^ 1);               // the unit that last used this stage has retired
             if (elect_one()) {
                 issue_w(r.stage);
                 issue_x(r.stage, g);
             }
             __syncwarp();
             advance_w();
-            r.advance(kWRing);
-        }
+            r.advance(kStages);
         }
         if (lane == 0) UMB_TRACE(10);
-    } else if (kXWarp && warp == GemmCfg<MPAD>::kThreadsAwq / 32 - 1) {
-        // ===================== x-slab producer (AWQ, kXWarp) =====================
-        const uint64_t pol_x = l2_policy_evict_last();
-        pdl_wait();                                              // x is the predecessor's output
-        int gx = in_tile0, stage = 0, use = 0;
-        for (int i = 0; i < n_units; ++i) {
-            if (use > 0) UMB_WAIT(done + stage, (use - 1) & 1); // the unit that last used this stage has retired
-            if (elect_one()) {
-                mbar_arrive_expect_tx(full_x + stage, (uint32_t)kXBytes);
-                unsigned char* xs = s_x + stage * kXBytes;
-                if constexpr (UMB_X_3D) {
-                    tma_tensor3d_g2s(xs, &tmap_w, 0, 0, gx * 2, full_x + stage, pol_x);
-                } else {
-                    tma_tensor2d_g2s(xs, &tmap_x, gx * kGroup, 0, full_x + stage, pol_x);
-                    tma_tensor2d_g2s(xs + MPAD * 128, &tmap_x, gx * kGroup + 64, 0, full_x + stage, pol_x);
-                }
-            }
-            __syncwarp();
-            if (++gx == p.units_per_tile) gx = 0;
-            if (++stage == kStages) {
-                stage = 0;
-                ++use;
-            }
-        }
     } else if (warp <= 2) {
         // ===================== MMA issuers: warp 1 takes even CTA-local units, warp 2 odd ones =====================
         const int par = warp - 1;
@@ -942,13 +506,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                 float v[16];
                 load_acc_sum<kAccUsed, MPAD>(tmem_base + lane_addr + m0, v, use_mask);
                 reduce_others(v, m0, tile_, c_first, c_last - c_first);
-                epilogue_chunk<MPAD>(p, tile_, fl, m0, v, ex, bar);
+                epilogue_chunk(p, tile_, fl, m0, v, ex, bar);
             }
         };
         if (!is_epi) {
             // ===================== dequant warps (AWQ): group g takes CTA-local units g, g + kDqGroups, ... =====================
             if constexpr (kAwq) {
-                int dq_st = grp % kWRing, dq_ph = 0, dq_ts = grp % kAStages;      // ring positions of unit `mine`
+                int dq_st = grp % kStages, dq_ph = 0, dq_ts = grp % kAStages;      // ring positions of unit `mine`
                 int w_first = grp;                                                 // first unit of this group that re-uses a TMEM stage
                 while (w_first < kAStages) w_first += kDq;
                 int w_st = (w_first - kAStages) % kStages, w_ph = 0;               // ring position of unit `mine - kAStages`
@@ -963,19 +527,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                     zw = lds32(rec + kRecZeroOff + (fl >> 3) * 4);
                 };
                 if (grp < n_units) {
-                    UMB_WAIT(full_w + (kPair ? (dq_st & ~1) : dq_st), dq_ph);
+                    UMB_WAIT(full_w + dq_st, dq_ph);
                     if (grp == 0 && q == 0 && lane == 0) UMB_TRACE(4);
                     fetch(dq_st);
-                    if constexpr (kSplit) {
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(w_empty + dq_st);
-                    }
                 }
                 for (int mine = grp; mine < n_units; mine += kDq) {
                     const int ts = dq_ts;
                     dq_st += kDq;
-                    if (dq_st >= kWRing) {
-                        dq_st -= kWRing;
+                    if (dq_st >= kStages) {
+                        dq_st -= kStages;
                         dq_ph ^= 1;
                     }
                     dq_ts += kDq;
@@ -1011,9 +571,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                         //     done[v - kAStages] implies done[v - kStages]: both ring depths are even, so the two units were
                         //     issued and committed, in order, by the same MMA thread; a retired occupant has landed, so
                         //     full_w is at most one use behind.  (v < kAStages: first use of both stages, nothing to wait for.)
-                        //     kSplit: the producer no longer orders the records behind done, so (1) itself has to know that
-                        //     done[v - 2 kAStages] is over, and (2) that record v - kWStages was read: this group has waited
-                        //     for both itself, both depths being multiples of the number of groups.
                         if (mine + kDq >= kAStages) {
                             UMB_WAIT(done + w_st, w_ph);
                             tc_fence_after();
@@ -1023,19 +580,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                                 w_ph ^= 1;
                             }
                         }
-                        UMB_WAIT(full_w + (kPair ? (dq_st & ~1) : dq_st), dq_ph);
+                        UMB_WAIT(full_w + dq_st, dq_ph);
                         fetch(dq_st);
-                        if constexpr (kSplit) {
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(w_empty + dq_st);
-                        }
                     }
                 }
                 if constexpr (kShare) {
                     // The head of a split tile is reduced by all groups of warps, one chunk of 16 columns each in turn: a chunk
                     // waits for two or three round trips to the other CTAs' sums, 24 of them in series with one group
-                    // when five CTAs share a tile (849 -> 683 us, see kSplit; four sums in flight a thread instead of two
-                    // spill registers: 753).
+                    // when five CTAs share a tile.
                     const int tile_ = (int)((u_end - 1) / p.units_per_tile);
                     const long long tile_u0 = (long long)tile_ * p.units_per_tile;
                     const int c_first = sk_owner(tile_u0, U, P), c_last = sk_owner(tile_u0 + p.units_per_tile - 1, U, P);
@@ -1082,7 +634,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                             if (lane == 0) mbar_arrive(acc_empty);
                         }
                         if (m0 < p.M || p.mode == UMB_EPI_SILU_MUL || p.mode == UMB_EPI_ROPE_QKV)
-                            epilogue_chunk<MPAD>(p, tile, fl, m0, v, s_exch);
+                            epilogue_chunk(p, tile, fl, m0, v, s_exch);
                     }
                 } else {
                     // Partial tile.  The CTA that owns the HEAD of the tile (c_first; that part is the last
@@ -1306,22 +858,6 @@ awq_gemm_simt_kernel(const unsigned char* __restrict__ packed, const __half* __r
 // ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
-typedef CUresult (*PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static PFN_encodeTiled get_encode() {
-    static PFN_encodeTiled fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* sym = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres) == cudaSuccess &&
-            qres == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_encodeTiled>(sym);
-    }
-    return fn;
-}
 // fp16 row-major [rows, cols] (leading dimension ld elements) -> tiled map, box [64 cols, box_rows], SW128
 static int make_tmap(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
     PFN_encodeTiled enc = get_encode();
@@ -1334,22 +870,6 @@ static int make_tmap(CUtensorMap* map, const void* base, uint64_t rows, uint64_t
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return arg_fail(__FILE__, __LINE__, "cuTensorMapEncodeTiled");
-    return UMB_OK;
-}
-
-// fp16 row-major x [rows, cols] as (64 cols, rows, cols / 64 atoms): box [64, box_rows, 2] = the two 128-byte-swizzled
-// atoms of one 128-k slab in ONE copy
-static int make_tmap_x3d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
-    PFN_encodeTiled enc = get_encode();
-    if (!enc) return UMB_ERR_DRIVER;
-    const cuuint64_t dims[3] = {64, rows, cols / 64};
-    const cuuint64_t strides[2] = {ld * sizeof(__half), 64 * sizeof(__half)};
-    const cuuint32_t box[3] = {64, box_rows, 2};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return arg_fail(__FILE__, __LINE__, "cuTensorMapEncodeTiled(3d)");
     return UMB_OK;
 }
 
@@ -1381,8 +901,6 @@ static unsigned long long* trace_for_this_launch() {
     return (want < 0 || idx == want) ? buf : nullptr;
 }
 
-// Rows one launch takes (internal.h: UMB_MAX_ROWS; 64 splits 65..128 rows into two launches).
-constexpr int kMaxRowsPerLaunch = UMB_MAX_ROWS;
 static int mpad_of(int M) { return M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128)); }
 
 template <int MPAD, bool kAwq>
@@ -1394,7 +912,7 @@ static int launch_gemm(const CUtensorMap& tx, const CUtensorMap& tw, GemmParams 
             const char* e = getenv("UMB_GEMM_STAGES");
             env_stages = e ? atoi(e) : 0;
         }
-        if (env_stages > 0 && env_stages <= 16 && (env_stages % 2) == 0 && !(kAwq && GemmCfg<MPAD>::kSplit) && GemmCfg<MPAD>::smem_bytes(kAwq, env_stages) <= 227 * 1024)
+        if (env_stages > 0 && env_stages <= 16 && (env_stages % 2) == 0 && GemmCfg<MPAD>::smem_bytes(kAwq, env_stages) <= 227 * 1024)
             p.stages = env_stages;                                   // even: see the static_assert on the ring depths
     }
     p.trace = trace_for_this_launch();
@@ -1412,34 +930,7 @@ static int gemm_common(bool awq, const void* x, int64_t ldx, const void* w, int6
                        cudaStream_t st) {
     UMB_CHECK_ARG(x && w && y && M >= 1 && K >= 1 && N_total >= 1);
     UMB_CHECK_ARG((((uintptr_t)x | (uintptr_t)w) & 15) == 0 && (ldx % 8) == 0 && ldx >= K);
-    if (M > 128) return UMB_ERR_UNSUPPORTED;
-    if (M > kMaxRowsPerLaunch) {
-        // only with -DUMB_MAX_ROWS=64: 65..128 rows run as two launches of <= 64 rows
-        const int m0 = kMaxRowsPerLaunch;
-        umb_epilogue_t e0{}, e1{};
-        umb_rope_epilogue_t r1{};
-        if (epi) {
-            e0 = *epi;
-            e1 = *epi;
-            const size_t esz = (e1.mode == UMB_EPI_LOGITS) ? sizeof(float) : sizeof(__half);
-            (void)esz;
-            if (e1.residual) e1.residual = (const __half*)e1.residual + (int64_t)m0 * e1.ld_residual;
-            if (e1.argmax) e1.argmax += m0;
-            if (e1.mode == UMB_EPI_ROPE_QKV && e1.rope) {
-                r1 = *e1.rope;
-                r1.q_out = (__half*)r1.q_out + (int64_t)m0 * r1.num_q_heads * r1.head_dim;
-                if (r1.n_dev) r1.row_offset += m0; else r1.position_ids += m0;
-                r1.kv_offset += m0;
-                e1.rope = &r1;
-            }
-        }
-        const bool f32 = epi && epi->mode == UMB_EPI_LOGITS;
-        int rc = gemm_common(awq, x, ldx, w, ldw, y, ldy, m0, K, N_total, epi ? &e0 : nullptr, workspace, workspace_bytes, st);
-        if (rc != UMB_OK) return rc;
-        void* y1 = f32 ? (void*)((float*)y + (int64_t)m0 * ldy) : (void*)((__half*)y + (int64_t)m0 * ldy);
-        return gemm_common(awq, (const __half*)x + (int64_t)m0 * ldx, ldx, w, ldw, y1, ldy, M - m0, K, N_total,
-                           epi ? &e1 : nullptr, workspace, workspace_bytes, st);
-    }
+    if (M > (awq ? 512 : 128)) return UMB_ERR_UNSUPPORTED;
     if (awq ? (K % kGroup) != 0 : (K % 64) != 0) return UMB_ERR_UNSUPPORTED;
     if (N_total % 8) return UMB_ERR_UNSUPPORTED;
     GemmParams p{};
@@ -1473,6 +964,14 @@ static int gemm_common(bool awq, const void* x, int64_t ldx, const void* w, int6
                 (p.mode != UMB_EPI_RESIDUAL || ((((uintptr_t)p.residual) & 15) == 0 && (p.ld_residual % 8) == 0))) ? 1 : 0;
     if (p.mode == UMB_EPI_SILU_MUL) UMB_CHECK_ARG((N_total % kTileN) == 0 && p.bias == nullptr);
 
+    if (awq && M > 64) {
+        const size_t need = awq_wide_ws_bytes(M, N_total);
+        if (!workspace || workspace_bytes < need || (M <= 128 && workspace_bytes < umb_gemm_workspace_bytes(M, K, N_total))) return UMB_ERR_WORKSPACE;
+        UMB_CHECK_ARG(((uintptr_t)workspace & 15) == 0);
+        if ((long long)(p.tiles + 1) * p.units_per_tile * 2 >= (1ll << 31)) return UMB_ERR_UNSUPPORTED;
+        p.slots = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(workspace) + (((size_t)p.tiles * 4 + 255) & ~(size_t)255));
+        return launch_awq_wide(x, ldx, p, st);
+    }
     const int mpad = mpad_of(M);
     const long long U = (long long)p.tiles * p.units_per_tile;
     if (U >= (1ll << 31)) return UMB_ERR_UNSUPPORTED;
@@ -1503,11 +1002,9 @@ static int gemm_common(bool awq, const void* x, int64_t ldx, const void* w, int6
         UMB_CHECK_ARG((ldw % 8) == 0 && ldw >= K);
         rc = make_tmap(&tw, w, (uint64_t)N_total, (uint64_t)K, (uint64_t)ldw, (uint32_t)kTileN);
         if (rc != UMB_OK) return rc;
-    } else if (UMB_X_3D) {
+    } else {
         rc = make_tmap_x3d(&tw, x, (uint64_t)M, (uint64_t)K, (uint64_t)ldx, (uint32_t)mpad);   // AWQ: tmap_w = x as slabs
         if (rc != UMB_OK) return rc;
-    } else {
-        tw = tx;
     }
     if (sync_debug())
         fprintf(stderr, "umbrella_b200: gemm awq=%d M=%d K=%d N=%d mode=%d grid=%d mpad=%d\n", (int)awq, M, K, N_total, p.mode,
@@ -1518,15 +1015,14 @@ static int gemm_common(bool awq, const void* x, int64_t ldx, const void* w, int6
         case 16: UMB_DISPATCH(16);
         case 32: UMB_DISPATCH(32);
         case 64: UMB_DISPATCH(64);
-        default:
-#if UMB_MAX_ROWS > 64
-            UMB_DISPATCH(128);
-#else
-            if (awq) return UMB_ERR_UNSUPPORTED;      // never reached: gemm_common splits more than 64 rows
-            return launch_gemm<128, false>(tx, tw, p, grid, st);
-#endif
+        default: return launch_gemm<128, false>(tx, tw, p, grid, st);
     }
 #undef UMB_DISPATCH
+}
+
+int awq_gemm_rows(const void* x, int64_t ldx, const void* packed, void* y, int64_t ldy, int M, int K, int N_total, const umb_epilogue_t* epi,
+                  void* workspace, size_t workspace_bytes, cudaStream_t st) {
+    return gemm_common(true, x, ldx, packed, 0, y, ldy, M, K, N_total, epi, workspace, workspace_bytes, st);
 }
 
 }  // namespace umb
@@ -1594,9 +1090,22 @@ extern "C" int umb_awq_unpack_f16(const void* packed, int K, int N_total, int gr
 extern "C" int umb_awq_gemm_f16(const void* x, int64_t ldx, const void* packed, void* y, int64_t ldy, int M, int K,
                                 int N_total, int group, const umb_epilogue_t* epilogue, void* workspace,
                                 size_t workspace_bytes, umb_stream_t stream) {
-    if (group != kGroup) return UMB_ERR_UNSUPPORTED;
+    if (group != kGroup || M > 128) return UMB_ERR_UNSUPPORTED;
     return gemm_common(true, x, ldx, packed, 0, y, ldy, M, K, N_total, epilogue, workspace, workspace_bytes,
                        (cudaStream_t)stream);
+}
+
+extern "C" size_t umb_awq_gemm_rows_ws_bytes(int M, int K, int N_total) {
+    if (M < 1 || M > 512 || N_total < 1) return 0;
+    const size_t few = umb_gemm_workspace_bytes(M, K, N_total), many = M > 64 ? awq_wide_ws_bytes(M, N_total) : 0;
+    return few > many ? few : many;
+}
+
+extern "C" int umb_awq_gemm_rows_f16(const void* x, int64_t ldx, const void* packed, void* y, int64_t ldy, int M, int K,
+                                     int N_total, int group, const umb_epilogue_t* epilogue, void* workspace,
+                                     size_t workspace_bytes, umb_stream_t stream) {
+    if (group != kGroup) return UMB_ERR_UNSUPPORTED;
+    return awq_gemm_rows(x, ldx, packed, y, ldy, M, K, N_total, epilogue, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 extern "C" int umb_gemm_f16(const void* x, int64_t ldx, const void* w, int64_t ldw, void* y, int64_t ldy, int M, int K,

@@ -6,14 +6,6 @@
 
 #include <utility>
 
-// Token rows one GEMM launch takes (and the forward drivers' chunk size).  It was 64 while the
-// 128-column AWQ instantiation died about once in 150-300 launches; the cause (a parity wait that could run two phases
-// ahead of its barrier in the 4-deep ring) was found and fixed -- profiles/r2_m128_root_cause.txt.
-// -DUMB_MAX_ROWS=64 restores the split into two launches.
-#ifndef UMB_MAX_ROWS
-#define UMB_MAX_ROWS 128
-#endif
-
 namespace umb {
 // Programmatic dependent launch (PDL): every kernel of the forward chain is launched with the
 // programmatic-stream-serialization attribute, so its CTAs may start (barrier init, TMEM allocation,
@@ -43,6 +35,13 @@ inline cudaError_t launch_pdl(const char* name, void (*kernel)(KArgs...), dim3 g
 #define UMB_LAUNCH_PDL(kernel, ...) do { cudaError_t e__ = umb::launch_pdl(#kernel, kernel, __VA_ARGS__); if (e__ != cudaSuccess) return (int)e__; } while (0)
 // every host entry point reports the kernels it enqueued (umb_launch_count)
 void count_launches(unsigned n);
+// gemm_wide.cu: AWQ products of 65 to 512 token rows by pairs of SMs, with a workspace of awq_wide_ws_bytes() bytes
+struct GemmParams;
+size_t awq_wide_ws_bytes(int M, int N_total);
+int launch_awq_wide(const void* x, int64_t ldx, const GemmParams& p, cudaStream_t st);
+// gemm.cu: umb_awq_gemm_f16 of up to 512 token rows
+int awq_gemm_rows(const void* x, int64_t ldx, const void* packed, void* y, int64_t ldy, int M, int K, int N_total, const umb_epilogue_t* epi,
+                  void* workspace, size_t workspace_bytes, cudaStream_t st);
 // number of SMs of the current device (cached)
 int sm_count();
 // graph-replay variants (device-resident prefix length), used by the native forward driver

@@ -22,7 +22,8 @@ import torch
 from .. import _lib, ops
 from ..attn.cache import KV_Cache
 
-MAX_ROWS = 128   # rows per forward chunk (UMMA N limit of the swap-AB GEMM)
+MAX_ROWS = 128   # rows per forward chunk of fp16 layers and of layer ranges
+AWQ_ROWS = 512   # rows per pass over AWQ layers
 
 
 @dataclass
@@ -98,6 +99,7 @@ def rope_tables(inv_freq: torch.Tensor, attention_scaling: float, max_length: in
 class Llama:
     """fp16-weight Llama (reference ``Llama``, llama.py:11-142) on the native forward."""
     awq = False
+    rows_per_pass = MAX_ROWS
 
     def __init__(self, shape: LlamaShape, max_length: int = 256, device: str = "cuda:0", dtype=torch.float16,
                  batch_size: int = 1, model_name: str | None = None, num_layers: int | None = None):
@@ -133,12 +135,12 @@ class Llama:
         self.cos_cache, self.sin_cache = cos.to(dev), sin.to(dev)
         H, I, Hq, Hkv, D = sh.hidden_size, sh.intermediate_size, self.num_heads, self.num_key_value_heads, self.head_dim
         f16 = dict(dtype=torch.float16, device=dev)
-        self._hidden = torch.zeros(MAX_ROWS, H, **f16)
-        self._normed = torch.zeros(MAX_ROWS, H, **f16)
-        self._qkv = torch.zeros(MAX_ROWS, (Hq + 2 * Hkv) * D, **f16)
-        self._q_rot = torch.zeros(MAX_ROWS, Hq * D, **f16)
-        self._attn_out = torch.zeros(MAX_ROWS, Hq * D, **f16)
-        self._act = torch.zeros(MAX_ROWS, I, **f16)
+        self._hidden = torch.zeros(self.rows_per_pass, H, **f16)
+        self._normed = torch.zeros(self.rows_per_pass, H, **f16)
+        self._qkv = torch.zeros(self.rows_per_pass, (Hq + 2 * Hkv) * D, **f16)
+        self._q_rot = torch.zeros(self.rows_per_pass, Hq * D, **f16)
+        self._attn_out = torch.zeros(self.rows_per_pass, Hq * D, **f16)
+        self._act = torch.zeros(self.rows_per_pass, I, **f16)
         lib = _lib.load()
         self._gemm_ws = torch.zeros(lib.umb_llama_gemm_ws_bytes(H, I, Hq, Hkv, D, sh.vocab_size), dtype=torch.uint8,
                                     device=dev)
@@ -245,8 +247,8 @@ class Llama:
         logits = None
         if want_logits:
             logits = torch.empty((rows - logits_from, self.config.vocab_size), dtype=torch.float32, device=self.device)
-        _lib.check(_lib.load().umb_llama_forward(
-            C.byref(self._model_struct()), C.c_void_p(ids.data_ptr()), C.c_void_p(pos.data_ptr()), rows, kv_offset,
+        _lib.check(_lib.load().umb_llama_forward_passes(
+            C.byref(self._model_struct()), self.rows_per_pass, C.c_void_p(ids.data_ptr()), C.c_void_p(pos.data_ptr()), rows, kv_offset,
             C.byref(mask), C.c_void_p(logits.data_ptr()) if logits is not None else None, logits_from,
             C.c_void_p(argmax_keys.data_ptr()) if argmax_keys is not None else None,
             C.c_void_p(torch.cuda.current_stream().cuda_stream)), "llama_forward")
@@ -342,6 +344,7 @@ class LlamaAwq(Llama):
     """AWQ INT4 Llama (reference ``LlamaAwq``, llama.py:222-322): the seven linears of a layer become
     three fused packed streams (q|k|v, gate|up interleaved for the SiLU epilogue) + o + down."""
     awq = True
+    rows_per_pass = AWQ_ROWS
 
     def load_awq_layer(self, idx: int, w: dict):
         """w[name] = (qweight int32 [K, N/8], qzeros int32 [K/g, N/8], scales fp16 [K/g, N]) for the

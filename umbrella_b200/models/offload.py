@@ -19,7 +19,7 @@ Host-side mirror of the reference's ``LlamaOffload`` / ``LlamaAwqOffload`` (umbr
     into the staging buffer every time as well, llama_layer.py:251-258).
 
 Compute is the same native path as the resident model: ``umb_llama_forward_range`` runs one layer of
-<= 128 rows per call; larger inputs keep one hidden-state buffer per 128-row chunk so the weights are
+``rows_per_pass`` rows per call; larger inputs keep one hidden-state buffer per chunk of that many so the weights are
 streamed once per forward, not once per chunk.
 """
 from __future__ import annotations
@@ -29,10 +29,9 @@ import ctypes as C
 import torch
 
 from .. import _lib, ops
-from .llama import MAX_ROWS, Llama, LlamaAwq
+from .llama import Llama, LlamaAwq
 
 _ALIGN = 256
-CHUNK_ROWS = 128     # rows per chunk of a paged forward (matches kChunkRows of csrc/forward.cu)
 _PARTS = ("wqkv", "wo", "wgu", "wdown", "input_norm", "post_norm")
 
 
@@ -152,10 +151,10 @@ class _Paged:
 
     # ------------------------------------------------------------------ forward
     def _chunk_models(self, n_chunks: int):
-        """One model struct per 128-row chunk, differing only in the hidden-state buffer."""
+        """One model struct per chunk of rows, differing only in the hidden-state buffer."""
         H = self.config.hidden_size
         if self._chunk_hidden is None or self._chunk_hidden.shape[0] < n_chunks:
-            self._chunk_hidden = torch.zeros(n_chunks, MAX_ROWS, H, dtype=torch.float16, device=self.device)
+            self._chunk_hidden = torch.zeros(n_chunks, self.rows_per_pass, H, dtype=torch.float16, device=self.device)
             self._chunk_structs = []
         base = self._model_struct()
         while len(self._chunk_structs) < n_chunks:
@@ -183,7 +182,7 @@ class _Paged:
             raise RuntimeError(f"KV cache overflow: {kv_offset} + {rows} > {self.max_length}")
         lib, cur = _lib.load(), torch.cuda.current_stream()
         st = C.c_void_p(cur.cuda_stream)
-        n_chunks = (rows + CHUNK_ROWS - 1) // CHUNK_ROWS
+        n_chunks = (rows + self.rows_per_pass - 1) // self.rows_per_pass
         chunk = (rows + n_chunks - 1) // n_chunks
         spans = [(r0, min(chunk, rows - r0)) for r0 in range(0, rows, chunk)]
         models = self._chunk_models(len(spans))
@@ -210,8 +209,8 @@ class _Paged:
             r0, n = spans[ci]
             if kvp is not None:
                 models[ci].k_cache, models[ci].v_cache = kvp.base_ptrs(l0)
-            _lib.check(lib.umb_llama_forward_range(
-                C.byref(models[ci]), C.c_void_p(ip + 8 * r0), C.c_void_p(pp + 8 * r0), n, kv_offset + r0,
+            _lib.check(lib.umb_llama_forward_range_passes(
+                C.byref(models[ci]), self.rows_per_pass, C.c_void_p(ip + 8 * r0), C.c_void_p(pp + 8 * r0), n, kv_offset + r0,
                 C.byref(masks[ci]), l0, l1, int(embed), lg, lg_from, keys, st), "llama_forward_range")
 
         for l in range(self.num_layers):
