@@ -2,10 +2,10 @@
 // in tensor memory.
 //
 // A persistent block per SM walks output tiles of 128 rows x BN columns.  Warp 0 copies weight tiles (and, for dense rows,
-// activation tiles) with TMA into a ring of 64-wide k steps, one thread of warp 1 issues tcgen05.mma, warps 2-5 empty the
-// accumulators -- two sets of them, so that a tile is stored while the next one is summed.  Rows that are gathered or sorted by
-// expert come from four more warps through 16-byte cp.async: which rows a tile has is known on the device alone, and a tile
-// of few rows fetches only those.
+// activation tiles) with TMA into a ring of 64-wide k steps, one thread of warp 1 issues tcgen05.mma, four or eight more empty the
+// accumulators -- two sets of them, so that a tile is stored while the next one is summed.  Which rows a tile has of those that are gathered or
+// sorted by expert is known on the device alone: a full tile of neighbouring rows is one box for a warp more, a tile of few rows comes four rows at a time
+// from its lanes (tile::gather4), the others through 16-byte cp.async from four to eight more warps.
 //
 // An output element is one fp32 sum over k in the same order whatever its tile's size, so a row's result does not depend on
 // the rest of the batch; against float64 it is as far off as the mma.sync tiles that this replaced (2.1e-6 at K = 2048, in
@@ -13,16 +13,20 @@
 //
 // Bound for dense prompts: a block's shared memory, 48 KB in and 48 KB out for 512 clocks of products at 256 columns (690 clocks a step); the
 // large ones go to pairs of SMs (seq_gemm_pair.cu).  With few steps: launch, first operands, last results (8.0 us for K = 1024 to 1024
-// columns, 3.8 of them steps).  16 experts, top 2, 4096 tokens of width 2048 with the routing around it: 808 us on mma.sync tiles, 232 here,
-// 207 without clearing the results first (gate|up 890 clocks a step: the copying warps' loads); 64 tokens: 213 -> 99 -> 86 us (gate|up at
-// the memory's rate inside: 134 MB in 23.5 us).
+// columns, 3.8 of them steps).  Sorted rows: the copying warps' loads (890 clocks a step of gathered ones; leaving them out: 7 us of 193) and the results
+// (25 us of 193 with four warps that store).  16 experts, top 2, of width 2048 with the routing around it, us, four warps that store and all rows copied
+// / this: 64 tokens 85 / 73, 200 98 / 82, 500 101 / 89, 4096 206 / 200; gate|up of 64 tokens reads its 134 MB at the memory's rate.
 #include <cuda.h>
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 
 #include "seq_gemm_walk.cuh"
 
 namespace umbs {
+
+// Up to so many rows of a tile come by tile::gather4: four rows cost the copy engine 60 clocks, 128 rows 1900 a k step where 64 threads' copies take 890.
+constexpr int kTcGather = 40;
 
 template <int BN, bool DUAL>
 struct TcCfg {
@@ -31,21 +35,36 @@ struct TcCfg {
     // (Warps that serve the stages in turn publish one only when they come back for another: 1.5 us per k step, a round trip
     // between the tensor core and the copies.)
     static constexpr int kWarpsPerStage = BN == 256 ? 2 : 1, kCopyWarps = kStages * kWarpsPerStage;
-    static constexpr int threads(bool a_tma) { return a_tma ? 192 : 192 + 32 * kCopyWarps; }
+    // Warps that store: at 256 columns eight, half of the columns each four, 16 at a time (their staging blocks fit beside four stages).
+    static constexpr int kStore = BN == 256 ? 8 : 4, kStoreCols = BN == 256 ? 16 : 32, kStoreBlock = 32 * (kStoreCols + 4);
+    static constexpr int threads(bool dense) { return 64 + 32 * kStore + (dense ? 0 : 32 * (1 + kCopyWarps)); }
     static constexpr int kABytes = kTcRows * 128, kWBytes = BN * 128, kStage = kABytes + kWBytes;
     static constexpr int kOut = DUAL ? BN / 2 : BN;         // output columns of a tile
-    static constexpr int kSmem = 1024 + kStages * kStage + 4 * 32 * kTcStageRow * 4 + 256 + kCopyWarps * kTcRows * 4;
+    static constexpr int kSmem = 1024 + kStages * kStage + kStore * kStoreBlock * 4 + 256 + kCopyWarps * kTcRows * 4;
 };
 
-template <int BN, bool DUAL, bool A_TMA, typename TC>
-__global__ void __launch_bounds__(TcCfg<BN, DUAL>::threads(A_TMA), 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const GemmArgs a, const TcArgs t) {
+__device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap* map, int c, int r0, int r1, int r2, int r3, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+                 ::"r"(dst), "l"(map), "r"(c), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(smem_u32(bar)) : "memory");
+}
+
+// how the rows of a tile that is gathered or sorted come
+enum { kTcCopied, kTcBox, kTcByFours };
+__device__ __forceinline__ int tc_rows_kind(const GemmArgs& a, const TcArgs& t, int rows) {
+    if (!t.maps) return kTcCopied;
+    if (rows <= kTcGather) return kTcByFours;
+    return a.row_src == nullptr && rows == kTcRows ? kTcBox : kTcCopied;
+}
+
+template <int BN, bool DUAL, bool DENSE, typename TC>
+__global__ void __launch_bounds__(TcCfg<BN, DUAL>::threads(DENSE), 1)
+gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_r, const __grid_constant__ CUtensorMap map_w, const GemmArgs a, const TcArgs t) {
     using Cfg = TcCfg<BN, DUAL>;
     constexpr int kStages = Cfg::kStages, kOut = Cfg::kOut;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     float* s_out = reinterpret_cast<float*>(smem + kStages * Cfg::kStage);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(s_out + 4 * 32 * kTcStageRow);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(s_out + Cfg::kStore * Cfg::kStoreBlock);
     uint64_t *full = bars, *empty = bars + kStages, *acc_full = bars + 2 * kStages, *acc_empty = acc_full + 2;
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* quit = reinterpret_cast<volatile int*>(s_tmem + 1);
@@ -53,14 +72,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
     if (threadIdx.x == 0) {
         umb::tma_prefetch_desc(&map_w);
-        if (A_TMA) umb::tma_prefetch_desc(&map_a);
+        if (DENSE || t.maps) umb::tma_prefetch_desc(&map_a);
         for (int i = 0; i < kStages; ++i) {
-            umb::mbar_init(full + i, A_TMA ? 1 : 1 + Cfg::kWarpsPerStage);          // the TMA thread, and the stage's copying warps
+            umb::mbar_init(full + i, DENSE ? 1 : 2 + Cfg::kWarpsPerStage);         // the TMA thread, warp 6 and the stage's copying warps
             umb::mbar_init(empty + i, 1);
         }
         for (int i = 0; i < 2; ++i) {
             umb::mbar_init(acc_full + i, 1);
-            umb::mbar_init(acc_empty + i, 4);
+            umb::mbar_init(acc_empty + i, Cfg::kStore);
         }
         *quit = 0;
         umb::fence_barrier_init();
@@ -87,8 +106,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 const uint32_t s2 = s + 1 == kStages ? 0 : s + 1, ph2 = s + 1 == kStages ? ph ^ 1 : ph;
                 const bool next = tc_test(empty + s2, ph2);             // (known behind the copies: no wait of its own where it is free)
                 if (umb::elect_one()) {
-                    umb::mbar_arrive_expect_tx(full + s, (A_TMA ? Cfg::kABytes : 0) + Cfg::kWBytes);
-                    if (A_TMA) tma_3d(st, &map_a, k * kTcK, w.m0, ga, full + s);
+                    umb::mbar_arrive_expect_tx(full + s, (DENSE ? Cfg::kABytes : 0) + Cfg::kWBytes);
+                    if (DENSE) tma_3d(st, &map_a, k * kTcK, w.m0, ga, full + s);
                     tma_3d(st + Cfg::kABytes, &map_w, k * kTcK, n0, gw, full + s);
                     if (DUAL) tma_3d(st + Cfg::kABytes + kOut * 128, &map_w, k * kTcK, a.N + n0, gw, full + s);
                 }
@@ -126,20 +145,75 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 ph = ph2;
             }
         }
-    } else if (warp < 6) {
-        const int q = warp & 3;                             // the quarter of tensor-memory lanes this warp may read
-        float* so = s_out + (warp - 2) * 32 * kTcStageRow;
+    } else if (warp < 2 + Cfg::kStore) {
+        constexpr int kPart = kOut / (Cfg::kStore / 4);     // of the columns
+        const int q = warp & 3, part = (warp - 2) >> 2;     // the quarter of tensor-memory lanes this warp may read
+        float* so = s_out + (warp - 2) * Cfg::kStoreBlock;
         for (uint32_t it = 0; w.step(); ++it) {
             const uint32_t acc = it & 1;
             if (!__all_sync(0xffffffffu, tc_poll(acc_full + acc, (it >> 1) & 1, quit))) break;      // (and the warp is one again)
             umb::tc_fence_after();
-            tc_store_tile<kOut, kOut, DUAL, TC>(a, t.vec_c, tmem + acc * BN + ((uint32_t)(q * 32) << 16), so, w.g, w.row_lo + w.m0 + q * 32,
-                                          w.rows - w.m0 - q * 32, w.n0 * kOut, [&] { umb::mbar_arrive(acc_empty + acc); });
+            tc_store_tile<kPart, kOut, DUAL, TC, Cfg::kStoreCols>(a, t.vec_c, tmem + acc * BN + part * kPart + ((uint32_t)(q * 32) << 16), so, w.g, w.row_lo + w.m0 + q * 32,
+                                          w.rows - w.m0 - q * 32, w.n0 * kOut + part * kPart, [&] { umb::mbar_arrive(acc_empty + acc); });
         }
-    } else if (!A_TMA) {
+    } else if (!DENSE && warp == 2 + Cfg::kStore) {
+        // a box, or lane l: rows 4 l .. 4 l + 3 of the tile (behind the last row: that one again)
+        const __nv_bfloat16* A = (const __nv_bfloat16*)a.A;
+        uint32_t s = 0, ph = 1;
+        bool ok = true;
+        while (ok && w.step()) {
+            const int rows = min(kTcRows, w.rows - w.m0), kind = tc_rows_kind(a, t, rows), n4 = (rows + 3) >> 2;
+            int r[4] = {0, 0, 0, 0}, n_map = 0;
+            bool mine = false, in_map = true;
+            if (kind == kTcByFours) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    r[e] = w.row_lo + w.m0 + min(min(lane, n4 - 1) * 4 + e, rows - 1);
+                    if (a.row_src != nullptr) r[e] = a.row_src[r[e]];
+                }
+                // (rows in front of A have no place in a map: they are copied)
+                mine = lane < n4;
+                in_map = min(min(r[0], r[1]), min(r[2], r[3])) >= 0;
+                n_map = __popc(__ballot_sync(0xffffffffu, mine && in_map));
+            }
+            for (int k = 0; k < t.k_steps; ++k) {
+                if (!(ok = tc_spin_warp(empty + s, ph, quit))) break;
+                unsigned char* st = smem + s * Cfg::kStage;
+                if (kind == kTcByFours) {
+                    const uint32_t dst = smem_u32(st) + lane * 512;
+                    if (n_map != n4) {
+                        if (mine && !in_map)
+                            for (int e = 0; e < 4; ++e)
+                                for (int c = 0; c < 8; ++c) {
+                                    uint4 v = make_uint4(0, 0, 0, 0);
+                                    if (k * kTcK + c * 8 < a.K) v = *reinterpret_cast<const uint4*>(A + (int64_t)r[e] * a.lda + k * kTcK + c * 8);
+                                    *reinterpret_cast<uint4*>(st + lane * 512 + e * 128 + ((c ^ ((lane * 4 + e) & 7)) << 4)) = v;
+                                }
+                        umb::fence_proxy_async_smem();
+                        __syncwarp();
+                    }
+                    if (lane == 0) umb::mbar_arrive_expect_tx(full + s, n_map * 512);
+                    __syncwarp();
+                    if (mine && in_map) tma_gather4(dst, &map_r, k * kTcK, r[0], r[1], r[2], r[3], full + s);
+                } else if (umb::elect_one()) {
+                    if (kind == kTcBox) {
+                        umb::mbar_arrive_expect_tx(full + s, Cfg::kABytes);
+                        tma_3d(st, &map_a, k * kTcK, w.row_lo + w.m0, 0, full + s);
+                    } else {
+                        umb::mbar_arrive(full + s);
+                    }
+                }
+                __syncwarp();
+                if (++s == kStages) {
+                    s = 0;
+                    ph ^= 1;
+                }
+            }
+        }
+    } else if (!DENSE) {
         // eight lanes copy a row's 128 bytes of the k step; the image is the one a 128-byte-swizzled TMA box would leave
         constexpr int PW = Cfg::kWarpsPerStage, RS = 4 * PW;                // rows a stage's warps copy side by side
-        const int cw = warp - 6, st = cw / PW, ch = lane & 7, r0 = (cw % PW) * 4 + (lane >> 3);
+        const int cw = warp - 3 - Cfg::kStore, st = cw / PW, ch = lane & 7, r0 = (cw % PW) * 4 + (lane >> 3);
         int* src = reinterpret_cast<int*>(bars + 32) + cw * kTcRows;        // this warp's list of the tile's source rows
         const __nv_bfloat16* A = (const __nv_bfloat16*)a.A + ch * 8;
         const uint32_t base = smem_u32(smem + st * Cfg::kStage);
@@ -147,14 +221,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         int unit = 0;                                       // k steps of the tiles before, modulo the ring
         bool ok = true;
         while (ok && w.step()) {
+            const int rows = min(kTcRows, w.rows - w.m0);
+            const bool copied = tc_rows_kind(a, t, rows) == kTcCopied;          // (else the warp in front brings them)
             __syncwarp();
 #pragma unroll
-            for (int i = 0; i < kTcRows / 32; ++i) {
+            for (int i = 0; copied && i < kTcRows / 32; ++i) {
                 const int r = w.m0 + i * 32 + lane;
                 src[i * 32 + lane] = r < w.rows ? (a.row_src ? a.row_src[w.row_lo + r] : w.row_lo + r) : -1;
             }
             __syncwarp();
-            const int rows = min(kTcRows, w.rows - w.m0);
             const __nv_bfloat16* Ag = A + (t.a_grouped ? (int64_t)w.g * a.a_goff : 0);
             for (int k = (st - unit + kStages) % kStages; k < t.k_steps; k += kStages, ++uses) {
                 if (!(ok = __all_sync(0xffffffffu, tc_poll(empty + st, (uses & 1) ^ 1, quit)))) break;
@@ -162,18 +237,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 const int bytes = kc < a.K ? 16 : 0;        // behind the last column: zeros (K is a multiple of 8)
                 // (rows that are not there keep what the stage held: their sums are not stored)
 #pragma unroll 8
-                for (int r = r0; r < rows; r += RS)
+                for (int r = copied ? r0 : rows; r < rows; r += RS)
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + r * 128 + ((ch ^ (r & 7)) << 4)),
                                  "l"(Ag + (int64_t)src[r] * a.lda + (bytes ? k * kTcK : 0)), "r"(bytes) : "memory");
-                asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-                umb::fence_proxy_async_smem();              // the copies of this thread are complete: show them to the tensor core
-                __syncwarp();
+                if (copied) {
+                    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+                    umb::fence_proxy_async_smem();          // the copies of this thread are complete: show them to the tensor core
+                    __syncwarp();
+                }
                 if (lane == 0) umb::mbar_arrive(full + st);
             }
             unit = (unit + t.k_steps) % kStages;
         }
     }
-    if (!A_TMA && warp >= 2 && warp < 6 && a.rows_total > 0) {             // rows of no group: in front of the first, behind the last
+    if (!DENSE && warp >= 2 && warp < 6 && a.rows_total > 0) {             // rows of no group: in front of the first, behind the last
         const int64_t lo = min(a.grp_off[0], a.rows_total), gap = a.grp_off[t.groups] - lo;
         for (int64_t i = (int64_t)blockIdx.x * 4 + warp - 2; i < a.rows_total - gap; i += (int64_t)gridDim.x * 4) {
             const int64_t r = i < lo ? i : i + gap;
@@ -240,31 +317,50 @@ int encode_map(CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows,
                ? 0 : UMB_ERR_DRIVER;
 }
 
-template <int BN, bool DUAL, bool A_TMA, typename TC>
-static int launch_tc(const GemmArgs& a, TcArgs t, int sms, cudaStream_t st) {
+// bf16 rows of `cols` numbers, ld apart, as a map whose boxes are pieces of 64 of one row: what tile::gather4 takes four of
+static int encode_rows(CUtensorMap* map, const void* base, uint64_t cols, uint64_t ld) {
+    const EncodeTiled enc = encode_tiled();
+    if (enc == nullptr) return UMB_ERR_DRIVER;
+    const cuuint64_t dims[2] = {cols, 0x7fffffff}, strides[1] = {ld * 2};       // (as many rows as an index names)
+    const cuuint32_t box[2] = {64, 1}, one[2] = {1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
+               ? 0 : UMB_ERR_DRIVER;
+}
+
+template <int BN, bool DUAL, bool DENSE, typename TC>
+static int launch_tc(const GemmArgs& a, TcArgs t, const CUtensorMap& ma, const CUtensorMap& mr, int sms, cudaStream_t st) {
     using Cfg = TcCfg<BN, DUAL>;
     t.n_tiles = (a.N + Cfg::kOut - 1) / Cfg::kOut;
     t.k_steps = (a.K + kTcK - 1) / kTcK;
-    const int ga = a.a_goff != 0 ? t.groups : 1, gw = a.w_gstride != 0 ? t.groups : 1;
-    t.a_grouped = ga > 1;
+    const int gw = a.w_gstride != 0 ? t.groups : 1;
     t.w_grouped = gw > 1;
-    CUtensorMap ma{}, mw;
-    int rc = encode_map(&mw, a.W, a.K, (uint64_t)a.N * (DUAL ? 2 : 1), gw, a.ldw, a.w_gstride, Cfg::kOut);
-    if (rc == 0 && A_TMA) rc = encode_map(&ma, a.A, a.K, a.M, ga, a.lda, a.a_goff, kTcRows);
+    CUtensorMap mw;
+    const int rc = encode_map(&mw, a.W, a.K, (uint64_t)a.N * (DUAL ? 2 : 1), gw, a.ldw, a.w_gstride, Cfg::kOut);
     if (rc != 0) return rc;
-    auto kernel = gemm_tc_kernel<BN, DUAL, A_TMA, TC>;
+    auto kernel = gemm_tc_kernel<BN, DUAL, DENSE, TC>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
     if (e != cudaSuccess) return (int)e;
     const int64_t tiles = (int64_t)t.groups * t.m_tiles * t.n_tiles;            // (sorted by expert: at most)
-    return chain_launch(kernel, (int)(tiles < sms ? tiles : sms), Cfg::threads(A_TMA), Cfg::kSmem, st, ma, mw, a, t);
+    return chain_launch(kernel, (int)(tiles < sms ? tiles : sms), Cfg::threads(DENSE), Cfg::kSmem, st, ma, mr, mw, a, t);
 }
 
 template <int BN>
-static int launch_tc_any(const GemmArgs& a, const TcArgs& t, bool dual, bool c_f32, int sms, cudaStream_t st) {
-    const bool sorted = a.grp_off != nullptr || a.row_src != nullptr;
-#define UMBS_TC(D, S) (c_f32 ? launch_tc<BN, D, S, float>(a, t, sms, st) : launch_tc<BN, D, S, __nv_bfloat16>(a, t, sms, st))
-    if (dual) return sorted ? UMBS_TC(true, false) : UMBS_TC(true, true);
-    return sorted ? UMBS_TC(false, false) : UMBS_TC(false, true);
+static int launch_tc_any(const GemmArgs& a, TcArgs t, bool dual, bool c_f32, int sms, cudaStream_t st) {
+    const int ga = a.a_goff != 0 ? t.groups : 1;
+    const bool dense = a.grp_off == nullptr && a.row_src == nullptr;
+    t.a_grouped = ga > 1;
+    CUtensorMap ma{}, mr{};
+    if (dense) {
+        const int rc = encode_map(&ma, a.A, a.K, a.M, ga, a.lda, a.a_goff, kTcRows);
+        if (rc != 0) return rc;
+    } else {
+        // (how many rows A has is not known here: the maps have more, and what is asked for are rows of the tile)
+        t.maps = ga == 1 && encode_rows(&mr, a.A, a.K, a.lda) == 0 && encode_map(&ma, a.A, a.K, std::min<uint64_t>(0x7fffffff, (1ull << 38) / a.lda), 1, a.lda, 0, kTcRows) == 0;
+    }
+#define UMBS_TC(D, S) (c_f32 ? launch_tc<BN, D, S, float>(a, t, ma, mr, sms, st) : launch_tc<BN, D, S, __nv_bfloat16>(a, t, ma, mr, sms, st))
+    if (dual) return dense ? UMBS_TC(true, true) : UMBS_TC(true, false);
+    return dense ? UMBS_TC(false, true) : UMBS_TC(false, false);
 #undef UMBS_TC
 }
 

@@ -11,6 +11,7 @@ struct TcArgs {
     int groups, n_tiles, m_tiles, k_steps;
     int vec_c;                                              // rows of C take 16-byte (fp32) / 8-byte (bf16) stores of 4 columns
     int a_grouped, w_grouped;                               // the group coordinate of the tensor maps is used
+    int maps;                                               // gathered or sorted rows may come by tensor map
     unsigned int* report;                                   // give_up_word()
 };
 
@@ -39,23 +40,23 @@ struct TileWalk {
     }
 };
 
-constexpr int kTcStageRow = 36;                             // fp32 row stride of an epilogue warp's 32 x 32 staging block
+constexpr int kTcStageRow = 36;                             // fp32 row stride of an epilogue warp's 32 x 32 staging block (32 x 16: 20)
 
-// Bias and activation of 32 neighbouring columns of a row, v (and u, the up half) in place.  One choice of activation in
+// Bias and activation of C neighbouring columns of a row, v (and u, the up half) in place.  One choice of activation in
 // front of a loop over independent elements: chosen element by element, every exponential and every quotient waited for the
 // one before it (25 to 40 us for a tile's 128 x 128 outputs, several times its products).
-template <bool DUAL>
-__device__ __forceinline__ void tc_finish(const GemmArgs& a, uint32_t (&v)[32], uint32_t (&u)[DUAL ? 32 : 1], int n0) {
+template <bool DUAL, int C>
+__device__ __forceinline__ void tc_finish(const GemmArgs& a, uint32_t (&v)[C], uint32_t (&u)[DUAL ? C : 1], int n0) {
 #define UMBS_F(x) __uint_as_float(x)
 #define UMBS_EACH(expr)                                                                     \
-    _Pragma("unroll") for (int j = 0; j < 32; ++j) {                                        \
+    _Pragma("unroll") for (int j = 0; j < C; ++j) {                                        \
         const float x = UMBS_F(v[j]), y = DUAL ? UMBS_F(u[DUAL ? j : 0]) : 0.f;              \
         v[j] = __float_as_uint(expr);                                                       \
         (void)y;                                                                            \
     }
     if (a.bias != nullptr) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
+        for (int j = 0; j < C; ++j) {
             const int n = min(n0 + j, a.N - 1);
             v[j] = __float_as_uint(UMBS_F(v[j]) + a.bias[n]);
             if (DUAL) u[DUAL ? j : 0] = __float_as_uint(UMBS_F(u[DUAL ? j : 0]) + a.bias[a.N + n]);
@@ -65,7 +66,7 @@ __device__ __forceinline__ void tc_finish(const GemmArgs& a, uint32_t (&v)[32], 
         if (a.act == UMBS_ACT_GELU_TANH) UMBS_EACH(gated_act(x, y, a.limit, UMBS_ACT_GELU_TANH))
         else if (a.act == UMBS_ACT_SILU) UMBS_EACH(x * tc_sigmoid(x) * y)
         else UMBS_EACH(fminf(x, a.limit) * tc_sigmoid(1.702f * fminf(x, a.limit)) * (fminf(fmaxf(y, -a.limit), a.limit) + 1.f))
-    } else if (a.unary && n0 + 32 <= a.unary_cols && (a.unary == UMBS_UNARY_SILU || a.unary == UMBS_UNARY_RELU2 || a.unary == UMBS_UNARY_SCALE)) {
+    } else if (a.unary && n0 + C <= a.unary_cols && (a.unary == UMBS_UNARY_SILU || a.unary == UMBS_UNARY_RELU2 || a.unary == UMBS_UNARY_SCALE)) {
         if (a.unary == UMBS_UNARY_SILU) UMBS_EACH(x * tc_sigmoid(x))
         else if (a.unary == UMBS_UNARY_RELU2) UMBS_EACH(unary_act(x, UMBS_UNARY_RELU2, a.p0, a.p1))
         else UMBS_EACH(unary_act(x, UMBS_UNARY_SCALE, a.p0, a.p1))
@@ -76,33 +77,39 @@ __device__ __forceinline__ void tc_finish(const GemmArgs& a, uint32_t (&v)[32], 
 #undef UMBS_F
 }
 
+template <int C> __device__ __forceinline__ void tc_load(uint32_t addr, uint32_t (&v)[C]) {
+    if constexpr (C == 32) UMB_TMEM_LD_X32(addr, v);
+    else UMB_TMEM_LD_X16(addr, v);
+}
 // 32 rows of a finished tile, by a warp: kOut columns from tensor memory `src` (DUAL: the gate columns, the up columns kUp behind them) through
-// its staging block to rows grow .. of C, of which `rows` are there, from column col on.  read_done: by one lane once tensor memory is read.
-template <int kOut, int kUp, bool DUAL, typename TC, typename F>
+// its staging block, CW columns at a time, to rows grow .. of C, of which `rows` are there, from column col on.  read_done: by one lane once tensor
+// memory is read.
+template <int kOut, int kUp, bool DUAL, typename TC, int CW = 32, typename F>
 __device__ __forceinline__ void tc_store_tile(const GemmArgs& a, int vec_c, uint32_t src, float* so, int g, int64_t grow, int rows, int col, F&& read_done) {
-    const int lane = threadIdx.x & 31, rr = lane >> 3, cc = (lane & 7) * 4, n_hi = a.N - col;
+    constexpr int kRow = CW + 4, kLanes = CW / 4, kRows = 32 / kLanes;      // staging row; lanes of a row piece; rows side by side
+    const int lane = threadIdx.x & 31, rr = lane / kLanes, cc = lane % kLanes * 4, n_hi = a.N - col;
     TC* C = (TC*)a.C + (int64_t)g * a.c_goff + grow * a.ldc + col;
 #pragma unroll 1
-    for (int c0 = 0; c0 < kOut; c0 += 32) {
-        uint32_t v[32], u[DUAL ? 32 : 1];
-        UMB_TMEM_LD_X32(src + c0, v);
-        if (DUAL) UMB_TMEM_LD_X32(src + kUp + c0, u);
+    for (int c0 = 0; c0 < kOut; c0 += CW) {
+        uint32_t v[CW], u[DUAL ? CW : 1];
+        tc_load(src + c0, v);
+        if constexpr (DUAL) tc_load(src + kUp + c0, u);
         umb::tc_wait_ld();
-        if (c0 + 32 >= kOut) {                              // read to the end: the next tile but one may be summed here
+        if (c0 + CW >= kOut) {                              // read to the end: the next tile but one may be summed here
             umb::tc_fence_before();
             __syncwarp();
             if (lane == 0) read_done();
         }
         if (c0 >= n_hi || rows <= 0) continue;
-        if (DUAL || a.bias != nullptr || a.unary) tc_finish<DUAL>(a, v, u, col + c0);
+        if (DUAL || a.bias != nullptr || a.unary) tc_finish<DUAL, CW>(a, v, u, col + c0);
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(so + lane * kTcStageRow + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        for (int j = 0; j < CW; j += 4) *reinterpret_cast<uint4*>(so + lane * kRow + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
         __syncwarp();
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int r = i * 4 + rr, n = c0 + cc;
+        for (int i = 0; i < 32 / kRows; ++i) {
+            const int r = i * kRows + rr, n = c0 + cc;
             if (r < rows && n < n_hi) {
-                const float4 f = *reinterpret_cast<const float4*>(so + r * kTcStageRow + cc);
+                const float4 f = *reinterpret_cast<const float4*>(so + r * kRow + cc);
                 float o[4] = {f.x, f.y, f.z, f.w};
                 if (a.out_gate != nullptr) {
 #pragma unroll
