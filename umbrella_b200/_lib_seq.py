@@ -230,6 +230,31 @@ SIGNATURES = {
 }
 
 _lib = None
+calls = None        # the module of csrc/seq/calls.cpp, bound to the library that load() loaded
+_CALLED = ("umbs_gemm", "umbs_gemm_sorted", "umbs_moe_route", "umbs_add_norm", "umbs_kv_pool", "umbs_cached_attention_ex", "umbs_ring_append",
+           "umbs_window_attention_gated", "umbs_retention_ex")       # its Entries, in order
+
+
+def load_calls():
+    """The native way from tensors to the library that ops_seq takes for its most frequent calls."""
+    global calls
+    if calls is None:
+        import importlib.machinery
+        import importlib.util
+
+        from . import build
+        lib = load()
+        try:
+            build.build_calls()
+        except RuntimeError:
+            if not os.path.exists(build.CALLS):
+                raise
+        loader = importlib.machinery.ExtensionFileLoader("_seq_calls", build.CALLS)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_seq_calls", build.CALLS, loader=loader))
+        loader.exec_module(mod)
+        mod.bind(*(C.cast(getattr(lib, name), c_void_p).value for name in _CALLED))
+        calls = mod
+    return calls
 
 
 def load() -> C.CDLL:

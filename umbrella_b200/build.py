@@ -114,14 +114,44 @@ def build_seq(force: bool = False, verbose: bool = False) -> str:
     return SEQ_LIB
 
 
+CALLS_SOURCE = os.path.join(CSRC, "seq", "calls.cpp")
+CALLS = os.path.join(HERE, "_seq_calls.so")
+
+
+def build_calls(force: bool = False, verbose: bool = False) -> str:
+    """_seq_calls.so: the tensor-level calls' way into libumbrella_b200_seq.so (a Python module over torch's own headers; the torch
+    libraries are the ones the process has loaded)."""
+    deps = [CALLS_SOURCE, os.path.join(CSRC, "..", "..", "include", "umbrella_b200_seq.h"), os.path.join(CSRC, "..", "..", "include", "umbrella_b200.h")]
+    if not force and not _stale(CALLS, deps):
+        return CALLS
+    import sysconfig
+
+    import torch
+    t = os.path.dirname(torch.__file__)
+    cuda = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
+    tmp = f"{CALLS}.{os.getpid()}.tmp"
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I", os.path.join(t, "include"), "-I", os.path.join(t, "include", "torch", "csrc", "api", "include"), "-I", sysconfig.get_path("include"), "-I", cuda,
+           CALLS_SOURCE, "-o", tmp, "-L", os.path.join(t, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    if verbose:
+        print(" ".join(cmd))
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on {CALLS_SOURCE}:\n{r.stdout}")
+    os.replace(tmp, CALLS)
+    return CALLS
+
+
 if __name__ == "__main__":
     # python -m umbrella_b200.build [--force] [--variant NAME -DFOO=1 ...]
     argv = sys.argv[1:]
     if "--seq" in argv:
         print(build_seq(force="--force" in argv, verbose=True))
+        print(build_calls(force="--force" in argv, verbose=True))
         sys.exit(0)
     variant = argv[argv.index("--variant") + 1] if "--variant" in argv else ""
     print(build(force="--force" in argv, verbose=True, extra_flags=[a for a in argv if a.startswith("-D")],
                 variant=variant))
     if not variant:
         print(build_seq(force="--force" in argv, verbose=True))
+        print(build_calls(force="--force" in argv, verbose=True))

@@ -12,8 +12,18 @@ import torch
 from . import _lib_seq as S
 
 
-# Plain numbers, not ctypes or Stream objects: a call's own host work is what bounds small steps (gemm 17.2 -> 10.1 us, of which
-# torch.cuda.current_stream() was 3.4 and the objects 1.5).
+# A call's own host work is what bounds small steps.  The most frequent calls go through _lib_seq.calls (csrc/seq/calls.cpp), which does what the
+# wrapper below it does and says so with None where it does not; the others hand over plain numbers, not ctypes or Stream objects (gemm 17.2
+# -> 10.1 us, of which torch.cuda.current_stream() was 3.4 and the objects 1.5).
+_NUMBER = {torch.bfloat16: S.UMBS_BF16, torch.float32: S.UMBS_F32}
+
+
+def _done(out, what):
+    if out.__class__ is int:
+        S.check(out, what)
+    return out
+
+
 def _p(t):
     return t.data_ptr() if t is not None else None
 
@@ -65,6 +75,10 @@ def gemm(a: torch.Tensor, w: torch.Tensor, *, out_f32: bool = False, groups: int
          n: int | None = None, k: int | None = None, grp_off=None, row_src=None, rows: int | None = None,
          dual: bool = False, limit: float = 0.0, max_rows: int | None = None) -> torch.Tensor:
     """a [M, lda] x w ([groups,] N(or 2N if dual), K) -> [rows, groups * c_goff or N].  See umbs_gemm."""
+    if a.is_cuda:
+        out = (S.calls or S.load_calls()).gemm(a, w, out_f32, groups, a_goff, c_goff, n, k, grp_off, row_src, rows, dual, limit, max_rows)
+        if out is not None:
+            return _done(out, "gemm")
     mode = _mode(a)
     assert w.dtype == a.dtype and a.stride(-1) == 1 and w.is_contiguous()
     ws = w.shape                                          # [groups,] outputs, inputs, contiguous
@@ -103,6 +117,11 @@ def retention(qkvg, batch: RaggedBatch, heads, dim, vdim, rot_dims, inv_freq, de
     """``segments``: give the kernel room to cut few long sequences into segments that run side by side.  ``k_scale`` (0:
     dim^-1/2), ``norm_w`` (RMS norm over the concatenated heads in ``norm_parts`` parts instead of one per head), ``gate_act``:
     the options of umbs_retention_ex."""
+    if qkvg.is_cuda and dtype in _NUMBER:
+        out = (S.calls or S.load_calls()).retention(qkvg, C.addressof(batch.c), heads, dim, vdim, rot_dims, inv_freq, decay, eps, state, _NUMBER[dtype], segments,
+                                                   k_scale, norm_w, norm_parts, gate_act)
+        if out is not None:
+            return _done(out, "retention")
     T = qkvg.shape[0]
     seg = torch.empty(32 * heads * dim * vdim, dtype=torch.float32, device=qkvg.device) if segments and T >= 128 else None
     o32 = torch.empty((T, heads * vdim), dtype=torch.float32, device=qkvg.device)
@@ -154,6 +173,10 @@ def window_attention(q, k, v, batch: RaggedBatch, heads: int, window: int, scale
 
 def moe_route(h, w_router, top: int):
     """-> (sel_w [n, top] fp32, grp_off [E + 1], pair_tok [n top], pair_pos [n top], sel_e [n top])."""
+    if h.is_cuda:
+        out = (S.calls or S.load_calls()).moe_route(h, w_router, top)
+        if out is not None:
+            return _done(out, "moe_route")
     n, width = h.shape
     E = w_router.shape[0]
     dev = h.device
@@ -211,6 +234,11 @@ def cached_attention(q, kv, kv_cache, batch: RaggedBatch, heads, kv_heads, dim, 
                      split=True, sink=None):
     """One attention step over the step's kv rows and the slots' caches (pooling the blocks the step completes first and
     appending the step's rows afterwards, as umbs_forward does)."""
+    if q.is_cuda:
+        out = (S.calls or S.load_calls()).cached_attention(q, kv, kv_cache, C.addressof(batch.c), heads, kv_heads, dim, vdim, scale, mode, window, pool, pool_cache,
+                                                          head_bias, gate, gate_per_head, append, split, sink)
+        if out is not None:
+            return _done(out, "cached_attention")
     T = q.shape[0]
     lib, row = S.load(), kv_heads * (dim + vdim)
     out = torch.empty((T, heads * vdim), dtype=q.dtype, device=q.device)
@@ -272,6 +300,11 @@ def add_norm(x, w, b, eps: float, kind: int = S.UMBS_NORM_LAYER, w_offset: float
              want_copy: bool = False):
     """x [n, width] fp32 += (delta + routed pairs + gated shared) * scale * mult (in place when ``rows`` is None), then the
     norm of the sum as ``dtype`` (and a copy of the sum)."""
+    if x.is_cuda and dtype in _NUMBER:
+        out = (S.calls or S.load_calls()).add_norm(x, w, b, eps, kind, w_offset, _NUMBER[dtype], rows, delta, pair_out, sel_w, pair_pos, shared, shared_gate,
+                                                  scale, mult, want_copy)
+        if out is not None:
+            return _done(out, "add_norm")
     n = x.shape[0] if rows is None else rows.numel()
     y = torch.empty((n, x.shape[1]), dtype=dtype, device=x.device)
     copy = torch.empty((n, x.shape[1]), dtype=torch.float32, device=x.device) if want_copy else None
@@ -324,6 +357,10 @@ def window_attention_shared(q, k, k_shared, v, batch: RaggedBatch, heads: int, s
                             use_sink: bool = True, gate=None, gate_per_head: bool = False):
     """q [T, heads (dim + shared)], k [T, heads dim], k_shared [T, shared], v [T, heads vdim] (row-strided views are fine)
     -> [T, heads vdim]: attention among the step's own tokens with a key part all heads share, a sink and an output gate."""
+    if q.is_cuda:
+        out = (S.calls or S.load_calls()).window_attention(q, k, k_shared, v, C.addressof(batch.c), heads, scale, window, sink, use_sink, gate, gate_per_head)
+        if out is not None:
+            return _done(out, "window_attention_gated")
     T = q.shape[0]
     sd = k_shared.shape[1] if k_shared is not None else 0
     dim, vdim = k.shape[1] // heads, v.shape[1] // heads
