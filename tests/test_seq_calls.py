@@ -95,3 +95,11 @@ def test_tensor_memory_is_taken_before_the_next_kernel_is_let_in():
             if alloc and "chain_wait_only()" in body:
                 assert let_in, path
     assert seen >= 5
+
+
+def test_the_native_calls_load_in_a_process_without_torch():
+    """A build check imports the package and nothing else."""
+    import subprocess
+    import sys
+    code = "import sys; from umbrella_b200 import _lib_seq; assert 'torch' not in sys.modules; assert _lib_seq.load_calls().gemm"
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=S.__file__.rsplit("/", 2)[0])

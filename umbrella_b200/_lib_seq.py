@@ -242,6 +242,8 @@ def load_calls():
         import importlib.machinery
         import importlib.util
 
+        import torch  # noqa: F401  (the module finds the libraries that it needs among those that are loaded)
+
         from . import build
         lib = load()
         try:
