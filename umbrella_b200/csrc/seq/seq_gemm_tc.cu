@@ -3,9 +3,9 @@
 //
 // A persistent block per SM walks output tiles of 128 rows x BN columns.  Warp 0 copies weight tiles (and, for dense rows,
 // activation tiles) with TMA into a ring of 64-wide k steps, one thread of warp 1 issues tcgen05.mma, four or eight more empty the
-// accumulators -- two sets of them, so that a tile is stored while the next one is summed.  Which rows a tile has of those that are gathered or
-// sorted by expert is known on the device alone: a full tile of neighbouring rows is one box for a warp more, a tile of few rows comes four rows at a time
-// from its lanes (tile::gather4), the others through 16-byte cp.async from four to eight more warps.
+// accumulators -- two sets of them, so that a tile is stored while the next one is summed.  Rows that are gathered or sorted by
+// expert come from four to eight more warps through 16-byte cp.async: which rows a tile has is known on the device alone, and a tile
+// of few rows fetches only those.
 //
 // An output element is one fp32 sum over k in the same order whatever its tile's size, so a row's result does not depend on
 // the rest of the batch; against float64 it is as far off as the mma.sync tiles that this replaced (2.1e-6 at K = 2048, in
@@ -14,19 +14,17 @@
 // Bound for dense prompts: a block's shared memory, 48 KB in and 48 KB out for 512 clocks of products at 256 columns (690 clocks a step); the
 // large ones go to pairs of SMs (seq_gemm_pair.cu).  With few steps: launch, first operands, last results (8.0 us for K = 1024 to 1024
 // columns, 3.8 of them steps).  Sorted rows: the copying warps' loads (890 clocks a step of gathered ones; leaving them out: 7 us of 193) and the results
-// (25 us of 193 with four warps that store).  16 experts, top 2, of width 2048 with the routing around it, us, four warps that store and all rows copied
-// / this: 64 tokens 85 / 73, 200 98 / 82, 500 101 / 89, 4096 206 / 200; gate|up of 64 tokens reads its 134 MB at the memory's rate.
+// (25 us of 193 with four warps that store).  16 experts, top 2, of width 2048 with the routing around it, us, four warps that store / eight:
+// 64 tokens 85 / 73, 4096 210 / 208; gate|up of 64 tokens reads its 134 MB at the memory's rate.
+// (tile::gather4 for tiles of few rows and boxes for full ones, with maps that went on behind the rows' memory, gave no more, and one run of them ended with an
+// illegal address.)
 #include <cuda.h>
-#include <algorithm>
 #include <atomic>
 #include <mutex>
 
 #include "seq_gemm_walk.cuh"
 
 namespace umbs {
-
-// Up to so many rows of a tile come by tile::gather4: four rows cost the copy engine 60 clocks, 128 rows 1900 a k step where 64 threads' copies take 890.
-constexpr int kTcGather = 40;
 
 template <int BN, bool DUAL>
 struct TcCfg {
@@ -37,28 +35,15 @@ struct TcCfg {
     static constexpr int kWarpsPerStage = BN == 256 ? 2 : 1, kCopyWarps = kStages * kWarpsPerStage;
     // Warps that store: at 256 columns eight, half of the columns each four, 16 at a time (their staging blocks fit beside four stages).
     static constexpr int kStore = BN == 256 ? 8 : 4, kStoreCols = BN == 256 ? 16 : 32, kStoreBlock = 32 * (kStoreCols + 4);
-    static constexpr int threads(bool dense) { return 64 + 32 * kStore + (dense ? 0 : 32 * (1 + kCopyWarps)); }
+    static constexpr int threads(bool dense) { return 64 + 32 * kStore + (dense ? 0 : 32 * kCopyWarps); }
     static constexpr int kABytes = kTcRows * 128, kWBytes = BN * 128, kStage = kABytes + kWBytes;
     static constexpr int kOut = DUAL ? BN / 2 : BN;         // output columns of a tile
     static constexpr int kSmem = 1024 + kStages * kStage + kStore * kStoreBlock * 4 + 256 + kCopyWarps * kTcRows * 4;
 };
 
-__device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap* map, int c, int r0, int r1, int r2, int r3, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
-                 ::"r"(dst), "l"(map), "r"(c), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(smem_u32(bar)) : "memory");
-}
-
-// how the rows of a tile that is gathered or sorted come
-enum { kTcCopied, kTcBox, kTcByFours };
-__device__ __forceinline__ int tc_rows_kind(const GemmArgs& a, const TcArgs& t, int rows) {
-    if (!t.maps) return kTcCopied;
-    if (rows <= kTcGather) return kTcByFours;
-    return a.row_src == nullptr && rows == kTcRows ? kTcBox : kTcCopied;
-}
-
 template <int BN, bool DUAL, bool DENSE, typename TC>
 __global__ void __launch_bounds__(TcCfg<BN, DUAL>::threads(DENSE), 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_r, const __grid_constant__ CUtensorMap map_w, const GemmArgs a, const TcArgs t) {
+gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const GemmArgs a, const TcArgs t) {
     using Cfg = TcCfg<BN, DUAL>;
     constexpr int kStages = Cfg::kStages, kOut = Cfg::kOut;
     extern __shared__ unsigned char smem_raw[];
@@ -72,9 +57,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
     if (threadIdx.x == 0) {
         umb::tma_prefetch_desc(&map_w);
-        if (DENSE || t.maps) umb::tma_prefetch_desc(&map_a);
+        if (DENSE) umb::tma_prefetch_desc(&map_a);
         for (int i = 0; i < kStages; ++i) {
-            umb::mbar_init(full + i, DENSE ? 1 : 2 + Cfg::kWarpsPerStage);         // the TMA thread, warp 6 and the stage's copying warps
+            umb::mbar_init(full + i, DENSE ? 1 : 1 + Cfg::kWarpsPerStage);         // the TMA thread and the stage's copying warps
             umb::mbar_init(empty + i, 1);
         }
         for (int i = 0; i < 2; ++i) {
@@ -156,64 +141,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             tc_store_tile<kPart, kOut, DUAL, TC, Cfg::kStoreCols>(a, t.vec_c, tmem + acc * BN + part * kPart + ((uint32_t)(q * 32) << 16), so, w.g, w.row_lo + w.m0 + q * 32,
                                           w.rows - w.m0 - q * 32, w.n0 * kOut + part * kPart, [&] { umb::mbar_arrive(acc_empty + acc); });
         }
-    } else if (!DENSE && warp == 2 + Cfg::kStore) {
-        // a box, or lane l: rows 4 l .. 4 l + 3 of the tile (behind the last row: that one again)
-        const __nv_bfloat16* A = (const __nv_bfloat16*)a.A;
-        uint32_t s = 0, ph = 1;
-        bool ok = true;
-        while (ok && w.step()) {
-            const int rows = min(kTcRows, w.rows - w.m0), kind = tc_rows_kind(a, t, rows), n4 = (rows + 3) >> 2;
-            int r[4] = {0, 0, 0, 0}, n_map = 0;
-            bool mine = false, in_map = true;
-            if (kind == kTcByFours) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    r[e] = w.row_lo + w.m0 + min(min(lane, n4 - 1) * 4 + e, rows - 1);
-                    if (a.row_src != nullptr) r[e] = a.row_src[r[e]];
-                }
-                // (rows in front of A have no place in a map: they are copied)
-                mine = lane < n4;
-                in_map = min(min(r[0], r[1]), min(r[2], r[3])) >= 0;
-                n_map = __popc(__ballot_sync(0xffffffffu, mine && in_map));
-            }
-            for (int k = 0; k < t.k_steps; ++k) {
-                if (!(ok = tc_spin_warp(empty + s, ph, quit))) break;
-                unsigned char* st = smem + s * Cfg::kStage;
-                if (kind == kTcByFours) {
-                    const uint32_t dst = smem_u32(st) + lane * 512;
-                    if (n_map != n4) {
-                        if (mine && !in_map)
-                            for (int e = 0; e < 4; ++e)
-                                for (int c = 0; c < 8; ++c) {
-                                    uint4 v = make_uint4(0, 0, 0, 0);
-                                    if (k * kTcK + c * 8 < a.K) v = *reinterpret_cast<const uint4*>(A + (int64_t)r[e] * a.lda + k * kTcK + c * 8);
-                                    *reinterpret_cast<uint4*>(st + lane * 512 + e * 128 + ((c ^ ((lane * 4 + e) & 7)) << 4)) = v;
-                                }
-                        umb::fence_proxy_async_smem();
-                        __syncwarp();
-                    }
-                    if (lane == 0) umb::mbar_arrive_expect_tx(full + s, n_map * 512);
-                    __syncwarp();
-                    if (mine && in_map) tma_gather4(dst, &map_r, k * kTcK, r[0], r[1], r[2], r[3], full + s);
-                } else if (umb::elect_one()) {
-                    if (kind == kTcBox) {
-                        umb::mbar_arrive_expect_tx(full + s, Cfg::kABytes);
-                        tma_3d(st, &map_a, k * kTcK, w.row_lo + w.m0, 0, full + s);
-                    } else {
-                        umb::mbar_arrive(full + s);
-                    }
-                }
-                __syncwarp();
-                if (++s == kStages) {
-                    s = 0;
-                    ph ^= 1;
-                }
-            }
-        }
     } else if (!DENSE) {
         // eight lanes copy a row's 128 bytes of the k step; the image is the one a 128-byte-swizzled TMA box would leave
         constexpr int PW = Cfg::kWarpsPerStage, RS = 4 * PW;                // rows a stage's warps copy side by side
-        const int cw = warp - 3 - Cfg::kStore, st = cw / PW, ch = lane & 7, r0 = (cw % PW) * 4 + (lane >> 3);
+        const int cw = warp - 2 - Cfg::kStore, st = cw / PW, ch = lane & 7, r0 = (cw % PW) * 4 + (lane >> 3);
         int* src = reinterpret_cast<int*>(bars + 32) + cw * kTcRows;        // this warp's list of the tile's source rows
         const __nv_bfloat16* A = (const __nv_bfloat16*)a.A + ch * 8;
         const uint32_t base = smem_u32(smem + st * Cfg::kStage);
@@ -222,10 +153,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         bool ok = true;
         while (ok && w.step()) {
             const int rows = min(kTcRows, w.rows - w.m0);
-            const bool copied = tc_rows_kind(a, t, rows) == kTcCopied;          // (else the warp in front brings them)
             __syncwarp();
 #pragma unroll
-            for (int i = 0; copied && i < kTcRows / 32; ++i) {
+            for (int i = 0; i < kTcRows / 32; ++i) {
                 const int r = w.m0 + i * 32 + lane;
                 src[i * 32 + lane] = r < w.rows ? (a.row_src ? a.row_src[w.row_lo + r] : w.row_lo + r) : -1;
             }
@@ -237,14 +167,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 const int bytes = kc < a.K ? 16 : 0;        // behind the last column: zeros (K is a multiple of 8)
                 // (rows that are not there keep what the stage held: their sums are not stored)
 #pragma unroll 8
-                for (int r = copied ? r0 : rows; r < rows; r += RS)
+                for (int r = r0; r < rows; r += RS)
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + r * 128 + ((ch ^ (r & 7)) << 4)),
                                  "l"(Ag + (int64_t)src[r] * a.lda + (bytes ? k * kTcK : 0)), "r"(bytes) : "memory");
-                if (copied) {
-                    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-                    umb::fence_proxy_async_smem();          // the copies of this thread are complete: show them to the tensor core
-                    __syncwarp();
-                }
+                asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+                umb::fence_proxy_async_smem();              // the copies of this thread are complete: show them to the tensor core
+                __syncwarp();
                 if (lane == 0) umb::mbar_arrive(full + st);
             }
             unit = (unit + t.k_steps) % kStages;
@@ -317,19 +245,8 @@ int encode_map(CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows,
                ? 0 : UMB_ERR_DRIVER;
 }
 
-// bf16 rows of `cols` numbers, ld apart, as a map whose boxes are pieces of 64 of one row: what tile::gather4 takes four of
-static int encode_rows(CUtensorMap* map, const void* base, uint64_t cols, uint64_t ld) {
-    const EncodeTiled enc = encode_tiled();
-    if (enc == nullptr) return UMB_ERR_DRIVER;
-    const cuuint64_t dims[2] = {cols, 0x7fffffff}, strides[1] = {ld * 2};       // (as many rows as an index names)
-    const cuuint32_t box[2] = {64, 1}, one[2] = {1, 1};
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
-               ? 0 : UMB_ERR_DRIVER;
-}
-
 template <int BN, bool DUAL, bool DENSE, typename TC>
-static int launch_tc(const GemmArgs& a, TcArgs t, const CUtensorMap& ma, const CUtensorMap& mr, int sms, cudaStream_t st) {
+static int launch_tc(const GemmArgs& a, TcArgs t, const CUtensorMap& ma, int sms, cudaStream_t st) {
     using Cfg = TcCfg<BN, DUAL>;
     t.n_tiles = (a.N + Cfg::kOut - 1) / Cfg::kOut;
     t.k_steps = (a.K + kTcK - 1) / kTcK;
@@ -342,7 +259,7 @@ static int launch_tc(const GemmArgs& a, TcArgs t, const CUtensorMap& ma, const C
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
     if (e != cudaSuccess) return (int)e;
     const int64_t tiles = (int64_t)t.groups * t.m_tiles * t.n_tiles;            // (sorted by expert: at most)
-    return chain_launch(kernel, (int)(tiles < sms ? tiles : sms), Cfg::threads(DENSE), Cfg::kSmem, st, ma, mr, mw, a, t);
+    return chain_launch(kernel, (int)(tiles < sms ? tiles : sms), Cfg::threads(DENSE), Cfg::kSmem, st, ma, mw, a, t);
 }
 
 template <int BN>
@@ -350,15 +267,12 @@ static int launch_tc_any(const GemmArgs& a, TcArgs t, bool dual, bool c_f32, int
     const int ga = a.a_goff != 0 ? t.groups : 1;
     const bool dense = a.grp_off == nullptr && a.row_src == nullptr;
     t.a_grouped = ga > 1;
-    CUtensorMap ma{}, mr{};
+    CUtensorMap ma{};
     if (dense) {
         const int rc = encode_map(&ma, a.A, a.K, a.M, ga, a.lda, a.a_goff, kTcRows);
         if (rc != 0) return rc;
-    } else {
-        // (how many rows A has is not known here: the maps have more, and what is asked for are rows of the tile)
-        t.maps = ga == 1 && encode_rows(&mr, a.A, a.K, a.lda) == 0 && encode_map(&ma, a.A, a.K, std::min<uint64_t>(0x7fffffff, (1ull << 38) / a.lda), 1, a.lda, 0, kTcRows) == 0;
     }
-#define UMBS_TC(D, S) (c_f32 ? launch_tc<BN, D, S, float>(a, t, ma, mr, sms, st) : launch_tc<BN, D, S, __nv_bfloat16>(a, t, ma, mr, sms, st))
+#define UMBS_TC(D, S) (c_f32 ? launch_tc<BN, D, S, float>(a, t, ma, sms, st) : launch_tc<BN, D, S, __nv_bfloat16>(a, t, ma, sms, st))
     if (dual) return dense ? UMBS_TC(true, true) : UMBS_TC(true, false);
     return dense ? UMBS_TC(false, true) : UMBS_TC(false, false);
 #undef UMBS_TC

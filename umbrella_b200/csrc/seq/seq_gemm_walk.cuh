@@ -11,7 +11,6 @@ struct TcArgs {
     int groups, n_tiles, m_tiles, k_steps;
     int vec_c;                                              // rows of C take 16-byte (fp32) / 8-byte (bf16) stores of 4 columns
     int a_grouped, w_grouped;                               // the group coordinate of the tensor maps is used
-    int maps;                                               // gathered or sorted rows may come by tensor map
     unsigned int* report;                                   // give_up_word()
 };
 
