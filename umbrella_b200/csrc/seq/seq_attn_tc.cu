@@ -582,6 +582,21 @@ bool attention_tc_fits(const CachedAttnArgs& a, const StepKeys* s) {
     return al(a.q) && al(a.kv) && al(a.kv_cache) && (a.pool <= 0 || al(a.pool_cache)) && al(a.out);
 }
 
+// from p to the end of the allocation that it points into; 0 where that is not known
+static uint64_t bytes_from(const void* p) {
+    typedef CUresult (*AddressRange)(CUdeviceptr*, size_t*, CUdeviceptr);
+    static const AddressRange fn = [] {
+        void* sym = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        return cudaGetDriverEntryPoint("cuMemGetAddressRange", &sym, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess ? (AddressRange)sym
+                                                                                                                                            : nullptr;
+    }();
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    if (fn == nullptr || fn(&base, &size, (CUdeviceptr)p) != CUDA_SUCCESS || (CUdeviceptr)p < base) return 0;
+    return base + size - (CUdeviceptr)p;
+}
+
 template <int MODE, bool SHAPED, bool STEP>
 static int launch_ta(const CachedAttnArgs& a, const StepKeys& x, const Batch& b, cudaStream_t st) {
     TaDims z = ta_dims(a);
@@ -600,11 +615,11 @@ static int launch_ta(const CachedAttnArgs& a, const StepKeys& x, const Batch& b,
             if (rc == 0 && x.kdim < a.dim) rc = encode_map(&ms, x.ks, a.dim - x.kdim, b.n_tokens, 1, x.ldks, 0, kTaK);
             if (rc == 0) rc = encode_map(&mv, x.v, (uint64_t)a.heads * a.vdim, b.n_tokens, 1, x.ldv, 0, kTaK);
         } else {
-            // (the ring's slots are as many as the caller's cache has: the map's rows go on as far as a map can describe)
+            // (how many slots the caller's cache has is not known here: the map ends with the memory that the cache is in)
             const uint64_t row = (uint64_t)a.kv_heads * ((a.maps > 1 ? a.maps : 1) * a.dim + a.vdim);
-            z.ring_rows = (int64_t)std::min<uint64_t>(0x7fffffff, (1ull << 38) / row);
+            z.ring_rows = (int64_t)std::min<uint64_t>({0x7fffffff, (1ull << 38) / row, bytes_from(a.kv_cache) / (row * 2)});
             rc = encode_map(&mk, a.kv, row, b.n_tokens, 1, row, 0, kTaK);
-            if (rc == 0) rc = encode_map(&ms, a.kv_cache, row, z.ring_rows, 1, row, 0, kTaK);
+            if (rc == 0 && z.ring_rows > 0) rc = encode_map(&ms, a.kv_cache, row, z.ring_rows, 1, row, 0, kTaK);
             mv = mk;
         }
         z.tma = rc == 0;
