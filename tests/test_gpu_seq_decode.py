@@ -1,8 +1,13 @@
-"""What a decode step reads of a cache: means of whole blocks (umbs_kv_pool), bit for bit."""
+"""What a decode step reads of a cache: means of whole blocks (umbs_kv_pool) bit for bit, and the grouped attention with four and with six warps
+a block (unsplit steps from 148 blocks on) against float64.
+
+Tolerance: results are bf16 (2^-9 of their size at most, 2^-9 / sqrt(3) in the norm); the fp32 work inside is four orders below."""
 import ctypes as C
 
 import pytest
 import torch
+
+import seq_helpers as H
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -28,3 +33,26 @@ def test_means_of_blocks(dt, row, pool, pos0, tokens, kv_len):
                 acc += (kv[s * tokens + j - pos0] if j >= pos0 else ring[slot, j % kv_len]).float()
             want[slot, blk] = (acc / torch.tensor(float(pool))).to(dt)
     assert torch.equal(means.cpu(), want)
+
+
+@pytest.mark.parametrize("mode", ["SOFTMAX", "SOFTMAX_SINK", "SIGMOID"])
+@pytest.mark.parametrize("seqs,kv_heads,group,dim,ctx", [(37, 4, 2, 64, 230), (36, 4, 2, 64, 230), (148, 1, 9, 40, 193), (150, 1, 3, 128, 33), (75, 2, 4, 96, 400)])
+def test_groups_of_heads(mode, seqs, kv_heads, group, dim, ctx):
+    from umbrella_b200 import _lib_seq as S, ops_seq as K
+    g = torch.Generator(device=DEV).manual_seed(8)
+    r = lambda *s: torch.randn(*s, generator=g, device=DEV).bfloat16()
+    heads, row = kv_heads * group, 2 * kv_heads * dim
+    pos = [max(0, ctx - 1 - 7 * (i % 5)) for i in range(seqs)]
+    q, kv, cache, sink = r(seqs, heads * dim), r(seqs, row), r(seqs, ctx + 3, row), r(heads).float()
+    b = K.RaggedBatch([(i, 1, p, 0) for i, p in enumerate(pos)], DEV)
+    out = K.cached_attention(q, kv, cache.clone(), b, heads, kv_heads, dim, dim, dim ** -0.5, mode=getattr(S, "UMBS_ATTN_" + mode), sink=sink if "SINK" in mode else None)
+    for i in range(0, seqs, 7):
+        rows = torch.cat([cache[i, :pos[i]], kv[i:i + 1]]).double().view(pos[i] + 1, 2, kv_heads, dim)
+        z = torch.einsum("hgd,jhd->hgj", q[i].double().view(kv_heads, group, dim), rows[:, 0]) * dim ** -0.5
+        if mode == "SIGMOID":
+            w = torch.sigmoid(z)
+        else:
+            e = torch.cat([z, sink.double().view(kv_heads, group, 1)], 2) if "SINK" in mode else z
+            w = torch.softmax(e, 2)[..., :pos[i] + 1]
+        want = torch.einsum("hgj,jhd->hgd", w, rows[:, 1]).reshape(-1)
+        assert H.rel_err(out[i], want) < 2.0 ** -9

@@ -372,8 +372,8 @@ __global__ void __launch_bounds__(32 * kCdWarps) cached_attention_decode_kernel(
 }
 
 // Decode steps over bf16 rows: the query heads that share a key/value head together, so that a key and a value are fetched
-// once for all of them.  One block = (split, up to eight heads of a key/value head, sequence), four warps that each take every
-// fourth tile of 32 keys of the split, with running (maximum, sum, output) of their own.  A tile's rows come to shared memory
+// once for all of them.  One block = (split, up to eight heads of a key/value head, sequence), four or six (NW) warps that each take every
+// fourth or sixth tile of 32 keys of the split, with running (maximum, sum, output) of their own.  A tile's rows come to shared memory
 // by 16-byte copies, keys and values as groups of their own, the next tile's while this one is worked on.  Both products are
 // 16 x 8 x 16 warp-level tensor-core products with the heads as rows (half of the 16 are empty: the step is bound by its
 // bytes, and these take a tenth of the instructions that FMAs would): bf16 products are exact, a product's sums are added up
@@ -381,8 +381,8 @@ __global__ void __launch_bounds__(32 * kCdWarps) cached_attention_decode_kernel(
 // weights go in as three bf16 numbers that add up to them exactly.  The warps' triples are merged in warp order, splits by
 // cached_attention_merge_kernel as before.
 // 64 sequences x 1040 keys, 16 heads over 4 of 128 (136 MB): a warp per (head, key) took 407 us, heads together with FMAs 65 us,
-// this 51 us in two splits, 44 in one.
-constexpr int kCgWarps = 4, kCgKeys = 32, kCgHeads = 8;
+// this with four warps 51 us in two splits, 43 in one, with six warps 37 (3.7 TB/s).
+constexpr int kCgKeys = 32, kCgHeads = 8;
 
 struct GroupSizes { int ks16, vs16, warp_bytes; };          // 16-byte pieces between key rows and between value rows (odd: no bank conflicts)
 __host__ __device__ __forceinline__ GroupSizes group_sizes(int dim, int vdim) {
@@ -404,15 +404,15 @@ __device__ __forceinline__ void mma_top(float (&d)[4], uint32_t a0, uint32_t a2,
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
 }
 
-// A warp's triple of one head in plain fp32: every fourth tile of the keys [lo, hi) from the warp's own, key after key.
-template <int MODE>
+// A warp's triple of one head in plain fp32: every NW-th tile of the keys [lo, hi) from the warp's own, key after key.
+template <int MODE, int NW>
 __device__ __forceinline__ void plain_part(const CachedAttnArgs& a, const VHead& v, const __nv_bfloat16* q, int h, const __nv_bfloat16* own, int slot, int p, int n_pool,
                                         int j_lo, int first, int hi, float* s_o, float* s_ml) {
     const int lane = threadIdx.x & 31;
     PlainRow s;
     plain_start(s, q, a.dim, -INFINITY, 0.f);
     bool go = true;
-    for (int k0 = first; go && k0 < hi; k0 += kCgWarps * kCgKeys)
+    for (int k0 = first; go && k0 < hi; k0 += NW * kCgKeys)
         for (int k = k0; go && k < min(k0 + kCgKeys, hi); ++k) {
             const int j = j_lo + (k - n_pool);
             const __nv_bfloat16* row = k < n_pool ? (const __nv_bfloat16*)a.pool_cache + ((int64_t)slot * a.pool_len + k) * v.row_kv
@@ -425,8 +425,8 @@ __device__ __forceinline__ void plain_part(const CachedAttnArgs& a, const VHead&
     if (lane == 0) { s_ml[0] = s.m; s_ml[1] = s.l; }
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(32 * kCgWarps, 3) cached_attention_decode_group_kernel(const __grid_constant__ CachedAttnArgs a, const __grid_constant__ Batch b,
+template <int MODE, int NW>
+__global__ void __launch_bounds__(32 * NW, NW == 4 ? 3 : 2) cached_attention_decode_group_kernel(const __grid_constant__ CachedAttnArgs a, const __grid_constant__ Batch b,
                                                                                          int n_split, float* __restrict__ part) {
     extern __shared__ __align__(16) unsigned char smem[];
     chain_wait();
@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(32 * kCgWarps, 3) cached_attention_decode_grou
         const int j = j_lo + (k0 - n_pool);                                 // the first key's position
         return k0 >= n_pool && k0 + kCgKeys <= hi && j + kCgKeys <= p && j % a.kv_len + kCgKeys <= a.kv_len;
     };
-    const int step = kCgWarps * kCgKeys;
+    const int step = NW * kCgKeys;
     int k0 = lo + w * kCgKeys;
     if (k0 < hi) {
         const __nv_bfloat16* row = row_of(k0);
@@ -601,7 +601,7 @@ __global__ void __launch_bounds__(32 * kCgWarps, 3) cached_attention_decode_grou
     __syncthreads();
     // merge: the warps' triples over the tiles' memory
     float* s_o = reinterpret_cast<float*>(smem);                            // [warps][heads][vdim]
-    float* s_ml = s_o + kCgWarps * kCgHeads * vdim;                         // [warps][heads][2]
+    float* s_ml = s_o + NW * kCgHeads * vdim;                         // [warps][heads][2]
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
 #pragma unroll
@@ -614,20 +614,20 @@ __global__ void __launch_bounds__(32 * kCgWarps, 3) cached_attention_decode_grou
     if (__any_sync(0xffffffffu, hr < nh && odd != 0.f)) {
         __syncwarp();
         for (int g = 0; g < nh; ++g)
-            plain_part<MODE>(a, v0, (const __nv_bfloat16*)a.q + (int64_t)t * v0.qstride + (h0 + g) * dim, h0 + g, own, slot, p, n_pool, j_lo,
+            plain_part<MODE, NW>(a, v0, (const __nv_bfloat16*)a.q + (int64_t)t * v0.qstride + (h0 + g) * dim, h0 + g, own, slot, p, n_pool, j_lo,
                              lo + w * kCgKeys, hi, s_o + (w * kCgHeads + g) * vdim, s_ml + (w * kCgHeads + g) * 2);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < nh * vdim; i += 32 * kCgWarps) {
+    for (int i = threadIdx.x; i < nh * vdim; i += 32 * NW) {
         const int g = i / vdim, c = i - g * vdim, hh = h0 + g;
         float Mx = -INFINITY, L = 0.f, O = 0.f;
         if (MODE == UMBS_ATTN_SIGMOID) {
-            for (int ww = 0; ww < kCgWarps; ++ww) O += s_o[(ww * kCgHeads + g) * vdim + c];
+            for (int ww = 0; ww < NW; ++ww) O += s_o[(ww * kCgHeads + g) * vdim + c];
         } else {
             const float sk = (n_split == 1 && MODE == UMBS_ATTN_SOFTMAX_SINK) ? sink_score(a, hh) : -INFINITY;
-            for (int ww = 0; ww < kCgWarps; ++ww) Mx = fmaxf(Mx, s_ml[(ww * kCgHeads + g) * 2]);
+            for (int ww = 0; ww < NW; ++ww) Mx = fmaxf(Mx, s_ml[(ww * kCgHeads + g) * 2]);
             Mx = fmaxf(Mx, sk);
-            for (int ww = 0; ww < kCgWarps; ++ww) {
+            for (int ww = 0; ww < NW; ++ww) {
                 const float mw = s_ml[(ww * kCgHeads + g) * 2], f = mw > -INFINITY ? expf(mw - Mx) : 0.f;
                 L = fmaf(s_ml[(ww * kCgHeads + g) * 2 + 1], f, L);
                 O = fmaf(s_o[(ww * kCgHeads + g) * vdim + c], f, O);
@@ -705,29 +705,35 @@ static bool capturing(cudaStream_t st) {
     cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(st, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone;
 }
+// Unsplit steps of a block per SM and more take blocks of six warps: what bounds one is the chain of a warp's rounds (issue slots 33 %), and with two
+// blocks of four warps on an SM 1040 keys are nine of them, with six warps six.  us, four warps / six, 16 heads over 4 of 128: 64 sequences x 1024 keys
+// 42.9 / 37.1, x 128 14.4 / 10.7, 128 x 2048 156 / 119; 12 over 2 of 96, 128 x 700 29.0 / 24.4; 16 over 4 of 64, 256 x 300 38.1 / 38.0.  Fewer blocks: 32 x 256
+// 10.6 and a merge / 13.5, 8 x 1024 10.5 / 11.4, 1 x 4096 10.0 / 11.2.
+constexpr int kCgManyBlocks = 148;
 static int group_blocks(const CachedAttnArgs& a) {
     return a.kv_heads * ((a.heads / a.kv_heads + kCgHeads - 1) / kCgHeads);
 }
 
-template <int MODE>
+template <int MODE, int NW>
 static int launch_group(const CachedAttnArgs& a, const Batch& b, int n_split, float* part, cudaStream_t st) {
-    const int tiles = kCgWarps * group_sizes(a.dim, a.vdim).warp_bytes, merge = kCgWarps * kCgHeads * (a.vdim + 2) * 4, smem = tiles > merge ? tiles : merge;
-    auto kernel = cached_attention_decode_group_kernel<MODE>;
+    const int tiles = NW * group_sizes(a.dim, a.vdim).warp_bytes, merge = NW * kCgHeads * (a.vdim + 2) * 4, smem = tiles > merge ? tiles : merge;
+    auto kernel = cached_attention_decode_group_kernel<MODE, NW>;
     if (smem > 48 * 1024) {                                 // (always the same limit: another thread may be between setting it and its launch)
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCgWarps * group_sizes(128, 128).warp_bytes);
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NW * group_sizes(128, 128).warp_bytes);
         if (e != cudaSuccess) return (int)e;
     }
     // (one or two blocks to an SM: brought in while the means in front of them end, they fall on the SMs unevenly, 60 -> 62 us of 64
     // sequences; in a model's step the kernel in front is over sooner)
-    chain_launch_if(in_chain(), kernel, dim3(n_split, group_blocks(a), b.n_seqs), 32 * kCgWarps, smem, st, a, b, n_split, part);
+    chain_launch_if(in_chain(), kernel, dim3(n_split, group_blocks(a), b.n_seqs), 32 * NW, smem, st, a, b, n_split, part);
     if (n_split > 1) chain_launch(cached_attention_merge_kernel<__nv_bfloat16, MODE>, b.n_tokens * a.heads, a.vdim <= 128 ? 128 : 256, 0, st, a, n_split, part);
     return 0;
 }
+template <int NW>
 static int launch_group_any(int mode, const CachedAttnArgs& a, const Batch& b, int n_split, float* part, cudaStream_t st) {
     switch (mode) {
-        case UMBS_ATTN_SOFTMAX: return launch_group<UMBS_ATTN_SOFTMAX>(a, b, n_split, part, st);
-        case UMBS_ATTN_SOFTMAX_SINK: return launch_group<UMBS_ATTN_SOFTMAX_SINK>(a, b, n_split, part, st);
-        case UMBS_ATTN_SIGMOID: return launch_group<UMBS_ATTN_SIGMOID>(a, b, n_split, part, st);
+        case UMBS_ATTN_SOFTMAX: return launch_group<UMBS_ATTN_SOFTMAX, NW>(a, b, n_split, part, st);
+        case UMBS_ATTN_SOFTMAX_SINK: return launch_group<UMBS_ATTN_SOFTMAX_SINK, NW>(a, b, n_split, part, st);
+        case UMBS_ATTN_SIGMOID: return launch_group<UMBS_ATTN_SIGMOID, NW>(a, b, n_split, part, st);
     }
     return UMB_ERR_ARG;
 }
@@ -859,6 +865,7 @@ extern "C" int umbs_cached_attention_ex(int dtype, int mode, const void* q, cons
         const size_t per_split = (size_t)rows * (vdim + 2) * sizeof(float);
         const int room = split_scratch == nullptr || per_split == 0 ? 1 : (int)std::clamp<size_t>(split_bytes / per_split, 1, 32);
         int n_split = 1;
+        bool group_many = false;
         if (group) {
             // heads that share a key/value head in one block, three blocks on an SM, 128 keys a round of its warps: the split with
             // the fewest rounds from first to last block, one more per block for its start and end
@@ -868,12 +875,13 @@ extern "C" int umbs_cached_attention_ex(int dtype, int mode, const void* q, cons
                 const int64_t cost = (blocks * n + 443) / 444 * ((keys + n * 128 - 1) / (n * 128) + 1) + (n > 1);
                 if (cost < best) { best = cost; n_split = n; }
             }
+            group_many = n_split == 1 && blocks >= kCgManyBlocks;
         } else {
             n_split = (keys + 255) / 256;
             n_split = n_split < 1 ? 1 : (n_split > 32 ? 32 : n_split);
             n_split = std::min(n_split, std::min((296 + rows - 1) / rows, room));
         }
-        if (group) rc = launch_group_any(mode, a, *batch, n_split, split_scratch, st);
+        if (group) rc = (group_many ? launch_group_any<6> : launch_group_any<4>)(mode, a, *batch, n_split, split_scratch, st);
         else if (dtype == UMBS_BF16) rc = launch_decode_any<__nv_bfloat16>(mode, a, *batch, n_split, split_scratch, st);
         else if (dtype == UMBS_F32) rc = launch_decode_any<float>(mode, a, *batch, n_split, split_scratch, st);
         else return UMB_ERR_ARG;
