@@ -1,4 +1,4 @@
-"""What a decode step reads of a cache: means of whole blocks (umbs_kv_pool) bit for bit, and the grouped attention with four and with six warps
+"""What a decode step reads of a cache: means of whole blocks (umbs_kv_pool) bit for bit, the routing of up to 64 tokens bit for bit, and the grouped attention with four and with six warps
 a block (unsplit steps from 148 blocks on) against float64.
 
 Tolerance: results are bf16 (2^-9 of their size at most, 2^-9 / sqrt(3) in the norm); the fp32 work inside is four orders below."""
@@ -56,3 +56,21 @@ def test_groups_of_heads(mode, seqs, kv_heads, group, dim, ctx):
             w = torch.softmax(e, 2)[..., :pos[i] + 1]
         want = torch.einsum("hgj,jhd->hgd", w, rows[:, 1]).reshape(-1)
         assert H.rel_err(out[i], want) < 2.0 ** -9
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,experts,width,top,gate", [(17, 15, 100, 2, True), (17, 16, 1024, 3, False), (64, 16, 1152, 2, True), (64, 17, 2052, 1, False), (64, 300, 64, 9, True),
+                                                      (20, 1024, 1030, 4, False), (20, 1025, 128, 4, False)])
+def test_routing_of_few_tokens(dt, n, experts, width, top, gate):
+    """A block to a token and warps with one or two experts choose what four tokens to a block and four experts to a warp do (the same tokens among 70)."""
+    from umbrella_b200 import _lib_seq as S, ops_seq as K
+    g = torch.Generator().manual_seed(9)
+    h, w, gw = torch.randn(70, width, generator=g).to(dt).to(DEV), torch.randn(experts, width, generator=g).to(DEV), torch.randn(width, generator=g).to(DEV)
+    few, many = (K.moe_route_ex(h[:m], w, top, S.UMBS_ROUTE_SOFTMAX_TOP, gate_w=gw if gate else None) for m in (n, 70))
+    for i in [0, 4] + [5] * gate:
+        assert torch.equal(few[i], many[i][:n])
+    off, tok, pos, sel = (t.cpu() for t in few[1:5])
+    assert torch.equal(off, torch.cat([torch.zeros(1), torch.bincount(sel.flatten().long(), minlength=experts).cumsum(0)]).int())
+    place = pos.view(n, top).long()
+    assert torch.equal(tok[place], torch.arange(n, dtype=torch.int32)[:, None].expand(n, top)) and torch.equal(place.flatten().sort().values, torch.arange(n * top))
+    assert bool(((place >= off[sel.long()]) & (place < off[sel.long() + 1])).all())

@@ -601,7 +601,7 @@ __device__ __forceinline__ void router_logits(const T* const (&hr)[TT], const fl
         for (int e = 0; e < EE; ++e) s[t][e] = 0.f;
     if (vec) {
         // several pieces of 128 in flight at a time: a step of few tokens is a chain of load latencies (64 tokens, 16 experts of
-        // width 2048: 23.6 us a piece at a time, 13.7 us four; with eight tokens to a warp two are what the registers hold)
+        // width 2048: 23.6 us a piece at a time, 13.7 us four; one token to a warp: eight; with eight tokens to a warp two are what the registers hold)
         auto pieces = [&](auto count, int k0) {
             constexpr int U = decltype(count)::value;
             typename Raw4<T>::type hr4[U][TT];
@@ -629,7 +629,7 @@ __device__ __forceinline__ void router_logits(const T* const (&hr)[TT], const fl
             }
         };
         int k = lane * 4;
-        constexpr int U = TT <= 4 ? 4 : 2;
+        constexpr int U = TT == 1 ? 8 : (TT <= 4 ? 4 : 2);
         for (; k + 128 * (U - 1) < width; k += 128 * U) pieces(std::integral_constant<int, U>{}, k);
         for (; k < width; k += 128) pieces(std::integral_constant<int, 1>{}, k);
     } else {
@@ -746,14 +746,13 @@ __device__ __forceinline__ void route_choose(float* z, int experts, int top, int
     for (int k = 0; k < top; ++k) w_out[k] = w_out[k] / den * wscale;
 }
 
-// One block per kRtTok tokens: a warp works out the logits of kRtExp experts for all of them, so that a router weight is
+// One block per kRtTok tokens (which and kRtExp: at the launch): a warp works out the logits of kRtExp experts for all of them, so that a router weight is
 // fetched once per kRtTok tokens and a token's number once per kRtExp experts; then a thread per token chooses.  (A block per
 // token read all weights for each token: 512 MB through L2 for 4096 tokens, 16 experts of width 2048, 112 us.)
-constexpr int kRtExp = 4;
 constexpr int kRtPairs = 1024;         // up to so many pairs are handed out by the router's last block
 
-template <typename T, int kRtTok>
-__global__ void __launch_bounds__(256, kRtTok > 4 ? 2 : 1) moe_router_kernel(const T* __restrict__ h, int n, int width, const float* __restrict__ wr,
+template <typename T, int kRtTok, int kRtExp = 4>
+__global__ void __launch_bounds__(kRtTok == 1 ? 512 : 256, kRtTok > 4 ? 2 : 1) moe_router_kernel(const T* __restrict__ h, int n, int width, const float* __restrict__ wr,
                                                          int experts, int top, int mode, int groups, int keep, float wscale,
                                                          float* __restrict__ sel_w, int32_t* __restrict__ sel_e,
                                                          int32_t* __restrict__ counts, const float* __restrict__ gate_w,
@@ -1318,20 +1317,26 @@ extern "C" int umbs_moe_route_scaled(int dtype, const void* h, int n, int width,
     int32_t* sel_e = scratch + 2 * experts;    // [n top]
     cudaError_t e = cudaMemsetAsync(counts, 0, (experts + 1) * sizeof(int32_t), st);         // (and cursor[0])
     if (e != cudaSuccess) return (int)e;
-    const int rthreads = 32 * std::min(8, (experts + (gate_w != nullptr) + kRtExp - 1) / kRtExp);
-    // (more tokens to a block once there are blocks enough; thousands of experts need the larger shared memory)
-#define UMBS_ROUTER(TT)                                                                                                          \
+    // Tokens to a block, experts to a warp: few tokens are a chain of load latencies, so a block each, its warps with a row or two of the router and
+    // eight pieces in flight; more share the router's rows, most once there are blocks enough.  us for the whole call, four tokens with four experts / one with
+    // one / one with two / eight with four: width 2048, 16 experts, 20 tokens 11.4 / 9.5 / 10.4 / 14.4, 64 12.4 / 10.3 / 10.4 / 14.6, 256 13.5 / 15.5 / 16.1 /
+    // 16.5, 4096 34 / 131 / 88 / 25; 64 tokens, 128 experts 41 / 29 / 27 / 62, 256 of width 4096 91 / 57 / 52 / 154, 8 of width 4096 14.5 / 10.4 / 10.5 / 18.5.
+    // (thousands of experts need the larger shared memory)
+    const int rrows = experts + (gate_w != nullptr);
+#define UMBS_ROUTER(TT, EE, NW)                                                                                                          \
     UMBS_DISPATCH_T(dtype, {                                                                                                     \
         const size_t smem = (size_t)TT * experts * sizeof(float);                                                                \
         if (smem > 48 * 1024) {     /* always the same limit: another thread may be between setting it and its launch */          \
-            e = cudaFuncSetAttribute(moe_router_kernel<T, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);          \
+            e = cudaFuncSetAttribute((moe_router_kernel<T, TT, EE>), cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);          \
             if (e != cudaSuccess) return (int)e;                                                                                 \
         }                                                                                                                        \
-        chain_launch(moe_router_kernel<T, TT>, (n + TT - 1) / TT, rthreads, smem, st, (const T*)h, n, width, w_router, experts, top, mode, groups, keep, \
+        chain_launch((moe_router_kernel<T, TT, EE>), (n + TT - 1) / TT, 32 * std::min(NW, (rrows + EE - 1) / EE), smem, st, (const T*)h, n, width, w_router, experts, top, mode, groups, keep, \
                                                                             weight_scale, sel_w, sel_e, counts, gate_w, gate_out, cursor, grp_off, pair_tok, pair_pos); \
     })
-    if (n > 1024 && experts <= 1024) UMBS_ROUTER(8);
-    else UMBS_ROUTER(4);
+    if (n <= 64 && rrows <= 16) UMBS_ROUTER(1, 1, 16);
+    else if (n <= 64 && experts <= 1024) UMBS_ROUTER(1, 2, 16);
+    else if (n > 1024 && experts <= 1024) UMBS_ROUTER(8, 4, 8);
+    else UMBS_ROUTER(4, 4, 8);
 #undef UMBS_ROUTER
     const int pairs = n * top;
     if (pairs > kRtPairs) chain_launch(moe_scatter_kernel, (pairs + 255) / 256, 256, 0, st, (const int32_t*)sel_e, pairs, top, (const int32_t*)grp_off, cursor, pair_tok, pair_pos);
