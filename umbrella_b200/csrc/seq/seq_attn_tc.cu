@@ -196,10 +196,12 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
         };
         for (int i = 0; i < kt.n; ++i) {
             const int base = kt.base(i), last = kt.last(i), ks = i % z.k_held, vs = i % z.v_held;
-            // rows that are neighbours: of the step, or of the ring where it does not begin again
-            const bool of_step = base >= pos0 && base + kTaK - 1 <= last, of_ring = !STEP && base + kTaK <= pos0 && base % a.kv_len + kTaK <= a.kv_len && (int64_t)(slot + 1) * a.kv_len <= z.ring_rows;
+            // rows that are neighbours: of the step (behind its sequence's last come the next one's, whose weights are 0, and zeros behind the step's:
+            // prompts of 20 tokens 13.3 us when those tiles were copied row by row), or of the ring where it does not begin again
+            const int at0 = STEP ? 0 : base % a.kv_len;     // the first key's place in the ring
+            const bool of_step = base >= pos0, of_ring = !STEP && base + kTaK <= pos0 && at0 + kTaK <= a.kv_len && (int64_t)(slot + 1) * a.kv_len <= z.ring_rows;
             const bool tma = z.tma && !kt.pooled(i) && (of_step || of_ring);
-            const int row = of_step ? start + base - pos0 : (of_ring ? slot * a.kv_len + base % a.kv_len : 0);
+            const int row = of_step ? start + base - pos0 : (of_ring ? slot * a.kv_len + at0 : 0);
             // this thread's row p of four, 32 h behind the tile's first: where its keys and its values are (behind the last row: anywhere)
             auto row_of = [&](int h, int p, const __nv_bfloat16*& kp, const __nv_bfloat16*& vp) -> bool {
                 const int j = base + r0 + 32 * h + 8 * p;
@@ -210,10 +212,12 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
                     vp = (const __nv_bfloat16*)x.v + t * x.ldv + (int64_t)vh * a.vdim;
                 } else {
                     const __nv_bfloat16* row = (const __nv_bfloat16*)a.kv;
+                    int place = at0 + j - base;
+                    if (place >= a.kv_len) place = a.kv_len >= kTaK ? place - a.kv_len : j % a.kv_len;
                     if (ok)
                         row = kt.pooled(i) ? (const __nv_bfloat16*)a.pool_cache + ((int64_t)slot * a.pool_len + j) * vhd.row_kv
                             : j >= pos0 ? (const __nv_bfloat16*)a.kv + (int64_t)(start + j - pos0) * vhd.row_kv
-                                        : (const __nv_bfloat16*)a.kv_cache + ((int64_t)slot * a.kv_len + j % a.kv_len) * vhd.row_kv;
+                                        : (const __nv_bfloat16*)a.kv_cache + ((int64_t)slot * a.kv_len + place) * vhd.row_kv;
                     kp = row + vhd.koff;
                     vp = row + vhd.voff;
                 }
