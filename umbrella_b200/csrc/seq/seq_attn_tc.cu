@@ -4,8 +4,8 @@
 // A block = 128 consecutive query rows of one (sequence, head) = the 128 lanes of tensor memory; two blocks share an
 // SM.  Tiles of 64 keys:
 //   warps 9-10 bring key and value rows into the 128-byte-swizzled images the tensor core reads, ahead of their use: with TMA
-//              where the 64 rows are neighbours in the step and heads are whole pieces of 64 numbers, else with 16-byte
-//              cp.async, each row from where it lives (step, ring, block table), zeros where there is none;
+//              where the 64 rows are neighbours in the step or in the ring, else (the tile between the two, pooled blocks) with
+//              16-byte cp.async, each row from where it lives (step, ring, block table), zeros where there is none;
 //   warp 8     one thread issues S = Q K^T of the next tile, then O += P V of this one, accumulators in tensor memory;
 //   warps 0-7  two threads per row, 32 keys each: scores to weights in fp32 in the base-2 domain, an online reference that only moves
 //              when a score of either passes it by 2^8 (then O is rescaled, half of its columns each), the row's sum.
@@ -21,8 +21,10 @@
 //
 // Bound: two blocks take 2200 to 2400 ns a tile each (one alone 1650): a row's weights behind the scores and in front of the products (560 instructions a
 // warp and tile, issue slots 52 % taken, tensor pipe 35 % active), and blocks that fill the SMs 1.7 times.  us, 32 keys a tile / this: 4096 tokens, 16 heads of 128 over 4 key/value heads,
-// window 1024, pooled blocks 115 / 109; two prompts of 2000 tokens, 16 heads of 128 + 64 shared, a gate per column 156 / 111 (blocks that see most keys first,
-// over all heads: 40 of it; results through shared memory: 4 to 12 us of a block's 60); 3 x 700 tokens behind 700, heads of 96, 56 / 50; 300 tokens 27 / 27.
+// window 1024, pooled blocks 115 / 100; two prompts of 2000 tokens, 16 heads of 128 + 64 shared, a gate per column 156 / 103 (blocks that see most keys first,
+// over all heads: 40 of it; results through shared memory: 4 to 12 us of a block's 60); 106 tokens behind 700, heads of 96, 49 / 32.  A short prompt's block runs
+// every instruction once, and what it waits for is the next ones (2500 clocks for the first tile's weights, 3000 for 16 unrolled rows of results, 1250 as a
+// loop): eight prompts of 20 tokens 10.3 / 9.4, of 110 13.0 / 11.5, three of 77, 8 heads of 64, 9.8 / 10.1.
 #include <algorithm>
 
 #include "seq_attn.h"
@@ -124,23 +126,6 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
     uint64_t *k_full = bars, *k_empty = k_full + kTaHeld, *v_full = k_empty + kTaHeld, *v_empty = v_full + kTaHeld, *s_full = v_empty + kTaHeld, *p_full = s_full + 2,
              *o_full = s_full + 4, *q_full = s_full + 5, *lo_full = s_full + 6;       // (p_full: two in turn, a warp may be a tile ahead of another there)
     volatile int* quit = &s_quit;
-    chain_wait_only();
-    // heads fastest, query tiles slowest and the last ones first: the blocks that see most keys start first, over all heads and sequences
-    const int s = blockIdx.y, vh = blockIdx.x, q0 = (int)(gridDim.z - 1 - blockIdx.z) * kTaQ;
-    const int len = b.seq_len[s], start = b.seq_start[s], pos0 = STEP ? 0 : b.seq_pos0[s], slot = STEP ? 0 : b.seq_slot[s];
-    if (q0 >= len) return;
-    VHead vhd;
-    if (STEP) { vhd.h = vh; vhd.qoff = vh * a.dim; vhd.nv = a.heads; }
-    else vhd = virtual_head(a, vh);
-    const int h = vhd.h, window = a.window > 0 ? a.window : (1 << 30);
-    const KeyTiles kt(a, window, pos0, q0, len);
-    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-    const int k_bytes = z.q_atoms * (kTaK * 128), v_bytes = z.v_atoms * (kTaK * 128);
-    unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    unsigned char* s_k = smem + z.q_atoms * (kTaQ * 128);   // Q [q_atoms][128 rows][128 B], tiles of K [q_atoms][64][128 B], of V [v_atoms][64][128 B]
-    unsigned char* s_v = s_k + z.k_held * k_bytes;
-    unsigned char* s_lo = s_v + z.v_held * v_bytes;         // third parts of the weights [128 rows][64 keys]
-
     if (threadIdx.x == 0) {
         for (int i = 0; i < kTaHeld; ++i) {
             umb::mbar_init(k_full + i, 2);
@@ -158,6 +143,23 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
         s_quit = 0;
         umb::fence_barrier_init();
     }
+    chain_wait_only();
+    // heads fastest, query tiles slowest and the last ones first: the blocks that see most keys start first, over all heads and sequences
+    const int s = blockIdx.y, vh = blockIdx.x, q0 = (int)(gridDim.z - 1 - blockIdx.z) * kTaQ;
+    const int len = b.seq_len[s], start = b.seq_start[s], pos0 = STEP ? 0 : b.seq_pos0[s], slot = STEP ? 0 : b.seq_slot[s];
+    if (q0 >= len) return;
+    VHead vhd;
+    if (STEP) { vhd.h = vh; vhd.qoff = vh * a.dim; vhd.nv = a.heads; }
+    else vhd = virtual_head(a, vh);
+    const int h = vhd.h, window = a.window > 0 ? a.window : (1 << 30);
+    const KeyTiles kt(a, window, pos0, q0, len);
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int k_bytes = z.q_atoms * (kTaK * 128), v_bytes = z.v_atoms * (kTaK * 128);
+    unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* s_k = smem + z.q_atoms * (kTaQ * 128);   // Q [q_atoms][128 rows][128 B], tiles of K [q_atoms][64][128 B], of V [v_atoms][64][128 B]
+    unsigned char* s_v = s_k + z.k_held * k_bytes;
+    unsigned char* s_lo = s_v + z.v_held * v_bytes;         // third parts of the weights [128 rows][64 keys]
+
     if (warp == 8) {
         umb::tmem_alloc(&s_tmem, 256);
         umb::tmem_relinquish();
@@ -352,6 +354,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
         const float r1h = SHAPED && a.r1 ? a.r1[h] : 0.f, r2h = SHAPED && a.r1 ? a.r2[h] : 0.f;
         float m = MODE == UMBS_ATTN_SOFTMAX_SINK ? sink_score(a, h) * kLog2e : -INFINITY;      // the sink: a key of this score ...
         float l = MODE == UMBS_ATTN_SOFTMAX_SINK && half == 0 ? 1.f : 0.f;                     // ... without a value; the sum over this thread's keys
+        const float gl = a.gate != nullptr && a.gate_per_head && r < len ? a.gate[(int64_t)(start + r) * a.ldg + h] : 0.f;
         const int tok_lo = max(rp - window + 1, a.chunk > 0 ? rp / a.chunk * a.chunk : 0);
         const int pool_hi = pooled_visible(rp, window, a.pool);
         {   // the queries: 8 threads per 128-byte row piece
@@ -499,7 +502,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
         if (ok) {
             umb::tc_fence_after();
             const float inv = MODE == UMBS_ATTN_SIGMOID ? 1.f : 1.f / l;
-            const float gh = a.gate != nullptr && a.gate_per_head && r < len ? sigmoidf_(a.gate[(int64_t)(start + r) * a.ldg + h]) : 1.f;
+            const float gh = a.gate != nullptr && a.gate_per_head && r < len ? sigmoidf_(gl) : 1.f;
             for (int c0 = half * 64; c0 < min(a.vdim, half * 64 + 64); c0 += 32) {
                 uint32_t v[32];
                 UMB_TMEM_LD_X32(t0 + 128 + c0, v);
@@ -524,24 +527,31 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
             const bool gates = a.gate != nullptr && !a.gate_per_head;
             __nv_bfloat16* op = STEP ? (__nv_bfloat16*)x.out + (int64_t)h * a.vdim + c : (__nv_bfloat16*)a.out + (int64_t)h * a.vdim + c;
             const int64_t ldout = STEP ? x.ldo : (int64_t)a.heads * a.vdim;
+            // (loops rather than one long stretch: each instruction of a short prompt's block is fetched for it alone)
+            auto put = [&](int orow, float4 o) {
+                const __nv_bfloat162 w0 = __floats2bfloat162_rn(o.x, o.y), w1 = __floats2bfloat162_rn(o.z, o.w);
+                *reinterpret_cast<uint2*>(op + (int64_t)(start + q0 + orow) * ldout) = make_uint2(*reinterpret_cast<const uint32_t*>(&w0), *reinterpret_cast<const uint32_t*>(&w1));
+            };
+            const int rows = c < a.vdim ? min(16, len - q0 - row0) : 0;
+            if (!gates) {
+#pragma unroll 4
+                for (int e = 0; e < rows; ++e) put(row0 + e, *reinterpret_cast<const float4*>(s_o + (row0 + e) * ldo + c));
+            } else {
+#pragma unroll 1
+                for (int e0 = 0; e0 < rows; e0 += 8) {
+                    float4 g[8];
 #pragma unroll
-            for (int e0 = 0; e0 < 16; e0 += 8) {
-                float4 g[8];
+                    for (int e = 0; e < 8; ++e)
+                        if (e0 + e < rows) {
+                            const float* gp = a.gate + (int64_t)(start + q0 + row0 + e0 + e) * a.ldg + h * a.vdim + c;
+                            g[e] = ((uintptr_t)gp & 15) == 0 ? *reinterpret_cast<const float4*>(gp) : make_float4(gp[0], gp[1], gp[2], gp[3]);
+                        }
 #pragma unroll
-                for (int e = 0; e < 8; ++e)
-                    if (gates && q0 + row0 + e0 + e < len && c < a.vdim) {
-                        const float* gp = a.gate + (int64_t)(start + q0 + row0 + e0 + e) * a.ldg + h * a.vdim + c;
-                        g[e] = ((uintptr_t)gp & 15) == 0 ? *reinterpret_cast<const float4*>(gp) : make_float4(gp[0], gp[1], gp[2], gp[3]);
-                    }
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const int orow = row0 + e0 + e;
-                    if (q0 + orow < len && c < a.vdim) {
-                        float4 o = *reinterpret_cast<const float4*>(s_o + orow * ldo + c);
-                        if (gates) o = make_float4(o.x * tc_sigmoid(g[e].x), o.y * tc_sigmoid(g[e].y), o.z * tc_sigmoid(g[e].z), o.w * tc_sigmoid(g[e].w));
-                        const __nv_bfloat162 w0 = __floats2bfloat162_rn(o.x, o.y), w1 = __floats2bfloat162_rn(o.z, o.w);
-                        *reinterpret_cast<uint2*>(op + (int64_t)(start + q0 + orow) * ldout) = make_uint2(*reinterpret_cast<const uint32_t*>(&w0), *reinterpret_cast<const uint32_t*>(&w1));
-                    }
+                    for (int e = 0; e < 8; ++e)
+                        if (e0 + e < rows) {
+                            const float4 o = *reinterpret_cast<const float4*>(s_o + (row0 + e0 + e) * ldo + c);
+                            put(row0 + e0 + e, make_float4(o.x * tc_sigmoid(g[e].x), o.y * tc_sigmoid(g[e].y), o.z * tc_sigmoid(g[e].z), o.w * tc_sigmoid(g[e].w)));
+                        }
                 }
             }
         }
