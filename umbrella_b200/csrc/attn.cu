@@ -127,7 +127,10 @@ __device__ __forceinline__ unsigned long long row_window(const AttnParams& p, in
     return allow & exist;
 }
 
-template <int D, bool kSoftCap>
+// kTwoParts: a weight goes into the second product as two fp16 numbers (what is left of it behind the first one's rounding is the second).  The
+// slab kernel below rounds each warp's largest weight to itself (it is 1), this kernel one weight of the row: 500 rows 2.46e-4 from float64 with
+// one part against the slabs' 2.39e-4, with two the rounding of the result alone.
+template <int D, bool kSoftCap, bool kTwoParts>
 __global__ void __launch_bounds__(kAttnThreads) tree_attn_kernel(const AttnParams p) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __half* sK = reinterpret_cast<__half*>(smem_raw);                 // [2][kBN][D]
@@ -142,7 +145,8 @@ __global__ void __launch_bounds__(kAttnThreads) tree_attn_kernel(const AttnParam
     const int prefix_len = p.dyn ? p.dyn[0] + p.prefix_len : p.prefix_len;
     const int kv_len = p.dyn ? p.dyn[0] + p.kv_len : p.kv_len;
 
-    const int row_base = blockIdx.x * kBM + warp * 16;
+    const int bx = p.mask_mode == UMB_MASK_CAUSAL ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;      // (rows that see most start first)
+    const int row_base = bx * kBM + warp * 16;
     // the two rows this thread owns inside its warp's 16-row slab
     int row[2], tok[2];
     bool row_ok[2];
@@ -174,7 +178,7 @@ __global__ void __launch_bounds__(kAttnThreads) tree_attn_kernel(const AttnParam
     // ---- kv range of this CTA ----
     int kv_hi = kv_len;
     if (p.mask_mode == UMB_MASK_CAUSAL) {
-        const int last_row = min(rows_total, (int)(blockIdx.x + 1) * kBM) - 1;
+        const int last_row = min(rows_total, (bx + 1) * kBM) - 1;
         kv_hi = min(kv_hi, prefix_len + last_row / p.G + 1);
     } else if (p.mask_mode == UMB_MASK_TREE) {
         kv_hi = min(kv_hi, prefix_len + p.tree_words * 32);   // columns the bitmask can describe
@@ -295,6 +299,14 @@ __global__ void __launch_bounds__(kAttnThreads) tree_attn_kernel(const AttnParam
             a[1] = pack_half2(s[2 * ks][2], s[2 * ks][3]);
             a[2] = pack_half2(s[2 * ks + 1][0], s[2 * ks + 1][1]);
             a[3] = pack_half2(s[2 * ks + 1][2], s[2 * ks + 1][3]);
+            uint32_t low[4];
+            if constexpr (kTwoParts) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 hi = __half22float2(*reinterpret_cast<const __half2*>(&a[i]));
+                    low[i] = pack_half2(s[2 * ks + (i >> 1)][(i & 1) * 2] - hi.x, s[2 * ks + (i >> 1)][(i & 1) * 2 + 1] - hi.y);
+                }
+            }
 #pragma unroll
             for (int db = 0; db < D / 8; db += 2) {
                 uint32_t b[4];
@@ -303,6 +315,10 @@ __global__ void __launch_bounds__(kAttnThreads) tree_attn_kernel(const AttnParam
                 ldmatrix_x4_trans(b, tile_ptr<D>(const_cast<__half*>(tV), r, c));
                 mma_16816(o_acc[db], a, b[0], b[1]);
                 mma_16816(o_acc[db + 1], a, b[2], b[3]);
+                if constexpr (kTwoParts) {
+                    mma_16816(o_acc[db], low, b[0], b[1]);
+                    mma_16816(o_acc[db + 1], low, b[2], b[3]);
+                }
             }
         }
         __syncthreads();   // the buffer is re-filled two iterations later
@@ -342,6 +358,11 @@ __global__ void __launch_bounds__(kAttnThreads) tree_attn_kernel(const AttnParam
 // in the loop), and merge their (m, l, o) partials through shared memory at the end.
 // ------------------------------------------------------------------------------------------------
 constexpr int kSBN = 32;
+// From so many tiles of 64 rows on (over all key/value heads) rows share a tile's keys: slabs of 16 rows, one to an SM, are then several rounds that each fetch
+// all of them again.  us, slabs / tiles with weights in two parts, heads of 128, 32 over 8: 500 rows 47.6 / 27.9, behind 1000 cached 96.5 / 73.0, 256 rows 18.1 / 15.4
+// (128 tiles), 128 rows 8.3 / 8.7, behind 1000 27.2 / 25.5; 64 over 8: 500 rows 89.4 / 44.2, a tree of 385 behind 500 120 / 92, of 64 18.5 / 20.0; heads of 64, 200 rows behind
+// 3000 44 / 54 (104 tiles).  Distance to float64 2.6e-4 / 2.1e-4.
+constexpr int kManyRowTiles = 128;
 constexpr int kSlabTilesPerCta = 32;     // minimum kv tiles per slab CTA before the KV range is split across CTAs
 
 template <int D>
@@ -1108,16 +1129,23 @@ static int launch_slab(const AttnParams& p, dim3 grid, cudaStream_t st) {
     return UMB_OK;
 }
 
+template <int D, bool kSoftCap, bool kTwoParts>
+static int launch_tile(const AttnParams& p, dim3 grid, cudaStream_t st) {
+    const size_t smem = (size_t)4 * kBN * D * sizeof(__half);
+    if (smem > 48 * 1024)
+        UMB_CUDA(cudaFuncSetAttribute(tree_attn_kernel<D, kSoftCap, kTwoParts>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    UMB_LAUNCH_PDL((tree_attn_kernel<D, kSoftCap, kTwoParts>), grid, dim3(kAttnThreads), smem, st, p);
+    return UMB_OK;
+}
+
 template <int D, bool kSoftCap>
-static int launch_attn(const AttnParams& p, bool slab, int slab_warps, dim3 grid, cudaStream_t st) {
+static int launch_attn(const AttnParams& p, bool slab, int slab_warps, bool two_parts, dim3 grid, cudaStream_t st) {
     if (slab) {
         const int rc = slab_warps == 8 ? launch_slab<D, kSoftCap, 8>(p, grid, st) : launch_slab<D, kSoftCap, 4>(p, grid, st);
         if (rc != UMB_OK) return rc;
     } else {
-        const size_t smem = (size_t)4 * kBN * D * sizeof(__half);
-        if (smem > 48 * 1024)
-            UMB_CUDA(cudaFuncSetAttribute(tree_attn_kernel<D, kSoftCap>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        UMB_LAUNCH_PDL(tree_attn_kernel<D, kSoftCap>, grid, dim3(kAttnThreads), smem, st, p);
+        const int rc = two_parts ? launch_tile<D, kSoftCap, true>(p, grid, st) : launch_tile<D, kSoftCap, false>(p, grid, st);
+        if (rc != UMB_OK) return rc;
     }
     int launches = 1;
     if (p.splits > 1) {
@@ -1209,10 +1237,11 @@ extern "C" int umb_tree_attn_f16(const void* q, const void* k_cache, const void*
 
 #endif
     // kernel + split selection.  slab kernel: K/V is re-read once per 16-row slab (L2), so it is used
-    // while that re-read is cheap; long contexts with many slabs go to the 64-row tile kernel.
+    // while that re-read is cheap; long contexts with many slabs, and many rows, go to the 64-row tile kernel.
     const int rows_total = qo * p.G;
     const int slabs = (rows_total + 15) / 16;
-    const bool slab = !(kv_bound > 8192 && slabs > 2);
+    const bool near = !(kv_bound > 8192 && slabs > 2);
+    const bool many_rows = near && (rows_total + kBM - 1) / kBM * p.Hkv >= kManyRowTiles, slab = near && !many_rows;
     const int ctas_base = (slab ? slabs : (rows_total + kBM - 1) / kBM) * p.Hkv;
     const int kv_tiles = (kv_bound + (slab ? kSBN : kBN) - 1) / (slab ? kSBN : kBN);
     static int slab_tiles = 0;                                // UMB_ATTN_SLAB_TILES: tuning override (read once)
@@ -1251,7 +1280,8 @@ extern "C" int umb_tree_attn_f16(const void* q, const void* k_cache, const void*
     if (warps_override == 4 || warps_override == 8) slab_warps = warps_override;
     cudaStream_t st = (cudaStream_t)stream;
     if (head_dim == 128)
-        return soft_cap > 0.f ? launch_attn<128, true>(p, slab, slab_warps, grid, st)
-                              : launch_attn<128, false>(p, slab, slab_warps, grid, st);
-    return soft_cap > 0.f ? launch_attn<64, true>(p, slab, slab_warps, grid, st) : launch_attn<64, false>(p, slab, slab_warps, grid, st);
+        return soft_cap > 0.f ? launch_attn<128, true>(p, slab, slab_warps, many_rows, grid, st)
+                              : launch_attn<128, false>(p, slab, slab_warps, many_rows, grid, st);
+    return soft_cap > 0.f ? launch_attn<64, true>(p, slab, slab_warps, many_rows, grid, st)
+                          : launch_attn<64, false>(p, slab, slab_warps, many_rows, grid, st);
 }
