@@ -20,7 +20,7 @@
 // and one score tile, so that scores, weights and output products take turns: 4500 per tile, with one thread per row 5800.)
 //
 // Bound: two blocks take 2200 to 2400 ns a tile each (one alone 1650): a row's weights behind the scores and in front of the products (560 instructions a
-// warp and tile, issue slots 52 % taken, tensor pipe 35 % active), and blocks that fill the SMs 1.7 times.  us, 32 keys a tile / this: 4096 tokens, 16 heads of 128 over 4 key/value heads,
+// warp and tile, issue slots 56 % taken, tensor pipe 39 % active), and blocks that fill the SMs 1.7 times.  us, 32 keys a tile / this: 4096 tokens, 16 heads of 128 over 4 key/value heads,
 // window 1024, pooled blocks 115 / 100; two prompts of 2000 tokens, 16 heads of 128 + 64 shared, a gate per column 156 / 103 (blocks that see most keys first,
 // over all heads: 40 of it; results through shared memory: 4 to 12 us of a block's 60); 106 tokens behind 700, heads of 96, 49 / 32.  A short prompt's block runs
 // every instruction once, and what it waits for is the next ones (2500 clocks for the first tile's weights, 3000 for 16 unrolled rows of results, 1250 as a

@@ -705,7 +705,7 @@ static bool capturing(cudaStream_t st) {
     cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(st, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone;
 }
-// Unsplit steps of a block per SM and more take blocks of six warps: what bounds one is the chain of a warp's rounds (issue slots 33 %), and with two
+// Unsplit steps of a block per SM and more take blocks of six warps: what bounds one is the chain of a warp's rounds (issue slots 33 %, with six warps 40 %), and with two
 // blocks of four warps on an SM 1040 keys are nine of them, with six warps six.  us, four warps / six, 16 heads over 4 of 128: 64 sequences x 1024 keys
 // 42.9 / 37.1, x 128 14.4 / 10.7, 128 x 2048 156 / 119; 12 over 2 of 96, 128 x 700 29.0 / 24.4; 16 over 4 of 64, 256 x 300 38.1 / 38.0.  Fewer blocks: 32 x 256
 // 10.6 and a merge / 13.5, 8 x 1024 10.5 / 11.4, 1 x 4096 10.0 / 11.2.
