@@ -27,6 +27,7 @@
 #include <mutex>
 
 #include "gemm_core.cuh"
+#include "group_gate.h"
 
 namespace umb {
 namespace {
@@ -111,7 +112,7 @@ __device__ __forceinline__ bool spin_bar(uint64_t* bar, uint32_t parity, volatil
         : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return __all_sync(0xffffffffu, ok) || give_up(quit);
 }
-// The four warps of a group go on together or not at all: what follows holds barriers of theirs.
+// The four warps of a group go on together or not at all (GroupGate): what follows holds barriers of theirs.
 __device__ __forceinline__ bool group_all(bool ok, int bar) {
     int all = ok;
     asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %0, 0;\n\tbarrier.cta.red.and.pred q, %1, 128, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
@@ -255,6 +256,8 @@ awq_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         const int q = warp & 3, fl = q * 32 + lane;         // quarter of tensor memory, feature of the tile
         const uint32_t quarter = tmem + ((uint32_t)(q * 32) << 16);
         __half* exch = s_exch + grp * (kWideExch / 2);
+        GroupGate gate;
+        auto together = [&](bool ok) { return gate.pass(ok, [&](bool mine) { return group_all(mine, 1 + grp); }); };
         // words of a part: [4 token columns][feature][4]; which: 0 of the tile that the range begins within, 1 of a tile that it begins
         auto slot = [&](int c, int which) {
             return reinterpret_cast<uint32_t*>(p.slots) + ((size_t)(c * 2 + rank) * kWideSlots + which) * ((size_t)NPAD * kTileN) + fl * 4;
@@ -276,7 +279,7 @@ awq_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         // A tile that is not the range's last, by all three groups: finished when it is whole, else published (it is the first, and its
         // other parts are not this pair's to add).
         auto leave_tile = [&](int t) -> bool {
-            if (!group_all(wait_bar(acc_full, (t - t_first) & 1, quit), 1 + grp)) return false;
+            if (!together(wait_bar(acc_full, (t - t_first) & 1, quit))) return false;
             tc_fence_after();
             const int rows = rows_of(t);
             const bool whole = t > t_first || g_first == 0;
@@ -344,7 +347,7 @@ awq_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         pdl_wait();                                         // residual, workspace and y belong to the kernels in front
         for (; ok && t < t_last; ++t) ok = leave_tile(t);
         // ------------------------------------------------------------------------------------ the range's last tile
-        ok = group_all(ok && n_units > 0 && wait_bar(last_full, 0, quit), 1 + grp);
+        ok = together(ok && n_units > 0 && wait_bar(last_full, 0, quit));
         if (ok) {
             tc_fence_after();
             const int rows = rows_of(t);                    // (t is t_last)
@@ -403,7 +406,7 @@ awq_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     const int next = c + 1 == me ? c + 2 : c + 1;
                     if (next <= c1) load(next, j);
                 }
-                if (!(ok = group_all(ok, 1 + grp))) break;
+                if (!(ok = together(ok))) break;
                 to_rows(t, j, v);
             }
         }
