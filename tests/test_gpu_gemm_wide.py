@@ -104,3 +104,15 @@ def test_passes_of_a_prompt_agree(rows):
         out.append((m.prefill_forward(ids, pos, last_only=False), m.k_cache[:, :rows].clone() if m.k_cache.shape[1] >= rows else m.k_cache.clone()))
     (a, ka), (b, kb) = out
     assert float((a - b).norm() / a.norm()) < 4e-3 and float((ka - kb).float().norm() / ka.float().norm()) < 4e-3        # fp16: a few roundings of 2^-11
+
+
+@pytest.mark.parametrize("M", [13, 64, 100, 300])
+def test_silu_rounds_its_quotient(M):
+    """fp16(g / (1 + e^-g)) * up with the quotient rounded once in fp32, bit for bit (an approximate reciprocal moves one result in some ten thousand)."""
+    from umbrella_b200 import ops
+    K, N = 256, 16384
+    packed, x, ws = _setup(M, K, N, scale=0.05)
+    gate, up = _run(x, packed, K, N, ws).view(M, N // 128, 2, 64).unbind(2)
+    g = gate.float()
+    want = (g / (1 + torch.exp(-g))).to(torch.float16) * up
+    assert torch.equal(_run(x, packed, K, N, ws, mode=ops.UMB_EPI_SILU_MUL), want.reshape(M, N // 2))

@@ -94,12 +94,7 @@ struct GemmParams {
     unsigned long long* trace;     // debug timeline [grid][16] (UMB_GEMM_TRACE=1), else NULL
 };
 
-// The quotient without the rounded division's branch, which keeps a thread's eight apart: the hardware's approximate reciprocal and a
-// Newton-Raphson step, within 2^-22 of f / (1 + e^-f), which is rounded to fp16 next; behind 2^126 the reciprocal is 0.
-__device__ __forceinline__ float silu_f(float f) {
-    const float x = 1.f + expf(-f), r = __fdividef(1.f, x);
-    return f * (x >= 0x1p126f ? 0.f : fmaf(r, fmaf(-x, r, 1.f), r));
-}
+__device__ __forceinline__ float silu_f(float f) { return f / (1.f + expf(-f)); }
 __device__ __forceinline__ unsigned int orderable_f32_g(float f) {
     const unsigned int u = __float_as_uint(f);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
