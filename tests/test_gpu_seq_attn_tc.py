@@ -288,3 +288,21 @@ def test_decode_steps_of_few_keys(ops, heads, kv_heads, dim, keys):
             short.t[name].copy_(t)
         graph.replay()
         assert H.rel_err(out, ref.cpu()) < TOL
+
+
+@pytest.mark.parametrize("own_keys", [False, True])
+def test_gates_are_rounded_quotients(ops, own_keys):
+    """A row that sees itself alone with a score of 0 is its value times its gates: fp32 1 / (1 + e^-g) rounded once, bit for bit, down to the quotients
+    below the smallest normal number (where an approximate reciprocal is 0)."""
+    T, heads, D = 2048, 16, 128
+    batch = ops.RaggedBatch([(0, T, 0, 0)], DEV)
+    g = torch.Generator(device=DEV).manual_seed(5)
+    q, k, v = torch.zeros(T, heads * D, device=DEV).bfloat16(), _r(g, T, heads * D), _r(g, T, heads * D, s=1e4)
+    gate = torch.randn(T, heads * D, generator=g, device=DEV) * 2
+    gate[:, ::16] = -87 - 1.7 * torch.rand(T, heads * D // 16, generator=g, device=DEV)
+    if own_keys:
+        got = ops.window_attention_shared(q, k, None, v, batch, heads, 1.0, window=1, use_sink=False, gate=gate)
+    else:
+        got = ops.cached_attention(q, torch.cat([k, v], 1), torch.zeros(1, 8, 2 * heads * D, device=DEV).bfloat16(), batch, heads, heads, D, D, 1.0, window=1,
+                                   gate=gate, append=False)
+    assert torch.equal(got, (v.float() * (1 / (1 + torch.exp(-gate)))).bfloat16())

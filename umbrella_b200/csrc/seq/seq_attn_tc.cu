@@ -550,7 +550,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
                     for (int e = 0; e < 8; ++e)
                         if (e0 + e < rows) {
                             const float4 o = *reinterpret_cast<const float4*>(s_o + (row0 + e0 + e) * ldo + c);
-                            put(row0 + e0 + e, make_float4(o.x * tc_sigmoid(g[e].x), o.y * tc_sigmoid(g[e].y), o.z * tc_sigmoid(g[e].z), o.w * tc_sigmoid(g[e].w)));
+                            put(row0 + e0 + e, make_float4(o.x * sigmoidf_(g[e].x), o.y * sigmoidf_(g[e].y), o.z * sigmoidf_(g[e].z), o.w * sigmoidf_(g[e].w)));
                         }
                 }
             }
