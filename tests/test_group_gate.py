@@ -91,3 +91,21 @@ def test_the_kernels_barriers_pass_the_gate():
     text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "gemm_wide.cu")).read())
     uses = re.findall(r"[^\n]*\bgroup_all\([^\n]*", text)
     assert len(uses) == 2 and uses[0].startswith("__device__") and "gate.pass" in uses[1]
+
+
+def test_what_is_handed_to_the_other_block_is_released_and_acquired_there():
+    """An arrival without a scope orders what its own block sees; the barriers of a pair are arrived at from the other block.  So every remote arrival releases in
+    cluster scope, and every barrier that has one is waited for with a look that acquires in it."""
+    seen = 0
+    for name in ("gemm_wide.cu", os.path.join("seq", "seq_gemm_pair.cu")):
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
+        remote = re.findall(r"mbarrier\.arrive[^ ]*shared::cluster[^ ]*", text)
+        remote = [r for r in remote if "tcgen05" not in r and "::one" not in r]
+        assert remote and all(".release.cluster." in r for r in remote), (name, remote)
+        bars = set(re.findall(r"arrive_at\((?:first_block\()?(\w+)", text)) - {"uint32_t"}
+        for bar in bars:
+            waits = re.findall(r"(\w+)\(%s\b[^;]*quit\)" % bar, text)
+            assert waits and set(waits) == {"spin_pair"}, (name, bar, waits)
+            seen += 1
+        assert "mbarrier.test_wait.parity.acquire.cluster" in text
+    assert seen >= 3

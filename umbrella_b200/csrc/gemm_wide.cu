@@ -22,7 +22,7 @@
 // before (5 us where it is published, 10 where it is finished: the accumulator fills half of tensor memory, so there is one), and the end of
 // a range is 12 us of 100.  us, four passes of 125 rows through gemm.cu's kernel / one of 500 here: a layer of width 4096 and its head 682 / 472, of width 8192
 // 1349 / 1110; 1000 rows 1230 / 802, 300 524 / 374, 128 289 / 278, 65 272 / 262 (one pass on both sides).  Of no effect: fewer records, fewer or no x
-// copies, no arithmetic in the dequantisation (2 to 8 % each), deeper record rings; waits that acquire in cluster scope cost 1.5 times the whole.
+// copies, no arithmetic in the dequantisation (2 to 8 % each), deeper record rings.
 #include <atomic>
 #include <mutex>
 
@@ -58,7 +58,7 @@ __device__ __forceinline__ uint32_t first_block(const void* p) {            // t
     return r;
 }
 __device__ __forceinline__ void arrive_at(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tma_3d_pair(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
@@ -109,6 +109,19 @@ __device__ __forceinline__ bool spin_bar(uint64_t* bar, uint32_t parity, volatil
         "@p bra DONE_%=;\n\t"
         "add.u32 n, n, 1;\n\tsetp.lt.u32 q, n, 67108864;\n\t@q bra AGAIN_%=;\n\t"
         "DONE_%=:\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return __all_sync(0xffffffffu, ok) || give_up(quit);
+}
+// The same for a barrier that the other block's threads arrive at (arrive_at): what they did in front of that is done for this thread too.  One more look, in
+// cluster scope, once the barrier is known to be done, costs nothing that could be measured (a prompt of 500 rows 495.9 / 495.7 us with and without it; every look in
+// cluster scope: 1.5 times the whole).
+__device__ __forceinline__ bool spin_pair(uint64_t* bar, uint32_t parity, volatile int* quit) {
+    if (!spin_bar(bar, parity, quit)) return false;
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return __all_sync(0xffffffffu, ok) || give_up(quit);
 }
@@ -230,10 +243,10 @@ awq_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             bool ok = true;
             while (ok && u < n_units) {
                 const int end = u + min(n_units - u, G - in_tile);
-                if (seg > 0 && !(ok = spin_bar(acc_empty, (seg - 1) & 1, quit))) break;
+                if (seg > 0 && !(ok = spin_pair(acc_empty, (seg - 1) & 1, quit))) break;
                 for (const int first = u; u < end; ++u) {
                     const int s = u % kX, ph = (u / kX) & 1;
-                    if (!(ok = spin_bar(full_x + s, ph, quit)) || !(ok = spin_bar(full_a + s, ph, quit))) break;
+                    if (!(ok = spin_bar(full_x + s, ph, quit)) || !(ok = spin_pair(full_a + s, ph, quit))) break;
                     tc_fence_after();
                     const uint64_t bd = umma_smem_desc_sw128(smem_u32(s_x + s * Cfg::kXBytes));
                     const uint32_t a = tmem + kACol + s * 64;
