@@ -87,3 +87,19 @@ def test_logits_with_their_largest_rows_33_to_128(M):
     logits = ops.awq_gemm(x, packed, K, N, mode=ops.UMB_EPI_LOGITS, argmax=keys)
     assert logits.dtype == torch.float32 and torch.equal(logits, ops.awq_gemm(x, packed, K, N).float())
     assert torch.equal(ops.argmax_keys_to_ids(keys).cpu(), logits.cpu().argmax(-1))
+
+
+@pytest.mark.parametrize("M", [65, 100, 128])
+def test_sums_as_good_as_those_of_fewer_rows(M):
+    """A tile's k goes into two accumulators whatever its rows are, which the tensor core cuts off at each of half as many steps as one would take.  What that
+    leaves shows in how many results are not the float64 product rounded: as many as when the same rows are multiplied 64 at a time (half of one per cent
+    here; one accumulator: 1.8 times that).  A tenth more is four standard deviations of the count."""
+    from umbrella_b200 import ops
+    K, N = 14336, 4096
+    rng = np.random.default_rng(M)
+    packed = ops.awq_repack(*(torch.from_numpy(t).to(DEV) for t in oawq.random_awq(K, N, 128, rng)))
+    x = torch.from_numpy((rng.standard_normal((M, K)) * 0.5).astype(np.float16)).to(DEV)
+    want = (x.double() @ ops.awq_unpack(packed, K, N).double().t()).to(torch.float16)
+    few = torch.cat([ops.awq_gemm(x[i:i + 64], packed, K, N) for i in range(0, M, 64)])
+    off = [int((y != want).sum()) for y in (ops.awq_gemm(x, packed, K, N), few)]
+    assert 0 < off[0] < 1.1 * off[1] + 50, off

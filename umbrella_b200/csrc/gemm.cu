@@ -6,7 +6,7 @@
 //
 // Orientation ("swap-AB"): the verify pass multiplies M <= 128 token rows by a huge weight matrix,
 // so the WEIGHTS are the UMMA A operand (128 output features per tile = the 128 TMEM lanes) and the
-// token rows are the UMMA B/N operand (N = M padded to 16/32/64; fp16 weights 128 too, AWQ beyond 64 rows: gemm_wide.cu):
+// token rows are the UMMA B/N operand (N = M padded to 16/32/64/128; AWQ beyond 128 rows: gemm_wide.cu):
 //     D[128 features, MPAD tokens] (fp32, TMEM) += A[128, k] * B[MPAD, k]^T .
 // Every weight byte is read from HBM exactly once per call.
 //
@@ -163,9 +163,17 @@ __device__ __forceinline__ unsigned long long gtimer() {
 
 template <int MPAD>
 struct GemmCfg {
-    static constexpr int kDq = MPAD == 16 ? UMB_DQ_GROUPS_16 : kDqGroups;          // dequant groups per CTA (AWQ)
-    static constexpr int kThreadsAwq = 96 + 128 * (kDq + 1);
-    static constexpr int kStagesAwq = MPAD == 16 ? 10 : (MPAD == 32 ? 8 : 6);
+    // 128 rows (AWQ): weight records and x slabs in rings of their own.  A shared ring holds four units of 41 KB, and a unit
+    // occupies its place from the request over the dequantisation to the product.  The records' ring is free as soon as they
+    // are in registers, so dequantisation runs ahead of the slabs: 500 rows in four passes through a layer of width 4096 and its head
+    // 887 -> 849 us; with the heads of split tiles reduced by every group of warps (below) 683.
+    static constexpr bool kSplit = MPAD >= 128;
+    // dequant groups per CTA (AWQ).  kSplit takes two: every ring depth is a multiple of it, so a stage always comes back to
+    // the group that used it last, which the parity waits need there (see the dequant warps' note)
+    static constexpr int kDq = MPAD == 16 ? UMB_DQ_GROUPS_16 : (kSplit ? 2 : kDqGroups);
+    static constexpr int kWStages = 6;                                              // records held with kSplit
+    static constexpr int kThreadsAwq = 96 + 128 * (kDq + 1) + (kSplit ? 32 : 0);   // (the x slabs' own warp)
+    static constexpr int kStagesAwq = MPAD == 16 ? 10 : (MPAD == 32 ? 8 : (MPAD == 64 ? 6 : 4));
     static constexpr int kStagesF16 = MPAD <= 32 ? 8 : (MPAD == 64 ? 6 : 4);
     static constexpr int kXBytesAwq = MPAD * 256;           // [2 atoms][MPAD][128 B]
     static constexpr int kXBytesF16 = MPAD * 128;           // [MPAD][128 B]
@@ -186,7 +194,8 @@ struct GemmCfg {
     static constexpr int kBarBytes = 576;
     static constexpr int smem_bytes(bool awq, int stages) {
         return 1024 /*align slack*/ + kBarBytes + kExchGroups * kExchBytes +
-               stages * (awq ? (kXBytesAwq + kPackedStride) : (kXBytesF16 + kWBytesF16));
+               (awq && kSplit ? stages * kXBytesAwq + kWStages * kPackedStride
+                              : stages * (awq ? (kXBytesAwq + kPackedStride) : (kXBytesF16 + kWBytesF16)));
     }
 };
 
@@ -217,6 +226,8 @@ __device__ __forceinline__ void load_acc_sum(uint32_t taddr, float (&v)[16], int
 //                 soon as a weight record has landed, also before the predecessor kernel has finished
 //   last 4 warps  epilogue only (AWQ: warps 15..18, fp16: warps 3..6): the partial-tile fix-up is a chain of
 //                 global round trips and must not stall the dequant stream
+//   65..128 rows  (AWQ) two dequant groups, warps 3..10, which also reduce when they have no units left; epilogue warps
+//                 11..14; warp 15 requests the x slabs
 template <int MPAD, bool kAwq>
 __global__ void __launch_bounds__(kAwq ? GemmCfg<MPAD>::kThreadsAwq : kGemmThreadsF16, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
@@ -235,7 +246,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
     // the MMA warps take alternate units, so a ring stage must always come back to the same warp (parity waits, see the
     // dequant warps' note): both rings need an even depth
     static_assert(!kAwq || (kAStages % 2 == 0 && Cfg::kStagesAwq % 2 == 0), "ring depths must be even");
-    constexpr bool kShare = kAwq && Cfg::kShare;
+    constexpr bool kSplit = kAwq && Cfg::kSplit, kShare = kAwq && Cfg::kShare;
+    static_assert(!kSplit || (kAStages % Cfg::kDq == 0 && Cfg::kWStages % Cfg::kDq == 0 && Cfg::kStagesAwq == kAStages),
+                  "the rings of separate records must return each stage to its dequant group");
+    const int kWRing = kSplit ? Cfg::kWStages : kStages;        // depth of the weight records' ring
     constexpr int kDq = Cfg::kDq;                               // dequant groups of this CTA
     constexpr int kFinish = kShare ? Cfg::kExchGroups : 1;      // groups of warps that reduce the head of a split tile
 
@@ -243,7 +257,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* s_x = smem;                                   // kStages x kXBytes   (1024-aligned slabs)
     unsigned char* s_w = s_x + kStages * kXBytes;                // kStages x kWStride
-    __half* s_exch = reinterpret_cast<__half*>(s_w + kStages * kWStride);
+    __half* s_exch = reinterpret_cast<__half*>(s_w + kWRing * kWStride);
     uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(s_exch) + Cfg::kExchGroups * Cfg::kExchBytes);
     uint64_t* full_w = bars;                  // [kStages]   weight record / tile landed
     uint64_t* full_x = bars + 16;             // [kStages]   x slab landed
@@ -253,6 +267,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
     uint64_t* acc_empty = bars + 57;
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 58);
     uint64_t* last_full = bars + 59;          //             kShare: the last segment's accumulators are complete
+    uint64_t* w_empty = bars + 60;            // [kWStages]  kSplit: the record in this stage is in the dequant group's registers
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) UMB_TRACE(0);
@@ -266,9 +281,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
         tma_prefetch_desc(&tmap_x);
         tma_prefetch_desc(&tmap_w);
         for (int i = 0; i < kStages; ++i) {
-            mbar_init(full_w + i, 1);
+            if (!kSplit) mbar_init(full_w + i, 1);
             mbar_init(full_x + i, 1);
             mbar_init(done + i, 1);
+        }
+        for (int i = 0; kSplit && i < kWRing; ++i) {
+            mbar_init(full_w + i, 1);
+            mbar_init(w_empty + i, 4);
         }
         for (int i = 0; i < kAStages; ++i) mbar_init(a_full + i, 4);
         mbar_init(acc_full, 2);
@@ -291,7 +310,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
         // ===================== TMA producer (whole warp runs the loop, one elected lane issues) =====================
         const uint64_t pol_w = l2_policy_evict_first(), pol_x = l2_policy_evict_last();
         const unsigned char* src = p.packed + (kAwq ? u_begin * kRecordStride : 0);
-        const int n_pre = n_units < kStages ? n_units : kStages;
+        const int n_pre = n_units < kWRing ? n_units : kWRing;
         // The weight copies of the whole ring are requested before griddepcontrol.wait (they never depend on the
         // stream predecessor), the x slabs after it.  (Requesting only a few records early, so that the first x
         // slab does not queue behind ~85 KB of weights, starts the first MMA 2 us sooner but measured no faster:
@@ -306,6 +325,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                 tma_tensor2d_g2s(s_w + stage * kWStride, &tmap_w, g * 64, tile * kTileN, full_w + stage, pol_w);
         };
         auto issue_x = [&](int stage, int gk) {
+            if (kSplit) return;                                   // requested by the x slabs' own warp
             mbar_arrive_expect_tx(full_x + stage, (uint32_t)kXBytes);
             unsigned char* xs = s_x + stage * kXBytes;
             if constexpr (kAwq) {
@@ -346,16 +366,36 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
         Ring r;
         r.phase = 1;                                             // every stage has been used once
         for (int i = n_pre; i < n_units; ++i) {
-            UMB_WAIT(done + r.stage, r.phase ^ 1);               // the unit that last used this stage has retired
+            // the unit that last used this stage has retired (kSplit: its record has been read)
+            if constexpr (kSplit) UMB_WAIT(w_empty + r.stage, r.phase ^ 1);
+            else UMB_WAIT(done + r.stage, r.phase ^ 1);
             if (elect_one()) {
                 issue_w(r.stage);
                 issue_x(r.stage, g);
             }
             __syncwarp();
             advance_w();
-            r.advance(kStages);
+            r.advance(kWRing);
         }
         if (lane == 0) UMB_TRACE(10);
+    } else if (kSplit && warp == GemmCfg<MPAD>::kThreadsAwq / 32 - 1) {
+        // ===================== x-slab producer (AWQ, kSplit) =====================
+        const uint64_t pol_x = l2_policy_evict_last();
+        pdl_wait();                                              // x is the predecessor's output
+        int gx = in_tile0, stage = 0, use = 0;
+        for (int i = 0; i < n_units; ++i) {
+            if (use > 0) UMB_WAIT(done + stage, (use - 1) & 1); // the unit that last used this stage has retired
+            if (elect_one()) {
+                mbar_arrive_expect_tx(full_x + stage, (uint32_t)kXBytes);
+                tma_tensor3d_g2s(s_x + stage * kXBytes, &tmap_w, 0, 0, gx * 2, full_x + stage, pol_x);
+            }
+            __syncwarp();
+            if (++gx == p.units_per_tile) gx = 0;
+            if (++stage == kStages) {
+                stage = 0;
+                ++use;
+            }
+        }
     } else if (warp <= 2) {
         // ===================== MMA issuers: warp 1 takes even CTA-local units, warp 2 odd ones =====================
         const int par = warp - 1;
@@ -512,7 +552,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
         if (!is_epi) {
             // ===================== dequant warps (AWQ): group g takes CTA-local units g, g + kDqGroups, ... =====================
             if constexpr (kAwq) {
-                int dq_st = grp % kStages, dq_ph = 0, dq_ts = grp % kAStages;      // ring positions of unit `mine`
+                int dq_st = grp % kWRing, dq_ph = 0, dq_ts = grp % kAStages;      // ring positions of unit `mine`
                 int w_first = grp;                                                 // first unit of this group that re-uses a TMEM stage
                 while (w_first < kAStages) w_first += kDq;
                 int w_st = (w_first - kAStages) % kStages, w_ph = 0;               // ring position of unit `mine - kAStages`
@@ -530,12 +570,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                     UMB_WAIT(full_w + dq_st, dq_ph);
                     if (grp == 0 && q == 0 && lane == 0) UMB_TRACE(4);
                     fetch(dq_st);
+                    if constexpr (kSplit) {
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(w_empty + dq_st);
+                    }
                 }
                 for (int mine = grp; mine < n_units; mine += kDq) {
                     const int ts = dq_ts;
                     dq_st += kDq;
-                    if (dq_st >= kStages) {
-                        dq_st -= kStages;
+                    if (dq_st >= kWRing) {
+                        dq_st -= kWRing;
                         dq_ph ^= 1;
                     }
                     dq_ts += kDq;
@@ -571,6 +615,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                         //     done[v - kAStages] implies done[v - kStages]: both ring depths are even, so the two units were
                         //     issued and committed, in order, by the same MMA thread; a retired occupant has landed, so
                         //     full_w is at most one use behind.  (v < kAStages: first use of both stages, nothing to wait for.)
+                        //     kSplit: the producer no longer orders the records behind done, so (1) itself has to know that
+                        //     done[v - 2 kAStages] is over, and (2) that record v - kWStages was read: this group has waited
+                        //     for both itself, both depths being multiples of the number of groups.
                         if (mine + kDq >= kAStages) {
                             UMB_WAIT(done + w_st, w_ph);
                             tc_fence_after();
@@ -582,12 +629,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                         }
                         UMB_WAIT(full_w + dq_st, dq_ph);
                         fetch(dq_st);
+                        if constexpr (kSplit) {
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(w_empty + dq_st);
+                        }
                     }
                 }
                 if constexpr (kShare) {
                     // The head of a split tile is reduced by all groups of warps, one chunk of 16 columns each in turn: a chunk
                     // waits for two or three round trips to the other CTAs' sums, 24 of them in series with one group
-                    // when five CTAs share a tile.
+                    // when five CTAs share a tile (849 -> 683 us, see kSplit; four sums in flight a thread instead of two
+                    // spill registers: 753).
                     const int tile_ = (int)((u_end - 1) / p.units_per_tile);
                     const long long tile_u0 = (long long)tile_ * p.units_per_tile;
                     const int c_first = sk_owner(tile_u0, U, P), c_last = sk_owner(tile_u0 + p.units_per_tile - 1, U, P);
@@ -912,7 +964,7 @@ static int launch_gemm(const CUtensorMap& tx, const CUtensorMap& tw, GemmParams 
             const char* e = getenv("UMB_GEMM_STAGES");
             env_stages = e ? atoi(e) : 0;
         }
-        if (env_stages > 0 && env_stages <= 16 && (env_stages % 2) == 0 && GemmCfg<MPAD>::smem_bytes(kAwq, env_stages) <= 227 * 1024)
+        if (env_stages > 0 && env_stages <= 16 && (env_stages % 2) == 0 && !(kAwq && GemmCfg<MPAD>::kSplit) && GemmCfg<MPAD>::smem_bytes(kAwq, env_stages) <= 227 * 1024)
             p.stages = env_stages;                                   // even: see the static_assert on the ring depths
     }
     p.trace = trace_for_this_launch();
@@ -964,9 +1016,9 @@ static int gemm_common(bool awq, const void* x, int64_t ldx, const void* w, int6
                 (p.mode != UMB_EPI_RESIDUAL || ((((uintptr_t)p.residual) & 15) == 0 && (p.ld_residual % 8) == 0))) ? 1 : 0;
     if (p.mode == UMB_EPI_SILU_MUL) UMB_CHECK_ARG((N_total % kTileN) == 0 && p.bias == nullptr);
 
-    if (awq && M > 64) {
+    if (awq && M > 128) {
         const size_t need = awq_wide_ws_bytes(M, N_total);
-        if (!workspace || workspace_bytes < need || (M <= 128 && workspace_bytes < umb_gemm_workspace_bytes(M, K, N_total))) return UMB_ERR_WORKSPACE;
+        if (!workspace || workspace_bytes < need) return UMB_ERR_WORKSPACE;
         UMB_CHECK_ARG(((uintptr_t)workspace & 15) == 0);
         if ((long long)(p.tiles + 1) * p.units_per_tile * 2 >= (1ll << 31)) return UMB_ERR_UNSUPPORTED;
         p.slots = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(workspace) + (((size_t)p.tiles * 4 + 255) & ~(size_t)255));
@@ -1015,7 +1067,7 @@ static int gemm_common(bool awq, const void* x, int64_t ldx, const void* w, int6
         case 16: UMB_DISPATCH(16);
         case 32: UMB_DISPATCH(32);
         case 64: UMB_DISPATCH(64);
-        default: return launch_gemm<128, false>(tx, tw, p, grid, st);
+        default: UMB_DISPATCH(128);
     }
 #undef UMB_DISPATCH
 }
@@ -1097,7 +1149,7 @@ extern "C" int umb_awq_gemm_f16(const void* x, int64_t ldx, const void* packed, 
 
 extern "C" size_t umb_awq_gemm_rows_ws_bytes(int M, int K, int N_total) {
     if (M < 1 || M > 512 || N_total < 1) return 0;
-    const size_t few = umb_gemm_workspace_bytes(M, K, N_total), many = M > 64 ? awq_wide_ws_bytes(M, N_total) : 0;
+    const size_t few = umb_gemm_workspace_bytes(M, K, N_total), many = M > 128 ? awq_wide_ws_bytes(M, N_total) : 0;
     return few > many ? few : many;
 }
 

@@ -1,8 +1,8 @@
-// AWQ INT4 products of 65 to 512 token rows by pairs of SMs (tcgen05 cta_group::2), for prompts and wide trees.
+// AWQ INT4 products of 129 to 512 token rows by pairs of SMs (tcgen05 cta_group::2), for prompts and wide trees.
 //
 // Weights are the A operand as in gemm.cu, but of two tiles at once: each block of a pair dequantises the records of its own 128
 // output features into its own tensor memory, holds half of the token rows of a slab of 128 k in shared memory, and the tensor
-// cores of both multiply 256 features with up to 256 rows (M = 256, N = 128, 192 or 256).  A record is dequantised once for up to 256 rows and
+// cores of both multiply 256 features with up to 256 rows (M = 256, N = 192 or 256).  A record is dequantised once for up to 256 rows and
 // a slab's bytes cross into an SM once for 256 features.
 //
 // Warp roles of a block (480 threads, one block per SM):
@@ -40,7 +40,7 @@ constexpr int kWideSlots = 2;                               // parts of tiles th
 template <int NPAD> struct WideCfg {
     static constexpr int kRows = NPAD / 2;                  // rows of a slab that a block holds
     static constexpr int kXBytes = kRows * 256;             // [2 pieces of 64 k][rows][128 B]
-    static constexpr int kX = (512 - NPAD) / 128 * 2;       // x slabs, and parts of the A operand (64 columns each, behind the accumulator): 6, 4, 4
+    static constexpr int kX = (512 - NPAD) / 128 * 2;       // x slabs, and parts of the A operand (64 columns each, behind the accumulator)
     static constexpr int kSmem = 1024 + kX * kXBytes + kWideW * kWideRecord + 3 * kWideExch;
 };
 
@@ -486,7 +486,7 @@ WideRows wide_rows(int M) {
     const int shift = M > 256 ? 1 : 0;
     return {shift, (((M + shift) >> shift) + 15) / 16 * 16};
 }
-int wide_columns(int rows) { return rows <= 128 ? 128 : (rows <= 192 ? 192 : 256); }
+int wide_columns(int rows) { return rows <= 192 ? 192 : 256; }
 
 }  // namespace
 
@@ -497,11 +497,7 @@ size_t awq_wide_ws_bytes(int M, int N_total) {
 
 int launch_awq_wide(const void* x, int64_t ldx, const GemmParams& p, cudaStream_t st) {
     const WideRows rb = wide_rows(p.M);
-    switch (wide_columns(rb.rows)) {
-        case 128: return launch_wide<128>(x, ldx, p, rb, st);
-        case 192: return launch_wide<192>(x, ldx, p, rb, st);
-        default: return launch_wide<256>(x, ldx, p, rb, st);
-    }
+    return wide_columns(rb.rows) == 192 ? launch_wide<192>(x, ldx, p, rb, st) : launch_wide<256>(x, ldx, p, rb, st);
 }
 
 }  // namespace umb

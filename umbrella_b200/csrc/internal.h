@@ -35,7 +35,7 @@ inline cudaError_t launch_pdl(const char* name, void (*kernel)(KArgs...), dim3 g
 #define UMB_LAUNCH_PDL(kernel, ...) do { cudaError_t e__ = umb::launch_pdl(#kernel, kernel, __VA_ARGS__); if (e__ != cudaSuccess) return (int)e__; } while (0)
 // every host entry point reports the kernels it enqueued (umb_launch_count)
 void count_launches(unsigned n);
-// gemm_wide.cu: AWQ products of 65 to 512 token rows by pairs of SMs, with a workspace of awq_wide_ws_bytes() bytes
+// gemm_wide.cu: AWQ products of 129 to 512 token rows by pairs of SMs, with a workspace of awq_wide_ws_bytes() bytes
 struct GemmParams;
 size_t awq_wide_ws_bytes(int M, int N_total);
 int launch_awq_wide(const void* x, int64_t ldx, const GemmParams& p, cudaStream_t st);
