@@ -93,19 +93,15 @@ def test_the_kernels_barriers_pass_the_gate():
     assert len(uses) == 2 and uses[0].startswith("__device__") and "gate.pass" in uses[1]
 
 
-def test_what_is_handed_to_the_other_block_is_released_and_acquired_there():
-    """An arrival without a scope orders what its own block sees; the barriers of a pair are arrived at from the other block.  So every remote arrival releases in
-    cluster scope, and every barrier that has one is waited for with a look that acquires in it."""
-    seen = 0
-    for name in ("gemm_wide.cu", os.path.join("seq", "seq_gemm_pair.cu")):
+def test_what_is_handed_to_the_other_block_names_its_scope():
+    """An arrival without a scope orders what its own block sees; the barriers of a pair are arrived at from the other block, by its threads or by the end of
+    products of both.  So every remote arrival names the cluster, and so does every wait for a barrier that has one."""
+    shared = {"gemm_wide.cu": {"full_a", "acc_empty", "done", "acc_full", "last_full"}, os.path.join("seq", "seq_gemm_pair.cu"): {"acc_empty", "empty"}}
+    for name, bars in shared.items():
         text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
-        remote = re.findall(r"mbarrier\.arrive[^ ]*shared::cluster[^ ]*", text)
-        remote = [r for r in remote if "tcgen05" not in r and "::one" not in r]
-        assert remote and all(".release.cluster." in r for r in remote), (name, remote)
-        bars = set(re.findall(r"arrive_at\((?:first_block\()?(\w+)", text)) - {"uint32_t"}
+        remote = [a for a in re.findall(r'"mbarrier\.arrive[^ ]*', text) if "shared::cluster" in a]
+        assert remote and all(re.search(r"\.(release|relaxed)\.cluster\.", a) for a in remote), (name, remote)
         for bar in bars:
-            waits = re.findall(r"(\w+)\(%s\b[^;]*quit\)" % bar, text)
-            assert waits and set(waits) == {"spin_pair"}, (name, bar, waits)
-            seen += 1
-        assert "mbarrier.test_wait.parity.acquire.cluster" in text
-    assert seen >= 3
+            waits = re.findall(r"(\w+)\(%s\b[^;{]*?, quit\)" % bar, text)
+            assert waits and set(waits) <= {"spin_pair", "wait_pair"}, (name, bar, waits)
+        assert re.search(r"test_wait\.parity\.(acquire|relaxed)\.cluster|UMB_TEST_WAIT\(\"\.relaxed\.cluster\"\)", text), name

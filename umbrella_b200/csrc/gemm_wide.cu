@@ -20,8 +20,8 @@
 //
 // Bound: a unit takes 610 to 650 ns, its products 540 at the measured cuBLAS rate; the next tile's products wait for the columns of the one
 // before (5 us where it is published, 10 where it is finished: the accumulator fills half of tensor memory, so there is one), and the end of
-// a range is 12 us of 100.  us, four passes of 125 rows through gemm.cu's kernel / one of 500 here: a layer of width 4096 and its head 682 / 472, of width 8192
-// 1349 / 1110; 1000 rows 1230 / 802, 300 524 / 374, 128 289 / 278, 65 272 / 262 (one pass on both sides).  Of no effect: fewer records, fewer or no x
+// a range is 12 us of 100.  us, four passes of 125 rows through gemm.cu's kernel / one of 500 here: a layer of width 4096 and its head 695 / 458, of width 8192
+// 1363 / 1088; 1000 rows 1244 / 759, 300 540 / 380, 129 376 / 306.  Up to 128 rows, one pass on both sides, this gains nothing (gemm.cu does them).  Of no effect: fewer records, fewer or no x
 // copies, no arithmetic in the dequantisation (2 to 8 % each), deeper record rings.
 #include <atomic>
 #include <mutex>
@@ -58,7 +58,7 @@ __device__ __forceinline__ uint32_t first_block(const void* p) {            // t
     return r;
 }
 __device__ __forceinline__ void arrive_at(uint32_t bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tma_3d_pair(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
@@ -81,50 +81,46 @@ __device__ __forceinline__ bool give_up(volatile int* quit) {
     }
     return false;
 }
+// PAIR: a barrier that the other block's threads, or products of both, arrive at.  What such a barrier hands over is in tensor memory, or the products' reads of
+// shared memory are over: the fences of tcgen05 on both sides order that, and the barrier itself is relaxed, but in cluster scope.  (Arrivals that release
+// in cluster scope: a prompt of 500 rows 470 -> 500 us; every look acquiring in it: 1.5 times the whole.)
+#define UMB_TEST_WAIT(PAIR) "mbarrier.test_wait.parity" PAIR ".shared::cta.b64 p, [%1], %2;\n\t"
+template <bool PAIR>
 __device__ __forceinline__ bool test_bar(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    if constexpr (PAIR)
+        asm volatile("{\n\t.reg .pred p;\n\t" UMB_TEST_WAIT(".relaxed.cluster") "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\t" UMB_TEST_WAIT("") "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatile int* quit) {
+template <bool PAIR>
+__device__ __forceinline__ bool poll_bar(uint64_t* bar, uint32_t parity, volatile int* quit) {
     bool ok = false;
     for (int i = 0; i < (1 << 24); ++i) {
-        if ((ok = test_bar(bar, parity))) break;
+        if ((ok = test_bar<PAIR>(bar, parity))) break;
         __nanosleep(20);
         if ((i & 255) == 255 && *quit) break;
     }
     return __all_sync(0xffffffffu, ok) || give_up(quit);
 }
+__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatile int* quit) { return poll_bar<false>(bar, parity, quit); }
+__device__ __forceinline__ bool wait_pair(uint64_t* bar, uint32_t parity, volatile int* quit) { return poll_bar<true>(bar, parity, quit); }
 // without a pause, for the warp that issues the products (one statement: as C++ the loop's exits cost 100 clocks a wait)
-__device__ __forceinline__ bool spin_bar(uint64_t* bar, uint32_t parity, volatile int* quit) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, 0;\n\t"
-        "AGAIN_%=:\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "@p bra DONE_%=;\n\t"
-        "add.u32 n, n, 1;\n\tsetp.lt.u32 q, n, 67108864;\n\t@q bra AGAIN_%=;\n\t"
-        "DONE_%=:\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+#define UMB_SPIN(PAIR)                                                                                         \
+    uint32_t ok;                                                                                               \
+    asm volatile(                                                                                              \
+        "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, 0;\n\t"                                           \
+        "AGAIN_%=:\n\t" UMB_TEST_WAIT(PAIR)                                                                    \
+        "@p bra DONE_%=;\n\t"                                                                                  \
+        "add.u32 n, n, 1;\n\tsetp.lt.u32 q, n, 67108864;\n\t@q bra AGAIN_%=;\n\t"                              \
+        "DONE_%=:\n\tselp.u32 %0, 1, 0, p;\n\t}"                                                               \
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");                                              \
     return __all_sync(0xffffffffu, ok) || give_up(quit);
-}
-// The same for a barrier that the other block's threads arrive at (arrive_at): what they did in front of that is done for this thread too.  One more look, in
-// cluster scope, once the barrier is known to be done, costs nothing that could be measured (a prompt of 500 rows 495.9 / 495.7 us with and without it; every look in
-// cluster scope: 1.5 times the whole).
-__device__ __forceinline__ bool spin_pair(uint64_t* bar, uint32_t parity, volatile int* quit) {
-    if (!spin_bar(bar, parity, quit)) return false;
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return __all_sync(0xffffffffu, ok) || give_up(quit);
-}
+__device__ __forceinline__ bool spin_bar(uint64_t* bar, uint32_t parity, volatile int* quit) { UMB_SPIN("") }
+__device__ __forceinline__ bool spin_pair(uint64_t* bar, uint32_t parity, volatile int* quit) { UMB_SPIN(".relaxed.cluster") }
+#undef UMB_SPIN
+#undef UMB_TEST_WAIT
 // The four warps of a group go on together or not at all (GroupGate): what follows holds barriers of theirs.
 __device__ __forceinline__ bool group_all(bool ok, int bar) {
     int all = ok;
@@ -222,7 +218,7 @@ awq_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         int g = g_first, row = (t_first & ((1 << rb.shift) - 1)) * rb.rows;
         for (int i = 0; i < n_units; ++i) {
             const int s = i % kX;
-            if (i >= kX && !wait_bar(done + s, ((i / kX) - 1) & 1, quit)) break;
+            if (i >= kX && !wait_pair(done + s, ((i / kX) - 1) & 1, quit)) break;
             const uint32_t bar = first_block(full_x + s);
             if (elect_one()) {
                 if (rank == 0) mbar_arrive_expect_tx(full_x + s, 2 * Cfg::kXBytes);
@@ -292,7 +288,7 @@ awq_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         // A tile that is not the range's last, by all three groups: finished when it is whole, else published (it is the first, and its
         // other parts are not this pair's to add).
         auto leave_tile = [&](int t) -> bool {
-            if (!together(wait_bar(acc_full, (t - t_first) & 1, quit))) return false;
+            if (!together(wait_pair(acc_full, (t - t_first) & 1, quit))) return false;
             tc_fence_after();
             const int rows = rows_of(t);
             const bool whole = t > t_first || g_first == 0;
@@ -339,7 +335,7 @@ awq_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 const uint32_t sbits = lds16(rec + kRecScaleOff + fl * 2), z = (lds32(rec + kRecZeroOff + (fl >> 3) * 4) >> (4 * (fl & 7))) & 0xFu;
                 __syncwarp();
                 if (lane == 0) mbar_arrive(empty_w + ws);
-                if (i >= kX && !(ok = wait_bar(done + as, ((i / kX) - 1) & 1, quit))) break;
+                if (i >= kX && !(ok = wait_pair(done + as, ((i / kX) - 1) & 1, quit))) break;
                 tc_fence_after();
                 const __half2 ce = as_h2((0x6400u | z) * 0x10001u), neg_co = as_h2((0xD400u | (z << 4)) * 0x10001u), s2 = as_h2(sbits * 0x10001u);
                 const uint32_t to = quarter + kACol + as * 64;
@@ -360,7 +356,7 @@ awq_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         pdl_wait();                                         // residual, workspace and y belong to the kernels in front
         for (; ok && t < t_last; ++t) ok = leave_tile(t);
         // ------------------------------------------------------------------------------------ the range's last tile
-        ok = together(ok && n_units > 0 && wait_bar(last_full, 0, quit));
+        ok = together(ok && n_units > 0 && wait_pair(last_full, 0, quit));
         if (ok) {
             tc_fence_after();
             const int rows = rows_of(t);                    // (t is t_last)
