@@ -19,13 +19,13 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libumbrella_b200.so")
 SOURCES = ["api.cu", "tree.cu", "glue.cu", "attn.cu", "gemm.cu", "gemm_wide.cu", "forward.cu", "sampler.cu"]
-HEADERS = ["common.cuh", "gemm_core.cuh", "group_gate.h", "internal.h", os.path.join("..", "..", "include", "umbrella_b200.h")]
+HEADERS = ["common.cuh", "gemm_core.cuh", "group_gate.h", "attn_rules.h", "internal.h", os.path.join("..", "..", "include", "umbrella_b200.h")]
 SEQ_LIB = os.path.join(HERE, "libumbrella_b200_seq.so")
 SEQ_SOURCES = [os.path.join("seq", f) for f in ("seq_kernels.cu", "seq_window_attn.cu", "seq_gemm.cu", "seq_gemm_tc.cu", "seq_gemm_split.cu", "seq_gemm_pair.cu", "seq_forward.cu",
                                                       "seq_prenorm.cu", "seq_cached_attn.cu", "seq_attn_tc.cu", "seq_mlstm.cu", "seq_chunk.cu", "seq_chunk_tc.cu", "seq_timemix.cu",
                                                       "seq_memory.cu")]
 SEQ_HEADERS = [os.path.join("seq", "seq_internal.h"), os.path.join("seq", "seq_gemm.h"), os.path.join("seq", "seq_gemm_walk.cuh"), os.path.join("seq", "seq_attn.h"), os.path.join("seq", "seq_tc.cuh"),
-               os.path.join("seq", "seq_chunk.h"), "common.cuh", os.path.join("..", "..", "include", "umbrella_b200.h"),
+               os.path.join("seq", "seq_chunk.h"), "common.cuh", "attn_rules.h", os.path.join("..", "..", "include", "umbrella_b200.h"),
                os.path.join("..", "..", "include", "umbrella_b200_seq.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "--use_fast_math=false", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=default"]

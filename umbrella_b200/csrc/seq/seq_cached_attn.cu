@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <stdint.h>
 
+#include "../attn_rules.h"
 #include "seq_attn.h"
 
 namespace umbs {
@@ -705,11 +706,10 @@ static bool capturing(cudaStream_t st) {
     cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(st, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone;
 }
-// Unsplit steps of a block per SM and more take blocks of six warps: what bounds one is the chain of a warp's rounds (issue slots 33 %, with six warps 40 %), and with two
-// blocks of four warps on an SM 1040 keys are nine of them, with six warps six.  us, four warps / six, 16 heads over 4 of 128: 64 sequences x 1024 keys
-// 42.9 / 37.1, x 128 14.4 / 10.7, 128 x 2048 156 / 119; 12 over 2 of 96, 128 x 700 29.0 / 24.4; 16 over 4 of 64, 256 x 300 38.1 / 38.0.  Fewer blocks: 32 x 256
-// 10.6 and a merge / 13.5, 8 x 1024 10.5 / 11.4, 1 x 4096 10.0 / 11.2.
-constexpr int kCgManyBlocks = 148;
+// Unsplit steps of a block per SM and more may take blocks of six warps (six_warps_pay: waves against rounds): what bounds a block is the chain of a warp's rounds (issue
+// slots 33 %, with six warps 40 %), and with two blocks of four warps on an SM 1040 keys are nine of them, with six warps six.  us, four warps / six, fewer blocks, 16
+// heads over 4 of 128: 32 x 256 10.6 and a merge / 13.5, 8 x 1024 10.5 / 11.4, 1 x 4096 10.0 / 11.2.
+constexpr int kCgSms = 148;
 static int group_blocks(const CachedAttnArgs& a) {
     return a.kv_heads * ((a.heads / a.kv_heads + kCgHeads - 1) / kCgHeads);
 }
@@ -872,10 +872,13 @@ extern "C" int umbs_cached_attention_ex(int dtype, int mode, const void* q, cons
             const int64_t blocks = (int64_t)batch->n_seqs * group_blocks(a);
             int64_t best = INT64_MAX;
             for (int n = 1; n <= room && (n == 1 || (n - 1) * 128 < keys); ++n) {
-                const int64_t cost = (blocks * n + 443) / 444 * ((keys + n * 128 - 1) / (n * 128) + 1) + (n > 1);
+                const int64_t cost = (blocks * n + 3 * kCgSms - 1) / (3 * kCgSms) * ((keys + n * 128 - 1) / (n * 128) + 1) + (n > 1);
                 if (cost < best) { best = cost; n_split = n; }
             }
-            group_many = n_split == 1 && blocks >= kCgManyBlocks;
+            // (a captured step is replayed for longer contexts: by the most that its ring and its window hold)
+            const int most = std::max(keys, std::min(kv_len, window > 0 ? window : kv_len));
+            group_many = n_split == 1 && umb::six_warps_pay(blocks, keys, kCgSms);
+            if (n_split == 1 && group_many != umb::six_warps_pay(blocks, most, kCgSms) && capturing(st)) group_many = !group_many;
         } else {
             n_split = (keys + 255) / 256;
             n_split = n_split < 1 ? 1 : (n_split > 32 ? 32 : n_split);
