@@ -33,3 +33,20 @@ def test_warps_of_a_decode_block(ask):
     """Never more than 3 % behind the better one where six warps are taken, nor 7 % where four are."""
     for (at, (four, six)), took_six in zip(DECODE.items(), ask("six_warps_pay", DECODE)):
         assert (six <= 1.03 * four) if took_six else (four <= 1.07 * six), (at, four, six)
+
+
+# (mask mode, rows, keys, heads, key/value heads, head size): us in slabs of 16 rows, in tiles of 64
+ROWS = {(2, 256, 256, 32, 8, 128): (18.4, 15.3), (2, 256, 7256, 32, 8, 128): (204.8, 172.6), (2, 128, 628, 64, 8, 128): (34.8, 29.1), (2, 300, 300, 32, 8, 128): (27.9, 17.2),
+        (2, 300, 1800, 32, 8, 128): (76.2, 82.9), (2, 300, 7300, 32, 8, 128): (253.0, 320.0), (2, 296, 7296, 32, 8, 128): (211.0, 320.0), (2, 512, 512, 32, 8, 128): (49.0, 28.0),
+        (2, 512, 7512, 32, 8, 128): (367.0, 331.0), (2, 520, 7520, 32, 8, 128): (410.0, 332.0), (2, 600, 600, 32, 8, 128): (60.0, 33.0), (2, 600, 3100, 32, 8, 128): (200.0, 208.0),
+        (2, 600, 7600, 32, 8, 128): (459.0, 546.0), (2, 512, 512, 64, 8, 128): (91.0, 43.0), (2, 192, 7192, 64, 8, 128): (302.0, 317.0), (2, 1000, 8000, 32, 32, 128): (799.0, 688.0),
+        (0, 512, 1012, 64, 8, 128): (162.0, 124.0), (0, 256, 1256, 64, 8, 128): (92.0, 66.0), (0, 300, 7300, 32, 8, 128): (261.0, 331.0), (0, 800, 1300, 32, 8, 128): (163.0, 170.0),
+        (0, 800, 1300, 24, 8, 128): (130.0, 169.0), (0, 400, 900, 32, 8, 128): (68.0, 57.0), (1, 300, 2300, 32, 8, 128): (235.0, 387.0), (1, 300, 800, 64, 8, 128): (199.0, 248.0),
+        (2, 256, 256, 32, 8, 64): (9.1, 10.9), (2, 300, 300, 32, 8, 64): (17.0, 12.0), (2, 512, 512, 32, 8, 64): (30.0, 22.0), (2, 512, 1512, 32, 8, 64): (57.0, 61.0),
+        (2, 384, 7384, 32, 8, 64): (175.0, 265.0), (0, 384, 4384, 32, 8, 64): (117.0, 169.0), (2, 768, 7768, 16, 16, 64): (180.0, 278.0), (2, 600, 600, 16, 16, 64): (21.0, 23.0)}
+
+
+def test_rows_of_an_attention_block(ask):
+    """Never more than 2 % behind the better one where tiles are taken, nor 10 % where slabs are."""
+    for (at, (slabs, tiles)), took in zip(ROWS.items(), ask("row_tiles_pay", ROWS)):
+        assert (tiles <= 1.02 * slabs) if took else (slabs <= 1.1 * tiles), (at, slabs, tiles)

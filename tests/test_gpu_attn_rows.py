@@ -1,8 +1,9 @@
-"""Attention of many query rows (64-row tiles, weights in two fp16 parts) against float64, on both sides of the line to the slabs of 16 rows (128 tiles
-over all key/value heads) and at the edges of its tiles.
+"""Attention of many query rows against float64: tiles of 64 rows with weights in two fp16 parts (csrc/attn_rules.h says when) and slabs of 16 rows beside them, at the edges
+of both.
 
-Tolerance: results are fp16, 2^-11 of their size at most and 2^-11 / sqrt(3) = 2.8e-4 in the norm; the two parts leave 2^-22 of a weight, one part (the
-slabs) 2^-12 / sqrt(3) = 1.4e-4: together 3.2e-4."""
+Tolerance: a result is rounded to fp16, which leaves 2^-11 / sqrt(3) of its binade and 2.03e-4 in the norm of results of all sizes; two parts leave 2^-22 of a weight,
+nothing to that, one part (the slabs) 2^-12 / sqrt(3) = 1.4e-4 of each: in all 2.46e-4 where a row's weights are of all sizes.  So tiles stay below 2.25e-4,
+which one part would pass, slabs below 3.2e-4."""
 import pytest
 import torch
 
@@ -11,9 +12,11 @@ DEV = "cuda:0"
 
 
 @pytest.mark.parametrize("mode", ["causal", "tree", "dense"])
-@pytest.mark.parametrize("qo,prefix,heads,kv_heads,dim,cap", [(256, 0, 32, 8, 128, 0.0), (240, 70, 32, 8, 128, 0.0), (241, 70, 32, 8, 128, 0.0), (505, 3, 16, 16, 64, 0.0),
-                                                             (130, 500, 64, 8, 64, 30.0), (333, 1, 24, 8, 128, 20.0)])
-def test_many_rows(mode, qo, prefix, heads, kv_heads, dim, cap):
+@pytest.mark.parametrize("qo,prefix,heads,kv_heads,dim,cap,tiled", [(256, 0, 32, 8, 128, 0.0, "causal"), (240, 70, 32, 8, 128, 0.0, ""), (241, 70, 32, 8, 128, 0.0, "causal"),
+                                                                   (505, 3, 16, 16, 64, 0.0, ""), (130, 500, 64, 8, 64, 30.0, ""), (333, 1, 24, 8, 128, 20.0, "causal"),
+                                                                   (300, 500, 64, 8, 128, 0.0, "causal tree"), (257, 300, 64, 8, 128, 20.0, "causal tree"),
+                                                                   (300, 0, 32, 8, 64, 0.0, "causal"), (200, 80, 64, 8, 64, 30.0, "causal")])
+def test_many_rows(mode, qo, prefix, heads, kv_heads, dim, cap, tiled):
     from umbrella_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(5)
     kv, G = prefix + qo, heads // kv_heads
@@ -40,4 +43,4 @@ def test_many_rows(mode, qo, prefix, heads, kv_heads, dim, cap):
     if cap:
         z = cap * torch.tanh(z / cap)
     want = torch.einsum("hqk,khd->qhd", torch.softmax(z.masked_fill(~see, -torch.inf), -1), v[:kv].double().repeat_interleave(G, 1))
-    assert float((out.double() - want).norm() / want.norm()) < 3.2e-4
+    assert float((out.double() - want).norm() / want.norm()) < (2.25e-4 if mode in tiled else 3.2e-4)

@@ -16,6 +16,7 @@
 #include <stdio.h>
 #include <stdlib.h>
 
+#include "attn_rules.h"
 #include "common.cuh"
 #include "internal.h"
 
@@ -128,8 +129,9 @@ __device__ __forceinline__ unsigned long long row_window(const AttnParams& p, in
 }
 
 // kTwoParts: a weight goes into the second product as two fp16 numbers (what is left of it behind the first one's rounding is the second).  The
-// slab kernel below rounds each warp's largest weight to itself (it is 1), this kernel one weight of the row: 500 rows 2.46e-4 from float64 with
-// one part against the slabs' 2.39e-4, with two the rounding of the result alone.
+// slab kernel below rounds each warp's largest weight to itself (it is 1), this kernel one weight of the row: 500 causal rows, 32 heads over 8 of 128, 2.46e-4 from
+// float64 with one part against the slabs' 2.39e-4, with two 2.0e-4, the rounding of the result alone.  Where this kernel is taken for its keys (more than 8192) it
+// keeps the one part that it always had there.
 template <int D, bool kSoftCap, bool kTwoParts>
 __global__ void __launch_bounds__(kAttnThreads) tree_attn_kernel(const AttnParams p) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -358,11 +360,6 @@ __global__ void __launch_bounds__(kAttnThreads) tree_attn_kernel(const AttnParam
 // in the loop), and merge their (m, l, o) partials through shared memory at the end.
 // ------------------------------------------------------------------------------------------------
 constexpr int kSBN = 32;
-// From so many tiles of 64 rows on (over all key/value heads) rows share a tile's keys: slabs of 16 rows, one to an SM, are then several rounds that each fetch
-// all of them again.  us, slabs / tiles with weights in two parts, heads of 128, 32 over 8: 500 rows 47.6 / 27.9, behind 1000 cached 96.5 / 73.0, 256 rows 18.1 / 15.4
-// (128 tiles), 128 rows 8.3 / 8.7, behind 1000 27.2 / 25.5; 64 over 8: 500 rows 89.4 / 44.2, a tree of 385 behind 500 120 / 92, of 64 18.5 / 20.0; heads of 64, 200 rows behind
-// 3000 44 / 54 (104 tiles).  Distance to float64 2.6e-4 / 2.1e-4.
-constexpr int kManyRowTiles = 128;
 constexpr int kSlabTilesPerCta = 32;     // minimum kv tiles per slab CTA before the KV range is split across CTAs
 
 template <int D>
@@ -1237,11 +1234,11 @@ extern "C" int umb_tree_attn_f16(const void* q, const void* k_cache, const void*
 
 #endif
     // kernel + split selection.  slab kernel: K/V is re-read once per 16-row slab (L2), so it is used
-    // while that re-read is cheap; long contexts with many slabs, and many rows, go to the 64-row tile kernel.
+    // while that re-read is cheap; long contexts with many slabs, and many rows where they pay, go to the 64-row tile kernel.
     const int rows_total = qo * p.G;
     const int slabs = (rows_total + 15) / 16;
     const bool near = !(kv_bound > 8192 && slabs > 2);
-    const bool many_rows = near && (rows_total + kBM - 1) / kBM * p.Hkv >= kManyRowTiles, slab = near && !many_rows;
+    const bool many_rows = near && row_tiles_pay(mask->mask_mode, qo, kv_bound, num_q_heads, num_kv_heads, head_dim, sm_count()), slab = near && !many_rows;
     const int ctas_base = (slab ? slabs : (rows_total + kBM - 1) / kBM) * p.Hkv;
     const int kv_tiles = (kv_bound + (slab ? kSBN : kBN) - 1) / (slab ? kSBN : kBN);
     static int slab_tiles = 0;                                // UMB_ATTN_SLAB_TILES: tuning override (read once)
