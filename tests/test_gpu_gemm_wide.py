@@ -116,3 +116,21 @@ def test_silu_rounds_its_quotient(M):
     g = gate.float()
     want = (g / (1 + torch.exp(-g))).to(torch.float16) * up
     assert torch.equal(_run(x, packed, K, N, ws, mode=ops.UMB_EPI_SILU_MUL), want.reshape(M, N // 2))
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])
+@pytest.mark.parametrize("M", [129, 300, 512])
+def test_the_longest_sums_go_in_passes(M, mode):
+    """More than 16384 k: the bits of equal passes of up to 128 rows, whose sums are shorter, with every epilogue's rows where they belong."""
+    from umbrella_b200 import ops
+    K, N = 16512, 384
+    packed, x, ws = _setup(M, K, N)
+    res = torch.randn(M, N, device=DEV).to(torch.float16)
+    passes = -(-M // 128)
+    rows = -(-M // passes)
+    keys, want_keys = torch.zeros(M, dtype=torch.int64, device=DEV), torch.zeros(M, dtype=torch.int64, device=DEV)
+    logits = mode == ops.UMB_EPI_LOGITS
+    want = torch.cat([ops.awq_gemm(x[i:i + rows], packed, K, N, mode=mode, residual=res[i:i + rows] if mode == ops.UMB_EPI_RESIDUAL else None,
+                                   argmax=want_keys[i:i + rows] if logits else None) for i in range(0, M, rows)])
+    got = _run(x, packed, K, N, ws, mode=mode, residual=res if mode == ops.UMB_EPI_RESIDUAL else None, argmax=keys if logits else None)
+    assert torch.equal(got, want) and torch.equal(keys, want_keys)

@@ -1072,9 +1072,27 @@ static int gemm_common(bool awq, const void* x, int64_t ldx, const void* w, int6
 #undef UMB_DISPATCH
 }
 
+// The pair kernel sums a tile's k in one accumulator, the kernel of up to 128 rows in two, and has twice the k of a tile to a block; the tensor core cuts a sum
+// off at every step.  Distance to float64 of fp16 results, 300 to 512 rows, passes of up to 128 rows / pairs: K = 4096 2.0732e-4 / 2.0735e-4 (28672 features), 8192 + 0.04 to
+// 0.05 %, 14336 + 0.045 %, 28672 2.072e-4 / 2.083e-4, for 10 % of the time (28672 -> 8192, 500 rows, us: 218 / 193; 300 rows 149 / 170).  So the longest go in passes.
+constexpr int kWideK = 16384;
 int awq_gemm_rows(const void* x, int64_t ldx, const void* packed, void* y, int64_t ldy, int M, int K, int N_total, const umb_epilogue_t* epi,
                   void* workspace, size_t workspace_bytes, cudaStream_t st) {
-    return gemm_common(true, x, ldx, packed, 0, y, ldy, M, K, N_total, epi, workspace, workspace_bytes, st);
+    const int mode = epi ? epi->mode : UMB_EPI_STORE;
+    if (M <= 128 || M > 512 || K <= kWideK || mode == UMB_EPI_ROPE_QKV)
+        return gemm_common(true, x, ldx, packed, 0, y, ldy, M, K, N_total, epi, workspace, workspace_bytes, st);
+    const int passes = (M + 127) / 128, rows = (M + passes - 1) / passes;
+    for (int r0 = 0; r0 < M; r0 += rows) {
+        umb_epilogue_t e{};
+        if (epi) e = *epi;
+        if (e.residual) e.residual = (const __half*)e.residual + (int64_t)r0 * e.ld_residual;
+        if (e.argmax) e.argmax += r0;
+        const size_t size = mode == UMB_EPI_LOGITS ? sizeof(float) : sizeof(__half);
+        const int rc = gemm_common(true, (const __half*)x + (int64_t)r0 * ldx, ldx, packed, 0, (unsigned char*)y + (int64_t)r0 * ldy * size, ldy, M - r0 < rows ? M - r0 : rows, K,
+                                   N_total, epi ? &e : nullptr, workspace, workspace_bytes, st);
+        if (rc != UMB_OK) return rc;
+    }
+    return UMB_OK;
 }
 
 }  // namespace umb
