@@ -48,6 +48,13 @@ unsigned long long umb_launch_count(void);
 /* A replayed CUDA graph re-issues the launches recorded at capture: the host adds them here. */
 void umb_launch_count_add(unsigned long long n);
 
+/* Whether a block has given up on a bounded wait so far (1 or 0; only if something is broken).  Does not synchronise: behind a
+ * synchronisation it covers all work in front of it, replayed graphs too.  From then on every product is refused with
+ * UMB_ERR_TIMEOUT: caches, results and workspaces written since are not to be used, and the process is to be started again. */
+unsigned int umb_give_ups_seen(void);
+/* The word that such a block sets, in host memory (allocated on the first call); NULL where there is no device. */
+unsigned int* umb_give_up_word(void);
+
 /* ------------------------------------------------------------------------------------------------
  * (i) AWQ INT4 GEMM  --  y[M,N] = x[M,K] . W,  W[k, n] = (q[k,n] - z[k/g,n]) * s[k/g,n]
  *

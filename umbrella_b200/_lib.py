@@ -58,6 +58,8 @@ SIGNATURES = {
     "umb_error_string": (C.c_char_p, [c_int]),
     "umb_launch_count": (C.c_ulonglong, []),
     "umb_launch_count_add": (None, [C.c_ulonglong]),
+    "umb_give_ups_seen": (C.c_uint, []),
+    "umb_give_up_word": (C.POINTER(C.c_uint), []),
     "umb_awq_packed_bytes": (c_size_t, [c_int, c_int, c_int]),
     "umb_awq_repack": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_int, c_int,
                                c_int, c_void_p]),
@@ -134,6 +136,13 @@ def check(rc: int, what: str = "") -> None:
     if rc != 0:
         msg = load().umb_error_string(rc).decode()
         raise RuntimeError(f"umbrella_b200 {what} failed: status {rc} ({msg})")
+
+
+def raise_if_given_up() -> None:
+    """Raise if a kernel has reported that it gave up on a bounded wait.  Does not synchronise: called behind a copy to the host
+    it covers everything the copy waited for, replayed graphs too."""
+    if load().umb_give_ups_seen():
+        check(-5, "kernel")
 
 
 def launch_count() -> int:

@@ -1,5 +1,6 @@
 // Library bookkeeping: version, error strings, launch counter, device properties.
 #include <atomic>
+#include <mutex>
 #include <stdio.h>
 #include <stdlib.h>
 
@@ -42,6 +43,30 @@ int arg_fail(const char* file, int line, const char* what) {
     if (dbg) fprintf(stderr, "umbrella_b200: argument check failed at %s:%d: %s\n", file, line, what);
     return UMB_ERR_ARG;
 }
+static std::atomic<unsigned int*> g_give_up{nullptr};
+int give_up_word(unsigned int** word) {
+    static std::mutex making;
+    unsigned int* w = g_give_up.load(std::memory_order_acquire);
+    if (w == nullptr) {
+        std::lock_guard<std::mutex> lock(making);
+        w = g_give_up.load(std::memory_order_acquire);
+        if (w == nullptr) {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // (the first call may be inside a capture)
+            UMB_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+            const cudaError_t e = cudaHostAlloc((void**)&w, sizeof *w, cudaHostAllocPortable | cudaHostAllocMapped);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            if (e != cudaSuccess) return (int)e;
+            *w = 0u;
+            g_give_up.store(w, std::memory_order_release);
+        }
+    }
+    *word = w;
+    return UMB_OK;
+}
+int give_up_status() {
+    const volatile unsigned int* w = g_give_up.load(std::memory_order_acquire);
+    return w != nullptr && *w != 0u ? UMB_ERR_TIMEOUT : UMB_OK;
+}
 int sm_count() {
     // cached per device ordinal: one process may drive several GPUs (benign race: every thread computes the same value)
     static int cached[64] = {0};
@@ -69,6 +94,13 @@ extern "C" const char* umb_error_string(int code) {
     }
     if (code > 0) return cudaGetErrorString((cudaError_t)code);
     return "unknown error";
+}
+
+extern "C" unsigned int umb_give_ups_seen(void) { return umb::give_up_status() != UMB_OK; }
+
+extern "C" unsigned int* umb_give_up_word(void) {
+    unsigned int* w = nullptr;
+    return umb::give_up_word(&w) == UMB_OK ? w : nullptr;
 }
 
 extern "C" void umb_launch_count_add(unsigned long long n) { umb::g_launches.fetch_add(n, std::memory_order_relaxed); }

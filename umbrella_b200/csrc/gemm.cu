@@ -982,6 +982,7 @@ static int gemm_common(bool awq, const void* x, int64_t ldx, const void* w, int6
                        cudaStream_t st) {
     UMB_CHECK_ARG(x && w && y && M >= 1 && K >= 1 && N_total >= 1);
     UMB_CHECK_ARG((((uintptr_t)x | (uintptr_t)w) & 15) == 0 && (ldx % 8) == 0 && ldx >= K);
+    if (const int gave_up = give_up_status()) return gave_up;
     if (M > (awq ? 512 : 128)) return UMB_ERR_UNSUPPORTED;
     if (awq ? (K % kGroup) != 0 : (K % 64) != 0) return UMB_ERR_UNSUPPORTED;
     if (N_total % 8) return UMB_ERR_UNSUPPORTED;

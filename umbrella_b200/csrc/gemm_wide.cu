@@ -23,9 +23,6 @@
 // a range is 12 us of 100.  us, four passes of 125 rows through gemm.cu's kernel / one of 500 here: a layer of width 4096 and its head 695 / 458, of width 8192
 // 1363 / 1088; 1000 rows 1244 / 759, 300 540 / 380, 129 376 / 306.  Up to 128 rows, one pass on both sides, this gains nothing (gemm.cu does them).  Of no effect: fewer records, fewer or no x
 // copies, no arithmetic in the dequantisation (2 to 8 % each), deeper record rings.
-#include <atomic>
-#include <mutex>
-
 #include "gemm_core.cuh"
 #include "group_gate.h"
 
@@ -43,8 +40,6 @@ template <int NPAD> struct WideCfg {
     static constexpr int kX = (512 - NPAD) / 128 * 2;       // x slabs, and parts of the A operand (64 columns each, behind the accumulator)
     static constexpr int kSmem = 1024 + kX * kXBytes + kWideW * kWideRecord + 3 * kWideExch;
 };
-
-__device__ unsigned int g_wide_timeouts;
 
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
@@ -75,10 +70,7 @@ __device__ __forceinline__ void commit_pair(uint64_t* bar) {                // t
 
 // Every wait is bounded (seconds): a block that gives up raises its flag and all of its roles leave their loops.
 __device__ __forceinline__ bool give_up(volatile int* quit) {
-    if (!*quit) {
-        *quit = 1;
-        atomicAdd(&g_wide_timeouts, 1u);
-    }
+    *quit = 1;
     return false;
 }
 // PAIR: a barrier that the other block's threads, or products of both, arrive at.  What such a barrier hands over is in tensor memory, or the products' reads of
@@ -438,33 +430,11 @@ awq_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     }
 }
 
-// A word of host memory that a block which gave up sets: later launches are refused, results since then are not to be used.
-std::atomic<unsigned int*> g_gave_up{nullptr};
-int gave_up_word(unsigned int** word) {
-    static std::mutex making;
-    unsigned int* w = g_gave_up.load(std::memory_order_acquire);
-    if (w == nullptr) {
-        std::lock_guard<std::mutex> lock(making);
-        w = g_gave_up.load(std::memory_order_acquire);
-        if (w == nullptr) {
-            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // (the first call may be inside a capture)
-            UMB_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-            const cudaError_t e = cudaHostAlloc((void**)&w, sizeof *w, cudaHostAllocPortable | cudaHostAllocMapped);
-            cudaThreadExchangeStreamCaptureMode(&mode);
-            if (e != cudaSuccess) return (int)e;
-            *w = 0u;
-            g_gave_up.store(w, std::memory_order_release);
-        }
-    }
-    *word = w;
-    return *(volatile unsigned int*)w != 0u ? UMB_ERR_TIMEOUT : UMB_OK;
-}
-
 template <int NPAD>
 int launch_wide(const void* x, int64_t ldx, GemmParams p, WideRows rb, cudaStream_t st) {
     p.rope_vec_ok = 0;                                      // (kWideExch)
     unsigned int* report = nullptr;
-    int rc = gave_up_word(&report);
+    int rc = give_up_word(&report);
     if (rc != UMB_OK) return rc;
     CUtensorMap map;
     rc = make_tmap_x3d(&map, x, (uint64_t)p.M, (uint64_t)p.K, (uint64_t)ldx, WideCfg<NPAD>::kRows);

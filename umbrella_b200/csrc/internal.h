@@ -35,6 +35,10 @@ inline cudaError_t launch_pdl(const char* name, void (*kernel)(KArgs...), dim3 g
 #define UMB_LAUNCH_PDL(kernel, ...) do { cudaError_t e__ = umb::launch_pdl(#kernel, kernel, __VA_ARGS__); if (e__ != cudaSuccess) return (int)e__; } while (0)
 // every host entry point reports the kernels it enqueued (umb_launch_count)
 void count_launches(unsigned n);
+// 4 bytes of host memory for the process, shared by its devices, streams and threads, that a block which gave up on a bounded wait sets: results since then are
+// not to be used, workspaces may hold words that are not theirs.  Made on the first call; an error of the runtime, or 0.
+int give_up_word(unsigned int** word);
+int give_up_status();                                       // 0, or UMB_ERR_TIMEOUT
 // gemm_wide.cu: AWQ products of 129 to 512 token rows by pairs of SMs, with a workspace of awq_wide_ws_bytes() bytes
 struct GemmParams;
 size_t awq_wide_ws_bytes(int M, int N_total);

@@ -21,7 +21,7 @@ import time
 
 import torch
 
-from .. import ops
+from .. import _lib, ops
 from ..models.auto_model import AutoModelLM
 from .base import BaseEngine
 from .speculation_utils import (is_sentence_complete_regex, sample_topk_topp_torch, split_model_config,
@@ -216,6 +216,7 @@ class DynamicSpeculationEngine(BaseEngine):
         self.parents.zero_()                     # dynamic...:325-326
         self.tree_score.zero_()
         torch.cuda.current_stream().synchronize()
+        _lib.raise_if_given_up()
         accept_length, cont, new_n = (int(x) for x in self._result_host[:3])
         self.draft_model.kv_cache.kv_offset = n + accept_length
         self.target_model.kv_cache.kv_offset = n + accept_length

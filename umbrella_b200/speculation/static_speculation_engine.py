@@ -264,6 +264,7 @@ class StaticSpeculationEngine(BaseEngine):
             g[0].replay()
             _lib.load().umb_launch_count_add(g[1])
             torch.cuda.current_stream().synchronize()
+        _lib.raise_if_given_up()
         accept_length, cont, new_n = (int(x) for x in self._result_host[:3])
         self.draft_model.kv_cache.kv_offset = n + accept_length
         self.target_model.kv_cache.kv_offset = n + accept_length
@@ -355,6 +356,7 @@ class StaticSpeculationEngine(BaseEngine):
         self.target_model.kv_cache.gather_from_result(self._result, n, 0)
         self._result_host.copy_(self._result, non_blocking=True)
         torch.cuda.current_stream().synchronize()
+        _lib.raise_if_given_up()
         accept_length, cont, new_n = (int(x) for x in self._result_host[:3])
         self.draft_model.kv_cache.kv_offset = n + accept_length
         self.target_model.kv_cache.kv_offset = n + accept_length
