@@ -103,3 +103,24 @@ def test_the_native_calls_load_in_a_process_without_torch():
     import sys
     code = "import sys; from umbrella_b200 import _lib_seq; assert 'torch' not in sys.modules; assert _lib_seq.load_calls().gemm"
     subprocess.run([sys.executable, "-c", code], check=True, cwd=S.__file__.rsplit("/", 2)[0])
+
+
+def test_the_native_calls_are_found_for_what_they_were_made_with(monkeypatch):
+    """Sources, torch and Python: the module holds layouts of all three, and a file made for others must not be loaded."""
+    import os
+    import sysconfig
+
+    from umbrella_b200 import build
+    here = build.calls_path()
+    assert build.calls_path() == here and build.build_calls() == here and os.path.exists(here)
+    paths = {here}
+    with monkeypatch.context() as m:
+        m.setattr(torch, "__version__", "2.99.0")
+        paths.add(build.calls_path())
+    with monkeypatch.context() as m:
+        m.setattr(sysconfig, "get_config_var", lambda name: "cpython-399")
+        paths.add(build.calls_path())
+    with monkeypatch.context() as m:
+        m.setattr(build, "_CALLS_DEPS", build._CALLS_DEPS[:1] + [__file__])
+        paths.add(build.calls_path())
+    assert len(paths) == 4 and sum(map(os.path.exists, paths)) == 1

@@ -246,13 +246,9 @@ def load_calls():
 
         from . import build
         lib = load()
-        try:
-            build.build_calls()
-        except RuntimeError:
-            if not os.path.exists(build.CALLS):
-                raise
-        loader = importlib.machinery.ExtensionFileLoader("_seq_calls", build.CALLS)
-        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_seq_calls", build.CALLS, loader=loader))
+        path = build.build_calls()
+        loader = importlib.machinery.ExtensionFileLoader("_seq_calls", path)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_seq_calls", path, loader=loader))
         loader.exec_module(mod)
         mod.bind(*(C.cast(getattr(lib, name), c_void_p).value for name in _CALLED))
         calls = mod

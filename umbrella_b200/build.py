@@ -115,21 +115,34 @@ def build_seq(force: bool = False, verbose: bool = False) -> str:
 
 
 CALLS_SOURCE = os.path.join(CSRC, "seq", "calls.cpp")
-CALLS = os.path.join(HERE, "_seq_calls.so")
+_CALLS_DEPS = [CALLS_SOURCE] + [os.path.join(CSRC, "..", "..", "include", h) for h in ("umbrella_b200_seq.h", "umbrella_b200.h")]
+
+
+def calls_path() -> str:
+    """The module's file for these sources, this torch and this Python: it holds layouts of all three, so its name holds a digest of them and
+    a file made for others is never found."""
+    import hashlib
+    import sysconfig
+
+    import torch
+    h = hashlib.sha256(f"{torch.__version__} {torch._C._GLIBCXX_USE_CXX11_ABI} {sysconfig.get_config_var('SOABI')}".encode())
+    for d in _CALLS_DEPS:
+        h.update(open(d, "rb").read())
+    return os.path.join(HERE, f"_seq_calls.{h.hexdigest()[:16]}.so")
 
 
 def build_calls(force: bool = False, verbose: bool = False) -> str:
-    """_seq_calls.so: the tensor-level calls' way into libumbrella_b200_seq.so (a Python module over torch's own headers; the torch
+    """_seq_calls.*.so: the tensor-level calls' way into libumbrella_b200_seq.so (a Python module over torch's own headers; the torch
     libraries are the ones the process has loaded)."""
-    deps = [CALLS_SOURCE, os.path.join(CSRC, "..", "..", "include", "umbrella_b200_seq.h"), os.path.join(CSRC, "..", "..", "include", "umbrella_b200.h")]
-    if not force and not _stale(CALLS, deps):
-        return CALLS
+    path = calls_path()
+    if not force and os.path.exists(path):
+        return path
     import sysconfig
 
     import torch
     t = os.path.dirname(torch.__file__)
     cuda = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
-    tmp = f"{CALLS}.{os.getpid()}.tmp"
+    tmp = f"{path}.{os.getpid()}.tmp"
     cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            "-I", os.path.join(t, "include"), "-I", os.path.join(t, "include", "torch", "csrc", "api", "include"), "-I", sysconfig.get_path("include"), "-I", cuda,
            CALLS_SOURCE, "-o", tmp, "-L", os.path.join(t, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
@@ -138,8 +151,8 @@ def build_calls(force: bool = False, verbose: bool = False) -> str:
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed on {CALLS_SOURCE}:\n{r.stdout}")
-    os.replace(tmp, CALLS)
-    return CALLS
+    os.replace(tmp, path)
+    return path
 
 
 if __name__ == "__main__":
