@@ -101,7 +101,7 @@ def test_the_native_calls_load_in_a_process_without_torch():
     """A build check imports the package and nothing else."""
     import subprocess
     import sys
-    code = "import sys; from umbrella_b200 import _lib_seq; assert 'torch' not in sys.modules; assert _lib_seq.load_calls().gemm"
+    code = "import sys; from umbrella_b200 import _lib_seq; assert 'torch' not in sys.modules; assert _lib_seq.load_calls() is not _lib_seq.DECLINES"
     subprocess.run([sys.executable, "-c", code], check=True, cwd=S.__file__.rsplit("/", 2)[0])
 
 
@@ -124,3 +124,22 @@ def test_the_native_calls_are_found_for_what_they_were_made_with(monkeypatch):
         m.setattr(build, "_CALLS_DEPS", build._CALLS_DEPS[:1] + [__file__])
         paths.add(build.calls_path())
     assert len(paths) == 4 and sum(map(os.path.exists, paths)) == 1
+
+
+@pytest.mark.parametrize("what", ["no compiler", "a build that fails", "a file that does not load"])
+def test_calls_do_without_the_native_way(monkeypatch, recorder, tmp_path, what):
+    """Whatever keeps the module from being had is said once, and the wrappers' own way goes on."""
+    from umbrella_b200 import build
+    monkeypatch.setattr(S, "calls", None)
+    if what == "a file that does not load":
+        (tmp_path / "x.so").write_bytes(b"not a library")
+        monkeypatch.setattr(build, "build_calls", lambda *a, **k: str(tmp_path / "x.so"))
+    else:
+        monkeypatch.setattr(build, "calls_path", lambda: str(tmp_path / "none.so"))
+        monkeypatch.setattr(build.shutil, "which", lambda name: str(tmp_path / "g++") if what == "no compiler" else "/bin/false")
+        monkeypatch.setattr(build, "_nvcc", lambda: "/usr/local/cuda/bin/nvcc")
+    with pytest.warns(RuntimeWarning, match="ctypes"):
+        assert S.load_calls() is S.DECLINES
+    assert S.load_calls() is S.DECLINES and S.DECLINES.gemm(1, 2) is None
+    a, w = torch.ones(6, 8, dtype=torch.bfloat16), torch.ones(4, 8, dtype=torch.bfloat16)
+    assert K.gemm(a, w).shape == (6, 4)

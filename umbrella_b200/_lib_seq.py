@@ -235,8 +235,21 @@ _CALLED = ("umbs_gemm", "umbs_gemm_sorted", "umbs_moe_route", "umbs_add_norm", "
            "umbs_window_attention_gated", "umbs_retention_ex")       # its Entries, in order
 
 
+class _Declines:
+    """Stands in for the module where it cannot be had: takes no call, so every wrapper of ops_seq goes its own way."""
+
+    def __getattr__(self, name):
+        if name.startswith("__"):
+            raise AttributeError(name)
+        return lambda *a: None
+
+
+DECLINES = _Declines()
+
+
 def load_calls():
-    """The native way from tensors to the library that ops_seq takes for its most frequent calls."""
+    """The native way from tensors to the library that ops_seq takes for its most frequent calls; DECLINES, with a warning, where it cannot be
+    built or loaded (no C++ compiler, other headers)."""
     global calls
     if calls is None:
         import importlib.machinery
@@ -246,11 +259,16 @@ def load_calls():
 
         from . import build
         lib = load()
-        path = build.build_calls()
-        loader = importlib.machinery.ExtensionFileLoader("_seq_calls", path)
-        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_seq_calls", path, loader=loader))
-        loader.exec_module(mod)
-        mod.bind(*(C.cast(getattr(lib, name), c_void_p).value for name in _CALLED))
+        try:
+            path = build.build_calls()
+            loader = importlib.machinery.ExtensionFileLoader("_seq_calls", path)
+            mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_seq_calls", path, loader=loader))
+            loader.exec_module(mod)
+            mod.bind(*(C.cast(getattr(lib, name), c_void_p).value for name in _CALLED))
+        except Exception as e:                              # (a compiler that is not there, a build or an import that fails: the wrappers do without)
+            import warnings
+            warnings.warn(f"umbrella_b200: tensor-level calls go through ctypes, {type(e).__name__}: {str(e)[:300]}", RuntimeWarning, stacklevel=3)
+            mod = DECLINES
         calls = mod
     return calls
 
