@@ -143,3 +143,27 @@ def test_calls_do_without_the_native_way(monkeypatch, recorder, tmp_path, what):
     assert S.load_calls() is S.DECLINES and S.DECLINES.gemm(1, 2) is None
     a, w = torch.ones(6, 8, dtype=torch.bfloat16), torch.ones(4, 8, dtype=torch.bfloat16)
     assert K.gemm(a, w).shape == (6, 4)
+
+
+def test_threads_at_their_first_call_build_once(monkeypatch, recorder, tmp_path):
+    """Two builds at a time would write and move the same temporary file."""
+    import threading
+    import time
+
+    from umbrella_b200 import build
+    made = []
+
+    def slow(*a, **k):
+        made.append(threading.get_ident())
+        time.sleep(0.2)
+        raise RuntimeError("not here")
+    monkeypatch.setattr(build, "build_calls", slow)
+    monkeypatch.setattr(S, "calls", None)
+    got = []
+    with pytest.warns(RuntimeWarning, match="not here"):
+        threads = [threading.Thread(target=lambda: got.append(S.load_calls())) for _ in range(4)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    assert got == [S.DECLINES] * 4 and len(made) == 1

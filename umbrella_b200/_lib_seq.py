@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import threading
 
 from ._lib import c_float, c_int, c_int64, c_size_t, c_void_p
 
@@ -245,13 +246,18 @@ class _Declines:
 
 
 DECLINES = _Declines()
+_loading = threading.RLock()     # what is built and loaded at the first call is so once, whichever threads make it
 
 
 def load_calls():
     """The native way from tensors to the library that ops_seq takes for its most frequent calls; DECLINES, with a warning, where it cannot be
     built or loaded (no C++ compiler, other headers)."""
     global calls
-    if calls is None:
+    if calls is not None:
+        return calls
+    with _loading:
+        if calls is not None:
+            return calls
         import importlib.machinery
         import importlib.util
 
@@ -278,19 +284,22 @@ def load() -> C.CDLL:
     global _lib
     if _lib is not None:
         return _lib
-    from . import build
-    try:
-        build.build_seq()
-    except RuntimeError:
-        if not os.path.exists(LIB_PATH):
-            raise
-    lib = C.CDLL(LIB_PATH)
-    for name, (res, args) in SIGNATURES.items():
-        fn = getattr(lib, name)
-        fn.restype = res
-        fn.argtypes = args
-    _lib = lib
-    return lib
+    with _loading:
+        if _lib is not None:
+            return _lib
+        from . import build
+        try:
+            build.build_seq()
+        except RuntimeError:
+            if not os.path.exists(LIB_PATH):
+                raise
+        lib = C.CDLL(LIB_PATH)
+        for name, (res, args) in SIGNATURES.items():
+            fn = getattr(lib, name)
+            fn.restype = res
+            fn.argtypes = args
+        _lib = lib
+        return lib
 
 
 GAVE_UP = "an earlier kernel gave up on a wait: results since then, cached states among them, are not to be used"
