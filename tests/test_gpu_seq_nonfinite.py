@@ -190,3 +190,29 @@ def test_attention_of_a_steps_own_keys(what, shared, window):
         want = seen_only(q[:, h * (dim + shared):(h + 1) * (dim + shared)].double(), keys, v[:, h * dim:(h + 1) * dim].double(), visible,
                          float(torch.tensor((dim + shared) ** -0.5)), sink[h].double())
         assert_same(out[:, h * dim:(h + 1) * dim], want)
+
+
+@pytest.mark.parametrize("what", list(BAD))
+@pytest.mark.parametrize("tokens,past", [(20, 0), (77, 0), (130, 0), (40, 90), (65, 700)])
+@pytest.mark.parametrize("dim,window", [(64, 0), (128, 100), (40, 30)])
+def test_a_neighbours_numbers_do_not_reach_a_sequence(what, tokens, past, dim, window):
+    """Numbers that are not finite in the rows behind a sequence's own leave it as it is, bit for bit: neither in its results nor on the way of the plain
+    rows, which sum in another order."""
+    from umbrella_b200 import _lib_seq as S, ops_seq as K
+    heads, kv_heads, more = 4, 2, 50
+    kdim, n = kv_heads * dim, tokens + more
+    q, rows = rnd(n, heads * dim, seed=1).bfloat16(), rnd(n, 2 * kdim, seed=2).bfloat16()
+    cache = rnd(2, past + tokens + 64, 2 * kdim, seed=4).bfloat16().to(DEV)
+    sink = rnd(heads, seed=3).to(DEV)
+    bad = rows.clone()
+    for at in (tokens, tokens + 3):
+        for g in range(kv_heads):
+            BAD[what](bad[at] if what == "token" else bad[at, kdim + g * dim:kdim + (g + 1) * dim], 0)
+    batch = K.RaggedBatch([(0, tokens, past, 0), (1, more, 0, 0)], DEV)
+    cached = [K.cached_attention(q.to(DEV), r.to(DEV), cache, batch, heads, kv_heads, dim, dim, dim ** -0.5, mode=S.UMBS_ATTN_SOFTMAX_SINK, window=window, sink=sink,
+                                 append=False)[:tokens] for r in (rows, bad)]
+    assert torch.equal(*cached) and bool(torch.isfinite(cached[0]).all())
+    if past == 0:
+        own = [K.window_attention_shared(q[:, :kdim].contiguous().to(DEV), r[:, :kdim].to(DEV), None, r[:, kdim:].to(DEV), batch, kv_heads, dim ** -0.5, window=window,
+                                         use_sink=False)[:tokens] for r in (rows, bad)]
+        assert torch.equal(*own)

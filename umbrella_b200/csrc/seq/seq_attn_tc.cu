@@ -119,12 +119,13 @@ template <int MODE, bool SHAPED, bool STEP>
 __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_s, const __grid_constant__ CUtensorMap map_v,
                                                                         const __grid_constant__ CachedAttnArgs a, const __grid_constant__ StepKeys x, const __grid_constant__ Batch b, const TaDims z) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ uint64_t bars[4 * kTaHeld + 7];
+    __shared__ uint64_t bars[4 * kTaHeld + 8];
     __shared__ float s_row[2][2][kTaQ];                     // what a row's two threads tell each other: [tile parity][half]
     __shared__ uint32_t s_tmem;
     __shared__ int s_quit;
     uint64_t *k_full = bars, *k_empty = k_full + kTaHeld, *v_full = k_empty + kTaHeld, *v_empty = v_full + kTaHeld, *s_full = v_empty + kTaHeld, *p_full = s_full + 2,
-             *o_full = s_full + 4, *q_full = s_full + 5, *lo_full = s_full + 6;       // (p_full: two in turn, a warp may be a tile ahead of another there)
+             *o_full = s_full + 4, *q_full = s_full + 5, *lo_full = s_full + 6,        // (p_full: two in turn, a warp may be a tile ahead of another there)
+             *v_landed = s_full + 7;                        // values of a last tile with rows behind the last
     volatile int* quit = &s_quit;
     if (threadIdx.x == 0) {
         for (int i = 0; i < kTaHeld; ++i) {
@@ -140,6 +141,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
         umb::mbar_init(o_full, 1);
         umb::mbar_init(q_full, 8);
         umb::mbar_init(lo_full, 8);
+        umb::mbar_init(v_landed, 1);
         s_quit = 0;
         umb::fence_barrier_init();
     }
@@ -198,8 +200,8 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
         };
         for (int i = 0; i < kt.n; ++i) {
             const int base = kt.base(i), last = kt.last(i), ks = i % z.k_held, vs = i % z.v_held;
-            // rows that are neighbours: of the step (behind its sequence's last come the next one's, whose weights are 0, and zeros behind the step's:
-            // prompts of 20 tokens 13.3 us when those tiles were copied row by row), or of the ring where it does not begin again
+            // rows that are neighbours: of the step (behind the last that a query sees come others', whose weights are 0: their scores are never looked at, their
+            // values are cleared below; prompts of 20 tokens 13.3 us when those tiles were copied row by row), or of the ring where it does not begin again
             const int at0 = STEP ? 0 : base % a.kv_len;     // the first key's place in the ring
             const bool of_step = base >= pos0, of_ring = !STEP && base + kTaK <= pos0 && at0 + kTaK <= a.kv_len && (int64_t)(slot + 1) * a.kv_len <= z.ring_rows;
             const bool tma = z.tma && !kt.pooled(i) && (of_step || of_ring);
@@ -266,16 +268,28 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
             if (i >= z.v_held) free = tc_spin_warp(v_empty + vs, (i / z.v_held - 1) & 1, quit);
             if (!__all_sync(0xffffffffu, free)) break;
             if (tma) {
+                const int rows = last - base + 1;           // fewer than a tile's: of the last tile alone
+                uint64_t* bar = rows < kTaK ? v_landed : v_full + vs;
                 if (umb::elect_one()) {
                     if (warp == 10) {
-                        umb::mbar_arrive_expect_tx(v_full + vs, (uint32_t)v_bytes);
+                        umb::mbar_arrive_expect_tx(bar, (uint32_t)v_bytes);
                         for (int at = 0; at < z.v_atoms; ++at)
-                            tma_3d(s_v + vs * v_bytes + at * (kTaK * 128), STEP || of_step ? &map_v : &map_s, (STEP ? vh * a.vdim : vhd.voff) + at * 64, row, 0, v_full + vs);
+                            tma_3d(s_v + vs * v_bytes + at * (kTaK * 128), STEP || of_step ? &map_v : &map_s, (STEP ? vh * a.vdim : vhd.voff) + at * 64, row, 0, bar);
                     } else {
                         umb::mbar_arrive(v_full + vs);
                     }
                 }
                 __syncwarp();
+                // a value of another sequence that is not finite, times a weight of 0, would send this one's rows through plain_row
+                if (warp == 10 && rows < kTaK) {
+                    if (!tc_spin_warp(v_landed, 0, quit)) break;
+                    for (int at = 0; at < z.v_atoms; ++at)
+                        for (int e = rows * 8 + lane; e < kTaK * 8; e += 32)
+                            *reinterpret_cast<uint4*>(s_v + vs * v_bytes + at * (kTaK * 128) + e * 16) = make_uint4(0u, 0u, 0u, 0u);
+                    umb::fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) umb::mbar_arrive(v_full + vs);
+                }
             } else {
                 for (int h = 0; h < 2; ++h)
 #pragma unroll
