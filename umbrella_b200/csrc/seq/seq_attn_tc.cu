@@ -198,6 +198,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
             publish(false);
             pending = bar;
         };
+        int last_vs = -1;
         for (int i = 0; i < kt.n; ++i) {
             const int base = kt.base(i), last = kt.last(i), ks = i % z.k_held, vs = i % z.v_held;
             // rows that are neighbours: of the step (behind the last that a query sees come others', whose weights are 0: their scores are never looked at, their
@@ -268,10 +269,10 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
             if (i >= z.v_held) free = tc_spin_warp(v_empty + vs, (i / z.v_held - 1) & 1, quit);
             if (!__all_sync(0xffffffffu, free)) break;
             if (tma) {
-                const int rows = last - base + 1;           // fewer than a tile's: of the last tile alone
-                uint64_t* bar = rows < kTaK ? v_landed : v_full + vs;
+                const bool clear = base + kTaK - 1 > last;  // (of the last tile alone)
                 if (umb::elect_one()) {
                     if (warp == 10) {
+                        uint64_t* bar = clear ? v_landed : v_full + vs;
                         umb::mbar_arrive_expect_tx(bar, (uint32_t)v_bytes);
                         for (int at = 0; at < z.v_atoms; ++at)
                             tma_3d(s_v + vs * v_bytes + at * (kTaK * 128), STEP || of_step ? &map_v : &map_s, (STEP ? vh * a.vdim : vhd.voff) + at * 64, row, 0, bar);
@@ -280,16 +281,7 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
                     }
                 }
                 __syncwarp();
-                // a value of another sequence that is not finite, times a weight of 0, would send this one's rows through plain_row
-                if (warp == 10 && rows < kTaK) {
-                    if (!tc_spin_warp(v_landed, 0, quit)) break;
-                    for (int at = 0; at < z.v_atoms; ++at)
-                        for (int e = rows * 8 + lane; e < kTaK * 8; e += 32)
-                            *reinterpret_cast<uint4*>(s_v + vs * v_bytes + at * (kTaK * 128) + e * 16) = make_uint4(0u, 0u, 0u, 0u);
-                    umb::fence_proxy_async_smem();
-                    __syncwarp();
-                    if (lane == 0) umb::mbar_arrive(v_full + vs);
-                }
+                last_vs = clear ? vs : -1;
             } else {
                 for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -307,6 +299,17 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
             }
         }
         publish(true);
+        if (warp == 10 && last_vs >= 0 && tc_spin_warp(v_landed, 0, quit)) {
+            const int rows = kt.last(kt.n - 1) - kt.base(kt.n - 1) + 1;
+#pragma unroll 1
+            for (int at = 0; at < z.v_atoms; ++at)
+#pragma unroll 1
+                for (int e = rows * 8 + lane; e < kTaK * 8; e += 32)
+                    *reinterpret_cast<uint4*>(s_v + last_vs * v_bytes + at * (kTaK * 128) + e * 16) = make_uint4(0u, 0u, 0u, 0u);
+            umb::fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) umb::mbar_arrive(v_full + last_vs);
+        }
     } else if (warp == 8) {
         // ------------------------------------------------------------------------------------ products
         const uint32_t idesc_s = tc_idesc(kTaQ, kTaK), idesc_o = tc_idesc(kTaQ, 64, true) + ((z.v_atoms - 1) * (64u >> 3) << 17);
