@@ -115,6 +115,14 @@ __device__ __noinline__ void plain_row(const CachedAttnArgs& a, const StepKeys& 
     }
 }
 
+// A gate's sigmoid.  The approximate reciprocal and one Newton-Raphson step are the rounded quotient for every 1 + e^-g below 2^126 (all of them compared); behind
+// that come quotients below the smallest normal number, which the caller works out by the division (far).
+__device__ __forceinline__ float gate_of(float g, bool& far) {
+    const float x = 1.f + expf(-g), r = __fdividef(1.f, x);
+    far |= x >= 0x1p126f;
+    return fmaf(r, fmaf(-x, r, 1.f), r);
+}
+
 template <int MODE, bool SHAPED, bool STEP>
 __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_s, const __grid_constant__ CUtensorMap map_v,
                                                                         const __grid_constant__ CachedAttnArgs a, const __grid_constant__ StepKeys x, const __grid_constant__ Batch b, const TaDims z) {
@@ -563,12 +571,22 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
                             const float* gp = a.gate + (int64_t)(start + q0 + row0 + e0 + e) * a.ldg + h * a.vdim + c;
                             g[e] = ((uintptr_t)gp & 15) == 0 ? *reinterpret_cast<const float4*>(gp) : make_float4(gp[0], gp[1], gp[2], gp[3]);
                         }
+                    bool far = false;
 #pragma unroll
                     for (int e = 0; e < 8; ++e)
                         if (e0 + e < rows) {
                             const float4 o = *reinterpret_cast<const float4*>(s_o + (row0 + e0 + e) * ldo + c);
-                            put(row0 + e0 + e, make_float4(o.x * sigmoidf_(g[e].x), o.y * sigmoidf_(g[e].y), o.z * sigmoidf_(g[e].z), o.w * sigmoidf_(g[e].w)));
+                            const float4 w = make_float4(gate_of(g[e].x, far), gate_of(g[e].y, far), gate_of(g[e].z, far), gate_of(g[e].w, far));
+                            put(row0 + e0 + e, make_float4(o.x * w.x, o.y * w.y, o.z * w.z, o.w * w.w));
                         }
+                    if (far) {                              // rare: these rows once more
+#pragma unroll 1
+                        for (int e = e0; e < min(rows, e0 + 8); ++e) {
+                            const float* gp = a.gate + (int64_t)(start + q0 + row0 + e) * a.ldg + h * a.vdim + c;
+                            const float4 o = *reinterpret_cast<const float4*>(s_o + (row0 + e) * ldo + c);
+                            put(row0 + e, make_float4(o.x * sigmoidf_(gp[0]), o.y * sigmoidf_(gp[1]), o.z * sigmoidf_(gp[2]), o.w * sigmoidf_(gp[3])));
+                        }
+                    }
                 }
             }
         }
