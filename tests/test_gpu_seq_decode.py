@@ -1,4 +1,4 @@
-"""What a decode step reads of a cache: means of whole blocks (umbs_kv_pool) bit for bit, the routing of up to 64 tokens bit for bit, and the grouped attention with four and with six warps
+"""What a decode step reads of a cache: means of whole blocks (umbs_kv_pool) bit for bit, the routing of up to 148 tokens bit for bit, and the grouped attention with four and with six warps
 a block (unsplit steps from 148 blocks on) against float64.
 
 Tolerance: results are bf16 (2^-9 of their size at most, 2^-9 / sqrt(3) in the norm); the fp32 work inside is four orders below."""
@@ -60,13 +60,13 @@ def test_groups_of_heads(mode, seqs, kv_heads, group, dim, ctx):
 
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("n,experts,width,top,gate", [(17, 15, 100, 2, True), (17, 16, 1024, 3, False), (64, 16, 1152, 2, True), (64, 17, 2052, 1, False), (64, 300, 64, 9, True),
-                                                      (20, 1024, 1030, 4, False), (20, 1025, 128, 4, False)])
+                                                      (20, 1024, 1030, 4, False), (20, 1025, 128, 4, False), (148, 8, 1152, 2, False), (148, 130, 512, 6, True)])
 def test_routing_of_few_tokens(dt, n, experts, width, top, gate):
-    """A block to a token and warps with one or two experts choose what four tokens to a block and four experts to a warp do (the same tokens among 70)."""
+    """A block to a token and warps with one or two experts choose what four tokens to a block and four experts to a warp do (the same tokens among 170)."""
     from umbrella_b200 import _lib_seq as S, ops_seq as K
     g = torch.Generator().manual_seed(9)
-    h, w, gw = torch.randn(70, width, generator=g).to(dt).to(DEV), torch.randn(experts, width, generator=g).to(DEV), torch.randn(width, generator=g).to(DEV)
-    few, many = (K.moe_route_ex(h[:m], w, top, S.UMBS_ROUTE_SOFTMAX_TOP, gate_w=gw if gate else None) for m in (n, 70))
+    h, w, gw = torch.randn(170, width, generator=g).to(dt).to(DEV), torch.randn(experts, width, generator=g).to(DEV), torch.randn(width, generator=g).to(DEV)
+    few, many = (K.moe_route_ex(h[:m], w, top, S.UMBS_ROUTE_SOFTMAX_TOP, gate_w=gw if gate else None) for m in (n, 170))
     for i in [0, 4] + [5] * gate:
         assert torch.equal(few[i], many[i][:n])
     off, tok, pos, sel = (t.cpu() for t in few[1:5])

@@ -1321,7 +1321,10 @@ extern "C" int umbs_moe_route_scaled(int dtype, const void* h, int n, int width,
     // eight pieces in flight; more share the router's rows, most once there are blocks enough.  us for the whole call, four tokens with four experts / one with
     // one / one with two / eight with four: width 2048, 16 experts, 20 tokens 11.4 / 9.5 / 10.4 / 14.4, 64 12.4 / 10.3 / 10.4 / 14.6, 256 13.5 / 15.5 / 16.1 /
     // 16.5, 4096 34 / 131 / 88 / 25; 64 tokens, 128 experts 41 / 29 / 27 / 62, 256 of width 4096 91 / 57 / 52 / 154, 8 of width 4096 14.5 / 10.4 / 10.5 / 18.5.
+    // The line is where these blocks fill the SMs: 128 tokens, width 2048, 8 to 32 experts 12.4 to 14.4 / 10.4 to 12.4, 128 experts 29.6 / 18.5; 160 tokens 13 to 14 / 11
+    // to 16, 30 / 27.  A row a warp while there are no more than its 16 warps: 40 tokens, 16 experts 10.3 / 10.3, 17 experts 11.8 / 10.4.
     // (thousands of experts need the larger shared memory)
+    constexpr int kRtFew = 148;
     const int rrows = experts + (gate_w != nullptr);
 #define UMBS_ROUTER(TT, EE, NW)                                                                                                          \
     UMBS_DISPATCH_T(dtype, {                                                                                                     \
@@ -1333,8 +1336,8 @@ extern "C" int umbs_moe_route_scaled(int dtype, const void* h, int n, int width,
         chain_launch((moe_router_kernel<T, TT, EE>), (n + TT - 1) / TT, 32 * std::min(NW, (rrows + EE - 1) / EE), smem, st, (const T*)h, n, width, w_router, experts, top, mode, groups, keep, \
                                                                             weight_scale, sel_w, sel_e, counts, gate_w, gate_out, cursor, grp_off, pair_tok, pair_pos); \
     })
-    if (n <= 64 && rrows <= 16) UMBS_ROUTER(1, 1, 16);
-    else if (n <= 64 && experts <= 1024) UMBS_ROUTER(1, 2, 16);
+    if (n <= kRtFew && rrows <= 16) UMBS_ROUTER(1, 1, 16);
+    else if (n <= kRtFew && experts <= 1024) UMBS_ROUTER(1, 2, 16);
     else if (n > 1024 && experts <= 1024) UMBS_ROUTER(8, 4, 8);
     else UMBS_ROUTER(4, 4, 8);
 #undef UMBS_ROUTER
