@@ -1,5 +1,5 @@
 """The AWQ product with 33 to 128 token rows, where the head of a split tile is reduced by all groups of warps in turn, and
-beyond 64 rows with weight records and x slabs in rings of their own.  K from one unit of 128 (fewer units than a ring is deep) to many tiles a
+beyond 64 rows with weight records and x slabs in rings of their own (csrc/gemm.cu, kSplit).  K from one unit of 128 (fewer units than a ring is deep) to many tiles a
 block shares, rows at the edges of the 16-row chunks, every epilogue that stages rows."""
 import numpy as np
 import pytest

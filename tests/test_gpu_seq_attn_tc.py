@@ -1,6 +1,6 @@
 """The tensor-core attention of steps with several tokens per sequence (csrc/seq/seq_attn_tc.cu; bf16 storage) against the
 general kernel run in float32 on the same bf16 numbers: every mask, score option and output form, at the sizes where tiles
-of 128 rows and 32 keys end.
+of 128 rows and 64 keys end.
 
 Tolerance: both sum exact products of bf16 numbers in fp32; what is left is the rounding of the bf16 result, at most 2^-8 of a
 value and so of the norm (the weights' and sums' 32-bit errors are below 1e-4 of that)."""
@@ -288,6 +288,34 @@ def test_decode_steps_of_few_keys(ops, heads, kv_heads, dim, keys):
             short.t[name].copy_(t)
         graph.replay()
         assert H.rel_err(out, ref.cpu()) < TOL
+
+
+# (tokens, position of the first): whole tiles of 64 keys and one key less and more, of the step, of the ring and of both; more rows than a block
+ENDS = [(63, 0), (64, 0), (127, 0), (129, 0), (191, 0), (193, 0), (2, 62), (2, 63), (2, 126), (40, 64), (64, 128), (65, 127), (129, 191)]
+
+
+@pytest.mark.parametrize("dim,vdim", [(40, 64), (64, 128), (128, 128), (192, 128)])         # two places for keys and values; one for keys; one for either
+@pytest.mark.parametrize("window", [0, 64, 100])
+def test_ends_of_key_tiles(ops, dim, vdim, window):
+    """Tiles that come by tensor map, the one between ring and step that is copied row by row, and both in turn with one place for them."""
+    for tokens, past in ENDS:
+        _both(ops, [(1, tokens, past, 0), (0, 3, past // 2, 0)], 4, 2, dim, vdim, window=window)
+        if window:
+            _both(ops, [(1, tokens, past, 0)], 2, 2, dim, vdim, window=window, pool=16)
+
+
+@pytest.mark.parametrize("slots,ring", [(1, 128), (3, 192), (2, 100)])
+def test_a_cache_that_ends_with_its_allocation(ops, slots, ring):
+    """The ring's tensor map ends with the memory that the cache is in: its last slot's last rows are read, and nothing behind them."""
+    heads, dim = 2, 64
+    g = torch.Generator(device=DEV).manual_seed(3)
+    T, row = 70, 2 * heads * dim
+    q, kv = _r(g, T, heads * dim), _r(g, T, row)
+    cache = _r(g, slots, ring, row)
+    assert cache.untyped_storage().nbytes() == cache.numel() * 2
+    batch = ops.RaggedBatch([(slots - 1, T, ring, 0)], DEV)
+    out = [ops.cached_attention(q.to(dt), kv.to(dt), cache.to(dt), batch, heads, heads, dim, dim, dim ** -0.5, window=ring, append=False) for dt in (torch.bfloat16, torch.float32)]
+    assert torch.isfinite(out[0].float()).all() and H.rel_err(out[0], out[1].cpu()) < TOL
 
 
 @pytest.mark.parametrize("own_keys", [False, True])
