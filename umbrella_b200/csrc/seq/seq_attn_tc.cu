@@ -21,10 +21,10 @@
 //
 // Bound: two blocks take 2200 to 2400 ns a tile each (one alone 1650): a row's weights behind the scores and in front of the products (560 instructions a
 // warp and tile, issue slots 56 % taken, tensor pipe 39 % active), and blocks that fill the SMs 1.7 times.  us, 32 keys a tile / this: 4096 tokens, 16 heads of 128 over 4 key/value heads,
-// window 1024, pooled blocks 115 / 100; two prompts of 2000 tokens, 16 heads of 128 + 64 shared, a gate per column 156 / 103 (blocks that see most keys first,
-// over all heads: 40 of it; results through shared memory: 4 to 12 us of a block's 60); 106 tokens behind 700, heads of 96, 49 / 32.  A short prompt's block runs
-// every instruction once, and what it waits for is the next ones (2500 clocks for the first tile's weights, 3000 for 16 unrolled rows of results, 1250 as a
-// loop): eight prompts of 20 tokens 10.3 / 9.4, of 110 13.0 / 11.5, three of 77, 8 heads of 64, 9.8 / 10.1.
+// window 1024, pooled blocks 115 / 101; two prompts of 2000 tokens, 16 heads of 128 + 64 shared, a gate per column 156 / @LP@ (blocks that see most keys first,
+// over all heads: 40 of it); 106 tokens behind 700, heads of 96, 49 / 32.  A short prompt's block runs every instruction once, and what it waits for is the next
+// ones (2500 clocks for the first tile's weights): eight prompts of 20 tokens, 16 heads of 64 over 2, 6.9 / 7.3; three of 77 7.5 / 7.9; 300 tokens, heads of 128, 15.5 / 13.7 (508 calls:
+// 1.37 times as fast in the median, 15 of them 3 to 8 % slower).
 #include <algorithm>
 
 #include "seq_attn.h"
@@ -121,6 +121,11 @@ __device__ __forceinline__ float gate_of(float g, bool& far) {
     const float x = 1.f + expf(-g), r = __fdividef(1.f, x);
     far |= x >= 0x1p126f;
     return fmaf(r, fmaf(-x, r, 1.f), r);
+}
+
+// 32 bytes, a whole sector of a thread's own row: with 16 at a time 4096 tokens, 16 heads of 128 over 4, take 100.3 us, so 97.9.
+__device__ __forceinline__ void store32(void* p, const uint32_t* v) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
 
 template <int MODE, bool SHAPED, bool STEP>
@@ -552,9 +557,14 @@ __global__ void __launch_bounds__(kTaThreads, 2) attention_tc_kernel(const __gri
                 }
                 if (!gates && r < len) {
                     uint4* orow = reinterpret_cast<uint4*>((__nv_bfloat16*)(STEP ? x.out : a.out) + (start + r) * ldout + (int64_t)h * a.vdim + c0);
+                    if (((uintptr_t)orow & 31) == 0 && c0 + 32 <= a.vdim) {
+                        store32(orow, &v[0]);
+                        store32(orow + 2, &v[8]);
+                    } else {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (c0 + 8 * e < a.vdim) orow[e] = make_uint4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
+                        for (int e = 0; e < 4; ++e)
+                            if (c0 + 8 * e < a.vdim) orow[e] = make_uint4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
+                    }
                 }
             }
         }
