@@ -302,8 +302,8 @@ typedef struct {
     const void* sin;         /* fp16 [S, D]                                                           */
     void* k_cache;           /* fp16 [L, S, Hkv, D]  (KV_Cache layout, cache.py:18-34)                */
     void* v_cache;
-    /* activations for up to 128 rows: hidden [128,H], normed [128,H], qkv [128,(Hq+2Hkv)*D],
-     * q_rot [128,Hq*D], attn_out [128,Hq*D], act [128,I]                                             */
+    /* activations for the rows R of a pass (128, or rows_per_pass of umb_llama_forward_passes): hidden [R,H],
+     * normed [R,H], qkv [R,(Hq+2Hkv)*D], q_rot [R,Hq*D], attn_out [R,Hq*D], act [R,I]                */
     void* hidden;
     void* normed;
     void* qkv;

@@ -20,8 +20,8 @@
 //
 // Bound: a unit takes 610 to 650 ns, its products 540 at the measured cuBLAS rate; the next tile's products wait for the columns of the one
 // before (5 us where it is published, 10 where it is finished: the accumulator fills half of tensor memory, so there is one), and the end of
-// a range is 12 us of 100.  us, four passes of 125 rows through gemm.cu's kernel / one of 500 here: a layer of width 4096 and its head 695 / 458, of width 8192
-// 1363 / 1088; 1000 rows 1244 / 759, 300 540 / 380, 129 376 / 306.  Up to 128 rows, one pass on both sides, this gains nothing (gemm.cu does them).  Of no effect: fewer records, fewer or no x
+// a range is 12 us of 100.  us, four passes of 125 rows through gemm.cu's kernel / one of 500 here: a layer of width 4096 and its head, weights from memory, 695 / 456, of width
+// 8192 1363 / 1129 (its 28672 k in passes); width 4096, 1000 rows 1244 / 757, 300 540 / 374, 129 376 / 304.  Up to 128 rows, one pass on both sides, this gains nothing (gemm.cu does them).  Of no effect: fewer records, fewer or no x
 // copies, no arithmetic in the dequantisation (2 to 8 % each), deeper record rings.
 #include "gemm_core.cuh"
 #include "group_gate.h"

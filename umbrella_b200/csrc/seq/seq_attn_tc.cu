@@ -21,7 +21,7 @@
 //
 // Bound: two blocks take 2200 to 2400 ns a tile each (one alone 1650): a row's weights behind the scores and in front of the products (560 instructions a
 // warp and tile, issue slots 56 % taken, tensor pipe 39 % active), and blocks that fill the SMs 1.7 times.  us, 32 keys a tile / this: 4096 tokens, 16 heads of 128 over 4 key/value heads,
-// window 1024, pooled blocks 115 / 101; two prompts of 2000 tokens, 16 heads of 128 + 64 shared, a gate per column 156 / @LP@ (blocks that see most keys first,
+// window 1024, pooled blocks 115 / 101; two prompts of 2000 tokens, 16 heads of 128 + 64 shared, a gate per column 156 / 106 (blocks that see most keys first,
 // over all heads: 40 of it); 106 tokens behind 700, heads of 96, 49 / 32.  A short prompt's block runs every instruction once, and what it waits for is the next
 // ones (2500 clocks for the first tile's weights): eight prompts of 20 tokens, 16 heads of 64 over 2, 6.9 / 7.3; three of 77 7.5 / 7.9; 300 tokens, heads of 128, 15.5 / 13.7 (508 calls:
 // 1.37 times as fast in the median, 15 of them 3 to 8 % slower).

@@ -71,8 +71,8 @@ __host__ __device__ constexpr uint32_t tc_idesc(uint32_t M, uint32_t N, bool w_m
 }
 
 // The sigmoids' quotient without the rounded division's branch, which costs 12 us of 50 over 4096 rows of 2 x 2048 sums: the
-// hardware's approximate reciprocal and one Newton-Raphson step, r (2 - x r) with the residual in one rounding.  Behind 2^126 the
-// quotient is below the smallest normal number and becomes 0.
+// hardware's approximate reciprocal and one Newton-Raphson step, r (2 - x r) with the residual in one rounding: the rounded quotient for every x
+// below 2^126 (all 1.06e9 compared).  Behind that the quotient is below the smallest normal number and becomes 0.
 __device__ __forceinline__ float tc_sigmoid(float z) {
     const float x = 1.f + expf(-z), r = __fdividef(1.f, x);
     return x >= 0x1p126f ? 0.f : fmaf(r, fmaf(-x, r, 1.f), r);

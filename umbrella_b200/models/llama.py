@@ -22,8 +22,8 @@ import torch
 from .. import _lib, ops
 from ..attn.cache import KV_Cache
 
-MAX_ROWS = 128   # rows per forward chunk of fp16 layers and of layer ranges
-AWQ_ROWS = 512   # rows per pass over AWQ layers
+MAX_ROWS = 128   # rows per pass over fp16 layers, and of a replayed graph
+AWQ_ROWS = 512   # rows per pass over AWQ layers, resident or paged
 
 
 @dataclass

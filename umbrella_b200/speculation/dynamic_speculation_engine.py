@@ -10,7 +10,7 @@ kwargs ``width / num_beams / depth``, same BaseEngine surface, same bookkeeping)
     ``bool[S, S]`` master mask and its per-level row copies do not exist: a node's mask row is
     ``ceil(N/32)`` words (child = parent row | own bit).
   * verify() (dynamic...:250-327): one native target forward over the N = width*depth+1 tree rows
-    (chunks of <= 128 rows inside the C call), arg-max fused into the lm_head epilogue for greedy
+    (passes of up to 128 rows, 512 over AWQ layers, inside the C call), arg-max fused into the lm_head epilogue for greedy
     decoding, then the same accept / gather kernels as the static engine.  The path test of the
     reference (``rowsum(accept * tree_mask) == depth + 1``) is the parent-chain walk of
     umb_tree_accept.
