@@ -15,7 +15,7 @@ DEV = "cuda:0"
 
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("row", [8, 12, 136, 264])                                   # one piece; no whole pieces; a tail behind 128 columns
-@pytest.mark.parametrize("pool,pos0,tokens,kv_len", [(1, 3, 2, 8), (16, 15, 1, 40), (64, 63, 1, 64), (64, 70, 130, 90), (100, 150, 60, 128)])
+@pytest.mark.parametrize("pool,pos0,tokens,kv_len", [(1, 3, 2, 8), (16, 15, 1, 40), (7, 20, 40, 50), (8, 20, 40, 50), (33, 30, 80, 64), (64, 63, 1, 64), (64, 70, 130, 90), (100, 150, 60, 128)])
 def test_means_of_blocks(dt, row, pool, pos0, tokens, kv_len):
     from umbrella_b200 import _lib_seq as S, ops_seq as K
     g = torch.Generator().manual_seed(7)

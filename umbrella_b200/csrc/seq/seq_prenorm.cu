@@ -534,21 +534,25 @@ __global__ void attention_prep_kernel(const float* __restrict__ proj, int64_t ld
 
 // One block per (block of tokens completed by the step, sequence, 128 columns): the fp32 mean, in position order, of the
 // block's kv rows as the cache holds them; a row's place in the ring is the one before it plus one.  All latency: VEC (rows of 16-byte
-// pieces) copies 64 rows to shared memory at once and adds from there; other rows are loaded sixteen ahead of the additions.  us for the
-// blocks that 64 decoding sequences complete, 64 rows of 1024 columns: 34 eight loads at a time with a division per row, 7.3 sixteen, 4.5 VEC.
+// pieces) copies 16 KB of them to shared memory at once and adds from there; other rows are loaded sixteen ahead of the additions.  us for the
+// blocks that 64 decoding sequences complete, 64 rows of 1024 columns: 34 eight loads at a time with a division per row, 7.3 sixteen, 4.5 VEC.  Means of four
+// rows: one round of either, and 4096 tokens of them are as many small blocks, 2.0 / 2.6 in VEC; of eight 1.0 to 1.05 times as fast, of sixteen 1.3.  Most decode
+// steps complete no block, and are a launch: 32 KB of shared memory a block made that 12 % longer.  Ten blocks fit on an SM: with as many registers as the compiler likes,
+// rows of 1028 columns took 1.3 times as long (4096 tokens, means of 32: 5.8 / 9.2).
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(128) kv_pool_kernel(const T* __restrict__ kv, const T* __restrict__ kv_cache, int kv_len, T* __restrict__ pool_cache,
+__global__ void __launch_bounds__(128, 10) kv_pool_kernel(const T* __restrict__ kv, const T* __restrict__ kv_cache, int kv_len, T* __restrict__ pool_cache,
                                                       int pool_len, Batch b, int row, int pool) {
-    constexpr int R = 64, W = 16 / (int)sizeof(T), P = 128 / W;  // rows of a round; numbers to a piece; pieces to 128 columns
+    constexpr int R = 128 / (int)sizeof(T), W = 16 / (int)sizeof(T), P = 128 / W;        // rows of a round; numbers to a piece; pieces to 128 columns
     __shared__ __align__(16) T s_x[VEC ? R * 128 : 1];
     chain_wait();
     const int s = blockIdx.y, pos0 = b.seq_pos0[s], len = b.seq_len[s], start = b.seq_start[s], slot = b.seq_slot[s];
     const int blk = pos0 / pool + blockIdx.x;                    // first block whose last token is in the step, onwards
     if ((int64_t)(blk + 1) * pool > (int64_t)pos0 + len || blk >= pool_len) return;
     const int c0 = blockIdx.z * 128, c = c0 + threadIdx.x;
-    const int j0 = blk * pool;
-    const T* step = kv + ((int64_t)start - pos0) * row;          // row j of the step's own rows at step + j row
-    const T* ring = kv_cache + (int64_t)slot * kv_len * row;
+    if (!VEC && c >= row) return;
+    const int j0 = blk * pool, piece = threadIdx.x % P, r0 = threadIdx.x / P, of = VEC ? c0 + piece * W : c;
+    const T* step = kv + ((int64_t)start - pos0) * row + of;     // row j of the step's own rows at step + j row
+    const T* ring = kv_cache + (int64_t)slot * kv_len * row + of;
     const int at = j0 % kv_len;                                  // row j0 + j of the ring: at + j, less its length behind its end
     auto place = [&](int j) -> const T* {
         const int r = at + j;
@@ -556,14 +560,13 @@ __global__ void __launch_bounds__(128) kv_pool_kernel(const T* __restrict__ kv, 
     };
     float acc = 0.f;
     if (VEC) {
-        const int piece = threadIdx.x % P, r0 = threadIdx.x / P;
         const unsigned dst = (unsigned)__cvta_generic_to_shared(s_x) + piece * 16;
         for (int j = 0; j < pool; j += R) {
             const int n = min(R, pool - j);
-            if (c0 + piece * W < row)
+            if (of < row)
 #pragma unroll 8
                 for (int r = r0; r < n; r += 128 / P)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + r * 128 * (int)sizeof(T)), "l"(place(j + r) + c0 + piece * W) : "memory");
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + r * 128 * (int)sizeof(T)), "l"(place(j + r)) : "memory");
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
 #pragma unroll 16
@@ -572,17 +575,16 @@ __global__ void __launch_bounds__(128) kv_pool_kernel(const T* __restrict__ kv, 
         }
         if (c >= row) return;
     } else {
-        if (c >= row) return;
         constexpr int U = 16;
         int j = 0;
         for (; j + U <= pool; j += U) {
             T x[U];
 #pragma unroll
-            for (int u = 0; u < U; ++u) x[u] = place(j + u)[c];
+            for (int u = 0; u < U; ++u) x[u] = *place(j + u);
 #pragma unroll
             for (int u = 0; u < U; ++u) acc += to_f32(x[u]);
         }
-        for (; j < pool; ++j) acc += to_f32(place(j)[c]);
+        for (; j < pool; ++j) acc += to_f32(*place(j));
     }
     pool_cache[((int64_t)slot * pool_len + blk) * row + c] = from_f32<T>(acc / (float)pool);
 }
@@ -766,7 +768,7 @@ extern "C" int umbs_kv_pool(int dtype, const void* kv, const void* kv_cache, int
     if (kv_len < pool) return UMB_ERR_ARG;               // a block's older tokens must still sit in the cache
     cudaStream_t st = (cudaStream_t)stream;
     const dim3 grid(batch->max_seq_len / pool + 1, batch->n_seqs, (row + 127) / 128);
-    const bool vec = ((uintptr_t)kv | (uintptr_t)kv_cache) % 16 == 0 && row % 8 == 0;
+    const bool vec = pool >= 8 && ((uintptr_t)kv | (uintptr_t)kv_cache) % 16 == 0 && row % 8 == 0;
     UMBS_DISPATCH_T(dtype, chain_launch(vec ? kv_pool_kernel<T, true> : kv_pool_kernel<T, false>, grid, 128, 0, st, (const T*)kv,
                                         (const T*)kv_cache, kv_len, (T*)pool_cache, pool_len, *batch, row, pool));
     count_launches(1);
